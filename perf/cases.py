@@ -117,8 +117,7 @@ def _scales(g, groups, n):
 
 
 def _awq(g, k, n, group):
-    return PackedQuantLinear(QuantWeight.new_awq(4, _words(g, k, n // 8), _words(g, k // group, n // 8),
-                                                 _scales(g, k // group, n)))
+    return _words(g, k, n // 8), _words(g, k // group, n // 8), _scales(g, k // group, n)
 
 
 def _f16_bytes(v):
@@ -156,35 +155,49 @@ def _mxfp4_experts(g, experts, rows, k):
     return torch.stack([b for b, _ in made]), torch.stack([s for _, s in made])
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """The tensors of a case: activations and packed weights as a checkpoint holds them."""
     g = _gen(seed)
     m, kind = case["tokens"], case["kind"]
     if kind == "awq_layer":
         h, i, grp = case["hidden"], case["inter"], case["group"]
-        return {"kind": kind, "x": _x(g, m, h), "attn": _x(g, m, h), "ffn_in": _x(g, m, h),
-                "qkv": _awq(g, h, h + 2 * case["kv"], grp), "o": _awq(g, h, h, grp),
-                "ffn": GatedFfnProjection(_awq(g, h, 2 * i, grp), "silu"), "down": _awq(g, i, h, grp)}
+        return {"x": _x(g, m, h), "attn": _x(g, m, h), "ffn_in": _x(g, m, h), "qkv": _awq(g, h, h + 2 * case["kv"], grp),
+                "o": _awq(g, h, h, grp), "ffn": _awq(g, h, 2 * i, grp), "down": _awq(g, i, h, grp)}
     if kind == "moe":
         e, h, i = case["experts"], case["hidden"], case["inter"]
-        gu_b, gu_s = _mxfp4_experts(g, e, 2 * i, h)
-        dn_b, dn_s = _mxfp4_experts(g, e, h, i)
+        gate_up, down = _mxfp4_experts(g, e, 2 * i, h), _mxfp4_experts(g, e, h, i)
         small = lambda *shape: (torch.randn(*shape, generator=g, device="cuda") * 0.02).to(torch.bfloat16)  # noqa: E731
-        layer = GptOssMoe(gu_b, gu_s, small(e, 2 * i), dn_b, dn_s, small(e, h), h, i, top_k=case["top_k"],
-                          router_weight=small(e, h), router_bias=small(e))
-        return {"kind": kind, "x": _x(g, m, h), "layer": layer}
+        return {"gate_up": gate_up, "gate_up_bias": small(e, 2 * i), "down": down, "down_bias": small(e, h),
+                "router": small(e, h), "router_bias": small(e), "x": _x(g, m, h)}
     k, n = case["k"], case["n"]
     if kind == "gptq":
         zeros = None if case["sym"] else _words(g, k // case["group"], n // 8)
-        layer = PackedQuantLinear(QuantWeight.new_gptq(4, case["sym"], _words(g, k // 8, n), zeros,
-                                                       _scales(g, k // case["group"], n)))
+        weight = _words(g, k // 8, n), zeros, _scales(g, k // case["group"], n)
     elif kind == "gguf":
-        layer = QLinear(GGUF_TYPES[case["type"]], _gguf_blocks(g, case["type"], n, k), n, k)
+        weight = _gguf_blocks(g, case["type"], n, k)
     else:
         w = torch.randn(n // 128, 128, k // 128, 128, generator=g, device="cuda") * 0.02
         scale = w.abs().amax(dim=(1, 3)) / 448.0
-        w = (w / scale[:, None, :, None]).clamp(-448.0, 448.0).reshape(n, k).to(torch.float8_e4m3fn)
-        layer = Fp8Linear(w, scale)
-    return {"kind": kind, "x": _x(g, m, k), "layer": layer}
+        weight = (w / scale[:, None, :, None]).clamp(-448.0, 448.0).reshape(n, k).to(torch.float8_e4m3fn), scale
+    return {"x": _x(g, m, k), "weight": weight}
+
+
+def prepare(case, seed):
+    t, kind = _inputs(case, seed), case["kind"]
+    if kind == "awq_layer":
+        lin = {name: PackedQuantLinear(QuantWeight.new_awq(4, *t[name])) for name in ("qkv", "o", "ffn", "down")}
+        return {"kind": kind, "x": t["x"], "attn": t["attn"], "ffn_in": t["ffn_in"], "qkv": lin["qkv"], "o": lin["o"],
+                "ffn": GatedFfnProjection(lin["ffn"], "silu"), "down": lin["down"]}
+    if kind == "moe":
+        layer = GptOssMoe(*t["gate_up"], t["gate_up_bias"], *t["down"], t["down_bias"], case["hidden"], case["inter"],
+                          top_k=case["top_k"], router_weight=t["router"], router_bias=t["router_bias"])
+    elif kind == "gptq":
+        layer = PackedQuantLinear(QuantWeight.new_gptq(4, case["sym"], *t["weight"]))
+    elif kind == "gguf":
+        layer = QLinear(GGUF_TYPES[case["type"]], t["weight"], case["n"], case["k"])
+    else:
+        layer = Fp8Linear(*t["weight"])
+    return {"kind": kind, "x": t["x"], "layer": layer}
 
 
 def run(state):
@@ -233,3 +246,95 @@ def tolerance(case):
     """
     return {"awq_layer": {"rel": 1.8e-2, "max": 0.15}, "moe": {"rel": 1.2e-2, "max": 0.075}}.get(
         case["kind"], {"rel": 1e-2, "max": 0.05})
+
+
+# ---------------------------------------------------------------------------------------- the same in 64 bits, plain torch
+def _nibbles(words, order):
+    """The eight 4-bit codes of each 32-bit word, as a last dimension: code ``c`` from nibble ``order[c]``."""
+    return torch.stack([(words >> (4 * s)) & 15 for s in order], dim=-1)
+
+
+def _awq64(qweight, qzeros, scales):
+    k, (groups, n) = qweight.shape[0], scales.shape
+    order = (0, 4, 1, 5, 2, 6, 3, 7)  # the nibble that holds column 0, 1, ... of a word
+    q = _nibbles(qweight, order).reshape(groups, k // groups, n)
+    z = _nibbles(qzeros, order).reshape(groups, 1, n)
+    return ((q - z) * scales.double()[:, None]).reshape(k, n)
+
+
+def _gptq64(qweight, qzeros, scales):
+    (rows, n), groups = qweight.shape, scales.shape[0]
+    q = _nibbles(qweight, range(8)).permute(0, 2, 1).reshape(groups, 8 * rows // groups, n)
+    z = 8 if qzeros is None else _nibbles(qzeros, range(8)).reshape(groups, 1, n) + 1
+    return ((q - z) * scales.double()[:, None]).reshape(8 * rows, n)
+
+
+def _f16(raw):
+    return raw.contiguous().view(torch.float16).double()
+
+
+def _gguf64(type_, raw, n, k):
+    """``[n, k]`` from raw blocks."""
+    per, size = F.GGML_BLOCK[GGUF_TYPES[type_]]
+    b = raw.reshape(n, k // per, size)
+    if type_ == "Q4_0":
+        q = torch.cat([b[..., 2:] & 15, b[..., 2:] >> 4], dim=-1).double() - 8
+        return (_f16(b[..., :2]) * q).reshape(n, k)
+    if type_ == "Q8_0":
+        return (_f16(b[..., :2]) * b[..., 2:].view(torch.int8).double()).reshape(n, k)
+    if type_ == "Q4_K":  # eight sub-blocks of 32: 6-bit scales and minima in 12 bytes
+        p = b[..., 4:16]
+        sc = torch.cat([p[..., 0:4] & 63, (p[..., 8:12] & 15) | ((p[..., 0:4] >> 6) << 4)], dim=-1).double()
+        mn = torch.cat([p[..., 4:8] & 63, (p[..., 8:12] >> 4) | ((p[..., 4:8] >> 6) << 4)], dim=-1).double()
+        qs = b[..., 16:].reshape(n, -1, 4, 32)
+        q = torch.stack([qs & 15, qs >> 4], dim=-2).reshape(n, -1, 8, 32).double()
+        return ((_f16(b[..., 0:2]) * sc)[..., None] * q - (_f16(b[..., 2:4]) * mn)[..., None]).reshape(n, k)
+    low, high = b[..., :128].reshape(n, -1, 2, 1, 64), b[..., 128:192].reshape(n, -1, 2, 1, 32)
+    nib = torch.cat([low & 15, low >> 4], dim=-2).reshape(n, -1, 2, 4, 32)
+    two = torch.cat([(high >> (2 * j)) & 3 for j in range(4)], dim=-2)
+    q = (nib | (two << 4)).reshape(n, -1, 16, 16).double() - 32
+    return ((_f16(b[..., 208:]) * b[..., 192:208].view(torch.int8).double())[..., None] * q).reshape(n, k)
+
+
+def _mxfp4_64(blocks, scales):
+    """``[rows, k]`` of one expert."""
+    value = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], device="cuda", dtype=torch.float64)
+    codes = torch.stack([blocks & 15, blocks >> 4], dim=-1).reshape(*blocks.shape[:2], 32)
+    return (value[codes.long()] * torch.exp2(scales.double() - 127)[..., None]).reshape(blocks.shape[0], -1)
+
+
+def _moe64(case, t):
+    """Router logits are a bf16 linear's, rounded as such; all that follows them is in 64 bits."""
+    x, top = t["x"].double(), case["top_k"]
+    logits = (x @ t["router"].double().T + t["router_bias"].double()).to(torch.bfloat16).double()
+    best, chosen = torch.sort(torch.softmax(logits, dim=-1), dim=-1, descending=True, stable=True)
+    weight, chosen = best[:, :top] / best[:, :top].sum(-1, keepdim=True), chosen[:, :top]
+    out = torch.zeros_like(x)
+    for e in range(case["experts"]):
+        token, slot = torch.nonzero(chosen == e, as_tuple=True)
+        gu = x[token] @ _mxfp4_64(t["gate_up"][0][e], t["gate_up"][1][e]).T + t["gate_up_bias"][e].double()
+        gate, up = gu[:, 0::2].clamp(max=7.0), gu[:, 1::2].clamp(-7.0, 7.0)
+        h = (up + 1) * gate * torch.sigmoid(1.702 * gate)
+        y = h @ _mxfp4_64(t["down"][0][e], t["down"][1][e]).T + t["down_bias"][e].double()
+        out.index_add_(0, token, y * weight[token, slot][:, None])
+    return out
+
+
+def exact(case, seed):
+    t, kind = _inputs(case, seed), case["kind"]
+    x = t["x"].double()
+    if kind == "awq_layer":
+        gate, up = (t["ffn_in"].double() @ _awq64(*t["ffn"])).chunk(2, dim=-1)
+        act = torch.nn.functional.silu(gate) * up
+        return {"qkv": x @ _awq64(*t["qkv"]), "o": t["attn"].double() @ _awq64(*t["o"]), "ffn": act,
+                "down": act @ _awq64(*t["down"])}
+    if kind == "moe":
+        return _moe64(case, t)
+    if kind == "gptq":
+        return x @ _gptq64(*t["weight"])
+    if kind == "gguf":
+        return x @ _gguf64(case["type"], t["weight"], case["n"], case["k"]).T
+    w, scale = t["weight"]
+    n, k = w.shape
+    w = w.double().reshape(n // 128, 128, k // 128, 128) * scale.double()[:, None, :, None]
+    return x @ w.reshape(n, k).T

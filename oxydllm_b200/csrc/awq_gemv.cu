@@ -1055,7 +1055,7 @@ OXQ_EXPORT int oxq_awq_gemv(const void *x, int x_dtype, const uint32_t *qweight,
         const int gsteps = group_size / 16;
         const int n_tiles = ceil_div(p.packed_out, 8 * fv) * split;
         int r = 0;
-        for (int cand : {8, 4, 2, 1}) {
+        for (int cand : {8, 7, 6, 5, 4, 3, 2, 1}) { // any cluster size that leaves even slices (14336 x 4096: 24.6 us at 4, 18.9 at 7)
             if (total_steps % (GK_KW * cand) != 0) continue;
             const int sl = total_steps / (GK_KW * cand);
             if (!(sl % gsteps == 0 || gsteps % sl == 0) || sl % depth != 0) continue;

@@ -93,7 +93,7 @@ int oxq_awq_gemv_check(void *stream);
  * up_proj, ffn.rs:235-254): y[m, inter] = act(x . W_gate^T) * (x . W_up^T), act = 1 SiLU, 2 GeLU-tanh
  * (FeedForward::forward, ffn.rs:385-470; gated_silu_fused / gated_gelu_tanh_fused, metal_ops.rs:1243-1277).
  * x, y bf16. qweight u32 [k, 2*inter/8], qzeros u32 [k/g, 2*inter/8], scales [k/g, 2*inter].
- * m <= 16 runs the GEMV and a small activation kernel; 17 .. 256 tokens run the kernel that unpacks inside
+ * m <= 8 runs the GEMV and a small activation kernel; 9 .. 256 tokens run the kernel that unpacks inside
  * the tensor-core loop (on the shapes oxq_awq_gemm takes it for; the GEMV up to 32 tokens elsewhere) and the
  * same activation kernel; larger m dequantizes the weight with gate row j and up row j side by side and applies the activation in the tensor-core GEMM's epilogue (no
  * [m, 2*inter] round trip). Workspace as for oxq_awq_gemm with n = 2*inter; oxq_gemm_check applies. */
@@ -217,14 +217,23 @@ int oxq_gemm_check(const void *workspace, void *stream);
 
 /* PackedQuantLinear::forward beyond the decode GEMV: maybe_mpp_quant_matmul, else
  * dequantize_w4 + matmul (linear.rs:494-524, metal_ops.rs:2771-2797). Up to 256
- * tokens, when n % 128 == 0, k % 128 == 0, group_size is a power of two >= 64 and
- * the scales are f16 or bf16, one kernel unpacks the words into its shared-memory
- * operand and multiplies on tcgen05 (same bf16 weights, no slab written); all
- * other calls dequantize slabs into the workspace. The workspace is required
+ * tokens, when n % 128 == 0, k % 128 == 0, group_size is a power of two >= 32 (64
+ * above 128 tokens on wide layers) and the scales are f16 or bf16, one kernel unpacks
+ * the words into its shared-memory operand and multiplies on tcgen05 (no slab
+ * written); all other calls dequantize slabs into the workspace. The workspace is required
  * (and its flag word used) either way. */
 int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
                  int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                  int group_size, void *workspace, size_t workspace_bytes, void *stream);
+
+/* The kernel that oxq_awq_gemm / oxq_gptq_gemm (4-bit) run up to 128 tokens (256 on layers of at most 74 tiles of 128 out
+ * features), with scratch of its own: oxq_packed4_scratch_bytes(m, n) bytes with any contents, 256-byte aligned, one per
+ * call in flight. flag_word: the first word of a gemm workspace (oxq_gemm_check reads it). OXQ_ERR_UNSUPPORTED for shapes the
+ * kernel does not take. gptq = 0: AWQ layout (qzeros required); 1: GPTQ layout (sym != 0 or qzeros null: zero point 8). */
+size_t oxq_packed4_scratch_bytes(int m, int n);
+int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
+                       int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
+                       int group_size, int gptq, int sym, void *flag_word, void *scratch, size_t scratch_bytes, void *stream);
 
 /* Tensor-parallel column shard of the same matmul (no counterpart in the reference, which runs on one device; the
  * sharding rule is the column-slice property concat_awq_along_out relies on, awq.rs:256-323). The packed tensors are

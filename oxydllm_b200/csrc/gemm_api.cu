@@ -24,6 +24,12 @@ int mxfp4_dequant_rows_bf16(const uint8_t *blocks, const uint8_t *scales, __nv_b
 bool gguf_block_layout_host(int ggml_type, int &bel, int &bby);
 bool awq_fused_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
                          const void *scales);
+size_t group_tc_scratch_bytes(int m, int n);
+bool group_tc_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
+                        const void *scales);
+int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
+                    int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
+                    cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
 bool fp8_fused_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
 int fp8_fused_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in,
                      const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st,
@@ -31,6 +37,22 @@ int fp8_fused_matmul(const void *x, const uint8_t *weight, const float *scale_in
 int awq_fused_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy,
                      int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
+
+// The 4-bit matmuls without a dense copy of the weight: csrc/group_tc.cu, or csrc/fused_tc.cu for 129..256 tokens on wide layers.
+static bool packed4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
+                              const void *qzeros, const void *scales)
+{
+    return group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
+           (aligned(qzeros, 16) && awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales));
+}
+static int packed4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype,
+                          const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base,
+                          int ldy, int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes)
+{
+    auto run = group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ? group_tc_matmul : awq_fused_matmul;
+    return run(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base, ldy, flag, st, gptq,
+               sym, scratch, scratch_bytes);
+}
 
 constexpr size_t WS_HEADER = 256;                // flag word + padding, keeps the slab 256-byte aligned
 constexpr size_t SLAB_LIMIT_BYTES = 128u << 20;  // dequantized rows held at once (whole weight if it fits)
@@ -156,15 +178,42 @@ OXQ_EXPORT int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight,
     int rc = prepare("oxq_awq_gemm", c, x, x_dtype, bias, bias_dtype, y, y_dtype, m, k, n, workspace, workspace_bytes, stream);
     if (rc) return rc;
     // Up to 256 tokens: unpack inside the tensor-core kernel, no dense copy of the weight.
-    if (awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales))
+    if (packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales))
     {
-        rc = awq_fused_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n, c.flag,
+        rc = packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n, c.flag,
                               c.st, 0, 0, c.slab, c.slab_bytes);
         if (rc != OXQ_ERR_UNSUPPORTED) return rc;
     }
     return run_slabs(c, [&](int n_off, int cnt) {
         return awq_dequant_rows_bf16(qweight, qzeros, scales, scales_dtype, c.slab, k, n, group_size, n_off, cnt, c.st);
     });
+}
+
+// The same matmul for AWQ and GPTQ 4-bit with scratch of its own instead of the workspace's slab, so that calls on different
+// streams only share the flag word; OXQ_ERR_UNSUPPORTED where the kernel does not take the shape.
+OXQ_EXPORT size_t oxq_packed4_scratch_bytes(int m, int n)
+{
+    return m > 0 && n > 0 && n % 128 == 0 ? group_tc_scratch_bytes(m, n) : 0;
+}
+
+OXQ_EXPORT int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
+                                  int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
+                                  int group_size, int gptq, int sym, void *flag_word, void *scratch, size_t scratch_bytes, void *stream)
+{
+    clear_error();
+    const int use_sym = gptq && (sym != 0 || qzeros == nullptr);
+    OXQ_REQUIRE(x && y && qweight && scales && flag_word && (qzeros || use_sym), OXQ_ERR_NULL, "oxq_packed4_matmul: null pointer");
+    OXQ_REQUIRE(x_dtype == OXQ_BF16, OXQ_ERR_UNSUPPORTED, "oxq_packed4_matmul: activations must be bf16");
+    OXQ_REQUIRE(valid_dtype(scales_dtype) && valid_dtype(y_dtype) && (!bias || valid_dtype(bias_dtype)), OXQ_ERR_UNSUPPORTED,
+                "oxq_packed4_matmul: unsupported dtype");
+    OXQ_REQUIRE(m >= 1 && k > 0 && n > 0 && group_size > 0 && k % group_size == 0 && n % 8 == 0 && k % 8 == 0, OXQ_ERR_BAD_SHAPE,
+                "oxq_packed4_matmul: shape [%d, %d] incompatible with pack factor 8 / group size %d", n, k, group_size);
+    OXQ_REQUIRE(aligned(scratch, 256) && aligned(flag_word, 4), OXQ_ERR_BAD_ALIGN, "oxq_packed4_matmul: scratch must be 256-byte aligned");
+    if (use_sym) qzeros = nullptr;
+    OXQ_REQUIRE(group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales), OXQ_ERR_UNSUPPORTED,
+                "oxq_packed4_matmul: out_features %d, in_features %d, group size %d or the alignment are not served", n, k, group_size);
+    return group_tc_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n,
+                           reinterpret_cast<int *>(flag_word), (cudaStream_t)stream, gptq, use_sym, scratch, scratch_bytes);
 }
 
 // Column block [rows x chunks * 16 bytes] at byte offset col_off of every row of `src` -> the same place in each peer's
@@ -207,8 +256,8 @@ OXQ_EXPORT int oxq_awq_gemm_tp(const void *x, int x_dtype, const uint32_t *qweig
     if (rc) return rc;
     c.col_base = col_base; c.ldy = n_full;
     rc = OXQ_ERR_UNSUPPORTED;
-    if (awq_fused_supported(m, k, n_local, group_size, scales_dtype, x, qweight, scales)) // decode-sized batches: no slab
-        rc = awq_fused_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n_local, group_size,
+    if (packed4_supported(m, k, n_local, group_size, scales_dtype, x, qweight, qzeros, scales)) // decode-sized batches: no slab
+        rc = packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n_local, group_size,
                               col_base, n_full, c.flag, c.st, 0, 0, c.slab, c.slab_bytes);
     if (rc == OXQ_ERR_UNSUPPORTED)
         rc = run_slabs(c, [&](int n_off, int cnt) {
@@ -250,10 +299,9 @@ OXQ_EXPORT int oxq_gptq_gemm(const void *x, int x_dtype, const uint32_t *qweight
     int rc = prepare("oxq_gptq_gemm", c, x, x_dtype, bias, bias_dtype, y, y_dtype, m, k, n, workspace, workspace_bytes, stream);
     if (rc) return rc;
     // 4-bit, up to 256 tokens: unpack inside the tensor-core kernel (the same kernel as AWQ with the K-major operand).
-    if (bits == 4 && (use_sym || aligned(qzeros, 16)) &&
-        awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales))
+    if (bits == 4 && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, use_sym ? nullptr : qzeros, scales))
     {
-        rc = awq_fused_matmul(x, qweight, use_sym ? nullptr : qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n,
+        rc = packed4_matmul(x, qweight, use_sym ? nullptr : qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n,
                               group_size, 0, n, c.flag, c.st, 1, use_sym, c.slab, c.slab_bytes);
         if (rc != OXQ_ERR_UNSUPPORTED) return rc;
     }
@@ -396,10 +444,11 @@ OXQ_EXPORT int oxq_awq_ffn_gate_up(const void *x, int x_dtype, const uint32_t *q
         OXQ_LAUNCH_CHECK("gated_act_rows_kernel");
         return OXQ_OK;
     };
-    if (m > 16 && gu_bytes <= c.slab_bytes && awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales)) {
-        // Decode batches of 17 .. 256 tokens: the kernel that unpacks inside the tensor-core loop writes the
-        // row block (no dense copy of the weight); what the slab holds behind the block is its scratch.
-        rc = awq_fused_matmul(x, qweight, qzeros, scales, scales_dtype, nullptr, 0, c.slab, OXQ_BF16, m, k, n, group_size, 0, n,
+    if (m > 8 && gu_bytes <= c.slab_bytes && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales)) {
+        // The kernel that unpacks inside the tensor-core loop writes the row block (no dense copy of the weight); what the slab
+        // holds behind the block is its scratch. 2 x 14336 out features, k = 4096, at 8 / 16 tokens: the GEMV 33 / 48 us, this
+        // kernel 30 us.
+        rc = packed4_matmul(x, qweight, qzeros, scales, scales_dtype, nullptr, 0, c.slab, OXQ_BF16, m, k, n, group_size, 0, n,
                               c.flag, c.st, 0, 0, (unsigned char *)c.slab + gu_bytes, c.slab_bytes - gu_bytes);
         if (rc == OXQ_OK) return activate();
         if (rc != OXQ_ERR_UNSUPPORTED) return rc;

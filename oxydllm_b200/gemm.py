@@ -87,6 +87,24 @@ def awq_matmul(lin, x2, y):
               lin.group_size, _p(ws), ws.numel(), _st())
 
 
+def packed4_matmul(lin, x2, y):
+    """``y = x2 . deq(W) (+ bias)`` for the 4-bit layouts by the grouped unpack + tcgen05 kernel (``oxq_packed4_matmul``). The
+    scratch is this call's own, so calls on several streams do not meet; the workspace lends its flag word."""
+    from .linear import _dt
+    m, n = x2.shape[0], lin.out_features
+    ws = _workspaces.get(x2.device.index)
+    if ws is None:
+        ws = workspace(n, lin.in_features, x2.device)
+    need = lin._scratch_bytes.get(m)
+    if need is None:
+        need = lin._scratch_bytes[m] = int(_lib.load().oxq_packed4_scratch_bytes(m, n))
+    scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
+    qw, qz, sc, sc_dt, b, b_dt = lin._const
+    _lib.call("oxq_packed4_matmul", x2.data_ptr(), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, y.data_ptr(), _dt(y.dtype), m,
+              lin.in_features, n, lin.group_size, int(lin.pack_dim == "in"), int(lin.sym), ws.data_ptr(), scratch.data_ptr(), need,
+              torch._C._cuda_getCurrentRawStream(x2.device.index))
+
+
 def w8a16_matmul(lin, x2, y):
     """``y = x2 . deq(W)^T (+ bias)`` for the 8-bit AWQ layout (``oxq_w8a16_gemm``)."""
     from .linear import _dt

@@ -24,14 +24,18 @@ _DT = {torch.float32: _lib.OXQ_F32, torch.float16: _lib.OXQ_F16, torch.bfloat16:
 GEMV_MAX_M = 32
 #: The same for the GPTQ and 8-bit GEMVs (one 8-token chunk of the reference's batched GEMV, linear.rs:461-478).
 PACKED_SIMT_GEMV_MAX_M = 8
-# AWQ 4-bit layers whose shape the fused unpack + tcgen05 kernel serves (out_features % 128, in_features % 128,
-# group size a power of two >= 64, 16-bit scales) leave the split-k GEMV at this batch: measured on a 4096 x 14336 layer the GEMV
-# takes 24 us at 16 tokens and 47 us at 32, the fused kernel 28 to 31 us for any batch up to 128.
+# FP8 layers whose shape the fused unpack + tcgen05 kernel serves leave the GEMV at this batch: 24 us for up to 32 tokens on a
+# 14336 x 4096 layer against 25 / 45 us for the GEMV at 16 / 32.
 AWQ_FUSED_MIN_M = 17
-AWQ_FUSED_SPLIT_K_TILES = 74  # at most this many 128-row tiles: the fused kernel runs two or more k splits per tile
-# GPTQ 4-bit layers of such shapes: the GEMV takes 25 / 28 / 35 / 48 us at 1 / 2 / 4 / 8 tokens on the same layer, the fused
-# kernel 30 us for any batch up to 64.
-GPTQ_FUSED_MIN_M = 3
+# AWQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu) leave the GEMV above this batch: us at
+# 8 / 16 tokens, GEMV against kernel: 4096 x 4096 8.4 / 23.7 against 10, 4096 x 28672 33 / 48 against 28, whatever the batch up to 32.
+AWQ_GEMV_MAX_M = 8
+# ... and that kernel takes them to 128 tokens, or 256 where a layer has few tiles of 128 out features.
+GROUPED_MAX_M, GROUPED_NARROW_MAX_M, GROUPED_NARROW_TILES = 128, 256, 74
+# GPTQ 4-bit layers of such shapes: 4096 x 14336 takes 25 / 28 / 48 us at 1 / 2 / 8 tokens in the GEMV, 18 us in the kernel;
+# the GEMV is the faster one for a single token on layers of up to GPTQ_GEMV_MAX_WEIGHTS weights (2048 x 3072: 7.3 us against 8.1).
+GPTQ_FUSED_MIN_M = 2
+GPTQ_GEMV_MAX_WEIGHTS = 8 << 20
 
 
 def _dt(t: torch.dtype) -> int:
@@ -263,24 +267,41 @@ class PackedQuantLinear:
         self.bias = None if bias is None else bias.contiguous()
         self.dtype = dtype
         self._resident = all(t is None or t.is_cuda for t in (self.qweight, self.qzeros, self.scales, self.bias))
-        # constant arguments of the GEMV call, converted once
+        self._grouped_max_m, self._gemv_max_m = self._pick_batches()
+        self._scratch_bytes: dict = {}  # by batch
+        # constant arguments of the calls, converted once
         b = self.bias
         self._const = (_p(self.qweight), _p(self.qzeros), _p(self.scales), _dt(self.scales.dtype), _p(b),
                        _dt(b.dtype) if b is not None else 0)
 
     def gemv_max_m(self) -> int:
         """Largest batch the decode kernels take before the tensor-core GEMM is the better tool: 32 for the
-        4-bit AWQ tensor-core GEMV (16 where the fused unpack + tcgen05 kernel takes over), 8 (one chunk of the
-        reference's batched GEMV) for GPTQ and 8-bit (2 for 4-bit GPTQ shapes the fused kernel serves)."""
-        fused = (self.bits == 4 and self.out_features % 128 == 0 and self.in_features % 128 == 0 and self.group_size % 64 == 0
-                 and self.group_size & (self.group_size - 1) == 0 and self.scales.dtype in (torch.float16, torch.bfloat16))
-        if self.pack_dim == "out" and self.bits == 4:
-            if fused and self.out_features // 128 <= AWQ_FUSED_SPLIT_K_TILES:
-                return 8  # narrow layer: the fused kernel splits k over the SMs (4096 x 4096: 14 us at 16 tokens, GEMV 23 us)
-            return AWQ_FUSED_MIN_M - 1 if fused else GEMV_MAX_M
-        if fused:
-            return GPTQ_FUSED_MIN_M - 1
-        return PACKED_SIMT_GEMV_MAX_M
+        4-bit AWQ tensor-core GEMV, 8 (one chunk of the reference's batched GEMV) for GPTQ and 8-bit; on shapes the
+        grouped unpack + tcgen05 kernel serves, 8 for AWQ (0 where the GEMV cannot split k well) and 1 or 0 for GPTQ."""
+        return self._gemv_max_m
+
+    def _pick_batches(self):
+        """Largest batches of the grouped unpack + tcgen05 kernel (0: not this layer) and of the GEMV."""
+        k, n, g = self.in_features, self.out_features, self.group_size
+        awq = self.pack_dim == "out"
+        grouped = (self.bits == 4 and n % 128 == 0 and k % 128 == 0 and g >= 32 and g & (g - 1) == 0
+                   and self.scales.dtype in (torch.float16, torch.bfloat16)
+                   and all(t is None or t.data_ptr() % 16 == 0 for t in (self.qweight, self.qzeros, self.scales)))
+        if not grouped:
+            return 0, GEMV_MAX_M if awq and self.bits == 4 else PACKED_SIMT_GEMV_MAX_M
+        most = GROUPED_NARROW_MAX_M if n // 128 <= GROUPED_NARROW_TILES else GROUPED_MAX_M
+        if not awq:
+            return most, GPTQ_FUSED_MIN_M - 1 if k * n <= GPTQ_GEMV_MAX_WEIGHTS else 0
+        # The GEMV gives each of 4 warps x up to 8 CTAs a k slice of whole groups or an even part of one. Where that leaves few
+        # CTAs it is slow (11008 x 4096: 39 us against 15 us; 5632 x 4096: 27 to 47 us against 11 us), and on long k, where the
+        # slices are long, it loses from the first token on (14336 x 4096, groups of 128: 19 to 27 us against 18 us; with groups of
+        # 32 its 25 to 32 us stand against 33 us).
+        steps, per_group = k // 16, g // 16
+        split = max((r for r in range(1, 9) if steps % (4 * r) == 0 and steps // (4 * r) % 2 == 0
+                     and (steps // (4 * r) % per_group == 0 or per_group % (steps // (4 * r)) == 0)), default=0)
+        if k >= 2048 and (split == 0 or n // 128 * split < 64 or (k > 8192 and g >= 64)):
+            return most, 0
+        return most, AWQ_GEMV_MAX_M
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""
@@ -297,11 +318,13 @@ class PackedQuantLinear:
             y = out
         if m == 0:
             return y.reshape(*lead, self.out_features)
-        if m <= self.gemv_max_m():
+        if m <= self._gemv_max_m:
             self._gemv(x2, y, m)
         else:
             from . import gemm
-            if self.pack_dim == "out" and self.bits == 4:
+            if m <= self._grouped_max_m and x2.data_ptr() % 16 == 0:
+                gemm.packed4_matmul(self, x2, y)
+            elif self.pack_dim == "out" and self.bits == 4:
                 gemm.awq_matmul(self, x2, y)
             elif self.pack_dim == "out":
                 gemm.w8a16_matmul(self, x2, y)

@@ -1,0 +1,75 @@
+"""The grouped unpack + tcgen05 kernel of the 4-bit layouts (``oxq_packed4_matmul``): sizes at its edges.
+
+Products of integers and bf16 values are exact, a group's sum and the totals are kept in f32: against 64-bit sums over the
+exact weights a value is off by a few dozen f32 roundings of the sum of |x w| at most, so 2^-17 of that sum bounds it (plus one
+bf16 rounding where y is bf16).
+"""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from oxydllm_b200 import gemm, synth
+from oxydllm_b200 import linear as L
+
+pytestmark = pytest.mark.gpu
+
+
+def layer(k, n, g, gptq, seed):
+    rng = np.random.default_rng(seed)
+    shape_w, shape_z = ((k // 8, n), (k // g, n // 8)) if gptq else ((k, n // 8), (k // g, n // 8))
+    qw, qz = (rng.integers(0, 2**32, size=s, dtype=np.uint64).astype(np.uint32) for s in (shape_w, shape_z))
+    sc = (np.abs(rng.standard_normal((k // g, n)) * 0.02) / 7 + 1e-4).astype(np.float16)
+    new = (lambda *a: L.QuantWeight.new_gptq(4, False, *a)) if gptq else (lambda *a: L.QuantWeight.new_awq(4, *a))
+    lin = L.PackedQuantLinear(new(*(torch.from_numpy(a.view(np.int32)).cuda() for a in (qw, qz)), torch.from_numpy(sc).cuda()))
+    return lin, (oracle.gptq_dequant(qw, qz, sc, 4, False) if gptq else oracle.awq_dequant(qw, qz, sc)).astype(np.float64)
+
+
+def check(y, x, w):
+    ref, mass = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    rounding = 2.0**-8 * np.abs(ref) if y.dtype == torch.bfloat16 else 0.0
+    assert (np.abs(y.double().cpu().numpy() - ref) <= 2.0**-17 * mass + rounding).all()
+
+
+# one unit and one tile; units beyond every ring (k = 5632); groups of 32, 64, 128 and more; tiles shared by two, three and many
+# CTAs; whole tiles (148 of them); one token, the edges of the tile widths and two tiles of tokens
+@pytest.mark.parametrize("gptq", [False, True])
+@pytest.mark.parametrize("k,n,g", [(128, 128, 32), (5632, 256, 32), (5632, 128, 64), (2048, 1152, 128), (1024, 18944, 256)])
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 97, 128, 129, 256])
+def test_grouped_kernel_matches_64_bit_sums(cuda, m, k, n, g, gptq):
+    if m > 128 and n // 128 > L.GROUPED_NARROW_TILES:
+        pytest.skip("wide layers leave the kernel above 128 tokens")
+    lin, w = layer(k, n, g, gptq, seed=k + n + m)
+    x = synth.activations(m, k, seed=m)
+    xd = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    gemm.packed4_matmul(lin, xd, y)
+    check(y, x, w)
+    again = torch.empty_like(y)
+    gemm.packed4_matmul(lin, xd, again)
+    assert torch.equal(y, again)  # the parts of a shared tile are added in the order of k, not of arrival
+    if m > lin.gemv_max_m():
+        check(lin.forward(xd), x, w)
+    gemm.check(gemm.workspace(n, k, "cuda"))
+
+
+def test_calls_on_two_streams_and_a_replayed_graph_do_not_meet(cuda):
+    lin, w = layer(4096, 1024, 128, False, seed=5)
+    xs = [torch.from_numpy(np.ascontiguousarray(synth.activations(48, 4096, seed=s))).to(torch.bfloat16).cuda() for s in range(2)]
+    want = [lin.forward(x) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = [[], []]
+    for _ in range(20):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[i].append(lin.forward(xs[i]))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = lin.forward(xs[0])
+    for _ in range(3):
+        y.zero_()
+        graph.replay()
+        assert torch.equal(y, want[0])

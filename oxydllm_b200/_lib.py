@@ -44,6 +44,7 @@ SIGNATURES = {
     "oxq_awq_gemv_check": [_vp],
     "oxq_gemm_workspace_init": [_vp, _vp],
     "oxq_awq_gemm": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp],
+    "oxq_packed4_max_m": [_i, _i, _i],
     "oxq_packed4_scratch_bytes": [_i, _i],
     "oxq_packed4_matmul": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _sz, _vp],
     "oxq_awq_gemm_tp": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp],
@@ -100,10 +101,24 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+_entries: dict = {}
+
+
+def entry(name: str):
+    """The entry point itself, for callers that make the same call again and again (``fail`` if it returns non-zero)."""
+    fn = _entries.get(name)
+    if fn is None:
+        fn = _entries[name] = getattr(load(), name)
+    return fn
+
+
+def fail(name: str, rc: int) -> None:
+    lib = load()
+    raise OxqError(name, rc, lib.oxq_last_error().decode() or lib.oxq_status_string(rc).decode())
+
+
 def call(name: str, *args) -> None:
     """Call an entry point; raise :class:`OxqError` with the library's message on failure."""
-    lib = load()
-    rc = getattr(lib, name)(*args)
+    rc = entry(name)(*args)
     if rc != 0:
-        msg = lib.oxq_last_error().decode() or lib.oxq_status_string(rc).decode()
-        raise OxqError(name, rc, msg)
+        fail(name, rc)

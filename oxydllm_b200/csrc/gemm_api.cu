@@ -25,6 +25,7 @@ bool gguf_block_layout_host(int ggml_type, int &bel, int &bby);
 bool awq_fused_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
                          const void *scales);
 size_t group_tc_scratch_bytes(int m, int n);
+int group_tc_max_m(int n, int group_size);
 bool group_tc_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
                         const void *scales);
 int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
@@ -38,7 +39,7 @@ int awq_fused_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy,
                      int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
 
-// The 4-bit matmuls without a dense copy of the weight: csrc/group_tc.cu, or csrc/fused_tc.cu for 129..256 tokens on wide layers.
+// The 4-bit matmuls without a dense copy of the weight: csrc/group_tc.cu up to group_tc_max_m tokens, then csrc/fused_tc.cu up to 256.
 static bool packed4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
                               const void *qzeros, const void *scales)
 {
@@ -191,6 +192,12 @@ OXQ_EXPORT int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight,
 
 // The same matmul for AWQ and GPTQ 4-bit with scratch of its own instead of the workspace's slab, so that calls on different
 // streams only share the flag word; OXQ_ERR_UNSUPPORTED where the kernel does not take the shape.
+OXQ_EXPORT int oxq_packed4_max_m(int k, int n, int group_size)
+{
+    return k > 0 && n > 0 && n % 128 == 0 && k % 128 == 0 && group_size >= 32 && (group_size & (group_size - 1)) == 0
+               ? group_tc_max_m(n, group_size) : 0;
+}
+
 OXQ_EXPORT size_t oxq_packed4_scratch_bytes(int m, int n)
 {
     return m > 0 && n > 0 && n % 128 == 0 ? group_tc_scratch_bytes(m, n) : 0;

@@ -563,15 +563,26 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     }
 }
 
-// True when this kernel serves the call. More than 128 tokens are two tiles that unpack the same weights twice: worth it where
-// that fills idle SMs (256 tokens, 4096 x 4096: 23 us against 34 us in the kernel of fused_tc.cu; 4096 x 14336: 51 us against 41 us).
+// Largest batch for this kernel. Above it the kernel of fused_tc.cu, which scales and rounds the weights as it unpacks them and
+// folds nothing, is the faster one, us there / here: groups of 64, where every stage is folded, 3072 x 5120 at 16 / 77 tokens
+// 14.6 / 12.8 and 18.9 / 21.6, 3072 x 16384 25.4 / 18.6 and 26.6 / 34.5, but 8192 x 3072 at 77 26.3 / 24.6; one tile per CTA, 4096 x
+// 14336, 31.1 / 32.9 at 128 tokens. More than 128 tokens are two tiles that unpack the same weights twice: worth it where that
+// fills idle SMs (256 tokens, 4096 x 4096: 34 / 23; 4096 x 14336: 41 / 51). Groups of 32 have no other such kernel (4096 x 14336
+// through the dense copy: 71 us).
+int group_tc_max_m(int n, int group_size)
+{
+    const int tiles = n / GT_ROWS;
+    if (group_size == 64 && tiles > 32) return 48;
+    return tiles <= GT_NARROW_TILES ? GROUP_TC_MAX_M : tiles <= 148 && group_size > 32 ? 96 : GT_MAX_TOKENS;
+}
+
+// True when this kernel serves the call.
 bool group_tc_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
                         const void *scales)
 {
-    return m >= 1 && (m <= GT_MAX_TOKENS || (m <= GROUP_TC_MAX_M && n / GT_ROWS <= GT_NARROW_TILES)) && n % GT_ROWS == 0 &&
-           k % GT_UNIT == 0 && group_size >= 32 && (group_size & (group_size - 1)) == 0 &&
-           (scales_dtype == OXQ_F16 || scales_dtype == OXQ_BF16) && aligned(x, 16) && aligned(qweight, 16) && aligned(qzeros, 16) &&
-           aligned(scales, 16);
+    return m >= 1 && m <= group_tc_max_m(n, group_size) && n % GT_ROWS == 0 && k % GT_UNIT == 0 && group_size >= 32 &&
+           (group_size & (group_size - 1)) == 0 && (scales_dtype == OXQ_F16 || scales_dtype == OXQ_BF16) && aligned(x, 16) &&
+           aligned(qweight, 16) && aligned(qzeros, 16) && aligned(scales, 16);
 }
 
 static size_t group_tc_ticket_bytes(int tiles) { return ((size_t)tiles * sizeof(unsigned long long) + 255) / 256 * 256; }

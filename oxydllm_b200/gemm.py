@@ -12,11 +12,20 @@ import torch
 
 from . import _lib
 
+_DT = {torch.float32: _lib.OXQ_F32, torch.float16: _lib.OXQ_F16, torch.bfloat16: _lib.OXQ_BF16}
+
+
+def _dt(t: torch.dtype) -> int:
+    try:
+        return _DT[t]
+    except KeyError:
+        raise ValueError(f"unsupported dtype {t}") from None
+
 _workspaces: dict = {}
 
 
 def workspace_bytes(n: int, k: int) -> int:
-    return int(_lib.load().oxq_gemm_workspace_bytes(n, k))
+    return int(_lib.entry("oxq_gemm_workspace_bytes")(n, k))
 
 
 def workspace(n: int, k: int, device) -> torch.Tensor:
@@ -34,7 +43,7 @@ _decode_ws: dict = {}
 
 
 def _dev_index(device) -> int:
-    idx = torch.device(device).index
+    idx = (device if isinstance(device, torch.device) else torch.device(device)).index
     return torch.cuda.current_device() if idx is None else idx
 
 
@@ -51,7 +60,6 @@ def decode_workspace(m: int, k: int, n: int, device) -> torch.Tensor:
 
 def awq_decode_matmul(lin, x2, y):
     """``y = x2 . deq(W)`` for decode-sized batches on the tensor cores (``oxq_awq_decode_matmul``)."""
-    from .linear import _dt
     ws = decode_workspace(x2.shape[0], lin.in_features, lin.out_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_awq_decode_matmul", _p(x2), _dt(x2.dtype), _p(lin.qweight), _p(lin.qzeros), _p(lin.scales),
@@ -65,21 +73,19 @@ def check(ws: torch.Tensor) -> None:
               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
 
 
-def _p(t):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _p(t) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def _st():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _st() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _bias(b):
-    from .linear import _dt
     return _p(b), (_dt(b.dtype) if b is not None else 0)
 
 
 def awq_matmul(lin, x2, y):
-    from .linear import _dt
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_awq_gemm", _p(x2), _dt(x2.dtype), _p(lin.qweight), _p(lin.qzeros), _p(lin.scales),
@@ -90,7 +96,6 @@ def awq_matmul(lin, x2, y):
 def packed4_matmul(lin, x2, y):
     """``y = x2 . deq(W) (+ bias)`` for the 4-bit layouts by the grouped unpack + tcgen05 kernel (``oxq_packed4_matmul``). The
     scratch is this call's own, so calls on several streams do not meet; the workspace lends its flag word."""
-    from .linear import _dt
     m, n = x2.shape[0], lin.out_features
     ws = _workspaces.get(x2.device.index)
     if ws is None:
@@ -102,12 +107,11 @@ def packed4_matmul(lin, x2, y):
     qw, qz, sc, sc_dt, b, b_dt = lin._const
     _lib.call("oxq_packed4_matmul", x2.data_ptr(), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, y.data_ptr(), _dt(y.dtype), m,
               lin.in_features, n, lin.group_size, int(lin.pack_dim == "in"), int(lin.sym), ws.data_ptr(), scratch.data_ptr(), need,
-              torch._C._cuda_getCurrentRawStream(x2.device.index))
+              _st())
 
 
 def w8a16_matmul(lin, x2, y):
     """``y = x2 . deq(W)^T (+ bias)`` for the 8-bit AWQ layout (``oxq_w8a16_gemm``)."""
-    from .linear import _dt
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_w8a16_gemm", _p(x2), _dt(x2.dtype), _p(lin.qweight), _p(lin.qzeros), _p(lin.scales),
@@ -132,15 +136,12 @@ def gptq_matmul(raw, x2, y, bias=None):
 
 def awq_ffn_gate_up(lin, x2, y, activation: int):
     """``y[m, inter] = act(x . W_gate^T) * (x . W_up^T)`` on the fused ``[gate | up]`` AWQ linear ``lin``."""
-    from .linear import _dt
     ws = workspace(lin.out_features, lin.in_features, x2.device)
-    _lib.call("oxq_awq_ffn_gate_up", _p(x2), _dt(x2.dtype), _p(lin.qweight), _p(lin.qzeros), _p(lin.scales),
-              _dt(lin.scales.dtype), activation, _p(y), x2.shape[0], lin.in_features, lin.out_features // 2,
+    _lib.call("oxq_awq_ffn_gate_up", x2.data_ptr(), _lib.OXQ_BF16, *lin._const[:4], activation, y.data_ptr(), x2.shape[0], lin.in_features, lin.out_features // 2,
               lin.group_size, _p(ws), ws.numel(), _st())
 
 
 def fp8_matmul(lin, s, s_out, s_in, x2, y):
-    from .linear import _dt
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_fp8_gemm", _p(x2), _dt(x2.dtype), _p(lin.weight), _p(s), s_out, s_in, bp, bd, _p(y), _dt(y.dtype),
@@ -148,7 +149,6 @@ def fp8_matmul(lin, s, s_out, s_in, x2, y):
 
 
 def gguf_matmul(lin, x2, y):
-    from .linear import _dt
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_gguf_gemm", lin.ggml_type, _p(x2), _dt(x2.dtype), _p(lin.blocks), bp, bd, _p(y), _dt(y.dtype),
@@ -156,7 +156,6 @@ def gguf_matmul(lin, x2, y):
 
 
 def mxfp4_matmul(lin, x2, y):
-    from .linear import _dt
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_mxfp4_gemm", _p(x2), _dt(x2.dtype), _p(lin.blocks), _p(lin.scales), bp, bd, _p(y), _dt(y.dtype),

@@ -9,16 +9,14 @@ CPU path.
 """
 from __future__ import annotations
 
-import ctypes
 from dataclasses import dataclass
 from typing import Optional
 
 import torch
 
-from . import _lib
+from . import _lib, gemm
 from .formats import GGML_BLOCK
-
-_DT = {torch.float32: _lib.OXQ_F32, torch.float16: _lib.OXQ_F16, torch.bfloat16: _lib.OXQ_BF16}
+from .gemm import _dt
 
 #: Largest m handled by the decode GEMV kernels; larger batches go to the tensor-core GEMM.
 GEMV_MAX_M = 32
@@ -30,28 +28,19 @@ AWQ_FUSED_MIN_M = 17
 # AWQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu) leave the GEMV above this batch: us at
 # 8 / 16 tokens, GEMV against kernel: 4096 x 4096 8.4 / 23.7 against 10, 4096 x 28672 33 / 48 against 28, whatever the batch up to 32.
 AWQ_GEMV_MAX_M = 8
-# ... and that kernel takes them to 128 tokens, or 256 where a layer has few tiles of 128 out features.
-GROUPED_MAX_M, GROUPED_NARROW_MAX_M, GROUPED_NARROW_TILES = 128, 256, 74
 # GPTQ 4-bit layers of such shapes: 4096 x 14336 takes 25 / 28 / 48 us at 1 / 2 / 8 tokens in the GEMV, 18 us in the kernel;
 # the GEMV is the faster one for a single token on layers of up to GPTQ_GEMV_MAX_WEIGHTS weights (2048 x 3072: 7.3 us against 8.1).
 GPTQ_FUSED_MIN_M = 2
 GPTQ_GEMV_MAX_WEIGHTS = 8 << 20
 
 
-def _dt(t: torch.dtype) -> int:
-    try:
-        return _DT[t]
-    except KeyError:
-        raise ValueError(f"unsupported dtype {t}") from None
+def _p(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def _p(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
-
-
-def _stream():
+def _stream() -> int:
     # raw handle of torch's current stream on the current device, without building a Stream object
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _require_cuda(*tensors):
@@ -273,6 +262,9 @@ class PackedQuantLinear:
         b = self.bias
         self._const = (_p(self.qweight), _p(self.qzeros), _p(self.scales), _dt(self.scales.dtype), _p(b),
                        _dt(b.dtype) if b is not None else 0)
+        self._const_shape = (self.in_features, self.out_features, self.group_size)
+        if self.pack_dim == "in":
+            self._const_shape += (self.bits, int(self.sym))
 
     def gemv_max_m(self) -> int:
         """Largest batch the decode kernels take before the tensor-core GEMM is the better tool: 32 for the
@@ -289,7 +281,7 @@ class PackedQuantLinear:
                    and all(t is None or t.data_ptr() % 16 == 0 for t in (self.qweight, self.qzeros, self.scales)))
         if not grouped:
             return 0, GEMV_MAX_M if awq and self.bits == 4 else PACKED_SIMT_GEMV_MAX_M
-        most = GROUPED_NARROW_MAX_M if n // 128 <= GROUPED_NARROW_TILES else GROUPED_MAX_M
+        most = int(_lib.load().oxq_packed4_max_m(k, n, g))
         if not awq:
             return most, GPTQ_FUSED_MIN_M - 1 if k * n <= GPTQ_GEMV_MAX_WEIGHTS else 0
         # The GEMV gives each of 4 warps x up to 8 CTAs a k slice of whole groups or an even part of one. Where that leaves few
@@ -309,20 +301,17 @@ class PackedQuantLinear:
         if not (self._resident and x2.is_cuda):
             _require_cuda(x2, self.qweight, self.qzeros, self.scales, self.bias)
         if out is None:
-            y = torch.empty((m, self.out_features), dtype=x2.dtype, device=x2.device)
+            y = x2.new_empty((m, self.out_features))
         else:
             if (out.shape != (m, self.out_features) or out.dtype != x2.dtype or out.device != x2.device
                     or not out.is_contiguous()):
                 raise ValueError(f"PackedQuantLinear: out must be a contiguous [{m}, {self.out_features}] {x2.dtype} tensor "
                                  f"on {x2.device}")
             y = out
-        if m == 0:
-            return y.reshape(*lead, self.out_features)
-        if m <= self._gemv_max_m:
-            self._gemv(x2, y, m)
-        else:
-            from . import gemm
-            if m <= self._grouped_max_m and x2.data_ptr() % 16 == 0:
+        if m:
+            if m <= self._gemv_max_m:
+                self._gemv(x2, y, m)
+            elif m <= self._grouped_max_m and x2.data_ptr() % 16 == 0:
                 gemm.packed4_matmul(self, x2, y)
             elif self.pack_dim == "out" and self.bits == 4:
                 gemm.awq_matmul(self, x2, y)
@@ -330,19 +319,14 @@ class PackedQuantLinear:
                 gemm.w8a16_matmul(self, x2, y)
             else:
                 gemm.gptq_matmul(self, x2, y, self.bias)
-        return y.reshape(*lead, self.out_features)
+        return y if x2 is x else y.reshape(*lead, self.out_features)
 
     def _gemv(self, x2, y, m):
-        qw, qz, sc, sc_dt, b, b_dt = self._const
-        if self.pack_dim == "out" and self.bits == 4:
-            _lib.call("oxq_awq_gemv", _p(x2), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, _p(y), _dt(y.dtype), m,
-                      self.in_features, self.out_features, self.group_size, _stream())
-        elif self.pack_dim == "out":
-            _lib.call("oxq_w8a16_gemv", _p(x2), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, _p(y), _dt(y.dtype), m,
-                      self.in_features, self.out_features, self.group_size, _stream())
-        else:
-            _lib.call("oxq_gptq_gemv", _p(x2), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, _p(y), _dt(y.dtype), m,
-                      self.in_features, self.out_features, self.group_size, self.bits, int(self.sym), _stream())
+        dt = _dt(x2.dtype)
+        name = "oxq_gptq_gemv" if self.pack_dim == "in" else "oxq_awq_gemv" if self.bits == 4 else "oxq_w8a16_gemv"
+        rc = _lib.entry(name)(x2.data_ptr(), dt, *self._const, y.data_ptr(), dt, m, *self._const_shape, _stream())
+        if rc:
+            _lib.fail(name, rc)
 
     # the attributes gemm.gptq_matmul reads from a QuantWeight
     def pack_factor(self) -> int:
@@ -378,14 +362,14 @@ class GatedFfnProjection:
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lin = self.gate_up
         x2, lead, m = _flatten_x(x, lin.in_features, "GatedFfnProjection")
-        _require_cuda(x2, lin.qweight, lin.qzeros, lin.scales)
+        if not (lin._resident and x2.is_cuda):
+            _require_cuda(x2, lin.qweight, lin.qzeros, lin.scales)
         if x2.dtype != torch.bfloat16:
             raise ValueError("GatedFfnProjection: activations must be bf16")
-        y = torch.empty((m, self.intermediate), dtype=x2.dtype, device=x2.device)
+        y = x2.new_empty((m, self.intermediate))
         if m:
-            from . import gemm
             gemm.awq_ffn_gate_up(lin, x2, y, ACTIVATIONS[self.activation])
-        return y.reshape(*lead, self.intermediate)
+        return y if x2 is x else y.reshape(*lead, self.intermediate)
 
 
 class Fp8Linear:
@@ -411,7 +395,8 @@ class Fp8Linear:
         s = self.scale_inv
         if s is None:
             return None, 0, 0
-        s = s.to(torch.float32)
+        if s.dtype != torch.float32:
+            s = s.to(torch.float32)
         if s.dim() == 2:
             pass
         elif s.dim() == 1:
@@ -454,18 +439,15 @@ class Fp8Linear:
         s, s_out, s_in = self._grid()
         x2, lead, m = _flatten_x(x, self.in_features, "Fp8Linear")
         _require_cuda(x2, self.weight, self.bias)
-        y = torch.empty((m, self.out_features), dtype=x2.dtype, device=x2.device)
-        if m == 0:
-            return y.reshape(*lead, self.out_features)
-        if m <= self.gemv_max_m(s_out, s_in):
+        y = x2.new_empty((m, self.out_features))
+        if m and m <= self.gemv_max_m(s_out, s_in):
             b = self.bias
-            _lib.call("oxq_fp8_gemv", _p(x2), _dt(x2.dtype), _p(self.weight), _p(s), s_out, s_in, _p(b),
-                      _dt(b.dtype) if b is not None else 0, _p(y), _dt(y.dtype), m, self.in_features,
+            _lib.call("oxq_fp8_gemv", x2.data_ptr(), _dt(x2.dtype), self.weight.data_ptr(), _p(s), s_out, s_in, _p(b),
+                      _dt(b.dtype) if b is not None else 0, y.data_ptr(), _dt(y.dtype), m, self.in_features,
                       self.out_features, _stream())
-        else:
-            from . import gemm
+        elif m:
             gemm.fp8_matmul(self, s, s_out, s_in, x2, y)
-        return y.reshape(*lead, self.out_features)
+        return y if x2 is x else y.reshape(*lead, self.out_features)
 
 
 class QLinear:
@@ -504,18 +486,15 @@ class QLinear:
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         x2, lead, m = _flatten_x(x, self.in_features, "QLinear")
         _require_cuda(x2, self.blocks, self.bias)
-        y = torch.empty((m, self.out_features), dtype=self.out_dtype, device=x2.device)
-        if m == 0:
-            return y.reshape(*lead, self.out_features)
-        if m <= GEMV_MAX_M:
+        y = x2.new_empty((m, self.out_features), dtype=self.out_dtype)
+        if m and m <= GEMV_MAX_M:
             b = self.bias
-            _lib.call("oxq_gguf_gemv", self.ggml_type, _p(x2), _dt(x2.dtype), _p(self.blocks), _p(b),
-                      _dt(b.dtype) if b is not None else 0, _p(y), _dt(y.dtype), m, self.in_features,
+            _lib.call("oxq_gguf_gemv", self.ggml_type, x2.data_ptr(), _dt(x2.dtype), self.blocks.data_ptr(), _p(b),
+                      _dt(b.dtype) if b is not None else 0, y.data_ptr(), _dt(self.out_dtype), m, self.in_features,
                       self.out_features, _stream())
-        else:
-            from . import gemm
+        elif m:
             gemm.gguf_matmul(self, x2, y)
-        return y.reshape(*lead, self.out_features)
+        return y if x2 is x else y.reshape(*lead, self.out_features)
 
 
 class Mxfp4Linear:
@@ -555,7 +534,6 @@ class Mxfp4Linear:
                       _dt(b.dtype) if b is not None else 0, _p(y), _dt(y.dtype), m, self.in_features,
                       self.out_features, _stream())
         else:
-            from . import gemm
             gemm.mxfp4_matmul(self, x2, y)
         return y.reshape(*lead, self.out_features)
 

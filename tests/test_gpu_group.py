@@ -37,9 +37,9 @@ def check(y, x, w):
 @pytest.mark.parametrize("k,n,g", [(128, 128, 32), (5632, 256, 32), (5632, 128, 64), (2048, 1152, 128), (1024, 18944, 256)])
 @pytest.mark.parametrize("m", [1, 16, 17, 33, 97, 128, 129, 256])
 def test_grouped_kernel_matches_64_bit_sums(cuda, m, k, n, g, gptq):
-    if m > 128 and n // 128 > L.GROUPED_NARROW_TILES:
-        pytest.skip("wide layers leave the kernel above 128 tokens")
     lin, w = layer(k, n, g, gptq, seed=k + n + m)
+    if m > lin._grouped_max_m:
+        pytest.skip("wide layers leave the kernel earlier")
     x = synth.activations(m, k, seed=m)
     xd = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
     y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")

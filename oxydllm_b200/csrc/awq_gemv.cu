@@ -35,6 +35,8 @@ namespace cg = cooperative_groups;
 
 namespace oxq {
 
+int q6k_gemv_take_flag(int &flag); // q6k_gemv.cu
+
 constexpr int GEMV_STAGES = 8;
 
 #ifdef OXQ_TUNING
@@ -1114,8 +1116,12 @@ OXQ_EXPORT int oxq_awq_gemv_check(void *stream)
         const int zero = 0;
         OXQ_CUDA(cudaMemcpyToSymbol(g_awq_gemv_flag, &zero, sizeof(int)));
     }
+    int other = 0;
+    const int rc = q6k_gemv_take_flag(other);
+    if (rc) return rc;
+    flag |= other;
     OXQ_REQUIRE(flag == 0, OXQ_ERR_DEVICE_FLAG,
-                "oxq_awq_gemv: a bounded wait on a weight box ran out in a call since the last check (outputs of those calls are not valid)");
+                "oxq_awq_gemv, oxq_gguf_gemv: a bounded wait on a weight box ran out in a call since the last check (outputs of those calls are not valid)");
     return OXQ_OK;
 }
 

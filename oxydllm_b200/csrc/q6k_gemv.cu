@@ -22,6 +22,7 @@
 #include <cstdlib>
 
 #include "oxq_common.cuh"
+#include "tc_common.cuh"
 
 namespace oxq {
 
@@ -207,6 +208,256 @@ __global__ void __launch_bounds__(256, 3) q6k_gemv_kernel(const Q6kGemvParams p)
     if (ks > 1) cluster.sync(); // nobody leaves while a peer may still read its shared memory
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Wide layers (the vocabulary projection), m <= 8: one CTA per SM walks 16-row tiles, x staged once for all of them.
+//
+// A CTA holds two engines that take its tiles in turn: a producer warp that copies stages of 16 rows x 8 super-blocks
+// (16 bulk copies of 1680 bytes) into the engine's ring, and eight warps that take one super-block of the stage each, so the k
+// split is the warp and a row's alignment (every other super-block starts 2 bytes off a word) is a constant of the warp. The rows'
+// pitch of 420 words puts the 8 rows x 4 words of a fragment read on distinct banks. 6-bit values become f16 1024 + v, minus 1056
+// exactly, so no sums of x are needed; a step's accumulators are multiplied by d * scale in f32.
+//
+// What bounds it: instruction issue, about 3.6 per weight (9.1 in the kernel above, which stages x in every CTA, loads every
+// word of a misaligned super-block as halfwords from global memory and folds sums of x).
+constexpr int Q6W_ROWS = 16, Q6W_SB = 8, Q6W_ENGINES = 2, Q6W_WARPS = 8;
+constexpr int Q6W_ROW_BYTES = Q6W_SB * 210, Q6W_STAGE_BYTES = Q6W_ROWS * Q6W_ROW_BYTES;
+constexpr int Q6W_THREADS = Q6W_ENGINES * (Q6W_WARPS + 1) * 32, Q6W_MAX_RING = 4;
+constexpr int Q6W_RED = Q6W_WARPS * 4 * 32; // floats of one tile's partial sums
+static_assert(Q6W_ROW_BYTES % 16 == 0, "bulk copies");
+
+__device__ int g_q6k_gemv_flag; // a bounded wait ran out
+
+struct Q6kWideParams {
+    const __nv_bfloat16 *x;
+    const uint8_t *blocks;
+    const void *bias;
+    void *y;
+    int bias_dtype, y_dtype;
+    int m, k, n, tiles, ring;
+};
+
+__device__ __forceinline__ uint32_t q6w_lds32(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+// 32-bit word at addr, which is 2 bytes off a word where ODD.
+template <bool ODD> __device__ __forceinline__ uint32_t q6w_word(uint32_t addr)
+{
+    if (!ODD) return q6w_lds32(addr);
+    return __byte_perm(q6w_lds32(addr - 2), q6w_lds32(addr + 2), 0x5432);
+}
+__device__ __forceinline__ uint32_t q6w_sub(uint32_t v) // f16 pairs 1024 + v -> v - 32, exact
+{
+    const uint32_t off = 0x64206420u; // 1056
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&v), *reinterpret_cast<const __half2 *>(&off));
+    return *reinterpret_cast<const uint32_t *>(&d);
+}
+
+// One super-block of 16 rows (this lane: rows g and g + 8, words 4c of every piece) times x.
+template <bool ODD>
+__device__ __forceinline__ void q6w_superblock(float (&tot)[4], uint32_t blk0, uint32_t blk1, int c, const __half *xp, int xmul)
+{
+    uint32_t sc0[4], sc1[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        sc0[i] = q6w_word<ODD>(blk0 + 192 + 4 * i) ^ 0x80808080u; // signed byte + 128
+        sc1[i] = q6w_word<ODD>(blk1 + 192 + 4 * i) ^ 0x80808080u;
+    }
+    uint16_t dr0, dr1;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dr0) : "r"(blk0 + 208));
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dr1) : "r"(blk1 + 208));
+    const float d0 = __half2float(__ushort_as_half(dr0)), d1 = __half2float(__ushort_as_half(dr1));
+#pragma unroll
+    for (int combo = 0; combo < 4; combo++) {
+        const int h = combo >> 1, s = combo & 1;
+        const uint32_t at = 64 * h + 16 * s + 4 * c, hat = 128 + 32 * h + 16 * s + 4 * c;
+        const uint32_t le0 = q6w_word<ODD>(blk0 + at), lo0 = q6w_word<ODD>(blk0 + at + 32), qh0 = q6w_word<ODD>(blk0 + hat);
+        const uint32_t le1 = q6w_word<ODD>(blk1 + at), lo1 = q6w_word<ODD>(blk1 + at + 32), qh1 = q6w_word<ODD>(blk1 + hat);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t l0 = (q & 1) ? lo0 : le0, l1 = (q & 1) ? lo1 : le1;
+            const uint32_t b0 = (q == 0 ? qh0 << 4 : q == 1 ? qh0 << 2 : q == 2 ? qh0 : qh0 >> 2) & 0x30303030u;
+            const uint32_t b1 = (q == 0 ? qh1 << 4 : q == 1 ? qh1 << 2 : q == 2 ? qh1 : qh1 >> 2) & 0x30303030u;
+            const uint32_t v0 = ((q < 2 ? l0 : l0 >> 4) & 0x0F0F0F0Fu) | b0, v1 = ((q < 2 ? l1 : l1 >> 4) & 0x0F0F0F0Fu) | b1;
+            const uint32_t a[4] = {q6w_sub(__byte_perm(v0, 0x64646464u, 0x5140)), q6w_sub(__byte_perm(v1, 0x64646464u, 0x5140)),
+                                   q6w_sub(__byte_perm(v0, 0x64646464u, 0x7362)), q6w_sub(__byte_perm(v1, 0x64646464u, 0x7362))};
+            const uint2 xv = *reinterpret_cast<const uint2 *>(xp + xmul * (128 * h + 32 * q + 16 * s));
+            const uint32_t b[2] = {xv.x, xv.y};
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            q6k_mma_f16(acc, a, b);
+            const int si = 8 * h + 2 * q + s;
+            const float f0 = d0 * (__uint_as_float(__byte_perm(sc0[si >> 2], 0x4B000000u, 0x7440 + (si & 3))) - 8388736.0f); // 2^23 + 128
+            const float f1 = d1 * (__uint_as_float(__byte_perm(sc1[si >> 2], 0x4B000000u, 0x7440 + (si & 3))) - 8388736.0f);
+            tot[0] = fmaf(f0, acc[0], tot[0]);
+            tot[1] = fmaf(f0, acc[1], tot[1]);
+            tot[2] = fmaf(f1, acc[2], tot[2]);
+            tot[3] = fmaf(f1, acc[3], tot[3]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6kWideParams p)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int engine = warp / (Q6W_WARPS + 1), ew = warp % (Q6W_WARPS + 1); // ew == Q6W_WARPS: the engine's producer
+    const int chunks = p.k / (Q6W_SB * 256), xrow = p.k + 16;
+    const size_t row_bytes = (size_t)chunks * Q6W_ROW_BYTES;
+    // rings of both engines | partial sums (two tiles per engine) | barriers | zeros | x
+    const uint32_t base = smem_u32(smem);
+    const uint32_t ring = base + (uint32_t)(engine * p.ring * Q6W_STAGE_BYTES);
+    unsigned char *rest = smem + (size_t)Q6W_ENGINES * p.ring * Q6W_STAGE_BYTES;
+    float *red = reinterpret_cast<float *>(rest) + engine * 2 * Q6W_RED;
+    rest += Q6W_ENGINES * 2 * Q6W_RED * sizeof(float);
+    const uint32_t bars = smem_u32(rest) + (uint32_t)(engine * 2 * Q6W_MAX_RING * 8);
+    auto full = [&](int r) { return bars + 8u * r; };
+    auto empty = [&](int r) { return bars + 8u * (Q6W_MAX_RING + r); };
+    rest += Q6W_ENGINES * 2 * Q6W_MAX_RING * 8;
+    float *zeros = reinterpret_cast<float *>(rest); // 16 bytes: what lanes without a token read as x
+    __half *xs = reinterpret_cast<__half *>(rest + 16);
+
+    if (ew == Q6W_WARPS && lane < Q6W_MAX_RING) {
+        mbar_init(full(lane), 1);
+        mbar_init(empty(lane), Q6W_WARPS);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < 4) zeros[threadIdx.x] = 0.0f;
+    __syncthreads();
+
+    const int first = (int)blockIdx.x + engine * (int)gridDim.x, step = Q6W_ENGINES * (int)gridDim.x; // this engine's tiles
+    if (ew == Q6W_WARPS) {
+        // ---- producer: weights are read before the previous kernel has finished; lane r copies row r -------------
+        int r = 0;
+        uint32_t ph = 0;
+        long long it = 0;
+        bool ok = true;
+        for (int t = first; t < p.tiles && ok; t += step) {
+            const int row = min(t * Q6W_ROWS + min(lane, Q6W_ROWS - 1), p.n - 1); // past-the-end rows re-read the last row
+            const uint8_t *src = p.blocks + (size_t)row * row_bytes;
+            for (int ch = 0; ch < chunks && ok; ch++, it++) {
+                if (it >= p.ring) ok = __all_sync(0xFFFFFFFFu, mbar_wait(empty(r), ph ^ 1u, &g_q6k_gemv_flag, 1));
+                if (ok) {
+                    if (lane == 0) mbar_arrive_expect_tx(full(r), Q6W_STAGE_BYTES);
+                    __syncwarp();
+                    if (lane < Q6W_ROWS)
+                        bulk_copy_g2s(ring + (uint32_t)(r * Q6W_STAGE_BYTES + lane * Q6W_ROW_BYTES), src + (size_t)ch * Q6W_ROW_BYTES,
+                                      Q6W_ROW_BYTES, full(r));
+                }
+                if (++r == p.ring) { r = 0; ph ^= 1u; }
+            }
+        }
+        return;
+    }
+
+    // ---- x as f16, once for all tiles; the first stages are on their way --------------------------------------------
+    pdl_wait(); // x may come from the kernel before this one, y may still be read by it
+    {
+        const int ct = (engine * Q6W_WARPS + ew) * 32 + lane, per_row = p.k / 4;
+        for (int idx = ct; idx < p.m * per_row; idx += Q6W_ENGINES * Q6W_WARPS * 32) {
+            const int row = idx / per_row, q4 = idx - row * per_row;
+            const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p.x + (size_t)row * p.k) + q4);
+            uint2 o;
+            o.x = f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x));
+            o.y = f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y));
+            reinterpret_cast<uint2 *>(xs + (size_t)row * xrow)[q4] = o;
+        }
+    }
+    asm volatile("bar.sync 3, %0;" ::"n"(Q6W_ENGINES * Q6W_WARPS * 32) : "memory"); // all but the producers
+
+    const int g = lane >> 2, c = lane & 3;
+    const bool real = g < p.m;
+    const __half *xbase = real ? xs + (size_t)g * xrow + ew * 256 + 4 * c : reinterpret_cast<const __half *>(zeros);
+    const int xmul = real ? 1 : 0;
+    const uint32_t row_off = (uint32_t)(g * Q6W_ROW_BYTES + ew * 210);
+    int r = 0, buf = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int t = first; t < p.tiles; t += step, buf ^= 1) {
+        float tot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int ch = 0; ch < chunks && ok; ch++) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(full(r), ph, &g_q6k_gemv_flag, 2));
+            if (!ok) break;
+            const uint32_t blk0 = ring + (uint32_t)(r * Q6W_STAGE_BYTES) + row_off, blk1 = blk0 + 8 * Q6W_ROW_BYTES;
+            const __half *xp = xbase + xmul * (ch * Q6W_SB * 256);
+            if (ew & 1) q6w_superblock<true>(tot, blk0, blk1, c, xp, xmul);
+            else q6w_superblock<false>(tot, blk0, blk1, c, xp, xmul);
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty(r)) : "memory");
+            if (++r == p.ring) { r = 0; ph ^= 1u; }
+        }
+        // the engine's warps meet once per tile (also after a wait gave up); the other buffer is free again by then
+        float *mine = red + buf * Q6W_RED;
+#pragma unroll
+        for (int e = 0; e < 4; e++) mine[(ew * 4 + e) * 32 + lane] = tot[e];
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + engine), "n"(Q6W_WARPS * 32) : "memory");
+        const int o = ew * 32 + lane; // 0 .. 255: accumulator slot and lane, in ascending k over the warps
+        if (o < 4 * 32 && ok) {
+            const int ln = o & 31, e = o >> 5;
+            const int nn = t * Q6W_ROWS + (ln >> 2) + 8 * (e >> 1), row = 2 * (ln & 3) + (e & 1);
+            if (nn < p.n && row < p.m) {
+                float sum = 0.0f;
+#pragma unroll
+                for (int w = 0; w < Q6W_WARPS; w++) sum += mine[(w * 4 + e) * 32 + ln];
+                if (p.bias) sum += load_as_f32(p.bias, p.bias_dtype, nn);
+                store_as(p.y, p.y_dtype, (size_t)row * p.n + nn, sum);
+            }
+        }
+    }
+}
+
+static size_t q6w_fixed(int m, int k)
+{
+    return (size_t)Q6W_ENGINES * 2 * Q6W_RED * 4 + Q6W_ENGINES * 2 * Q6W_MAX_RING * 8 + 16 + (size_t)m * (k + 16) * 2;
+}
+
+// Ring depth of an engine, 0 where the kernel does not apply: rows of whole stages (8 super-blocks), at least four tiles per
+// SM (below that the last wave costs more than the staging saves), room for two stages per engine beside x.
+static int q6w_ring(int m, int k, int n, const void *blocks)
+{
+    if (m > 8 || k % (Q6W_SB * 256) != 0 || !aligned(blocks, 16) || ceil_div(n, Q6W_ROWS) < 4 * sm_count()) return 0;
+    const long long room = 227 * 1024 - (long long)q6w_fixed(m, k);
+    const int ring = room > 0 ? (int)(room / (Q6W_ENGINES * Q6W_STAGE_BYTES)) : 0;
+    return ring < 2 ? 0 : ring < Q6W_MAX_RING ? ring : Q6W_MAX_RING;
+}
+
+static int launch_q6k_wide(const Q6kGemvParams &g, int ring, cudaStream_t st)
+{
+    Q6kWideParams p = {g.x, g.blocks, g.bias, g.y, g.bias_dtype, g.y_dtype, g.m, g.k, g.n, ceil_div(g.n, Q6W_ROWS), ring};
+    const size_t smem = (size_t)Q6W_ENGINES * ring * Q6W_STAGE_BYTES + q6w_fixed(g.m, g.k);
+    static size_t configured[64] = {};
+    int device = 0;
+    OXQ_CUDA(cudaGetDevice(&device));
+    if (device >= 64 || configured[device] < smem) {
+        OXQ_CUDA(cudaFuncSetAttribute(q6k_gemv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (device < 64) configured[device] = smem;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count(), 1, 1);
+    cfg.blockDim = dim3(Q6W_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    cfg.numAttrs = 0;
+    allow_early_start(attr, cfg.numAttrs);
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, q6k_gemv_wide_kernel, p));
+    return OXQ_OK;
+}
+
+// The code of a bounded wait that ran out since the last call, 0 if none (synchronises the device's copy).
+int q6k_gemv_take_flag(int &flag)
+{
+    OXQ_CUDA(cudaMemcpyFromSymbol(&flag, g_q6k_gemv_flag, sizeof(int)));
+    if (flag != 0) {
+        const int zero = 0;
+        OXQ_CUDA(cudaMemcpyToSymbol(g_q6k_gemv_flag, &zero, sizeof(int)));
+    }
+    return OXQ_OK;
+}
+
 static size_t q6k_smem(int m_cta, int kl, int warps)
 {
     return (size_t)m_cta * (kl + 16) * 2 + (size_t)(kl / 16) * 8 * 4 + (size_t)warps * 4 * 32 * 4 + 16;
@@ -268,6 +519,7 @@ int q6k_gemv(const void *x, const void *blocks, const void *bias, int bias_dtype
     Q6kGemvParams p;
     p.x = (const __nv_bfloat16 *)x; p.blocks = (const uint8_t *)blocks; p.bias = bias; p.y = y;
     p.bias_dtype = bias_dtype; p.y_dtype = y_dtype; p.m = m; p.k = k; p.n = n;
+    if (const int ring = q6w_ring(m, k, n, blocks)) return launch_q6k_wide(p, ring, st);
     int nrt = 2, kw = 4, ks = 1;
     q6k_pick(m, k, nrt, kw, ks);
     if (const char *env = tuning_env("OXQ_Q6K_GEMV_TUNE")) { // bench-harness knob: "row_tiles,k_warps,cluster"

@@ -73,3 +73,22 @@ def test_calls_on_two_streams_and_a_replayed_graph_do_not_meet(cuda):
         y.zero_()
         graph.replay()
         assert torch.equal(y, want[0])
+
+
+# ------------------------------------------------------------------ the GGUF GEMV of wide layers (vocabulary projections)
+@pytest.mark.parametrize("m,k,n", [(1, 2048, 9472), (3, 4096, 9480), (8, 4096, 9479), (4, 14336, 9472), (8, 2048, 9472)])
+def test_wide_q6k_gemv_matches_64_bit_sums(cuda, m, k, n):
+    """x and the 6-bit integers are exact in f16; 16-wide sums, times d * scale (one rounding), are added in f32."""
+    from oxydllm_b200 import formats as F
+    data = synth.gguf_layer(F.GGML_Q6_K, 64, k, seed=k + m)
+    data = np.tile(np.asarray(data).reshape(64, -1), (n // 64 + 1, 1))[:n].reshape(-1)
+    w = oracle.gguf_dequant(F.GGML_Q6_K, data[: 64 * (data.size // n)], 64, k).astype(np.float64)
+    bias = torch.arange(n, dtype=torch.float32, device="cuda") / n
+    lin = L.QLinear(F.GGML_Q6_K, torch.from_numpy(data).cuda(), n, k, bias=bias, out_dtype=torch.float32)
+    x = synth.activations(m, k, seed=m)
+    y = lin.forward(torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()).double().cpu().numpy()
+    rows = np.arange(n) % 64
+    ref, mass = (x.astype(np.float64) @ w.T)[:, rows] + bias.cpu().numpy(), (np.abs(x).astype(np.float64) @ np.abs(w).T)[:, rows] + 1
+    assert (np.abs(y - ref) <= 2.0**-17 * mass).all()
+    from oxydllm_b200 import _lib
+    assert _lib.load().oxq_awq_gemv_check(None) == 0

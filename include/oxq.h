@@ -296,6 +296,13 @@ int oxq_gptoss_moe_forward(const void *x, int x_dtype, const float *router_logit
                            const uint8_t *dn_scales, const void *dn_bias, int bias_dtype, float limit, int expert_lo,
                            int expert_hi, void *out, int out_dtype, void *workspace, size_t workspace_bytes,
                            void *stream);
+/* The same on router logits of any dtype (as the router's linear returns them). */
+int oxq_gptoss_moe_forward_logits(const void *x, int x_dtype, const void *router_logits, int logits_dtype, int tokens, int num_experts,
+                           int top_k, int norm_topk, int hidden, int inter, const uint8_t *gu_blocks,
+                           const uint8_t *gu_scales, const void *gu_bias, const uint8_t *dn_blocks,
+                           const uint8_t *dn_scales, const void *dn_bias, int bias_dtype, float limit, int expert_lo,
+                           int expert_hi, void *out, int out_dtype, void *workspace, size_t workspace_bytes,
+                           void *stream);
 
 /* The owner side of expert parallelism (no counterpart in the reference, which dispatches on one device,
  * moe.rs:563-607): rows that already carry their expert id go through that expert with weight one,

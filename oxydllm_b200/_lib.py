@@ -55,6 +55,8 @@ SIGNATURES = {
     "oxq_gptoss_moe_workspace_bytes": [_i, _i, _i, _i, _i],
     "oxq_gptoss_moe_forward": [_vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, ctypes.c_float,
                                _i, _i, _vp, _i, _vp, _sz, _vp],
+    "oxq_gptoss_moe_forward_logits": [_vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, ctypes.c_float,
+                                      _i, _i, _vp, _i, _vp, _sz, _vp],
     "oxq_gptoss_experts_forward": [_vp, _i, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, ctypes.c_float, _i, _i,
                                    _vp, _i, _vp, _sz, _vp],
     "oxq_moe_combine": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _i, _vp],

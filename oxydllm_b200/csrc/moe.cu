@@ -23,7 +23,7 @@ int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const ui
 bool mxfp4_gemv_batched_supported(int k, const void *blocks);
 int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const uint8_t *scales, const void *bias,
                        int bias_dtype, const int *pair_expert, int pairs, int e_lo, int e_hi, void *y, int y_dtype, int k,
-                       int n, cudaStream_t st);
+                       int n, cudaStream_t st, const float *gu = nullptr, float limit = 0.0f);
 
 constexpr int MOE_MAX_EXPERTS = 256;
 constexpr int MOE_MAX_TOPK = 8;
@@ -35,19 +35,18 @@ constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
 // One warp per token: f32 softmax over all experts, k rounds of arg-max (ties: lower index),
 // optional renormalisation by the sum of the selected probabilities (moe.rs:472-487).
 __global__ void __launch_bounds__(256)
-moe_route_kernel(const float *__restrict__ logits, int tokens, int experts, int top_k, int norm_topk,
+moe_route_kernel(const void *__restrict__ logits, int dtype, int tokens, int experts, int top_k, int norm_topk,
                  int *__restrict__ top_idx, float *__restrict__ top_w)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= tokens) return;
-    const float *l = logits + (size_t)warp * experts;
     constexpr int PER = MOE_MAX_EXPERTS / 32;
     float v[PER];
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < PER; i++) {
         const int e = lane + 32 * i;
-        v[i] = e < experts ? l[e] : -INFINITY;
+        v[i] = e < experts ? load_as_f32(logits, dtype, (size_t)warp * experts + e) : -INFINITY;
         mx = fmaxf(mx, v[i]);
     }
 #pragma unroll
@@ -139,28 +138,94 @@ __global__ void moe_plan_kernel(const int *__restrict__ counts, int n_exp, int e
     grp_beg[g] = mt;
 }
 
-// The same offsets; token blocks for the kernel that unpacks MXFP4 inside the tensor-core loop: every expert's rows cut into
-// the fewest blocks of at most max_rows rows, of equal size rounded up to 16. n_blocks[0] = how many.
-__global__ void moe_plan_blocks_kernel(const int *__restrict__ counts, int n_exp, int e_lo, int max_rows, int *__restrict__ offsets,
-                                       int4 *__restrict__ entries, int *__restrict__ n_blocks)
+// Inclusive scan over the block's threads (at most 1024) of two values at once; scratch: 64 ints.
+__device__ __forceinline__ int2 moe_block_scan(int2 v, int *scratch)
 {
-    __shared__ int cnt_s[MOE_MAX_EXPERTS];
-    for (int i = threadIdx.x; i < n_exp; i += blockDim.x) cnt_s[i] = counts[i]; // one round trip for all counts
-    __syncthreads();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int off = 0, nb = 0;
-    for (int i = 0; i < n_exp; i++) {
-        offsets[i] = off;
-        const int c = cnt_s[i];
-        if (c > 0) {
-            const int parts = (c + max_rows - 1) / max_rows;
-            const int size = ((c + parts - 1) / parts + 15) / 16 * 16;
-            for (int r = 0; r < c; r += size) entries[nb++] = make_int4(off + r, min(size, c - r), e_lo + i, 0);
-        }
-        off += c;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xFFFFFFFFu, v.x, o), y = __shfl_up_sync(0xFFFFFFFFu, v.y, o);
+        if (lane >= o) v.x += x, v.y += y;
     }
-    offsets[n_exp] = off;
-    n_blocks[0] = nb;
+    if (lane == 31) scratch[warp] = v.x, scratch[32 + warp] = v.y;
+    __syncthreads();
+    for (int w = 0; w < warp && w < warps; w++) v.x += scratch[w], v.y += scratch[32 + w];
+    __syncthreads();
+    return v;
+}
+
+// Offsets (exclusive scan of counts) and token blocks for the kernel that unpacks MXFP4 inside the tensor-core loop: every
+// expert's rows cut into the fewest blocks of at most max_rows rows, of equal size rounded up to 16. n_blocks[0] = how many.
+// Thread i is expert i (one thread walking 32 experts took 10 us). Returns the expert's first row.
+__device__ __forceinline__ int moe_plan_expert(int c, int n_exp, int e_lo, int max_rows, int *offsets, int4 *entries, int *n_blocks,
+                                               int *scratch)
+{
+    const int i = threadIdx.x;
+    const int parts = (c + max_rows - 1) / max_rows;
+    const int size = parts ? ((c + parts - 1) / parts + 15) / 16 * 16 : 1;
+    const int blocks = (c + size - 1) / size;
+    const int2 incl = moe_block_scan(make_int2(c, blocks), scratch);
+    const int off = incl.x - c;
+    if (i < n_exp) {
+        offsets[i] = off;
+        for (int q = 0; q < blocks; q++) entries[incl.y - blocks + q] = make_int4(off + q * size, min(size, c - q * size), e_lo + i, 0);
+        if (i == n_exp - 1) offsets[n_exp] = incl.x, n_blocks[0] = incl.y;
+    }
+    return off;
+}
+
+__global__ void __launch_bounds__(MOE_MAX_EXPERTS)
+moe_plan_blocks_kernel(const int *__restrict__ counts, int n_exp, int e_lo, int max_rows, int *__restrict__ offsets,
+                       int4 *__restrict__ entries, int *__restrict__ n_blocks)
+{
+    __shared__ int scratch[64];
+    moe_plan_expert((int)threadIdx.x < n_exp ? counts[threadIdx.x] : 0, n_exp, e_lo, max_rows, offsets, entries, n_blocks, scratch);
+}
+
+// Count, plan and scatter of a small batch in one launch of one CTA (a launch each took 16 us for 200 pairs): pairs are taken
+// 1024 at a time, a warp's hits of an expert are counted by match, and the warps' counts are scanned per expert, so that
+// positions keep the order of the pairs.
+constexpr int MOE_SMALL_PAIRS = 2048;
+__global__ void __launch_bounds__(1024)
+moe_dispatch_small_kernel(const int *__restrict__ top_idx, int pairs, int e_lo, int n_exp, int max_rows, int *__restrict__ counts,
+                          int *__restrict__ offsets, int4 *__restrict__ entries, int *__restrict__ n_blocks, int *__restrict__ perm,
+                          int *__restrict__ inv)
+{
+    constexpr int ROUNDS = MOE_SMALL_PAIRS / 1024, GROUPS = ROUNDS * 32;
+    __shared__ unsigned short cnt[GROUPS][MOE_MAX_EXPERTS]; // hits of an expert in a warp of a round, then the hits before it
+    __shared__ int base_s[MOE_MAX_EXPERTS], scratch[64];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int groups = (pairs + 31) / 32;
+    for (int i = tid; i < groups * MOE_MAX_EXPERTS; i += blockDim.x) (&cnt[0][0])[i] = 0;
+    __syncthreads();
+    int id[ROUNDS];
+    unsigned peers[ROUNDS];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const int pair = r * 1024 + tid;
+        id[r] = pair < pairs ? top_idx[pair] - e_lo : -1;
+        if (id[r] >= n_exp || id[r] < 0) id[r] = -1;
+        peers[r] = __match_any_sync(0xFFFFFFFFu, id[r]);
+        if (id[r] >= 0 && (peers[r] & ((1u << lane) - 1u)) == 0) cnt[r * 32 + warp][id[r]] = (unsigned short)__popc(peers[r]);
+    }
+    __syncthreads();
+    int c = 0;
+    if (tid < n_exp)
+        for (int q = 0; q < groups; q++) {
+            const int h = cnt[q][tid];
+            cnt[q][tid] = (unsigned short)c;
+            c += h;
+        }
+    const int off = moe_plan_expert(c, n_exp, e_lo, max_rows, offsets, entries, n_blocks, scratch);
+    if (tid < n_exp) counts[tid] = c, base_s[tid] = off;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++)
+        if (id[r] >= 0) {
+            const int pair = r * 1024 + tid, pos = base_s[id[r]] + cnt[r * 32 + warp][id[r]] + __popc(peers[r] & ((1u << lane) - 1u));
+            perm[pos] = pair;
+            inv[pair] = pos;
+        }
 }
 
 // Stable partition: position of pair i among the pairs of its expert, in pair (= token) order.
@@ -240,10 +305,13 @@ moe_combine_kernel(const __nv_bfloat16 *__restrict__ yp, const int *__restrict__
                    const int *__restrict__ inv, int tokens, int top_k, int hidden, int e_lo, int e_hi, void *out,
                    int out_dtype)
 {
-    const int chunks = hidden / 8;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < (size_t)tokens * chunks;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(idx / chunks), c = (int)(idx % chunks);
+    // a warp takes part `seg` of a token's 16-byte pieces: the slots are put in order once for all of them (once per piece it took
+    // 44 us for 4096 tokens of 2880)
+    const int chunks = hidden / 8, lane = threadIdx.x & 31, warps = (int)((gridDim.x * blockDim.x) >> 5);
+    const bool out16 = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    const int segs = min((chunks + 31) / 32, (warps + tokens - 1) / tokens);
+    for (int job = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); job < tokens * segs; job += warps) {
+        const int t = job / segs, seg = job - t * segs;
         int order[MOE_MAX_TOPK], ids[MOE_MAX_TOPK];
 #pragma unroll
         for (int s = 0; s < MOE_MAX_TOPK; s++) {
@@ -267,9 +335,10 @@ moe_combine_kernel(const __nv_bfloat16 *__restrict__ yp, const int *__restrict__
         for (int s = 0; s < MOE_MAX_TOPK; s++) {
             use[s] = s < top_k && ids[s] >= e_lo && ids[s] < e_hi;
             const size_t pair = (size_t)t * top_k + order[s];
-            pos[s] = use[s] ? __ldg(inv + pair) : 0;
+            pos[s] = !use[s] ? 0 : inv ? __ldg(inv + pair) : (int)pair;
             wv[s] = use[s] ? __ldg(top_w + pair) : 0.0f;
         }
+        for (int c = seg * 32 + lane; c < chunks; c += segs * 32) {
         uint4 rows[MOE_MAX_TOPK];
 #pragma unroll
         for (int s = 0; s < MOE_MAX_TOPK; s++)
@@ -286,23 +355,19 @@ moe_combine_kernel(const __nv_bfloat16 *__restrict__ yp, const int *__restrict__
                 acc[2 * q + 1] = fmaf(w, __uint_as_float(vv[q] & 0xFFFF0000u), acc[2 * q + 1]);
             }
         }
-        for (int q = 0; q < 8; q++) store_as(out, out_dtype, (size_t)t * hidden + c * 8 + q, acc[q]);
-    }
-}
-
-// Decode path: h[pair, j] = clamped SwiGLU of the interleaved (gate, up) columns 2j, 2j+1 of gu[pair, :]
-// (moe.rs:152-173; the same arithmetic as the grouped GEMM's epilogue), and inv[pair] = pair.
-__global__ void __launch_bounds__(256)
-moe_swiglu_kernel(const float *__restrict__ gu, int pairs, int inter, float limit, __nv_bfloat16 *__restrict__ h,
-                  int *__restrict__ inv)
-{
-    const size_t total = (size_t)pairs * inter;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
-        const float2 v = reinterpret_cast<const float2 *>(gu)[idx];
-        const float gate = fminf(v.x, limit), up = fminf(fmaxf(v.y, -limit), limit);
-        const float sig = __fdividef(1.0f, __expf(-1.702f * gate) + 1.0f);
-        h[idx] = __float2bfloat16_rn((up + 1.0f) * (gate * sig));
-        if (idx < (size_t)pairs) inv[idx] = (int)idx;
+        if (out_dtype == OXQ_BF16 && out16) {
+            uint4 o;
+            uint32_t *ov = reinterpret_cast<uint32_t *>(&o);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const __nv_bfloat162 b = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
+                ov[q] = *reinterpret_cast<const uint32_t *>(&b);
+            }
+            reinterpret_cast<uint4 *>(out)[(size_t)t * chunks + c] = o;
+        } else {
+            for (int q = 0; q < 8; q++) store_as(out, out_dtype, (size_t)t * hidden + c * 8 + q, acc[q]);
+        }
+        }
     }
 }
 
@@ -400,7 +465,7 @@ __global__ void __launch_bounds__(256) moe_assign_kernel(const int32_t *__restri
     if (i < rows) { top_idx[i] = ids[i]; top_w[i] = 1.0f; }
 }
 
-static int moe_forward_impl(const void *x, int x_dtype, const float *router_logits, const int32_t *given_ids, int tokens,
+static int moe_forward_impl(const void *x, int x_dtype, const void *router_logits, int logits_dtype, const int32_t *given_ids, int tokens,
                             int num_experts, int top_k, int norm_topk, int hidden, int inter, const uint8_t *gu_blocks,
                             const uint8_t *gu_scales, const void *gu_bias, const uint8_t *dn_blocks,
                             const uint8_t *dn_scales, const void *dn_bias, int bias_dtype, float limit,
@@ -441,8 +506,8 @@ static int moe_forward_impl(const void *x, int x_dtype, const float *router_logi
     const int pairs = tokens * top_k;
 
     if (given_ids) moe_assign_kernel<<<ceil_div(tokens, 256), 256, 0, st>>>(given_ids, tokens, top_idx, top_w);
-    else moe_route_kernel<<<ceil_div(tokens * 32, 256), 256, 0, st>>>(router_logits, tokens, num_experts, top_k, norm_topk,
-                                                                      top_idx, top_w);
+    else moe_route_kernel<<<ceil_div(tokens * 32, 256), 256, 0, st>>>(router_logits, logits_dtype, tokens, num_experts, top_k,
+                                                                      norm_topk, top_idx, top_w);
     const int a_rows = pairs + 128;
     // Both projections through the kernel that unpacks the MXFP4 blocks inside the tensor-core loop, where it takes the shapes:
     // no dequantized slab, one launch per projection over all experts.
@@ -454,28 +519,32 @@ static int moe_forward_impl(const void *x, int x_dtype, const float *router_logi
         OXQ_REQUIRE(aligned(gu_blocks, 16) && aligned(dn_blocks, 16), OXQ_ERR_BAD_ALIGN,
                     "oxq_gptoss_moe_forward: expert blocks must be 16-byte aligned");
         // Decode: only the selected experts' packed weights are read. gate_up (f32 out, bias folded) ->
-        // SwiGLU -> down (into the xs buffer, bf16) -> combine with inv = identity.
+        // down on its SwiGLU (into the xs buffer, bf16) -> combine, row = pair.
         OXQ_LAUNCH_CHECK("moe_route_kernel");
         float *gu = reinterpret_cast<float *>(slab);
         int rc = mxfp4_gemv_batched(x, top_k, gu_blocks, gu_scales, gu_bias, bias_dtype, top_idx, pairs, expert_lo, expert_hi,
                                     gu, OXQ_F32, hidden, 2 * inter, st);
         if (rc) return rc;
-        moe_swiglu_kernel<<<ceil_div(pairs * inter, 256), 256, 0, st>>>(gu, pairs, inter, limit, h, inv);
-        OXQ_LAUNCH_CHECK("moe_swiglu_kernel");
-        rc = mxfp4_gemv_batched(h, 1, dn_blocks, dn_scales, dn_bias, bias_dtype, top_idx, pairs, expert_lo, expert_hi, xs,
-                                OXQ_BF16, inter, hidden, st);
+        rc = mxfp4_gemv_batched(x, 1, dn_blocks, dn_scales, dn_bias, bias_dtype, top_idx, pairs, expert_lo, expert_hi, xs,
+                                OXQ_BF16, inter, hidden, st, gu, limit);
         if (rc) return rc;
-        moe_combine_kernel<<<ceil_div(tokens * (hidden / 8), 256), 256, 0, st>>>(xs, top_idx, top_w, inv, tokens, top_k,
+        moe_combine_kernel<<<ceil_div(tokens * ceil_div(hidden / 8, 32) * 32, 256), 256, 0, st>>>(xs, top_idx, top_w, nullptr, tokens, top_k,
                                                                                  hidden, expert_lo, expert_hi, out, out_dtype);
         OXQ_LAUNCH_CHECK("moe_combine_kernel");
         return OXQ_OK;
     }
-    moe_count_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, counts);
     // the grouped kernel's table of token blocks goes where the m-tile table of the dense path would (same capacity bound);
     // grp_beg[0] then holds the number of blocks
-    if (fused) moe_plan_blocks_kernel<<<1, 32, 0, st>>>(counts, n_exp, expert_lo, moe_fused_block_rows(), offsets, entries, grp_beg);
-    else moe_plan_kernel<<<1, 32, 0, st>>>(counts, n_exp, expert_lo, L.group_experts, offsets, entries, grp_beg);
-    moe_scatter_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, offsets, perm, inv);
+    if (fused && pairs <= MOE_SMALL_PAIRS) {
+        moe_dispatch_small_kernel<<<1, 1024, 0, st>>>(top_idx, pairs, expert_lo, n_exp, moe_fused_block_rows(), counts, offsets, entries,
+                                                      grp_beg, perm, inv);
+    } else {
+        moe_count_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, counts);
+        if (fused) moe_plan_blocks_kernel<<<1, MOE_MAX_EXPERTS, 0, st>>>(counts, n_exp, expert_lo, moe_fused_block_rows(), offsets,
+                                                                         entries, grp_beg);
+        else moe_plan_kernel<<<1, 32, 0, st>>>(counts, n_exp, expert_lo, L.group_experts, offsets, entries, grp_beg);
+        moe_scatter_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, offsets, perm, inv);
+    }
     moe_gather_kernel<<<sm_count() * 8, 256, 0, st>>>((const __nv_bfloat16 *)x, perm, offsets + n_exp, top_k, hidden, xs);
     OXQ_LAUNCH_CHECK("moe routing kernels");
 
@@ -527,8 +596,24 @@ OXQ_EXPORT int oxq_gptoss_moe_forward(const void *x, int x_dtype, const float *r
 {
     clear_error();
     OXQ_REQUIRE(router_logits != nullptr, OXQ_ERR_NULL, "oxq_gptoss_moe_forward: null pointer");
-    return moe_forward_impl(x, x_dtype, router_logits, nullptr, tokens, num_experts, top_k, norm_topk, hidden, inter, gu_blocks,
+    return moe_forward_impl(x, x_dtype, router_logits, OXQ_F32, nullptr, tokens, num_experts, top_k, norm_topk, hidden, inter, gu_blocks,
                             gu_scales, gu_bias, dn_blocks, dn_scales, dn_bias, bias_dtype, limit, expert_lo, expert_hi, out,
+                            out_dtype, workspace, workspace_bytes, stream);
+}
+
+// The same on router logits of any supported dtype, as the router's linear returns them.
+OXQ_EXPORT int oxq_gptoss_moe_forward_logits(const void *x, int x_dtype, const void *router_logits, int logits_dtype, int tokens,
+                                             int num_experts, int top_k, int norm_topk, int hidden, int inter, const uint8_t *gu_blocks,
+                                             const uint8_t *gu_scales, const void *gu_bias, const uint8_t *dn_blocks,
+                                             const uint8_t *dn_scales, const void *dn_bias, int bias_dtype, float limit,
+                                             int expert_lo, int expert_hi, void *out, int out_dtype, void *workspace,
+                                             size_t workspace_bytes, void *stream)
+{
+    clear_error();
+    OXQ_REQUIRE(router_logits != nullptr, OXQ_ERR_NULL, "oxq_gptoss_moe_forward: null pointer");
+    OXQ_REQUIRE(valid_dtype(logits_dtype), OXQ_ERR_UNSUPPORTED, "oxq_gptoss_moe_forward: unsupported dtype");
+    return moe_forward_impl(x, x_dtype, router_logits, logits_dtype, nullptr, tokens, num_experts, top_k, norm_topk, hidden, inter,
+                            gu_blocks, gu_scales, gu_bias, dn_blocks, dn_scales, dn_bias, bias_dtype, limit, expert_lo, expert_hi, out,
                             out_dtype, workspace, workspace_bytes, stream);
 }
 
@@ -541,7 +626,7 @@ OXQ_EXPORT int oxq_gptoss_experts_forward(const void *rows, int x_dtype, const i
 {
     clear_error();
     OXQ_REQUIRE(expert_ids != nullptr, OXQ_ERR_NULL, "oxq_gptoss_experts_forward: null pointer");
-    return moe_forward_impl(rows, x_dtype, nullptr, expert_ids, n_rows, num_experts, 1, 0, hidden, inter, gu_blocks, gu_scales,
+    return moe_forward_impl(rows, x_dtype, nullptr, OXQ_F32, expert_ids, n_rows, num_experts, 1, 0, hidden, inter, gu_blocks, gu_scales,
                             gu_bias, dn_blocks, dn_scales, dn_bias, bias_dtype, limit, expert_lo, expert_hi, out, out_dtype,
                             workspace, workspace_bytes, stream);
 }
@@ -573,7 +658,7 @@ OXQ_EXPORT int oxq_moe_route(const float *router_logits, int tokens, int num_exp
                     top_k <= num_experts,
                 OXQ_ERR_BAD_SHAPE, "oxq_moe_route: tokens %d, experts %d (max %d), top_k %d (max %d)", tokens, num_experts,
                 MOE_MAX_EXPERTS, top_k, MOE_MAX_TOPK);
-    moe_route_kernel<<<ceil_div(tokens * 32, 256), 256, 0, (cudaStream_t)stream>>>(router_logits, tokens, num_experts,
+    moe_route_kernel<<<ceil_div(tokens * 32, 256), 256, 0, (cudaStream_t)stream>>>(router_logits, OXQ_F32, tokens, num_experts,
                                                                                     top_k, norm_topk, top_idx, top_w);
     OXQ_LAUNCH_CHECK("moe_route_kernel");
     return OXQ_OK;

@@ -36,6 +36,9 @@ struct Mx4GemvParams {
     // the weight, bias and scale slices, its token (pair / x_div) the x row, and y row = pair.
     const int *pair_expert; // null: plain mode
     int x_div, e_lo, e_hi;
+    const float *gu; // not null: the x row of a pair is the clamped SwiGLU of gu[pair][2 k] (gate and up columns in turn), as bf16
+    float limit;
+    int tiles;       // row groups (16 * row_tiles rows): a CTA takes every gridDim.x-th of them with the x it has staged
 };
 
 __device__ __forceinline__ void mx4_mma_f16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2])
@@ -69,7 +72,6 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     const int rt = warp % nrt, kw = warp / nrt;
     const int zt = blockIdx.x % p.token_split, bx = blockIdx.x / p.token_split;
     const int m0 = zt * 8 * MT, m_loc = min(8 * MT, p.m - m0); // this CTA's tokens [m0, m0 + m_loc)
-    const int n0 = (bx * nrt + rt) * 16;
     const int nb = p.k >> 5;                       // blocks per row
     const uint8_t *blocks = p.blocks, *scales = p.scales;
     const __nv_bfloat16 *xin = p.x;
@@ -91,25 +93,46 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     float *red = reinterpret_cast<float *>(smem + (size_t)m_loc * xrow * 2); // [warp][MT*4][lane]
     float *zeros = red + blockDim.x * MT * 4; // 16 bytes of zeros: what lanes without a token read as x
 
-    const int r0 = min(n0 + g, p.n - 1), r1 = min(n0 + g + 8, p.n - 1); // past-the-end rows re-read the last row
-    const uint32_t *q0 = reinterpret_cast<const uint32_t *>(blocks + ((size_t)r0 * nb + b_cta + b_off) * 16) + c;
-    const uint32_t *q1 = reinterpret_cast<const uint32_t *>(blocks + ((size_t)r1 * nb + b_cta + b_off) * 16) + c;
-    const uint8_t *s0p = scales + (size_t)r0 * nb + b_cta + b_off;
-    const uint8_t *s1p = scales + (size_t)r1 * nb + b_cta + b_off;
-
+    const uint32_t *q0, *q1;
+    const uint8_t *s0p, *s1p;
     uint32_t buf0[D], buf1[D], sb0[D], sb1[D];
+    auto start = [&](int group) { // the first blocks of a row group
+        const int n0 = (group * nrt + rt) * 16;
+        const int r0 = min(n0 + g, p.n - 1), r1 = min(n0 + g + 8, p.n - 1); // past-the-end rows re-read the last row
+        q0 = reinterpret_cast<const uint32_t *>(blocks + ((size_t)r0 * nb + b_cta + b_off) * 16) + c;
+        q1 = reinterpret_cast<const uint32_t *>(blocks + ((size_t)r1 * nb + b_cta + b_off) * 16) + c;
+        s0p = scales + (size_t)r0 * nb + b_cta + b_off;
+        s1p = scales + (size_t)r1 * nb + b_cta + b_off;
 #pragma unroll
-    for (int d = 0; d < D; d++)
-        if (d < wb) {
-            buf0[d] = __ldg(q0 + 4 * d);
-            buf1[d] = __ldg(q1 + 4 * d);
-            sb0[d] = __ldg(s0p + d);
-            sb1[d] = __ldg(s1p + d);
-        }
+        for (int d = 0; d < D; d++)
+            if (d < wb) {
+                buf0[d] = __ldg(q0 + 4 * d);
+                buf1[d] = __ldg(q1 + 4 * d);
+                sb0[d] = __ldg(s0p + d);
+                sb1[d] = __ldg(s1p + d);
+            }
+    };
+    const int stride = (int)gridDim.x / p.token_split;
+    int group = bx;
+    start(group);
 
     if (tid < 4) zeros[tid] = 0.0f;
     if (!p.pair_expert) pdl_wait(); // x may come from the kernel before this one; the first weights are already on their way
-    for (int row = 0; row < m_loc; row++) {
+    if (p.gu) { // one row: SwiGLU of the pair's gate and up values, rounded to bf16 as the layer's activations are
+        const float4 *src = reinterpret_cast<const float4 *>(p.gu + (size_t)blockIdx.z * 2 * p.k + 2 * k_cta);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(xs);
+        for (int i = tid; i < (kl >> 1); i += blockDim.x) {
+            const float4 v = __ldg(src + i);
+            float h[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float gate = fminf(e ? v.z : v.x, p.limit), up = fminf(fmaxf(e ? v.w : v.y, -p.limit), p.limit);
+                const float sig = __fdividef(1.0f, __expf(-1.702f * gate) + 1.0f);
+                h[e] = __bfloat162float(__float2bfloat16_rn((up + 1.0f) * (gate * sig)));
+            }
+            dst[i] = f32x2_to_f16x2_sat(h[0], h[1]);
+        }
+    } else for (int row = 0; row < m_loc; row++) {
         const uint2 *src = reinterpret_cast<const uint2 *>(xin + (size_t)(m0 + row) * p.k + k_cta);
         uint2 *dst = reinterpret_cast<uint2 *>(xs + (size_t)row * xrow);
         for (int q4 = tid; q4 < (kl >> 2); q4 += blockDim.x) {
@@ -120,6 +143,7 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     }
     __syncthreads();
 
+    for (;;) {
     // This lane's x for fragment column g of token tile mt: 8 halves per block, or the zeros (stride 0).
     const uint4 *xp[MT];
     int xstep[MT];
@@ -174,13 +198,16 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
         for (int e = 0; e < 4; e++) red[(warp * MT * 4 + mt * 4 + e) * 32 + lane] = tot[mt][e];
+    const int done = group;
+    group += stride;
+    if (group < p.tiles) start(group); // the next rows are on their way while this group is put together
     if (ks > 1) cluster.sync(); else __syncthreads();
 
     // Every (row tile, accumulator slot, lane) is summed by one thread of the cluster, in ascending k.
     const int slots = nrt * MT * 4 * 32;
     for (int o = rank * blockDim.x + tid; o < slots; o += ks * blockDim.x) {
         const int ln = o & 31, e = (o >> 5) & 3, mt = (o >> 7) % MT, wt = (o >> 7) / MT;
-        const int nn = (bx * nrt + wt) * 16 + (ln >> 2) + 8 * (e >> 1), row = 8 * mt + 2 * (ln & 3) + (e & 1);
+        const int nn = (done * nrt + wt) * 16 + (ln >> 2) + 8 * (e >> 1), row = 8 * mt + 2 * (ln & 3) + (e & 1);
         if (nn < p.n && row < m_loc) {
             float sum = 0.0f;
             for (int q = 0; q < ks; q++) {
@@ -191,11 +218,22 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
             store_as(p.y, p.y_dtype, y_off + (size_t)(m0 + row) * p.n + nn, sum);
         }
     }
-    if (ks > 1) cluster.sync(); // nobody leaves while a peer may still read its shared memory
+    if (ks > 1) cluster.sync(); // nobody leaves, or writes the next sums, while a peer may still read its shared memory
+    if (group >= p.tiles) break;
+    if (ks == 1) __syncthreads();
+    }
 }
 
-template <int MT, int D> static int launch_mx4(const Mx4GemvParams &p, int ks, cudaStream_t st, int batch = 1)
+template <int MT, int D> static int launch_mx4(Mx4GemvParams p, int ks, cudaStream_t st, int batch = 1)
 {
+    p.tiles = ceil_div(p.n, 16 * p.row_tiles);
+    // Batched: as many CTAs per pair as fit the SMs five to one (of 192 threads) in one wave, each with an equal share of the row
+    // groups, so that a pair's x is staged about 90 times and not 360 (8 pairs, 5760 x 2880: 37 -> 27 us).
+    int ctas = p.tiles;
+    if (batch > 1 && ks == 1) {
+        const int want = ceil_div(5 * sm_count(), batch);
+        ctas = ceil_div(p.tiles, ceil_div(p.tiles, want < p.tiles ? want : p.tiles));
+    }
     const int nw = p.row_tiles * p.k_warps;
     const int m_cta = p.m < 8 * MT ? p.m : 8 * MT;
     const size_t smem = (size_t)m_cta * (p.k / ks + 8) * 2 + (size_t)nw * MT * 4 * 32 * 4 + 16;
@@ -208,7 +246,7 @@ template <int MT, int D> static int launch_mx4(const Mx4GemvParams &p, int ks, c
         if (device < 64) configured[device] = smem;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ceil_div(p.n, 16 * p.row_tiles) * p.token_split, ks, batch);
+    cfg.gridDim = dim3(ctas * p.token_split, ks, batch);
     cfg.blockDim = dim3(nw * 32, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -267,13 +305,14 @@ int mxfp4_gemv_fast(const void *x, const uint8_t *blocks, const uint8_t *scales,
     }
     p.row_tiles = nrt; p.k_warps = kw;
     p.token_split = ceil_div(m, 8); // 8 tokens per CTA; more on neighbouring CTAs
-    p.pair_expert = nullptr; p.x_div = 1; p.e_lo = p.e_hi = 0;
+    p.pair_expert = nullptr; p.x_div = 1; p.e_lo = p.e_hi = 0; p.gu = nullptr; p.limit = 0.0f;
     return launch_mx4<1, 4>(p, ks, st);
 }
 
 // One single-token GEMV per (token, slot) pair against the pair's expert, all pairs in one launch:
 // y[pair, :] = x[pair / x_div, :] . W[expert(pair)]^T + bias[expert(pair)]; pairs whose expert lies
-// outside [e_lo, e_hi) are skipped (their y rows stay untouched). blocks / scales / bias are the
+// outside [e_lo, e_hi) are skipped (their y rows stay untouched). gu not null: the x row of a pair is the clamped SwiGLU of
+// gu[pair, 2 k] instead. blocks / scales / bias are the
 // stacked tensors of all experts ([E, n, k/32, 16], [E, n, k/32], [E, n]).
 bool mxfp4_gemv_batched_supported(int k, const void *blocks)
 {
@@ -284,9 +323,10 @@ bool mxfp4_gemv_batched_supported(int k, const void *blocks)
 
 int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const uint8_t *scales, const void *bias,
                        int bias_dtype, const int *pair_expert, int pairs, int e_lo, int e_hi, void *y, int y_dtype, int k,
-                       int n, cudaStream_t st)
+                       int n, cudaStream_t st, const float *gu, float limit)
 {
     Mx4GemvParams p;
+    p.gu = gu; p.limit = limit;
     p.x = (const __nv_bfloat16 *)x; p.blocks = blocks; p.scales = scales; p.bias = bias; p.y = y;
     p.bias_dtype = bias_dtype; p.y_dtype = y_dtype; p.m = 1; p.k = k; p.n = n;
     int nrt = 2, kw = 4, ks = 1;

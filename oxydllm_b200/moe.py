@@ -108,8 +108,12 @@ class GptOssMoe:
         if self.router_weight is None:
             raise ValueError("GptOssMoe.forward needs router weights; use forward_with_logits")
         flat = x.reshape(-1, self.hidden)
-        logits = torch.nn.functional.linear(flat, self.router_weight.to(flat.dtype),
-                                            None if self.router_bias is None else self.router_bias.to(flat.dtype))
+        w, b = self.router_weight, self.router_bias
+        if w.dtype != flat.dtype:
+            w = w.to(flat.dtype)
+        if b is not None and b.dtype != flat.dtype:
+            b = b.to(flat.dtype)
+        logits = torch.nn.functional.linear(flat, w, b)
         return self.forward_with_logits(x, logits, expert_range)
 
     def forward_with_logits(self, x: torch.Tensor, logits: torch.Tensor, expert_range=None) -> torch.Tensor:
@@ -120,17 +124,19 @@ class GptOssMoe:
         shape = x.shape
         x2 = x.reshape(-1, self.hidden).contiguous()
         t = x2.shape[0]
-        logits = logits.reshape(t, self.num_experts).to(torch.float32).contiguous()
+        logits = logits.reshape(t, self.num_experts).contiguous()
+        if logits.dtype not in (torch.float32, torch.bfloat16, torch.float16):
+            logits = logits.to(torch.float32)
         lo, hi = (0, self.num_experts) if expert_range is None else expert_range
         out = torch.empty_like(x2)
         if t == 0:
             return out.reshape(shape)
-        need = int(_lib.load().oxq_gptoss_moe_workspace_bytes(t, self.top_k, hi - lo, self.hidden, self.inter))
+        need = int(_lib.entry("oxq_gptoss_moe_workspace_bytes")(t, self.top_k, hi - lo, self.hidden, self.inter))
         ws = _workspace(need, x2.device)
-        _lib.call("oxq_gptoss_moe_forward", _p(x2), _dt(x2.dtype), _p(logits), t, self.num_experts, self.top_k,
+        _lib.call("oxq_gptoss_moe_forward_logits", _p(x2), _dt(x2.dtype), _p(logits), _dt(logits.dtype), t, self.num_experts, self.top_k,
                   int(self.norm_topk), self.hidden, self.inter, _p(self.gu_blocks), _p(self.gu_scales), _p(self.gu_bias),
                   _p(self.dn_blocks), _p(self.dn_scales), _p(self.dn_bias), _dt(self.gu_bias.dtype),
-                  ctypes.c_float(self.limit), lo, hi, _p(out), _dt(out.dtype), _p(ws), ws.numel(), _stream())
+                  self.limit, lo, hi, _p(out), _dt(out.dtype), _p(ws), ws.numel(), _stream())
         self.last_workspace = ws
         return out.reshape(shape)
 

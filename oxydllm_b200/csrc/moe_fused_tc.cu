@@ -231,30 +231,31 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
         int my_units = 0;
         if ((int)blockIdx.x < n_units) my_units = (n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
         const uint32_t total_rounds = (uint32_t)my_units * (uint32_t)rpu;
-        uint32_t cur_ul = 0xFFFFFFFFu, r_in_unit = 0, ul = 0;
+        // every counter steps along (divisions by the rounds of a unit were a third of a stage's instructions)
+        static_assert(MF_TEAMS * MF_ROUND <= MF_RAW_SLOTS && MF_RAW_SLOTS % (MF_TEAMS * MF_ROUND) == 0 && MF_A_SLOTS % (MF_TEAMS * MF_ROUND) == 0,
+                      "a slot meets one team");
+        int u = (int)blockIdx.x, r_in_unit = team;
+        uint32_t r0 = (uint32_t)team * MF_ROUND, rph = 0, s0 = (uint32_t)team * MF_ROUND, aph = 0;
         const uint8_t *srow = nullptr;
+        auto unit_scales = [&]() { // this thread's row of the scale bytes
+            if (u >= n_units) return;
+            const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
+            const int e = __ldg(p.entries + tb).z;
+            srow = (f * MF_ROWS + row < p.n) ? p.scales + ((size_t)e * p.n + f * MF_ROWS + row) * p.nkb : nullptr;
+        };
+        while (r_in_unit >= rpu) { r_in_unit -= rpu; u += (int)gridDim.x; }
+        unit_scales();
         bool ok = true;
         // rounds are counted over all units of this CTA, so slots and teams keep alternating across unit boundaries
         for (uint32_t gr = (uint32_t)team; gr < total_rounds; gr += MF_TEAMS) {
-            ul = gr / (uint32_t)rpu;
-            r_in_unit = gr - ul * (uint32_t)rpu;
-            if (ul != cur_ul) { // first round of this team in a new unit: this thread's row of the scale bytes
-                cur_ul = ul;
-                const int u = (int)blockIdx.x + (int)ul * (int)gridDim.x;
-                const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
-                const int e = __ldg(p.entries + tb).z;
-                srow = (f * MF_ROWS + row < p.n) ? p.scales + ((size_t)e * p.n + f * MF_ROWS + row) * p.nkb : nullptr;
-            }
             // the scale bytes of the round's two blocks come straight from L2 (the row's bytes are neighbours, so most loads
             // hit L1); they are asked for before the polls, which hide their latency. Past k (zero-filled boxes) and past the
             // expert's last out feature: 1.0
-            const int kb0 = (int)r_in_unit * (2 * MF_ROUND) + half;
+            const int kb0 = r_in_unit * (2 * MF_ROUND) + half;
             uint32_t sbv[MF_ROUND];
 #pragma unroll
             for (int h = 0; h < MF_ROUND; h++) sbv[h] = (srow != nullptr && kb0 + 2 * h < p.nkb) ? (uint32_t)__ldg(srow + kb0 + 2 * h) : 127u;
             const uint32_t gs0 = gr * MF_ROUND;
-            const uint32_t r0 = gs0 % MF_RAW_SLOTS, rph = (gs0 / MF_RAW_SLOTS) & 1u;
-            const uint32_t s0 = gs0 % MF_A_SLOTS, aph = (gs0 / MF_A_SLOTS) & 1u;
             // all polls of the round first (they do not depend on each other), the bounded waits only where one failed
             bool tr[MF_ROUND], ta[MF_ROUND];
 #pragma unroll
@@ -279,8 +280,8 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                 if (sb >= 4u && sb <= 250u) { // 2^(s-127) as a bf16 pair: the products are exact
                     // The block's eight magnitudes 0, .5, 1, 1.5, 2, 3, 4, 6 times its scale, as bf16 (four multiplies for
                     // 32 weights), split into a table of low bytes and a table of high bytes; the byte permute unit then looks
-                    // up four nibbles at a time, and each nibble's sign bit is copied onto its element (prmt's sign-replicate
-                    // mode turns bit 7 of a byte into a mask).
+                    // up four nibbles at a time, and the nibbles' sign bits go into the high bytes, four at a time, before
+                    // high and low bytes are paired.
                     const uint32_t s2 = (sb << 7) | (sb << 23);
                     const __nv_bfloat162 sc = *reinterpret_cast<const __nv_bfloat162 *>(&s2);
                     const uint32_t mags[4] = {0x3F000000u, 0x3FC03F80u, 0x40404000u, 0x40C04080u}; // (0, .5) (1, 1.5) (2, 3) (4, 6)
@@ -296,18 +297,17 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                     for (int q = 0; q < 4; q++) {
                         const uint32_t w = v[q];
                         const uint32_t sel_l = w & 0x77777777u, sel_h = sel_l >> 16, wl = w << 4;
-                        const uint32_t lo_a = __byte_perm(tlo_a, tlo_b, sel_l), hi_a = __byte_perm(thi_a, thi_b, sel_l);
-                        const uint32_t lo_b = __byte_perm(tlo_a, tlo_b, sel_h), hi_b = __byte_perm(thi_a, thi_b, sel_h);
-                        const uint32_t pr[4] = {__byte_perm(lo_a, hi_a, 0x5140u), __byte_perm(lo_a, hi_a, 0x7362u),
-                                                __byte_perm(lo_b, hi_b, 0x5140u), __byte_perm(lo_b, hi_b, 0x7362u)};
+                        const uint32_t lo_a = __byte_perm(tlo_a, tlo_b, sel_l), lo_b = __byte_perm(tlo_a, tlo_b, sel_h);
+                        uint32_t hi_a = __byte_perm(thi_a, thi_b, sel_l), hi_b = __byte_perm(thi_a, thi_b, sel_h);
+                        // bit 7 of byte i <- sign of nibble i (4 + i): even nibbles from w << 4, odd ones from w
+                        const uint32_t sg_a = __byte_perm(wl, w, 0x5140u), sg_b = __byte_perm(wl, w, 0x7362u);
+                        asm("lop3.b32 %0, %1, %2, %0, 0x6A;" : "+r"(hi_a) : "r"(sg_a), "r"(0x80808080u)); // (sg & mask) ^ hi
+                        asm("lop3.b32 %0, %1, %2, %0, 0x6A;" : "+r"(hi_b) : "r"(sg_b), "r"(0x80808080u));
                         uint4 o;
-                        uint32_t *ov = reinterpret_cast<uint32_t *>(&o);
-#pragma unroll
-                        for (int b = 0; b < 4; b++) {
-                            // byte 1 <- sign of the low nibble of byte b (bit 7 of (w << 4)), byte 3 <- sign of the high nibble
-                            const uint32_t sm = __byte_perm(wl, w, 0xC080u + 0x1010u * b);
-                            asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(ov[b]) : "r"(sm), "r"(0x80008000u), "r"(pr[b])); // (sm & mask) ^ pr
-                        }
+                        o.x = __byte_perm(lo_a, hi_a, 0x5140u);
+                        o.y = __byte_perm(lo_a, hi_a, 0x7362u);
+                        o.z = __byte_perm(lo_b, hi_b, 0x5140u);
+                        o.w = __byte_perm(lo_b, hi_b, 0x7362u);
                         mf_sts128(dst + ((((uint32_t)(half * 4 + q)) ^ sw) << 4), o);
                     }
                 } else { // scales whose products leave the normal range (NaN, 2^-127 among them): f32 product, one rounding
@@ -338,6 +338,15 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                 }
             }
             if (ut == 0) MF_TRACE(6, gs0);
+            r0 += MF_TEAMS * MF_ROUND;
+            if (r0 == MF_RAW_SLOTS + (uint32_t)team * MF_ROUND) { r0 = (uint32_t)team * MF_ROUND; rph ^= 1u; }
+            s0 += MF_TEAMS * MF_ROUND;
+            if (s0 == MF_A_SLOTS + (uint32_t)team * MF_ROUND) { s0 = (uint32_t)team * MF_ROUND; aph ^= 1u; }
+            r_in_unit += MF_TEAMS;
+            if (r_in_unit >= rpu) { // the next unit (rounds are counted on: slots and teams keep alternating)
+                do { r_in_unit -= rpu; u += (int)gridDim.x; } while (r_in_unit >= rpu);
+                unit_scales();
+            }
         }
     } else if (warp >= 4 + MF_UNPACK_WARPS) {
         // ---- epilogue: lane = out feature inside this warp's quarter of the accumulator rows ---------------

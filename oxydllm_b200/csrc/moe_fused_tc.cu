@@ -7,11 +7,11 @@
 // persistent: CTA b takes units b, b + grid, ... of a device-side table, feature tiles fastest, so that CTAs
 // running at the same time share their token block in L2. Per CTA:
 //   warp 0 (one lane)   TMA: boxes of packed nibbles (128 out features x 32 bytes = 64 input columns) into a
-//                       ring of six slots;
+//                       ring of eight slots;
 //   warp 2 (one lane)   TMA: the stage's tile of the activations ([rows, 64] bf16 in boxes of 64 rows, 128-byte
 //                       swizzle) into one of four slots;
-//   warps 4..19         unpack, two teams of eight warps taking stages in turn: a thread turns one 16-byte block
-//                       (32 weights; its E8M0 scale byte read through L1/L2) into 32 bf16 weights, the bits the
+//   warps 4..19         unpack, four teams of four warps taking stages in turn: a thread turns two 16-byte blocks
+//                       (32 weights each; E8M0 scale bytes read through L1/L2) into bf16 weights, the bits the
 //                       dequantization kernel writes, as four 16-byte chunks of the K-major operand row (128-byte
 //                       swizzle) in one of four slots;
 //   warp 1 (one lane)   tcgen05.mma kind::f16, A = weights [128, 64], B = activations, D[128, rows] f32 in one of
@@ -38,12 +38,12 @@ __device__ long long g_mf_trace[10][256]; // clock stamps of CTA 0, per role and
 
 constexpr int MF_ROWS = 128;                   // out features per unit
 constexpr int MF_BK = 64;                      // input columns per stage
-constexpr int MF_UNPACK_WARPS = 16, MF_TEAMS = 2, MF_TEAM_WARPS = 8, MF_ROUND = 1;
+constexpr int MF_UNPACK_WARPS = 16, MF_TEAMS = 4, MF_TEAM_WARPS = 4, MF_ROUND = 1; // four teams: a stage's chain of poll, unpack, fence and arrival overlaps with three others
 constexpr int MF_EPI_WARPS = 4;
 constexpr int MF_THREADS = (4 + MF_UNPACK_WARPS + MF_EPI_WARPS) * 32;
 constexpr int MF_SLOTS = 4;                    // operand slots: an unpacked weight tile and an activation tile each, one pair of barriers
 constexpr int MF_A_SLOTS = MF_SLOTS, MF_X_SLOTS = MF_SLOTS;
-constexpr int MF_RAW_SLOTS = 6;
+constexpr int MF_RAW_SLOTS = 8;
 constexpr int MF_MAX_TOK = 256;                // rows of a token block
 constexpr int MF_TMEM_BUF = 256;               // accumulator columns per buffer
 constexpr int MF_A_BYTES = MF_ROWS * MF_BK * 2;
@@ -223,8 +223,9 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
         // ---- unpack ---------------------------------------------------------------------------------------
         const int team = (warp - 4) / MF_TEAM_WARPS;
         const int ut = (threadIdx.x - 128) % (MF_TEAM_WARPS * 32);
-        const int row = ut >> 1, half = ut & 1;                   // this thread: one 16-byte block of one out feature per stage
-        const uint32_t raw_off = (uint32_t)row * 32u + (uint32_t)half * 16u;
+        const int row = ut;                                       // this thread: both 16-byte blocks of one out feature per stage
+        static_assert(MF_TEAM_WARPS * 32 == MF_ROWS && MF_ROUND == 1, "a thread per out feature");
+        const uint32_t raw_off = (uint32_t)row * 32u;
         const uint32_t a_row = (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u;
         const uint32_t sw = (uint32_t)(row & 7);
         const int rpu = nk2 / MF_ROUND;                            // rounds per unit
@@ -251,10 +252,10 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
             // the scale bytes of the round's two blocks come straight from L2 (the row's bytes are neighbours, so most loads
             // hit L1); they are asked for before the polls, which hide their latency. Past k (zero-filled boxes) and past the
             // expert's last out feature: 1.0
-            const int kb0 = r_in_unit * (2 * MF_ROUND) + half;
-            uint32_t sbv[MF_ROUND];
+            const int kb0 = r_in_unit * 2;
+            uint32_t sbv[2];
 #pragma unroll
-            for (int h = 0; h < MF_ROUND; h++) sbv[h] = (srow != nullptr && kb0 + 2 * h < p.nkb) ? (uint32_t)__ldg(srow + kb0 + 2 * h) : 127u;
+            for (int h = 0; h < 2; h++) sbv[h] = (srow != nullptr && kb0 + h < p.nkb) ? (uint32_t)__ldg(srow + kb0 + h) : 127u;
             const uint32_t gs0 = gr * MF_ROUND;
             // all polls of the round first (they do not depend on each other), the bounded waits only where one failed
             bool tr[MF_ROUND], ta[MF_ROUND];
@@ -272,11 +273,11 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
             if (ut == 0) MF_TRACE(4, gs0);
             if (!MF_DBG(1))
 #pragma unroll
-            for (int h = 0; h < MF_ROUND; h++) {
-                const uint32_t sb = sbv[h];
-                const uint4 rawv = mf_lds128(raw_base + (r0 + h) * MF_RAW_BYTES + raw_off);
+            for (int half = 0; half < 2; half++) {
+                const uint32_t sb = sbv[half];
+                const uint4 rawv = mf_lds128(raw_base + r0 * MF_RAW_BYTES + raw_off + 16u * half);
                 const uint32_t v[4] = {rawv.x, rawv.y, rawv.z, rawv.w};
-                const uint32_t dst = base + (s0 + h) * MF_A_BYTES + a_row;
+                const uint32_t dst = base + s0 * MF_A_BYTES + a_row;
                 if (sb >= 4u && sb <= 250u) { // 2^(s-127) as a bf16 pair: the products are exact
                     // The block's eight magnitudes 0, .5, 1, 1.5, 2, 3, 4, 6 times its scale, as bf16 (four multiplies for
                     // 32 weights), split into a table of low bytes and a table of high bytes; the byte permute unit then looks

@@ -11,7 +11,7 @@
 // across tile borders. Roles:
 //   warp 0        TMA: units of packed words (128 out features), the zero points of their groups and the scales of each fold, as
 //                 far ahead as the ring allows: this is what is in flight from HBM;
-//   warp 2        TMA: the unit's tile of x ([tokens, 128] bf16, two 128-byte swizzled halves);
+//   warp 2        TMA: the stage's tile of x ([tokens, 64] bf16, 128-byte swizzle);
 //   warps 4..11   unpack, four teams of two warps that take the stages (64 input rows) in turn: a packed word becomes one
 //                 16-byte chunk of the operand tile (AWQ: eight out features of one input row, MN-major; GPTQ: eight input
 //                 rows of one out feature, K-major);
@@ -24,8 +24,8 @@
 // What bounds it: shared memory. A stage moves 4 KB of packed words in and out, 16 KB of operand in and out, and the x
 // tile: at 128 B per clock about 350 clocks for 64 x 128 weights at 16 tokens; 430 measured. Beside that about 6 us a
 // launch go into filling the pipeline and putting shared tiles together. Measured in a graph, us at 16 / 77 / 128 tokens (the
-// kernel with scaled bf16 weights before it): 4096 x 4096 10 / 17 / 20 (14 / 19 / 22), 4096 x 28672 28 / 43 / 53 (55 / 59 / 61),
-// 14336 x 4096 18 / 27 / 33 (28 / 34 / 38).
+// kernel with scaled bf16 weights before it): 4096 x 4096 10 / 16 / 20 (14 / 19 / 22), 4096 x 28672 30 / 49 / 55 (55 / 59 / 61),
+// 14336 x 4096 20 / 27 / 33 (28 / 34 / 38).
 #include <atomic>
 
 #include <cuda_bf16.h>
@@ -47,19 +47,18 @@ constexpr int GT_ROW_BYTES = 64;             // packed words of one input row of
 constexpr int GT_ZERO_BYTES = 64;            // zero points of one group of the tile: 16 words
 constexpr int GT_RAW_BYTES = GT_UNIT * GT_ROW_BYTES + GT_UNIT / 32 * GT_ZERO_BYTES; // a unit holds up to four groups
 constexpr int GT_A_BYTES = GT_ROWS * GT_BK * 2;
-constexpr int GT_MAX_RAW = 32, GT_MAX_SLOTS = 8, GT_MAX_X = 4;
+constexpr int GT_MAX_RAW = 32, GT_MAX_SLOTS = 8, GT_MAX_X = 8;
 constexpr int GT_ISSUERS = 2;                // warps that issue MMAs, on alternate units: one warp alone issues one every 90 clocks
 constexpr int GT_ACC = 4;                    // accumulator buffers
 constexpr int GT_SC = 16, GT_SC_BYTES = 256; // ring of scales: one 128-wide row of 16-bit scales per fold
 constexpr int GT_NUM_BARS = 2 * GT_MAX_RAW + 2 * GT_MAX_SLOTS + 2 * GT_MAX_X + 2 * GT_ACC + 2 * GT_SC;
 constexpr int GT_MAX_TOKENS = 128;           // per tile
 constexpr int GROUP_TC_MAX_M = 256, GT_NARROW_TILES = 74;
-constexpr int GT_SHARE_COST = 512;
 constexpr int GT_SMEM_BUDGET = 227 * 1024;
 // A parity wait tells a phase from the next one only: whoever waits on a barrier has to see every one of its phases. So a slot
 // always meets the same team and the same issuer, and a ring slot the same teams: their counts are multiples of these.
 static_assert(GT_SC % (GT_UNIT / 32) == 0 && GT_MAX_SLOTS % GT_TEAMS == 0 && GT_TEAMS % (GT_UNIT_STAGES * GT_ISSUERS) == 0 &&
-                  GT_MAX_RAW % GT_TEAMS == 0 && GT_MAX_X % GT_ISSUERS == 0,
+                  GT_MAX_RAW % GT_TEAMS == 0 && GT_MAX_X % (GT_UNIT_STAGES * GT_ISSUERS) == 0,
               "slots and who meets them");
 
 template <int V> struct GtInt { static constexpr int value = V; };
@@ -72,8 +71,8 @@ struct GroupTcParams {
     int m, n, packed_out;
     int mpad;                       // tokens of a tile, a multiple of 16
     int token_blocks;               // tiles of the same out features: tile = feature tile * token_blocks + token block
-    int slots, x_slots, raw_slots;  // operand tiles, units of x, units of packed words in shared memory
-    int x_bytes;                    // of a unit
+    int slots, x_slots, raw_slots;  // operand tiles, x tiles (a stage each), units of packed words in shared memory
+    int x_bytes;                    // of an x tile
     int acc_cols;                   // tensor-memory columns of an accumulator buffer, a power of two
     int gshift;                     // log2(group size)
     int fold_rows;                  // min(group size, 128): input rows per accumulator buffer
@@ -146,7 +145,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand tiles want 1 KB alignment
     unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    // operand tiles | units of x | ring of packed units | ring of scales | barriers | tensor-memory address, ticket
+    // operand tiles | x tiles | ring of packed units | ring of scales | barriers | tensor-memory address, ticket
     const int S = p.slots, X = p.x_slots, R = p.raw_slots;
     const uint32_t x_base = base + (uint32_t)(S * GT_A_BYTES), raw_base = x_base + (uint32_t)(X * p.x_bytes);
     const uint32_t sc_base = raw_base + (uint32_t)(R * GT_RAW_BYTES);
@@ -244,31 +243,30 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             }
         }
     } else if (warp == 2) {
-        // ---- x, a unit at a time, as soon as the MMAs that read the slot have completed ------------------------------
+        // ---- x, a stage at a time, as soon as the MMAs that read the slot have completed -----------------------------
         const bool leader = elect_one();
-        int tb = first_tile % p.token_blocks, uk = first_unit, x = 0;
+        int tb = first_tile % p.token_blocks, k0 = first_unit * GT_UNIT, x = 0;
         uint32_t ph = 0;
         bool ok = true;
         pdl_wait();
-        for (int it = 0; it < nunits && ok; it++) {
+        for (int it = 0; it < nstages && ok; it++) {
             if (it >= X) ok = gt_wait(xempty + 8 * x, ph ^ 1u, p.flag, 5);
             if (ok && leader) {
-                const uint32_t dst = x_base + (uint32_t)(x * p.x_bytes), bar = xfull + 8 * x;
-                mbar_arrive_expect_tx(bar, (uint32_t)p.x_bytes);
-                tma_load_2d(dst, &xmap, bar, uk * GT_UNIT, tb * p.mpad);
-                tma_load_2d(dst + p.mpad * 128, &xmap, bar, uk * GT_UNIT + GT_BK, tb * p.mpad);
+                mbar_arrive_expect_tx(xfull + 8 * x, (uint32_t)p.x_bytes);
+                tma_load_2d(x_base + (uint32_t)(x * p.x_bytes), &xmap, xfull + 8 * x, k0, tb * p.mpad);
             }
             __syncwarp();
             if (++x == X) { x = 0; ph ^= 1u; }
-            if (++uk == G) {
-                uk = 0;
+            k0 += GT_BK;
+            if (k0 == G * GT_UNIT) {
+                k0 = 0;
                 if (++tb == p.token_blocks) tb = 0;
             }
         }
         // The commits of the last stages arrive here asynchronously: the CTA stays until they have.
         for (int left = min(S, nstages), q = nstages - left; left > 0 && ok; left--, q++)
             ok = gt_wait(empty + 8 * (q % S), (uint32_t)(q / S) & 1u, p.flag, 11);
-        for (int left = min(X, nunits), q = nunits - left; left > 0 && ok; left--, q++)
+        for (int left = min(X, nstages), q = nstages - left; left > 0 && ok; left--, q++)
             ok = gt_wait(xempty + 8 * (q % X), (uint32_t)(q / X) & 1u, p.flag, 11);
     } else if (warp < 4) {
         // ---- MMA issue: warps 1 and 3 take the units in turn -------------------------------------------------------
@@ -277,17 +275,17 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         const int me = warp >> 1;
         const uint32_t idesc = tc_idesc(GT_ROWS, p.mpad) | (GPTQ ? 0u : (1u << 15)); // bit 15: A is MN-major
         const uint64_t adesc0 = GPTQ ? kmajor_sw128_desc(base) : gt_mn_desc(base), bdesc0 = kmajor_sw128_desc(x_base);
-        const uint32_t x16 = (uint32_t)p.x_bytes >> 4, xstage16 = (uint32_t)p.mpad * 8; // 16-byte units
+        const uint32_t x16 = (uint32_t)p.x_bytes >> 4; // 16-byte units
         auto issue = [&](auto fold_mmas) { // MMAs (16 input rows each) per accumulator buffer
             constexpr int FM = decltype(fold_mmas)::value, US = GT_UNIT_STAGES;
             constexpr int UF = US * 4 / FM; // folds of a unit
-            int s = me * US, a = me * UF, x = me;
+            int s = me * US, a = me * UF, x = me * US;
             uint32_t ph = 0, xph = 0, aph = 1; // aph: parity of the last release of the buffer (a fresh barrier passes parity 1)
             for (int ui = me; ui < nunits; ui += issuers) {
-                bool ok = gt_wait(xfull + 8 * x, xph, p.flag, 6);
+                bool ok = true;
 #pragma unroll
                 for (int st = 0; st < US; st++) {
-                    if (ok) ok = gt_wait(full + 8 * s, ph, p.flag, 2);
+                    ok = ok && gt_wait(xfull + 8 * x, xph, p.flag, 6) && gt_wait(full + 8 * s, ph, p.flag, 2);
 #pragma unroll
                     for (int part = 0; part < (FM < 4 ? 4 / FM : 1); part++) {
                         const bool first = FM <= 4 || st == 0, last = FM <= 4 || st == US - 1;
@@ -295,7 +293,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                         if (ok) {
                             tc_fence_after();
                             const uint32_t d = tmem_base + (uint32_t)(a * p.acc_cols);
-                            const uint64_t da = adesc0 + (uint64_t)(s * (GT_A_BYTES >> 4)), db = bdesc0 + (uint64_t)(x * x16 + st * xstage16);
+                            const uint64_t da = adesc0 + (uint64_t)(s * (GT_A_BYTES >> 4)), db = bdesc0 + (uint64_t)(x * x16);
                             if (leader) {
 #pragma unroll
                                 for (int kk = 0; kk < (FM < 4 ? FM : 4); kk++) { // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes of a K-major row
@@ -308,15 +306,17 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                         }
                         if (last) a++;
                     }
-                    if (ok && leader) umma_commit(empty + 8 * s);
+                    if (ok && leader) {
+                        umma_commit(empty + 8 * s);
+                        umma_commit(xempty + 8 * x);
+                    }
                     __syncwarp();
                     if (++s == S) { s = 0; ph ^= 1u; }
+                    if (++x == X) { x = 0; xph ^= 1u; }
                 }
                 if (!ok) break;
-                if (leader) umma_commit(xempty + 8 * x);
-                __syncwarp();
                 // on to this warp's next unit
-                x += issuers;
+                x += (issuers - 1) * US;
                 if (x >= X) { x -= X; xph ^= 1u; }
                 s += (issuers - 1) * US;
                 if (s >= S) { s -= S; ph ^= 1u; }
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                     const unsigned last = (unsigned)(i_hi - i_lo);
                     unsigned count;
                     __threadfence(); // the parts of the whole CTA (ordered before this by the barrier) before the ticket
-                    for (;;) {
+                    for (;;) { // (with a ticket read at the start of the segment the swap mostly failed at first: 4096 x 1024 15 -> 21 us)
                         count = (old >> 8) == p.mark ? (unsigned)(old & 0xFFu) : 0u;
                         seen = atomicCAS(ticket, old, (p.mark << 8) | (count == last ? 0u : count + 1u));
                         if (seen == old) break; // fails only when another of the tile's few CTAs came in between
@@ -564,15 +564,14 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
 }
 
 // Largest batch for this kernel. Above it the kernel of fused_tc.cu, which scales and rounds the weights as it unpacks them and
-// folds nothing, is the faster one, us there / here: groups of 64, where every stage is folded, 3072 x 5120 at 16 / 77 tokens
-// 14.6 / 12.8 and 18.9 / 21.6, 3072 x 16384 25.4 / 18.6 and 26.6 / 34.5, but 8192 x 3072 at 77 26.3 / 24.6; one tile per CTA, 4096 x
-// 14336, 31.1 / 32.9 at 128 tokens. More than 128 tokens are two tiles that unpack the same weights twice: worth it where that
+// folds nothing, is the faster one, us there / here: groups of 64, where every stage is folded, 3072 x 5120 at 16 / 48 tokens
+// 14.6 / 12.8 and 16.6 / 19.3, 3072 x 16384 25.4 / 18.6 and 25.8 / 26.9; one tile per CTA, 4096 x 14336, 31.1 / 31.5 at 128 tokens. More than 128 tokens are two tiles that unpack the same weights twice: worth it where that
 // fills idle SMs (256 tokens, 4096 x 4096: 34 / 23; 4096 x 14336: 41 / 51). Groups of 32 have no other such kernel (4096 x 14336
 // through the dense copy: 71 us).
 int group_tc_max_m(int n, int group_size)
 {
     const int tiles = n / GT_ROWS;
-    if (group_size == 64 && tiles > 32) return 48;
+    if (group_size == 64) return 32;
     return tiles <= GT_NARROW_TILES ? GROUP_TC_MAX_M : tiles <= 148 && group_size > 32 ? 96 : GT_MAX_TOKENS;
 }
 
@@ -633,12 +632,12 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
     p.mpad = ceil_div(ceil_div(m, p.token_blocks), 16) * 16;
     p.units_per_tile = k / GT_UNIT;
     p.tiles = n / GT_ROWS * p.token_blocks;
-    p.x_bytes = GT_UNIT * p.mpad * 2;
+    p.x_bytes = GT_BK * p.mpad * 2;
     // Shared memory: two operand tiles per team (with one, a team waits for the MMAs of its own last stage: 4096 x 28672 at 32
     // tokens 39.6 us against 29.6) while at least four units of packed words, 33 KB, stay in flight.
     const int fixed = 1024 + GT_SC * GT_SC_BYTES + 8 * GT_NUM_BARS + 16;
     p.slots = p.mpad <= 96 ? 2 * GT_TEAMS : GT_TEAMS;
-    p.x_slots = p.mpad <= 32 ? GT_MAX_X : GT_ISSUERS;
+    p.x_slots = p.mpad <= 32 ? GT_MAX_X : GT_MAX_X / 2;
     p.raw_slots = (GT_SMEM_BUDGET - fixed - p.slots * GT_A_BYTES - p.x_slots * p.x_bytes) / GT_RAW_BYTES;
     if (p.raw_slots > GT_MAX_RAW) p.raw_slots = GT_MAX_RAW;
     p.raw_slots -= p.raw_slots % (GT_TEAMS / GT_UNIT_STAGES);
@@ -646,21 +645,29 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
     while (p.acc_cols < p.mpad) p.acc_cols *= 2;
     const size_t smem = (size_t)p.slots * GT_A_BYTES + (size_t)p.x_slots * p.x_bytes + (size_t)p.raw_slots * GT_RAW_BYTES + fixed;
 
-    // Equal shares of the (tile, unit) list, one CTA per SM: at least two units a share, and at most `most` shares of a tile,
-    // because the last of them reads all parts of the tile by itself. The parts must fit the scratch area; otherwise, and where it
-    // does not pay, shares are whole tiles. A shared tile costs its CTAs about as much as GT_SHARE_COST input rows of work.
+    // Equal shares of the (tile, unit) list. Sharing a tile costs its last CTA time that grows with the number of parts and their
+    // size; in units (about 0.34 us at 16 tokens) 7.5 + 0.75 x parts x (1 + tokens / 32) follows what was measured: whole tiles against
+    // shares on all SMs 9.6 / 10 us at 2048 x 1024 and 9.7 / 12 at 2048 x 3072 (8 tokens), 12 / 19 at 2048 x 3072 (48 tokens), 23 / 25 at
+    // 4096 x 14336 (64 tokens); 16 parts of a 4096 x 1024 tile 15 us. The parts must fit the scratch area.
     const long long total = (long long)p.tiles * p.units_per_tile;
-    const int most = p.mpad <= 16 ? 16 : p.mpad <= 64 ? 8 : 6;
     const size_t part_bytes = (size_t)p.mpad * GT_ROWS * sizeof(float), ticket_bytes = group_tc_ticket_bytes(p.tiles);
-    long long ctas = sm_count();
-    if (ctas > total / 2) ctas = total / 2;
-    if (ctas > (long long)p.tiles * most) ctas = (long long)p.tiles * most;
     const long long fit = scratch && scratch_bytes > ticket_bytes ? (long long)((scratch_bytes - ticket_bytes) / part_bytes) - p.tiles : 0;
-    if (ctas > fit) ctas = fit;
-    const int whole = ceil_div(p.tiles, sm_count()) * p.units_per_tile;
-    p.split = ctas >= 1 && (ctas >= p.tiles || ctas == sm_count()) &&
-              whole > ceil_div((int)total, (int)ctas) + ceil_div(GT_SHARE_COST, GT_UNIT);
-    if (!p.split) ctas = p.tiles < sm_count() ? p.tiles : sm_count();
+    long long ctas = p.tiles < sm_count() ? p.tiles : sm_count();
+    int cost4 = 4 * ceil_div(p.tiles, (int)ctas) * p.units_per_tile; // quarter units
+    p.split = 0;
+    for (int c = 2; c <= 16; c++) {
+        long long cand = (long long)p.tiles * c;
+        if (cand > sm_count()) cand = sm_count();
+        if (cand > total / 2) cand = total / 2;
+        if (cand > fit) cand = fit;
+        if (cand < p.tiles && cand < sm_count()) break; // shares of more than a tile only with every SM at work
+        const int parts = ceil_div((int)cand, p.tiles) + (cand % p.tiles ? 1 : 0);
+        int share = 30 + 3 * parts * (32 + p.mpad) / 32;
+        if (p.mpad > 64) share = share * 7 / 10; // the units take longer too (3072 x 1024 at 100 tokens: 22 us on whole tiles, 17 shared)
+        const int cost = 4 * ceil_div((int)total, (int)cand) + share;
+        if (cost < cost4) { cost4 = cost; ctas = cand; p.split = 1; }
+        if (cand == sm_count()) break;
+    }
     static std::atomic<unsigned long long> calls{0}; // marks differ between calls, in no order that a stale value would have by chance
     p.mark = ((calls.fetch_add(1, std::memory_order_relaxed) + 1) * 0x9E3779B97F4A7C15ull) >> 8;
     p.tickets = reinterpret_cast<unsigned long long *>(scratch);

@@ -1,5 +1,5 @@
-// AWQ W4A16 matmul for batches of up to 256 tokens with the dequantization fused into the tensor-core
-// kernel: the packed words are read from HBM once and no dense copy of the weight is ever written.
+// AWQ / GPTQ W4A16 (above the batches that group_tc.cu takes) and FP8 matmul of up to 256 tokens with the dequantization
+// fused into the tensor-core kernel: the packed words are read from HBM once and no dense copy of the weight is ever written.
 //
 // One CTA owns 128 out features and walks k in stages of 64 input rows:
 //   warp 0 (one lane)   TMA: boxes of packed words (64 rows x 16 words, 4 KB) into a ring of up to 32 slots,

@@ -217,8 +217,7 @@ int oxq_gemm_check(const void *workspace, void *stream);
 
 /* PackedQuantLinear::forward beyond the decode GEMV: maybe_mpp_quant_matmul, else
  * dequantize_w4 + matmul (linear.rs:494-524, metal_ops.rs:2771-2797). Up to 256
- * tokens, when n % 128 == 0, k % 128 == 0, group_size is a power of two >= 32 (64
- * above 128 tokens on wide layers) and the scales are f16 or bf16, one kernel unpacks
+ * tokens, when n % 128 == 0, k % 128 == 0, group_size is a power of two >= 64 and the scales are f16 or bf16, one kernel unpacks
  * the words into its shared-memory operand and multiplies on tcgen05 (no slab
  * written); all other calls dequantize slabs into the workspace. The workspace is required
  * (and its flag word used) either way. */

@@ -194,7 +194,7 @@ OXQ_EXPORT int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight,
 // streams only share the flag word; OXQ_ERR_UNSUPPORTED where the kernel does not take the shape.
 OXQ_EXPORT int oxq_packed4_max_m(int k, int n, int group_size)
 {
-    return k > 0 && n > 0 && n % 128 == 0 && k % 128 == 0 && group_size >= 32 && (group_size & (group_size - 1)) == 0
+    return k > 0 && n > 0 && n % 128 == 0 && k % 128 == 0 && group_size >= 64 && (group_size & (group_size - 1)) == 0
                ? group_tc_max_m(n, group_size) : 0;
 }
 

@@ -45,7 +45,7 @@ constexpr int GT_FOLD_WARP0 = 4 + GT_UNPACK_WARPS; // a multiple of four: warp %
 constexpr int GT_THREADS = (GT_FOLD_WARP0 + GT_FOLD_WARPS) * 32;
 constexpr int GT_ROW_BYTES = 64;             // packed words of one input row of the tile (GPTQ: 1 / 8 of a packed row's 512 bytes)
 constexpr int GT_ZERO_BYTES = 64;            // zero points of one group of the tile: 16 words
-constexpr int GT_RAW_BYTES = GT_UNIT * GT_ROW_BYTES + GT_UNIT / 32 * GT_ZERO_BYTES; // a unit holds up to four groups
+constexpr int GT_RAW_BYTES = GT_UNIT * GT_ROW_BYTES + GT_UNIT / GT_BK * GT_ZERO_BYTES; // a unit holds up to two groups
 constexpr int GT_A_BYTES = GT_ROWS * GT_BK * 2;
 constexpr int GT_MAX_RAW = 32, GT_MAX_SLOTS = 8, GT_MAX_X = 8;
 constexpr int GT_ISSUERS = 2;                // warps that issue MMAs, on alternate units: one warp alone issues one every 90 clocks
@@ -57,7 +57,7 @@ constexpr int GROUP_TC_MAX_M = 256, GT_NARROW_TILES = 74;
 constexpr int GT_SMEM_BUDGET = 227 * 1024;
 // A parity wait tells a phase from the next one only: whoever waits on a barrier has to see every one of its phases. So a slot
 // always meets the same team and the same issuer, and a ring slot the same teams: their counts are multiples of these.
-static_assert(GT_SC % (GT_UNIT / 32) == 0 && GT_MAX_SLOTS % GT_TEAMS == 0 && GT_TEAMS % (GT_UNIT_STAGES * GT_ISSUERS) == 0 &&
+static_assert(GT_MAX_SLOTS % GT_TEAMS == 0 && GT_TEAMS % (GT_UNIT_STAGES * GT_ISSUERS) == 0 &&
                   GT_MAX_RAW % GT_TEAMS == 0 && GT_MAX_X % (GT_UNIT_STAGES * GT_ISSUERS) == 0,
               "slots and who meets them");
 
@@ -271,7 +271,6 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     } else if (warp < 4) {
         // ---- MMA issue: warps 1 and 3 take the units in turn -------------------------------------------------------
         const bool leader = elect_one();
-        const int issuers = p.fold_rows == 32 ? 1 : GT_ISSUERS; // four folds a unit: every unit uses all buffers, so one warp issues all
         const int me = warp >> 1;
         const uint32_t idesc = tc_idesc(GT_ROWS, p.mpad) | (GPTQ ? 0u : (1u << 15)); // bit 15: A is MN-major
         const uint64_t adesc0 = GPTQ ? kmajor_sw128_desc(base) : gt_mn_desc(base), bdesc0 = kmajor_sw128_desc(x_base);
@@ -281,31 +280,26 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             constexpr int UF = US * 4 / FM; // folds of a unit
             int s = me * US, a = me * UF, x = me * US;
             uint32_t ph = 0, xph = 0, aph = 1; // aph: parity of the last release of the buffer (a fresh barrier passes parity 1)
-            for (int ui = me; ui < nunits; ui += issuers) {
+            for (int ui = me; ui < nunits; ui += GT_ISSUERS) {
                 bool ok = true;
 #pragma unroll
                 for (int st = 0; st < US; st++) {
                     ok = ok && gt_wait(xfull + 8 * x, xph, p.flag, 6) && gt_wait(full + 8 * s, ph, p.flag, 2);
+                    const bool first = FM == 4 || st == 0, last = FM == 4 || st == US - 1; // of the buffer's stages
+                    if (first && ok) ok = gt_wait(accempty + 8 * a, aph, p.flag, 9);
+                    if (ok) {
+                        tc_fence_after();
+                        const uint32_t d = tmem_base + (uint32_t)(a * p.acc_cols);
+                        const uint64_t da = adesc0 + (uint64_t)(s * (GT_A_BYTES >> 4)), db = bdesc0 + (uint64_t)(x * x16);
+                        if (leader) {
 #pragma unroll
-                    for (int part = 0; part < (FM < 4 ? 4 / FM : 1); part++) {
-                        const bool first = FM <= 4 || st == 0, last = FM <= 4 || st == US - 1;
-                        if (first && ok) ok = gt_wait(accempty + 8 * a, aph, p.flag, 9);
-                        if (ok) {
-                            tc_fence_after();
-                            const uint32_t d = tmem_base + (uint32_t)(a * p.acc_cols);
-                            const uint64_t da = adesc0 + (uint64_t)(s * (GT_A_BYTES >> 4)), db = bdesc0 + (uint64_t)(x * x16);
-                            if (leader) {
-#pragma unroll
-                                for (int kk = 0; kk < (FM < 4 ? FM : 4); kk++) { // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes of a K-major row
-                                    const int q = part * FM + kk;
-                                    umma_bf16(d, da + (uint64_t)(q * (GPTQ ? 2 : (2048 >> 4))), db + 2 * q, idesc, !(first && kk == 0));
-                                }
-                                if (last) umma_commit(accfull + 8 * a);
-                            }
-                            __syncwarp();
+                            for (int kk = 0; kk < 4; kk++) // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes of a K-major row
+                                umma_bf16(d, da + (uint64_t)(kk * (GPTQ ? 2 : (2048 >> 4))), db + 2 * kk, idesc, !(first && kk == 0));
+                            if (last) umma_commit(accfull + 8 * a);
                         }
-                        if (last) a++;
+                        __syncwarp();
                     }
+                    if (last) a++;
                     if (ok && leader) {
                         umma_commit(empty + 8 * s);
                         umma_commit(xempty + 8 * x);
@@ -316,18 +310,16 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                 }
                 if (!ok) break;
                 // on to this warp's next unit
-                x += (issuers - 1) * US;
+                x += (GT_ISSUERS - 1) * US;
                 if (x >= X) { x -= X; xph ^= 1u; }
-                s += (issuers - 1) * US;
+                s += (GT_ISSUERS - 1) * US;
                 if (s >= S) { s -= S; ph ^= 1u; }
-                a += (issuers - 1) * UF;
+                a += (GT_ISSUERS - 1) * UF;
                 if (a >= GT_ACC) { a -= GT_ACC; aph ^= 1u; }
             }
         };
-        if (me >= issuers) {
-        } else if (p.fold_rows == 128) issue(GtInt<8>{});
-        else if (p.fold_rows == 64) issue(GtInt<4>{});
-        else issue(GtInt<2>{});
+        if (p.fold_rows == GT_UNIT) issue(GtInt<8>{});
+        else issue(GtInt<4>{});
     } else if (warp < GT_FOLD_WARP0) {
         // ---- unpack ----------------------------------------------------------------------------------------------
         const int team = (warp - 4) / GT_TEAM_WARPS;
@@ -342,9 +334,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         uint32_t ph = 0, rph = 0;
         const uint32_t half_unit = (uint32_t)(team % GT_UNIT_STAGES);
         const uint32_t part = half_unit * (GT_BK * GT_ROW_BYTES);
-        // groups of 128 rows and more: one zero point per unit; 64: one per stage; 32: two
-        const uint32_t zeros_at = GT_UNIT * GT_ROW_BYTES + (p.fold_rows == 128 ? 0u : half_unit * (uint32_t)(GT_BK / p.fold_rows) * GT_ZERO_BYTES);
-        const bool two_groups = p.fold_rows < GT_BK;
+        // groups of 128 rows and more: one zero point per unit; 64: one per stage
+        const uint32_t zeros_at = GT_UNIT * GT_ROW_BYTES + (p.fold_rows == GT_UNIT ? 0u : half_unit * GT_ZERO_BYTES);
         bool ok = true;
         for (int it = team; it < nstages; it += GT_TEAMS) {
             const bool t0 = mbar_test(rawfull + 8 * r, rph);
@@ -358,15 +349,11 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                 const uint32_t src = box + (uint32_t)(r0 * 16 + j) * 4u, zsrc = zeros_addr + 4u * j;
                 const uint32_t dst = slot + (uint32_t)(j >> 3) * 8192u;
                 uint32_t zp[4];
-                auto zeros = [&](uint32_t addr) {
-                    const uint32_t zw = gt_lds32(addr);
+                const uint32_t zw = gt_lds32(zsrc);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) zp[q] = gt_and_or(zw >> (4 * q), nib_mask, nib_magic);
-                };
-                zeros(zsrc);
+                for (int q = 0; q < 4; q++) zp[q] = gt_and_or(zw >> (4 * q), nib_mask, nib_magic);
 #pragma unroll
                 for (int half = 0; half < 2; half++) {
-                    if (half == 1 && two_groups) zeros(zsrc + GT_ZERO_BYTES);
                     uint32_t w[8];
 #pragma unroll
                     for (int i = 0; i < 8; i++) w[i] = gt_lds32(src + (uint32_t)(half * 8 + i) * 256u);
@@ -390,17 +377,13 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
 #pragma unroll
                     for (int c = 0; c < 8; c++) w[c] = gt_lds32(box + (uint32_t)(c * 128 + f) * 4u);
                     uint32_t zp = 0x43084308u; // symmetric: zero 7, + 1
-                    auto zeros = [&](int z) {
-                        if (!p.sym) {
-                            const uint32_t z1 = ((gt_lds32(zeros_addr + z * GT_ZERO_BYTES + 4u * (f >> 3)) >> (4 * (f & 7))) & 0xFu) + 1u;
-                            zp = 0x43004300u | z1 | (z1 << 16); // bf16 pair (128 + z + 1)
-                        }
-                    };
-                    zeros(0);
+                    if (!p.sym) {
+                        const uint32_t z1 = ((gt_lds32(zeros_addr + 4u * (f >> 3)) >> (4 * (f & 7))) & 0xFu) + 1u;
+                        zp = 0x43004300u | z1 | (z1 << 16); // bf16 pair (128 + z + 1)
+                    }
                     const uint32_t dst = slot + (uint32_t)(f >> 3) * 1024u + (uint32_t)(f & 7) * 128u;
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
-                        if (c == 4 && two_groups) zeros(1);
                         // byte b of the word: rows 2b (low nibble) and 2b + 1 (high nibble), neighbours in the K-major row
                         const uint32_t w4 = w[c] >> 4;
                         uint4 o;
@@ -566,20 +549,20 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
 // Largest batch for this kernel. Above it the kernel of fused_tc.cu, which scales and rounds the weights as it unpacks them and
 // folds nothing, is the faster one, us there / here: groups of 64, where every stage is folded, 3072 x 5120 at 16 / 48 tokens
 // 14.6 / 12.8 and 16.6 / 19.3, 3072 x 16384 25.4 / 18.6 and 25.8 / 26.9; one tile per CTA, 4096 x 14336, 31.1 / 31.5 at 128 tokens. More than 128 tokens are two tiles that unpack the same weights twice: worth it where that
-// fills idle SMs (256 tokens, 4096 x 4096: 34 / 23; 4096 x 14336: 41 / 51). Groups of 32 have no other such kernel (4096 x 14336
-// through the dense copy: 71 us).
+// fills idle SMs (256 tokens, 4096 x 4096: 34 / 23; 4096 x 14336: 41 / 51). Groups of 32 would be
+// folded four times a unit: 4096 x 28672 took 58 us at any batch, the GEMV 38 at 8 tokens, and above 32 tokens the dense copy wins.
 int group_tc_max_m(int n, int group_size)
 {
     const int tiles = n / GT_ROWS;
     if (group_size == 64) return 32;
-    return tiles <= GT_NARROW_TILES ? GROUP_TC_MAX_M : tiles <= 148 && group_size > 32 ? 96 : GT_MAX_TOKENS;
+    return tiles <= GT_NARROW_TILES ? GROUP_TC_MAX_M : tiles <= 148 ? 96 : GT_MAX_TOKENS;
 }
 
 // True when this kernel serves the call.
 bool group_tc_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
                         const void *scales)
 {
-    return m >= 1 && m <= group_tc_max_m(n, group_size) && n % GT_ROWS == 0 && k % GT_UNIT == 0 && group_size >= 32 &&
+    return m >= 1 && m <= group_tc_max_m(n, group_size) && n % GT_ROWS == 0 && k % GT_UNIT == 0 && group_size >= 64 &&
            (group_size & (group_size - 1)) == 0 && (scales_dtype == OXQ_F16 || scales_dtype == OXQ_BF16) && aligned(x, 16) &&
            aligned(qweight, 16) && aligned(qzeros, 16) && aligned(scales, 16);
 }

@@ -276,7 +276,7 @@ class PackedQuantLinear:
         """Largest batches of the grouped unpack + tcgen05 kernel (0: not this layer) and of the GEMV."""
         k, n, g = self.in_features, self.out_features, self.group_size
         awq = self.pack_dim == "out"
-        grouped = (self.bits == 4 and n % 128 == 0 and k % 128 == 0 and g >= 32 and g & (g - 1) == 0
+        grouped = (self.bits == 4 and n % 128 == 0 and k % 128 == 0 and g >= 64 and g & (g - 1) == 0
                    and self.scales.dtype in (torch.float16, torch.bfloat16)
                    and all(t is None or t.data_ptr() % 16 == 0 for t in (self.qweight, self.qzeros, self.scales)))
         if not grouped:
@@ -286,12 +286,11 @@ class PackedQuantLinear:
             return most, GPTQ_FUSED_MIN_M - 1 if k * n <= GPTQ_GEMV_MAX_WEIGHTS else 0
         # The GEMV gives each of 4 warps x up to 8 CTAs a k slice of whole groups or an even part of one. Where that leaves few
         # CTAs it is slow (11008 x 4096: 39 us against 15 us; 5632 x 4096: 27 to 47 us against 11 us), and on long k, where the
-        # slices are long, it loses from the first token on (14336 x 4096, groups of 128: 19 to 27 us against 18 us; with groups of
-        # 32 its 25 to 32 us stand against 33 us).
+        # slices are long, it loses from the first token on (14336 x 4096, groups of 128: 19 to 27 us against 18 us).
         steps, per_group = k // 16, g // 16
         split = max((r for r in range(1, 9) if steps % (4 * r) == 0 and steps // (4 * r) % 2 == 0
                      and (steps // (4 * r) % per_group == 0 or per_group % (steps // (4 * r)) == 0)), default=0)
-        if k >= 2048 and (split == 0 or n // 128 * split < 64 or (k > 8192 and g >= 64)):
+        if k >= 2048 and (split == 0 or n // 128 * split < 64 or k > 8192):
             return most, 0
         return most, AWQ_GEMV_MAX_M
 

@@ -31,10 +31,10 @@ def check(y, x, w):
     assert (np.abs(y.double().cpu().numpy() - ref) <= 2.0**-17 * mass + rounding).all()
 
 
-# one unit and one tile; units beyond every ring (k = 5632); groups of 32, 64, 128 and more; tiles shared by two, three and many
+# one unit and one tile; units beyond every ring (k = 5632); groups of 64, 128 and more; tiles shared by two, three and many
 # CTAs; whole tiles (148 of them); one token, the edges of the tile widths and two tiles of tokens
 @pytest.mark.parametrize("gptq", [False, True])
-@pytest.mark.parametrize("k,n,g", [(128, 128, 32), (5632, 256, 32), (5632, 128, 64), (2048, 1152, 128), (1024, 18944, 256)])
+@pytest.mark.parametrize("k,n,g", [(128, 128, 64), (5632, 256, 64), (5632, 128, 512), (2048, 1152, 128), (1024, 18944, 256)])
 @pytest.mark.parametrize("m", [1, 16, 17, 33, 97, 128, 129, 256])
 def test_grouped_kernel_matches_64_bit_sums(cuda, m, k, n, g, gptq):
     lin, w = layer(k, n, g, gptq, seed=k + n + m)

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(256, 3) q6k_gemv_kernel(const Q6kGemvParams p)
 // pitch of 420 words puts the 8 rows x 4 words of a fragment read on distinct banks. 6-bit values become f16 1024 + v, minus 1056
 // exactly, so no sums of x are needed; a step's accumulators are multiplied by d * scale in f32.
 //
-// What bounds it: instruction issue, about 3.6 per weight (9.1 in the kernel above, which stages x in every CTA, loads every
+// What bounds it: instruction issue, 5.2 per weight (9.1 in the kernel above, which stages x in every CTA, loads every
 // word of a misaligned super-block as halfwords from global memory and folds sums of x).
 constexpr int Q6W_ROWS = 16, Q6W_SB = 8, Q6W_ENGINES = 2, Q6W_WARPS = 8;
 constexpr int Q6W_ROW_BYTES = Q6W_SB * 210, Q6W_STAGE_BYTES = Q6W_ROWS * Q6W_ROW_BYTES;

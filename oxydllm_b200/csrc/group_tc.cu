@@ -21,9 +21,11 @@
 //                 ascending k (no CTA waits for another, the result does not depend on the order of arrival).
 // Every wait is bounded and reports through the workspace flag word.
 //
-// What bounds it at up to 32 tokens: the unpack warps' latency. Time stamps show the four teams always at work (about 1250
-// clocks a stage each, 320 a stage together) while the issuing warps and the fold wait for them; issue slots are 47 % and shared
-// memory 36 % busy, DRAM 22 % (4096 x 28672, 12 tokens). Beside that about 6 us a launch go into filling the pipeline and putting
+// What bounds it at up to 32 tokens: the unpack, as far as time stamps show (its four teams always at work, about 1250 clocks a
+// stage each, 320 a stage together, and the others waiting for them), and behind it most likely shared memory: a stage moves 4 KB
+// of packed words in and out and 16 KB of operand in and out, 320 clocks at 128 B, of which ncu's L1 figure (36 %) leaves out the
+// MMA's reads; sixteen unpack warps instead of eight were 2 to 5 % slower. Issue slots are 47 %, DRAM 22 % busy (4096 x 28672).
+// Beside that about 6 us a launch go into filling the pipeline and putting
 // shared tiles together. Measured in a graph, us at 16 / 77 / 128 tokens (the
 // kernel with scaled bf16 weights before it): 4096 x 4096 10 / 16 / 20 (14 / 19 / 22), 4096 x 28672 30 / 49 / 55 (55 / 59 / 61),
 // 14336 x 4096 20 / 27 / 33 (28 / 34 / 38).

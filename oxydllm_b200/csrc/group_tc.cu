@@ -202,12 +202,15 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tail[0];
+    // The kernel ahead may have written anything this one reads, the packed weights included, and its time must not count as this
+    // kernel's waits: only what is above overlaps with it.
+    pdl_wait();
 
     // The single-thread roles run as whole warps with one elected lane at the instruction itself: loop counters, addresses
     // and descriptors stay in uniform registers (with the loop inside the elected branch an MMA took 90 clocks to issue
     // and a stage of this kernel 890).
     if (warp == 0) {
-        // ---- packed words, zero points and scales, a unit at a time: weights are read before the previous kernel has finished
+        // ---- packed words, zero points and scales, a unit at a time ----------------------------------------------------
         const bool leader = elect_one();
         const int unit_folds = GT_UNIT / p.fold_rows, zgroups = GPTQ && p.sym ? 0 : unit_folds;
         const uint32_t bytes = (uint32_t)(GT_UNIT * GT_ROW_BYTES + zgroups * GT_ZERO_BYTES);
@@ -251,7 +254,6 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         int tb = first_tile % p.token_blocks, k0 = first_unit * GT_UNIT, x = 0;
         uint32_t ph = 0;
         bool ok = true;
-        pdl_wait();
         for (int it = 0; it < nstages && ok; it++) {
             if (it >= X) ok = gt_wait(xempty + 8 * x, ph ^ 1u, p.flag, 5);
             if (ok && leader) {
@@ -411,7 +413,6 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         }
     } else {
         // ---- fold and store: lane = out feature inside the warp's quarter of the accumulator rows ----------------
-        pdl_wait(); // y and the scratch area may still be in use by the kernel before this one
         const int fw = warp - GT_FOLD_WARP0, quad = warp & 3, half = fw >> 2;
         const int feature = quad * 32 + lane, mh = p.mpad / 2, col0 = half * mh;
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)col0;

@@ -632,15 +632,19 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
     while (p.acc_cols < p.mpad) p.acc_cols *= 2;
     const size_t smem = (size_t)p.slots * GT_A_BYTES + (size_t)p.x_slots * p.x_bytes + (size_t)p.raw_slots * GT_RAW_BYTES + fixed;
 
-    // Equal shares of the (tile, unit) list. Sharing a tile costs its last CTA time that grows with the number of parts and their
-    // size; in units (about 0.34 us at 16 tokens) 7.5 + 0.75 x parts x (1 + tokens / 32) follows what was measured: whole tiles against
-    // shares on all SMs 9.6 / 10 us at 2048 x 1024 and 9.7 / 12 at 2048 x 3072 (8 tokens), 12 / 19 at 2048 x 3072 (48 tokens), 23 / 25 at
-    // 4096 x 14336 (64 tokens); 16 parts of a 4096 x 1024 tile 15 us. The parts must fit the scratch area.
+    // Equal shares of the (tile, unit) list. A unit takes about 0.46 us where it is folded once and 0.67 us where twice (groups of
+    // 64), up to 32 tokens; sharing a tile costs its last CTA time that grows with the number of parts and their size. In quarters of
+    // the shorter unit that is 10 + (4 + tokens / 10) a part, above 64 tokens (more registers at work) 3 + 7 a part, as long as no share
+    // crosses a tile border, and 30 + 3 (1 + tokens / 32) a part where shares do. Measured, us, whole tiles / 2 / 4 / 8 parts: 2048 x
+    // 1024 at 16 tokens 10.9 / 9.8 / 9.4 / 11.5, groups of 64 13.2 / 10.7 / 9.8 / 11.8, at 77 tokens 17.1 / 14.1 / 13.7 / 16.6; 1024 x
+    // 1024 at 16 tokens 7.1 / 7.8 / 8.5; 4096 x 512 18.1 / 13.3 / 11.2 / 12.1; shares across borders: 2048 x 4096 at 16 tokens 10.0
+    // with 128 CTAs, 14.0 with 148. The parts must fit the scratch area.
     const long long total = (long long)p.tiles * p.units_per_tile;
     const size_t part_bytes = (size_t)p.mpad * GT_ROWS * sizeof(float), ticket_bytes = group_tc_ticket_bytes(p.tiles);
     const long long fit = scratch && scratch_bytes > ticket_bytes ? (long long)((scratch_bytes - ticket_bytes) / part_bytes) - p.tiles : 0;
     long long ctas = p.tiles < sm_count() ? p.tiles : sm_count();
-    int cost4 = 4 * ceil_div(p.tiles, (int)ctas) * p.units_per_tile; // quarter units
+    const int unit = p.fold_rows == GT_UNIT ? 4 : 6;
+    int best = unit * ceil_div(p.tiles, (int)ctas) * p.units_per_tile;
     p.split = 0;
     for (int c = 2; c <= 16; c++) {
         long long cand = (long long)p.tiles * c;
@@ -649,10 +653,10 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
         if (cand > fit) cand = fit;
         if (cand < p.tiles && cand < sm_count()) break; // shares of more than a tile only with every SM at work
         const int parts = ceil_div((int)cand, p.tiles) + (cand % p.tiles ? 1 : 0);
-        int share = 30 + 3 * parts * (32 + p.mpad) / 32;
-        if (p.mpad > 64) share = share * 7 / 10; // the units take longer too (3072 x 1024 at 100 tokens: 22 us on whole tiles, 17 shared)
-        const int cost = 4 * ceil_div((int)total, (int)cand) + share;
-        if (cost < cost4) { cost4 = cost; ctas = cand; p.split = 1; }
+        int share = p.mpad > 64 ? 3 + 7 * parts : (unit == 4 ? 10 : 16) + parts * (40 + p.mpad) / 10;
+        if (cand % p.tiles) share = (30 + 3 * parts * (32 + p.mpad) / 32) * (p.mpad > 64 ? 7 : 10) / 10;
+        const int cost = unit * ceil_div((int)total, (int)cand) + share;
+        if (cost < best) { best = cost; ctas = cand; p.split = 1; }
         if (cand == sm_count()) break;
     }
     static std::atomic<unsigned long long> calls{0}; // marks differ between calls, in no order that a stale value would have by chance

@@ -53,6 +53,30 @@ def test_grouped_kernel_matches_64_bit_sums(cuda, m, k, n, g, gptq):
     gemm.check(gemm.workspace(n, k, "cuda"))
 
 
+# whole tiles; two to six shares a tile, all inside it; 148 shares of 149 tiles, nearly all of which cross a tile border
+@pytest.mark.parametrize("gptq", [False, True])
+@pytest.mark.parametrize("k,n,g", [(1024, 1024, 128), (2048, 1024, 128), (2048, 1024, 64), (4096, 512, 64), (2048, 19072, 128)])
+@pytest.mark.parametrize("m", [6, 77])
+def test_shared_tiles_match_64_bit_sums(cuda, m, k, n, g, gptq):
+    lin, w = layer(k, n, g, gptq, seed=k + n + m)
+    if m > lin._grouped_max_m:
+        pytest.skip("groups of 64 leave the kernel at 32 tokens")
+    bias = torch.from_numpy(np.random.default_rng(m).standard_normal(n).astype(np.float32)).cuda()
+    x = synth.activations(m, k, seed=m)
+    xd = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
+    y, yb = (torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2))
+    gemm.packed4_matmul(lin, xd, y)
+    check(y, x, w)
+    gemm.packed4_matmul(L.PackedQuantLinear(lin_raw(lin), bias), xd, yb)
+    assert torch.equal(yb, y + bias)  # added to the finished sum, one f32 rounding
+    gemm.check(gemm.workspace(n, k, "cuda"))
+
+
+def lin_raw(lin):
+    new = (lambda *a: L.QuantWeight.new_gptq(4, False, *a)) if lin.pack_dim == "in" else (lambda *a: L.QuantWeight.new_awq(4, *a))
+    return new(lin.qweight, lin.qzeros, lin.scales)
+
+
 def test_calls_on_two_streams_and_a_replayed_graph_do_not_meet(cuda):
     lin, w = layer(4096, 1024, 128, False, seed=5)
     xs = [torch.from_numpy(np.ascontiguousarray(synth.activations(48, 4096, seed=s))).to(torch.bfloat16).cuda() for s in range(2)]

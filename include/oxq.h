@@ -84,6 +84,10 @@ int oxq_awq_gemv(const void *x, int x_dtype, const uint32_t *qweight, const uint
                  int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                  int group_size, void *stream);
 
+/* Largest m for which oxq_awq_gemv is the better kernel on a shape that oxq_packed4_max_m is not 0 for (0 .. 8, by how far
+ * k can be split; elsewhere oxq_awq_gemv serves up to 32 tokens). No counterpart in the reference. */
+int oxq_awq_gemv_max_m(int k, int n, int group_size);
+
 /* oxq_awq_gemv streams weight boxes into shared memory with the TMA unit and waits for each with a
  * bounded wait. Synchronises `stream`; returns OXQ_ERR_DEVICE_FLAG (once) if such a wait ran out on
  * the current device in any oxq_awq_gemv call since the last check. No counterpart in the reference. */
@@ -93,10 +97,10 @@ int oxq_awq_gemv_check(void *stream);
  * up_proj, ffn.rs:235-254): y[m, inter] = act(x . W_gate^T) * (x . W_up^T), act = 1 SiLU, 2 GeLU-tanh
  * (FeedForward::forward, ffn.rs:385-470; gated_silu_fused / gated_gelu_tanh_fused, metal_ops.rs:1243-1277).
  * x, y bf16. qweight u32 [k, 2*inter/8], qzeros u32 [k/g, 2*inter/8], scales [k/g, 2*inter].
- * m <= 8 runs the GEMV and a small activation kernel; 9 .. 256 tokens run the kernel that unpacks inside
- * the tensor-core loop (on the shapes oxq_awq_gemm takes it for; the GEMV up to 32 tokens elsewhere) and the
- * same activation kernel; larger m dequantizes the weight with gate row j and up row j side by side and applies the activation in the tensor-core GEMM's epilogue (no
- * [m, 2*inter] round trip). Workspace as for oxq_awq_gemm with n = 2*inter; oxq_gemm_check applies. */
+ * m <= oxq_awq_gemv_max_m(k, 2*inter, group_size) runs the GEMV and a small activation kernel; larger m up to
+ * 256 runs the kernel that unpacks inside the tensor-core loop (on the shapes oxq_awq_gemm takes it for; the GEMV
+ * up to 32 tokens elsewhere) and the same activation kernel; above, the weight is dequantized with gate row j and
+ * up row j side by side and the activation applied in the tensor-core GEMM's epilogue (no [m, 2*inter] round trip). Workspace as for oxq_awq_gemm with n = 2*inter; oxq_gemm_check applies. */
 int oxq_awq_ffn_gate_up(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
                         int scales_dtype, int activation, void *y, int m, int k, int inter, int group_size,
                         void *workspace, size_t workspace_bytes, void *stream);

@@ -21,6 +21,7 @@ SIGNATURES = {
     "oxq_version": [],
     "oxq_awq_dequant": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
     "oxq_awq_gemv": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
+    "oxq_awq_gemv_max_m": [_i, _i, _i],
     "oxq_decode_max_m": [],
     "oxq_decode_workspace_bytes": [_i, _i, _i],
     "oxq_awq_decode_matmul": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp],

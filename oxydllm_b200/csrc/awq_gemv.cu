@@ -993,9 +993,42 @@ static int launch_awq_gemv(const AwqGemvParams &p, int ksplit, cudaStream_t stre
     return OXQ_OK;
 }
 
+// A cluster of `cand` CTAs of GK_KW warps splits k into even slices, each a whole number of groups or an even part of one.
+static bool gemv_even_slices(int total_steps, int gsteps, int cand)
+{
+    if (total_steps % (GK_KW * cand) != 0) return false;
+    const int sl = total_steps / (GK_KW * cand);
+    return sl % gsteps == 0 || gsteps % sl == 0;
+}
+
 } // namespace oxq
 
 using namespace oxq;
+
+// Largest batch at which this kernel is the better one on shapes that group_tc.cu serves. What counts is how far k can be split: us
+// here / there at 1, 4, 8 tokens, groups of 128: 4096 x 4096 (8 slices of 512 rows) 6.7 / 11.5, 7.0 / 11.5, 8.4 / 11.6; 8192 x 4096
+// (8 of 1024) 11.1 / 15.1, 12.2 / 15.1, 14.2 / 15.3; 12288 x 4096 (8 of 1536) 14.9 / 19.1, 17.0 / 19.1, 21.9 / 19.2; 14336 x 4096 (7 of
+// 2048) 19.4 / 20.9, 22.1 / 21.1, 26.8 / 21.2, x 1024 11.8 / 16.1, 14.9 / 16.2, 19.1 / 16.5; 28672 x 8192 (8 of 3584) 33.7 / 55.3,
+// 39.9 / 55.5, 72.8 / 55.8, x 1024 18.8 / 21.0, 29.3 / 21.1, 32.0 / 21.4; 13824 x 5120 (3 of 4608) 29.4 / 24.4 at one token, 5632 x 2048
+// (not split) 27.3 / 12.2. Very wide layers run in waves from few tokens on (14336 x 28672 66.9 / 92.5 at 2, 120 / 92.7 at 4). Short k
+// needs no split (1024 x 4096 5.3 / 7.6 at 8 tokens).
+OXQ_EXPORT int oxq_awq_gemv_max_m(int k, int n, int group_size)
+{
+    if (k < 2048) return 8;
+    if (group_size < 16) return 0;
+    int split = 8;
+    while (split > 0 && !(gemv_even_slices(k / 16, group_size / 16, split) && k / (16 * GK_KW * split) % 2 == 0)) split--;
+    if (split <= 2) return 0;
+    const int rows = k / split;
+    if (rows <= 1024) return 8;
+    if (rows > 4096 || (rows > 2048 && split < 6)) return 0;
+    if (n > 16384) return 2;
+    if (rows > 2048) return n >= 4096 ? 4 : 2;
+    // up to 32 tiles, four whole shares of each keep nearly every SM of the other kernel at work; it folds groups of 64 twice as often
+    // (14336 x 4096, groups of 64: 21.8 / 25.9 at 4 tokens, 25.6 / 25.9 at 8)
+    if (rows > 1536 && n > 2048 && n <= 4096) return group_size > 64 ? 2 : 8;
+    return rows <= 1536 && split == 8 ? 6 : 4;
+}
 
 OXQ_EXPORT int oxq_awq_gemv(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros,
                             const void *scales, int scales_dtype, const void *bias, int bias_dtype, void *y,
@@ -1056,14 +1089,20 @@ OXQ_EXPORT int oxq_awq_gemv(const void *x, int x_dtype, const uint32_t *qweight,
         const int m_cta = m < 8 * mtc ? m : 8 * mtc;
         const int gsteps = group_size / 16;
         const int n_tiles = ceil_div(p.packed_out, 8 * fv) * split;
+        // The smallest cluster that fills the chip, among the powers of two if one does, else among all sizes that leave even slices
+        // (14336 x 4096: 24.6 us at 4, 18.9 at 7; 28672 x 8192 at 4 tokens: 39.9 us at 8, 52.1 at 7); the largest if none does.
         int r = 0;
-        for (int cand : {8, 7, 6, 5, 4, 3, 2, 1}) { // any cluster size that leaves even slices (14336 x 4096: 24.6 us at 4, 18.9 at 7)
-            if (total_steps % (GK_KW * cand) != 0) continue;
-            const int sl = total_steps / (GK_KW * cand);
-            if (!(sl % gsteps == 0 || gsteps % sl == 0) || sl % depth != 0) continue;
-            if ((size_t)m_cta * (GK_KW * sl * 16 + 16) * 2 > 160 * 1024) continue;
-            if (r_force ? cand == r_force : (r == 0 || (m > 8 ? cand >= 2 : n_tiles * GK_KW * cand >= 1700))) r = cand;
-        }
+        bool fills = false;
+        for (int pass = 0; pass < 2 && !fills; pass++)
+            for (int cand = 8, largest = r = 0; cand >= 1; cand--) {
+                if (pass == 0 && (cand & (cand - 1)) != 0) continue;
+                if (!gemv_even_slices(total_steps, gsteps, cand) || total_steps / (GK_KW * cand) % depth != 0) continue;
+                if ((size_t)m_cta * (total_steps / cand * 16 + 16) * 2 > 160 * 1024) continue;
+                const bool enough = m > 8 ? cand >= 2 : n_tiles * GK_KW * cand >= 1700;
+                if (r_force ? cand == r_force : (largest == 0 || enough)) r = cand;
+                if (largest == 0) largest = cand;
+                fills = fills || enough || r_force;
+            }
         if (ok && r != 0) {
             p.steps_per_cta = total_steps / (GK_KW * r);
             p.token_split = split;

@@ -455,6 +455,7 @@ static void *g_noalloc_scratch_addr[64] = {};
 extern "C" int oxq_awq_gemv(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
                             int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                             int group_size, void *stream);
+extern "C" int oxq_awq_gemv_max_m(int k, int n, int group_size);
 
 OXQ_EXPORT int oxq_awq_ffn_gate_up(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros,
                                    const void *scales, int scales_dtype, int activation, void *y, int m, int k, int inter,
@@ -485,7 +486,7 @@ OXQ_EXPORT int oxq_awq_ffn_gate_up(const void *x, int x_dtype, const uint32_t *q
         OXQ_CUDA(cudaLaunchKernelEx(&cfg, gated_act_rows_kernel, (const __nv_bfloat16 *)c.slab, (__nv_bfloat16 *)y, m, inter, activation));
         return OXQ_OK;
     };
-    if (m > 8 && gu_bytes <= c.slab_bytes && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales)) {
+    if (m > oxq_awq_gemv_max_m(k, n, group_size) && gu_bytes <= c.slab_bytes && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales)) {
         // The kernel that unpacks inside the tensor-core loop writes the row block (no dense copy of the weight); what the slab
         // holds behind the block is its scratch. 2 x 14336 out features, k = 4096, at 8 / 16 tokens: the GEMV 33 / 48 us, this
         // kernel 30 us.

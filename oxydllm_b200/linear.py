@@ -25,13 +25,12 @@ PACKED_SIMT_GEMV_MAX_M = 8
 # FP8 layers whose shape the fused unpack + tcgen05 kernel serves leave the GEMV at this batch: 24 us for up to 32 tokens on a
 # 14336 x 4096 layer against 25 / 45 us for the GEMV at 16 / 32.
 AWQ_FUSED_MIN_M = 17
-# AWQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu) leave the GEMV above this batch: us at
-# 8 / 16 tokens, GEMV against kernel: 4096 x 4096 8.4 / 23.7 against 10, 4096 x 28672 33 / 48 against 28, whatever the batch up to 32.
-AWQ_GEMV_MAX_M = 8
-# GPTQ 4-bit layers of such shapes: 4096 x 14336 takes 25 / 28 / 48 us at 1 / 2 / 8 tokens in the GEMV, 18 us in the kernel;
-# the GEMV is the faster one for a single token on layers of up to GPTQ_GEMV_MAX_WEIGHTS weights (2048 x 3072: 7.3 us against 8.1).
-GPTQ_FUSED_MIN_M = 2
-GPTQ_GEMV_MAX_WEIGHTS = 8 << 20
+# GPTQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu): the GEMV does not split k, so it is the
+# faster one on short k only, us at 1 / 2 tokens against the kernel: groups of 128, 1024 x 4096 4.8 / 5.2 against 7.7, 2048 x 6144
+# 7.7 / 8.6 against 10.0, 3072 x 4096 10.3 / 11.7 against 10.9, 2048 x 14336 14.2 / 16.2 against 12.4; groups of 64, 1024 x 4096
+# 6.6 / 7.4 against 8.4, 2048 x 4096 11.6 / 13.5 against 10.4.
+GPTQ_FUSED_MIN_M = 3
+GPTQ_GEMV_MAX_N = 6144
 
 
 def _p(t: Optional[torch.Tensor]) -> int:
@@ -269,7 +268,7 @@ class PackedQuantLinear:
     def gemv_max_m(self) -> int:
         """Largest batch the decode kernels take before the tensor-core GEMM is the better tool: 32 for the
         4-bit AWQ tensor-core GEMV, 8 (one chunk of the reference's batched GEMV) for GPTQ and 8-bit; on shapes the
-        grouped unpack + tcgen05 kernel serves, 8 for AWQ (0 where the GEMV cannot split k well) and 1 or 0 for GPTQ."""
+        grouped unpack + tcgen05 kernel serves, 0 to 8 for AWQ (``oxq_awq_gemv_max_m``) and 0 to 2 for GPTQ."""
         return self._gemv_max_m
 
     def _pick_batches(self):
@@ -282,17 +281,11 @@ class PackedQuantLinear:
         if not grouped:
             return 0, GEMV_MAX_M if awq and self.bits == 4 else PACKED_SIMT_GEMV_MAX_M
         most = int(_lib.load().oxq_packed4_max_m(k, n, g))
-        if not awq:
-            return most, GPTQ_FUSED_MIN_M - 1 if k * n <= GPTQ_GEMV_MAX_WEIGHTS else 0
-        # The GEMV gives each of 4 warps x up to 8 CTAs a k slice of whole groups or an even part of one. Where that leaves few
-        # CTAs it is slow (11008 x 4096: 39 us against 15 us; 5632 x 4096: 27 to 47 us against 11 us), and on long k, where the
-        # slices are long, it loses from the first token on (14336 x 4096, groups of 128: 19 to 27 us against 18 us).
-        steps, per_group = k // 16, g // 16
-        split = max((r for r in range(1, 9) if steps % (4 * r) == 0 and steps // (4 * r) % 2 == 0
-                     and (steps // (4 * r) % per_group == 0 or per_group % (steps // (4 * r)) == 0)), default=0)
-        if k >= 2048 and (split == 0 or n // 128 * split < 64 or k > 8192):
+        if awq:
+            return most, int(_lib.load().oxq_awq_gemv_max_m(k, n, g))
+        if n > GPTQ_GEMV_MAX_N or k > 3072 or (g == 64 and k > 1024):
             return most, 0
-        return most, AWQ_GEMV_MAX_M
+        return most, GPTQ_FUSED_MIN_M - 1 if k <= 2048 else 1
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""

@@ -227,16 +227,24 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
 template <int MT, int D> static int launch_mx4(Mx4GemvParams p, int ks, cudaStream_t st, int batch = 1)
 {
     p.tiles = ceil_div(p.n, 16 * p.row_tiles);
-    // Batched: as many CTAs per pair as fit the SMs five to one (of 192 threads) in one wave, each with an equal share of the row
-    // groups, so that a pair's x is staged about 90 times and not 360 (8 pairs, 5760 x 2880: 37 -> 27 us).
-    int ctas = p.tiles;
-    if (batch > 1 && ks == 1) {
-        const int want = ceil_div(5 * sm_count(), batch);
-        ctas = ceil_div(p.tiles, ceil_div(p.tiles, want < p.tiles ? want : p.tiles));
-    }
     const int nw = p.row_tiles * p.k_warps;
     const int m_cta = p.m < 8 * MT ? p.m : 8 * MT;
     const size_t smem = (size_t)m_cta * (p.k / ks + 8) * 2 + (size_t)nw * MT * 4 * 32 * 4 + 16;
+    // Batched: a CTA takes `groups` row groups of a pair with the x it has staged once. A launch is as many rounds of resident CTAs
+    // (at 64 registers a thread 1024 threads fit an SM) as it needs, each of `groups` steps plus the staging: a quarter of a step,
+    // three quarters where the activation is computed with it. The cheapest of 1 .. 8 is taken: with shares that just miss one round
+    // (32 pairs, 5760 x 2880: 768 CTAs where 740 fit) the expert layer took 235 us for 8 tokens.
+    int ctas = p.tiles;
+    if (batch > 1 && ks == 1) {
+        const int by_smem = (int)(228 * 1024 / (smem + 1024)), by_threads = 1024 / (nw * 32);
+        const int resident = sm_count() * (by_smem < by_threads ? by_smem : by_threads);
+        long long least = -1;
+        for (int groups = 1; groups <= 8; groups++) {
+            const int cand = ceil_div(p.tiles, groups);
+            const long long cost = (long long)ceil_div(cand * batch, resident) * (8 * groups + (p.gu ? 6 : 2));
+            if (least < 0 || cost < least) { least = cost; ctas = cand; }
+        }
+    }
     auto kern = mxfp4_gemv_kernel<MT, D>;
     static size_t configured[64] = {};
     int device = 0;

@@ -226,3 +226,19 @@ def test_dispatch_plan_gather_and_ids_match_torch(cuda, tokens, experts, k):
     ids = moe.expand_ids(grp, n_local, lo, int(grp.sum()))
     ref_ids = torch.repeat_interleave(torch.arange(lo, lo + n_local, device="cuda", dtype=torch.int32).repeat(world), grp.long())
     assert torch.equal(ids, ref_ids)
+
+
+@pytest.mark.parametrize("hidden,inter", [(2048, 1024), (2880, 416), (160, 2880)])
+def test_decode_rows_do_not_depend_on_the_batch(cuda, hidden, inter):
+    """How many row groups a CTA takes follows from the number of pairs: 1 to 8, the last CTA fewer; the sums stay the same."""
+    d = synth.gptoss_moe(8, hidden, inter, 12, seed=hidden)
+    layer = build(d)
+    x, logits = dev(d["x"], torch.bfloat16), dev(d["logits"])
+    alone = torch.cat([layer.forward_with_logits(x[t:t + 1], logits[t:t + 1]) for t in range(12)])
+    for tokens in (2, 3, 5, 8, 12):
+        assert torch.equal(layer.forward_with_logits(x[:tokens], logits[:tokens]), alone[:tokens])
+    idx, w = oracle.moe_route(d["logits"], 4, True)
+    ref = oracle.gptoss_moe(d["x"], idx, w, d["gu_blocks"], d["gu_scales"], d["gu_bias"], d["dn_blocks"], d["dn_scales"],
+                            d["dn_bias"], hidden, inter, 7.0)
+    row_inf = np.abs(ref).max(axis=1, keepdims=True)
+    assert (np.abs(alone.float().cpu().numpy() - ref) <= 2e-2 * row_inf + 1e-5).all()

@@ -10,6 +10,7 @@ CPU path.
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import cached_property
 from typing import Optional
 
 import torch
@@ -255,7 +256,6 @@ class PackedQuantLinear:
         self.bias = None if bias is None else bias.contiguous()
         self.dtype = dtype
         self._resident = all(t is None or t.is_cuda for t in (self.qweight, self.qzeros, self.scales, self.bias))
-        self._grouped_max_m, self._gemv_max_m = self._pick_batches()
         self._scratch_bytes: dict = {}  # by batch
         # constant arguments of the calls, converted once
         b = self.bias
@@ -269,10 +269,16 @@ class PackedQuantLinear:
         """Largest batch the decode kernels take before the tensor-core GEMM is the better tool: 32 for the
         4-bit AWQ tensor-core GEMV, 8 (one chunk of the reference's batched GEMV) for GPTQ and 8-bit; on shapes the
         grouped unpack + tcgen05 kernel serves, 0 to 8 for AWQ (``oxq_awq_gemv_max_m``) and 0 to 2 for GPTQ."""
-        return self._gemv_max_m
+        return self._batches[1]
 
-    def _pick_batches(self):
-        """Largest batches of the grouped unpack + tcgen05 kernel (0: not this layer) and of the GEMV."""
+    @property
+    def _grouped_max_m(self) -> int:
+        return self._batches[0]
+
+    @cached_property
+    def _batches(self):
+        """Largest batches of the grouped unpack + tcgen05 kernel (0: not this layer) and of the GEMV; asked of the library at the
+        first call, so that a layer can be built on a host that cannot load it."""
         k, n, g = self.in_features, self.out_features, self.group_size
         awq = self.pack_dim == "out"
         grouped = (self.bits == 4 and n % 128 == 0 and k % 128 == 0 and g >= 64 and g & (g - 1) == 0
@@ -301,9 +307,10 @@ class PackedQuantLinear:
                                  f"on {x2.device}")
             y = out
         if m:
-            if m <= self._gemv_max_m:
+            grouped_max_m, gemv_max_m = self._batches
+            if m <= gemv_max_m:
                 self._gemv(x2, y, m)
-            elif m <= self._grouped_max_m and x2.data_ptr() % 16 == 0:
+            elif m <= grouped_max_m and x2.data_ptr() % 16 == 0:
                 gemm.packed4_matmul(self, x2, y)
             elif self.pack_dim == "out" and self.bits == 4:
                 gemm.awq_matmul(self, x2, y)

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from oxydllm_b200 import _lib
 from oxydllm_b200 import formats as F
 from oxydllm_b200 import linear as L
 
@@ -55,6 +56,18 @@ def test_batches_of_the_4_bit_gemvs(gptq, k, n, g, gemv):
     new = (lambda *a: L.QuantWeight.new_gptq(4, False, *a)) if gptq else (lambda *a: L.QuantWeight.new_awq(4, *a))
     lin = L.PackedQuantLinear(new(words, torch.zeros((k // g, n // 8), dtype=torch.int32), torch.zeros((k // g, n), dtype=torch.float16)))
     assert lin.gemv_max_m() == gemv
+
+
+def test_layers_are_built_without_the_library(monkeypatch):
+    def missing(*_):
+        raise ImportError("liboxq.so cannot be built here")
+    monkeypatch.setattr(_lib, "load", missing)
+    monkeypatch.setattr(_lib, "entry", missing)
+    lin = L.PackedQuantLinear(_awq(k=256, n=128, g=128))
+    half = L.QuantWeight.new_awq(4, lin.qweight, lin.qzeros, lin.scales.half())
+    L.GatedFfnProjection(L.PackedQuantLinear(half))
+    with pytest.raises(ValueError, match="CUDA tensors only"):
+        L.PackedQuantLinear(half).forward(torch.zeros((1, 256), dtype=torch.bfloat16))
 
 
 def test_any_linear_selects_fp8_variant_for_fp8_weights():

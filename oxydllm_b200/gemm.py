@@ -93,7 +93,7 @@ def awq_matmul(lin, x2, y):
               lin.group_size, _p(ws), ws.numel(), _st())
 
 
-def packed4_matmul(lin, x2, y):
+def packed4_matmul(lin, x2, y, tensors=None):
     """``y = x2 . deq(W) (+ bias)`` for the 4-bit layouts by the grouped unpack + tcgen05 kernel (``oxq_packed4_matmul``). The
     scratch is this call's own, so calls on several streams do not meet; the workspace lends its flag word."""
     m, n = x2.shape[0], lin.out_features
@@ -104,7 +104,7 @@ def packed4_matmul(lin, x2, y):
     if need is None:
         need = lin._scratch_bytes[m] = int(_lib.load().oxq_packed4_scratch_bytes(m, n))
     scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
-    qw, qz, sc, sc_dt, b, b_dt = lin._const
+    qw, qz, sc, sc_dt, b, b_dt = tensors or lin._tensors()
     _lib.call("oxq_packed4_matmul", x2.data_ptr(), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, y.data_ptr(), _dt(y.dtype), m,
               lin.in_features, n, lin.group_size, int(lin.pack_dim == "in"), int(lin.sym), ws.data_ptr(), scratch.data_ptr(), need,
               _st())
@@ -134,11 +134,11 @@ def gptq_matmul(raw, x2, y, bias=None):
               x2.shape[0], k, n, g, raw.bits, int(sym), _p(ws), ws.numel(), _st())
 
 
-def awq_ffn_gate_up(lin, x2, y, activation: int):
+def awq_ffn_gate_up(lin, x2, y, activation: int, tensors=None):
     """``y[m, inter] = act(x . W_gate^T) * (x . W_up^T)`` on the fused ``[gate | up]`` AWQ linear ``lin``."""
     ws = workspace(lin.out_features, lin.in_features, x2.device)
-    _lib.call("oxq_awq_ffn_gate_up", x2.data_ptr(), _lib.OXQ_BF16, *lin._const[:4], activation, y.data_ptr(), x2.shape[0], lin.in_features, lin.out_features // 2,
-              lin.group_size, _p(ws), ws.numel(), _st())
+    _lib.call("oxq_awq_ffn_gate_up", x2.data_ptr(), _lib.OXQ_BF16, *(tensors or lin._tensors())[:4], activation, y.data_ptr(),
+              x2.shape[0], lin.in_features, lin.out_features // 2, lin.group_size, _p(ws), ws.numel(), _st())
 
 
 def fp8_matmul(lin, s, s_out, s_in, x2, y):

@@ -255,15 +255,30 @@ class PackedQuantLinear:
         self.scales = raw.scales.contiguous()
         self.bias = None if bias is None else bias.contiguous()
         self.dtype = dtype
-        self._resident = all(t is None or t.is_cuda for t in (self.qweight, self.qzeros, self.scales, self.bias))
+        for t in (self.scales, self.bias):
+            if t is not None:
+                _dt(t.dtype)  # raises where the kernels have no such type
         self._scratch_bytes: dict = {}  # by batch
-        # constant arguments of the calls, converted once
-        b = self.bias
-        self._const = (_p(self.qweight), _p(self.qzeros), _p(self.scales), _dt(self.scales.dtype), _p(b),
-                       _dt(b.dtype) if b is not None else 0)
         self._const_shape = (self.in_features, self.out_features, self.group_size)
         if self.pack_dim == "in":
             self._const_shape += (self.bits, int(self.sym))
+
+    def __setattr__(self, name, value):
+        # a packed tensor or bias that a caller puts in later takes the form the kernels read, as in the constructor
+        if value is not None and name in ("qweight", "qzeros"):
+            value = _as_u32_words(value)
+        elif value is not None and name in ("scales", "bias"):
+            value = value.contiguous()
+            self.__dict__.pop("_batches", None)  # they depend on the dtype of the scales
+        super().__setattr__(name, value)
+
+    def _tensors(self):
+        """Pointers and dtypes of the tensors as they are now, in the order of the C entry points: nothing is kept between calls."""
+        qw, qz, sc, b = self.qweight, self.qzeros, self.scales, self.bias
+        if not (qw.is_cuda and sc.is_cuda and (qz is None or qz.is_cuda) and (b is None or b.is_cuda)):
+            _require_cuda(qw, qz, sc, b)
+        return (qw.data_ptr(), 0 if qz is None else qz.data_ptr(), sc.data_ptr(), _dt(sc.dtype),
+                0 if b is None else b.data_ptr(), 0 if b is None else _dt(b.dtype))
 
     def gemv_max_m(self) -> int:
         """Largest batch the decode kernels take before the tensor-core GEMM is the better tool: 32 for the
@@ -296,8 +311,9 @@ class PackedQuantLinear:
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""
         x2, lead, m = _flatten_x(x, self.in_features, "PackedQuantLinear")
-        if not (self._resident and x2.is_cuda):
-            _require_cuda(x2, self.qweight, self.qzeros, self.scales, self.bias)
+        if not x2.is_cuda:
+            _require_cuda(x2)
+        tensors = self._tensors()
         if out is None:
             y = x2.new_empty((m, self.out_features))
         else:
@@ -309,9 +325,9 @@ class PackedQuantLinear:
         if m:
             grouped_max_m, gemv_max_m = self._batches
             if m <= gemv_max_m:
-                self._gemv(x2, y, m)
+                self._gemv(x2, y, m, tensors)
             elif m <= grouped_max_m and x2.data_ptr() % 16 == 0:
-                gemm.packed4_matmul(self, x2, y)
+                gemm.packed4_matmul(self, x2, y, tensors)
             elif self.pack_dim == "out" and self.bits == 4:
                 gemm.awq_matmul(self, x2, y)
             elif self.pack_dim == "out":
@@ -320,10 +336,10 @@ class PackedQuantLinear:
                 gemm.gptq_matmul(self, x2, y, self.bias)
         return y if x2 is x else y.reshape(*lead, self.out_features)
 
-    def _gemv(self, x2, y, m):
+    def _gemv(self, x2, y, m, tensors):
         dt = _dt(x2.dtype)
         name = "oxq_gptq_gemv" if self.pack_dim == "in" else "oxq_awq_gemv" if self.bits == 4 else "oxq_w8a16_gemv"
-        rc = _lib.entry(name)(x2.data_ptr(), dt, *self._const, y.data_ptr(), dt, m, *self._const_shape, _stream())
+        rc = _lib.entry(name)(x2.data_ptr(), dt, *tensors, y.data_ptr(), dt, m, *self._const_shape, _stream())
         if rc:
             _lib.fail(name, rc)
 
@@ -361,13 +377,14 @@ class GatedFfnProjection:
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lin = self.gate_up
         x2, lead, m = _flatten_x(x, lin.in_features, "GatedFfnProjection")
-        if not (lin._resident and x2.is_cuda):
-            _require_cuda(x2, lin.qweight, lin.qzeros, lin.scales)
+        if not x2.is_cuda:
+            _require_cuda(x2)
+        tensors = lin._tensors()
         if x2.dtype != torch.bfloat16:
             raise ValueError("GatedFfnProjection: activations must be bf16")
         y = x2.new_empty((m, self.intermediate))
         if m:
-            gemm.awq_ffn_gate_up(lin, x2, y, ACTIVATIONS[self.activation])
+            gemm.awq_ffn_gate_up(lin, x2, y, ACTIVATIONS[self.activation], tensors)
         return y if x2 is x else y.reshape(*lead, self.intermediate)
 
 

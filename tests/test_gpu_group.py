@@ -77,6 +77,33 @@ def lin_raw(lin):
     return new(lin.qweight, lin.qzeros, lin.scales)
 
 
+@pytest.mark.parametrize("gptq", [False, True])
+def test_a_replaced_tensor_is_the_one_that_counts(cuda, gptq):
+    k, n, g = 256, 512, 128
+    lin, _ = layer(k, n, g, gptq, seed=1)
+    bias = torch.arange(n, dtype=torch.float32, device="cuda") / n
+    want = L.PackedQuantLinear(lin_raw(layer(k, n, g, gptq, seed=2)[0]), bias)
+    xs = [torch.from_numpy(np.ascontiguousarray(synth.activations(m, k, seed=m))).to(torch.bfloat16).cuda() for m in (1, 2, 16, 300)]
+    gated, gated_want = (None if gptq else L.GatedFfnProjection(L.PackedQuantLinear(lin_raw(q))) for q in (lin, want))
+    for x in xs:
+        lin.forward(x)
+    for one in [lin] if gptq else [lin, gated.gate_up]:
+        one.qweight = want.qweight.to(torch.int64)  # as a checkpoint may hold them
+        one.qzeros, one.scales = want.qzeros.t().contiguous().t(), want.scales
+    lin.bias = bias
+    for x in xs:
+        assert torch.equal(lin.forward(x), want.forward(x))
+        if not gptq:
+            assert torch.equal(gated.forward(x), gated_want.forward(x))
+    lin.scales = want.scales.float()  # the same values in a type that the grouped kernel does not take
+    for x in xs:
+        y, ref = lin.forward(x).float(), want.forward(x).float()
+        assert ((y - ref).abs() <= 2e-2 * ref.abs().amax(1, keepdim=True)).all()
+    lin.qweight = want.qweight.cpu()
+    with pytest.raises(ValueError, match="CUDA tensors only"):
+        lin.forward(xs[0])
+
+
 def test_calls_on_two_streams_and_a_replayed_graph_do_not_meet(cuda):
     lin, w = layer(4096, 1024, 128, False, seed=5)
     xs = [torch.from_numpy(np.ascontiguousarray(synth.activations(48, 4096, seed=s))).to(torch.bfloat16).cuda() for s in range(2)]

@@ -58,6 +58,14 @@ def test_batches_of_the_4_bit_gemvs(gptq, k, n, g, gemv):
     assert lin.gemv_max_m() == gemv
 
 
+def test_dtypes_the_kernels_do_not_have_are_refused_at_once():
+    raw = _awq(k=16, n=16, g=16)
+    with pytest.raises(ValueError, match="unsupported dtype"):
+        L.PackedQuantLinear(L.QuantWeight.new_awq(4, raw.qweight, raw.qzeros, raw.scales.double()))
+    with pytest.raises(ValueError, match="unsupported dtype"):
+        L.PackedQuantLinear(raw, torch.zeros(16, dtype=torch.float64))
+
+
 def test_layers_are_built_without_the_library(monkeypatch):
     def missing(*_):
         raise ImportError("liboxq.so cannot be built here")

@@ -336,8 +336,9 @@ class PackedQuantLinear:
                 gemm.gptq_matmul(self, x2, y, self.bias)
         return y if x2 is x else y.reshape(*lead, self.out_features)
 
-    def _gemv(self, x2, y, m, tensors):
+    def _gemv(self, x2, y, m, tensors=None):
         dt = _dt(x2.dtype)
+        tensors = tensors or self._tensors()
         name = "oxq_gptq_gemv" if self.pack_dim == "in" else "oxq_awq_gemv" if self.bits == 4 else "oxq_w8a16_gemv"
         rc = _lib.entry(name)(x2.data_ptr(), dt, *tensors, y.data_ptr(), dt, m, *self._const_shape, _stream())
         if rc:

@@ -292,21 +292,23 @@ class PackedQuantLinear:
 
     @cached_property
     def _batches(self):
-        """Largest batches of the grouped unpack + tcgen05 kernel (0: not this layer) and of the GEMV; asked of the library at the
-        first call, so that a layer can be built on a host that cannot load it."""
+        """Largest batches of the grouped unpack + tcgen05 kernel (0: not this layer), of the GEMV, and of the GEMV in calls that the
+        kernel cannot take for their alignment; asked of the library at the first call, so that a layer can be built on a host
+        that cannot load it."""
         k, n, g = self.in_features, self.out_features, self.group_size
         awq = self.pack_dim == "out"
         grouped = (self.bits == 4 and n % 128 == 0 and k % 128 == 0 and g >= 64 and g & (g - 1) == 0
-                   and self.scales.dtype in (torch.float16, torch.bfloat16)
-                   and all(t is None or t.data_ptr() % 16 == 0 for t in (self.qweight, self.qzeros, self.scales)))
+                   and self.scales.dtype in (torch.float16, torch.bfloat16))
         if not grouped:
-            return 0, GEMV_MAX_M if awq and self.bits == 4 else PACKED_SIMT_GEMV_MAX_M
+            few = GEMV_MAX_M if awq and self.bits == 4 else PACKED_SIMT_GEMV_MAX_M
+            return 0, few, few
         most = int(_lib.load().oxq_packed4_max_m(k, n, g))
-        if awq:
-            return most, int(_lib.load().oxq_awq_gemv_max_m(k, n, g))
+        if awq:  # the AWQ GEMV wants x and qweight on 16 bytes too: above its batches the GEMM on slabs takes any weight
+            return most, int(_lib.load().oxq_awq_gemv_max_m(k, n, g)), 8 if n <= 9472 else 16
+        few = GPTQ_FUSED_MIN_M - 1  # the GPTQ GEMV takes x on any 4 bytes, the GEMM does not
         if n > GPTQ_GEMV_MAX_N or k > 3072 or (g == 64 and k > 1024):
-            return most, 0
-        return most, GPTQ_FUSED_MIN_M - 1 if k <= 2048 else 1
+            return most, 0, few
+        return most, few if k <= 2048 else 1, few
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""
@@ -323,10 +325,11 @@ class PackedQuantLinear:
                                  f"on {x2.device}")
             y = out
         if m:
-            grouped_max_m, gemv_max_m = self._batches
-            if m <= gemv_max_m:
+            grouped_max_m, gemv_max_m, unaligned_max_m = self._batches
+            aligned = (x2.data_ptr() | tensors[0] | tensors[1] | tensors[2]) & 15 == 0
+            if m <= (gemv_max_m if aligned else unaligned_max_m):
                 self._gemv(x2, y, m, tensors)
-            elif m <= grouped_max_m and x2.data_ptr() % 16 == 0:
+            elif aligned and m <= grouped_max_m:
                 gemm.packed4_matmul(self, x2, y, tensors)
             elif self.pack_dim == "out" and self.bits == 4:
                 gemm.awq_matmul(self, x2, y)

@@ -104,6 +104,47 @@ def test_a_replaced_tensor_is_the_one_that_counts(cuda, gptq):
         lin.forward(xs[0])
 
 
+def off16(t, offset):
+    """The same values `offset` elements behind a 16-byte boundary."""
+    room = torch.zeros(t.numel() + offset, dtype=t.dtype, device=t.device)
+    room[offset:] = t.reshape(-1)
+    return room[offset:].view(t.shape)
+
+
+@pytest.mark.parametrize("k,n", [(1024, 512), (4096, 1024), (2048, 8192)])  # GEMV up to two tokens, none
+@pytest.mark.parametrize("m", [1, 2])
+def test_gptq_decode_takes_x_on_any_4_bytes(cuda, m, k, n):
+    """A row of a fused projection's output is such an x. f32 sums of products that are exact but for the scale's rounding."""
+    lin, w = layer(k, n, 128, True, seed=k + m)
+    x = synth.activations(m, k, seed=m)
+    xd = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
+    for offset in (2, 4, 6):
+        check(lin.forward(off16(xd, offset)), x, w)
+    check(lin.forward(xd), x, w)
+
+
+# AWQ words, zero points or scales off 16 bytes: the GEMV to 8 tokens (it wants the words aligned), then the GEMM on slabs, which
+# rounds the weights to bf16 (2^-9 each) before it multiplies
+@pytest.mark.parametrize("gptq", [False, True])
+@pytest.mark.parametrize("m", [2, 9, 16, 17, 32])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_packed_tensors_off_16_bytes(cuda, which, m, gptq):
+    k, n, g = 512, 256, 128
+    lin, w = layer(k, n, g, gptq, seed=m)
+    tensors = [lin.qweight, lin.qzeros, lin.scales]
+    tensors[which] = off16(tensors[which], 2 if which == 2 else 1)
+    new = (lambda *a: L.QuantWeight.new_gptq(4, False, *a)) if gptq else (lambda *a: L.QuantWeight.new_awq(4, *a))
+    odd = L.PackedQuantLinear(new(*tensors))
+    x = synth.activations(m, k, seed=m)
+    xd = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
+    if m == 2 and which == 0 and not gptq:
+        with pytest.raises(Exception, match="16-byte aligned"):  # as ever
+            odd.forward(xd)
+        return
+    ref, mass = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    assert (np.abs(odd.forward(xd).double().cpu().numpy() - ref) <= 2.0**-8 * mass + 2.0**-8 * np.abs(ref)).all()
+
+
 def test_calls_on_two_streams_and_a_replayed_graph_do_not_meet(cuda):
     lin, w = layer(4096, 1024, 128, False, seed=5)
     xs = [torch.from_numpy(np.ascontiguousarray(synth.activations(48, 4096, seed=s))).to(torch.bfloat16).cuda() for s in range(2)]

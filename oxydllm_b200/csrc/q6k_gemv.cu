@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6k
             const int row = min(t * Q6W_ROWS + min(lane, Q6W_ROWS - 1), p.n - 1); // past-the-end rows re-read the last row
             const uint8_t *src = p.blocks + (size_t)row * row_bytes;
             for (int ch = 0; ch < chunks && ok; ch++, it++) {
+                if (it == p.ring) pdl_wait(); // slots come free only after x: that time must not count as this wait
                 if (it >= p.ring) ok = __all_sync(0xFFFFFFFFu, mbar_wait(empty(r), ph ^ 1u, &g_q6k_gemv_flag, 1));
                 if (ok) {
                     if (lane == 0) mbar_arrive_expect_tx(full(r), Q6W_STAGE_BYTES);

@@ -31,7 +31,7 @@ def test_grouped_kernel_reads_nothing_before_the_wait():
     assert not re.search(r"tma_load|bulk_copy|__ldg|__ldcg|ld\.global|p\.(qzeros|scales|bias|y)\b", before)
 
 
-@pytest.mark.parametrize("name", ["packed_group_tc_kernel", "awq_gemv_tma_kernel"])
+@pytest.mark.parametrize("name", ["packed_group_tc_kernel", "awq_gemv_tma_kernel", "q6k_gemv_wide_kernel"])
 def test_bounded_waits_do_not_count_the_time_of_the_kernel_ahead(name):
     body = kernels()[name]
     assert body.index("pdl_wait()") < re.search(r"\b(mbar_wait|gt_wait|mbar_test)\w*\(", body).start()

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(GK_KW * 32, MINB) awq_gemv_group_kernel(const 
         const uint2 *src = reinterpret_cast<const uint2 *>(p.x + (size_t)(m0 + row) * p.k + k_cta);
         uint2 *dst = reinterpret_cast<uint2 *>(xs + (size_t)row * xrow);
         for (int q4 = tid; q4 < (kr >> 2); q4 += KW * 32) {
-            const uint2 raw = __ldg(src + q4);
+            const uint2 raw = ld_produced(src + q4);
             dst[q4] = make_uint2(f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x)),
                                  f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y)));
         }
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(GT_KW * 32, MINB)
                 at[j4] = -1;
                 if (idx < items) {
                     const int row = idx / per, q4 = idx - row * per;
-                    raw[j4] = __ldg(reinterpret_cast<const uint2 *>(p.x + (size_t)(m0 + row) * p.k + k_cta) + q4);
+                    raw[j4] = ld_produced(reinterpret_cast<const uint2 *>(p.x + (size_t)(m0 + row) * p.k + k_cta) + q4);
                     at[j4] = row * xrow + (q4 >> 2) * 16 + (q4 & 3); // x[16 blk + 4 i + cc] -> element 16 blk + 4 cc + i
                 }
             }

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) fp8_gemv_k
         const uint2 *src = reinterpret_cast<const uint2 *>(p.x + (size_t)(m0 + row) * p.k + k_cta);
         uint2 *dst = reinterpret_cast<uint2 *>(xs + (size_t)row * xrow);
         for (int q4 = tid; q4 < (kl >> 2); q4 += blockDim.x) {
-            const uint2 raw = __ldg(src + q4);
+            const uint2 raw = ld_produced(src + q4);
             dst[q4] = make_uint2(f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x)),
                                  f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y)));
         }

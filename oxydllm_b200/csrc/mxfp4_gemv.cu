@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
         const float4 *src = reinterpret_cast<const float4 *>(p.gu + (size_t)blockIdx.z * 2 * p.k + 2 * k_cta);
         uint32_t *dst = reinterpret_cast<uint32_t *>(xs);
         for (int i = tid; i < (kl >> 1); i += blockDim.x) {
-            const float4 v = __ldg(src + i);
+            const float4 v = ld_produced(src + i);
             float h[2];
 #pragma unroll
             for (int e = 0; e < 2; e++) {
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
         const uint2 *src = reinterpret_cast<const uint2 *>(xin + (size_t)(m0 + row) * p.k + k_cta);
         uint2 *dst = reinterpret_cast<uint2 *>(xs + (size_t)row * xrow);
         for (int q4 = tid; q4 < (kl >> 2); q4 += blockDim.x) {
-            const uint2 raw = __ldg(src + q4);
+            const uint2 raw = ld_produced(src + q4);
             dst[q4] = make_uint2(f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x)),
                                  f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y)));
         }

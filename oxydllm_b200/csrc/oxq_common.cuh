@@ -143,6 +143,9 @@ __device__ __forceinline__ float bf16_hi_f32(uint32_t w) { return __uint_as_floa
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What a kernel ahead writes (x, a routing table, another projection's result) is read by an ordinary load behind pdl_wait(). The
+// read-only path of __ldg is for data that nobody writes while the kernel runs, and one that starts early runs while x is written.
+template <typename T> __device__ __forceinline__ T ld_produced(const T *p) { return *p; }
 #endif
 inline void allow_early_start(cudaLaunchAttribute *attrs, unsigned int &count)
 {

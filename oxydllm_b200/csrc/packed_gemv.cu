@@ -41,7 +41,7 @@ __device__ __forceinline__ void stage_x(const PackedGemvParams &p, float *xs, fl
     const int mloc = min(MT, p.m - p.y_row0);
     for (int idx = tid; idx < mloc * (p.k >> 1); idx += PG_WARPS * 32) {
         const int tok = idx / (p.k >> 1), i2 = idx - tok * (p.k >> 1);
-        const uint32_t raw = __ldg(reinterpret_cast<const uint32_t *>(p.x + (size_t)(p.y_row0 + tok) * p.k) + i2);
+        const uint32_t raw = ld_produced(reinterpret_cast<const uint32_t *>(p.x + (size_t)(p.y_row0 + tok) * p.k) + i2);
         *reinterpret_cast<float2 *>(xs + (size_t)tok * p.k + 2 * i2) = make_float2(bf16_lo_f32(raw), bf16_hi_f32(raw));
     }
     __syncthreads();
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(PG_WARPS * 32) gptq4_gemv_mma_kernel(const Pac
     const int blocks_per_row = p.k >> 3;
     for (int idx = tid; idx < mloc * blocks_per_row; idx += PG_WARPS * 32) {
         const int tok = idx / blocks_per_row, b = idx - tok * blocks_per_row;
-        const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(p.x + (size_t)(p.y_row0 + tok) * p.k) + b);
+        const uint4 raw = ld_produced(reinterpret_cast<const uint4 *>(p.x + (size_t)(p.y_row0 + tok) * p.k) + b);
         const float v[8] = {bf16_lo_f32(raw.x), bf16_hi_f32(raw.x), bf16_lo_f32(raw.y), bf16_hi_f32(raw.y),
                             bf16_lo_f32(raw.z), bf16_hi_f32(raw.z), bf16_lo_f32(raw.w), bf16_hi_f32(raw.w)};
         uint4 o;

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256, 3) q6k_gemv_kernel(const Q6kGemvParams p)
         const uint2 *src = reinterpret_cast<const uint2 *>(p.x + (size_t)(m0 + row) * p.k + k_cta);
         uint2 *dst = reinterpret_cast<uint2 *>(xs + (size_t)row * xrow);
         for (int q4 = tid; q4 < (kl >> 2); q4 += blockDim.x) { // kl / 4 is a multiple of 64: whole warps
-            const uint2 raw = __ldg(src + q4);
+            const uint2 raw = ld_produced(src + q4);
             uint2 o;
             o.x = f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x));
             o.y = f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y));
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6k
         const int ct = (engine * Q6W_WARPS + ew) * 32 + lane, per_row = p.k / 4;
         for (int idx = ct; idx < p.m * per_row; idx += Q6W_ENGINES * Q6W_WARPS * 32) {
             const int row = idx / per_row, q4 = idx - row * per_row;
-            const uint2 raw = __ldg(reinterpret_cast<const uint2 *>(p.x + (size_t)row * p.k) + q4);
+            const uint2 raw = ld_produced(reinterpret_cast<const uint2 *>(p.x + (size_t)row * p.k) + q4);
             uint2 o;
             o.x = f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x));
             o.y = f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y));

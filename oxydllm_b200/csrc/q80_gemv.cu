@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(256, 3) q80_gemv_kernel(const Q80GemvParams p)
         // rounded up to whole warps because of the shuffles
         for (int q4 = tid; q4 < (((kl >> 2) + 31) & ~31); q4 += blockDim.x) {
             const bool valid = q4 < (kl >> 2);
-            const uint2 raw = valid ? __ldg(src + q4) : make_uint2(0u, 0u);
+            const uint2 raw = valid ? ld_produced(src + q4) : make_uint2(0u, 0u);
             uint2 o;
             o.x = f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x));
             o.y = f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y));

@@ -35,3 +35,13 @@ def test_grouped_kernel_reads_nothing_before_the_wait():
 def test_bounded_waits_do_not_count_the_time_of_the_kernel_ahead(name):
     body = kernels()[name]
     assert body.index("pdl_wait()") < re.search(r"\b(mbar_wait|gt_wait|mbar_test)\w*\(", body).start()
+
+
+def test_what_a_kernel_ahead_writes_is_not_read_through_the_read_only_path():
+    """``__ldg`` and ``const __restrict__`` may be served before ``pdl_wait``: for weights, scales and zero points only."""
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        if "pdl_wait()" in text:
+            assert not re.search(r"__ldg\([^;]*?\b(src|xin|p\.x|p\.gu|gu|pair_expert)\b", text), path
+    for name, body in kernels().items():
+        assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", body.split("{")[0]), name

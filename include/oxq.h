@@ -229,9 +229,11 @@ int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight, const uint
                  int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                  int group_size, void *workspace, size_t workspace_bytes, void *stream);
 
-/* The kernel that oxq_awq_gemm / oxq_gptq_gemm (4-bit) run up to oxq_packed4_max_m tokens (0: not this shape), with scratch of its own: oxq_packed4_scratch_bytes(m, n) bytes with any contents, 256-byte aligned, one per
- * call in flight. flag_word: the first word of a gemm workspace (oxq_gemm_check reads it). OXQ_ERR_UNSUPPORTED for shapes the
- * kernel does not take. gptq = 0: AWQ layout (qzeros required); 1: GPTQ layout (sym != 0 or qzeros null: zero point 8). */
+/* The kernel that oxq_awq_gemm / oxq_gptq_gemm (4-bit) run up to oxq_packed4_max_m tokens (0: not this shape), with scratch
+ * of its own: oxq_packed4_scratch_bytes(m, n) bytes with any contents, 256-byte aligned, one per call in flight. flag_word: the
+ * first word of a gemm workspace, or of 256 zeroed bytes that stand in for one (oxq_gemm_check reads and clears them).
+ * OXQ_ERR_UNSUPPORTED for shapes the kernel does not take. gptq = 0: AWQ layout (qzeros required); 1: GPTQ layout (sym != 0 or
+ * qzeros null: zero point 8). */
 int oxq_packed4_max_m(int k, int n, int group_size);
 size_t oxq_packed4_scratch_bytes(int m, int n);
 int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,

@@ -152,7 +152,9 @@ OXQ_EXPORT int oxq_gemm_check(const void *workspace, void *stream)
     }
     OXQ_REQUIRE(flag == 0, OXQ_ERR_DEVICE_FLAG,
                 "tensor-core kernel: bounded wait %d ran out (1 = ring slot, 2 = tile data, 3 = accumulator ready, "
-                "4 = accumulator free, 5 = meeting of the fold warps) in a call since the last check", flag);
+                "4 = accumulator free, 5 = meeting of the fold warps; grouped 4-bit kernel: 21 = ring slot, 22 = operand tile, "
+                "23 = packed words, 24 = accumulator ready, 25 = x slot, 26 = x, 27 = operand slot, 28 = slot for scales, "
+                "29 = accumulator free, 30 = scales, 31 = last MMAs) in a call since the last check", flag);
     return OXQ_OK;
 }
 

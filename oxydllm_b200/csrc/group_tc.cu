@@ -58,6 +58,7 @@ constexpr int GT_NUM_BARS = 2 * GT_MAX_RAW + 2 * GT_MAX_SLOTS + 2 * GT_MAX_X + 2
 constexpr int GT_MAX_TOKENS = 128;           // per tile
 constexpr int GROUP_TC_MAX_M = 256, GT_NARROW_TILES = 74;
 constexpr int GT_SMEM_BUDGET = 227 * 1024;
+constexpr int GT_CODE = 20;                  // wait codes 21 .. 31: oxq_gemm_check names them beside the other kernels' 1 .. 5
 // A parity wait tells a phase from the next one only: whoever waits on a barrier has to see every one of its phases. So a slot
 // always meets the same team and the same issuer, and a ring slot the same teams: their counts are multiples of these.
 static_assert(GT_MAX_SLOTS % GT_TEAMS == 0 && GT_TEAMS % (GT_UNIT_STAGES * GT_ISSUERS) == 0 &&
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             const size_t group = (size_t)(k0 >> p.gshift);
             const uint32_t *zsrc = p.qzeros + group * p.packed_out + n0 / 8;
             const uint16_t *ssrc = reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0;
-            if (it >= R) ok = gt_wait(rawempty + 8 * r, ph ^ 1u, p.flag, 1);
+            if (it >= R) ok = gt_wait(rawempty + 8 * r, ph ^ 1u, p.flag, GT_CODE + 1);
             if (ok && leader) {
                 const uint32_t dst = raw_base + (uint32_t)(r * GT_RAW_BYTES), bar = rawfull + 8 * r;
                 mbar_arrive_expect_tx(bar, bytes);
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             __syncwarp();
             if (++r == R) { r = 0; ph ^= 1u; }
             for (int f = 0; f < unit_folds && ok; f++, fold++) { // unit_folds > 1: groups shorter than a unit, one fold each
-                if (fold >= GT_SC) ok = gt_wait(scempty + 8 * c, cph ^ 1u, p.flag, 8);
+                if (fold >= GT_SC) ok = gt_wait(scempty + 8 * c, cph ^ 1u, p.flag, GT_CODE + 8);
                 if (ok && leader) {
                     mbar_arrive_expect_tx(scfull + 8 * c, GT_SC_BYTES);
                     bulk_copy_g2s(sc_base + c * GT_SC_BYTES, ssrc + (size_t)f * p.n, GT_SC_BYTES, scfull + 8 * c);
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         uint32_t ph = 0;
         bool ok = true;
         for (int it = 0; it < nstages && ok; it++) {
-            if (it >= X) ok = gt_wait(xempty + 8 * x, ph ^ 1u, p.flag, 5);
+            if (it >= X) ok = gt_wait(xempty + 8 * x, ph ^ 1u, p.flag, GT_CODE + 5);
             if (ok && leader) {
                 mbar_arrive_expect_tx(xfull + 8 * x, (uint32_t)p.x_bytes);
                 tma_load_2d(x_base + (uint32_t)(x * p.x_bytes), &xmap, xfull + 8 * x, k0, tb * p.mpad);
@@ -270,9 +271,9 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         }
         // The commits of the last stages arrive here asynchronously: the CTA stays until they have.
         for (int left = min(S, nstages), q = nstages - left; left > 0 && ok; left--, q++)
-            ok = gt_wait(empty + 8 * (q % S), (uint32_t)(q / S) & 1u, p.flag, 11);
+            ok = gt_wait(empty + 8 * (q % S), (uint32_t)(q / S) & 1u, p.flag, GT_CODE + 11);
         for (int left = min(X, nstages), q = nstages - left; left > 0 && ok; left--, q++)
-            ok = gt_wait(xempty + 8 * (q % X), (uint32_t)(q / X) & 1u, p.flag, 11);
+            ok = gt_wait(xempty + 8 * (q % X), (uint32_t)(q / X) & 1u, p.flag, GT_CODE + 11);
     } else if (warp < 4) {
         // ---- MMA issue: warps 1 and 3 take the units in turn -------------------------------------------------------
         const bool leader = elect_one();
@@ -289,9 +290,9 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                 bool ok = true;
 #pragma unroll
                 for (int st = 0; st < US; st++) {
-                    ok = ok && gt_wait(xfull + 8 * x, xph, p.flag, 6) && gt_wait(full + 8 * s, ph, p.flag, 2);
+                    ok = ok && gt_wait(xfull + 8 * x, xph, p.flag, GT_CODE + 6) && gt_wait(full + 8 * s, ph, p.flag, GT_CODE + 2);
                     const bool first = FM == 4 || st == 0, last = FM == 4 || st == US - 1; // of the buffer's stages
-                    if (first && ok) ok = gt_wait(accempty + 8 * a, aph, p.flag, 9);
+                    if (first && ok) ok = gt_wait(accempty + 8 * a, aph, p.flag, GT_CODE + 9);
                     if (ok) {
                         tc_fence_after();
                         const uint32_t d = tmem_base + (uint32_t)(a * p.acc_cols);
@@ -345,8 +346,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         for (int it = team; it < nstages; it += GT_TEAMS) {
             const bool t0 = mbar_test(rawfull + 8 * r, rph);
             const bool t1 = it < S || mbar_test(empty + 8 * s, ph ^ 1u);
-            if (!t0) ok = mbar_wait(rawfull + 8 * r, rph, p.flag, 3);
-            if (ok && !t1) ok = mbar_wait(empty + 8 * s, ph ^ 1u, p.flag, 7);
+            if (!t0) ok = mbar_wait(rawfull + 8 * r, rph, p.flag, GT_CODE + 3);
+            if (ok && !t1) ok = mbar_wait(empty + 8 * s, ph ^ 1u, p.flag, GT_CODE + 7);
             if (!ok) break;
             const uint32_t unit = raw_base + (uint32_t)(r * GT_RAW_BYTES), box = unit + part, zeros_addr = unit + zeros_at;
             const uint32_t slot = base + (uint32_t)(s * GT_A_BYTES);
@@ -430,7 +431,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             for (int i = 0; i < NCH * 8; i++) tot[i] = 0.0f;
 #pragma unroll 1
             for (int f = 0; f < folds && ok; f++) {
-                ok = gt_wait(scfull + 8 * c, cph, p.flag, 10) && gt_wait(accfull + 8 * a, aph, p.flag, 4);
+                ok = gt_wait(scfull + 8 * c, cph, p.flag, GT_CODE + 10) && gt_wait(accfull + 8 * a, aph, p.flag, GT_CODE + 4);
                 if (!ok) break;
                 tc_fence_after();
                 uint16_t sraw;

@@ -67,10 +67,25 @@ def awq_decode_matmul(lin, x2, y):
               lin.group_size, _p(ws), ws.numel(), _st())
 
 
+_flags: dict = {}
+
+
+def _flag_words(device) -> torch.Tensor:
+    """What ``oxq_packed4_matmul`` reports through on this device: a header of its own, which no larger layer ever replaces (a captured
+    graph keeps its address) and which costs no slab."""
+    key = _dev_index(device)
+    buf = _flags.get(key)
+    if buf is None:
+        buf = _flags[key] = torch.zeros(256, dtype=torch.uint8, device=torch.device("cuda", key))
+    return buf
+
+
 def check(ws: torch.Tensor) -> None:
-    """Synchronise and raise if a tensor-core kernel recorded a timed-out wait in ``ws``."""
-    _lib.call("oxq_gemm_check", ctypes.c_void_p(ws.data_ptr()),
-              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    """Synchronise and raise if a tensor-core kernel recorded a timed-out wait in ``ws`` or in its device's flag words."""
+    for buf in (ws, _flags.get(ws.device.index)):
+        if buf is not None:
+            _lib.call("oxq_gemm_check", ctypes.c_void_p(buf.data_ptr()),
+                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
 
 
 def _p(t) -> int:
@@ -95,18 +110,18 @@ def awq_matmul(lin, x2, y):
 
 def packed4_matmul(lin, x2, y, tensors=None):
     """``y = x2 . deq(W) (+ bias)`` for the 4-bit layouts by the grouped unpack + tcgen05 kernel (``oxq_packed4_matmul``). The
-    scratch is this call's own, so calls on several streams do not meet; the workspace lends its flag word."""
+    scratch is this call's own, so calls on several streams do not meet."""
     m, n = x2.shape[0], lin.out_features
-    ws = _workspaces.get(x2.device.index)
-    if ws is None:
-        ws = workspace(n, lin.in_features, x2.device)
+    flag = _flags.get(x2.device.index)
+    if flag is None:
+        flag = _flag_words(x2.device)
     need = lin._scratch_bytes.get(m)
     if need is None:
         need = lin._scratch_bytes[m] = int(_lib.load().oxq_packed4_scratch_bytes(m, n))
     scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
     qw, qz, sc, sc_dt, b, b_dt = tensors or lin._tensors()
     _lib.call("oxq_packed4_matmul", x2.data_ptr(), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, y.data_ptr(), _dt(y.dtype), m,
-              lin.in_features, n, lin.group_size, int(lin.pack_dim == "in"), int(lin.sym), ws.data_ptr(), scratch.data_ptr(), need,
+              lin.in_features, n, lin.group_size, int(lin.pack_dim == "in"), int(lin.sym), flag.data_ptr(), scratch.data_ptr(), need,
               _st())
 
 

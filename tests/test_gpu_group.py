@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import oracle
-from oxydllm_b200 import gemm, synth
+from oxydllm_b200 import _lib, gemm, synth
 from oxydllm_b200 import linear as L
 
 pytestmark = pytest.mark.gpu
@@ -102,6 +102,17 @@ def test_a_replaced_tensor_is_the_one_that_counts(cuda, gptq):
     lin.qweight = want.qweight.cpu()
     with pytest.raises(ValueError, match="CUDA tensors only"):
         lin.forward(xs[0])
+
+
+def test_a_wait_that_ran_out_is_reported_whatever_became_of_the_workspace(cuda):
+    lin, w = layer(256, 128, 128, False, seed=3)
+    x = torch.from_numpy(np.ascontiguousarray(synth.activations(16, 256, seed=3))).to(torch.bfloat16).cuda()
+    lin.forward(x)
+    _lib.call("oxq_selftest_wait_expiry", gemm._flag_words("cuda").data_ptr(), 29, None)  # where that call's kernel reports
+    ws = gemm.workspace(4096, 8192, "cuda")  # larger than a 256 x 128 layer's
+    with pytest.raises(_lib.OxqError, match="bounded wait 29 .*29 = accumulator free"):
+        gemm.check(ws)
+    gemm.check(ws)
 
 
 def off16(t, offset):

@@ -88,9 +88,10 @@ int oxq_awq_gemv(const void *x, int x_dtype, const uint32_t *qweight, const uint
  * k can be split; elsewhere oxq_awq_gemv serves up to 32 tokens). No counterpart in the reference. */
 int oxq_awq_gemv_max_m(int k, int n, int group_size);
 
-/* oxq_awq_gemv streams weight boxes into shared memory with the TMA unit and waits for each with a
- * bounded wait. Synchronises `stream`; returns OXQ_ERR_DEVICE_FLAG (once) if such a wait ran out on
- * the current device in any oxq_awq_gemv call since the last check. No counterpart in the reference. */
+/* oxq_awq_gemv streams weight boxes into shared memory with the TMA unit, oxq_gguf_gemv on wide Q6_K layers (vocabulary
+ * projections) weight rows with bulk copies, and both wait for them with bounded waits. Synchronises `stream`; returns
+ * OXQ_ERR_DEVICE_FLAG (once) if such a wait ran out on the current device in any call of either since the last check. No
+ * counterpart in the reference. */
 int oxq_awq_gemv_check(void *stream);
 
 /* Gated FFN projection on a fused AWQ [gate | up] weight (concat_awq_along_out of gate_proj and
@@ -209,6 +210,14 @@ int oxq_selftest_gemm_wait_expiry(void *workspace, size_t workspace_bytes, int m
  * workspace: at least 1 MiB, 256-byte aligned; oxq_gemm_check(workspace) afterwards returns
  * OXQ_ERR_DEVICE_FLAG once. No counterpart in the reference. */
 int oxq_selftest_moe_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
+
+/* The same for the grouped 4-bit kernel (oxq_packed4_matmul): its packed words and scales never come. Flag word, workspace and check as
+ * for the MoE kernel; the code is one of 21 .. 31. */
+int oxq_selftest_group_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
+
+/* The same for the Q6_K GEMV of wide layers: scratch of at least 256 KiB, 256-byte aligned; oxq_awq_gemv_check afterwards returns
+ * OXQ_ERR_DEVICE_FLAG once. */
+int oxq_selftest_q6k_wait_expiry(void *scratch, size_t scratch_bytes, void *stream);
 
 /* Zeroes the 256-byte header (flag word) of a fresh workspace on `stream`. */
 int oxq_gemm_workspace_init(void *workspace, void *stream);

@@ -84,6 +84,7 @@ struct GroupTcParams {
     int sym;                        // GPTQ without stored zero points (zero + 1 = 8)
     int col_base, ldy;
     int split;                      // shares may begin and end inside a tile
+    int test_skip_loads;            // self-test: packed words and scales are never loaded
     int *flag;
     float *partials;                // [CTA + tile][mpad][128] f32
     unsigned long long *tickets;    // per tile: this call's mark above, arrivals in the low byte
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             const uint32_t *zsrc = p.qzeros + group * p.packed_out + n0 / 8;
             const uint16_t *ssrc = reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0;
             if (it >= R) ok = gt_wait(rawempty + 8 * r, ph ^ 1u, p.flag, GT_CODE + 1);
-            if (ok && leader) {
+            if (ok && leader && !p.test_skip_loads) {
                 const uint32_t dst = raw_base + (uint32_t)(r * GT_RAW_BYTES), bar = rawfull + 8 * r;
                 mbar_arrive_expect_tx(bar, bytes);
                 if (GPTQ) tma_load_2d(dst, &wmap, bar, n0, k0 / 8);
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             if (++r == R) { r = 0; ph ^= 1u; }
             for (int f = 0; f < unit_folds && ok; f++, fold++) { // unit_folds > 1: groups shorter than a unit, one fold each
                 if (fold >= GT_SC) ok = gt_wait(scempty + 8 * c, cph ^ 1u, p.flag, GT_CODE + 8);
-                if (ok && leader) {
+                if (ok && leader && !p.test_skip_loads) {
                     mbar_arrive_expect_tx(scfull + 8 * c, GT_SC_BYTES);
                     bulk_copy_g2s(sc_base + c * GT_SC_BYTES, ssrc + (size_t)f * p.n, GT_SC_BYTES, scfull + 8 * c);
                 }
@@ -605,6 +606,8 @@ static int group_tc_launch(const GroupTcParams &p, const CUtensorMap &wmap, cons
     return OXQ_OK;
 }
 
+static thread_local int g_group_selftest_skip_loads = 0; // set only inside oxq_selftest_group_wait_expiry
+
 int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                     int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
                     cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes)
@@ -614,6 +617,7 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
     p.scales_f16 = scales_dtype == OXQ_F16; p.bias_dtype = bias_dtype; p.y_dtype = y_dtype;
     p.m = m; p.n = n; p.packed_out = n / 8; p.col_base = col_base; p.ldy = ldy; p.flag = flag;
     p.sym = (gptq && (sym || qzeros == nullptr)) ? 1 : 0;
+    p.test_skip_loads = g_group_selftest_skip_loads;
     while ((1 << p.gshift) < group_size) p.gshift += 1;
     p.fold_rows = group_size < GT_UNIT ? group_size : GT_UNIT;
     p.token_blocks = ceil_div(m, GT_MAX_TOKENS);
@@ -688,3 +692,22 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
 }
 
 } // namespace oxq
+
+// Self-test of the abort path: one tile of one unit (128 x 128, 16 tokens) whose packed words and scales never come. x arrives; the unpack
+// teams, the MMA issuers, the x producer's last waits and the fold warps each give up after their two seconds, side by side, the flag
+// word takes the first code, tensor memory is freed and the kernel returns with no copy in flight. Nothing faults or hangs.
+OXQ_EXPORT int oxq_selftest_group_wait_expiry(void *workspace, size_t workspace_bytes, void *stream)
+{
+    oxq::clear_error();
+    OXQ_REQUIRE(workspace && workspace_bytes >= (1u << 20) && oxq::aligned(workspace, 256), OXQ_ERR_WORKSPACE,
+                "oxq_selftest_group_wait_expiry: 256-byte aligned workspace of at least 1 MiB needed");
+    unsigned char *b = reinterpret_cast<unsigned char *>(workspace);
+    const int m = 16, k = 128, n = 128;
+    // x [16, 128] bf16 | words [128, 16] | zero points [1, 16] | scales [1, 128] | y [16, 128] f32, 64 KB apart
+    oxq::g_group_selftest_skip_loads = 1;
+    const int rc = oxq::group_tc_matmul(b + (1 << 16), reinterpret_cast<uint32_t *>(b + (2 << 16)), reinterpret_cast<uint32_t *>(b + (3 << 16)),
+                                        b + (4 << 16), OXQ_F16, nullptr, 0, b + (5 << 16), OXQ_F32, m, k, n, 128, 0, n,
+                                        reinterpret_cast<int *>(workspace), (cudaStream_t)stream, 0, 0, nullptr, 0);
+    oxq::g_group_selftest_skip_loads = 0;
+    return rc;
+}

@@ -234,6 +234,7 @@ struct Q6kWideParams {
     void *y;
     int bias_dtype, y_dtype;
     int m, k, n, tiles, ring;
+    int test_skip_loads; // self-test: no stage is ever loaded
 };
 
 __device__ __forceinline__ uint32_t q6w_lds32(uint32_t addr)
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6k
             for (int ch = 0; ch < chunks && ok; ch++, it++) {
                 if (it == p.ring) pdl_wait(); // slots come free only after x: that time must not count as this wait
                 if (it >= p.ring) ok = __all_sync(0xFFFFFFFFu, mbar_wait(empty(r), ph ^ 1u, &g_q6k_gemv_flag, 1));
-                if (ok) {
+                if (ok && !p.test_skip_loads) {
                     if (lane == 0) mbar_arrive_expect_tx(full(r), Q6W_STAGE_BYTES);
                     __syncwarp();
                     if (lane < Q6W_ROWS)
@@ -424,9 +425,9 @@ static int q6w_ring(int m, int k, int n, const void *blocks)
     return ring < 2 ? 0 : ring < Q6W_MAX_RING ? ring : Q6W_MAX_RING;
 }
 
-static int launch_q6k_wide(const Q6kGemvParams &g, int ring, cudaStream_t st)
+static int launch_q6k_wide(const Q6kGemvParams &g, int ring, cudaStream_t st, int test_skip_loads = 0)
 {
-    Q6kWideParams p = {g.x, g.blocks, g.bias, g.y, g.bias_dtype, g.y_dtype, g.m, g.k, g.n, ceil_div(g.n, Q6W_ROWS), ring};
+    Q6kWideParams p = {g.x, g.blocks, g.bias, g.y, g.bias_dtype, g.y_dtype, g.m, g.k, g.n, ceil_div(g.n, Q6W_ROWS), ring, test_skip_loads};
     const size_t smem = (size_t)Q6W_ENGINES * ring * Q6W_STAGE_BYTES + q6w_fixed(g.m, g.k);
     static size_t configured[64] = {};
     int device = 0;
@@ -536,3 +537,17 @@ int q6k_gemv(const void *x, const void *blocks, const void *bias, int bias_dtype
 }
 
 } // namespace oxq
+
+// Self-test of the wide kernel's abort path: one tile (16 rows x 2048) whose stage never comes. The eight warps that wait for it give up
+// after two seconds, side by side, the flag takes their code and the kernel returns; oxq_awq_gemv_check reports it.
+OXQ_EXPORT int oxq_selftest_q6k_wait_expiry(void *scratch, size_t scratch_bytes, void *stream)
+{
+    oxq::clear_error();
+    OXQ_REQUIRE(scratch && scratch_bytes >= (1u << 18) && oxq::aligned(scratch, 256), OXQ_ERR_WORKSPACE,
+                "oxq_selftest_q6k_wait_expiry: 256-byte aligned scratch of at least 256 KiB needed");
+    unsigned char *b = reinterpret_cast<unsigned char *>(scratch);
+    oxq::Q6kGemvParams p = {};
+    p.x = reinterpret_cast<__nv_bfloat16 *>(b); p.blocks = b + (1 << 16); p.y = b + (3 << 16);
+    p.y_dtype = OXQ_F32; p.m = 1; p.k = oxq::Q6W_SB * 256; p.n = oxq::Q6W_ROWS;
+    return oxq::launch_q6k_wide(p, 2, (cudaStream_t)stream, 1);
+}

@@ -115,6 +115,26 @@ def test_a_wait_that_ran_out_is_reported_whatever_became_of_the_workspace(cuda):
     gemm.check(ws)
 
 
+def test_grouped_kernel_survives_weights_that_never_come(cuda):
+    ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
+    _lib.call("oxq_selftest_group_wait_expiry", ws.data_ptr(), ws.numel(), None)
+    with pytest.raises(_lib.OxqError, match=r"bounded wait (2[1-9]|3[01]) "):
+        gemm.check(ws)
+    gemm.check(ws)  # reported once
+    lin, w = layer(1024, 256, 128, False, seed=4)
+    x = synth.activations(20, 1024, seed=4)
+    check(lin.forward(torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()), x, w)
+    gemm.check(gemm.workspace(256, 1024, "cuda"))
+
+
+def test_wide_q6k_gemv_survives_weights_that_never_come(cuda):
+    scratch = torch.zeros(1 << 18, dtype=torch.uint8, device="cuda")
+    _lib.call("oxq_selftest_q6k_wait_expiry", scratch.data_ptr(), scratch.numel(), None)
+    with pytest.raises(_lib.OxqError, match="oxq_gguf_gemv: a bounded wait"):
+        _lib.call("oxq_awq_gemv_check", None)
+    _lib.call("oxq_awq_gemv_check", None)
+
+
 def off16(t, offset):
     """The same values `offset` elements behind a 16-byte boundary."""
     room = torch.zeros(t.numel() + offset, dtype=t.dtype, device=t.device)

@@ -31,8 +31,8 @@ def check(y, x, w):
     assert (np.abs(y.double().cpu().numpy() - ref) <= 2.0**-17 * mass + rounding).all()
 
 
-# one unit and one tile; units beyond every ring (k = 5632); groups of 64, 128 and more; tiles shared by two, three and many
-# CTAs; whole tiles (148 of them); one token, the edges of the tile widths and two tiles of tokens
+# one unit and one tile; units beyond every ring (k = 5632, shares inside their tiles); groups of 64, 128 and more; whole tiles,
+# 148 of them too; one token, the edges of the tile widths and two tiles of tokens
 @pytest.mark.parametrize("gptq", [False, True])
 @pytest.mark.parametrize("k,n,g", [(128, 128, 64), (5632, 256, 64), (5632, 128, 512), (2048, 1152, 128), (1024, 18944, 256)])
 @pytest.mark.parametrize("m", [1, 16, 17, 33, 97, 128, 129, 256])
@@ -135,6 +135,20 @@ def test_wide_q6k_gemv_survives_weights_that_never_come(cuda):
     _lib.call("oxq_awq_gemv_check", None)
 
 
+@pytest.mark.parametrize("m", [1, 4, 12])
+def test_gated_projection_into_rows_off_16_bytes(cuda, m):
+    k, inter = 256, 264  # rows of 528 bytes: 16-byte pieces that all lie off a boundary once the first does
+    qw, qz, sc = synth.awq_layer(k, 2 * inter, 128, seed=m)
+    lin = L.PackedQuantLinear(L.QuantWeight.new_awq(4, *(torch.from_numpy(a.view(np.int32)).cuda() for a in (qw, qz)),
+                                                    torch.from_numpy(sc).cuda()))
+    x = torch.from_numpy(np.ascontiguousarray(synth.activations(m, k, seed=m))).to(torch.bfloat16).cuda()
+    for activation in ("silu", "gelu_tanh"):
+        want = L.GatedFfnProjection(lin, activation).forward(x)
+        y = off16(torch.full_like(want, float("nan")), 3)
+        gemm.awq_ffn_gate_up(lin, x, y, L.ACTIVATIONS[activation])
+        assert torch.equal(y, want)
+
+
 def off16(t, offset):
     """The same values `offset` elements behind a 16-byte boundary."""
     room = torch.zeros(t.numel() + offset, dtype=t.dtype, device=t.device)
@@ -199,7 +213,8 @@ def test_calls_on_two_streams_and_a_replayed_graph_do_not_meet(cuda):
 
 
 # ------------------------------------------------------------------ the GGUF GEMV of wide layers (vocabulary projections)
-@pytest.mark.parametrize("m,k,n", [(1, 2048, 9472), (3, 4096, 9480), (8, 4096, 9479), (4, 14336, 9472), (8, 2048, 9472)])
+# k = 14336: x of three tokens leaves room for two stages per engine, of four it does not (the narrow kernel)
+@pytest.mark.parametrize("m,k,n", [(1, 2048, 9472), (3, 4096, 9480), (8, 4096, 9479), (3, 14336, 9472), (4, 14336, 9472), (8, 2048, 9472)])
 def test_wide_q6k_gemv_matches_64_bit_sums(cuda, m, k, n):
     """x and the 6-bit integers are exact in f16; 16-wide sums, times d * scale (one rounding), are added in f32."""
     from oxydllm_b200 import formats as F

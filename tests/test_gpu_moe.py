@@ -242,3 +242,41 @@ def test_decode_rows_do_not_depend_on_the_batch(cuda, hidden, inter):
                             d["dn_bias"], hidden, inter, 7.0)
     row_inf = np.abs(ref).max(axis=1, keepdims=True)
     assert (np.abs(alone.float().cpu().numpy() - ref) <= 2e-2 * row_inf + 1e-5).all()
+
+
+@pytest.mark.parametrize("tokens", [13, 257, 511, 512, 513])
+def test_dispatch_over_256_experts(cuda, tokens):
+    """The table of the one-launch dispatch at its full width and at its limit of 2048 pairs, the separate launches above it; every
+    expert, and a range of them whose other pairs are left out."""
+    d = synth.gptoss_moe(256, 64, 64, tokens, seed=tokens)
+    layer = build(d)
+    x, logits = dev(d["x"], torch.bfloat16), dev(d["logits"])
+    idx, w = oracle.moe_route(d["logits"], 4, True)
+    for lo, hi in ((0, 256), (200, 256), (3, 4)):
+        y = layer.forward_with_logits(x, logits, expert_range=(lo, hi))
+        layer.check()
+        ref = oracle.gptoss_moe(d["x"], idx, w, d["gu_blocks"], d["gu_scales"], d["gu_bias"], d["dn_blocks"], d["dn_scales"],
+                                d["dn_bias"], 64, 64, 7.0, expert_range=(lo, hi))
+        row_inf = np.abs(ref).max(axis=1, keepdims=True)
+        assert (np.abs(y.float().cpu().numpy() - ref) <= 2e-2 * row_inf + 1e-5).all()
+
+
+@pytest.mark.parametrize("tokens,hidden", [(1, 8), (3, 264), (40, 2880)])
+def test_combine_into_rows_off_16_bytes(cuda, tokens, hidden):
+    from oxydllm_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    rows = torch.randn(tokens * 4, hidden, generator=g, device="cuda").to(torch.bfloat16)
+    idx = torch.stack([torch.randperm(8, generator=g, device="cuda")[:4] for _ in range(tokens)]).to(torch.int32)
+    w = torch.rand(tokens, 4, generator=g, device="cuda")
+    pos = torch.randperm(tokens * 4, generator=g, device="cuda").to(torch.int32).reshape(tokens, 4)
+    want = moe.combine(rows, idx, w, pos, 8)
+    room = torch.full((tokens * hidden + 1,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _lib.call("oxq_moe_combine", rows.data_ptr(), idx.data_ptr(), w.data_ptr(), pos.data_ptr(), tokens, 4, hidden, 8,
+              room[1:].data_ptr(), _lib.OXQ_BF16, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(room[1:].view(tokens, hidden), want)
+    order = idx.argsort(dim=1)
+    ref = torch.zeros(tokens, hidden, dtype=torch.float64, device="cuda")
+    for s in range(4):
+        at = order[:, s:s + 1]
+        ref += w.gather(1, at).double() * rows[pos.gather(1, at)[:, 0].long()].double()
+    assert ((want.double() - ref).abs() <= 2.0**-8 * ref.abs() + 1e-5).all()  # one bf16 rounding of the f32 sum

@@ -28,8 +28,8 @@ PACKED_SIMT_GEMV_MAX_M = 8
 AWQ_FUSED_MIN_M = 17
 # GPTQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu): the GEMV does not split k, so it is the
 # faster one on short k only, us at 1 / 2 tokens against the kernel: groups of 128, 1024 x 4096 4.8 / 5.2 against 7.7, 2048 x 6144
-# 7.7 / 8.6 against 10.0, 3072 x 4096 10.3 / 11.7 against 10.9, 2048 x 14336 14.2 / 16.2 against 12.4; groups of 64, 1024 x 4096
-# 6.6 / 7.4 against 8.4, 2048 x 4096 11.6 / 13.5 against 10.4.
+# 7.7 / 8.6 against 10.0, 3072 x 4096 10.3 / 11.7 against 10.9, 4096 x 512 10.7 / 11.9 against 11.2, 2048 x 14336 14.2 / 16.2 against
+# 12.4; groups of 64, 1024 x 4096 6.6 / 7.4 against 8.4, 2048 x 512 8.9 / 10.4 against 9.6, 2048 x 4096 11.6 / 13.5 against 10.4.
 GPTQ_FUSED_MIN_M = 3
 GPTQ_GEMV_MAX_N = 6144
 
@@ -306,9 +306,10 @@ class PackedQuantLinear:
         if awq:  # the AWQ GEMV wants x and qweight on 16 bytes too: above its batches the GEMM on slabs takes any weight
             return most, int(_lib.load().oxq_awq_gemv_max_m(k, n, g)), 8 if n <= 9472 else 16
         few = GPTQ_FUSED_MIN_M - 1  # the GPTQ GEMV takes x on any 4 bytes, the GEMM does not
-        if n > GPTQ_GEMV_MAX_N or k > 3072 or (g == 64 and k > 1024):
+        reach = (2048 if n <= 1024 else 1024) if g == 64 else (4096 if n <= 1024 else 3072)  # longest k, one token
+        if n > GPTQ_GEMV_MAX_N or k > reach:
             return most, 0, few
-        return most, few if k <= 2048 else 1, few
+        return most, few if k <= max(reach - 1024, 1024) else 1, few
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""

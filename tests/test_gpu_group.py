@@ -156,7 +156,7 @@ def off16(t, offset):
     return room[offset:].view(t.shape)
 
 
-@pytest.mark.parametrize("k,n", [(1024, 512), (4096, 1024), (2048, 8192)])  # GEMV up to two tokens, none
+@pytest.mark.parametrize("k,n", [(1024, 512), (4096, 1024), (2048, 8192)])  # GEMV up to two tokens, one, none
 @pytest.mark.parametrize("m", [1, 2])
 def test_gptq_decode_takes_x_on_any_4_bytes(cuda, m, k, n):
     """A row of a fused projection's output is such an x. f32 sums of products that are exact but for the scale's rounding."""

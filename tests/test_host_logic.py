@@ -49,8 +49,9 @@ def test_no_cpu_path():
     # not for the grouped kernel: groups of 32, out features off 128
     (False, 4096, 4096, 32, 32), (False, 4096, 4088, 128, 32), (True, 4096, 4088, 128, 8),
     # GPTQ: short k
-    (True, 1024, 4096, 128, 2), (True, 2048, 6144, 128, 2), (True, 3072, 1024, 128, 1), (True, 4096, 1024, 128, 0),
-    (True, 2048, 14336, 128, 0), (True, 1024, 1024, 64, 2), (True, 2048, 1024, 64, 0)])
+    (True, 1024, 4096, 128, 2), (True, 2048, 6144, 128, 2), (True, 3072, 1024, 128, 2), (True, 4096, 1024, 128, 1),
+    (True, 3072, 4096, 128, 1), (True, 4096, 4096, 128, 0), (True, 2048, 14336, 128, 0), (True, 1024, 4096, 64, 2), (True, 2048, 512, 64, 1),
+    (True, 2048, 4096, 64, 0)])
 def test_batches_of_the_4_bit_gemvs(gptq, k, n, g, gemv):
     words = torch.zeros((k // 8, n) if gptq else (k, n // 8), dtype=torch.int32)
     new = (lambda *a: L.QuantWeight.new_gptq(4, False, *a)) if gptq else (lambda *a: L.QuantWeight.new_awq(4, *a))

@@ -6,7 +6,12 @@
  * cudaStream_t passed as void*. The library never allocates or frees caller
  * memory, never synchronises the device and never aborts: it returns an
  * oxq_status and records a message retrievable with oxq_last_error().
- * All work is enqueued on the given stream. Results are deterministic: no
+ * All work is enqueued on the given stream. The GEMV entry points (awq, gguf, fp8 and
+ * mxfp4, and oxq_awq_ffn_gate_up at GEMV batches) start while the kernel ahead of them on
+ * the stream is still running and wait for it before they read x or write y, but not
+ * before they read weights, scales and zero points: these must not come from the kernel
+ * just ahead. All other entry points are ordered by the stream alone, weights included.
+ * Results are deterministic: no
  * floating-point atomics, fixed-order reductions (the reference's
  * bit-reproducibility contract, metal_ops.rs:4562-4625).
  *
@@ -230,10 +235,11 @@ int oxq_gemm_check(const void *workspace, void *stream);
 
 /* PackedQuantLinear::forward beyond the decode GEMV: maybe_mpp_quant_matmul, else
  * dequantize_w4 + matmul (linear.rs:494-524, metal_ops.rs:2771-2797). Up to 256
- * tokens, when n % 128 == 0, k % 128 == 0, group_size is a power of two >= 64 and the scales are f16 or bf16, one kernel unpacks
- * the words into its shared-memory operand and multiplies on tcgen05 (no slab
- * written); all other calls dequantize slabs into the workspace. The workspace is required
- * (and its flag word used) either way. */
+ * tokens, when n % 128 == 0, k % 128 == 0, group_size is a power of two >= 64, the scales are
+ * f16 or bf16 and the tensors 16-byte aligned, one kernel unpacks the words into its
+ * shared-memory operand and multiplies on tcgen05 (no slab written); all other calls
+ * dequantize slabs into the workspace. The workspace is required (and its flag word used)
+ * either way. */
 int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
                  int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                  int group_size, void *workspace, size_t workspace_bytes, void *stream);
@@ -310,7 +316,7 @@ int oxq_gptoss_moe_forward(const void *x, int x_dtype, const float *router_logit
                            const uint8_t *dn_scales, const void *dn_bias, int bias_dtype, float limit, int expert_lo,
                            int expert_hi, void *out, int out_dtype, void *workspace, size_t workspace_bytes,
                            void *stream);
-/* The same on router logits of any dtype (as the router's linear returns them). */
+/* The same on router logits of any oxq_dtype (as the router's linear returns them). */
 int oxq_gptoss_moe_forward_logits(const void *x, int x_dtype, const void *router_logits, int logits_dtype, int tokens, int num_experts,
                            int top_k, int norm_topk, int hidden, int inter, const uint8_t *gu_blocks,
                            const uint8_t *gu_scales, const void *gu_bias, const uint8_t *dn_blocks,

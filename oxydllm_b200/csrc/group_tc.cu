@@ -25,10 +25,9 @@
 // stage each, 320 a stage together, and the others waiting for them), and behind it most likely shared memory: a stage moves 4 KB
 // of packed words in and out and 16 KB of operand in and out, 320 clocks at 128 B, of which ncu's L1 figure (36 %) leaves out the
 // MMA's reads; sixteen unpack warps instead of eight were 2 to 5 % slower. Issue slots are 47 %, DRAM 22 % busy (4096 x 28672).
-// Beside that about 6 us a launch go into filling the pipeline and putting
-// shared tiles together. Measured in a graph, us at 16 / 77 / 128 tokens (the
-// kernel with scaled bf16 weights before it): 4096 x 4096 10 / 16 / 20 (14 / 19 / 22), 4096 x 28672 30 / 49 / 55 (55 / 59 / 61),
-// 14336 x 4096 20 / 27 / 33 (28 / 34 / 38).
+// Beside that about 7 us a launch go into filling the pipeline, which begins when the kernel ahead has finished, and putting shared
+// tiles together. Measured in a graph, us at 16 / 77 / 128 tokens (the kernel with scaled bf16 weights before it): 4096 x 4096
+// 12 / 17 / 20 (14 / 19 / 22), 4096 x 28672 32 / 50 / 56 (55 / 59 / 61), 14336 x 4096 22 / 30 / 34 (28 / 34 / 38).
 #include <atomic>
 
 #include <cuda_bf16.h>
@@ -553,10 +552,11 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
 }
 
 // Largest batch for this kernel. Above it the kernel of fused_tc.cu, which scales and rounds the weights as it unpacks them and
-// folds nothing, is the faster one, us there / here: groups of 64, where every stage is folded, 3072 x 5120 at 16 / 48 tokens
-// 14.6 / 12.8 and 16.6 / 19.3, 3072 x 16384 25.4 / 18.6 and 25.8 / 26.9; one tile per CTA, 4096 x 14336, 31.1 / 31.5 at 128 tokens. More than 128 tokens are two tiles that unpack the same weights twice: worth it where that
-// fills idle SMs (256 tokens, 4096 x 4096: 34 / 23; 4096 x 14336: 41 / 51). Groups of 32 would be
-// folded four times a unit: 4096 x 28672 took 58 us at any batch, the GEMV 38 at 8 tokens, and above 32 tokens the dense copy wins.
+// folds nothing, is the faster one, us there / here: groups of 64, where every stage is folded, 3072 x 4096 at 32 tokens 14.0 / 12.5,
+// 3072 x 14336 26.1 / 21.1, but 3072 x 5120 at 48 tokens 16.6 / 19.3 (when it still began ahead of the wait); one tile per CTA, 4096 x 14336,
+// 31.2 / 29.8 at 96 tokens, 31.1 / 31.5 at 128 (likewise). More than 128 tokens are two tiles that unpack the same weights twice: worth it where that fills idle SMs (256 tokens,
+// 4096 x 4096: 35 / 23; 4096 x 14336: 41 / 51). Groups of 32 would be folded four times a unit: 4096 x 28672 took 58 us at any batch,
+// the GEMV 38 at 8 tokens, and above 32 tokens the dense copy wins.
 int group_tc_max_m(int n, int group_size)
 {
     const int tiles = n / GT_ROWS;

@@ -513,8 +513,8 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     // no dequantized slab, one launch per projection over all experts.
     const bool fused = moe_fused_supported(2 * inter, hidden, gu_blocks, gu_scales, xs, h, inter) &&
                        moe_fused_supported(hidden, inter, dn_blocks, dn_scales, h, xs, hidden);
-    // The per-pair GEMVs cost about 6.3 us a pair on the GPT-OSS shape (201 us at 32 pairs); the grouped kernel reads every
-    // expert that has rows once, 0.32 ms at 128 pairs: it takes over from about 48 pairs.
+    // The per-pair GEMVs cost about 5.6 us a pair on the GPT-OSS shape (187 us at 32 pairs, 268 at 48); the grouped kernel reads every
+    // expert that has rows once, 196 us at 52 pairs, 219 at 128: it takes over from 49 pairs (by these figures about 35 would do).
     if (L.decode && !(fused && pairs > MOE_DECODE_FUSED_FROM_PAIRS)) {
         OXQ_REQUIRE(aligned(gu_blocks, 16) && aligned(dn_blocks, 16), OXQ_ERR_BAD_ALIGN,
                     "oxq_gptoss_moe_forward: expert blocks must be 16-byte aligned");

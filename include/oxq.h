@@ -215,6 +215,8 @@ int oxq_selftest_gemm_wait_expiry(void *workspace, size_t workspace_bytes, int m
  * workspace: at least 1 MiB, 256-byte aligned; oxq_gemm_check(workspace) afterwards returns
  * OXQ_ERR_DEVICE_FLAG once. No counterpart in the reference. */
 int oxq_selftest_moe_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
+/* ... and for its block-scaled counterpart of small batches (codes 61 .. 67). */
+int oxq_selftest_moe_mx_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
 
 /* The same for the grouped 4-bit kernel (oxq_packed4_matmul): its packed words and scales never come. Flag word, workspace and check as
  * for the MoE kernel; the code is one of 21 .. 31. */

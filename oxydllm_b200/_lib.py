@@ -42,6 +42,7 @@ SIGNATURES = {
     "oxq_selftest_wait_expiry": [_vp, ctypes.c_int, _vp],
     "oxq_selftest_gemm_wait_expiry": [_vp, ctypes.c_size_t, ctypes.c_int, _vp],
     "oxq_selftest_moe_wait_expiry": [_vp, ctypes.c_size_t, _vp],
+    "oxq_selftest_moe_mx_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_selftest_group_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_selftest_q6k_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_awq_gemv_check": [_vp],

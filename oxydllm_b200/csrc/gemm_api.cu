@@ -154,7 +154,9 @@ OXQ_EXPORT int oxq_gemm_check(const void *workspace, void *stream)
                 "tensor-core kernel: bounded wait %d ran out (1 = ring slot, 2 = tile data, 3 = accumulator ready, "
                 "4 = accumulator free, 5 = meeting of the fold warps; grouped 4-bit kernel: 21 = ring slot, 22 = operand tile, "
                 "23 = packed words, 24 = accumulator ready, 25 = x slot, 26 = x, 27 = operand slot, 28 = slot for scales, "
-                "29 = accumulator free, 30 = scales, 31 = last MMAs) in a call since the last check", flag);
+                "29 = accumulator free, 30 = scales, 31 = last MMAs; block-scaled kernel of the experts: 61 = weight slot, 62 = row slot, "
+                "63 = accumulator free, 64 = operands or accumulator ready, 65 = packed words, 66 = operand slot, 67 = last MMAs) in a call "
+                "since the last check", flag);
     return OXQ_OK;
 }
 

@@ -20,6 +20,14 @@ int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const ui
                       const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi,
                       float limit, int *flag, cudaStream_t st);
 
+int moe_mx_block_rows();
+size_t moe_mx_piece_bytes(int rows, int k);
+size_t moe_mx_scale_bytes(int rows, int k);
+bool moe_mx_supported(int n, int k, const void *blocks, const void *scales);
+int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, cudaStream_t st);
+int moe_mx_grouped(const void *pieces, const void *sfx, int rows_cap, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
+                   const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi, float limit,
+                   int *flag, cudaStream_t st);
 bool mxfp4_gemv_batched_supported(int k, const void *blocks);
 int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const uint8_t *scales, const void *bias,
                        int bias_dtype, const int *pair_expert, int pairs, int e_lo, int e_hi, void *y, int y_dtype, int k,
@@ -27,10 +35,19 @@ int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const ui
 
 constexpr int MOE_MAX_EXPERTS = 256;
 constexpr int MOE_MAX_TOPK = 8;
-// Up to this many (token, slot) pairs the layer runs as batched single-token GEMVs on the packed
+// Up to this many (token, slot) pairs the layer can run as batched single-token GEMVs on the packed
 // weights of the selected experts only (decode); above, it dequantizes expert groups for the grouped GEMM.
 constexpr int MOE_DECODE_MAX_PAIRS = 64;
+// From more pairs than this one of the grouped kernels takes over, which read every expert that has rows once. By time alone it would be
+// 8: us a layer, GEMVs / block-scaled kernel, 32 experts of 2880 x 2880 at 1, 2, 3, 4, 8, 12 tokens (4 pairs each) 43 / 48, 66 / 67,
+// 87 / 76, 107 / 81, 190 / 107, 268 / 124. But the GEMVs keep gate and up in f32 up to the down projection, and a token's result there
+// is the same bits alone and in a batch.
 constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
+// Rows per expert, on average, up to which the block-scaled kernel is the better one: above, most experts take two of its blocks of 48
+// rows, and the kernel that unpacks once for up to 256 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
+// 300, 384, 450 tokens: 124 / 183, 149 / 221, 169 / 228, 186 / 235, 237 / 240, 277 / 245; 16 of 2048 x 1024 at 30, 120, 200: 43 / 64,
+// 49 / 67, 70 / 70.
+constexpr int MOE_MX_ROWS = 44;
 
 // One warp per token: f32 softmax over all experts, k rounds of arg-max (ties: lower index),
 // optional renormalisation by the sum of the selected probabilities (moe.rs:472-487).
@@ -406,6 +423,7 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct MoeLayout {
     size_t top_idx, top_w, counts, offsets, grp_beg, entries, perm, inv, xs, h, slab, total;
+    size_t h_scales, x_scales; // inside the slab
     int group_experts, n_groups, max_mt;
     bool decode; // few pairs: no dequantized slab, the slab region holds the f32 gate_up outputs
 };
@@ -429,7 +447,7 @@ static MoeLayout moe_layout(int tokens, int top_k, int n_exp, int hidden, int in
     if (ge > n_exp) ge = n_exp;
     L.group_experts = ge;
     L.n_groups = (n_exp + ge - 1) / ge;
-    L.max_mt = (int)(pairs / 128) + n_exp + 1;
+    L.max_mt = (int)(pairs / moe_mx_block_rows()) + n_exp + 1;
     size_t off = 256;
     L.top_idx = off; off = align_up(off + pairs * 4, 256);
     L.top_w = off; off = align_up(off + pairs * 4, 256);
@@ -442,7 +460,14 @@ static MoeLayout moe_layout(int tokens, int top_k, int n_exp, int hidden, int in
     L.xs = off; off = align_up(off + (pairs + 128) * hidden * 2, 256); // also the down-projection output
     L.h = off; off = align_up(off + (pairs + 128) * inter * 2, 256);
     L.decode = moe_decode_shape(pairs, hidden, inter);
-    L.slab = off; off = align_up(off + (L.decode ? pairs * 2 * inter * sizeof(float) : (size_t)ge * per_expert), 256);
+    // dequantized experts; or the f32 gate_up outputs; or, for the block-scaled kernel, the pieces of h, their scales and those of x's
+    // (x's pieces take as much as xs)
+    const int cap = (int)pairs + 128;
+    L.h_scales = align_up(moe_mx_piece_bytes(cap, inter), 256);
+    L.x_scales = L.h_scales + align_up(moe_mx_scale_bytes(cap, inter), 256);
+    const size_t mx = L.x_scales + moe_mx_scale_bytes(cap, hidden), f32 = pairs * 2 * inter * sizeof(float);
+    const size_t dense = (size_t)ge * per_expert;
+    L.slab = off; off = align_up(off + (L.decode ? (f32 > mx ? f32 : mx) : dense > mx ? dense : mx), 256);
     L.total = off;
     return L;
 }
@@ -513,9 +538,10 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     // no dequantized slab, one launch per projection over all experts.
     const bool fused = moe_fused_supported(2 * inter, hidden, gu_blocks, gu_scales, xs, h, inter) &&
                        moe_fused_supported(hidden, inter, dn_blocks, dn_scales, h, xs, hidden);
-    // The per-pair GEMVs cost about 5.6 us a pair on the GPT-OSS shape (187 us at 32 pairs, 268 at 48); the grouped kernel reads every
-    // expert that has rows once, 196 us at 52 pairs, 219 at 128: it takes over from 49 pairs (by these figures about 35 would do).
-    if (L.decode && !(fused && pairs > MOE_DECODE_FUSED_FROM_PAIRS)) {
+    // Up to a few dozen rows per expert: the codes as tensor-core operands, nothing unpacked.
+    const bool mx = pairs <= MOE_MX_ROWS * n_exp && moe_mx_supported(2 * inter, hidden, gu_blocks, gu_scales) &&
+                    moe_mx_supported(hidden, inter, dn_blocks, dn_scales);
+    if (L.decode && !((fused || mx) && pairs > MOE_DECODE_FUSED_FROM_PAIRS)) {
         OXQ_REQUIRE(aligned(gu_blocks, 16) && aligned(dn_blocks, 16), OXQ_ERR_BAD_ALIGN,
                     "oxq_gptoss_moe_forward: expert blocks must be 16-byte aligned");
         // Decode: only the selected experts' packed weights are read. gate_up (f32 out, bias folded) ->
@@ -535,15 +561,33 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     }
     // the grouped kernel's table of token blocks goes where the m-tile table of the dense path would (same capacity bound);
     // grp_beg[0] then holds the number of blocks
-    if (fused && pairs <= MOE_SMALL_PAIRS) {
-        moe_dispatch_small_kernel<<<1, 1024, 0, st>>>(top_idx, pairs, expert_lo, n_exp, moe_fused_block_rows(), counts, offsets, entries,
+    const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows();
+    if ((fused || mx) && pairs <= MOE_SMALL_PAIRS) {
+        moe_dispatch_small_kernel<<<1, 1024, 0, st>>>(top_idx, pairs, expert_lo, n_exp, block_rows, counts, offsets, entries,
                                                       grp_beg, perm, inv);
     } else {
         moe_count_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, counts);
-        if (fused) moe_plan_blocks_kernel<<<1, MOE_MAX_EXPERTS, 0, st>>>(counts, n_exp, expert_lo, moe_fused_block_rows(), offsets,
+        if (fused || mx) moe_plan_blocks_kernel<<<1, MOE_MAX_EXPERTS, 0, st>>>(counts, n_exp, expert_lo, block_rows, offsets,
                                                                          entries, grp_beg);
         else moe_plan_kernel<<<1, 32, 0, st>>>(counts, n_exp, expert_lo, L.group_experts, offsets, entries, grp_beg);
         moe_scatter_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, offsets, perm, inv);
+    }
+    if (mx) {
+        unsigned char *sb = reinterpret_cast<unsigned char *>(slab);
+        OXQ_LAUNCH_CHECK("moe routing kernels");
+        int rc = moe_mx_split(x, perm, top_k, offsets + n_exp, hidden, a_rows, xs, sb + L.x_scales, st);
+        if (rc) return rc;
+        rc = moe_mx_grouped(xs, sb + L.x_scales, a_rows, gu_blocks, gu_scales, num_experts, 2 * inter, hidden, entries, grp_beg, gu_bias,
+                            bias_dtype, h, inter, 1, limit, flag, st);
+        if (rc) return rc;
+        rc = moe_mx_split(h, nullptr, 1, offsets + n_exp, inter, a_rows, sb, sb + L.h_scales, st);
+        if (rc) return rc;
+        rc = moe_mx_grouped(sb, sb + L.h_scales, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg, dn_bias,
+                            bias_dtype, xs, hidden, 0, limit, flag, st);
+        if (rc) return rc;
+        moe_combine_kernel<<<sm_count() * 8, 256, 0, st>>>(xs, top_idx, top_w, inv, tokens, top_k, hidden, expert_lo, expert_hi, out, out_dtype);
+        OXQ_LAUNCH_CHECK("moe_combine_kernel");
+        return OXQ_OK;
     }
     moe_gather_kernel<<<sm_count() * 8, 256, 0, st>>>((const __nv_bfloat16 *)x, perm, offsets + n_exp, top_k, hidden, xs);
     OXQ_LAUNCH_CHECK("moe routing kernels");

@@ -215,8 +215,9 @@ int oxq_selftest_gemm_wait_expiry(void *workspace, size_t workspace_bytes, int m
  * workspace: at least 1 MiB, 256-byte aligned; oxq_gemm_check(workspace) afterwards returns
  * OXQ_ERR_DEVICE_FLAG once. No counterpart in the reference. */
 int oxq_selftest_moe_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
-/* ... and for its block-scaled counterpart of small batches (codes 61 .. 67). */
+/* ... and for its block-scaled counterpart of small batches (codes 61 .. 67) and the block-scaled kernel of FP8 layers (41 .. 51). */
 int oxq_selftest_moe_mx_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
+int oxq_selftest_packed_mx_wait_expiry(void *workspace, size_t workspace_bytes, void *stream);
 
 /* The same for the grouped 4-bit kernel (oxq_packed4_matmul): its packed words and scales never come. Flag word, workspace and check as
  * for the MoE kernel; the code is one of 21 .. 31. */
@@ -247,12 +248,14 @@ int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight, const uint
                  int group_size, void *workspace, size_t workspace_bytes, void *stream);
 
 /* The kernel that oxq_awq_gemm / oxq_gptq_gemm (4-bit) run up to oxq_packed4_max_m tokens (0: not this shape), with scratch
- * of its own: oxq_packed4_scratch_bytes(m, n) bytes with any contents, 256-byte aligned, one per call in flight. flag_word: the
+ * of its own: oxq_packed4_scratch_bytes(m, n) bytes with any contents, 256-byte aligned, one per call in flight; with
+ * oxq_packed4_full_scratch_bytes large GPTQ layers of up to 16 tokens take a faster kernel. flag_word: the
  * first word of a gemm workspace, or of 256 zeroed bytes that stand in for one (oxq_gemm_check reads and clears them).
  * OXQ_ERR_UNSUPPORTED for shapes the kernel does not take. gptq = 0: AWQ layout (qzeros required); 1: GPTQ layout (sym != 0 or
  * qzeros null: zero point 8). */
 int oxq_packed4_max_m(int k, int n, int group_size);
 size_t oxq_packed4_scratch_bytes(int m, int n);
+size_t oxq_packed4_full_scratch_bytes(int m, int k, int n, int group_size, int gptq);
 int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qweight, const uint32_t *qzeros, const void *scales,
                        int scales_dtype, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                        int group_size, int gptq, int sym, void *flag_word, void *scratch, size_t scratch_bytes, void *stream);
@@ -287,12 +290,21 @@ int oxq_gptq_gemm(const void *x, int x_dtype, const uint32_t *qweight, const uin
 int oxq_gguf_gemm(int ggml_type, const void *x, int x_dtype, const void *blocks, const void *bias, int bias_dtype,
                   void *y, int y_dtype, int m, int k, int n, void *workspace, size_t workspace_bytes, void *stream);
 
-/* Fp8Linear::forward for m beyond the GEMV range (linear.rs:96-145). Up to 256 tokens, when n % 128 == 0,
- * k % 128 == 0 and the scale blocks are multiples of 128 rows and 64 columns, the bytes are widened inside the
- * tensor-core kernel (same bf16 weights as the dequantization kernel); otherwise slabs are dequantized. */
+/* Fp8Linear::forward for m beyond the GEMV range (linear.rs:96-145). Up to 512 or 768 tokens, when n % 128 == 0,
+ * k % 128 == 0, the scale blocks are multiples of 128 rows and 64 columns and the tensors 16-byte aligned, the bytes are operands of
+ * the tensor-core kernel as they are; otherwise slabs are dequantized to bf16. */
 int oxq_fp8_gemm(const void *x, int x_dtype, const uint8_t *weight, const float *scale_inv, int s_out, int s_in,
                  const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, void *workspace,
                  size_t workspace_bytes, void *stream);
+
+/* The kernel that oxq_fp8_gemm runs on medium batches, E4M3 weights as tensor-core operands and nothing rounded before the f32 sums, with
+ * scratch of its own: oxq_fp8_scratch_bytes(m, k, n, s_out, s_in) bytes (0: not this shape) with any contents, 256-byte aligned, one
+ * per call in flight. s_out, s_in: 0 without scales. flag_word as for oxq_packed4_matmul. OXQ_ERR_UNSUPPORTED for shapes that the
+ * kernel does not take. */
+size_t oxq_fp8_scratch_bytes(int m, int k, int n, int s_out, int s_in);
+int oxq_fp8_matmul(const void *x, int x_dtype, const uint8_t *weight, const float *scale_inv, int s_out, int s_in, const void *bias,
+                   int bias_dtype, void *y, int y_dtype, int m, int k, int n, void *flag_word, void *scratch, size_t scratch_bytes,
+                   void *stream);
 
 /* Mxfp4Linear::forward mul_mm branch (metal_ops.rs:6204-6222). */
 int oxq_mxfp4_gemm(const void *x, int x_dtype, const uint8_t *blocks, const uint8_t *scales, const void *bias,

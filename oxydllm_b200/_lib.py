@@ -43,6 +43,7 @@ SIGNATURES = {
     "oxq_selftest_gemm_wait_expiry": [_vp, ctypes.c_size_t, ctypes.c_int, _vp],
     "oxq_selftest_moe_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_selftest_moe_mx_wait_expiry": [_vp, ctypes.c_size_t, _vp],
+    "oxq_selftest_packed_mx_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_selftest_group_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_selftest_q6k_wait_expiry": [_vp, ctypes.c_size_t, _vp],
     "oxq_awq_gemv_check": [_vp],
@@ -50,11 +51,14 @@ SIGNATURES = {
     "oxq_awq_gemm": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp],
     "oxq_packed4_max_m": [_i, _i, _i],
     "oxq_packed4_scratch_bytes": [_i, _i],
+    "oxq_packed4_full_scratch_bytes": [_i, _i, _i, _i, _i],
     "oxq_packed4_matmul": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _sz, _vp],
     "oxq_awq_gemm_tp": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp],
     "oxq_gptq_gemm": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp],
     "oxq_gguf_gemm": [_i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp, _sz, _vp],
     "oxq_fp8_gemm": [_vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _vp, _sz, _vp],
+    "oxq_fp8_scratch_bytes": [_i, _i, _i, _i, _i],
+    "oxq_fp8_matmul": [_vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _vp, _vp, _sz, _vp],
     "oxq_mxfp4_gemm": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp, _sz, _vp],
     "oxq_gptoss_moe_workspace_bytes": [_i, _i, _i, _i, _i],
     "oxq_gptoss_moe_forward": [_vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, ctypes.c_float,
@@ -73,7 +77,7 @@ SIGNATURES = {
     "oxq_awq_gemm_noalloc_check": [_vp],
 }
 _RESTYPE = {"oxq_status_string": ctypes.c_char_p, "oxq_last_error": ctypes.c_char_p,
-            "oxq_gemm_workspace_bytes": ctypes.c_size_t, "oxq_packed4_scratch_bytes": ctypes.c_size_t, "oxq_decode_workspace_bytes": ctypes.c_size_t, "oxq_gptoss_moe_workspace_bytes": ctypes.c_size_t, "oxq_awq_gemm_noalloc_max_k": ctypes.c_size_t}
+            "oxq_gemm_workspace_bytes": ctypes.c_size_t, "oxq_packed4_scratch_bytes": ctypes.c_size_t, "oxq_packed4_full_scratch_bytes": ctypes.c_size_t, "oxq_fp8_scratch_bytes": ctypes.c_size_t, "oxq_decode_workspace_bytes": ctypes.c_size_t, "oxq_gptoss_moe_workspace_bytes": ctypes.c_size_t, "oxq_awq_gemm_noalloc_max_k": ctypes.c_size_t}
 
 _lib = None
 

@@ -31,6 +31,16 @@ bool group_tc_supported(int m, int k, int n, int group_size, int scales_dtype, c
 int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                     int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
                     cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
+size_t packed_mx_scratch_bytes(int m, int k, int n, int group_size);
+bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
+                         const void *scales);
+int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
+                     int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
+                     cudaStream_t st, int sym, void *scratch, size_t scratch_bytes);
+size_t fp8_mx_scratch_bytes(int m, int k, int n);
+bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
+int fp8_mx_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in, const void *bias,
+                  int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st, void *scratch, size_t scratch_bytes);
 bool fp8_fused_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
 int fp8_fused_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in,
                      const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st,
@@ -154,9 +164,10 @@ OXQ_EXPORT int oxq_gemm_check(const void *workspace, void *stream)
                 "tensor-core kernel: bounded wait %d ran out (1 = ring slot, 2 = tile data, 3 = accumulator ready, "
                 "4 = accumulator free, 5 = meeting of the fold warps; grouped 4-bit kernel: 21 = ring slot, 22 = operand tile, "
                 "23 = packed words, 24 = accumulator ready, 25 = x slot, 26 = x, 27 = operand slot, 28 = slot for scales, "
-                "29 = accumulator free, 30 = scales, 31 = last MMAs; block-scaled kernel of the experts: 61 = weight slot, 62 = row slot, "
-                "63 = accumulator free, 64 = operands or accumulator ready, 65 = packed words, 66 = operand slot, 67 = last MMAs) in a call "
-                "since the last check", flag);
+                "29 = accumulator free, 30 = scales, 31 = last MMAs; block-scaled kernels: 41 = weight slot, 42 = operands or accumulator free, "
+                "43 = packed words, 44 = accumulator ready, 45 = x slot, 47 = operand slot, 49 = accumulator free, 51 = last MMAs, of the "
+                "experts: 61 = weight slot, 62 = row slot, 63 = accumulator free, 64 = operands or accumulator ready, 65 = packed words, "
+                "66 = operand slot, 67 = last MMAs) in a call since the last check", flag);
     return OXQ_OK;
 }
 
@@ -202,6 +213,15 @@ OXQ_EXPORT int oxq_packed4_max_m(int k, int n, int group_size)
                ? group_tc_max_m(n, group_size) : 0;
 }
 
+OXQ_EXPORT size_t oxq_packed4_full_scratch_bytes(int m, int k, int n, int group_size, int gptq)
+{
+    if (m <= 0 || k <= 0 || n <= 0 || n % 128 != 0 || k % 128 != 0 || group_size <= 0) return 0;
+    const size_t own = group_tc_scratch_bytes(m, n);
+    const bool mxs = gptq && packed_mx_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr);
+    const size_t mx = mxs ? packed_mx_scratch_bytes(m, k, n, group_size) : 0;
+    return mx > own ? mx : own;
+}
+
 OXQ_EXPORT size_t oxq_packed4_scratch_bytes(int m, int n)
 {
     return m > 0 && n > 0 && n % 128 == 0 ? group_tc_scratch_bytes(m, n) : 0;
@@ -223,8 +243,8 @@ OXQ_EXPORT int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qw
     if (use_sym) qzeros = nullptr;
     OXQ_REQUIRE(group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales), OXQ_ERR_UNSUPPORTED,
                 "oxq_packed4_matmul: out_features %d, in_features %d, group size %d or the alignment are not served", n, k, group_size);
-    return group_tc_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n,
-                           reinterpret_cast<int *>(flag_word), (cudaStream_t)stream, gptq, use_sym, scratch, scratch_bytes);
+    return packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n,
+                          reinterpret_cast<int *>(flag_word), (cudaStream_t)stream, gptq, use_sym, scratch, scratch_bytes);
 }
 
 // Column block [rows x chunks * 16 bytes] at byte offset col_off of every row of `src` -> the same place in each peer's
@@ -359,6 +379,46 @@ OXQ_EXPORT int oxq_gguf_gemm(int ggml_type, const void *x, int x_dtype, const vo
     });
 }
 
+// E4M3 weights as tensor-core operands (csrc/packed_mx_tc.cu) with scratch of the call's own instead of the workspace's slab, so that calls
+// on different streams only share the flag word.
+static void fp8_block(int n, int k, int s_out, int s_in, int &bo, int &bi)
+{
+    const bool grid = s_out > 0 && s_in > 0;
+    bo = grid ? n / s_out : n;
+    bi = grid ? k / s_in : k;
+}
+
+OXQ_EXPORT size_t oxq_fp8_scratch_bytes(int m, int k, int n, int s_out, int s_in)
+{
+    if (m <= 0 || k <= 0 || n <= 0 || s_out < 0 || s_in < 0 || (s_out && n % s_out) || (s_in && k % s_in)) return 0;
+    int bo, bi;
+    fp8_block(n, k, s_out, s_in, bo, bi);
+    return fp8_mx_supported(m, k, n, bo, bi, nullptr, nullptr, nullptr) ? fp8_mx_scratch_bytes(m, k, n) : 0;
+}
+
+OXQ_EXPORT int oxq_fp8_matmul(const void *x, int x_dtype, const uint8_t *weight, const float *scale_inv, int s_out, int s_in,
+                              const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, void *flag_word, void *scratch,
+                              size_t scratch_bytes, void *stream)
+{
+    clear_error();
+    OXQ_REQUIRE(x && y && weight && flag_word && scratch, OXQ_ERR_NULL, "oxq_fp8_matmul: null pointer");
+    OXQ_REQUIRE(x_dtype == OXQ_BF16, OXQ_ERR_UNSUPPORTED, "oxq_fp8_matmul: activations must be bf16");
+    OXQ_REQUIRE(valid_dtype(y_dtype) && (!bias || valid_dtype(bias_dtype)), OXQ_ERR_UNSUPPORTED, "oxq_fp8_matmul: unsupported dtype");
+    OXQ_REQUIRE(m >= 1 && k > 0 && n > 0, OXQ_ERR_BAD_SHAPE, "oxq_fp8_matmul: non-positive size");
+    OXQ_REQUIRE(!scale_inv || (s_out > 0 && s_in > 0 && n % s_out == 0 && k % s_in == 0), OXQ_ERR_BAD_SHAPE,
+                "block-wise FP8 weight_scale_inv [%d, %d] does not tile weight [%d, %d] evenly", s_out, s_in, n, k);
+    OXQ_REQUIRE(aligned(scratch, 256) && aligned(flag_word, 4), OXQ_ERR_BAD_ALIGN, "oxq_fp8_matmul: scratch must be 256-byte aligned");
+    int bo, bi;
+    fp8_block(n, k, scale_inv ? s_out : 0, scale_inv ? s_in : 0, bo, bi);
+    int rc = OXQ_ERR_UNSUPPORTED;
+    if (fp8_mx_supported(m, k, n, bo, bi, x, weight, scale_inv))
+        rc = fp8_mx_matmul(x, weight, scale_inv, scale_inv ? s_in : 1, bo, bi, bias, bias_dtype, y, y_dtype, m, k, n,
+                           reinterpret_cast<int *>(flag_word), (cudaStream_t)stream, scratch, scratch_bytes);
+    OXQ_REQUIRE(rc != OXQ_ERR_UNSUPPORTED, OXQ_ERR_UNSUPPORTED,
+                "oxq_fp8_matmul: out_features %d, in_features %d, batch %d, the scale blocks, the alignment or the scratch are not served", n, k, m);
+    return rc;
+}
+
 OXQ_EXPORT int oxq_fp8_gemm(const void *x, int x_dtype, const uint8_t *weight, const float *scale_inv, int s_out,
                             int s_in, const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n,
                             void *workspace, size_t workspace_bytes, void *stream)
@@ -377,6 +437,11 @@ OXQ_EXPORT int oxq_fp8_gemm(const void *x, int x_dtype, const uint8_t *weight, c
     int rc = prepare("oxq_fp8_gemm", c, x, x_dtype, bias, bias_dtype, y, y_dtype, m, k, n, workspace, workspace_bytes, stream);
     if (rc) return rc;
     // Up to 256 tokens: widen the bytes inside the tensor-core kernel, no dense copy of the weight.
+    if (fp8_mx_supported(m, k, n, bo, bi, x, weight, scale_inv)) {
+        rc = fp8_mx_matmul(x, weight, scale_inv, scale_inv ? s_in : 1, bo, bi, bias, bias_dtype, y, y_dtype, m, k, n, c.flag, c.st, c.slab,
+                           c.slab_bytes);
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc;
+    }
     if (fp8_fused_supported(m, k, n, bo, bi, x, weight, scale_inv)) {
         rc = fp8_fused_matmul(x, weight, scale_inv, scale_inv ? s_in : 1, bo, bi, bias, bias_dtype, y, y_dtype, m, k, n, c.flag, c.st,
                               c.slab, c.slab_bytes);

@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
         bool ok = true;
         for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, ul++) {
             const int n16 = (ld_produced(p.entries + u / p.tiles_n).y + 15) & ~15;
-            const uint32_t idesc = mx_idesc(MX_E2M1, 2 * n16, false);
+            const uint32_t idesc = mx_idesc(MX_E2M1, 2 * n16);
             const int buf = ul & 1;
             const uint32_t d = tmem_acc + (uint32_t)((2 * buf + me) * MM_ACC_COLS);
             ok = mx_wait(tempty + 8 * buf, (((uint32_t)ul >> 1) & 1u) ^ 1u, p.flag, MM_CODE + 3);

@@ -49,19 +49,12 @@ __device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t (&r)[8])
 
 constexpr int MX_E4M3 = 0, MX_E2M1 = 5;
 // Instruction descriptor: A and B element types, E8M0 scales; bits 29 and 4 up choose the byte of A's and B's scale words.
-__host__ __device__ constexpr uint32_t mx_idesc(int a_type, int n, bool a_mn_major)
+__host__ __device__ constexpr uint32_t mx_idesc(int a_type, int n)
 {
-    return ((uint32_t)a_type << 7) | ((uint32_t)MX_E4M3 << 10) | (a_mn_major ? 1u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) | (1u << 23) |
+    return ((uint32_t)a_type << 7) | ((uint32_t)MX_E4M3 << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) |
            ((128u >> 4) << 24);
 }
 __host__ __device__ constexpr uint32_t mx_idesc_blocks(int a_block, int b_block) { return ((uint32_t)a_block << 29) | ((uint32_t)b_block << 4); }
-
-// 8-bit MN-major A: 128 out features of one input row are one swizzled 128-byte row, eight input rows 1 KB.
-__device__ __forceinline__ uint64_t mx_mn_desc(uint32_t smem_addr)
-{
-    return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
 
 // Eight neighbouring values of a block whose largest magnitude has the bits `amax`: hi and lo as E4M3 bytes, and the block's
 // scale byte (lo's is four less).

@@ -157,6 +157,16 @@ def awq_ffn_gate_up(lin, x2, y, activation: int, tensors=None):
 
 
 def fp8_matmul(lin, s, s_out, s_in, x2, y):
+    m, k, n, w = x2.shape[0], lin.in_features, lin.out_features, lin.weight
+    if not (x2.data_ptr() | w.data_ptr()) & 15:
+        need = int(_lib.entry("oxq_fp8_scratch_bytes")(m, k, n, s_out, s_in))
+        if need:  # scratch of this call's own: calls on several streams do not meet
+            bp, bd = _bias(lin.bias)
+            flag = _flag_words(x2.device)
+            scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
+            _lib.call("oxq_fp8_matmul", x2.data_ptr(), _dt(x2.dtype), w.data_ptr(), _p(s), s_out, s_in, bp, bd, y.data_ptr(), _dt(y.dtype),
+                      m, k, n, flag.data_ptr(), scratch.data_ptr(), need, _st())
+            return
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_fp8_gemm", _p(x2), _dt(x2.dtype), _p(lin.weight), _p(s), s_out, s_in, bp, bd, _p(y), _dt(y.dtype),

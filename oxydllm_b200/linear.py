@@ -23,9 +23,9 @@ from .gemm import _dt
 GEMV_MAX_M = 32
 #: The same for the GPTQ and 8-bit GEMVs (one 8-token chunk of the reference's batched GEMV, linear.rs:461-478).
 PACKED_SIMT_GEMV_MAX_M = 8
-# FP8 layers whose shape the fused unpack + tcgen05 kernel serves leave the GEMV at this batch: 24 us for up to 32 tokens on a
-# 14336 x 4096 layer against 25 / 45 us for the GEMV at 16 / 32.
-AWQ_FUSED_MIN_M = 17
+# FP8 layers whose shape the tcgen05 kernel on E4M3 operands serves leave the GEMV at this batch, us at 8 / 16 tokens there against the
+# GEMV: 14336 x 4096 17.5 / 17.5 against 18 / 25, 4096 x 4096 13.5 / 13.5 against 13.4 / 19.
+AWQ_FUSED_MIN_M = 9
 # GPTQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu): the GEMV does not split k, so it is the
 # faster one on short k only, us at 1 / 2 tokens against the kernel: groups of 128, 1024 x 4096 4.8 / 5.2 against 7.7, 2048 x 6144
 # 7.7 / 8.6 against 10.0, 3072 x 4096 10.3 / 11.7 against 10.9, 4096 x 512 10.7 / 11.9 against 11.2, 2048 x 14336 14.2 / 16.2 against
@@ -448,9 +448,8 @@ class Fp8Linear:
         return out
 
     def gemv_max_m(self, s_out: int, s_in: int) -> int:
-        """Largest batch for the decode GEMV: 16 where the fused widen + tcgen05 kernel serves the layer (out_features % 128,
-        in_features % 128, scale blocks of a multiple of 128 rows and 64 columns; 24 us for up to 32 tokens on a
-        14336 x 4096 layer against 25 / 45 us for the GEMV at 16 / 32), else 32."""
+        """Largest batch for the decode GEMV: 8 where the tcgen05 kernel on E4M3 operands serves the layer (out_features % 128,
+        in_features % 128, scale blocks of a multiple of 128 rows and 64 columns), else 32."""
         n, k = self.out_features, self.in_features
         bo, bi = (n // s_out, k // s_in) if s_out and s_in else (n, k)
         fused = n % 128 == 0 and k % 128 == 0 and bo % 128 == 0 and bi % 64 == 0

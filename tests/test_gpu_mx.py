@@ -1,4 +1,4 @@
-"""The block-scaled tensor-core kernels (MXFP4 experts of small batches): sizes at their edges.
+"""The block-scaled tensor-core kernels (E4M3 weights, MXFP4 experts of small batches): sizes at their edges.
 
 Weights are operands as stored and a bf16 activation is the sum of two E4M3 pieces, exact but for 2^-21 of the largest of its block
 of 32; products are exact and sums are f32. Against 64-bit sums over the exact weights a value is off by a few dozen f32 roundings
@@ -10,12 +10,101 @@ import torch
 
 import oracle
 from oxydllm_b200 import _lib, gemm, synth
+from oxydllm_b200 import linear as L
 
 pytestmark = pytest.mark.gpu
 
 
 def bf16(a):
     return torch.from_numpy(np.ascontiguousarray(a)).to(torch.bfloat16).cuda()
+
+
+def fp8_weights(n, k, s_out, s_in, seed):
+    rng = np.random.default_rng(seed)
+    w8 = rng.integers(0, 256, (n, k), dtype=np.uint8)
+    w8[(w8 & 0x7F) == 0x7F] = 0x08  # no NaN
+    scale = (rng.random((s_out, s_in)) * 0.01 + 1e-3).astype(np.float32)
+    full = np.repeat(np.repeat(scale.astype(np.float64), n // s_out, 0), k // s_in, 1)
+    return w8, scale, oracle.fp8_dequant(w8, None).astype(np.float64) * full
+
+
+def fp8_gemm(w8, scale, xd, n, k, bias=None):
+    m = xd.shape[0]
+    ws = gemm.workspace(n, k, "cuda")
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    wd, sd = torch.from_numpy(w8).cuda(), None if scale is None else torch.from_numpy(scale).cuda()
+    s_out, s_in = (0, 0) if scale is None else scale.shape
+    _lib.call("oxq_fp8_gemm", xd.data_ptr(), _lib.OXQ_BF16, wd.data_ptr(), 0 if sd is None else sd.data_ptr(), s_out, s_in,
+              0 if bias is None else bias.data_ptr(), _lib.OXQ_F32, y.data_ptr(), _lib.OXQ_F32, m, k, n, ws.data_ptr(), ws.numel(), None)
+    gemm.check(ws)
+    return y
+
+
+def close(y, x, w, extra=0.0):
+    ref, mass = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    assert (np.abs(y.double().cpu().numpy() - ref) <= 2.0**-17 * mass + extra).all()
+
+
+# one unit and one tile; blocks of 64 columns (two folds a unit) and of 192 rows' worth; whole rows; 148 tiles and more
+@pytest.mark.parametrize("n,k,s_out,s_in", [(128, 128, 1, 1), (256, 512, 1, 8), (384, 1536, 3, 8), (2048, 512, 16, 4), (19072, 256, 149, 2)])
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 97, 129, 512])
+def test_fp8_block_scaled_matches_64_bit_sums(cuda, m, n, k, s_out, s_in):
+    w8, scale, w = fp8_weights(n, k, s_out, s_in, seed=m + n)
+    x = synth.activations(m, k, seed=m)
+    y = fp8_gemm(w8, scale, bf16(x), n, k)
+    close(y, x, w)
+    assert torch.equal(y, fp8_gemm(w8, scale, bf16(x), n, k))  # parts of a shared tile are added in the order of k
+
+
+def test_fp8_block_scaled_bias_and_no_scale(cuda):
+    n, k, m = 256, 256, 40
+    w8, _, _ = fp8_weights(n, k, 1, 1, seed=1)
+    x = synth.activations(m, k, seed=2)
+    y = fp8_gemm(w8, None, bf16(x), n, k)
+    close(y, x, oracle.fp8_dequant(w8, None).astype(np.float64))
+    bias = torch.arange(n, dtype=torch.float32, device="cuda")
+    assert torch.equal(fp8_gemm(w8, None, bf16(x), n, k, bias), y + bias)
+
+
+def test_fp8_block_scaled_activations_of_every_magnitude(cuda):
+    """Outliers inside a block of 32, tokens far apart in size, zeros, subnormal scales: the pieces are exact or 2^-21 of the block's largest."""
+    n, k, m = 128, 256, 40
+    w8, scale, w = fp8_weights(n, k, 1, 2, seed=3)
+    x = synth.activations(m, k, seed=4)
+    x[1] *= 1e-30
+    x[2] *= 1e30
+    x[3, ::7] *= 3000.0
+    x[4, :128] = 0.0
+    x[5] = 0.0
+    x[6] = 2.0**-120
+    x[7, 5] = 1e4
+    x = synth.bf16_round(x)
+    y = fp8_gemm(w8, scale, bf16(x), n, k)
+    block = np.repeat(np.abs(x).reshape(m, -1, 32).max(-1), 32, -1).astype(np.float64)
+    close(y, x, w, extra=2.0**-20 * block @ np.abs(w).T)
+
+
+def test_fp8_block_scaled_special_values_stay_special(cuda):
+    n, k, m = 128, 256, 20
+    w8, scale, w = fp8_weights(n, k, 1, 2, seed=5)
+    w8[3, 7] = 0x7F
+    x = synth.activations(m, k, seed=6)
+    x[2, 9], x[4, 200] = np.inf, np.nan
+    y = fp8_gemm(w8, scale, bf16(x), n, k).cpu().numpy()
+    assert np.isnan(y[:, 3]).all() and not np.isfinite(y[2]).any() and np.isnan(y[4]).all()
+    rows, cols = [r for r in range(m) if r not in (2, 4)], [c for c in range(n) if c != 3]
+    assert np.isfinite(y[np.ix_(rows, cols)]).all()
+
+
+def test_fp8_block_scaled_kernel_survives_weights_that_never_come(cuda):
+    ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
+    _lib.call("oxq_selftest_packed_mx_wait_expiry", ws.data_ptr(), ws.numel(), None)
+    with pytest.raises(_lib.OxqError, match=r"bounded wait (4[1-9]|5[01]) "):
+        gemm.check(ws)
+    gemm.check(ws)  # reported once
+    w8, scale, w = fp8_weights(128, 128, 1, 1, seed=7)
+    x = synth.activations(20, 128, seed=8)
+    close(fp8_gemm(w8, scale, bf16(x), 128, 128), x, w)
 
 
 # ------------------------------------------------------------------------------------------------------- MXFP4 experts, small batches

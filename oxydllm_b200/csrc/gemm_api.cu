@@ -60,6 +60,11 @@ static int packed4_matmul(const void *x, const uint32_t *qweight, const uint32_t
                           const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base,
                           int ldy, int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes)
 {
+    if (gptq && packed_mx_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales)) {
+        const int rc = packed_mx_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base,
+                                        ldy, flag, st, sym, scratch, scratch_bytes);
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc; // scratch too small for the pieces of x
+    }
     auto run = group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ? group_tc_matmul : awq_fused_matmul;
     return run(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base, ldy, flag, st, gptq,
                sym, scratch, scratch_bytes);

@@ -117,7 +117,8 @@ def packed4_matmul(lin, x2, y, tensors=None):
         flag = _flag_words(x2.device)
     need = lin._scratch_bytes.get(m)
     if need is None:
-        need = lin._scratch_bytes[m] = int(_lib.load().oxq_packed4_scratch_bytes(m, n))
+        need = lin._scratch_bytes[m] = int(_lib.load().oxq_packed4_full_scratch_bytes(m, lin.in_features, n, lin.group_size,
+                                                                                                int(lin.pack_dim == "in")))
     scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
     qw, qz, sc, sc_dt, b, b_dt = tensors or lin._tensors()
     _lib.call("oxq_packed4_matmul", x2.data_ptr(), _dt(x2.dtype), qw, qz, sc, sc_dt, b, b_dt, y.data_ptr(), _dt(y.dtype), m,

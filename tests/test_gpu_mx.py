@@ -107,6 +107,32 @@ def test_fp8_block_scaled_kernel_survives_weights_that_never_come(cuda):
     close(fp8_gemm(w8, scale, bf16(x), 128, 128), x, w)
 
 
+# --------------------------------------------------------------------------------------------------------------- GPTQ, few tokens
+# large layers of groups of 128 and more: whole tiles and shares across their borders (288 and 65 tiles), shares inside tiles (24)
+@pytest.mark.parametrize("k,n,g,sym", [(1152, 36864, 128, False), (1152, 36864, 128, True), (14336, 3072, 512, False), (5120, 8320, 1024, False)])
+@pytest.mark.parametrize("m", [1, 3, 15, 16])
+def test_gptq_few_tokens_match_64_bit_sums(cuda, m, k, n, g, sym):
+    rng = np.random.default_rng(k + m)
+    qw, qz = (rng.integers(0, 2**32, size=s, dtype=np.uint64).astype(np.uint32) for s in ((k // 8, n), (k // g, n // 8)))
+    sc = (np.abs(rng.standard_normal((k // g, n)) * 0.02) / 7 + 1e-4).astype(np.float16)
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (qw, qz, sc)]
+    lin = L.PackedQuantLinear(L.QuantWeight.new_gptq(4, sym, dev[0], None if sym else dev[1], dev[2]))
+    codes = (torch.from_numpy(qw.view(np.int32)).cuda()[:, None] >> torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)[None, :, None]) & 15
+    zeros = 8 if sym else ((dev[1][:, :, None] >> torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)) & 15).reshape(k // g, 1, n) + 1
+    w = ((codes.reshape(k // g, g, n) - zeros) * dev[2].double()[:, None]).reshape(k, n)
+    x = bf16(synth.activations(m, k, seed=m))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    gemm.packed4_matmul(lin, x, y)
+    ref, mass = x.double() @ w, x.double().abs() @ w.abs()
+    assert ((y.double() - ref).abs() <= 2.0**-17 * mass).all()
+    again = torch.empty_like(y)
+    gemm.packed4_matmul(lin, x, again)
+    assert torch.equal(y, again)
+    if lin.gemv_max_m() < m:
+        assert ((lin.forward(x).double() - ref).abs() <= 2.0**-17 * mass + 2.0**-8 * ref.abs()).all()
+    gemm.check(gemm.workspace(n, k, "cuda"))
+
+
 # ------------------------------------------------------------------------------------------------------- MXFP4 experts, small batches
 def experts_layer(experts, hidden, inter, seed):
     from oxydllm_b200 import moe

@@ -20,7 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "tc_common.cuh"
+#include "mx_common.cuh"
 
 namespace oxq {
 
@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
     constexpr int BOX_BYTES = FP8 ? FT_ROWS * FT_BK : FT_BOX_BYTES; // one stage of packed weights
     constexpr int RAW_BYTES = BOX_BYTES + (FP8 ? 0 : 384);          // ring slot: box | zero points | scales | pad
     extern __shared__ unsigned char smem_raw[];
+    pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
     unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
     // operand slots (A tile + x tile) | ring of packed boxes | barriers | tensor-memory address
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
     float *fp8_scales = reinterpret_cast<float *>(tmem_slot + 4); // FP8: the tile's row of the scale grid, one float per k block
     const uint32_t b_off = FT_A_BYTES;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * FT_ROWS;
     const int nk = p.k / FT_BK / p.sk;        // stages of this CTA: split sk of the tile takes stages [sbase, sbase + nk)
     const int sbase = (int)blockIdx.y * nk;
@@ -159,6 +160,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
         tmem_alloc(smem_u32(tmem_slot), (uint32_t)p.tmem_cols);
         tmem_relinquish();
     }
+    // The kernel ahead may have written anything this one reads, and its time must not count as this kernel's waits: only the
+    // barriers and the allocation overlap with it.
+    pdl_wait();
     if (FP8 && warp == 3) {
         const int cnt = p.k / p.block_in;
         for (int i = lane; i < cnt; i += 32)
@@ -169,71 +173,80 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // The single-thread roles run as whole warps with one elected lane at the instruction itself: loop counters, addresses and
+    // descriptors stay in uniform registers (with the loop inside the elected branch an MMA takes 90 clocks to issue).
     if (warp == 0) {
         // ---- TMA, packed words: runs as far ahead of the unpack warps as the ring of boxes allows ------------
-        if (elect_one()) {
-            int r = 0;
-            uint32_t ph = 0;
-            for (int it = 0; it < nk; it++) {
-                if (it >= R && !mbar_wait(rawempty_bar(r), ph ^ 1u, p.flag, 1)) break;
+        const bool leader = elect_one(), with_zeros = !(GPTQ && p.sym);
+        int r = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int it = 0; it < nk && ok; it++) {
+            if (it >= R) ok = mx_wait(rawempty_bar(r), ph ^ 1u, p.flag, 1);
+            if (ok && leader) {
                 const uint32_t dst = base + raw_base + (uint32_t)r * RAW_BYTES;
-                const int qg = (sbase + it) * FT_BK / p.group_size;
+                const int qg = (sbase + it) >> p.gshift;
                 if (FP8) { // the box alone
                     mbar_arrive_expect_tx(rawfull_bar(r), BOX_BYTES);
                     tma_load_2d(dst, &wmap, rawfull_bar(r), (sbase + it) * FT_BK, n0);
-                    FT_TRACE(0, it);
-                    if (++r == R) { r = 0; ph ^= 1u; }
-                    continue;
+                } else {
+                    mbar_arrive_expect_tx(rawfull_bar(r), BOX_BYTES + (with_zeros ? FT_ZERO_BYTES : 0) + FT_SCALE_BYTES);
+                    if (GPTQ) tma_load_2d(dst, &wmap, rawfull_bar(r), n0, (sbase + it) * (FT_BK / 8));
+                    else tma_load_2d(dst, &wmap, rawfull_bar(r), n0 / 8, (sbase + it) * FT_BK);
+                    // the group's zero points and scales travel with the box: a plain load issued by the unpack threads
+                    // would wait a full DRAM round trip per group
+                    if (with_zeros)
+                        bulk_copy_g2s(dst + BOX_BYTES, p.qzeros + (size_t)qg * p.packed_out + n0 / 8, FT_ZERO_BYTES, rawfull_bar(r));
+                    bulk_copy_g2s(dst + BOX_BYTES + FT_ZERO_BYTES, reinterpret_cast<const uint16_t *>(p.scales) + (size_t)qg * p.n + n0,
+                                  FT_SCALE_BYTES, rawfull_bar(r));
                 }
-                const bool with_zeros = !(GPTQ && p.sym);
-                mbar_arrive_expect_tx(rawfull_bar(r), BOX_BYTES + (with_zeros ? FT_ZERO_BYTES : 0) + FT_SCALE_BYTES);
-                if (GPTQ) tma_load_2d(dst, &wmap, rawfull_bar(r), n0, (sbase + it) * (FT_BK / 8));
-                else tma_load_2d(dst, &wmap, rawfull_bar(r), n0 / 8, (sbase + it) * FT_BK);
-                // the group's zero points and scales travel with the box: a plain load issued by the unpack threads
-                // would wait a full DRAM round trip per group
-                if (with_zeros)
-                    bulk_copy_g2s(dst + BOX_BYTES, p.qzeros + (size_t)qg * p.packed_out + n0 / 8, FT_ZERO_BYTES, rawfull_bar(r));
-                bulk_copy_g2s(dst + BOX_BYTES + FT_ZERO_BYTES,
-                              reinterpret_cast<const uint16_t *>(p.scales) + (size_t)qg * p.n + n0, FT_SCALE_BYTES, rawfull_bar(r));
                 FT_TRACE(0, it);
-                if (++r == R) { r = 0; ph ^= 1u; }
             }
+            __syncwarp();
+            if (++r == R) { r = 0; ph ^= 1u; }
         }
     } else if (warp == 2) {
         // ---- TMA, x tiles: one per operand slot, as soon as the MMAs that read the slot have completed --------
-        if (elect_one()) {
-            int s = 0;
-            uint32_t ph = 0;
-            for (int it = 0; it < nk; it++) {
-                if (it >= S && !mbar_wait(empty_bar(s), ph ^ 1u, p.flag, 5)) break;
+        const bool leader = elect_one();
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int it = 0; it < nk && ok; it++) {
+            if (it >= S) ok = mx_wait(empty_bar(s), ph ^ 1u, p.flag, 5);
+            if (ok && leader) {
                 mbar_arrive_expect_tx(xfull_bar(s), (uint32_t)p.mpad * 128u);
                 tma_load_2d(base + (uint32_t)s * p.stage_bytes + b_off, &xmap, xfull_bar(s), (sbase + it) * FT_BK, 0);
-                if (++s == S) { s = 0; ph ^= 1u; }
             }
+            __syncwarp();
+            if (++s == S) { s = 0; ph ^= 1u; }
         }
     } else if (warp == 1) {
         // ---- MMA issue -------------------------------------------------------------------------------
-        if (elect_one()) {
-            const uint32_t idesc = (GPTQ || FP8) ? tc_idesc(FT_ROWS, p.mpad) : ft_idesc(p.mpad);
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int it = 0; it < nk; it++) {
-                ok = mbar_wait(ready_bar(s), ph, p.flag, 2) && mbar_wait(xfull_bar(s), ph, p.flag, 6);
-                if (!ok) break;
-                FT_TRACE(1, it);
+        const bool leader = elect_one();
+        const uint32_t idesc = (GPTQ || FP8) ? tc_idesc(FT_ROWS, p.mpad) : ft_idesc(p.mpad), stage16 = (uint32_t)p.stage_bytes >> 4;
+        const uint64_t da0 = (GPTQ || FP8) ? kmajor_sw128_desc(base) : ft_a_desc(base), db0 = kmajor_sw128_desc(base + b_off);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int it = 0; it < nk && ok; it++) {
+            ok = mx_wait2(ready_bar(s), ph, xfull_bar(s), ph, p.flag, 2);
+            if (ok) {
                 tc_fence_after();
-                const uint32_t slot = base + (uint32_t)s * p.stage_bytes;
-                const uint64_t da = (GPTQ || FP8) ? kmajor_sw128_desc(slot) : ft_a_desc(slot), db = kmajor_sw128_desc(slot + b_off);
+                const uint64_t da = da0 + (uint64_t)(s * stage16), db = db0 + (uint64_t)(s * stage16);
+                if (leader) {
+                    FT_TRACE(1, it);
 #pragma unroll
-                for (int kk = 0; kk < FT_BK / 16; kk++) // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes inside a swizzled K-major row
-                    umma_bf16(tmem_base, da + (uint64_t)kk * ((GPTQ || FP8) ? 2 : (2048 >> 4)), db + 2 * kk, idesc, (it | kk) != 0);
-                umma_commit(empty_bar(s));
-                FT_TRACE(2, it);
-                if (++s == S) { s = 0; ph ^= 1u; }
+                    for (int kk = 0; kk < FT_BK / 16; kk++) // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes inside a swizzled K-major row
+                        umma_bf16(tmem_base, da + (uint64_t)kk * ((GPTQ || FP8) ? 2 : (2048 >> 4)), db + 2 * kk, idesc, (it | kk) != 0);
+                    umma_commit(empty_bar(s));
+                    FT_TRACE(2, it);
+                }
+                __syncwarp();
             }
-            if (ok) umma_commit(acc_bar);
+            if (++s == S) { s = 0; ph ^= 1u; }
         }
+        if (ok && leader) umma_commit(acc_bar);
+        __syncwarp();
     } else if (warp >= 4) {
         // ---- unpack ------------------------------------------------------------------------------------
         // A slot always meets the same team (the slot counts are multiples of the teams' rounds), so every waiter of a
@@ -553,11 +566,17 @@ static int fused_launch(int layout, FusedParams p, const void *x, const void *qw
         else OXQ_CUDA(cudaFuncSetAttribute(awq_fused_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (device < 64) configured[layout][device] = smem;
     }
-    const dim3 grid(tiles, p.sk, 1);
-    if (layout == 1) awq_fused_tc_kernel<1><<<grid, FT_THREADS, smem, st>>>(p, wmap, xmap);
-    else if (layout == 2) awq_fused_tc_kernel<2><<<grid, FT_THREADS, smem, st>>>(p, wmap, xmap);
-    else awq_fused_tc_kernel<0><<<grid, FT_THREADS, smem, st>>>(p, wmap, xmap);
-    OXQ_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles, p.sk, 1);
+    cfg.blockDim = dim3(FT_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    cfg.numAttrs = 0;
+    allow_early_start(attr, cfg.numAttrs);
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, layout == 1 ? awq_fused_tc_kernel<1> : layout == 2 ? awq_fused_tc_kernel<2> : awq_fused_tc_kernel<0>, p, wmap,
+                                xmap));
     return OXQ_OK;
 }
 

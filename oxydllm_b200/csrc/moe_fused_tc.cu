@@ -23,7 +23,7 @@
 // Every wait is bounded and reports through the workspace flag word.
 #include <cuda_bf16.h>
 
-#include "tc_common.cuh"
+#include "mx_common.cuh"
 
 namespace oxq {
 
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
     auto tempty_bar = [&](int b) { return misc + 8u * (2 + b); };
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bars - base) + 8 * MF_NUM_BARS);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n_units = __ldg(p.n_blocks) * p.tiles_n;
     const int nk2 = p.nk2;
 
@@ -131,93 +131,80 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // The single-thread roles run as whole warps with one elected lane at the instruction itself: loop counters, addresses and
+    // descriptors stay in uniform registers (with the loop inside the elected branch an MMA takes 90 clocks to issue).
     if (warp == 0) {
         // ---- TMA, packed nibbles -----------------------------------------------------------------------
-        if (elect_one()) {
-            uint32_t gs = 0, ul = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; ok && u < n_units && !p.test_skip_loads; u += gridDim.x, ul++) {
-                const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
-                const int4 en = __ldg(p.entries + tb);
-                const int rowbase = en.z * p.n + f * MF_ROWS;
-                for (int it = 0; it < nk2; it++, gs++) {
-                    const uint32_t r = gs % MF_RAW_SLOTS;
-                    if (gs >= MF_RAW_SLOTS && !mbar_wait(rawempty_bar(r), ((gs / MF_RAW_SLOTS) & 1u) ^ 1u, p.flag, 1)) { ok = false; break; }
-                    MF_TRACE(0, gs);
-                    if (MF_DBG(8)) { mf_arrive(rawfull_bar(r)); continue; }
+        const bool leader = elect_one();
+        int r = 0;
+        uint32_t ph = 1; // a fresh barrier passes parity 1
+        bool ok = true;
+        for (int u = blockIdx.x; ok && u < n_units && !p.test_skip_loads; u += gridDim.x) {
+            const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
+            const int rowbase = __ldg(p.entries + tb).z * p.n + f * MF_ROWS;
+            for (int it = 0; it < nk2 && ok; it++) {
+                ok = mx_wait(rawempty_bar(r), ph, p.flag, 1);
+                if (ok && leader) {
                     mbar_arrive_expect_tx(rawfull_bar(r), MF_RAW_BYTES);
                     tma_load_2d(raw_base + r * MF_RAW_BYTES, &wmap, rawfull_bar(r), it * (MF_BK / 2), rowbase);
                 }
+                __syncwarp();
+                if (++r == MF_RAW_SLOTS) { r = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 2) {
         // ---- TMA, activation tiles ----------------------------------------------------------------------
-        if (elect_one()) {
-            int xs = 0;
-            uint32_t xph = 0, gx = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x) {
-                const int4 en = __ldg(p.entries + u / p.tiles_n);
-                const int boxes = (en.y + MF_XBOX_ROWS - 1) / MF_XBOX_ROWS;
-                for (int it = 0; it < nk2; it++, gx++) {
-                    if (gx >= MF_SLOTS && !mbar_wait(empty_bar(xs), xph ^ 1u, p.flag, 5)) { ok = false; break; }
+        const bool leader = elect_one();
+        int xs = 0;
+        uint32_t xph = 1;
+        bool ok = true;
+        for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x) {
+            const int4 en = __ldg(p.entries + u / p.tiles_n);
+            const int boxes = (en.y + MF_XBOX_ROWS - 1) / MF_XBOX_ROWS;
+            for (int it = 0; it < nk2 && ok; it++) {
+                ok = mx_wait(empty_bar(xs), xph, p.flag, 5);
+                if (ok && leader) {
                     const uint32_t dst = x_base + (uint32_t)xs * MF_X_BYTES;
-                    MF_TRACE(1, gx);
-                    if (MF_DBG(2)) mf_arrive(full_bar(xs));
-                    else {
                     mbar_arrive_expect_tx(full_bar(xs), (uint32_t)boxes * MF_XBOX_BYTES);
-                    for (int b = 0; b < boxes; b++)
-                        tma_load_2d(dst + (uint32_t)b * MF_XBOX_BYTES, &xmap, full_bar(xs), it * MF_BK, en.x + b * MF_XBOX_ROWS);
-                    }
-                    if (++xs == MF_X_SLOTS) { xs = 0; xph ^= 1u; }
+#pragma unroll
+                    for (int b = 0; b < MF_MAX_TOK / MF_XBOX_ROWS; b++)
+                        if (b < boxes)
+                            tma_load_2d(dst + (uint32_t)b * MF_XBOX_BYTES, &xmap, full_bar(xs), it * MF_BK, en.x + b * MF_XBOX_ROWS);
                 }
+                __syncwarp();
+                if (++xs == MF_X_SLOTS) { xs = 0; xph ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ---- MMA issue ----------------------------------------------------------------------------------
-        if (elect_one()) {
-            // One thread issues every MMA of the CTA, so its instruction count per stage is on the critical path: the loop
-            // runs over all stages of all this CTA's units, four at a time, so that slot, barrier and descriptor addresses are
-            // constants of the unrolled body; one poll (full) and one commit (empty) per stage.
-            int my_units = 0;
-            if ((int)blockIdx.x < n_units) my_units = (n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
-            const uint32_t total = (uint32_t)my_units * (uint32_t)nk2;
-            const uint64_t da0 = kmajor_sw128_desc(base), db0 = kmajor_sw128_desc(x_base);
-            const uint32_t full0 = full_bar(0), empty0 = empty_bar(0);
-            uint32_t ul = 0, idesc = 0, d_tmem = tmem_base, buf = 0;
-            int it = 0;
-            bool ok = true;
-            auto stage = [&](const uint32_t gs, const int j) { // j = gs % MF_SLOTS, a constant after unrolling
-                if (it == 0) { // first stage of a unit
-                    const int u = (int)blockIdx.x + (int)ul * (int)gridDim.x;
-                    const int rows = __ldg(p.entries + u / p.tiles_n).y;
-                    idesc = tc_idesc(MF_ROWS, (rows + 15) & ~15);
-                    buf = ul & 1u;
-                    if (ul >= 2 && !mbar_wait(tempty_bar(buf), ((ul >> 1) & 1u) ^ 1u, p.flag, 8)) { ok = false; return; }
-                    d_tmem = tmem_base + buf * MF_TMEM_BUF;
-                }
-                MF_TRACE(7, gs);
-                if (!mbar_wait(full0 + 8u * j, (gs / MF_SLOTS) & 1u, p.flag, 2)) { ok = false; return; }
-                MF_TRACE(2, gs);
-                tc_fence_after();
-                const uint64_t da = da0 + (uint64_t)(j * (MF_A_BYTES >> 4)), db = db0 + (uint64_t)(j * (MF_X_BYTES >> 4));
-                if (!MF_DBG(4))
+        // One warp issues every MMA of the CTA, so its instruction count per stage is on the critical path: one poll (full) and one
+        // commit (empty) per stage.
+        const bool leader = elect_one();
+        const uint64_t da0 = kmajor_sw128_desc(base), db0 = kmajor_sw128_desc(x_base);
+        int s = 0, ul = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, ul++) {
+            const uint32_t idesc = tc_idesc(MF_ROWS, (__ldg(p.entries + u / p.tiles_n).y + 15) & ~15);
+            const uint32_t buf = (uint32_t)ul & 1u, d_tmem = tmem_base + buf * MF_TMEM_BUF;
+            ok = mx_wait(tempty_bar(buf), (((uint32_t)ul >> 1) & 1u) ^ 1u, p.flag, 8);
+            for (int it = 0; it < nk2 && ok; it++) {
+                ok = mx_wait(full_bar(s), ph, p.flag, 2);
+                if (ok) {
+                    tc_fence_after();
+                    const uint64_t da = da0 + (uint64_t)(s * (MF_A_BYTES >> 4)), db = db0 + (uint64_t)(s * (MF_X_BYTES >> 4));
+                    if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < MF_BK / 16; kk++) // 16 input columns: 32 bytes inside a swizzled K-major row
-                    umma_bf16(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (it | kk) != 0);
-                umma_commit(empty0 + 8u * j);
-                MF_TRACE(3, gs);
-                if (++it == nk2) { // last stage of the unit: the accumulator is complete once these MMAs are
-                    umma_commit(tfull_bar(buf));
-                    it = 0;
-                    ul += 1;
+                        for (int kk = 0; kk < MF_BK / 16; kk++) // 16 input columns: 32 bytes inside a swizzled K-major row
+                            umma_bf16(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (it | kk) != 0);
+                        umma_commit(empty_bar(s));
+                    }
+                    __syncwarp();
                 }
-            };
-            for (uint32_t g = 0; ok && g < total; g += MF_SLOTS) {
-#pragma unroll
-                for (int j = 0; j < MF_SLOTS; j++)
-                    if (ok && g + j < total) stage(g + j, j);
+                if (++s == MF_SLOTS) { s = 0; ph ^= 1u; }
             }
+            if (ok && leader) umma_commit(tfull_bar(buf)); // the accumulator is complete once the unit's MMAs are
+            __syncwarp();
         }
     } else if (warp >= 4 && warp < 4 + MF_UNPACK_WARPS) {
         // ---- unpack ---------------------------------------------------------------------------------------

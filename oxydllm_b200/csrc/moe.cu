@@ -52,9 +52,10 @@ constexpr int MOE_MX_ROWS = 44;
 // One warp per token: f32 softmax over all experts, k rounds of arg-max (ties: lower index),
 // optional renormalisation by the sum of the selected probabilities (moe.rs:472-487).
 __global__ void __launch_bounds__(256)
-moe_route_kernel(const void *__restrict__ logits, int dtype, int tokens, int experts, int top_k, int norm_topk,
-                 int *__restrict__ top_idx, float *__restrict__ top_w)
+moe_route_kernel(const void *logits, int dtype, int tokens, int experts, int top_k, int norm_topk, int *top_idx, float *top_w)
 {
+    pdl_wait(); // the logits are the kernel ahead's, and what is written may still be read
+    pdl_launch_dependents();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= tokens) return;
     constexpr int PER = MOE_MAX_EXPERTS / 32;
@@ -204,16 +205,17 @@ moe_plan_blocks_kernel(const int *__restrict__ counts, int n_exp, int e_lo, int 
 // positions keep the order of the pairs.
 constexpr int MOE_SMALL_PAIRS = 2048;
 __global__ void __launch_bounds__(1024)
-moe_dispatch_small_kernel(const int *__restrict__ top_idx, int pairs, int e_lo, int n_exp, int max_rows, int *__restrict__ counts,
-                          int *__restrict__ offsets, int4 *__restrict__ entries, int *__restrict__ n_blocks, int *__restrict__ perm,
-                          int *__restrict__ inv)
+moe_dispatch_small_kernel(const int *top_idx, int pairs, int e_lo, int n_exp, int max_rows, int *counts, int *offsets, int4 *entries,
+                          int *n_blocks, int *perm, int *inv)
 {
+    pdl_launch_dependents();
     constexpr int ROUNDS = MOE_SMALL_PAIRS / 1024, GROUPS = ROUNDS * 32;
     __shared__ unsigned short cnt[GROUPS][MOE_MAX_EXPERTS]; // hits of an expert in a warp of a round, then the hits before it
     __shared__ int base_s[MOE_MAX_EXPERTS], scratch[64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int groups = (pairs + 31) / 32;
     for (int i = tid; i < groups * MOE_MAX_EXPERTS; i += blockDim.x) (&cnt[0][0])[i] = 0;
+    pdl_wait(); // the routing results are the kernel ahead's
     __syncthreads();
     int id[ROUNDS];
     unsigned peers[ROUNDS];
@@ -318,10 +320,11 @@ moe_gather_kernel(const __nv_bfloat16 *__restrict__ x, const int *__restrict__ p
 // out[t, :] = sum over the token's slots whose expert is in [e_lo, e_hi), in ascending expert id,
 // of w * yp[inv[pair], :] (f32 accumulation, one rounding). Tokens without such a slot get zeros.
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const __nv_bfloat16 *__restrict__ yp, const int *__restrict__ top_idx, const float *__restrict__ top_w,
-                   const int *__restrict__ inv, int tokens, int top_k, int hidden, int e_lo, int e_hi, void *out,
+moe_combine_kernel(const __nv_bfloat16 *yp, const int *top_idx, const float *top_w, const int *inv, int tokens, int top_k, int hidden, int e_lo, int e_hi, void *out,
                    int out_dtype)
 {
+    pdl_launch_dependents();
+    pdl_wait(); // rows and routing results come from kernels ahead
     // a warp takes part `seg` of a token's 16-byte pieces: the slots are put in order once for all of them (once per piece it took
     // 44 us for 4096 tokens of 2880)
     const int chunks = hidden / 8, lane = threadIdx.x & 31, warps = (int)((gridDim.x * blockDim.x) >> 5);
@@ -333,7 +336,7 @@ moe_combine_kernel(const __nv_bfloat16 *__restrict__ yp, const int *__restrict__
 #pragma unroll
         for (int s = 0; s < MOE_MAX_TOPK; s++) {
             order[s] = s;
-            ids[s] = s < top_k ? __ldg(top_idx + (size_t)t * top_k + s) : 0x7FFFFFFF;
+            ids[s] = s < top_k ? ld_produced(top_idx + (size_t)t * top_k + s) : 0x7FFFFFFF;
         }
 #pragma unroll
         for (int a = 1; a < MOE_MAX_TOPK; a++) // insertion sort by expert id (k <= 8), in registers
@@ -352,8 +355,8 @@ moe_combine_kernel(const __nv_bfloat16 *__restrict__ yp, const int *__restrict__
         for (int s = 0; s < MOE_MAX_TOPK; s++) {
             use[s] = s < top_k && ids[s] >= e_lo && ids[s] < e_hi;
             const size_t pair = (size_t)t * top_k + order[s];
-            pos[s] = !use[s] ? 0 : inv ? __ldg(inv + pair) : (int)pair;
-            wv[s] = use[s] ? __ldg(top_w + pair) : 0.0f;
+            pos[s] = !use[s] ? 0 : inv ? ld_produced(inv + pair) : (int)pair;
+            wv[s] = use[s] ? ld_produced(top_w + pair) : 0.0f;
         }
         for (int c = seg * 32 + lane; c < chunks; c += segs * 32) {
         uint4 rows[MOE_MAX_TOPK];
@@ -417,6 +420,19 @@ moe_expand_ids_kernel(const int *__restrict__ counts, int groups, int n_local, i
         const int a = start_s[g], b = start_s[g + 1], e = lo + g % n_local;
         for (int i = a + lane; i < b; i += 32) ids[i] = e;
     }
+}
+
+// Launch that may start while the kernel ahead is still running: the kernel waits for it itself.
+template <typename... P, typename... A> static cudaError_t launch_early(void (*kern)(P...), int grid, int block, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    allow_early_start(attr, cfg.numAttrs);
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -531,8 +547,8 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     const int pairs = tokens * top_k;
 
     if (given_ids) moe_assign_kernel<<<ceil_div(tokens, 256), 256, 0, st>>>(given_ids, tokens, top_idx, top_w);
-    else moe_route_kernel<<<ceil_div(tokens * 32, 256), 256, 0, st>>>(router_logits, logits_dtype, tokens, num_experts, top_k,
-                                                                      norm_topk, top_idx, top_w);
+    else OXQ_CUDA(launch_early(moe_route_kernel, ceil_div(tokens * 32, 256), 256, st, router_logits, logits_dtype, tokens, num_experts, top_k,
+                               norm_topk, top_idx, top_w));
     const int a_rows = pairs + 128;
     // Both projections through the kernel that unpacks the MXFP4 blocks inside the tensor-core loop, where it takes the shapes:
     // no dequantized slab, one launch per projection over all experts.
@@ -554,17 +570,16 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
         rc = mxfp4_gemv_batched(x, 1, dn_blocks, dn_scales, dn_bias, bias_dtype, top_idx, pairs, expert_lo, expert_hi, xs,
                                 OXQ_BF16, inter, hidden, st, gu, limit);
         if (rc) return rc;
-        moe_combine_kernel<<<ceil_div(tokens * ceil_div(hidden / 8, 32) * 32, 256), 256, 0, st>>>(xs, top_idx, top_w, nullptr, tokens, top_k,
-                                                                                 hidden, expert_lo, expert_hi, out, out_dtype);
-        OXQ_LAUNCH_CHECK("moe_combine_kernel");
+        OXQ_CUDA(launch_early(moe_combine_kernel, ceil_div(tokens * ceil_div(hidden / 8, 32) * 32, 256), 256, st, xs, top_idx, top_w, nullptr,
+                              tokens, top_k, hidden, expert_lo, expert_hi, out, out_dtype));
         return OXQ_OK;
     }
     // the grouped kernel's table of token blocks goes where the m-tile table of the dense path would (same capacity bound);
     // grp_beg[0] then holds the number of blocks
     const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows();
     if ((fused || mx) && pairs <= MOE_SMALL_PAIRS) {
-        moe_dispatch_small_kernel<<<1, 1024, 0, st>>>(top_idx, pairs, expert_lo, n_exp, block_rows, counts, offsets, entries,
-                                                      grp_beg, perm, inv);
+        OXQ_CUDA(launch_early(moe_dispatch_small_kernel, 1, 1024, st, top_idx, pairs, expert_lo, n_exp, block_rows, counts, offsets, entries,
+                              grp_beg, perm, inv));
     } else {
         moe_count_kernel<<<n_exp, 1024, 0, st>>>(top_idx, pairs, expert_lo, counts);
         if (fused || mx) moe_plan_blocks_kernel<<<1, MOE_MAX_EXPERTS, 0, st>>>(counts, n_exp, expert_lo, block_rows, offsets,
@@ -585,8 +600,8 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
         rc = moe_mx_grouped(sb, sb + L.h_scales, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg, dn_bias,
                             bias_dtype, xs, hidden, 0, limit, flag, st);
         if (rc) return rc;
-        moe_combine_kernel<<<sm_count() * 8, 256, 0, st>>>(xs, top_idx, top_w, inv, tokens, top_k, hidden, expert_lo, expert_hi, out, out_dtype);
-        OXQ_LAUNCH_CHECK("moe_combine_kernel");
+        OXQ_CUDA(launch_early(moe_combine_kernel, sm_count() * 8, 256, st, xs, top_idx, top_w, inv, tokens, top_k, hidden, expert_lo, expert_hi,
+                              out, out_dtype));
         return OXQ_OK;
     }
     moe_gather_kernel<<<sm_count() * 8, 256, 0, st>>>((const __nv_bfloat16 *)x, perm, offsets + n_exp, top_k, hidden, xs);

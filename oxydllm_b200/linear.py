@@ -26,6 +26,8 @@ PACKED_SIMT_GEMV_MAX_M = 8
 # FP8 layers whose shape the tcgen05 kernel on E4M3 operands serves leave the GEMV at this batch, us at 8 / 16 tokens there against the
 # GEMV: 14336 x 4096 17.5 / 17.5 against 18 / 25, 4096 x 4096 13.5 / 13.5 against 13.4 / 19.
 AWQ_FUSED_MIN_M = 9
+#: The same for calls that the kernel cannot take for their alignment.
+FP8_UNALIGNED_GEMV_MAX_M = 16
 # GPTQ 4-bit layers that the grouped unpack + tcgen05 kernel serves (csrc/group_tc.cu): the GEMV does not split k, so it is the
 # faster one on short k only, us at 1 / 2 tokens against the kernel: groups of 128, 1024 x 4096 4.8 / 5.2 against 7.7, 2048 x 6144
 # 7.7 / 8.6 against 10.0, 3072 x 4096 10.3 / 11.7 against 10.9, 4096 x 512 10.7 / 11.9 against 11.2, 2048 x 14336 14.2 / 16.2 against
@@ -460,7 +462,10 @@ class Fp8Linear:
         x2, lead, m = _flatten_x(x, self.in_features, "Fp8Linear")
         _require_cuda(x2, self.weight, self.bias)
         y = x2.new_empty((m, self.out_features))
-        if m and m <= self.gemv_max_m(s_out, s_in):
+        few = self.gemv_max_m(s_out, s_in)
+        if m > few and m <= FP8_UNALIGNED_GEMV_MAX_M and (x2.data_ptr() | self.weight.data_ptr()) & 15:
+            few = FP8_UNALIGNED_GEMV_MAX_M  # the GEMV takes x on any 8 bytes
+        if m and m <= few:
             b = self.bias
             _lib.call("oxq_fp8_gemv", x2.data_ptr(), _dt(x2.dtype), self.weight.data_ptr(), _p(s), s_out, s_in, _p(b),
                       _dt(b.dtype) if b is not None else 0, y.data_ptr(), _dt(y.dtype), m, self.in_features,

@@ -96,6 +96,19 @@ def test_fp8_block_scaled_special_values_stay_special(cuda):
     assert np.isfinite(y[np.ix_(rows, cols)]).all()
 
 
+@pytest.mark.parametrize("m", [9, 16])
+def test_fp8_decode_takes_x_on_any_8_bytes(cuda, m):
+    n, k = 256, 512
+    w8, scale, w = fp8_weights(n, k, 2, 4, seed=m)
+    lin = L.Fp8Linear(torch.from_numpy(w8).cuda(), torch.from_numpy(scale).cuda())
+    x = synth.activations(m, k, seed=m)
+    room = torch.zeros(m * k + 4, dtype=torch.bfloat16, device="cuda")
+    room[4:] = bf16(x).reshape(-1)
+    ref = x.astype(np.float64) @ w.T
+    for xd in (bf16(x), room[4:].view(m, k)):
+        close(lin.forward(xd), x, w, extra=2.0**-8 * np.abs(ref))
+
+
 def test_fp8_block_scaled_kernel_survives_weights_that_never_come(cuda):
     ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
     _lib.call("oxq_selftest_packed_mx_wait_expiry", ws.data_ptr(), ws.numel(), None)

@@ -1,18 +1,18 @@
-// AWQ / GPTQ W4A16 (above the batches that group_tc.cu takes) and FP8 matmul of up to 256 tokens with the dequantization
+// AWQ / GPTQ W4A16 matmul of up to 256 tokens (above the batches that group_tc.cu takes) with the dequantization
 // fused into the tensor-core kernel: the packed words are read from HBM once and no dense copy of the weight is ever written.
 //
 // One CTA owns 128 out features and walks k in stages of 64 input rows:
-//   warp 0 (one lane)   TMA: boxes of packed words (64 rows x 16 words, 4 KB) into a ring of up to 32 slots,
+//   warp 0              TMA: boxes of packed words (64 rows x 16 words, 4 KB) into a ring of up to 32 slots,
 //                       as far ahead as the ring allows: this ring is what is in flight from HBM;
-//   warp 2 (one lane)   TMA: the stage's tile of x ([tokens, 64] bf16, 128-byte swizzle) into one of the
-//                       two or four operand slots;
+//   warp 2              TMA: the stage's tile of x ([tokens, 64] bf16, 128-byte swizzle) into one of the
+//                       four operand slots;
 //   warps 4..19         unpack, two teams of eight warps taking rounds of two stages in turn: every thread
 //                       turns four packed words per stage into 4 x 8 bf16 weights, the same bits the dequantization kernel
 //                       writes ((128 + q) - (128 + z) exactly in bf16, times the scale with one
 //                       rounding: see split_scales), and stores each word's
 //                       eight out features, which are neighbours in memory in the MN-major operand
 //                       layout, with one 16-byte store;
-//   warp 1 (one lane)   tcgen05.mma kind::f16, A = weights (bf16, MN-major, 128-byte swizzle: 64 out
+//   warp 1              tcgen05.mma kind::f16, A = weights (bf16, MN-major, 128-byte swizzle: 64 out
 //                       features x 8 input rows per 1 KB atom), B = x (bf16, K-major), D[128, tokens] f32
 //                       in tensor memory for the whole of k; a commit per stage frees the slots;
 //   warps 4..19         epilogue: accumulator rows (out features) -> registers -> + bias -> y[token, n].
@@ -61,8 +61,6 @@ struct FusedParams {
     int stages, raw_slots, stage_bytes, tmem_cols;
     int gshift;        // log2(stages per quantization group)
     int sym;           // GPTQ: no stored zero points (zero + 1 = 8)
-    const float *scale_inv; // FP8: scale grid [s_out, s_in] or null
-    int s_in, block_out, block_in;
     int col_base, ldy; // y column of out feature 0 and the row pitch of y in elements
     int *flag;
     int sk;              // k splits per tile (grid y); > 1: partial tiles meet in `partials`, the last CTA of a tile adds them
@@ -109,17 +107,11 @@ __device__ __forceinline__ uint32_t ft_idesc(int n)
 // GPTQ = true:  GPTQ 4-bit layout (a word is eight input rows of one out feature, nibble i = row 8 r + i; A operand
 //               K-major: the word becomes one 16-byte chunk of the out feature's 128-byte row). The box is 8 packed
 //               rows x 128 words; the zero point is the stored nibble + 1, or 8 for symmetric weights (awq.rs:540-590).
-// LAYOUT 2: FP8 E4M3 [n, k] row-major with an f32 scale grid (Fp8Linear, linear.rs:96-145). The box is 128 rows x
-//               64 bytes, already K-major; every thread widens 32 bytes of one row (e4m3 -> f16 exactly in hardware,
-//               -> f32, times the block's scale, one rounding to bf16: the bits of the dequantization kernel). The
-//               tile's row of the scale grid is copied to shared memory once.
-template <int LAYOUT>
+template <bool GPTQ>
 __global__ void __launch_bounds__(FT_THREADS, 1)
     awq_fused_tc_kernel(const FusedParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
 {
-    constexpr bool GPTQ = LAYOUT == 1, FP8 = LAYOUT == 2;
-    constexpr int BOX_BYTES = FP8 ? FT_ROWS * FT_BK : FT_BOX_BYTES; // one stage of packed weights
-    constexpr int RAW_BYTES = BOX_BYTES + (FP8 ? 0 : 384);          // ring slot: box | zero points | scales | pad
+    constexpr int BOX_BYTES = FT_BOX_BYTES, RAW_BYTES = BOX_BYTES + 384; // one stage of packed weights; ring slot: box | zero points | scales | pad
     extern __shared__ unsigned char smem_raw[];
     pdl_launch_dependents();
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
@@ -135,7 +127,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
     auto empty_bar = [&](int s) { return bars + 8u * (2 * FT_MAX_RAW + 2 * FT_MAX_STAGES + s); };
     const uint32_t acc_bar = bars + 8u * (2 * FT_MAX_RAW + 3 * FT_MAX_STAGES);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + raw_base + (size_t)R * RAW_BYTES + 8 * FT_NUM_BARS);
-    float *fp8_scales = reinterpret_cast<float *>(tmem_slot + 4); // FP8: the tile's row of the scale grid, one float per k block
     const uint32_t b_off = FT_A_BYTES;
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -163,11 +154,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
     // The kernel ahead may have written anything this one reads, and its time must not count as this kernel's waits: only the
     // barriers and the allocation overlap with it.
     pdl_wait();
-    if (FP8 && warp == 3) {
-        const int cnt = p.k / p.block_in;
-        for (int i = lane; i < cnt; i += 32)
-            fp8_scales[i] = p.scale_inv ? __ldg(p.scale_inv + (size_t)(n0 / p.block_out) * p.s_in + i) : 1.0f;
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -186,20 +172,15 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
             if (ok && leader) {
                 const uint32_t dst = base + raw_base + (uint32_t)r * RAW_BYTES;
                 const int qg = (sbase + it) >> p.gshift;
-                if (FP8) { // the box alone
-                    mbar_arrive_expect_tx(rawfull_bar(r), BOX_BYTES);
-                    tma_load_2d(dst, &wmap, rawfull_bar(r), (sbase + it) * FT_BK, n0);
-                } else {
-                    mbar_arrive_expect_tx(rawfull_bar(r), BOX_BYTES + (with_zeros ? FT_ZERO_BYTES : 0) + FT_SCALE_BYTES);
-                    if (GPTQ) tma_load_2d(dst, &wmap, rawfull_bar(r), n0, (sbase + it) * (FT_BK / 8));
-                    else tma_load_2d(dst, &wmap, rawfull_bar(r), n0 / 8, (sbase + it) * FT_BK);
-                    // the group's zero points and scales travel with the box: a plain load issued by the unpack threads
-                    // would wait a full DRAM round trip per group
-                    if (with_zeros)
-                        bulk_copy_g2s(dst + BOX_BYTES, p.qzeros + (size_t)qg * p.packed_out + n0 / 8, FT_ZERO_BYTES, rawfull_bar(r));
-                    bulk_copy_g2s(dst + BOX_BYTES + FT_ZERO_BYTES, reinterpret_cast<const uint16_t *>(p.scales) + (size_t)qg * p.n + n0,
-                                  FT_SCALE_BYTES, rawfull_bar(r));
-                }
+                mbar_arrive_expect_tx(rawfull_bar(r), BOX_BYTES + (with_zeros ? FT_ZERO_BYTES : 0) + FT_SCALE_BYTES);
+                if (GPTQ) tma_load_2d(dst, &wmap, rawfull_bar(r), n0, (sbase + it) * (FT_BK / 8));
+                else tma_load_2d(dst, &wmap, rawfull_bar(r), n0 / 8, (sbase + it) * FT_BK);
+                // the group's zero points and scales travel with the box: a plain load issued by the unpack threads
+                // would wait a full DRAM round trip per group
+                if (with_zeros)
+                    bulk_copy_g2s(dst + BOX_BYTES, p.qzeros + (size_t)qg * p.packed_out + n0 / 8, FT_ZERO_BYTES, rawfull_bar(r));
+                bulk_copy_g2s(dst + BOX_BYTES + FT_ZERO_BYTES, reinterpret_cast<const uint16_t *>(p.scales) + (size_t)qg * p.n + n0,
+                              FT_SCALE_BYTES, rawfull_bar(r));
                 FT_TRACE(0, it);
             }
             __syncwarp();
@@ -223,8 +204,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
     } else if (warp == 1) {
         // ---- MMA issue -------------------------------------------------------------------------------
         const bool leader = elect_one();
-        const uint32_t idesc = (GPTQ || FP8) ? tc_idesc(FT_ROWS, p.mpad) : ft_idesc(p.mpad), stage16 = (uint32_t)p.stage_bytes >> 4;
-        const uint64_t da0 = (GPTQ || FP8) ? kmajor_sw128_desc(base) : ft_a_desc(base), db0 = kmajor_sw128_desc(base + b_off);
+        const uint32_t idesc = GPTQ ? tc_idesc(FT_ROWS, p.mpad) : ft_idesc(p.mpad), stage16 = (uint32_t)p.stage_bytes >> 4;
+        const uint64_t da0 = GPTQ ? kmajor_sw128_desc(base) : ft_a_desc(base), db0 = kmajor_sw128_desc(base + b_off);
         int s = 0;
         uint32_t ph = 0;
         bool ok = true;
@@ -237,7 +218,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
                     FT_TRACE(1, it);
 #pragma unroll
                     for (int kk = 0; kk < FT_BK / 16; kk++) // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes inside a swizzled K-major row
-                        umma_bf16(tmem_base, da + (uint64_t)kk * ((GPTQ || FP8) ? 2 : (2048 >> 4)), db + 2 * kk, idesc, (it | kk) != 0);
+                        umma_bf16(tmem_base, da + (uint64_t)kk * (GPTQ ? 2 : (2048 >> 4)), db + 2 * kk, idesc, (it | kk) != 0);
                     umma_commit(empty_bar(s));
                     FT_TRACE(2, it);
                 }
@@ -314,35 +295,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
 #pragma unroll
             for (int h = 0; h < FT_ROUND; h++) {
                 const uint32_t ring = (uint32_t)(r + h) * RAW_BYTES;
-                if constexpr (FP8) {
-                    // thread = (row, half): 32 bytes of the row -> 32 bf16 = four 16-byte chunks of the K-major row
-                    const int row = ut >> 1, half = ut & 1;
-                    const float sc = fp8_scales[((sbase + it0 + h) * FT_BK) / p.block_in];
-                    const uint32_t src = base + raw_base + ring + (uint32_t)row * 64u + (uint32_t)half * 32u;
-                    const uint4 lo = lds128(src), hi = lds128(src + 16);
-                    const uint32_t wv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-                    const uint32_t dst = base + (my_s + h) * p.stage_bytes + (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u;
-#pragma unroll
-                    for (int c4 = 0; c4 < 4; c4++) {
-                        uint4 o;
-                        uint32_t *ov = reinterpret_cast<uint32_t *>(&o);
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            uint32_t h01, h23;
-                            asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, lo;\n\t"
-                                "cvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
-                                : "=r"(h01), "=r"(h23)
-                                : "r"(wv[2 * c4 + q]));
-                            const float2 f01 = __half22float2(*reinterpret_cast<const __half2 *>(&h01));
-                            const float2 f23 = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
-                            const __nv_bfloat162 b01 = __floats2bfloat162_rn(__fmul_rn(sc, f01.x), __fmul_rn(sc, f01.y));
-                            const __nv_bfloat162 b23 = __floats2bfloat162_rn(__fmul_rn(sc, f23.x), __fmul_rn(sc, f23.y));
-                            ov[2 * q] = *reinterpret_cast<const uint32_t *>(&b01);
-                            ov[2 * q + 1] = *reinterpret_cast<const uint32_t *>(&b23);
-                        }
-                        sts128(dst + ((((uint32_t)(half * 4 + c4)) ^ (uint32_t)(row & 7)) << 4), o);
-                    }
-                } else {
                 uint32_t w[FT_WORDS];
 #pragma unroll
                 for (int i = 0; i < FT_WORDS; i++) w[i] = lds32(box_addr0 + ring + i * ROW_STEP * (GPTQ ? 512 : 64));
@@ -393,7 +345,6 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
                     } else
                     sts128(a_addr + (my_s + h) * p.stage_bytes + i * ROW_STEP * 128, o);
                 }
-                } // layouts with packed words
             }
             if (ut == 0) FT_TRACE(4, it0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
@@ -500,23 +451,19 @@ bool awq_fused_supported(int m, int k, int n, int group_size, int scales_dtype, 
            (scales_dtype == OXQ_F16 || scales_dtype == OXQ_BF16) && aligned(x, 16) && aligned(qweight, 16) && aligned(scales, 16);
 }
 
-// layout 0 = AWQ, 1 = GPTQ 4-bit (sym: no stored zero points), 2 = FP8 E4M3 (qweight = the bytes, scale_inv / s_in /
-// block_out / block_in describe the scale grid; qzeros, scales unused).
-static int fused_launch(int layout, FusedParams p, const void *x, const void *qweight, int m, int k, int n, cudaStream_t st,
+// sym: GPTQ without stored zero points.
+static int fused_launch(bool gptq, FusedParams p, const void *x, const void *qweight, int m, int k, int n, cudaStream_t st,
                         void *scratch, size_t scratch_bytes)
 {
-    const int raw_bytes = layout == 2 ? FT_ROWS * FT_BK : FT_BOX_BYTES + 384;
+    const int raw_bytes = FT_BOX_BYTES + 384;
     p.mpad = (m + 15) / 16 * 16;
     p.stage_bytes = FT_A_BYTES + p.mpad * 128;
-    const int fixed = 1024 + 8 * FT_NUM_BARS + 16 + (layout == 2 ? (k / p.block_in) * 4 + 16 : 0);
+    const int fixed = 1024 + 8 * FT_NUM_BARS + 16;
     const int nk = k / FT_BK;
-    // FP8: eight operand slots (each team two rounds ahead of the MMAs) when that leaves at least eight boxes in flight,
-    // else four; the rest of shared memory is the ring of packed boxes, a multiple of four. (FP8, 32 tokens on a
-    // 14336 x 4096 layer: 29.2 us with four slots, 24.3 us with eight; AWQ, bound by its unpack arithmetic: no change.)
+    // Four operand slots, the rest of shared memory is the ring of packed boxes, a multiple of four (eight slots and a shallower ring:
+    // GPTQ, 64 tokens, 31.4 -> 33.3 us).
     constexpr int UNIT = FT_ROUND * FT_TEAMS;
-    p.stages = layout == 2 ? 2 * UNIT : UNIT; // the 4-bit layouts lose a little to the shallower ring (GPTQ, 64 tokens: 31.4 -> 33.3 us)
-    if ((FT_SMEM_BUDGET - fixed - p.stages * p.stage_bytes) / raw_bytes < 8) p.stages = UNIT;
-    if (const char *env = tuning_env("OXQ_AWQ_FUSED_STAGES")) p.stages = atoi(env) == UNIT ? UNIT : p.stages;
+    p.stages = UNIT;
     p.raw_slots = (FT_SMEM_BUDGET - fixed - p.stages * p.stage_bytes) / raw_bytes / UNIT * UNIT;
     if (p.raw_slots > FT_MAX_RAW) p.raw_slots = FT_MAX_RAW;
     if (const char *env = tuning_env("OXQ_AWQ_FUSED_RAW")) p.raw_slots = atoi(env) < p.raw_slots ? atoi(env) : p.raw_slots;
@@ -543,11 +490,8 @@ static int fused_launch(int layout, FusedParams p, const void *x, const void *qw
 
     CUtensorMap wmap, xmap;
     CUresult r;
-    if (layout == 1)
+    if (gptq)
         r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, (uint64_t)n, (uint64_t)k / 8, (uint64_t)n * 4, 128, FT_BK / 8,
-                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    else if (layout == 2)
-        r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, qweight, (uint64_t)k, (uint64_t)n, (uint64_t)k, FT_BK, FT_ROWS,
                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     else
         r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, (uint64_t)p.packed_out, (uint64_t)k, (uint64_t)p.packed_out * 4,
@@ -557,14 +501,13 @@ static int fused_launch(int layout, FusedParams p, const void *x, const void *qw
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (x) failed with CUresult %d", (int)r);
 
-    static size_t configured[3][64] = {};
+    static size_t configured[2][64] = {};
     int device = 0;
     OXQ_CUDA(cudaGetDevice(&device));
-    if (device >= 64 || configured[layout][device] < smem) {
-        if (layout == 1) OXQ_CUDA(cudaFuncSetAttribute(awq_fused_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else if (layout == 2) OXQ_CUDA(cudaFuncSetAttribute(awq_fused_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else OXQ_CUDA(cudaFuncSetAttribute(awq_fused_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (device < 64) configured[layout][device] = smem;
+    auto kern = gptq ? awq_fused_tc_kernel<true> : awq_fused_tc_kernel<false>;
+    if (device >= 64 || configured[gptq][device] < smem) {
+        OXQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (device < 64) configured[gptq][device] = smem;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles, p.sk, 1);
@@ -575,8 +518,7 @@ static int fused_launch(int layout, FusedParams p, const void *x, const void *qw
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, layout == 1 ? awq_fused_tc_kernel<1> : layout == 2 ? awq_fused_tc_kernel<2> : awq_fused_tc_kernel<0>, p, wmap,
-                                xmap));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, kern, p, wmap, xmap));
     return OXQ_OK;
 }
 
@@ -592,28 +534,7 @@ int awq_fused_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
     p.sym = (gptq && (sym || qzeros == nullptr)) ? 1 : 0;
     p.gshift = 0;
     while ((FT_BK << p.gshift) < group_size) p.gshift += 1;
-    p.block_in = FT_BK; p.block_out = FT_ROWS; p.s_in = 1;
-    return fused_launch(gptq ? 1 : 0, p, x, qweight, m, k, n, st, scratch, scratch_bytes);
-}
-
-bool fp8_fused_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv)
-{
-    if (const char *env = tuning_env("OXQ_AWQ_FUSED"))
-        if (env[0] == '0') return false;
-    return m >= 1 && m <= FT_MAX_M && n % FT_ROWS == 0 && k % (FT_BK * FT_ROUND) == 0 && block_out % FT_ROWS == 0 &&
-           block_in % FT_BK == 0 && k / block_in <= 1024 && aligned(x, 16) && aligned(weight, 16) && aligned(scale_inv, 4);
-}
-
-int fp8_fused_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in,
-                     const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st,
-                     void *scratch, size_t scratch_bytes)
-{
-    FusedParams p = {};
-    p.bias = bias; p.y = y; p.bias_dtype = bias_dtype; p.y_dtype = y_dtype;
-    p.m = m; p.k = k; p.n = n; p.group_size = FT_BK; p.packed_out = n / 8;
-    p.col_base = 0; p.ldy = n; p.flag = flag;
-    p.scale_inv = scale_inv; p.s_in = s_in; p.block_out = block_out; p.block_in = block_in;
-    return fused_launch(2, p, x, weight, m, k, n, st, scratch, scratch_bytes);
+    return fused_launch(gptq != 0, p, x, qweight, m, k, n, st, scratch, scratch_bytes);
 }
 
 } // namespace oxq

@@ -41,10 +41,6 @@ size_t fp8_mx_scratch_bytes(int m, int k, int n);
 bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
 int fp8_mx_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in, const void *bias,
                   int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st, void *scratch, size_t scratch_bytes);
-bool fp8_fused_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
-int fp8_fused_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in,
-                     const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st,
-                     void *scratch, size_t scratch_bytes);
 int awq_fused_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy,
                      int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
@@ -441,15 +437,10 @@ OXQ_EXPORT int oxq_fp8_gemm(const void *x, int x_dtype, const uint8_t *weight, c
     GemmCommon c;
     int rc = prepare("oxq_fp8_gemm", c, x, x_dtype, bias, bias_dtype, y, y_dtype, m, k, n, workspace, workspace_bytes, stream);
     if (rc) return rc;
-    // Up to 256 tokens: widen the bytes inside the tensor-core kernel, no dense copy of the weight.
+    // Medium batches: the bytes are operands of the tensor-core kernel, no dense copy of the weight.
     if (fp8_mx_supported(m, k, n, bo, bi, x, weight, scale_inv)) {
         rc = fp8_mx_matmul(x, weight, scale_inv, scale_inv ? s_in : 1, bo, bi, bias, bias_dtype, y, y_dtype, m, k, n, c.flag, c.st, c.slab,
                            c.slab_bytes);
-        if (rc != OXQ_ERR_UNSUPPORTED) return rc;
-    }
-    if (fp8_fused_supported(m, k, n, bo, bi, x, weight, scale_inv)) {
-        rc = fp8_fused_matmul(x, weight, scale_inv, scale_inv ? s_in : 1, bo, bi, bias, bias_dtype, y, y_dtype, m, k, n, c.flag, c.st,
-                              c.slab, c.slab_bytes);
         if (rc != OXQ_ERR_UNSUPPORTED) return rc;
     }
     return run_slabs(c, [&](int n_off, int cnt) {

@@ -27,13 +27,15 @@
 // MMA's reads; sixteen unpack warps instead of eight were 2 to 5 % slower. Issue slots are 47 %, DRAM 22 % busy (4096 x 28672).
 // Beside that about 7 us a launch go into filling the pipeline, which begins when the kernel ahead has finished, and putting shared
 // tiles together. Measured in a graph, us at 16 / 77 / 128 tokens (the kernel with scaled bf16 weights before it): 4096 x 4096
-// 12 / 17 / 20 (14 / 19 / 22), 4096 x 28672 32 / 50 / 56 (55 / 59 / 61), 14336 x 4096 22 / 30 / 34 (28 / 34 / 38).
+// 11.4 / 16.6 / 19.4 (14 / 19 / 22), 4096 x 28672 30.5 / 48 / 54 (55 / 59 / 61), 14336 x 4096 21 / 28 / 32 (28 / 34 / 38). A poll costs
+// about 120 clocks even where the phase is complete, so the polls of a stage are under way together (one after the other: 11.8 / 17.0 /
+// 19.7, 32.1 / 51 / 56, 21.8 / 30 / 34).
 #include <atomic>
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "tc_common.cuh"
+#include "mx_common.cuh"
 
 namespace oxq {
 
@@ -100,16 +102,6 @@ __device__ __forceinline__ void gt_sts128(uint32_t addr, const uint4 &v)
 {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ void gt_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Bounded wait of a whole warp; the outcome is the same in all lanes (and known to be, so that the loops around it stay uniform).
-__device__ __forceinline__ bool gt_wait(uint32_t bar, uint32_t parity, int *flag, int code)
-{
-    if (__all_sync(0xFFFFFFFFu, mbar_test(bar, parity))) return true;
-    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, flag, code));
-}
 __device__ __forceinline__ uint32_t gt_and_or(uint32_t v, uint32_t mask, uint32_t magic) // (v & mask) | magic
 {
     uint32_t r;
@@ -128,14 +120,6 @@ __device__ __forceinline__ uint64_t gt_mn_desc(uint32_t smem_addr)
     return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-__device__ __forceinline__ void gt_tmem_ld8(uint32_t taddr, uint32_t (&r)[8])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-
 // Units [begin, end) of CTA `i`, and the CTA that holds unit u.
 __host__ __device__ __forceinline__ long long gt_share(long long total, int ctas, long long i) { return total * i / ctas; }
 __host__ __device__ __forceinline__ int gt_owner(long long total, int ctas, long long u) { return (int)(((u + 1) * ctas - 1) / total); }
@@ -216,15 +200,15 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         const int unit_folds = GT_UNIT / p.fold_rows, zgroups = GPTQ && p.sym ? 0 : unit_folds;
         const uint32_t bytes = (uint32_t)(GT_UNIT * GT_ROW_BYTES + zgroups * GT_ZERO_BYTES);
         int n0 = first_tile / p.token_blocks * GT_ROWS, tb = first_tile % p.token_blocks;
-        int uk = first_unit, r = 0, c = 0, fold = 0;
-        uint32_t ph = 0, cph = 0;
+        int uk = first_unit, r = 0, c = 0;
+        uint32_t ph = 1, cph = 1; // a fresh barrier passes parity 1
         bool ok = true;
         for (int it = 0; it < nunits && ok; it++) {
             const int k0 = uk * GT_UNIT;
             const size_t group = (size_t)(k0 >> p.gshift);
             const uint32_t *zsrc = p.qzeros + group * p.packed_out + n0 / 8;
             const uint16_t *ssrc = reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0;
-            if (it >= R) ok = gt_wait(rawempty + 8 * r, ph ^ 1u, p.flag, GT_CODE + 1);
+            ok = mx_wait2(rawempty + 8 * r, ph, scempty + 8 * c, cph, p.flag, GT_CODE + 1); // the ring slot, and the first fold's scales
             if (ok && leader && !p.test_skip_loads) {
                 const uint32_t dst = raw_base + (uint32_t)(r * GT_RAW_BYTES), bar = rawfull + 8 * r;
                 mbar_arrive_expect_tx(bar, bytes);
@@ -235,8 +219,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             }
             __syncwarp();
             if (++r == R) { r = 0; ph ^= 1u; }
-            for (int f = 0; f < unit_folds && ok; f++, fold++) { // unit_folds > 1: groups shorter than a unit, one fold each
-                if (fold >= GT_SC) ok = gt_wait(scempty + 8 * c, cph ^ 1u, p.flag, GT_CODE + 8);
+            for (int f = 0; f < unit_folds && ok; f++) { // unit_folds > 1: groups shorter than a unit, one fold each
+                if (f > 0) ok = mx_wait(scempty + 8 * c, cph, p.flag, GT_CODE + 8);
                 if (ok && leader && !p.test_skip_loads) {
                     mbar_arrive_expect_tx(scfull + 8 * c, GT_SC_BYTES);
                     bulk_copy_g2s(sc_base + c * GT_SC_BYTES, ssrc + (size_t)f * p.n, GT_SC_BYTES, scfull + 8 * c);
@@ -253,17 +237,21 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         // ---- x, a stage at a time, as soon as the MMAs that read the slot have completed -----------------------------
         const bool leader = elect_one();
         int tb = first_tile % p.token_blocks, k0 = first_unit * GT_UNIT, x = 0;
-        uint32_t ph = 0;
+        uint32_t ph = 1; // a fresh barrier passes parity 1
         bool ok = true;
-        for (int it = 0; it < nstages && ok; it++) {
-            if (it >= X) ok = gt_wait(xempty + 8 * x, ph ^ 1u, p.flag, GT_CODE + 5);
+        const int step = X == GT_MAX_X ? 2 : 1; // slots per poll; with few of them both would wait for the later one
+        for (int it = 0; it < nstages && ok; it += step) {
+            ok = mx_wait2(xempty + 8 * x, ph, xempty + 8 * (x + step - 1), ph, p.flag, GT_CODE + 5);
             if (ok && leader) {
-                mbar_arrive_expect_tx(xfull + 8 * x, (uint32_t)p.x_bytes);
-                tma_load_2d(x_base + (uint32_t)(x * p.x_bytes), &xmap, xfull + 8 * x, k0, tb * p.mpad);
+                for (int j = 0; j < step; j++) {
+                    mbar_arrive_expect_tx(xfull + 8 * (x + j), (uint32_t)p.x_bytes);
+                    tma_load_2d(x_base + (uint32_t)((x + j) * p.x_bytes), &xmap, xfull + 8 * (x + j), k0 + j * GT_BK, tb * p.mpad);
+                }
             }
             __syncwarp();
-            if (++x == X) { x = 0; ph ^= 1u; }
-            k0 += GT_BK;
+            x += step;
+            if (x == X) { x = 0; ph ^= 1u; }
+            k0 += step * GT_BK;
             if (k0 == G * GT_UNIT) {
                 k0 = 0;
                 if (++tb == p.token_blocks) tb = 0;
@@ -271,9 +259,9 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
         }
         // The commits of the last stages arrive here asynchronously: the CTA stays until they have.
         for (int left = min(S, nstages), q = nstages - left; left > 0 && ok; left--, q++)
-            ok = gt_wait(empty + 8 * (q % S), (uint32_t)(q / S) & 1u, p.flag, GT_CODE + 11);
+            ok = mx_wait(empty + 8 * (q % S), (uint32_t)(q / S) & 1u, p.flag, GT_CODE + 11);
         for (int left = min(X, nstages), q = nstages - left; left > 0 && ok; left--, q++)
-            ok = gt_wait(xempty + 8 * (q % X), (uint32_t)(q / X) & 1u, p.flag, GT_CODE + 11);
+            ok = mx_wait(xempty + 8 * (q % X), (uint32_t)(q / X) & 1u, p.flag, GT_CODE + 11);
     } else if (warp < 4) {
         // ---- MMA issue: warps 1 and 3 take the units in turn -------------------------------------------------------
         const bool leader = elect_one();
@@ -290,9 +278,9 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                 bool ok = true;
 #pragma unroll
                 for (int st = 0; st < US; st++) {
-                    ok = ok && gt_wait(xfull + 8 * x, xph, p.flag, GT_CODE + 6) && gt_wait(full + 8 * s, ph, p.flag, GT_CODE + 2);
                     const bool first = FM == 4 || st == 0, last = FM == 4 || st == US - 1; // of the buffer's stages
-                    if (first && ok) ok = gt_wait(accempty + 8 * a, aph, p.flag, GT_CODE + 9);
+                    if (ok && first) ok = mx_wait3(xfull + 8 * x, xph, full + 8 * s, ph, accempty + 8 * a, aph, p.flag, GT_CODE + 2);
+                    else if (ok) ok = mx_wait2(xfull + 8 * x, xph, full + 8 * s, ph, p.flag, GT_CODE + 2);
                     if (ok) {
                         tc_fence_after();
                         const uint32_t d = tmem_base + (uint32_t)(a * p.acc_cols);
@@ -302,15 +290,12 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                             for (int kk = 0; kk < 4; kk++) // 16 input rows: two 1 KB atoms of an MN-major A, 32 bytes of a K-major row
                                 umma_bf16(d, da + (uint64_t)(kk * (GPTQ ? 2 : (2048 >> 4))), db + 2 * kk, idesc, !(first && kk == 0));
                             if (last) umma_commit(accfull + 8 * a);
+                            umma_commit(empty + 8 * s);
+                            umma_commit(xempty + 8 * x);
                         }
                         __syncwarp();
                     }
                     if (last) a++;
-                    if (ok && leader) {
-                        umma_commit(empty + 8 * s);
-                        umma_commit(xempty + 8 * x);
-                    }
-                    __syncwarp();
                     if (++s == S) { s = 0; ph ^= 1u; }
                     if (++x == X) { x = 0; xph ^= 1u; }
                 }
@@ -404,8 +389,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
             __syncwarp();
             if (lane == 0) {
-                gt_arrive(full + 8 * s);
-                gt_arrive(rawempty + 8 * r);
+                mx_arrive(full + 8 * s);
+                mx_arrive(rawempty + 8 * r);
             }
             s += GT_TEAMS;
             if (s >= S) { s -= S; ph ^= 1u; }
@@ -431,7 +416,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
             for (int i = 0; i < NCH * 8; i++) tot[i] = 0.0f;
 #pragma unroll 1
             for (int f = 0; f < folds && ok; f++) {
-                ok = gt_wait(scfull + 8 * c, cph, p.flag, GT_CODE + 10) && gt_wait(accfull + 8 * a, aph, p.flag, GT_CODE + 4);
+                ok = mx_wait2(scfull + 8 * c, cph, accfull + 8 * a, aph, p.flag, GT_CODE + 4);
                 if (!ok) break;
                 tc_fence_after();
                 uint16_t sraw;
@@ -443,7 +428,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                     uint32_t rr[B][8];
 #pragma unroll
                     for (int i = 0; i < B; i++)
-                        if ((i0 + i) * 8 < mh) gt_tmem_ld8(tlane + (uint32_t)(a * p.acc_cols + (i0 + i) * 8), rr[i]);
+                        if ((i0 + i) * 8 < mh) tmem_ld_x8(tlane + (uint32_t)(a * p.acc_cols + (i0 + i) * 8), rr[i]);
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < B; i++)
@@ -456,8 +441,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    gt_arrive(accempty + 8 * a);
-                    gt_arrive(scempty + 8 * c);
+                    mx_arrive(accempty + 8 * a);
+                    mx_arrive(scempty + 8 * c);
                 }
                 if (++a == GT_ACC) { a = 0; aph ^= 1u; }
                 if (++c == GT_SC) { c = 0; cph ^= 1u; }

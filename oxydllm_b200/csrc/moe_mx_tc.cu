@@ -10,9 +10,12 @@
 //   warp 0        TMA: packed nibbles (128 out features x 64 bytes), as far ahead as the ring allows;
 //   warp 2        TMA: both pieces of the block's rows for a stage;
 //   warps 1, 3    tcgen05.mma kind::mxf8f6f4 and the copies of the block scales to tensor memory, even and odd stages;
-//   warps 4..11   two teams of four warps, even and odd stages: eight packed bytes (16 codes) to each 16-byte chunk of the operand
+//   warps 4..15   three teams of four warps that take the stages in turn: eight packed bytes (16 codes) to each 16-byte chunk of the operand
 //                 row, as the MMA wants 4-bit elements, and the block scales of weights and rows in tensor-memory order;
-//   warps 12..15  epilogue of the previous unit while the next one accumulates: bias, clamped SwiGLU (even row gate, odd row up).
+//   warps 16..19  epilogue of the previous unit while the next one accumulates: bias, clamped SwiGLU (even row gate, odd row up).
+//
+// What bounds it: a stage's chain of polls, operand rows and arrival in a team. us a layer at 13 / 50 / 200 / 340 tokens, 32 experts of
+// 2880 x 2880, with two teams 122 / 148 / 167 / 194, with three 108 / 130 / 144 / 170; packed weights alone take 66 from HBM.
 #include "mx_common.cuh"
 
 namespace oxq {
@@ -20,7 +23,7 @@ namespace oxq {
 constexpr int MM_ROWS = 128;                 // out features per unit
 constexpr int MM_BK = 128;                   // input columns per stage
 constexpr int MM_MAX_TOK = 48;               // rows of a token block
-constexpr int MM_TEAMS = 2, MM_TEAM_WARPS = 4, MM_UNPACK_WARPS = MM_TEAMS * MM_TEAM_WARPS, MM_EPI_WARPS = 4;
+constexpr int MM_TEAMS = 3, MM_ISSUERS = 2, MM_TEAM_WARPS = 4, MM_UNPACK_WARPS = MM_TEAMS * MM_TEAM_WARPS, MM_EPI_WARPS = 4;
 constexpr int MM_EPI_WARP0 = 4 + MM_UNPACK_WARPS;
 constexpr int MM_THREADS = (MM_EPI_WARP0 + MM_EPI_WARPS) * 32;
 constexpr int MM_SLOTS = 6, MM_RAW = 6;
@@ -33,7 +36,7 @@ constexpr int MM_NUM_BARS = 2 * MM_RAW + 2 * MM_SLOTS + 4;
 constexpr size_t MM_SMEM = 1024 + (size_t)MM_SLOTS * (MM_A_BYTES + MM_X_BYTES + 2 * MM_SF_BYTES) + MM_RAW * MM_RAW_BYTES + 8 * MM_NUM_BARS + 16;
 constexpr int MM_CODE = 60;                  // wait codes 61 .. 67: oxq_gemm_check names them
 static_assert(MM_SMEM <= 227 * 1024, "operand slots and the ring must fit one CTA's shared memory");
-static_assert(MM_SLOTS % MM_TEAMS == 0 && MM_RAW % MM_TEAMS == 0, "a slot always meets the same team and issuer: a parity wait tells a phase from the next one only");
+static_assert(MM_SLOTS % MM_TEAMS == 0 && MM_SLOTS % MM_ISSUERS == 0 && MM_RAW % MM_TEAMS == 0 && MM_EPI_WARP0 % 4 == 0, "a slot always meets the same team and issuer: a parity wait tells a phase from the next one only");
 static_assert(8 * MM_SLOTS <= MM_SF_COLS && MM_SF_COLS + 4 * MM_ACC_COLS <= 512, "tensor memory");
 
 struct MoeMxParams {
@@ -229,7 +232,8 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
         const uint32_t dst0 = (row >> 3) * 1024u + (row & 7) * 128u, c0 = ((2 * q) ^ (row & 7)) << 4, c1 = ((2 * q + 1) ^ (row & 7)) << 4;
         const uint32_t sf_at = (uint32_t)(ut & 31) * 16u + (uint32_t)(ut >> 5) * 4u; // row ut's scales
         int s = 0;
-        uint32_t ph = 0, parity = 0;
+        uint32_t ph = 0;
+        int turn = 0; // of the stages counted so far
         bool ok = true, reused = false; // reused: the slots have been used before
         static_assert(MM_SLOTS == MM_RAW, "one slot counter for both rings");
         for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x) {
@@ -243,7 +247,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
             const int lo_row = n16 + ut;
             const uint32_t lo_at = (uint32_t)(lo_row & 31) * 16u + (uint32_t)(lo_row >> 5) * 4u;
             for (int it = 0; it < T && ok; it++) {
-                if (parity == (uint32_t)team) {
+                if (turn == team) {
                     // the scales come straight from L2 and are asked for ahead of the polls, which hide their latency; past the last
                     // out feature and past k: 1.0 (never used there, but no NaN)
                     uint32_t sa = 0x7F7F7F7Fu;
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
                         mx_arrive(rawempty + 8 * s);
                     }
                 }
-                parity ^= 1u;
+                if (++turn == MM_TEAMS) turn = 0;
                 if (++s == MM_SLOTS) { s = 0; ph ^= 1u; reused = true; }
             }
         }

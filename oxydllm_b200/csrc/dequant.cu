@@ -234,6 +234,8 @@ awq_slab16_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__r
                        const void *__restrict__ scales, int scales_dtype, __nv_bfloat16 *__restrict__ out, int k,
                        int n_cnt, int group_size, int n_full, int n_off, int vec_ok, int row_mul, int row_add)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     __shared__ __align__(16) uint32_t raw[128][32];
     __shared__ __align__(16) unsigned char stage[2][32 * 272];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -326,6 +328,8 @@ __global__ void __launch_bounds__(256)
 fp8_slab16_bf16_kernel(const uint8_t *__restrict__ weight, const float *__restrict__ scale_inv, int s_in, int block_out,
                        int block_in, __nv_bfloat16 *__restrict__ out, int n_cnt, int k, int row_off)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     const int c16 = blockIdx.x * 256 + threadIdx.x;
     if (c16 * 16 >= k) return;
     const int kb = scale_inv ? (c16 * 16) / block_in : 0;
@@ -430,6 +434,8 @@ template <bool FIVE>
 __global__ void __launch_bounds__(256)
 q4k_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_groups)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_groups;
          idx += (size_t)gridDim.x * blockDim.x) {
         const size_t sb = idx >> 2;
@@ -498,6 +504,8 @@ __device__ __forceinline__ float small_int_f32(int v) // |v| < 2^22
 __global__ void __launch_bounds__(256)
 q80_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_blocks)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_blocks;
          idx += (size_t)gridDim.x * blockDim.x) {
         const unsigned short *h = reinterpret_cast<const unsigned short *>(blocks + idx * 34);
@@ -521,6 +529,8 @@ template <int V>
 __global__ void __launch_bounds__(256)
 q40_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_blocks)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     constexpr bool HAS_MIN = V == 1 || V == 3, FIVE = V >= 2;
     constexpr int BLK = 18 + 2 * V, QH = (HAS_MIN ? 4 : 2) / 2, QS = (2 + (HAS_MIN ? 2 : 0) + (FIVE ? 4 : 0)) / 2; // halfword offsets
     constexpr int OFF = V == 0 ? 8 : V == 2 ? 16 : 0;
@@ -556,6 +566,8 @@ q40_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
 __global__ void __launch_bounds__(256)
 q6k_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_groups)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_groups;
          idx += (size_t)gridDim.x * blockDim.x) {
         const size_t sb = idx >> 4;
@@ -591,6 +603,8 @@ gptq4_slab_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__r
                        const void *__restrict__ scales, int scales_dtype, __nv_bfloat16 *__restrict__ out, int k,
                        int n_cnt, int group_size, int sym, int n_full, int n_off)
 {
+    pdl_wait(); // the slab may still be read by the kernel ahead
+    pdl_launch_dependents();
     __shared__ uint32_t tile[32][33];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int c0 = blockIdx.x * 32, kp0 = blockIdx.y * 32, kwords = k >> 3;
@@ -644,8 +658,8 @@ int awq_dequant_rows_bf16(const uint32_t *qweight, const uint32_t *qzeros, const
     if (group_size % 16 == 0 && k % 16 == 0 && n_off % 8 == 0 && n_cnt % 8 == 0 && aligned(out, 16)) {
         const int vec_ok = aligned(qweight, 16) && (n_full >> 3) % 4 == 0 && (n_off >> 3) % 4 == 0;
         dim3 grid(ceil_div(n_cnt, 256), ceil_div(k, 128));
-        awq_slab16_bf16_kernel<<<grid, 256, 0, st>>>(qweight, qzeros, scales, scales_dtype, out, k, n_cnt, group_size,
-                                                     n_full, n_off, vec_ok, row_mul, row_add);
+        OXQ_CUDA(launch_early(awq_slab16_bf16_kernel, grid, 256, st, qweight, qzeros, scales, scales_dtype, out, k, n_cnt, group_size,
+                                                     n_full, n_off, vec_ok, row_mul, row_add));
         OXQ_LAUNCH_CHECK("awq_slab16_bf16_kernel");
         return OXQ_OK;
     }
@@ -662,8 +676,8 @@ int gptq_dequant_rows_bf16(const uint32_t *qweight, const uint32_t *qzeros, cons
 {
     if (bits == 4 && group_size % 8 == 0 && k % 8 == 0 && aligned(out, 16)) {
         dim3 grid(ceil_div(n_cnt, 32), ceil_div(k / 8, 32));
-        gptq4_slab_bf16_kernel<<<grid, 256, 0, st>>>(qweight, qzeros, scales, scales_dtype, out, k, n_cnt, group_size, sym,
-                                                     n_full, n_off);
+        OXQ_CUDA(launch_early(gptq4_slab_bf16_kernel, grid, 256, st, qweight, qzeros, scales, scales_dtype, out, k, n_cnt, group_size, sym,
+                                                     n_full, n_off));
         OXQ_LAUNCH_CHECK("gptq4_slab_bf16_kernel");
         return OXQ_OK;
     }
@@ -691,20 +705,20 @@ int gguf_dequant_rows_bf16(int ggml_type, const uint8_t *blocks, __nv_bfloat16 *
     const size_t total = (size_t)n_cnt * k;
     if ((ggml_type == OXQ_GGML_Q4_K || ggml_type == OXQ_GGML_Q5_K) && aligned(b, 16) && aligned(out, 16)) {
         const size_t groups = total / 64;
-        if (ggml_type == OXQ_GGML_Q5_K) q4k_slab_bf16_kernel<true><<<grid_for(groups), 256, 0, st>>>(b, out, groups);
-        else q4k_slab_bf16_kernel<false><<<grid_for(groups), 256, 0, st>>>(b, out, groups);
+        if (ggml_type == OXQ_GGML_Q5_K) OXQ_CUDA(launch_early(q4k_slab_bf16_kernel<true>, grid_for(groups), 256, st, b, out, groups));
+        else OXQ_CUDA(launch_early(q4k_slab_bf16_kernel<false>, grid_for(groups), 256, st, b, out, groups));
         OXQ_LAUNCH_CHECK("q4k_slab_bf16_kernel");
         return OXQ_OK;
     }
     if (aligned(b, 2) && aligned(out, 16) && ggml_type != OXQ_GGML_Q4_K && ggml_type != OXQ_GGML_Q5_K &&
         ggml_type != OXQ_GGML_Q2_K && ggml_type != OXQ_GGML_Q3_K) {
         const int g32 = grid_for(total / 32);
-        if (ggml_type == OXQ_GGML_Q8_0) q80_slab_bf16_kernel<<<g32, 256, 0, st>>>(b, out, total / 32);
-        else if (ggml_type == OXQ_GGML_Q4_0) q40_slab_bf16_kernel<0><<<g32, 256, 0, st>>>(b, out, total / 32);
-        else if (ggml_type == OXQ_GGML_Q4_1) q40_slab_bf16_kernel<1><<<g32, 256, 0, st>>>(b, out, total / 32);
-        else if (ggml_type == OXQ_GGML_Q5_0) q40_slab_bf16_kernel<2><<<g32, 256, 0, st>>>(b, out, total / 32);
-        else if (ggml_type == OXQ_GGML_Q5_1) q40_slab_bf16_kernel<3><<<g32, 256, 0, st>>>(b, out, total / 32);
-        else q6k_slab_bf16_kernel<<<grid_for(total / 16), 256, 0, st>>>(b, out, total / 16);
+        if (ggml_type == OXQ_GGML_Q8_0) OXQ_CUDA(launch_early(q80_slab_bf16_kernel, g32, 256, st, b, out, total / 32));
+        else if (ggml_type == OXQ_GGML_Q4_0) OXQ_CUDA(launch_early(q40_slab_bf16_kernel<0>, g32, 256, st, b, out, total / 32));
+        else if (ggml_type == OXQ_GGML_Q4_1) OXQ_CUDA(launch_early(q40_slab_bf16_kernel<1>, g32, 256, st, b, out, total / 32));
+        else if (ggml_type == OXQ_GGML_Q5_0) OXQ_CUDA(launch_early(q40_slab_bf16_kernel<2>, g32, 256, st, b, out, total / 32));
+        else if (ggml_type == OXQ_GGML_Q5_1) OXQ_CUDA(launch_early(q40_slab_bf16_kernel<3>, g32, 256, st, b, out, total / 32));
+        else OXQ_CUDA(launch_early(q6k_slab_bf16_kernel, grid_for(total / 16), 256, st, b, out, total / 16));
         OXQ_LAUNCH_CHECK("gguf slab kernel");
         return OXQ_OK;
     }
@@ -726,8 +740,8 @@ int fp8_dequant_rows_bf16(const uint8_t *weight, const float *scale_inv, int s_i
 {
     if (k % 16 == 0 && block_in % 16 == 0 && aligned(weight, 16) && aligned(out, 16)) {
         dim3 grid(ceil_div(k / 16, 256), ceil_div(n_cnt, FP8_SLAB_ROWS));
-        fp8_slab16_bf16_kernel<<<grid, 256, 0, st>>>(weight + (size_t)n_off * k, scale_inv, s_in, block_out, block_in,
-                                                     out, n_cnt, k, n_off);
+        OXQ_CUDA(launch_early(fp8_slab16_bf16_kernel, grid, 256, st, weight + (size_t)n_off * k, scale_inv, s_in, block_out, block_in,
+                                                     out, n_cnt, k, n_off));
         OXQ_LAUNCH_CHECK("fp8_slab16_bf16_kernel");
         return OXQ_OK;
     }

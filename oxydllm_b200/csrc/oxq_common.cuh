@@ -156,4 +156,19 @@ inline void allow_early_start(cudaLaunchAttribute *attrs, unsigned int &count)
     count += 1;
 }
 
+#ifdef __CUDACC__
+// Launch that may start while the kernel ahead is still running: the kernel waits for it itself.
+template <typename... P, typename... A> inline cudaError_t launch_early(void (*kern)(P...), dim3 grid, int block, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    allow_early_start(attr, cfg.numAttrs);
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+#endif
+
 } // namespace oxq

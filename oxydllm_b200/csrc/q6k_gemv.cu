@@ -217,8 +217,9 @@ __global__ void __launch_bounds__(256, 3) q6k_gemv_kernel(const Q6kGemvParams p)
 // pitch of 420 words puts the 8 rows x 4 words of a fragment read on distinct banks. 6-bit values become f16 1024 + v, minus 1056
 // exactly, so no sums of x are needed; a step's accumulators are multiplied by d * scale in f32.
 //
-// What bounds it: instruction issue, 5.2 per weight (9.1 in the kernel above, which stages x in every CTA, loads every
-// word of a misaligned super-block as halfwords from global memory and folds sums of x).
+// What bounds it: instruction issue (the kernel above spends 9.1 per weight: it stages x in every CTA, loads every word of a misaligned
+// super-block as halfwords from global memory and folds sums of x; 5.2 here while every lane converted all scales of its rows and
+// read x 8 bytes at a time). 128256 x 4096 at 3 / 8 tokens 105.9 / 113.0 us then, 90.9 / 95.2 now.
 constexpr int Q6W_ROWS = 16, Q6W_SB = 8, Q6W_ENGINES = 2, Q6W_WARPS = 8;
 constexpr int Q6W_ROW_BYTES = Q6W_SB * 210, Q6W_STAGE_BYTES = Q6W_ROWS * Q6W_ROW_BYTES;
 constexpr int Q6W_THREADS = Q6W_ENGINES * (Q6W_WARPS + 1) * 32, Q6W_MAX_RING = 4;
@@ -256,45 +257,57 @@ __device__ __forceinline__ uint32_t q6w_sub(uint32_t v) // f16 pairs 1024 + v ->
     return *reinterpret_cast<const uint32_t *>(&d);
 }
 
-// One super-block of 16 rows (this lane: rows g and g + 8, words 4c of every piece) times x.
+// One super-block of 16 rows at blk (this lane: rows g and g + 8, words 4c of every piece) times x, in halves of 128 weights: the 8
+// scales a row has there are multiplied by d once, by the lane that loads them, and handed to the row's other lanes through `scr`
+// (this warp's 16 x 8 floats; a row's two sets of four change places in every other group of four rows, so that the 8 rows of a
+// 16-byte read take distinct banks). Every lane used to work out all 32 for itself, 6 of about 40 instructions per 16 weights of k.
 template <bool ODD>
-__device__ __forceinline__ void q6w_superblock(float (&tot)[4], uint32_t blk0, uint32_t blk1, int c, const __half *xp, int xmul)
+__device__ __forceinline__ void q6w_superblock(float (&tot)[4], uint32_t blk, float *scr, int lane, const __half *xp, int xmul)
 {
-    uint32_t sc0[4], sc1[4];
+    const int g = lane >> 2, c = lane & 3;
+    const uint32_t blk0 = blk + (uint32_t)(g * Q6W_ROW_BYTES), blk1 = blk0 + 8 * Q6W_ROW_BYTES;
+    const uint32_t mine = blk + (uint32_t)((lane >> 1) * Q6W_ROW_BYTES); // the row whose scales this lane converts
+    uint16_t dr;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dr) : "r"(mine + 208));
+    const float d = __half2float(__ushort_as_half(dr));
+    float *put = scr + (lane >> 1) * 8 + 2 * (lane & 1);
+    const int put_s = 4 * ((lane >> 3) & 1), get_s = 4 * ((g >> 2) & 1);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        sc0[i] = q6w_word<ODD>(blk0 + 192 + 4 * i) ^ 0x80808080u; // signed byte + 128
-        sc1[i] = q6w_word<ODD>(blk1 + 192 + 4 * i) ^ 0x80808080u;
-    }
-    uint16_t dr0, dr1;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dr0) : "r"(blk0 + 208));
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(dr1) : "r"(blk1 + 208));
-    const float d0 = __half2float(__ushort_as_half(dr0)), d1 = __half2float(__ushort_as_half(dr1));
+    for (int h = 0; h < 2; h++) {
+        const uint32_t sc = q6w_word<ODD>(mine + 192 + 8 * h + 4 * (lane & 1)) ^ 0x80808080u; // signed byte + 128
+        float f[4]; // sixteens 2 (lane & 1) + {0, 0, 1, 1} of the pairs, s = 0, 1, 0, 1
 #pragma unroll
-    for (int combo = 0; combo < 4; combo++) {
-        const int h = combo >> 1, s = combo & 1;
-        const uint32_t at = 64 * h + 16 * s + 4 * c, hat = 128 + 32 * h + 16 * s + 4 * c;
-        const uint32_t le0 = q6w_word<ODD>(blk0 + at), lo0 = q6w_word<ODD>(blk0 + at + 32), qh0 = q6w_word<ODD>(blk0 + hat);
-        const uint32_t le1 = q6w_word<ODD>(blk1 + at), lo1 = q6w_word<ODD>(blk1 + at + 32), qh1 = q6w_word<ODD>(blk1 + hat);
+        for (int i = 0; i < 4; i++) f[i] = d * (__uint_as_float(__byte_perm(sc, 0x4B000000u, 0x7440 + i)) - 8388736.0f); // 2^23 + 128
+        __syncwarp(); // the half before, or the tile's partial sums, have been read
+        *reinterpret_cast<float2 *>(put + put_s) = make_float2(f[0], f[2]);
+        *reinterpret_cast<float2 *>(put + (put_s ^ 4)) = make_float2(f[1], f[3]);
+        __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t l0 = (q & 1) ? lo0 : le0, l1 = (q & 1) ? lo1 : le1;
-            const uint32_t b0 = (q == 0 ? qh0 << 4 : q == 1 ? qh0 << 2 : q == 2 ? qh0 : qh0 >> 2) & 0x30303030u;
-            const uint32_t b1 = (q == 0 ? qh1 << 4 : q == 1 ? qh1 << 2 : q == 2 ? qh1 : qh1 >> 2) & 0x30303030u;
-            const uint32_t v0 = ((q < 2 ? l0 : l0 >> 4) & 0x0F0F0F0Fu) | b0, v1 = ((q < 2 ? l1 : l1 >> 4) & 0x0F0F0F0Fu) | b1;
-            const uint32_t a[4] = {q6w_sub(__byte_perm(v0, 0x64646464u, 0x5140)), q6w_sub(__byte_perm(v1, 0x64646464u, 0x5140)),
-                                   q6w_sub(__byte_perm(v0, 0x64646464u, 0x7362)), q6w_sub(__byte_perm(v1, 0x64646464u, 0x7362))};
-            const uint2 xv = *reinterpret_cast<const uint2 *>(xp + xmul * (128 * h + 32 * q + 16 * s));
-            const uint32_t b[2] = {xv.x, xv.y};
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            q6k_mma_f16(acc, a, b);
-            const int si = 8 * h + 2 * q + s;
-            const float f0 = d0 * (__uint_as_float(__byte_perm(sc0[si >> 2], 0x4B000000u, 0x7440 + (si & 3))) - 8388736.0f); // 2^23 + 128
-            const float f1 = d1 * (__uint_as_float(__byte_perm(sc1[si >> 2], 0x4B000000u, 0x7440 + (si & 3))) - 8388736.0f);
-            tot[0] = fmaf(f0, acc[0], tot[0]);
-            tot[1] = fmaf(f0, acc[1], tot[1]);
-            tot[2] = fmaf(f1, acc[2], tot[2]);
-            tot[3] = fmaf(f1, acc[3], tot[3]);
+        for (int s = 0; s < 2; s++) {
+            const uint32_t at = 64 * h + 16 * s + 4 * c, hat = 128 + 32 * h + 16 * s + 4 * c;
+            const uint32_t le0 = q6w_word<ODD>(blk0 + at), lo0 = q6w_word<ODD>(blk0 + at + 32), qh0 = q6w_word<ODD>(blk0 + hat);
+            const uint32_t le1 = q6w_word<ODD>(blk1 + at), lo1 = q6w_word<ODD>(blk1 + at + 32), qh1 = q6w_word<ODD>(blk1 + hat);
+            const float4 s0 = *reinterpret_cast<const float4 *>(scr + g * 8 + (get_s ^ (4 * s)));
+            const float4 s1 = *reinterpret_cast<const float4 *>(scr + (g + 8) * 8 + (get_s ^ (4 * s)));
+            const float f0[4] = {s0.x, s0.y, s0.z, s0.w}, f1[4] = {s1.x, s1.y, s1.z, s1.w};
+            uint4 xv;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint32_t l0 = (q & 1) ? lo0 : le0, l1 = (q & 1) ? lo1 : le1;
+                const uint32_t b0 = (q == 0 ? qh0 << 4 : q == 1 ? qh0 << 2 : q == 2 ? qh0 : qh0 >> 2) & 0x30303030u;
+                const uint32_t b1 = (q == 0 ? qh1 << 4 : q == 1 ? qh1 << 2 : q == 2 ? qh1 : qh1 >> 2) & 0x30303030u;
+                const uint32_t v0 = ((q < 2 ? l0 : l0 >> 4) & 0x0F0F0F0Fu) | b0, v1 = ((q < 2 ? l1 : l1 >> 4) & 0x0F0F0F0Fu) | b1;
+                const uint32_t a[4] = {q6w_sub(__byte_perm(v0, 0x64646464u, 0x5140)), q6w_sub(__byte_perm(v1, 0x64646464u, 0x5140)),
+                                       q6w_sub(__byte_perm(v0, 0x64646464u, 0x7362)), q6w_sub(__byte_perm(v1, 0x64646464u, 0x7362))};
+                if ((q & 1) == 0) xv = *reinterpret_cast<const uint4 *>(xp + xmul * (128 * h + 64 * s + 16 * q));
+                const uint32_t b[2] = {(q & 1) ? xv.z : xv.x, (q & 1) ? xv.w : xv.y};
+                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                q6k_mma_f16(acc, a, b);
+                tot[0] = fmaf(f0[q], acc[0], tot[0]);
+                tot[1] = fmaf(f0[q], acc[1], tot[1]);
+                tot[2] = fmaf(f1[q], acc[2], tot[2]);
+                tot[3] = fmaf(f1[q], acc[3], tot[3]);
+            }
         }
     }
 }
@@ -305,7 +318,7 @@ __global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6k
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int engine = warp / (Q6W_WARPS + 1), ew = warp % (Q6W_WARPS + 1); // ew == Q6W_WARPS: the engine's producer
-    const int chunks = p.k / (Q6W_SB * 256), xrow = p.k + 16;
+    const int chunks = p.k / (Q6W_SB * 256), xrow = p.k + 32;
     const size_t row_bytes = (size_t)chunks * Q6W_ROW_BYTES;
     // rings of both engines | partial sums (two tiles per engine) | barriers | zeros | x
     const uint32_t base = smem_u32(smem);
@@ -364,34 +377,35 @@ __global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6k
             uint2 o;
             o.x = f32x2_to_f16x2_sat(bf16_lo_f32(raw.x), bf16_hi_f32(raw.x));
             o.y = f32x2_to_f16x2_sat(bf16_lo_f32(raw.y), bf16_hi_f32(raw.y));
-            reinterpret_cast<uint2 *>(xs + (size_t)row * xrow)[q4] = o;
+            // [half][sixteen of a pair][two pairs][word c][pair][4]: a lane reads two steps' words as 16 bytes
+            const int at = (q4 & ~63) | (q4 & 32) | ((q4 & 4) << 2) | ((q4 & 16) >> 1) | ((q4 & 3) << 1) | ((q4 & 8) >> 3);
+            reinterpret_cast<uint2 *>(xs + (size_t)row * xrow)[at] = o;
         }
     }
     asm volatile("bar.sync 3, %0;" ::"n"(Q6W_ENGINES * Q6W_WARPS * 32) : "memory"); // all but the producers
 
     const int g = lane >> 2, c = lane & 3;
     const bool real = g < p.m;
-    const __half *xbase = real ? xs + (size_t)g * xrow + ew * 256 + 4 * c : reinterpret_cast<const __half *>(zeros);
+    const __half *xbase = real ? xs + (size_t)g * xrow + ew * 256 + 8 * c : reinterpret_cast<const __half *>(zeros);
     const int xmul = real ? 1 : 0;
-    const uint32_t row_off = (uint32_t)(g * Q6W_ROW_BYTES + ew * 210);
     int r = 0, buf = 0;
     uint32_t ph = 0;
     bool ok = true;
     for (int t = first; t < p.tiles; t += step, buf ^= 1) {
         float tot[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float *mine = red + buf * Q6W_RED, *scr = mine + ew * 128; // the warp's own part, not yet written, holds scales till then
         for (int ch = 0; ch < chunks && ok; ch++) {
             ok = __all_sync(0xFFFFFFFFu, mbar_wait(full(r), ph, &g_q6k_gemv_flag, 2));
             if (!ok) break;
-            const uint32_t blk0 = ring + (uint32_t)(r * Q6W_STAGE_BYTES) + row_off, blk1 = blk0 + 8 * Q6W_ROW_BYTES;
+            const uint32_t blk = ring + (uint32_t)(r * Q6W_STAGE_BYTES + ew * 210);
             const __half *xp = xbase + xmul * (ch * Q6W_SB * 256);
-            if (ew & 1) q6w_superblock<true>(tot, blk0, blk1, c, xp, xmul);
-            else q6w_superblock<false>(tot, blk0, blk1, c, xp, xmul);
+            if (ew & 1) q6w_superblock<true>(tot, blk, scr, lane, xp, xmul);
+            else q6w_superblock<false>(tot, blk, scr, lane, xp, xmul);
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty(r)) : "memory");
             if (++r == p.ring) { r = 0; ph ^= 1u; }
         }
         // the engine's warps meet once per tile (also after a wait gave up); the other buffer is free again by then
-        float *mine = red + buf * Q6W_RED;
 #pragma unroll
         for (int e = 0; e < 4; e++) mine[(ew * 4 + e) * 32 + lane] = tot[e];
         asm volatile("bar.sync %0, %1;" ::"r"(1 + engine), "n"(Q6W_WARPS * 32) : "memory");
@@ -412,7 +426,7 @@ __global__ void __launch_bounds__(Q6W_THREADS, 1) q6k_gemv_wide_kernel(const Q6k
 
 static size_t q6w_fixed(int m, int k)
 {
-    return (size_t)Q6W_ENGINES * 2 * Q6W_RED * 4 + Q6W_ENGINES * 2 * Q6W_MAX_RING * 8 + 16 + (size_t)m * (k + 16) * 2;
+    return (size_t)Q6W_ENGINES * 2 * Q6W_RED * 4 + Q6W_ENGINES * 2 * Q6W_MAX_RING * 8 + 16 + (size_t)m * (k + 32) * 2;
 }
 
 // Ring depth of an engine, 0 where the kernel does not apply: rows of whole stages (8 super-blocks), at least four tiles per

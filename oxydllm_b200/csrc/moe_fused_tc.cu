@@ -3,23 +3,26 @@
 // Mirrors the expert half of MoeFeedForward::forward (moe.rs:466-499, dispatch_sparse 563-607) with the
 // experts' Mxfp4Linear weights (linear.rs, [experts, out, in / 32, 16] blocks + [experts, out, in / 32] scales).
 //
-// A unit of work is (token block of one expert: up to 256 expert-sorted rows) x (128 out features). The grid is
+// A unit of work is (token block of one expert: up to 192 expert-sorted rows) x (128 out features). The grid is
 // persistent: CTA b takes units b, b + grid, ... of a device-side table, feature tiles fastest, so that CTAs
-// running at the same time share their token block in L2. Per CTA:
-//   warp 0 (one lane)   TMA: boxes of packed nibbles (128 out features x 32 bytes = 64 input columns) into a
-//                       ring of eight slots;
-//   warp 2 (one lane)   TMA: the stage's tile of the activations ([rows, 64] bf16 in boxes of 64 rows, 128-byte
-//                       swizzle) into one of four slots;
-//   warps 4..19         unpack, four teams of four warps taking stages in turn: a thread turns two 16-byte blocks
-//                       (32 weights each; E8M0 scale bytes read through L1/L2) into bf16 weights, the bits the
-//                       dequantization kernel writes, as four 16-byte chunks of the K-major operand row (128-byte
-//                       swizzle) in one of four slots;
-//   warp 1 (one lane)   tcgen05.mma kind::f16, A = weights [128, 64], B = activations, D[128, rows] f32 in one of
-//                       two tensor-memory buffers for the whole of k; one commit per stage frees the slot (weights and
-//                       activations share a full / empty barrier pair per slot, so the issuer polls once per stage);
+// running at the same time share their token block in L2. Stages of 64 input columns are counted over all units of
+// a CTA and go round eight slots. Per CTA:
+//   warp 0              TMA: boxes of packed nibbles (128 out features x 32 bytes);
+//   warp 2              TMA: the stage's tile of the activations ([rows, 64] bf16 in boxes of 64 rows, 128-byte swizzle);
+//   warps 4..19         unpack, four teams of four warps taking stages in turn: a thread turns the two 16-byte blocks
+//                       (32 weights each; E8M0 scale bytes read through L1/L2) of one out feature into bf16 weights, the bits the
+//                       dequantization kernel writes, and stores them as 32 columns of its lane of tensor memory, where the
+//                       team has room for one stage;
+//   warp 1              tcgen05.mma kind::f16, A = weights [128, 64] from tensor memory, B = activations, D[128, rows] f32 in one
+//                       of two tensor-memory buffers for the whole of k; one commit per stage frees its slot and its weights;
 //   warps 20..23        epilogue of the previous unit while the next one accumulates: accumulator rows (out
 //                       features) -> + bias -> bf16 out[row, feature], or the clamped SwiGLU of GPT-OSS on
 //                       interleaved (gate, up) features -> out[row, feature / 2].
+// What bounds it: the unpack, about 640 clocks per stage for 350 of MMA at 176 rows. With the weights in shared memory a stage of 256 rows
+// moved 104 KB through it at 128 bytes a clock, 812 clocks for 512 of MMA, and a team could not start before its slot was free; now only
+// the store waits for that. 192 rows, because the weights of four stages (128 columns) and two accumulators have to fit 512 columns of
+// tensor memory. us a layer at 400 / 1024 / 4096 tokens, 32 experts of 2880 x 2880: 219 / 274 / 767 before, 204 / 247 / 738 now; 16 of 2048 x
+// 1024 at 200 tokens 63 / 57. Scale bytes a stage ahead and a swizzle against the bank conflicts of the packed rows gave nothing more.
 // Every wait is bounded and reports through the workspace flag word.
 #include <cuda_bf16.h>
 
@@ -38,19 +41,18 @@ __device__ long long g_mf_trace[10][256]; // clock stamps of CTA 0, per role and
 
 constexpr int MF_ROWS = 128;                   // out features per unit
 constexpr int MF_BK = 64;                      // input columns per stage
-constexpr int MF_UNPACK_WARPS = 16, MF_TEAMS = 4, MF_TEAM_WARPS = 4, MF_ROUND = 1; // four teams: a stage's chain of poll, unpack, fence and arrival overlaps with three others
+constexpr int MF_UNPACK_WARPS = 16, MF_TEAMS = 4, MF_TEAM_WARPS = 4; // four teams: a stage's chain of poll, unpack and arrival overlaps with three others
 constexpr int MF_EPI_WARPS = 4;
 constexpr int MF_THREADS = (4 + MF_UNPACK_WARPS + MF_EPI_WARPS) * 32;
-constexpr int MF_SLOTS = 4;                    // operand slots: an unpacked weight tile and an activation tile each, one pair of barriers
-constexpr int MF_A_SLOTS = MF_SLOTS, MF_X_SLOTS = MF_SLOTS;
-constexpr int MF_RAW_SLOTS = 8;
-constexpr int MF_MAX_TOK = 256;                // rows of a token block
-constexpr int MF_TMEM_BUF = 256;               // accumulator columns per buffer
-constexpr int MF_A_BYTES = MF_ROWS * MF_BK * 2;
+constexpr int MF_SLOTS = 8;                    // stages on their way: packed weights and activations, barriers
+constexpr int MF_MAX_TOK = 192;                // rows of a token block
+constexpr int MF_TMEM_BUF = MF_MAX_TOK;        // accumulator columns per buffer
+constexpr int MF_TMEM_A = 2 * MF_TMEM_BUF, MF_A_COLS = MF_BK / 2; // a team's unpacked weights, two to a column
 constexpr int MF_XBOX_ROWS = 64, MF_XBOX_BYTES = MF_XBOX_ROWS * MF_BK * 2, MF_X_BYTES = MF_MAX_TOK * MF_BK * 2; // activation rows travel in boxes of 64
 constexpr int MF_RAW_BYTES = MF_ROWS * MF_BK / 2;
-constexpr int MF_NUM_BARS = 2 * MF_RAW_SLOTS + 2 * MF_SLOTS + 4;
-static_assert(MF_RAW_SLOTS % MF_ROUND == 0 && MF_A_SLOTS % MF_ROUND == 0, "a round's slots are neighbours");
+constexpr int MF_NUM_BARS = 4 * MF_SLOTS + 4;
+static_assert(MF_TMEM_A + MF_TEAMS * MF_A_COLS <= 512, "tensor memory");
+static_assert(MF_SLOTS == 2 * MF_TEAMS, "a team meets two slots in turn");
 constexpr int MF_SMEM_BUDGET = 227 * 1024;
 
 struct MoeFusedParams {
@@ -60,7 +62,7 @@ struct MoeFusedParams {
     const void *bias;      // [experts, n] or null
     void *out;
     int *flag;
-    int n, k, nkb, nk2;    // out features per expert, in features, scale bytes per row, stages per unit (whole rounds)
+    int n, k, nkb, nk2;    // out features per expert, in features, scale bytes per row, stages per unit
     int tiles_n, bias_dtype, ldo, epi;
     float limit;
     int dbg;               // tuning builds: parts of the pipeline switched off for timing
@@ -73,9 +75,25 @@ __device__ __forceinline__ uint4 mf_lds128(uint32_t addr)
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ void mf_sts128(uint32_t addr, const uint4 &v)
+// 32 columns of this warp's quarter of tensor memory.
+__device__ __forceinline__ void mf_tmem_st32(uint32_t taddr, const uint32_t (&r)[32])
 {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+                 "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+                 "r"(r[30]), "r"(r[31])
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem desc], bf16 x bf16 -> f32; lane i of A's columns is row i, a column two elements of k.
+__device__ __forceinline__ void mf_umma(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+                 : "memory");
 }
 __device__ __forceinline__ void mf_arrive(uint32_t bar)
 {
@@ -88,17 +106,16 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
     unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    // A slots | activation slots | ring of packed boxes | barriers | tensor-memory address
-    const uint32_t x_base = base + MF_A_SLOTS * MF_A_BYTES;
-    const uint32_t raw_base = x_base + MF_X_SLOTS * MF_X_BYTES;
-    const uint32_t bars = raw_base + MF_RAW_SLOTS * MF_RAW_BYTES;
+    // activation slots | packed slots | barriers | tensor-memory address
+    const uint32_t x_base = base, raw_base = base + MF_SLOTS * MF_X_BYTES;
+    const uint32_t bars = raw_base + MF_SLOTS * MF_RAW_BYTES;
     auto rawfull_bar = [&](int r) { return bars + 8u * r; };
-    auto rawempty_bar = [&](int r) { return bars + 8u * (MF_RAW_SLOTS + r); };
-    // full: the slot's weight tile is unpacked (one arrival per warp of the team) and its activation tile has landed (the
-    // producer's arrival with the byte count); empty: the MMAs that read the slot have completed (one commit)
-    auto full_bar = [&](int s) { return bars + 8u * (2 * MF_RAW_SLOTS + s); };
-    auto empty_bar = [&](int s) { return bars + 8u * (2 * MF_RAW_SLOTS + MF_SLOTS + s); };
-    const uint32_t misc = bars + 8u * (2 * MF_RAW_SLOTS + 2 * MF_SLOTS);
+    auto rawempty_bar = [&](int r) { return bars + 8u * (MF_SLOTS + r); };
+    // full: the stage's weights are in tensor memory (one arrival per warp of the team) and its activation tile has landed (the
+    // producer's arrival with the byte count); empty: the MMAs that read both have completed (one commit)
+    auto full_bar = [&](int s) { return bars + 8u * (2 * MF_SLOTS + s); };
+    auto empty_bar = [&](int s) { return bars + 8u * (3 * MF_SLOTS + s); };
+    const uint32_t misc = bars + 8u * (4 * MF_SLOTS);
     auto tfull_bar = [&](int b) { return misc + 8u * b; };
     auto tempty_bar = [&](int b) { return misc + 8u * (2 + b); };
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bars - base) + 8 * MF_NUM_BARS);
@@ -108,11 +125,9 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
     const int nk2 = p.nk2;
 
     if (threadIdx.x == 0) {
-        for (int r = 0; r < MF_RAW_SLOTS; r++) {
-            mbar_init(rawfull_bar(r), 1);
-            mbar_init(rawempty_bar(r), MF_TEAM_WARPS);
-        }
         for (int s = 0; s < MF_SLOTS; s++) {
+            mbar_init(rawfull_bar(s), 1);
+            mbar_init(rawempty_bar(s), MF_TEAM_WARPS);
             mbar_init(full_bar(s), MF_TEAM_WARPS + 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -149,7 +164,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                     tma_load_2d(raw_base + r * MF_RAW_BYTES, &wmap, rawfull_bar(r), it * (MF_BK / 2), rowbase);
                 }
                 __syncwarp();
-                if (++r == MF_RAW_SLOTS) { r = 0; ph ^= 1u; }
+                if (++r == MF_SLOTS) { r = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 2) {
@@ -172,7 +187,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                             tma_load_2d(dst + (uint32_t)b * MF_XBOX_BYTES, &xmap, full_bar(xs), it * MF_BK, en.x + b * MF_XBOX_ROWS);
                 }
                 __syncwarp();
-                if (++xs == MF_X_SLOTS) { xs = 0; xph ^= 1u; }
+                if (++xs == MF_SLOTS) { xs = 0; xph ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -180,7 +195,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
         // One warp issues every MMA of the CTA, so its instruction count per stage is on the critical path: one poll (full) and one
         // commit (empty) per stage.
         const bool leader = elect_one();
-        const uint64_t da0 = kmajor_sw128_desc(base), db0 = kmajor_sw128_desc(x_base);
+        const uint64_t db0 = kmajor_sw128_desc(x_base);
         int s = 0, ul = 0;
         uint32_t ph = 0;
         bool ok = true;
@@ -192,11 +207,12 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                 ok = mx_wait(full_bar(s), ph, p.flag, 2);
                 if (ok) {
                     tc_fence_after();
-                    const uint64_t da = da0 + (uint64_t)(s * (MF_A_BYTES >> 4)), db = db0 + (uint64_t)(s * (MF_X_BYTES >> 4));
+                    const uint32_t a_tmem = tmem_base + MF_TMEM_A + (uint32_t)(s % MF_TEAMS) * MF_A_COLS;
+                    const uint64_t db = db0 + (uint64_t)(s * (MF_X_BYTES >> 4));
                     if (leader) {
 #pragma unroll
                         for (int kk = 0; kk < MF_BK / 16; kk++) // 16 input columns: 32 bytes inside a swizzled K-major row
-                            umma_bf16(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (it | kk) != 0);
+                            mf_umma(d_tmem, a_tmem + 8 * kk, db + 2 * kk, idesc, (it | kk) != 0);
                         umma_commit(empty_bar(s));
                     }
                     __syncwarp();
@@ -211,19 +227,15 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
         const int team = (warp - 4) / MF_TEAM_WARPS;
         const int ut = (threadIdx.x - 128) % (MF_TEAM_WARPS * 32);
         const int row = ut;                                       // this thread: both 16-byte blocks of one out feature per stage
-        static_assert(MF_TEAM_WARPS * 32 == MF_ROWS && MF_ROUND == 1, "a thread per out feature");
-        const uint32_t raw_off = (uint32_t)row * 32u;
-        const uint32_t a_row = (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u;
-        const uint32_t sw = (uint32_t)(row & 7);
-        const int rpu = nk2 / MF_ROUND;                            // rounds per unit
+        static_assert(MF_TEAM_WARPS * 32 == MF_ROWS, "a thread per out feature");
+        const uint32_t raw_addr = raw_base + (uint32_t)row * 32u;
+        const uint32_t a_tmem = tmem_base + ((uint32_t)(warp & 3) << 21) + MF_TMEM_A + (uint32_t)team * MF_A_COLS; // the team's four warps: one quarter each
         int my_units = 0;
         if ((int)blockIdx.x < n_units) my_units = (n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;
-        const uint32_t total_rounds = (uint32_t)my_units * (uint32_t)rpu;
-        // every counter steps along (divisions by the rounds of a unit were a third of a stage's instructions)
-        static_assert(MF_TEAMS * MF_ROUND <= MF_RAW_SLOTS && MF_RAW_SLOTS % (MF_TEAMS * MF_ROUND) == 0 && MF_A_SLOTS % (MF_TEAMS * MF_ROUND) == 0,
-                      "a slot meets one team");
-        int u = (int)blockIdx.x, r_in_unit = team;
-        uint32_t r0 = (uint32_t)team * MF_ROUND, rph = 0, s0 = (uint32_t)team * MF_ROUND, aph = 0;
+        const uint32_t total = (uint32_t)my_units * (uint32_t)nk2;
+        // every counter steps along (divisions by the stages of a unit were a third of a stage's instructions)
+        int u = (int)blockIdx.x, it = team;
+        uint32_t s = (uint32_t)team, ph = 0, other_ph = 1; // this stage's slot and its parity; that of the other slot, four stages back
         const uint8_t *srow = nullptr;
         auto unit_scales = [&]() { // this thread's row of the scale bytes
             if (u >= n_units) return;
@@ -231,40 +243,33 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
             const int e = __ldg(p.entries + tb).z;
             srow = (f * MF_ROWS + row < p.n) ? p.scales + ((size_t)e * p.n + f * MF_ROWS + row) * p.nkb : nullptr;
         };
-        while (r_in_unit >= rpu) { r_in_unit -= rpu; u += (int)gridDim.x; }
+        while (it >= nk2) { it -= nk2; u += (int)gridDim.x; }
         unit_scales();
         bool ok = true;
-        // rounds are counted over all units of this CTA, so slots and teams keep alternating across unit boundaries
-        for (uint32_t gr = (uint32_t)team; gr < total_rounds; gr += MF_TEAMS) {
-            // the scale bytes of the round's two blocks come straight from L2 (the row's bytes are neighbours, so most loads
+        for (uint32_t g = (uint32_t)team; g < total; g += MF_TEAMS) {
+            // the scale bytes of the stage's two blocks come straight from L2 (the row's bytes are neighbours, so most loads
             // hit L1); they are asked for before the polls, which hide their latency. Past k (zero-filled boxes) and past the
             // expert's last out feature: 1.0
-            const int kb0 = r_in_unit * 2;
+            const int kb0 = it * 2;
             uint32_t sbv[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) sbv[h] = (srow != nullptr && kb0 + h < p.nkb) ? (uint32_t)__ldg(srow + kb0 + h) : 127u;
-            const uint32_t gs0 = gr * MF_ROUND;
-            // all polls of the round first (they do not depend on each other), the bounded waits only where one failed
-            bool tr[MF_ROUND], ta[MF_ROUND];
-#pragma unroll
-            for (int h = 0; h < MF_ROUND; h++) {
-                tr[h] = mbar_test(rawfull_bar(r0 + h), rph);
-                ta[h] = gs0 < MF_SLOTS || mbar_test(empty_bar(s0 + h), aph ^ 1u);
-            }
-#pragma unroll
-            for (int h = 0; h < MF_ROUND; h++) {
-                if (ok && !tr[h]) ok = mbar_wait(rawfull_bar(r0 + h), rph, p.flag, 3);
-                if (ok && !ta[h]) ok = mbar_wait(empty_bar(s0 + h), aph ^ 1u, p.flag, 7);
-            }
+            // both polls first (they do not depend on each other), the bounded waits only where one failed
+            const uint32_t prev_empty = empty_bar((int)(s ^ MF_TEAMS)); // the team's stage before this one has been multiplied
+            const bool tr = mbar_test(rawfull_bar((int)s), ph);
+            bool free_a = g < MF_TEAMS || mbar_test(prev_empty, other_ph);
+            free_a = __all_sync(0xFFFFFFFFu, free_a);
+            ok = __all_sync(0xFFFFFFFFu, tr) || mx_wait(rawfull_bar((int)s), ph, p.flag, 3);
             if (!ok) break;
-            if (ut == 0) MF_TRACE(4, gs0);
-            if (!MF_DBG(1))
+            if (ut == 0) MF_TRACE(4, g);
+            uint4 rawv[2];
+#pragma unroll
+            for (int half = 0; half < 2; half++) rawv[half] = mf_lds128(raw_addr + s * MF_RAW_BYTES + 16u * half);
+            uint32_t o[MF_A_COLS]; // the row's weights, two to a word
 #pragma unroll
             for (int half = 0; half < 2; half++) {
                 const uint32_t sb = sbv[half];
-                const uint4 rawv = mf_lds128(raw_base + r0 * MF_RAW_BYTES + raw_off + 16u * half);
-                const uint32_t v[4] = {rawv.x, rawv.y, rawv.z, rawv.w};
-                const uint32_t dst = base + s0 * MF_A_BYTES + a_row;
+                const uint32_t v[4] = {rawv[half].x, rawv[half].y, rawv[half].z, rawv[half].w};
                 if (sb >= 4u && sb <= 250u) { // 2^(s-127) as a bf16 pair: the products are exact
                     // The block's eight magnitudes 0, .5, 1, 1.5, 2, 3, 4, 6 times its scale, as bf16 (four multiplies for
                     // 32 weights), split into a table of low bytes and a table of high bytes; the byte permute unit then looks
@@ -291,48 +296,43 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                         const uint32_t sg_a = __byte_perm(wl, w, 0x5140u), sg_b = __byte_perm(wl, w, 0x7362u);
                         asm("lop3.b32 %0, %1, %2, %0, 0x6A;" : "+r"(hi_a) : "r"(sg_a), "r"(0x80808080u)); // (sg & mask) ^ hi
                         asm("lop3.b32 %0, %1, %2, %0, 0x6A;" : "+r"(hi_b) : "r"(sg_b), "r"(0x80808080u));
-                        uint4 o;
-                        o.x = __byte_perm(lo_a, hi_a, 0x5140u);
-                        o.y = __byte_perm(lo_a, hi_a, 0x7362u);
-                        o.z = __byte_perm(lo_b, hi_b, 0x5140u);
-                        o.w = __byte_perm(lo_b, hi_b, 0x7362u);
-                        mf_sts128(dst + ((((uint32_t)(half * 4 + q)) ^ sw) << 4), o);
+                        o[half * 16 + q * 4] = __byte_perm(lo_a, hi_a, 0x5140u);
+                        o[half * 16 + q * 4 + 1] = __byte_perm(lo_a, hi_a, 0x7362u);
+                        o[half * 16 + q * 4 + 2] = __byte_perm(lo_b, hi_b, 0x5140u);
+                        o[half * 16 + q * 4 + 3] = __byte_perm(lo_b, hi_b, 0x7362u);
                     }
                 } else { // scales whose products leave the normal range (NaN, 2^-127 among them): f32 product, one rounding
                     const float s = e8m0_to_f32(sb);
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        uint4 o;
-                        uint32_t *ov = reinterpret_cast<uint32_t *>(&o);
 #pragma unroll
                         for (int b = 0; b < 4; b++) {
                             const uint32_t by = (v[q] >> (8 * b)) & 0xFFu;
                             const __nv_bfloat162 hh = __halves2bfloat162(narrow<__nv_bfloat16>(__fmul_rn(e2m1_to_f32(by & 0xFu), s)),
                                                                          narrow<__nv_bfloat16>(__fmul_rn(e2m1_to_f32(by >> 4), s)));
-                            ov[b] = *reinterpret_cast<const uint32_t *>(&hh);
+                            o[half * 16 + q * 4 + b] = *reinterpret_cast<const uint32_t *>(&hh);
                         }
-                        mf_sts128(dst + ((((uint32_t)(half * 4 + q)) ^ sw) << 4), o);
                     }
                 }
             }
-            if (ut == 0) MF_TRACE(5, gs0);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
+            if (ut == 0) MF_TRACE(5, g);
             __syncwarp();
-            if (lane == 0) {
-#pragma unroll
-                for (int h = 0; h < MF_ROUND; h++) {
-                    mf_arrive(full_bar(s0 + h));
-                    mf_arrive(rawempty_bar(r0 + h));
-                }
-            }
-            if (ut == 0) MF_TRACE(6, gs0);
-            r0 += MF_TEAMS * MF_ROUND;
-            if (r0 == MF_RAW_SLOTS + (uint32_t)team * MF_ROUND) { r0 = (uint32_t)team * MF_ROUND; rph ^= 1u; }
-            s0 += MF_TEAMS * MF_ROUND;
-            if (s0 == MF_A_SLOTS + (uint32_t)team * MF_ROUND) { s0 = (uint32_t)team * MF_ROUND; aph ^= 1u; }
-            r_in_unit += MF_TEAMS;
-            if (r_in_unit >= rpu) { // the next unit (rounds are counted on: slots and teams keep alternating)
-                do { r_in_unit -= rpu; u += (int)gridDim.x; } while (r_in_unit >= rpu);
+            if (lane == 0) mf_arrive(rawempty_bar((int)s));
+            if (!free_a) ok = mx_wait(prev_empty, other_ph, p.flag, 7);
+            if (!ok) break;
+            tc_fence_after();
+            mf_tmem_st32(a_tmem, o);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mf_arrive(full_bar((int)s));
+            if (ut == 0) MF_TRACE(6, g);
+            // slots of a team: t, t + 4, t, ...; a slot's parity changes when the first of the two comes round again
+            s ^= MF_TEAMS;
+            if (s == (uint32_t)team) ph ^= 1u;
+            else other_ph ^= 1u;
+            it += MF_TEAMS;
+            if (it >= nk2) { // the next unit (stages are counted on: slots and teams keep alternating)
+                do { it -= nk2; u += (int)gridDim.x; } while (it >= nk2);
                 unit_scales();
             }
         }
@@ -416,13 +416,13 @@ int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const ui
     p.entries = entries; p.n_blocks = n_blocks; p.scales = scales; p.bias = bias; p.out = out; p.flag = flag;
     p.n = n; p.k = k; p.nkb = k / 32;
     const int nk = (k + MF_BK - 1) / MF_BK;
-    p.nk2 = (nk + MF_ROUND - 1) / MF_ROUND * MF_ROUND;
+    p.nk2 = nk;
     p.tiles_n = (n + MF_ROWS - 1) / MF_ROWS;
     p.bias_dtype = bias_dtype; p.ldo = ldo; p.epi = epi; p.limit = limit;
     p.test_skip_loads = g_moe_selftest_skip_loads;
     if (const char *env = tuning_env("OXQ_MF_DBG")) p.dbg = atoi(env);
-    constexpr size_t smem = 1024 + MF_A_SLOTS * MF_A_BYTES + MF_X_SLOTS * MF_X_BYTES + MF_RAW_SLOTS * MF_RAW_BYTES + 8 * MF_NUM_BARS + 16;
-    static_assert(smem <= (size_t)MF_SMEM_BUDGET, "operand slots and the ring must fit one CTA's shared memory");
+    constexpr size_t smem = 1024 + MF_SLOTS * (MF_X_BYTES + MF_RAW_BYTES) + 8 * MF_NUM_BARS + 16;
+    static_assert(smem <= (size_t)MF_SMEM_BUDGET, "the slots must fit one CTA's shared memory");
     CUtensorMap wmap, xmap;
     CUresult r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, blocks, (uint64_t)k / 2, (uint64_t)experts * n, (uint64_t)k / 2,
                                  MF_BK / 2, MF_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);

@@ -180,6 +180,14 @@ def test_moe_small_batch_matches_64_bit_experts(cuda, hidden, inter, counts):
         assert (np.abs(got[rows] - ref) <= 2.0**-8 * (np.abs(h) @ np.abs(dn).T + np.abs(ref)) + 1e-6).all(), (e, c)
 
 
+# more than 44 rows an expert on average: blocks of up to 192 rows, weights unpacked into tensor memory by four teams in turn; fewer
+# stages of 64 columns than teams, a last stage half past k, more units than SMs
+@pytest.mark.parametrize("hidden,inter", [(32, 96), (96, 32), (224, 544), (2880, 64), (128, 9600)])
+@pytest.mark.parametrize("counts", [(192, 193, 0, 1), (385, 64, 191, 0)])
+def test_moe_large_batch_matches_64_bit_experts(cuda, hidden, inter, counts):
+    test_moe_small_batch_matches_64_bit_experts(cuda, hidden, inter, counts)
+
+
 def test_moe_small_batch_kernel_survives_weights_that_never_come(cuda):
     ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
     _lib.call("oxq_selftest_moe_mx_wait_expiry", ws.data_ptr(), ws.numel(), None)

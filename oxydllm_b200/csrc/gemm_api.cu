@@ -31,7 +31,7 @@ bool group_tc_supported(int m, int k, int n, int group_size, int scales_dtype, c
 int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                     int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
                     cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
-size_t packed_mx_scratch_bytes(int m, int k, int n, int group_size);
+size_t packed_mx_scratch_bytes(int m, int k, int n);
 bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
                          const void *scales);
 int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
@@ -219,7 +219,7 @@ OXQ_EXPORT size_t oxq_packed4_full_scratch_bytes(int m, int k, int n, int group_
     if (m <= 0 || k <= 0 || n <= 0 || n % 128 != 0 || k % 128 != 0 || group_size <= 0) return 0;
     const size_t own = group_tc_scratch_bytes(m, n);
     const bool mxs = gptq && packed_mx_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr);
-    const size_t mx = mxs ? packed_mx_scratch_bytes(m, k, n, group_size) : 0;
+    const size_t mx = mxs ? packed_mx_scratch_bytes(m, k, n) : 0;
     return mx > own ? mx : own;
 }
 

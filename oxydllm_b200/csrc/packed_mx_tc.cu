@@ -59,7 +59,7 @@ struct PackedMxParams {
     const uint32_t *qzeros;
     const void *scales, *bias;
     const unsigned char *sf;        // [unit][token block][1 or 2][512] block scales of x's pieces
-    const float *sx;                // [fold][token blocks * mpad] sums of x
+    const float *sx;                // GPTQ: [unit][token blocks * mpad] sums of x
     void *y;
     int scales_f16, bias_dtype, y_dtype;
     int m, n, packed_out;
@@ -72,7 +72,7 @@ struct PackedMxParams {
     int acc_cols;                   // tensor-memory columns of an accumulator buffer
     int tmem_cols;
     int gshift;                     // log2(group size)
-    int fold_rows;                  // min(group size, 128): input rows per accumulator buffer
+    int fold_rows;                  // input rows per accumulator buffer: 128, or 64 where E4M3 weights have scale blocks of an odd number of 64s
     int units_per_tile, tiles;
     const float *scale_inv;         // E4M3: one scale per block_out x block_in weights, s_in blocks a row; null: 1
     int s_in, block_out, block_in;
@@ -113,11 +113,11 @@ __host__ __device__ __forceinline__ int px_owner(long long total, int ctas, long
 // ---- x -> two E4M3 pieces, block scales, sums ---------------------------------------------------------------------------------
 // Sixteen lanes hold the 128 k of a unit of one token. xq: [token block][piece][mpad tokens][k]; sf: a piece's rows of a tile in the
 // order tmem_cp_scales wants (merged: both pieces' rows in one 512-byte chunk). GPTQ: within eight k the even ones come first, as
-// the unpack leaves them.
+// the unpack leaves them, and sx takes the sum of each unit; E4M3 weights need no sums, the scratch has no room for any.
 template <bool GPTQ>
 __global__ void __launch_bounds__(256)
     packed_mx_split_kernel(const __nv_bfloat16 *x, unsigned char *xq, unsigned char *sf, float *sx, int m, int k, int mpad, int token_blocks,
-                           int merged, int fold_rows)
+                           int merged)
 {
     // Behind the wait everything ahead of this kernel is complete, so what starts early after the trigger may read the weights at once.
     pdl_wait();
@@ -134,15 +134,13 @@ __global__ void __launch_bounds__(256)
         v[2 * i] = bf16_lo_f32(w[i]);
         v[2 * i + 1] = bf16_hi_f32(w[i]);
         amax = max(amax, max(w[i] << 16 & 0x7FFF0000u, w[i] & 0x7FFF0000u));
-        sum += v[2 * i] + v[2 * i + 1];
+        if (GPTQ) sum += v[2 * i] + v[2 * i + 1];
     }
 #pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) { // four lanes hold a block of 32
-        amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    }
-    const float sum64 = sum + __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
-    const float sum128 = sum64 + __shfl_xor_sync(0xFFFFFFFFu, sum64, 8);
+    for (int o = 1; o <= 2; o <<= 1) amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o)); // four lanes hold a block of 32
+    if (GPTQ)
+#pragma unroll
+        for (int o = 1; o <= 8; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     uint2 hi, lo;
     const uint32_t s = mx_split8(v, amax, hi, lo);
     if (GPTQ) {
@@ -160,10 +158,7 @@ __global__ void __launch_bounds__(256)
         c[(row & 31) * 16 + (row >> 5) * 4 + j] = (unsigned char)s;
         if (!merged) c += PX_SF_BYTES;
         c[(lrow & 31) * 16 + (lrow >> 5) * 4 + j] = (unsigned char)(s - 4u);
-        const int ld = token_blocks * mpad, at = tb * mpad + row;
-        if (fold_rows == 32) sx[(size_t)(4 * u + j) * ld + at] = sum;
-        else if (fold_rows == 64 && (j & 1) == 0) sx[(size_t)(2 * u + (j >> 1)) * ld + at] = sum64;
-        else if (fold_rows == 128 && j == 0) sx[(size_t)u * ld + at] = sum128;
+        if (GPTQ && j == 0) sx[(size_t)u * (token_blocks * mpad) + tb * mpad + row] = sum;
     }
 }
 
@@ -206,7 +201,7 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
     }
     const int nunits = (int)(u1 - u0);
     const int first_tile = (int)(u0 / G), first_unit = (int)(u0 - (long long)first_tile * G);
-    const int unit_folds = PX_UNIT / p.fold_rows;
+    const int unit_folds = FP8 ? PX_UNIT / p.fold_rows : 1;
 
     if (warp == 0) { // barrier b of each kind is initialised by lane b
         static_assert(PX_MAX_RAW <= 32, "one lane per barrier");
@@ -362,10 +357,9 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
             }
         };
         if (unit_folds == 1) issue(PxInt<1>{});
-        else if (unit_folds == 2) issue(PxInt<2>{});
-        else issue(PxInt<4>{});
+        else issue(PxInt<2>{});
     } else if (!FP8 && warp == 4) {
-        // ---- scales, zero points and sums of x, a fold at a time ---------------------------------------------------------
+        // ---- scales, zero points and sums of x, a unit at a time ---------------------------------------------------------
         const bool leader = elect_one();
         const int ld = p.token_blocks * p.mpad, zbytes = p.sym ? 0 : PX_Z_BYTES;
         int n0 = first_tile / p.token_blocks * PX_ROWS, tb = first_tile % p.token_blocks, uk = first_unit, c = 0;
@@ -374,18 +368,16 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
         pdl_wait(); // the sums come from the kernel ahead
         for (int it = 0; it < nunits && ok; it++) {
             const size_t group = (size_t)(((long long)uk * PX_UNIT) >> p.gshift);
-            for (int f = 0; f < unit_folds && ok; f++) { // more than one: groups shorter than a unit, one fold each
-                ok = mx_wait(frempty + 8 * c, cph, p.flag, PX_CODE + 8);
-                if (ok && leader && !p.test_skip_loads) {
-                    const uint32_t dst = fr_base + (uint32_t)(c * p.fr_bytes), bar = frfull + 8 * c;
-                    mbar_arrive_expect_tx(bar, (uint32_t)(PX_SC_BYTES + zbytes + 4 * p.mpad));
-                    bulk_copy_g2s(dst, reinterpret_cast<const uint16_t *>(p.scales) + (group + f) * p.n + n0, PX_SC_BYTES, bar);
-                    if (zbytes) bulk_copy_g2s(dst + PX_SC_BYTES, p.qzeros + (group + f) * p.packed_out + n0 / 8, PX_Z_BYTES, bar);
-                    bulk_copy_g2s(dst + PX_SC_BYTES + PX_Z_BYTES, p.sx + ((size_t)uk * unit_folds + f) * ld + tb * p.mpad, 4u * p.mpad, bar);
-                }
-                __syncwarp();
-                if (++c == PX_FR) { c = 0; cph ^= 1u; }
+            ok = mx_wait(frempty + 8 * c, cph, p.flag, PX_CODE + 8);
+            if (ok && leader && !p.test_skip_loads) {
+                const uint32_t dst = fr_base + (uint32_t)(c * p.fr_bytes), bar = frfull + 8 * c;
+                mbar_arrive_expect_tx(bar, (uint32_t)(PX_SC_BYTES + zbytes + 4 * p.mpad));
+                bulk_copy_g2s(dst, reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0, PX_SC_BYTES, bar);
+                if (zbytes) bulk_copy_g2s(dst + PX_SC_BYTES, p.qzeros + group * p.packed_out + n0 / 8, PX_Z_BYTES, bar);
+                bulk_copy_g2s(dst + PX_SC_BYTES + PX_Z_BYTES, p.sx + (size_t)uk * ld + tb * p.mpad, 4u * p.mpad, bar);
             }
+            __syncwarp();
+            if (++c == PX_FR) { c = 0; cph ^= 1u; }
             if (++uk == G) {
                 uk = 0;
                 if (++tb == p.token_blocks) { tb = 0; n0 += PX_ROWS; }
@@ -596,7 +588,7 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
 }
 
 // True when this kernel serves a GPTQ call and is the better one: its unpack is cheaper than that of csrc/group_tc.cu, but the kernel that
-// writes x's pieces costs a launch, so the layer has to be large, and a group shorter than a unit is folded more than once. us here /
+// writes x's pieces costs a launch, so the layer has to be large, and the groups at least a unit. us here /
 // there at 16 tokens: 4096 x 14336 17.2 / 20.5, 14336 x 4096 20.5 / 22.2, 4096 x 6144 14.1 / 12.7, 2048 x 4096 10.8 / 10.3, groups of 64,
 // 4096 x 4096 15.9 / 13.1; at 32 tokens 4096 x 14336 20.7 / 21.7, 14336 x 4096 24.2 / 23.2.
 bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
@@ -617,34 +609,36 @@ bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const vo
            aligned(x, 16) && aligned(weight, 16) && aligned(scale_inv, 4);
 }
 
-// The scratch area: x's pieces, their block scales and sums, then tickets and parts of shared tiles.
+// The scratch area: x's pieces, their block scales and (GPTQ) sums, then tickets and parts of shared tiles.
 struct PackedMxScratch {
     int token_blocks, mpad, merged, tiles;
     size_t sf, sx, tickets, partials, part_bytes; // offsets of the pieces' successors; bytes of a part
 };
-static PackedMxScratch packed_mx_layout(int m, int k, int n, int group_size)
+static PackedMxScratch packed_mx_layout(int wt, int m, int k, int n)
 {
     PackedMxScratch s;
     s.token_blocks = ceil_div(m, PX_MAX_TOKENS);
     s.mpad = ceil_div(ceil_div(m, s.token_blocks), 16) * 16;
     s.merged = s.mpad <= PX_MERGED_TOKENS;
     s.tiles = n / PX_ROWS * s.token_blocks;
-    const size_t rows = (size_t)s.token_blocks * s.mpad, units = (size_t)k / PX_UNIT, folds = (size_t)k / (group_size < PX_UNIT ? group_size : PX_UNIT);
+    const size_t rows = (size_t)s.token_blocks * s.mpad, units = (size_t)k / PX_UNIT;
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
     s.sf = up(2 * rows * k);
     s.sx = s.sf + up(units * s.token_blocks * (s.merged ? 1 : 2) * PX_SF_BYTES);
-    s.tickets = s.sx + up(folds * rows * sizeof(float));
+    s.tickets = s.sx + (wt == PX_GPTQ ? up(units * rows * sizeof(float)) : 0);
     s.partials = s.tickets + up((size_t)s.tiles * sizeof(unsigned long long));
     s.part_bytes = (size_t)s.mpad * PX_ROWS * sizeof(float);
     return s;
 }
 
 // Scratch that lets a call of this size share tiles over all SMs (with less it shares fewer, below the pieces it is not served).
-size_t packed_mx_scratch_bytes(int m, int k, int n, int group_size)
+static size_t packed_mx_full_bytes(int wt, int m, int k, int n)
 {
-    const PackedMxScratch s = packed_mx_layout(m, k, n, group_size);
+    const PackedMxScratch s = packed_mx_layout(wt, m, k, n);
     return s.partials + (size_t)(sm_count() + s.tiles) * s.part_bytes;
 }
+size_t packed_mx_scratch_bytes(int m, int k, int n) { return packed_mx_full_bytes(PX_GPTQ, m, k, n); }
+size_t fp8_mx_scratch_bytes(int m, int k, int n) { return packed_mx_full_bytes(PX_FP8, m, k, n); }
 
 template <int WT, int NCH, int PARTS>
 static int packed_mx_launch(const PackedMxParams &p, const CUtensorMap &wmap, const CUtensorMap &xmap, int ctas, size_t smem, cudaStream_t st)
@@ -754,7 +748,7 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
     OXQ_CUDA(cudaLaunchKernelEx(&cfg, wt == PX_GPTQ ? packed_mx_split_kernel<true> : packed_mx_split_kernel<false>, (const __nv_bfloat16 *)x, sb,
-                                sb + s.sf, reinterpret_cast<float *>(sb + s.sx), m, k, p.mpad, p.token_blocks, p.merged, p.fold_rows));
+                                sb + s.sf, reinterpret_cast<float *>(sb + s.sx), m, k, p.mpad, p.token_blocks, p.merged));
 #define OXQ_PX_LAUNCH(WT, NCH, PARTS) return packed_mx_launch<WT, NCH, PARTS>(p, wmap, xmap, (int)ctas, smem, st)
     if (wt == PX_FP8) {
         if (p.mpad <= 16) OXQ_PX_LAUNCH(PX_FP8, 1, 2);
@@ -770,7 +764,7 @@ int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
                      cudaStream_t st, int sym, void *scratch, size_t scratch_bytes)
 {
-    const PackedMxScratch s = packed_mx_layout(m, k, n, group_size);
+    const PackedMxScratch s = packed_mx_layout(PX_GPTQ, m, k, n);
     if (scratch == nullptr || scratch_bytes < s.tickets) return OXQ_ERR_UNSUPPORTED;
     PackedMxParams p = {};
     p.qzeros = qzeros; p.scales = scales; p.bias = bias; p.y = y;
@@ -779,22 +773,16 @@ int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
     p.sym = sym || qzeros == nullptr;
     p.test_skip_loads = g_packed_mx_selftest_skip_loads;
     while ((1 << p.gshift) < group_size) p.gshift += 1;
-    p.fold_rows = group_size < PX_UNIT ? group_size : PX_UNIT;
+    p.fold_rows = PX_UNIT;
     p.block_in = p.block_out = PX_UNIT;
     return packed_mx_run(p, PX_GPTQ, x, qweight, k, s, reinterpret_cast<unsigned char *>(scratch), scratch_bytes, st);
-}
-
-size_t fp8_mx_scratch_bytes(int m, int k, int n)
-{
-    const PackedMxScratch s = packed_mx_layout(m, k, n, PX_UNIT);
-    return s.partials + (size_t)(sm_count() + s.tiles) * s.part_bytes;
 }
 
 // E4M3 weights with one f32 scale per block_out x block_in of them.
 int fp8_mx_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in, const void *bias,
                   int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st, void *scratch, size_t scratch_bytes)
 {
-    const PackedMxScratch s = packed_mx_layout(m, k, n, PX_UNIT);
+    const PackedMxScratch s = packed_mx_layout(PX_FP8, m, k, n);
     if (scratch == nullptr || scratch_bytes < s.tickets) return OXQ_ERR_UNSUPPORTED;
     PackedMxParams p = {};
     p.bias = bias; p.y = y; p.bias_dtype = bias_dtype; p.y_dtype = y_dtype;

@@ -96,6 +96,37 @@ def test_fp8_block_scaled_special_values_stay_special(cuda):
     assert np.isfinite(y[np.ix_(rows, cols)]).all()
 
 
+# folds of 64 and of 128 columns; merged pieces, two MMAs, several token blocks; scratch from the least that is taken (the pieces and
+# their block scales) to all that helps
+@pytest.mark.parametrize("m,n,k,s_out,s_in", [(512, 512, 1024, 4, 16), (512, 512, 1024, 4, 8), (20, 256, 512, 2, 8), (65, 128, 256, 1, 4)])
+def test_fp8_block_scaled_stays_inside_its_scratch(cuda, m, n, k, s_out, s_in):
+    w8, scale, w = fp8_weights(n, k, s_out, s_in, seed=m)
+    x = synth.activations(m, k, seed=m)
+    xd, wd, sd = bf16(x), torch.from_numpy(w8).cuda(), torch.from_numpy(scale).cuda()
+    blocks = -(-m // 128)
+    mpad = -(-(-(-m // blocks)) // 16) * 16
+    up = lambda v: -(-v // 256) * 256  # noqa: E731
+    least = up(2 * blocks * mpad * k) + up(k // 128 * blocks * (512 if mpad <= 32 else 1024))
+    full = int(_lib.load().oxq_fp8_scratch_bytes(m, k, n, s_out, s_in))
+    assert least < full
+    for size in sorted({least, least + 256, least + (full - least) // 3, full, min(full, 1105920)}):
+        if size < least:
+            continue
+        room = torch.full((256 + full + (1 << 20),), 0xA5, dtype=torch.uint8, device="cuda")
+        room[:256] = 0
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        args = (xd.data_ptr(), _lib.OXQ_BF16, wd.data_ptr(), sd.data_ptr(), s_out, s_in, 0, _lib.OXQ_F32, y.data_ptr(), _lib.OXQ_F32, m, k, n)
+        _lib.call("oxq_fp8_matmul", *args, room.data_ptr(), room.data_ptr() + 256, size, None)
+        gemm.check(room)
+        close(y, x, w)
+        assert (room[256 + size:] == 0xA5).all()
+        if 256 + size >= int(_lib.load().oxq_gemm_workspace_bytes(n, k)):  # the same kernel inside a workspace
+            room[256:] = 0xA5
+            _lib.call("oxq_fp8_gemm", *args, room.data_ptr(), 256 + size, None)
+            gemm.check(room)
+            assert (room[256 + size:] == 0xA5).all()
+
+
 @pytest.mark.parametrize("m", [9, 16])
 def test_fp8_decode_takes_x_on_any_8_bytes(cuda, m):
     n, k = 256, 512

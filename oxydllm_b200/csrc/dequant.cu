@@ -230,11 +230,11 @@ __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi)
 // ((2^23 + q) - (2^23 + z)), multiplied by the scale in f32 and rounded to bf16 once, as the
 // element-wise kernel does. Needs group_size % 16 == 0 and k % 16 == 0.
 __global__ void __launch_bounds__(256)
-awq_slab16_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__restrict__ qzeros,
-                       const void *__restrict__ scales, int scales_dtype, __nv_bfloat16 *__restrict__ out, int k,
+awq_slab16_bf16_kernel(const uint32_t *qweight, const uint32_t *qzeros,
+                       const void *scales, int scales_dtype, __nv_bfloat16 *out, int k,
                        int n_cnt, int group_size, int n_full, int n_off, int vec_ok, int row_mul, int row_add)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    qweight += pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
     pdl_launch_dependents();
     __shared__ __align__(16) uint32_t raw[128][32];
     __shared__ __align__(16) unsigned char stage[2][32 * 272];
@@ -274,7 +274,7 @@ awq_slab16_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__r
     for (int c = 0; c < 8; c++) sc[c] = 0.0f;
     if (active) {
         const int g = kb / group_size;
-        zw = __ldg(qzeros + (size_t)g * packed_full + j);
+        zw = ld_produced(qzeros + (size_t)g * packed_full + j);
         const size_t s0 = (size_t)g * n_full + (size_t)j * 8;
 #pragma unroll
         for (int c = 0; c < 8; c++) sc[c] = load_as_f32(scales, scales_dtype, s0 + c);
@@ -325,20 +325,21 @@ awq_slab16_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__r
 // A CTA covers 256 * 16 columns of FP8_SLAB_ROWS rows.
 constexpr int FP8_SLAB_ROWS = 4;
 __global__ void __launch_bounds__(256)
-fp8_slab16_bf16_kernel(const uint8_t *__restrict__ weight, const float *__restrict__ scale_inv, int s_in, int block_out,
-                       int block_in, __nv_bfloat16 *__restrict__ out, int n_cnt, int k, int row_off)
+fp8_slab16_bf16_kernel(const uint8_t *weight, const float *scale_inv, int s_in, int block_out,
+                       int block_in, __nv_bfloat16 *out, int n_cnt, int k, int row_off)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    const uint32_t zero = pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
+    weight += zero;
     pdl_launch_dependents();
     const int c16 = blockIdx.x * 256 + threadIdx.x;
     if (c16 * 16 >= k) return;
-    const int kb = scale_inv ? (c16 * 16) / block_in : 0;
+    const int kb = scale_inv ? (int)zero + (c16 * 16) / block_in : 0;
 #pragma unroll
     for (int r = 0; r < FP8_SLAB_ROWS; r++) {
         const int row = blockIdx.y * FP8_SLAB_ROWS + r;
         if (row >= n_cnt) break;
         const uint4 wv = __ldcs(reinterpret_cast<const uint4 *>(weight + (size_t)row * k) + c16);
-        const float s = scale_inv ? __ldg(scale_inv + (size_t)((row_off + row) / block_out) * s_in + kb) : 1.0f;
+        const float s = scale_inv ? ld_ordered(scale_inv + (size_t)((row_off + row) / block_out) * s_in + kb) : 1.0f;
         const uint32_t v[4] = {wv.x, wv.y, wv.z, wv.w};
         uint32_t o[8];
 #pragma unroll
@@ -432,22 +433,22 @@ mxfp4_slab16_bf16_kernel(const uint8_t *__restrict__ blocks, const uint8_t *__re
 // FIVE: the Q5_K layout (176 bytes, 32 bytes of fifth bits after the header: bit j of qh[el] belongs to sub-block j).
 template <bool FIVE>
 __global__ void __launch_bounds__(256)
-q4k_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_groups)
+q4k_slab_bf16_kernel(const uint8_t *blocks, __nv_bfloat16 *out, size_t total_groups)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    blocks += pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
     pdl_launch_dependents();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_groups;
          idx += (size_t)gridDim.x * blockDim.x) {
         const size_t sb = idx >> 2;
         const int iq = (int)(idx & 3);
         const uint8_t *blk = blocks + sb * (FIVE ? 176 : 144);
-        const uint4 hdr = __ldg(reinterpret_cast<const uint4 *>(blk));
+        const uint4 hdr = ld_ordered(reinterpret_cast<const uint4 *>(blk));
         const uint4 qa = __ldcs(reinterpret_cast<const uint4 *>(blk + (FIVE ? 48 : 16) + 32 * iq));
         const uint4 qb = __ldcs(reinterpret_cast<const uint4 *>(blk + (FIVE ? 64 : 32) + 32 * iq));
         uint4 ha = make_uint4(0u, 0u, 0u, 0u), hb = ha;
         if (FIVE) {
-            ha = __ldg(reinterpret_cast<const uint4 *>(blk + 16));
-            hb = __ldg(reinterpret_cast<const uint4 *>(blk + 32));
+            ha = ld_ordered(reinterpret_cast<const uint4 *>(blk + 16));
+            hb = ld_ordered(reinterpret_cast<const uint4 *>(blk + 32));
         }
         const uint32_t qhw[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w}; // byte t = fifth bits of element t
         const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xFFFFu)));
@@ -502,18 +503,18 @@ __device__ __forceinline__ float small_int_f32(int v) // |v| < 2^22
 }
 
 __global__ void __launch_bounds__(256)
-q80_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_blocks)
+q80_slab_bf16_kernel(const uint8_t *blocks, __nv_bfloat16 *out, size_t total_blocks)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    blocks += pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
     pdl_launch_dependents();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_blocks;
          idx += (size_t)gridDim.x * blockDim.x) {
         const unsigned short *h = reinterpret_cast<const unsigned short *>(blocks + idx * 34);
-        const float d = __half2float(__ushort_as_half(__ldg(h)));
+        const float d = __half2float(__ushort_as_half(ld_ordered(h)));
         uint32_t o[16];
 #pragma unroll
         for (int t = 0; t < 16; t++) {
-            const uint32_t two = __ldg(h + 1 + t); // elements 2t, 2t+1
+            const uint32_t two = ld_ordered(h + 1 + t); // elements 2t, 2t+1
             const float a = __fmul_rn(small_int_f32((int)(signed char)(two & 0xFFu)), d);
             const float b = __fmul_rn(small_int_f32((int)(signed char)(two >> 8)), d);
             o[t] = pack_bf16x2_rn(a, b);
@@ -527,9 +528,9 @@ q80_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
 // V = 0 Q4_0 {d; qs} 18 B, 1 Q4_1 {d; m; qs} 20 B, 2 Q5_0 {d; qh; qs} 22 B, 3 Q5_1 {d; m; qh; qs} 24 B.
 template <int V>
 __global__ void __launch_bounds__(256)
-q40_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_blocks)
+q40_slab_bf16_kernel(const uint8_t *blocks, __nv_bfloat16 *out, size_t total_blocks)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    blocks += pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
     pdl_launch_dependents();
     constexpr bool HAS_MIN = V == 1 || V == 3, FIVE = V >= 2;
     constexpr int BLK = 18 + 2 * V, QH = (HAS_MIN ? 4 : 2) / 2, QS = (2 + (HAS_MIN ? 2 : 0) + (FIVE ? 4 : 0)) / 2; // halfword offsets
@@ -537,9 +538,9 @@ q40_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_blocks;
          idx += (size_t)gridDim.x * blockDim.x) {
         const unsigned short *h = reinterpret_cast<const unsigned short *>(blocks + idx * BLK);
-        const float d = __half2float(__ushort_as_half(__ldg(h)));
-        const float mn = HAS_MIN ? __half2float(__ushort_as_half(__ldg(h + 1))) : 0.0f;
-        const uint32_t qh = FIVE ? ((uint32_t)__ldg(h + QH) | ((uint32_t)__ldg(h + QH + 1) << 16)) : 0u;
+        const float d = __half2float(__ushort_as_half(ld_ordered(h)));
+        const float mn = HAS_MIN ? __half2float(__ushort_as_half(ld_ordered(h + 1))) : 0.0f;
+        const uint32_t qh = FIVE ? ((uint32_t)ld_ordered(h + QH) | ((uint32_t)ld_ordered(h + QH + 1) << 16)) : 0u;
         auto value = [&](int q) -> float {
             const float v = __fmul_rn(small_int_f32(q - OFF), d);
             return HAS_MIN ? __fadd_rn(v, mn) : v;
@@ -547,7 +548,7 @@ q40_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
         uint32_t lo[8], hi[8]; // elements 0..15 (low nibbles) and 16..31 (high nibbles)
 #pragma unroll
         for (int t = 0; t < 8; t++) {
-            const uint32_t two = __ldg(h + QS + t); // bytes 2t, 2t+1
+            const uint32_t two = ld_ordered(h + QS + t); // bytes 2t, 2t+1
             const int b0 = (int)(two & 0xFFu), b1 = (int)(two >> 8);
             const int f0 = (int)((qh >> (2 * t)) & 1u) << 4, f1 = (int)((qh >> (2 * t + 1)) & 1u) << 4;
             const int g0 = (int)((qh >> (16 + 2 * t)) & 1u) << 4, g1 = (int)((qh >> (17 + 2 * t)) & 1u) << 4;
@@ -564,9 +565,9 @@ q40_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
 
 // Q6_K: a thread takes the 16 weights that share one scale: super-block sb, half h, quad q, sixteen s.
 __global__ void __launch_bounds__(256)
-q6k_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restrict__ out, size_t total_groups)
+q6k_slab_bf16_kernel(const uint8_t *blocks, __nv_bfloat16 *out, size_t total_groups)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    blocks += pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
     pdl_launch_dependents();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_groups;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -575,13 +576,14 @@ q6k_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
         const uint8_t *blk = blocks + sb * 210;
         const unsigned short *ql = reinterpret_cast<const unsigned short *>(blk + 64 * h + 32 * (q & 1) + 16 * s);
         const unsigned short *qh = reinterpret_cast<const unsigned short *>(blk + 128 + 32 * h + 16 * s);
-        const float d = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(blk + 208))));
-        const int sc = (int)(signed char)blk[192 + 8 * h + 2 * q + s];
+        const float d = __half2float(__ushort_as_half(ld_ordered(reinterpret_cast<const unsigned short *>(blk + 208))));
+        const unsigned short sc2 = ld_ordered(reinterpret_cast<const unsigned short *>(blk + 192 + 8 * h + 2 * q));
+        const int sc = (int)(signed char)(sc2 >> (8 * s));
         const float ds = __fmul_rn(d, small_int_f32(sc));
         uint32_t o[8];
 #pragma unroll
         for (int t = 0; t < 8; t++) {
-            const uint32_t l2 = __ldg(ql + t), h2 = __ldg(qh + t); // bytes for elements 2t, 2t+1
+            const uint32_t l2 = ld_ordered(ql + t), h2 = ld_ordered(qh + t); // bytes for elements 2t, 2t+1
             const int n0 = (int)((l2 >> (q < 2 ? 0 : 4)) & 0x0Fu), n1 = (int)((l2 >> (q < 2 ? 8 : 12)) & 0x0Fu);
             const int b0 = (int)((h2 >> (2 * q)) & 3u), b1 = (int)((h2 >> (8 + 2 * q)) & 3u);
             o[t] = pack_bf16x2_rn(__fmul_rn(ds, small_int_f32((n0 | (b0 << 4)) - 32)),
@@ -599,11 +601,11 @@ q6k_slab_bf16_kernel(const uint8_t *__restrict__ blocks, __nv_bfloat16 *__restri
 // walk the word rows, so every column is stored as 512 contiguous bytes. Arithmetic as in the
 // element-wise kernel: (q - (zero + 1)) * scale in f32, one rounding. Needs group_size % 8 == 0.
 __global__ void __launch_bounds__(256)
-gptq4_slab_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__restrict__ qzeros,
-                       const void *__restrict__ scales, int scales_dtype, __nv_bfloat16 *__restrict__ out, int k,
+gptq4_slab_bf16_kernel(const uint32_t *qweight, const uint32_t *qzeros,
+                       const void *scales, int scales_dtype, __nv_bfloat16 *out, int k,
                        int n_cnt, int group_size, int sym, int n_full, int n_off)
 {
-    pdl_wait(); // the slab may still be read by the kernel ahead
+    qweight += pdl_wait_zero(); // the slab may still be read by the kernel ahead, which may also write weights
     pdl_launch_dependents();
     __shared__ uint32_t tile[32][33];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -617,22 +619,26 @@ gptq4_slab_bf16_kernel(const uint32_t *__restrict__ qweight, const uint32_t *__r
     const int kp = kp0 + lane;
     if (kp >= kwords) return;
     const int g = (kp * 8) / group_size;
+    uint32_t zero[4]; // all loads ahead of the first store
+    float sc[4];
+#pragma unroll
+    for (int it = 0; it < 4; it++) {
+        const int col = c0 + warp * 4 + it, o = n_off + min(col, n_cnt - 1);
+        zero[it] = sym ? 7u : (ld_produced(qzeros + (size_t)g * (n_full >> 3) + (o >> 3)) >> ((o & 7) * 4)) & 15u;
+        sc[it] = load_as_f32(scales, scales_dtype, (size_t)g * n_full + o);
+    }
 #pragma unroll
     for (int it = 0; it < 4; it++) {
         const int cl = warp * 4 + it, col = c0 + cl;
         if (col >= n_cnt) break;
-        const int o = n_off + col;
-        uint32_t zero = 7u;
-        if (!sym) zero = (__ldg(qzeros + (size_t)g * (n_full >> 3) + (o >> 3)) >> ((o & 7) * 4)) & 15u;
-        const float sc = load_as_f32(scales, scales_dtype, (size_t)g * n_full + o);
-        const float zf = __uint_as_float(0x4B000000u | (zero + 1u)); // 2^23 + zero + 1
+        const float zf = __uint_as_float(0x4B000000u | (zero[it] + 1u)); // 2^23 + zero + 1
         const uint32_t w = tile[lane][cl];
         uint32_t o4[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const float a = __uint_as_float(0x4B000000u | ((w >> (8 * j)) & 15u)) - zf;
             const float b = __uint_as_float(0x4B000000u | ((w >> (8 * j + 4)) & 15u)) - zf;
-            o4[j] = pack_bf16x2_rn(__fmul_rn(a, sc), __fmul_rn(b, sc));
+            o4[j] = pack_bf16x2_rn(__fmul_rn(a, sc[it]), __fmul_rn(b, sc[it]));
         }
         *reinterpret_cast<uint4 *>(out + (size_t)col * k + (size_t)kp * 8) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
     }

@@ -137,12 +137,40 @@ __device__ __forceinline__ float bf16_hi_f32(uint32_t w) { return __uint_as_floa
 // allow_early_start(), a kernel may become resident while the previous kernel on the stream is still
 // running; it calls pdl_launch_dependents() at entry (so that its own successor may do the same) and
 // pdl_wait() before it touches anything a previous kernel may write or still read (x, y, routing
-// tables). Only reads of weights, scales and zero points, which no kernel writes, go in front of
-// the wait. pdl_wait() returns when the previous kernel has completed and its writes are visible;
+// tables). Only the GEMVs that include/oxq.h names read weights, scales and zero points, which there no
+// kernel just ahead writes, in front of the wait or through the read-only path; every other kernel takes
+// them from the stream's order. pdl_wait() returns when the previous kernel has completed and its writes are visible;
 // without the launch attribute both calls do nothing.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// pdl_wait() with a zero for result that is known only behind it: no compiler moves a load from an address it is added to in front of
+// the wait, however the load is written (a streaming load has no other order with the wait). For kernels that must not read weights early.
+__device__ __forceinline__ uint32_t pdl_wait_zero()
+{
+    uint32_t zero;
+    asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
+    return zero;
+}
+// Loads for addresses that carry that zero: ordinary ones, but free to move among the stores around them.
+__device__ __forceinline__ unsigned short ld_ordered(const unsigned short *p)
+{
+    unsigned short v;
+    asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_ordered(const uint4 *p)
+{
+    uint4 v;
+    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ float ld_ordered(const float *p)
+{
+    float v;
+    asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
 // What a kernel ahead writes (x, a routing table, another projection's result) is read by an ordinary load behind pdl_wait(). The
 // read-only path of __ldg is for data that nobody writes while the kernel runs, and one that starts early runs while x is written.
 template <typename T> __device__ __forceinline__ T ld_produced(const T *p) { return *p; }

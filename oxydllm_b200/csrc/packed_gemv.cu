@@ -62,7 +62,7 @@ template <int BITS, int MT>
 __global__ void __launch_bounds__(PG_WARPS * 32) gptq_gemv_kernel(const PackedGemvParams p)
 {
     pdl_launch_dependents();
-    pdl_wait(); // x is staged first: only the start-up of the kernel overlaps the previous one
+    const uint32_t *qweight = p.qweight + pdl_wait_zero(); // x is staged first: only the start-up of the kernel overlaps the previous one
     constexpr int PF = 32 / BITS;
     constexpr uint32_t QMASK = (1u << BITS) - 1u;
     extern __shared__ __align__(16) float smem_f[];
@@ -85,11 +85,11 @@ __global__ void __launch_bounds__(PG_WARPS * 32) gptq_gemv_kernel(const PackedGe
         const float s = load_as_f32(p.scales, p.scales_dtype, (size_t)g * p.n + c);
         float zero;
         if (p.sym || p.qzeros == nullptr) zero = (float)(1u << (BITS - 1));
-        else zero = (float)(((__ldg(p.qzeros + (size_t)g * (p.n / PF) + c / PF) >> (BITS * (c % PF))) & QMASK) + 1u);
+        else zero = (float)(((ld_produced(p.qzeros + (size_t)g * (p.n / PF) + c / PF) >> (BITS * (c % PF))) & QMASK) + 1u);
         float acc[MT];
 #pragma unroll
         for (int t = 0; t < MT; t++) acc[t] = 0.0f;
-        const uint32_t *wp = p.qweight + (size_t)g * wpg * p.n + c;
+        const uint32_t *wp = qweight + (size_t)g * wpg * p.n + c;
         const float *xg = xs + (size_t)g * p.group_size;
 #pragma unroll 4
         for (int wi = 0; wi < wpg; wi++) {
@@ -135,7 +135,7 @@ template <int MT>
 __global__ void __launch_bounds__(PG_WARPS * 32) w8a16_gemv_kernel(const PackedGemvParams p)
 {
     pdl_launch_dependents();
-    pdl_wait(); // x is staged first: only the start-up of the kernel overlaps the previous one
+    const uint32_t *qweight = p.qweight + pdl_wait_zero(); // x is staged first: only the start-up of the kernel overlaps the previous one
     extern __shared__ __align__(16) float smem_f[];
     const int groups = p.k / p.group_size;
     float *xs = smem_f, *gsum = xs + (size_t)MT * p.k, *red = gsum + MT * groups;
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(PG_WARPS * 32) w8a16_gemv_kernel(const PackedG
 #pragma unroll
         for (int t = 0; t < MT; t++) tot[cc][t] = 0.0f;
     for (int g = g0; g < g1; g++) {
-        const uint32_t zw = __ldg(p.qzeros + (size_t)g * packed_out + j);
+        const uint32_t zw = ld_produced(p.qzeros + (size_t)g * packed_out + j);
         float s[4], zero[4];
 #pragma unroll
         for (int cc = 0; cc < 4; cc++) {
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(PG_WARPS * 32) w8a16_gemv_kernel(const PackedG
         for (int cc = 0; cc < 4; cc++)
 #pragma unroll
             for (int t = 0; t < MT; t++) acc[cc][t] = 0.0f;
-        const uint32_t *wp = p.qweight + (size_t)g * p.group_size * packed_out + j;
+        const uint32_t *wp = qweight + (size_t)g * p.group_size * packed_out + j;
         const float *xg = xs + (size_t)g * p.group_size;
 #pragma unroll 8
         for (int i = 0; i < p.group_size; i++) {
@@ -233,7 +233,7 @@ constexpr int GQ_TILES = 2; // 16-column tiles per warp: a CTA covers 32 output 
 __global__ void __launch_bounds__(PG_WARPS * 32) gptq4_gemv_mma_kernel(const PackedGemvParams p)
 {
     pdl_launch_dependents();
-    pdl_wait(); // x is staged first: only the start-up of the kernel overlaps the previous one
+    const uint32_t *qweight = p.qweight + pdl_wait_zero(); // x is staged first: only the start-up of the kernel overlaps the previous one
     extern __shared__ __align__(16) unsigned char smem_b[];
     const int groups = p.k / p.group_size;
     const int mloc = min(8, p.m - p.y_row0);
@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(PG_WARPS * 32) gptq4_gemv_mma_kernel(const Pac
             if (st0 + u < steps) {
 #pragma unroll
                 for (int t = 0; t < GQ_TILES; t++) {
-                    wbuf[u][t][0] = __ldcs(p.qweight + (prow0 + (size_t)4 * (st0 + u)) * p.n + col[t][0]);
-                    wbuf[u][t][1] = __ldcs(p.qweight + (prow0 + (size_t)4 * (st0 + u)) * p.n + col[t][1]);
+                    wbuf[u][t][0] = __ldcs(qweight + (prow0 + (size_t)4 * (st0 + u)) * p.n + col[t][0]);
+                    wbuf[u][t][1] = __ldcs(qweight + (prow0 + (size_t)4 * (st0 + u)) * p.n + col[t][1]);
                 }
             }
     };
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(PG_WARPS * 32) gptq4_gemv_mma_kernel(const Pac
                 const int cc = col[t][hrow];
                 sc[t][hrow] = load_as_f32(p.scales, p.scales_dtype, (size_t)gi * p.n + cc);
                 if (p.sym || p.qzeros == nullptr) zr[t][hrow] = 8.0f;
-                else zr[t][hrow] = (float)(((__ldg(p.qzeros + (size_t)gi * (p.n >> 3) + (cc >> 3)) >> (4 * (cc & 7))) & 0xFu) + 1u);
+                else zr[t][hrow] = (float)(((ld_produced(p.qzeros + (size_t)gi * (p.n >> 3) + (cc >> 3)) >> (4 * (cc & 7))) & 0xFu) + 1u);
             }
         const uint4 *xrow = has_tok ? reinterpret_cast<const uint4 *>(xs + (size_t)g * p.k + (size_t)gi * p.group_size) + c : zeros;
         const int xinc = has_tok ? 4 : 0;

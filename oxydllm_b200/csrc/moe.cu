@@ -14,11 +14,11 @@ int gemm_grouped(const void *a, int a_rows, const void *w, int slab_experts, int
                  const int4 *entries, const int *grp_beg, int group, const void *bias, int bias_dtype, void *out,
                  int ldo, int epi, float limit, int *flag, cudaStream_t stream);
 
-int moe_fused_block_rows();
+int moe_fused_block_rows(int rows);
 bool moe_fused_supported(int n, int k, const void *blocks, const void *scales, const void *a, const void *out, int ldo);
 int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
-                      const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi,
-                      float limit, int *flag, cudaStream_t st);
+                      const int4 *entries, const int *n_blocks, int block_rows, const void *bias, int bias_dtype, void *out, int ldo,
+                      int epi, float limit, int *flag, cudaStream_t st);
 
 int moe_mx_block_rows();
 size_t moe_mx_piece_bytes(int rows, int k);
@@ -44,10 +44,11 @@ constexpr int MOE_DECODE_MAX_PAIRS = 64;
 // is the same bits alone and in a batch.
 constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
 // Rows per expert, on average, up to which the block-scaled kernel is the better one: above, most experts take two of its blocks of 48
-// rows, and the kernel that unpacks once for up to 192 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
+// rows, and the kernel that unpacks once for up to 192 or 256 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
 // 300, 384, 450 tokens: 124 / 183, 149 / 221, 169 / 228, 186 / 235, 237 / 240, 277 / 245; 16 of 2048 x 1024 at 30, 120, 200: 43 / 64,
 // 49 / 67, 70 / 70. Both have come down by about a tenth since (340 tokens 170 here, 400 tokens 204 there).
 constexpr int MOE_MX_ROWS = 44;
+constexpr int MOE_BLOCK_ROWS = 192; // of a token block of the kernel that unpacks, but for one per expert that may be larger
 
 // One warp per token: f32 softmax over all experts, k rounds of arg-max (ties: lower index),
 // optional renormalisation by the sum of the selected probabilities (moe.rs:472-487).
@@ -173,20 +174,33 @@ __device__ __forceinline__ int2 moe_block_scan(int2 v, int *scratch)
 }
 
 // Offsets (exclusive scan of counts) and token blocks for the kernel that unpacks MXFP4 inside the tensor-core loop: every
-// expert's rows cut into the fewest blocks of at most max_rows rows, of equal size rounded up to 16. n_blocks[0] = how many.
-// Thread i is expert i (one thread walking 32 experts took 10 us). Returns the expert's first row.
+// expert's rows cut into the fewest blocks of at most max_rows rows, of equal size rounded up to 16; above MOE_BLOCK_ROWS that limit holds for
+// one block, and only where it saves one (see moe_fused_block_rows). n_blocks[0] = how many. Thread i is expert i (one thread walking 32
+// experts took 10 us). Returns the expert's first row.
 __device__ __forceinline__ int moe_plan_expert(int c, int n_exp, int e_lo, int max_rows, int *offsets, int4 *entries, int *n_blocks,
                                                int *scratch)
 {
     const int i = threadIdx.x;
-    const int parts = (c + max_rows - 1) / max_rows;
-    const int size = parts ? ((c + parts - 1) / parts + 15) / 16 * 16 : 1;
-    const int blocks = (c + size - 1) / size;
+    int size, first;
+    if (c > MOE_BLOCK_ROWS && (c - 1) % MOE_BLOCK_ROWS < max_rows - MOE_BLOCK_ROWS) { // one larger block instead of two smaller ones
+        size = MOE_BLOCK_ROWS;
+        first = c - (c / MOE_BLOCK_ROWS - 1) * MOE_BLOCK_ROWS;
+    } else {
+        max_rows = min(max_rows, MOE_BLOCK_ROWS);
+        const int parts = (c + max_rows - 1) / max_rows;
+        size = parts ? ((c + parts - 1) / parts + 15) / 16 * 16 : 1;
+        first = min(size, c);
+    }
+    const int blocks = c ? 1 + (c - first + size - 1) / size : 0;
     const int2 incl = moe_block_scan(make_int2(c, blocks), scratch);
     const int off = incl.x - c;
     if (i < n_exp) {
         offsets[i] = off;
-        for (int q = 0; q < blocks; q++) entries[incl.y - blocks + q] = make_int4(off + q * size, min(size, c - q * size), e_lo + i, 0);
+        for (int q = 0, r = 0; q < blocks; q++) {
+            const int rows = q ? min(size, c - r) : first;
+            entries[incl.y - blocks + q] = make_int4(off + r, rows, e_lo + i, 0);
+            r += rows;
+        }
         if (i == n_exp - 1) offsets[n_exp] = incl.x, n_blocks[0] = incl.y;
     }
     return off;
@@ -563,7 +577,7 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     }
     // the grouped kernel's table of token blocks goes where the m-tile table of the dense path would (same capacity bound);
     // grp_beg[0] then holds the number of blocks
-    const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows();
+    const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows(pairs / n_exp);
     if ((fused || mx) && pairs <= MOE_SMALL_PAIRS) {
         OXQ_CUDA(launch_early(moe_dispatch_small_kernel, 1, 1024, st, top_idx, pairs, expert_lo, n_exp, block_rows, counts, offsets, entries,
                               grp_beg, perm, inv));
@@ -595,11 +609,11 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     OXQ_LAUNCH_CHECK("moe routing kernels");
 
     if (fused) {
-        int rc = moe_fused_grouped(xs, a_rows, gu_blocks, gu_scales, num_experts, 2 * inter, hidden, entries, grp_beg, gu_bias,
-                                   bias_dtype, h, inter, 1, limit, flag, st);
+        int rc = moe_fused_grouped(xs, a_rows, gu_blocks, gu_scales, num_experts, 2 * inter, hidden, entries, grp_beg, block_rows,
+                                   gu_bias, bias_dtype, h, inter, 1, limit, flag, st);
         if (rc) return rc;
-        rc = moe_fused_grouped(h, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg, dn_bias, bias_dtype,
-                               xs, hidden, 0, limit, flag, st);
+        rc = moe_fused_grouped(h, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg, block_rows, dn_bias,
+                               bias_dtype, xs, hidden, 0, limit, flag, st);
         if (rc) return rc;
         moe_combine_kernel<<<sm_count() * 8, 256, 0, st>>>(xs, top_idx, top_w, inv, tokens, top_k, hidden, expert_lo, expert_hi,
                                                          out, out_dtype);

@@ -3,27 +3,35 @@
 // Mirrors the expert half of MoeFeedForward::forward (moe.rs:466-499, dispatch_sparse 563-607) with the
 // experts' Mxfp4Linear weights (linear.rs, [experts, out, in / 32, 16] blocks + [experts, out, in / 32] scales).
 //
-// A unit of work is (token block of one expert: up to 192 expert-sorted rows) x (128 out features). The grid is
+// A unit of work is (token block of one expert: up to 192 or 256 expert-sorted rows) x (128 out features). The grid is
 // persistent: CTA b takes units b, b + grid, ... of a device-side table, feature tiles fastest, so that CTAs
 // running at the same time share their token block in L2. Stages of 64 input columns are counted over all units of
-// a CTA and go round eight slots. Per CTA:
+// a CTA and go round eight slots (blocks of up to 192 rows) or six. Per CTA:
 //   warp 0              TMA: boxes of packed nibbles (128 out features x 32 bytes);
 //   warp 2              TMA: the stage's tile of the activations ([rows, 64] bf16 in boxes of 64 rows, 128-byte swizzle);
 //   warps 4..19         unpack, four teams of four warps taking stages in turn: a thread turns the two 16-byte blocks
 //                       (32 weights each; E8M0 scale bytes read through L1/L2) of one out feature into bf16 weights, the bits the
 //                       dequantization kernel writes, and stores them as 32 columns of its lane of tensor memory, where the
 //                       team has room for one stage;
-//   warp 1              tcgen05.mma kind::f16, A = weights [128, 64] from tensor memory, B = activations, D[128, rows] f32 in one
-//                       of two tensor-memory buffers for the whole of k; one commit per stage frees its slot and its weights;
+//   warp 1              tcgen05.mma kind::f16, A = weights [128, 64] from tensor memory, B = activations, D[128, rows] f32 in tensor
+//                       memory for the whole of k; the accumulators of successive units follow one another round a ring of six
+//                       chunks of 64 columns (two MMAs where one crosses its end); one commit per stage frees its slot and its weights;
 //   warps 20..23        epilogue of the previous unit while the next one accumulates: accumulator rows (out
 //                       features) -> + bias -> bf16 out[row, feature], or the clamped SwiGLU of GPT-OSS on
 //                       interleaved (gate, up) features -> out[row, feature / 2].
 // What bounds it: the unpack, about 640 clocks per stage for 350 of MMA at 176 rows. With the weights in shared memory a stage of 256 rows
 // moved 104 KB through it at 128 bytes a clock, 812 clocks for 512 of MMA, and a team could not start before its slot was free; now only
-// the store waits for that. 192 rows, because the weights of four stages (128 columns) and two accumulators have to fit 512 columns of
-// tensor memory. us a layer at 400 / 1024 / 4096 tokens, 32 experts of 2880 x 2880: 219 / 274 / 767 before, 204 / 247 / 738 now; 16 of 2048 x
-// 1024 at 200 tokens 63 / 57. Scale bytes a stage ahead and a swizzle against the bank conflicts of the packed rows gave nothing more.
+// the store waits for that. The weights of four stages take 128 columns of tensor memory, which leaves 384 for accumulators: two of 192
+// columns. A stage costs the unpack whatever its rows, so that an expert of 193 to 256 rows wants one block: the epilogue of 256 rows
+// takes about 8000 clocks, and hands back its columns a chunk at a time, so that the next block of 256 starts when half of it is done.
+// us a layer at 400 / 1024 / 1600 / 1800 / 3300 / 4096 tokens, 32 experts of 2880 x 2880: weights in shared memory, blocks of 256 rows
+// 236 / 283 / 338 / 374 / 655 / 784; blocks of 192 only 200 / 242 / 376 / 418 / 669 / 759; now 197 / 246 / 341 / 373 / 628 / 754.
+// 16 of 2048 x 1024 at 900 tokens 102 / 104 / 97. Scale bytes a stage ahead and a swizzle against the bank conflicts of the packed rows
+// gave nothing more; nor did a ring of 192-row entries of which a larger block takes two, up to 384 rows: with two accumulators at
+// once nothing hides the epilogue (4096 tokens 850).
 // Every wait is bounded and reports through the workspace flag word.
+#include <type_traits>
+
 #include <cuda_bf16.h>
 
 #include "mx_common.cuh"
@@ -44,19 +52,18 @@ constexpr int MF_BK = 64;                      // input columns per stage
 constexpr int MF_UNPACK_WARPS = 16, MF_TEAMS = 4, MF_TEAM_WARPS = 4; // four teams: a stage's chain of poll, unpack and arrival overlaps with three others
 constexpr int MF_EPI_WARPS = 4;
 constexpr int MF_THREADS = (4 + MF_UNPACK_WARPS + MF_EPI_WARPS) * 32;
-constexpr int MF_SLOTS = 8;                    // stages on their way: packed weights and activations, barriers
-constexpr int MF_MAX_TOK = 192;                // rows of a token block
-constexpr int MF_TMEM_BUF = MF_MAX_TOK;        // accumulator columns per buffer
-constexpr int MF_TMEM_A = 2 * MF_TMEM_BUF, MF_A_COLS = MF_BK / 2; // a team's unpacked weights, two to a column
-constexpr int MF_XBOX_ROWS = 64, MF_XBOX_BYTES = MF_XBOX_ROWS * MF_BK * 2, MF_X_BYTES = MF_MAX_TOK * MF_BK * 2; // activation rows travel in boxes of 64
+// Stages on their way (packed weights and activations, barriers) for blocks of at most MAX_TOK rows: as many as shared memory holds.
+template <int MAX_TOK> constexpr int MF_SLOTS = MAX_TOK <= 192 ? 8 : 6;
+constexpr int MF_CHUNKS = 6, MF_CHUNK = 64;    // accumulator columns are a ring of chunks
+constexpr int MF_TMEM_A = MF_CHUNKS * MF_CHUNK, MF_A_COLS = MF_BK / 2; // a team's unpacked weights, two to a column
+constexpr int MF_XBOX_ROWS = 64, MF_XBOX_BYTES = MF_XBOX_ROWS * MF_BK * 2; // activation rows travel in boxes of 64
 constexpr int MF_RAW_BYTES = MF_ROWS * MF_BK / 2;
-constexpr int MF_NUM_BARS = 4 * MF_SLOTS + 4;
 static_assert(MF_TMEM_A + MF_TEAMS * MF_A_COLS <= 512, "tensor memory");
-static_assert(MF_SLOTS == 2 * MF_TEAMS, "a team meets two slots in turn");
+static_assert(MF_SLOTS<256> > MF_TEAMS, "the slot of a team's stage before is another one");
 constexpr int MF_SMEM_BUDGET = 227 * 1024;
 
 struct MoeFusedParams {
-    const int4 *entries;   // token blocks: {first row in the expert-sorted matrix, rows (<= 256), expert, -}
+    const int4 *entries;   // token blocks: {first row in the expert-sorted matrix, rows, expert, -}
     const int *n_blocks;   // how many
     const uint8_t *scales; // [experts, n, k / 32]
     const void *bias;      // [experts, n] or null
@@ -100,38 +107,41 @@ __device__ __forceinline__ void mf_arrive(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+template <int MAX_TOK>
 __global__ void __launch_bounds__(MF_THREADS, 1)
     moe_mxfp4_fused_kernel(const MoeFusedParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
 {
+    constexpr int SLOTS = MF_SLOTS<MAX_TOK>, X_BYTES = MAX_TOK * MF_BK * 2, NUM_BARS = 4 * SLOTS + 2 * MF_CHUNKS;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
     unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
     // activation slots | packed slots | barriers | tensor-memory address
-    const uint32_t x_base = base, raw_base = base + MF_SLOTS * MF_X_BYTES;
-    const uint32_t bars = raw_base + MF_SLOTS * MF_RAW_BYTES;
+    const uint32_t x_base = base, raw_base = base + SLOTS * X_BYTES;
+    const uint32_t bars = raw_base + SLOTS * MF_RAW_BYTES;
     auto rawfull_bar = [&](int r) { return bars + 8u * r; };
-    auto rawempty_bar = [&](int r) { return bars + 8u * (MF_SLOTS + r); };
+    auto rawempty_bar = [&](int r) { return bars + 8u * (SLOTS + r); };
     // full: the stage's weights are in tensor memory (one arrival per warp of the team) and its activation tile has landed (the
     // producer's arrival with the byte count); empty: the MMAs that read both have completed (one commit)
-    auto full_bar = [&](int s) { return bars + 8u * (2 * MF_SLOTS + s); };
-    auto empty_bar = [&](int s) { return bars + 8u * (3 * MF_SLOTS + s); };
-    const uint32_t misc = bars + 8u * (4 * MF_SLOTS);
-    auto tfull_bar = [&](int b) { return misc + 8u * b; };
-    auto tempty_bar = [&](int b) { return misc + 8u * (2 + b); };
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bars - base) + 8 * MF_NUM_BARS);
+    auto full_bar = [&](int s) { return bars + 8u * (2 * SLOTS + s); };
+    auto empty_bar = [&](int s) { return bars + 8u * (3 * SLOTS + s); };
+    const uint32_t misc = bars + 8u * (4 * SLOTS);
+    // per chunk: the accumulator that begins there is complete (one commit); the chunk has been read
+    auto tfull_bar = [&](int c) { return misc + 8u * c; };
+    auto tempty_bar = [&](int c) { return misc + 8u * (MF_CHUNKS + c); };
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(base_ptr + (bars - base) + 8 * NUM_BARS);
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n_units = __ldg(p.n_blocks) * p.tiles_n;
     const int nk2 = p.nk2;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < MF_SLOTS; s++) {
+        for (int s = 0; s < SLOTS; s++) {
             mbar_init(rawfull_bar(s), 1);
             mbar_init(rawempty_bar(s), MF_TEAM_WARPS);
             mbar_init(full_bar(s), MF_TEAM_WARPS + 1);
             mbar_init(empty_bar(s), 1);
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < MF_CHUNKS; b++) {
             mbar_init(tfull_bar(b), 1);
             mbar_init(tempty_bar(b), MF_EPI_WARPS);
         }
@@ -164,7 +174,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                     tma_load_2d(raw_base + r * MF_RAW_BYTES, &wmap, rawfull_bar(r), it * (MF_BK / 2), rowbase);
                 }
                 __syncwarp();
-                if (++r == MF_SLOTS) { r = 0; ph ^= 1u; }
+                if (++r == SLOTS) { r = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 2) {
@@ -179,15 +189,15 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
             for (int it = 0; it < nk2 && ok; it++) {
                 ok = mx_wait(empty_bar(xs), xph, p.flag, 5);
                 if (ok && leader) {
-                    const uint32_t dst = x_base + (uint32_t)xs * MF_X_BYTES;
+                    const uint32_t dst = x_base + (uint32_t)xs * X_BYTES;
                     mbar_arrive_expect_tx(full_bar(xs), (uint32_t)boxes * MF_XBOX_BYTES);
 #pragma unroll
-                    for (int b = 0; b < MF_MAX_TOK / MF_XBOX_ROWS; b++)
+                    for (int b = 0; b < MAX_TOK / MF_XBOX_ROWS; b++)
                         if (b < boxes)
                             tma_load_2d(dst + (uint32_t)b * MF_XBOX_BYTES, &xmap, full_bar(xs), it * MF_BK, en.x + b * MF_XBOX_ROWS);
                 }
                 __syncwarp();
-                if (++xs == MF_SLOTS) { xs = 0; xph ^= 1u; }
+                if (++xs == SLOTS) { xs = 0; xph ^= 1u; }
             }
         }
     } else if (warp == 1) {
@@ -196,30 +206,49 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
         // commit (empty) per stage.
         const bool leader = elect_one();
         const uint64_t db0 = kmajor_sw128_desc(x_base);
-        int s = 0, ul = 0;
-        uint32_t ph = 0;
+        int s = 0, team = 0, chunk = 0; // slot of a stage, team that unpacks it; first chunk of a unit
+        uint32_t ph = 0, cph = ~0u;     // bit c: parity of chunk c's last release (a fresh barrier passes 1)
         bool ok = true;
-        for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, ul++) {
-            const uint32_t idesc = tc_idesc(MF_ROWS, (__ldg(p.entries + u / p.tiles_n).y + 15) & ~15);
-            const uint32_t buf = (uint32_t)ul & 1u, d_tmem = tmem_base + buf * MF_TMEM_BUF;
-            ok = mx_wait(tempty_bar(buf), (((uint32_t)ul >> 1) & 1u) ^ 1u, p.flag, 8);
-            for (int it = 0; it < nk2 && ok; it++) {
-                ok = mx_wait(full_bar(s), ph, p.flag, 2);
-                if (ok) {
-                    tc_fence_after();
-                    const uint32_t a_tmem = tmem_base + MF_TMEM_A + (uint32_t)(s % MF_TEAMS) * MF_A_COLS;
-                    const uint64_t db = db0 + (uint64_t)(s * (MF_X_BYTES >> 4));
-                    if (leader) {
-#pragma unroll
-                        for (int kk = 0; kk < MF_BK / 16; kk++) // 16 input columns: 32 bytes inside a swizzled K-major row
-                            mf_umma(d_tmem, a_tmem + 8 * kk, db + 2 * kk, idesc, (it | kk) != 0);
-                        umma_commit(empty_bar(s));
-                    }
-                    __syncwarp();
-                }
-                if (++s == MF_SLOTS) { s = 0; ph ^= 1u; }
+        for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x) {
+            // (shuffled: known to be the same in all lanes, so that what depends on it stays in uniform registers)
+            const int mpad = __shfl_sync(0xFFFFFFFFu, (__ldg(p.entries + u / p.tiles_n).y + 15) & ~15, 0);
+            const int n1 = min(mpad, (MF_CHUNKS - chunk) * MF_CHUNK), n2 = mpad - n1; // columns up to the ring's end, and from its start on
+            const uint32_t idesc = tc_idesc(MF_ROWS, n1), idesc2 = tc_idesc(MF_ROWS, n2 ? n2 : 16), d_tmem = tmem_base + (uint32_t)(chunk * MF_CHUNK);
+            const int first = chunk;
+            bool free_all = true; // the polls of all chunks are under way together
+            for (int c0 = 0; c0 < mpad; c0 += MF_CHUNK) {
+                free_all &= mbar_test(tempty_bar(chunk), (cph >> chunk) & 1u);
+                cph ^= 1u << chunk;
+                if (++chunk == MF_CHUNKS) chunk = 0;
             }
-            if (ok && leader) umma_commit(tfull_bar(buf)); // the accumulator is complete once the unit's MMAs are
+            if (!__all_sync(0xFFFFFFFFu, free_all))
+                for (int c0 = 0, c = first; c0 < mpad && ok; c0 += MF_CHUNK, c = c + 1 == MF_CHUNKS ? 0 : c + 1)
+                    ok = mx_wait(tempty_bar(c), (~cph >> c) & 1u, p.flag, 8);
+            auto stages = [&](auto split_) {
+                for (int it = 0; it < nk2 && ok; it++) {
+                    ok = mx_wait(full_bar(s), ph, p.flag, 2);
+                    if (ok) {
+                        tc_fence_after();
+                        const uint32_t a_tmem = tmem_base + MF_TMEM_A + (uint32_t)team * MF_A_COLS;
+                        const uint64_t db = db0 + (uint64_t)(s * (X_BYTES >> 4));
+                        if (leader) {
+#pragma unroll
+                            for (int kk = 0; kk < MF_BK / 16; kk++) { // 16 input columns: 32 bytes inside a swizzled K-major row
+                                mf_umma(d_tmem, a_tmem + 8 * kk, db + 2 * kk, idesc, (it | kk) != 0);
+                                if constexpr (decltype(split_)::value)
+                                    mf_umma(tmem_base, a_tmem + 8 * kk, db + (uint64_t)(n1 * (MF_BK * 2 >> 4)) + 2 * kk, idesc2, (it | kk) != 0);
+                            }
+                            umma_commit(empty_bar(s));
+                        }
+                        __syncwarp();
+                    }
+                    if (++team == MF_TEAMS) team = 0;
+                    if (++s == SLOTS) { s = 0; ph ^= 1u; }
+                }
+            };
+            if (n2) stages(std::true_type{});
+            else stages(std::false_type{});
+            if (ok && leader) umma_commit(tfull_bar(first)); // the accumulator is complete once the unit's MMAs are
             __syncwarp();
         }
     } else if (warp >= 4 && warp < 4 + MF_UNPACK_WARPS) {
@@ -235,7 +264,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
         const uint32_t total = (uint32_t)my_units * (uint32_t)nk2;
         // every counter steps along (divisions by the stages of a unit were a third of a stage's instructions)
         int u = (int)blockIdx.x, it = team;
-        uint32_t s = (uint32_t)team, ph = 0, other_ph = 1; // this stage's slot and its parity; that of the other slot, four stages back
+        uint32_t s = (uint32_t)team, ph = 0, prev = 0, prev_ph = 0; // this stage's slot and its parity; those of the team's stage before
         const uint8_t *srow = nullptr;
         auto unit_scales = [&]() { // this thread's row of the scale bytes
             if (u >= n_units) return;
@@ -255,9 +284,11 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
 #pragma unroll
             for (int h = 0; h < 2; h++) sbv[h] = (srow != nullptr && kb0 + h < p.nkb) ? (uint32_t)__ldg(srow + kb0 + h) : 127u;
             // both polls first (they do not depend on each other), the bounded waits only where one failed
-            const uint32_t prev_empty = empty_bar((int)(s ^ MF_TEAMS)); // the team's stage before this one has been multiplied
+            // The team's stage before this one has been multiplied. (The barrier cannot be a phase further: its slot's next stage is
+            // multiplied after this one.)
+            const uint32_t prev_empty = empty_bar((int)prev);
             const bool tr = mbar_test(rawfull_bar((int)s), ph);
-            bool free_a = g < MF_TEAMS || mbar_test(prev_empty, other_ph);
+            bool free_a = g < MF_TEAMS || mbar_test(prev_empty, prev_ph);
             free_a = __all_sync(0xFFFFFFFFu, free_a);
             ok = __all_sync(0xFFFFFFFFu, tr) || mx_wait(rawfull_bar((int)s), ph, p.flag, 3);
             if (!ok) break;
@@ -318,7 +349,7 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
             if (ut == 0) MF_TRACE(5, g);
             __syncwarp();
             if (lane == 0) mf_arrive(rawempty_bar((int)s));
-            if (!free_a) ok = mx_wait(prev_empty, other_ph, p.flag, 7);
+            if (!free_a) ok = mx_wait(prev_empty, prev_ph, p.flag, 7);
             if (!ok) break;
             tc_fence_after();
             mf_tmem_st32(a_tmem, o);
@@ -326,10 +357,10 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
             __syncwarp();
             if (lane == 0) mf_arrive(full_bar((int)s));
             if (ut == 0) MF_TRACE(6, g);
-            // slots of a team: t, t + 4, t, ...; a slot's parity changes when the first of the two comes round again
-            s ^= MF_TEAMS;
-            if (s == (uint32_t)team) ph ^= 1u;
-            else other_ph ^= 1u;
+            prev = s;
+            prev_ph = ph;
+            s += MF_TEAMS;
+            if (s >= SLOTS) { s -= SLOTS; ph ^= 1u; }
             it += MF_TEAMS;
             if (it >= nk2) { // the next unit (stages are counted on: slots and teams keep alternating)
                 do { it -= nk2; u += (int)gridDim.x; } while (it >= nk2);
@@ -339,21 +370,23 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
     } else if (warp >= 4 + MF_UNPACK_WARPS) {
         // ---- epilogue: lane = out feature inside this warp's quarter of the accumulator rows ---------------
         const int quad = warp & 3;
-        uint32_t ul = 0;
+        int chunk = 0;
+        uint32_t fph = 0; // bit c: parity of the next accumulator that begins at chunk c
         __nv_bfloat16 *outp = reinterpret_cast<__nv_bfloat16 *>(p.out);
-        for (int u = blockIdx.x; u < n_units; u += gridDim.x, ul++) {
+        bool ok = true;
+        for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x) {
             const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
             const int4 en = __ldg(p.entries + tb);
-            const int mpad = (en.y + 15) & ~15;
-            const uint32_t buf = ul & 1u;
-            if (!mbar_wait(tfull_bar(buf), (ul >> 1) & 1u, p.flag, 4)) break;
+            ok = mbar_wait(tfull_bar(chunk), (fph >> chunk) & 1u, p.flag, 4);
+            if (!ok) break;
+            fph ^= 1u << chunk;
             tc_fence_after();
             const int feat = f * MF_ROWS + quad * 32 + lane;
             const bool fv = feat < p.n;
             const float bv = (p.bias && fv) ? load_as_f32(p.bias, p.bias_dtype, (size_t)en.z * p.n + feat) : 0.0f;
-            for (int c0 = 0; c0 < mpad; c0 += 32) {
+            for (int c0 = 0; c0 < en.y; c0 += 32) {
                 uint32_t rr[32];
-                tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + buf * MF_TMEM_BUF + (uint32_t)c0, rr);
+                tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(chunk * MF_CHUNK + (c0 & (MF_CHUNK - 1))), rr);
                 tmem_ld_wait();
                 if (p.epi == 0) {
 #pragma unroll
@@ -377,10 +410,13 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
                             outp[(size_t)(en.x + rowi) * p.ldo + (feat >> 1)] = __float2bfloat16_rn((up + 1.0f) * (gate * sig));
                     }
                 }
+                if ((c0 & 32) || c0 + 32 >= en.y) { // the chunk has been read
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mf_arrive(tempty_bar(chunk));
+                    if (++chunk == MF_CHUNKS) chunk = 0;
+                }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mf_arrive(tempty_bar(buf));
         }
     }
     tc_fence_before();
@@ -393,8 +429,16 @@ __global__ void __launch_bounds__(MF_THREADS, 1)
 
 static thread_local int g_moe_selftest_skip_loads = 0; // set only inside oxq_selftest_moe_wait_expiry
 
-// Rows of a token block (the plan kernel cuts every expert's rows into blocks of at most this many).
-int moe_fused_block_rows() { return MF_MAX_TOK; }
+// Rows of the largest token block, for `rows` rows an expert on average: the plan cuts an expert's rows into blocks of at most 192, but where
+// 256 are allowed and 1 to 64 would be left over it makes one block of more than 192 instead of two. That form has six slots instead
+// of eight, so it is for averages at which many experts are there, us with 192 / 256, 32 experts of 2880 x 2880 at 32, 128, 175, 200, 225, 244,
+// 256, 300, 375, 412, 437, 475, 512 rows: 197 / 212, 246 / 253, 299 / 298, 374 / 341, 415 / 373, 433 / 413, 448 / 444, 483 / 489, 579 / 568,
+// 681 / 628, 701 / 678, 726 / 736, 754 / 760; 16 of 2048 x 1024 at 225, 250: 104 / 97, 110 / 122.
+int moe_fused_block_rows(int rows)
+{
+    const int over = rows % 192;
+    return rows >= 176 && (over < 56 || over >= 176) ? 256 : 192;
+}
 
 // True when the fused grouped kernel serves these expert weights; otherwise the caller dequantizes expert groups.
 bool moe_fused_supported(int n, int k, const void *blocks, const void *scales, const void *a, const void *out, int ldo)
@@ -406,12 +450,12 @@ bool moe_fused_supported(int n, int k, const void *blocks, const void *scales, c
     return aligned(blocks, 16) && aligned(a, 16) && aligned(out, 2) && ldo > 0;
 }
 
-// out = epilogue(a . W_e^T + bias_e) for every token block of the table: a = expert-sorted activations [a_rows, k] bf16,
-// blocks / scales = the MXFP4 weights of all `experts` experts, n out features each. epi 0: bias; epi 1: clamped SwiGLU.
-int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
-                      const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi,
-                      float limit, int *flag, cudaStream_t st)
+template <int MAX_TOK>
+static int moe_fused_launch(const void *a, int a_rows, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
+                            const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi,
+                            float limit, int *flag, cudaStream_t st)
 {
+    auto kern = moe_mxfp4_fused_kernel<MAX_TOK>;
     MoeFusedParams p = {};
     p.entries = entries; p.n_blocks = n_blocks; p.scales = scales; p.bias = bias; p.out = out; p.flag = flag;
     p.n = n; p.k = k; p.nkb = k / 32;
@@ -421,7 +465,7 @@ int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const ui
     p.bias_dtype = bias_dtype; p.ldo = ldo; p.epi = epi; p.limit = limit;
     p.test_skip_loads = g_moe_selftest_skip_loads;
     if (const char *env = tuning_env("OXQ_MF_DBG")) p.dbg = atoi(env);
-    constexpr size_t smem = 1024 + MF_SLOTS * (MF_X_BYTES + MF_RAW_BYTES) + 8 * MF_NUM_BARS + 16;
+    constexpr size_t smem = 1024 + MF_SLOTS<MAX_TOK> * (MAX_TOK * MF_BK * 2 + MF_RAW_BYTES) + 8 * (4 * MF_SLOTS<MAX_TOK> + 2 * MF_CHUNKS) + 16;
     static_assert(smem <= (size_t)MF_SMEM_BUDGET, "the slots must fit one CTA's shared memory");
     CUtensorMap wmap, xmap;
     CUresult r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, blocks, (uint64_t)k / 2, (uint64_t)experts * n, (uint64_t)k / 2,
@@ -434,12 +478,22 @@ int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const ui
     int device = 0;
     OXQ_CUDA(cudaGetDevice(&device));
     if (device >= 64 || configured[device] < smem) {
-        OXQ_CUDA(cudaFuncSetAttribute(moe_mxfp4_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        OXQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (device < 64) configured[device] = smem;
     }
-    moe_mxfp4_fused_kernel<<<sm_count(), MF_THREADS, smem, st>>>(p, wmap, xmap);
+    kern<<<sm_count(), MF_THREADS, smem, st>>>(p, wmap, xmap);
     OXQ_LAUNCH_CHECK("moe_mxfp4_fused_kernel");
     return OXQ_OK;
+}
+
+// out = epilogue(a . W_e^T + bias_e) for every token block of the table: a = expert-sorted activations [a_rows, k] bf16,
+// blocks / scales = the MXFP4 weights of all `experts` experts, n out features each. epi 0: bias; epi 1: clamped SwiGLU.
+int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
+                      const int4 *entries, const int *n_blocks, int block_rows, const void *bias, int bias_dtype, void *out, int ldo,
+                      int epi, float limit, int *flag, cudaStream_t st)
+{
+    return block_rows <= 192 ? moe_fused_launch<192>(a, a_rows, blocks, scales, experts, n, k, entries, n_blocks, bias, bias_dtype, out, ldo, epi, limit, flag, st)
+                             : moe_fused_launch<256>(a, a_rows, blocks, scales, experts, n, k, entries, n_blocks, bias, bias_dtype, out, ldo, epi, limit, flag, st);
 }
 
 } // namespace oxq
@@ -468,7 +522,7 @@ OXQ_EXPORT int oxq_selftest_moe_wait_expiry(void *workspace, size_t workspace_by
     OXQ_CUDA(cudaMemcpyAsync(n_blocks, &one, sizeof(one), cudaMemcpyHostToDevice, st));
     OXQ_CUDA(cudaStreamSynchronize(st)); // the two host words above live on this stack frame
     oxq::g_moe_selftest_skip_loads = 1;
-    const int rc = oxq::moe_fused_grouped(a, 384, blocks, scales, 1, n, k, entries, n_blocks, nullptr, 0, out, n, 0, 0.0f,
+    const int rc = oxq::moe_fused_grouped(a, 384, blocks, scales, 1, n, k, entries, n_blocks, 192, nullptr, 0, out, n, 0, 0.0f,
                                           reinterpret_cast<int *>(workspace), st);
     oxq::g_moe_selftest_skip_loads = 0;
     return rc;

@@ -211,10 +211,11 @@ def test_moe_small_batch_matches_64_bit_experts(cuda, hidden, inter, counts):
         assert (np.abs(got[rows] - ref) <= 2.0**-8 * (np.abs(h) @ np.abs(dn).T + np.abs(ref)) + 1e-6).all(), (e, c)
 
 
-# more than 44 rows an expert on average: blocks of up to 192 rows, weights unpacked into tensor memory by four teams in turn; fewer
-# stages of 64 columns than teams, a last stage half past k, more units than SMs
+# more than 44 rows an expert on average: weights unpacked into tensor memory by four teams in turn, accumulators round a ring of columns;
+# blocks of up to 192 rows (96, 160 and 300 rows an expert) and of up to 256, whole and beside smaller ones (201 and 218 rows); fewer
+# stages of 64 columns than teams, a last stage half past k, more units than SMs, so that blocks of all sizes follow one another in a CTA
 @pytest.mark.parametrize("hidden,inter", [(32, 96), (96, 32), (224, 544), (2880, 64), (128, 9600)])
-@pytest.mark.parametrize("counts", [(192, 193, 0, 1), (385, 64, 191, 0)])
+@pytest.mark.parametrize("counts", [(192, 193, 0, 1), (385, 64, 191, 0), (300, 260, 340, 300), (256, 225, 193, 130), (400, 209, 16, 250)])
 def test_moe_large_batch_matches_64_bit_experts(cuda, hidden, inter, counts):
     test_moe_small_batch_matches_64_bit_experts(cuda, hidden, inter, counts)
 

@@ -555,8 +555,11 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     // no dequantized slab, one launch per projection over all experts.
     const bool fused = moe_fused_supported(2 * inter, hidden, gu_blocks, gu_scales, xs, h, inter) &&
                        moe_fused_supported(hidden, inter, dn_blocks, dn_scales, h, xs, hidden);
+    // The experts that the pairs are spread over: with router logits all of them, whichever are local; rows that are given with
+    // their experts are all local.
+    const int spread = given_ids ? n_exp : num_experts;
     // Up to a few dozen rows per expert: the codes as tensor-core operands, nothing unpacked.
-    const bool mx = pairs <= MOE_MX_ROWS * n_exp && moe_mx_supported(2 * inter, hidden, gu_blocks, gu_scales) &&
+    const bool mx = pairs <= MOE_MX_ROWS * spread && moe_mx_supported(2 * inter, hidden, gu_blocks, gu_scales) &&
                     moe_mx_supported(hidden, inter, dn_blocks, dn_scales);
     if (L.decode && !((fused || mx) && pairs > MOE_DECODE_FUSED_FROM_PAIRS)) {
         OXQ_REQUIRE(aligned(gu_blocks, 16) && aligned(dn_blocks, 16), OXQ_ERR_BAD_ALIGN,
@@ -577,7 +580,7 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     }
     // the grouped kernel's table of token blocks goes where the m-tile table of the dense path would (same capacity bound);
     // grp_beg[0] then holds the number of blocks
-    const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows(pairs / n_exp);
+    const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows(pairs / spread);
     if ((fused || mx) && pairs <= MOE_SMALL_PAIRS) {
         OXQ_CUDA(launch_early(moe_dispatch_small_kernel, 1, 1024, st, top_idx, pairs, expert_lo, n_exp, block_rows, counts, offsets, entries,
                               grp_beg, perm, inv));

@@ -220,6 +220,21 @@ def test_moe_large_batch_matches_64_bit_experts(cuda, hidden, inter, counts):
     test_moe_small_batch_matches_64_bit_experts(cuda, hidden, inter, counts)
 
 
+@pytest.mark.parametrize("lo,hi", [(2, 4), (7, 8), (0, 5)])
+def test_moe_small_batch_of_a_part_of_the_experts(cuda, lo, hi):
+    """Rows per expert decide which kernel serves a call, not how many of the experts are local: with one expert a token, a rank with a part
+    of them gives the bits of the whole layer for its tokens, and zeros for the others."""
+    layer, _ = experts_layer(8, 256, 512, seed=9)
+    layer.top_k = 1
+    x = bf16(synth.activations(320, 256, seed=9))
+    ids = torch.from_numpy(np.random.default_rng(9).integers(0, 8, 320)).cuda()
+    logits = torch.nn.functional.one_hot(ids, 8).float()
+    whole, part = layer.forward_with_logits(x, logits), layer.forward_with_logits(x, logits, (lo, hi))
+    layer.check()
+    local = (ids >= lo) & (ids < hi)
+    assert torch.equal(part[local], whole[local]) and not part[~local].any()
+
+
 def test_moe_small_batch_kernel_survives_weights_that_never_come(cuda):
     ws = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
     _lib.call("oxq_selftest_moe_mx_wait_expiry", ws.data_ptr(), ws.numel(), None)

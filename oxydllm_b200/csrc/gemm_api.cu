@@ -37,7 +37,6 @@ bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, 
 int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
                      cudaStream_t st, int sym, void *scratch, size_t scratch_bytes);
-size_t fp8_mx_scratch_bytes(int m, int k, int n);
 bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
 int fp8_mx_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in, const void *bias,
                   int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st, void *scratch, size_t scratch_bytes);
@@ -394,7 +393,7 @@ OXQ_EXPORT size_t oxq_fp8_scratch_bytes(int m, int k, int n, int s_out, int s_in
     if (m <= 0 || k <= 0 || n <= 0 || s_out < 0 || s_in < 0 || (s_out && n % s_out) || (s_in && k % s_in)) return 0;
     int bo, bi;
     fp8_block(n, k, s_out, s_in, bo, bi);
-    return fp8_mx_supported(m, k, n, bo, bi, nullptr, nullptr, nullptr) ? fp8_mx_scratch_bytes(m, k, n) : 0;
+    return fp8_mx_supported(m, k, n, bo, bi, nullptr, nullptr, nullptr) ? packed_mx_scratch_bytes(m, k, n) : 0;
 }
 
 OXQ_EXPORT int oxq_fp8_matmul(const void *x, int x_dtype, const uint8_t *weight, const float *scale_inv, int s_out, int s_in,

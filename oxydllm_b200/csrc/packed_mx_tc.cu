@@ -1,24 +1,26 @@
 // GPTQ 4-bit and E4M3 matmul on the block-scaled 8-bit tensor cores: weights are operands in the bits that they have.
 //
-// Read as E4M3 a byte 0..15 is that integer times 2^-9 (subnormals and the first binade are evenly spaced), so unpacking 4-bit weights
-// is two masks and a shift per word of eight, and the operand takes half the shared memory of a bf16 one; E4M3 weights are not touched
-// at all. Activations are exact as two E4M3 pieces (mx_common.cuh); a small kernel in front writes them with their block scales and
-// the sums of x per quantization group. A group's product leaves tensor memory once and meets the group's scale and zero point in f32:
-//   y[t, n] = sum over groups of s[g, n] * (sum over the group's k of q[k, n] x[t, k] - z[g, n] * sum over the group's k of x[t, k]).
-// Nothing is rounded between the packed weight and the f32 total.
+// Read as E4M3 a byte 0..16 is that integer times 2^-9 (subnormals and the first binade are evenly spaced), with a sign bit its negative,
+// so q - z of 4-bit weights is one byte, looked up in a table of 16 that each out feature has per group; the operand takes half the
+// shared memory of a bf16 one. E4M3 weights are not touched at all. Activations are two E4M3 pieces (mx_common.cuh); a small kernel in
+// front writes them with their block scales. A group's product leaves tensor memory once and meets the group's scale in f32:
+//   y[t, n] = sum over groups of s[g, n] * (sum over the group's k of (q[k, n] - z[g, n]) x[t, k]).
+// Nothing is rounded between the packed weight and the f32 total. (With codes 0..15 as operands and z times the sum of x taken off
+// afterwards a weight of zero beside a large x left the rounding of two large f32 numbers behind.)
 //
 // One CTA per SM walks an equal share of all (tile, unit) pairs (a tile is 128 out features x at most 128 tokens, a unit 128 input
 // rows), so every SM works for the whole launch whatever the number of tiles; the pipeline runs on across tile borders. Roles:
-//   warp 0        TMA: units of weights (8 KB of packed words, or 16 KB of E4M3), as far ahead as the ring allows: this is what is in
+//   warp 0        TMA: units of weights (8 KB of packed words with their zero points, or 16 KB of E4M3), as far ahead as the ring allows: this is what is in
 //                 flight from HBM;
 //   warps 1, 3    tcgen05.mma kind::mxf8f6f4 on alternate units, weights [128 x 32] times both pieces of x, and the copies of x's
 //                 block scales to tensor memory;
 //   warp 2        TMA: the unit's pieces of x ([tokens, 128] bytes each, 128-byte swizzle) with their block scales;
-//   warp 4        4-bit weights: what a fold needs, scales and zero points of the tile's features, the tokens' sums of x (a warp of its
-//                 own: with these three copies warp 2 took 800 clocks a unit);
-//   8 warps       4-bit weights: unpack, two teams of four warps that take the units in turn: two packed words become one 16-byte chunk
-//                 of the operand tile (16 input rows of one out feature, K-major);
-//   8 or 16 warps fold: accumulators -> registers, scale and zero point, into the totals; at the end of a tile -> y, or, where the
+//   warp 4        4-bit weights: the scales of the tile's features, a unit at a time (a warp of its own: with more copies warp 2 took
+//                 800 clocks a unit);
+//   12 warps      4-bit weights: unpack, three teams of four warps that take the units in turn: two packed words become one 16-byte
+//                 chunk of the operand tile (16 input rows of one out feature, K-major); 4096 x 14336 at 6 tokens takes 18.3 us with
+//                 two teams, 17.1 with three, 17.3 with four;
+//   4 to 16 warps fold: accumulators -> registers, times the scale, into the totals; at the end of a tile -> y, or, where the
 //                 tile is shared with other CTAs, -> scratch, and the CTA that arrives last adds the parts in ascending k
 //                 (no CTA waits for another, the result does not depend on the order of arrival).
 // The pieces of up to 32 tokens are columns of one MMA (the fold adds them); above, two MMAs add into the same column.
@@ -37,21 +39,22 @@ __device__ long long g_px_trace[16][128]; // clock stamps of CTA 3, per role and
 
 constexpr int PX_ROWS = 128;                 // out features of a tile
 constexpr int PX_UNIT = 128;                 // input rows of a unit: what is loaded, unpacked and multiplied at a time
-constexpr int PX_TEAMS = 2, PX_TEAM_WARPS = 4, PX_UNPACK_WARPS = PX_TEAMS * PX_TEAM_WARPS;
+constexpr int PX_TEAMS = 3, PX_TEAM_WARPS = 4, PX_UNPACK_WARPS = PX_TEAMS * PX_TEAM_WARPS;
 constexpr int PX_ISSUERS = 2;                // warps that issue MMAs, on alternate units
 constexpr int PX_GPTQ = 0, PX_FP8 = 1;       // an AWQ word is eight out features of one row: MN-major, it was no faster than csrc/group_tc.cu
 constexpr int PX_UNPACK_WARP0 = 8;           // 4-bit weights; warps 5 to 7 are idle
 template <int WT> constexpr int PX_FOLD_WARP0 = WT == PX_FP8 ? 4 : PX_UNPACK_WARP0 + PX_UNPACK_WARPS; // a multiple of four: warp % 4 selects the quarter of the accumulator rows
-constexpr int PX_RAW_BYTES = PX_ROWS * PX_UNIT / 2, PX_A_BYTES = PX_ROWS * PX_UNIT;
+constexpr int PX_BOX_BYTES = PX_ROWS * PX_UNIT / 2, PX_A_BYTES = PX_ROWS * PX_UNIT;
+constexpr int PX_Z_BYTES = PX_ROWS / 2, PX_RAW_BYTES = PX_BOX_BYTES + 128; // ring slot: packed words, zero points of 128 features, pad
 constexpr int PX_SF_BYTES = 512;             // block scales of 128 rows of x and 128 k
 constexpr int PX_MAX_SLOTS = 8, PX_MAX_X = 4, PX_MAX_RAW = 24, PX_ACC = 4, PX_FR = 8;
-constexpr int PX_SC_BYTES = 256, PX_Z_BYTES = 64; // a fold's scales and zero points of 128 features
+constexpr int PX_SC_BYTES = 256;             // a fold's scales of 128 features
 constexpr int PX_NUM_BARS = 2 * (PX_MAX_RAW + PX_MAX_SLOTS + PX_MAX_X + PX_ACC + PX_FR);
 constexpr int PX_MAX_TOKENS = 128, PX_MERGED_TOKENS = 32; // per tile; both pieces as columns of one MMA up to here
 constexpr int PX_SF_COLS = 64;               // tensor-memory columns in front of the accumulators: the scales
 constexpr int PX_SMEM_BUDGET = 227 * 1024;
 constexpr int PX_CODE = 40;                  // wait codes 41 .. 51: oxq_gemm_check names them
-static_assert(PX_TEAMS % PX_ISSUERS == 0 && PX_MAX_SLOTS % PX_TEAMS == 0 && PX_MAX_RAW % PX_TEAMS == 0 && PX_MAX_X % PX_ISSUERS == 0,
+static_assert(2 * PX_TEAMS % PX_ISSUERS == 0 && 2 * PX_TEAMS <= PX_MAX_SLOTS && PX_MAX_RAW % PX_TEAMS == 0 && PX_MAX_X % PX_ISSUERS == 0,
               "a slot always meets the same team and issuer: a parity wait tells a phase from the next one only");
 static_assert(8 + 8 * PX_MAX_X <= PX_SF_COLS, "scales of A, then of every x slot");
 
@@ -59,7 +62,6 @@ struct PackedMxParams {
     const uint32_t *qzeros;
     const void *scales, *bias;
     const unsigned char *sf;        // [unit][token block][1 or 2][512] block scales of x's pieces
-    const float *sx;                // GPTQ: [unit][token blocks * mpad] sums of x
     void *y;
     int scales_f16, bias_dtype, y_dtype;
     int m, n, packed_out;
@@ -92,32 +94,45 @@ __device__ __forceinline__ uint32_t px_lds32(uint32_t addr)
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ float4 px_lds128f(uint32_t addr)
+// The E4M3 bytes of q - z for q = 0..15. Byte by byte 0x80 + q - z; a negative one is complemented, which makes it 0x80 + |q - z|, a
+// positive one loses its top bit.
+__device__ __forceinline__ void px_table(uint32_t (&t)[4], uint32_t z)
 {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint32_t v = 0x83828180u + 0x04040404u * j - z * 0x01010101u, neg = (~v >> 7) & 0x01010101u, mask = neg * 0xFFu;
+        t[j] = ((v ^ mask) + neg) ^ (~mask & 0x80808080u);
+    }
 }
-// Two packed words -> sixteen bytes: of each word nibbles 0, 2, 4, 6, then 1, 3, 5, 7.
-__device__ __forceinline__ void px_unpack(uint32_t dst, uint32_t w0, uint32_t w1)
+__device__ __forceinline__ uint32_t px_prmt(uint32_t a, uint32_t b, uint32_t sel) // a selector's top bit copies the byte's sign over it
 {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0 & 0x0F0F0F0Fu), "r"((w0 >> 4) & 0x0F0F0F0Fu),
-                 "r"(w1 & 0x0F0F0F0Fu), "r"((w1 >> 4) & 0x0F0F0F0Fu)
-                 : "memory");
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+// Eight codes -> their bytes of the table: both halves of it by the low three bits, then one of the two by the fourth.
+__device__ __forceinline__ uint2 px_lookup(const uint32_t (&t)[4], uint32_t w)
+{
+    const uint32_t sel = w & 0x77777777u, up = w << 4, m0 = px_prmt(up, w, 0xD9C8u), m1 = px_prmt(up, w, 0xFBEAu);
+    const uint32_t l0 = px_prmt(t[0], t[1], sel), h0 = px_prmt(t[2], t[3], sel);
+    const uint32_t l1 = px_prmt(t[0], t[1], sel >> 16), h1 = px_prmt(t[2], t[3], sel >> 16);
+    return make_uint2((l0 & ~m0) | (h0 & m0), (l1 & ~m1) | (h1 & m1));
+}
+__device__ __forceinline__ void px_unpack(uint32_t dst, const uint32_t (&t)[4], uint32_t w0, uint32_t w1)
+{
+    const uint2 a = px_lookup(t, w0), b = px_lookup(t, w1);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(a.x), "r"(a.y), "r"(b.x), "r"(b.y) : "memory");
 }
 
 // Units [begin, end) of CTA `i`, and the CTA that holds unit u.
 __host__ __device__ __forceinline__ long long px_share(long long total, int ctas, long long i) { return total * i / ctas; }
 __host__ __device__ __forceinline__ int px_owner(long long total, int ctas, long long u) { return (int)(((u + 1) * ctas - 1) / total); }
 
-// ---- x -> two E4M3 pieces, block scales, sums ---------------------------------------------------------------------------------
+// ---- x -> two E4M3 pieces, block scales ---------------------------------------------------------------------------------------
 // Sixteen lanes hold the 128 k of a unit of one token. xq: [token block][piece][mpad tokens][k]; sf: a piece's rows of a tile in the
-// order tmem_cp_scales wants (merged: both pieces' rows in one 512-byte chunk). GPTQ: within eight k the even ones come first, as
-// the unpack leaves them, and sx takes the sum of each unit; E4M3 weights need no sums, the scratch has no room for any.
-template <bool GPTQ>
+// order tmem_cp_scales wants (merged: both pieces' rows in one 512-byte chunk).
 __global__ void __launch_bounds__(256)
-    packed_mx_split_kernel(const __nv_bfloat16 *x, unsigned char *xq, unsigned char *sf, float *sx, int m, int k, int mpad, int token_blocks,
-                           int merged)
+    packed_mx_split_kernel(const __nv_bfloat16 *x, unsigned char *xq, unsigned char *sf, int m, int k, int mpad, int token_blocks, int merged)
 {
     // Behind the wait everything ahead of this kernel is complete, so what starts early after the trigger may read the weights at once.
     pdl_wait();
@@ -127,26 +142,18 @@ __global__ void __launch_bounds__(256)
     const int tok = real ? item / units : 0, u = real ? item - tok * units : 0;
     const uint4 raw = ld_produced(reinterpret_cast<const uint4 *>(x + (size_t)tok * k + (size_t)u * PX_UNIT) + lane);
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    float v[8], sum = 0.0f;
+    float v[8];
     uint32_t amax = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         v[2 * i] = bf16_lo_f32(w[i]);
         v[2 * i + 1] = bf16_hi_f32(w[i]);
         amax = max(amax, max(w[i] << 16 & 0x7FFF0000u, w[i] & 0x7FFF0000u));
-        if (GPTQ) sum += v[2 * i] + v[2 * i + 1];
     }
 #pragma unroll
     for (int o = 1; o <= 2; o <<= 1) amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o)); // four lanes hold a block of 32
-    if (GPTQ)
-#pragma unroll
-        for (int o = 1; o <= 8; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     uint2 hi, lo;
     const uint32_t s = mx_split8(v, amax, hi, lo);
-    if (GPTQ) {
-        hi = make_uint2(__byte_perm(hi.x, hi.y, 0x6420), __byte_perm(hi.x, hi.y, 0x7531));
-        lo = make_uint2(__byte_perm(lo.x, lo.y, 0x6420), __byte_perm(lo.x, lo.y, 0x7531));
-    }
     if (!real) return;
     const int tb = tok / mpad, row = tok - tb * mpad;
     unsigned char *dst = xq + ((size_t)(tb * 2) * mpad + row) * k + (size_t)u * PX_UNIT + lane * 8;
@@ -158,7 +165,6 @@ __global__ void __launch_bounds__(256)
         c[(row & 31) * 16 + (row >> 5) * 4 + j] = (unsigned char)s;
         if (!merged) c += PX_SF_BYTES;
         c[(lrow & 31) * 16 + (lrow >> 5) * 4 + j] = (unsigned char)(s - 4u);
-        if (GPTQ && j == 0) sx[(size_t)u * (token_blocks * mpad) + tb * mpad + row] = sum;
     }
 }
 
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
     if (warp == 0) {
         // ---- weights: everything ahead of the split kernel had finished when this kernel started -----------------------------
         const bool leader = elect_one();
-        const int ring = FP8 ? S : R;
+        const int ring = FP8 ? S : R, zbytes = p.sym ? 0 : PX_Z_BYTES;
         int n0 = first_tile / p.token_blocks * PX_ROWS, tb = first_tile % p.token_blocks;
         int uk = first_unit, r = 0;
         uint32_t ph = 0;
@@ -261,8 +267,12 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                     mbar_arrive_expect_tx(full + 8 * r, PX_A_BYTES);
                     tma_load_2d(base + (uint32_t)(r * PX_A_BYTES), &wmap, full + 8 * r, uk * PX_UNIT, n0);
                 } else {
-                    mbar_arrive_expect_tx(rawfull + 8 * r, PX_RAW_BYTES);
-                    tma_load_2d(raw_base + (uint32_t)(r * PX_RAW_BYTES), &wmap, rawfull + 8 * r, n0, uk * (PX_UNIT / 8));
+                    const uint32_t dst = raw_base + (uint32_t)(r * PX_RAW_BYTES);
+                    mbar_arrive_expect_tx(rawfull + 8 * r, (uint32_t)(PX_BOX_BYTES + zbytes));
+                    tma_load_2d(dst, &wmap, rawfull + 8 * r, n0, uk * (PX_UNIT / 8));
+                    if (zbytes) // fetched by the unpack warps they would cost a DRAM round trip per unit: 16.7 -> 23 us
+                        bulk_copy_g2s(dst + PX_BOX_BYTES, p.qzeros + (size_t)(((long long)uk * PX_UNIT) >> p.gshift) * p.packed_out + n0 / 8,
+                                      PX_Z_BYTES, rawfull + 8 * r);
                 }
             }
             __syncwarp();
@@ -359,22 +369,18 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
         if (unit_folds == 1) issue(PxInt<1>{});
         else issue(PxInt<2>{});
     } else if (!FP8 && warp == 4) {
-        // ---- scales, zero points and sums of x, a unit at a time ---------------------------------------------------------
+        // ---- scales, a unit at a time: weights, as warp 0's ---------------------------------------------------------------
         const bool leader = elect_one();
-        const int ld = p.token_blocks * p.mpad, zbytes = p.sym ? 0 : PX_Z_BYTES;
         int n0 = first_tile / p.token_blocks * PX_ROWS, tb = first_tile % p.token_blocks, uk = first_unit, c = 0;
         uint32_t cph = 1;
         bool ok = true;
-        pdl_wait(); // the sums come from the kernel ahead
         for (int it = 0; it < nunits && ok; it++) {
             const size_t group = (size_t)(((long long)uk * PX_UNIT) >> p.gshift);
             ok = mx_wait(frempty + 8 * c, cph, p.flag, PX_CODE + 8);
             if (ok && leader && !p.test_skip_loads) {
-                const uint32_t dst = fr_base + (uint32_t)(c * p.fr_bytes), bar = frfull + 8 * c;
-                mbar_arrive_expect_tx(bar, (uint32_t)(PX_SC_BYTES + zbytes + 4 * p.mpad));
-                bulk_copy_g2s(dst, reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0, PX_SC_BYTES, bar);
-                if (zbytes) bulk_copy_g2s(dst + PX_SC_BYTES, p.qzeros + group * p.packed_out + n0 / 8, PX_Z_BYTES, bar);
-                bulk_copy_g2s(dst + PX_SC_BYTES + PX_Z_BYTES, p.sx + (size_t)uk * ld + tb * p.mpad, 4u * p.mpad, bar);
+                mbar_arrive_expect_tx(frfull + 8 * c, PX_SC_BYTES);
+                bulk_copy_g2s(fr_base + (uint32_t)(c * p.fr_bytes), reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0, PX_SC_BYTES,
+                              frfull + 8 * c);
             }
             __syncwarp();
             if (++c == PX_FR) { c = 0; cph ^= 1u; }
@@ -402,8 +408,11 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
             uint32_t w[16];
 #pragma unroll
             for (int i = 0; i < 16; i++) w[i] = px_lds32(src + i * 512u);
+            uint32_t z = 8, table[4];
+            if (!p.sym) z = ((px_lds32(raw_base + (uint32_t)(r * PX_RAW_BYTES) + PX_BOX_BYTES + 4u * (ut >> 3)) >> (4 * (ut & 7))) & 0xFu) + 1u; // stored zero + 1
+            px_table(table, z);
 #pragma unroll
-            for (int i = 0; i < 8; i++) px_unpack(dst + (((uint32_t)i ^ swz) << 4), w[2 * i], w[2 * i + 1]);
+            for (int i = 0; i < 8; i++) px_unpack(dst + (((uint32_t)i ^ swz) << 4), table, w[2 * i], w[2 * i + 1]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
             __syncwarp();
             if (lane == 0) {
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
 #pragma unroll 1
             for (int f = 0; f < folds && ok; f++) {
                 if (et == 0) PX_TRACE(6, tr);
-                float sc = s_next, nz = 0.0f;
+                float sc = s_next;
                 if (FP8 && srow && f + 1 < folds) s_next = __ldg(srow + (k_first + (f + 1) * p.fold_rows) / p.block_in);
                 if (FP8) ok = mx_wait(accfull + 8 * a, aph, p.flag, PX_CODE + 4);
                 else ok = mx_wait2(frfull + 8 * c, cph, accfull + 8 * a, aph, p.flag, PX_CODE + 4);
@@ -451,9 +460,7 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                     uint16_t sraw;
                     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sraw) : "r"(fr + 2u * feature) : "memory");
                     sc = p.scales_f16 ? __half2float(__ushort_as_half(sraw)) : __uint_as_float((uint32_t)sraw << 16);
-                    nz = -(float)(p.sym ? 8 : (int)((px_lds32(fr + PX_SC_BYTES + 4u * (feature >> 3)) >> (4 * (feature & 7))) & 0xFu) + 1); // stored zero + 1
                 }
-                const uint32_t sx = fr + PX_SC_BYTES + PX_Z_BYTES + 4u * col0;
                 tc_fence_after();
                 const uint32_t tacc = tlane + (uint32_t)(a * p.acc_cols);
                 constexpr int B = NCH < 2 ? 1 : 2; // chunks in flight between tensor memory and the totals
@@ -470,17 +477,10 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
 #pragma unroll
                     for (int i = 0; i < B; i++)
                         if ((i0 + i) * 8 < mh) {
-                            float sxv[8];
-                            if constexpr (!FP8) {
-                                const float4 s0 = px_lds128f(sx + (uint32_t)(i0 + i) * 32u), s1 = px_lds128f(sx + (uint32_t)(i0 + i) * 32u + 16u);
-                                sxv[0] = s0.x; sxv[1] = s0.y; sxv[2] = s0.z; sxv[3] = s0.w;
-                                sxv[4] = s1.x; sxv[5] = s1.y; sxv[6] = s1.z; sxv[7] = s1.w;
-                            }
 #pragma unroll
                             for (int e = 0; e < 8; e++) { // two at a time (fma.rn.f32x2) was 3 to 9 % slower from 128 tokens on
                                 float v = __uint_as_float(rr[i][e]);
                                 if constexpr (MERGED) v += __uint_as_float(rl[i][e]);
-                                if constexpr (!FP8) v = fmaf(nz, sxv[e], v);
                                 tot[(i0 + i) * 8 + e] = fmaf(sc, v, tot[(i0 + i) * 8 + e]);
                             }
                         }
@@ -588,9 +588,9 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
 }
 
 // True when this kernel serves a GPTQ call and is the better one: its unpack is cheaper than that of csrc/group_tc.cu, but the kernel that
-// writes x's pieces costs a launch, so the layer has to be large, and the groups at least a unit. us here /
-// there at 16 tokens: 4096 x 14336 17.2 / 20.5, 14336 x 4096 20.5 / 22.2, 4096 x 6144 14.1 / 12.7, 2048 x 4096 10.8 / 10.3, groups of 64,
-// 4096 x 4096 15.9 / 13.1; at 32 tokens 4096 x 14336 20.7 / 21.7, 14336 x 4096 24.2 / 23.2.
+// writes x's pieces costs a launch, so the layer has to be large, and the groups at least a unit. us here / there at 6 tokens: 4096 x
+// 14336 17.1 / 20.4, 14336 x 4096 19.7 / 22.0, 6144 x 8192 17.0 / 18.7; at 16 17.9 / 20.5, 20.7 / 22.2; with two unpack teams and codes
+// 0..15 as operands 4096 x 6144 at 16 tokens took 14.1 / 12.7, 2048 x 4096 10.8 / 10.3, 4096 x 14336 at 32 20.7 / 21.7, 14336 x 4096 24.2 / 23.2.
 bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
                          const void *scales)
 {
@@ -609,12 +609,12 @@ bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const vo
            aligned(x, 16) && aligned(weight, 16) && aligned(scale_inv, 4);
 }
 
-// The scratch area: x's pieces, their block scales and (GPTQ) sums, then tickets and parts of shared tiles.
+// The scratch area: x's pieces and their block scales, then tickets and parts of shared tiles.
 struct PackedMxScratch {
     int token_blocks, mpad, merged, tiles;
-    size_t sf, sx, tickets, partials, part_bytes; // offsets of the pieces' successors; bytes of a part
+    size_t sf, tickets, partials, part_bytes; // offsets of the pieces' successors; bytes of a part
 };
-static PackedMxScratch packed_mx_layout(int wt, int m, int k, int n)
+static PackedMxScratch packed_mx_layout(int m, int k, int n)
 {
     PackedMxScratch s;
     s.token_blocks = ceil_div(m, PX_MAX_TOKENS);
@@ -624,21 +624,18 @@ static PackedMxScratch packed_mx_layout(int wt, int m, int k, int n)
     const size_t rows = (size_t)s.token_blocks * s.mpad, units = (size_t)k / PX_UNIT;
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
     s.sf = up(2 * rows * k);
-    s.sx = s.sf + up(units * s.token_blocks * (s.merged ? 1 : 2) * PX_SF_BYTES);
-    s.tickets = s.sx + (wt == PX_GPTQ ? up(units * rows * sizeof(float)) : 0);
+    s.tickets = s.sf + up(units * s.token_blocks * (s.merged ? 1 : 2) * PX_SF_BYTES);
     s.partials = s.tickets + up((size_t)s.tiles * sizeof(unsigned long long));
     s.part_bytes = (size_t)s.mpad * PX_ROWS * sizeof(float);
     return s;
 }
 
 // Scratch that lets a call of this size share tiles over all SMs (with less it shares fewer, below the pieces it is not served).
-static size_t packed_mx_full_bytes(int wt, int m, int k, int n)
+size_t packed_mx_scratch_bytes(int m, int k, int n)
 {
-    const PackedMxScratch s = packed_mx_layout(wt, m, k, n);
+    const PackedMxScratch s = packed_mx_layout(m, k, n);
     return s.partials + (size_t)(sm_count() + s.tiles) * s.part_bytes;
 }
-size_t packed_mx_scratch_bytes(int m, int k, int n) { return packed_mx_full_bytes(PX_GPTQ, m, k, n); }
-size_t fp8_mx_scratch_bytes(int m, int k, int n) { return packed_mx_full_bytes(PX_FP8, m, k, n); }
 
 template <int WT, int NCH, int PARTS>
 static int packed_mx_launch(const PackedMxParams &p, const CUtensorMap &wmap, const CUtensorMap &xmap, int ctas, size_t smem, cudaStream_t st)
@@ -673,10 +670,10 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
     const int m = p.m, n = p.n;
     p.token_blocks = s.token_blocks; p.mpad = s.mpad; p.merged = s.merged; p.tiles = s.tiles;
     p.units_per_tile = k / PX_UNIT;
-    p.sf = sb + s.sf; p.sx = reinterpret_cast<const float *>(sb + s.sx);
+    p.sf = sb + s.sf;
     p.x_bytes = 2 * p.mpad * PX_UNIT;
     p.sf_bytes = (p.merged ? 1 : 2) * PX_SF_BYTES;
-    p.fr_bytes = wt == PX_FP8 ? 0 : PX_SC_BYTES + PX_Z_BYTES + 4 * p.mpad;
+    p.fr_bytes = wt == PX_FP8 ? 0 : PX_SC_BYTES;
     const int fixed = 1024 + PX_FR * p.fr_bytes + 8 * PX_NUM_BARS + 16;
     p.x_slots = PX_MAX_X;
     const int room = PX_SMEM_BUDGET - fixed - p.x_slots * (p.x_bytes + p.sf_bytes);
@@ -684,7 +681,7 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
         p.slots = room / PX_A_BYTES < PX_MAX_SLOTS ? room / PX_A_BYTES : PX_MAX_SLOTS;
         p.slots -= p.slots % PX_ISSUERS;
     } else {
-        p.slots = p.mpad <= 96 ? 2 * PX_TEAMS : PX_TEAMS;
+        p.slots = 2 * PX_TEAMS;
         p.raw_slots = (room - p.slots * PX_A_BYTES) / PX_RAW_BYTES;
         if (p.raw_slots > PX_MAX_RAW) p.raw_slots = PX_MAX_RAW;
         p.raw_slots -= p.raw_slots % PX_TEAMS;
@@ -747,8 +744,7 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, wt == PX_GPTQ ? packed_mx_split_kernel<true> : packed_mx_split_kernel<false>, (const __nv_bfloat16 *)x, sb,
-                                sb + s.sf, reinterpret_cast<float *>(sb + s.sx), m, k, p.mpad, p.token_blocks, p.merged));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, packed_mx_split_kernel, (const __nv_bfloat16 *)x, sb, sb + s.sf, m, k, p.mpad, p.token_blocks, p.merged));
 #define OXQ_PX_LAUNCH(WT, NCH, PARTS) return packed_mx_launch<WT, NCH, PARTS>(p, wmap, xmap, (int)ctas, smem, st)
     if (wt == PX_FP8) {
         if (p.mpad <= 16) OXQ_PX_LAUNCH(PX_FP8, 1, 2);
@@ -756,7 +752,7 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
         if (p.mpad <= 64) OXQ_PX_LAUNCH(PX_FP8, 2, 4);
         OXQ_PX_LAUNCH(PX_FP8, 4, 4);
     }
-    OXQ_PX_LAUNCH(PX_GPTQ, 1, 2);
+    OXQ_PX_LAUNCH(PX_GPTQ, 2, 1);
 #undef OXQ_PX_LAUNCH
 }
 
@@ -764,7 +760,7 @@ int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag,
                      cudaStream_t st, int sym, void *scratch, size_t scratch_bytes)
 {
-    const PackedMxScratch s = packed_mx_layout(PX_GPTQ, m, k, n);
+    const PackedMxScratch s = packed_mx_layout(m, k, n);
     if (scratch == nullptr || scratch_bytes < s.tickets) return OXQ_ERR_UNSUPPORTED;
     PackedMxParams p = {};
     p.qzeros = qzeros; p.scales = scales; p.bias = bias; p.y = y;
@@ -782,7 +778,7 @@ int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
 int fp8_mx_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in, const void *bias,
                   int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st, void *scratch, size_t scratch_bytes)
 {
-    const PackedMxScratch s = packed_mx_layout(PX_FP8, m, k, n);
+    const PackedMxScratch s = packed_mx_layout(m, k, n);
     if (scratch == nullptr || scratch_bytes < s.tickets) return OXQ_ERR_UNSUPPORTED;
     PackedMxParams p = {};
     p.bias = bias; p.y = y; p.bias_dtype = bias_dtype; p.y_dtype = y_dtype;

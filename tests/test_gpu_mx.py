@@ -177,6 +177,31 @@ def test_gptq_few_tokens_match_64_bit_sums(cuda, m, k, n, g, sym):
     gemm.check(gemm.workspace(n, k, "cuda"))
 
 
+@pytest.mark.parametrize("sym", [False, True])
+def test_gptq_zero_weights_beside_large_activations(cuda, sym):
+    """Products with q = z are exact zeros: eight x of 8000 in every group of 128 leave nothing in the sums of the others (1 to 2 in
+    magnitude, so that both pieces are exact), whose f32 roundings stay below 2^-19 of the sum of |x w|."""
+    k, n, g, m = 1152, 36864, 128, 16
+    rng = np.random.default_rng(k)
+    x = (rng.uniform(1, 2, (m, k)) * rng.choice([-1, 1], (m, k))).astype(np.float32)
+    nib = rng.integers(0, 16, (k, n), dtype=np.uint32)
+    zero = np.full((k // g, n), 8, np.uint32) if sym else rng.integers(1, 16, (k // g, n), dtype=np.uint32)
+    x[:, ::16] = 8000.0
+    nib[::16] = np.repeat(zero, g // 16, 0)
+    qw = (nib.reshape(k // 8, 8, n) << (4 * np.arange(8, dtype=np.uint32))[None, :, None]).sum(1, dtype=np.uint32)
+    qz = ((zero - 1).reshape(k // g, n // 8, 8) << (4 * np.arange(8, dtype=np.uint32))).sum(2, dtype=np.uint32)
+    sc = (np.abs(rng.standard_normal((k // g, n)) * 0.02) / 7 + 1e-4).astype(np.float16)
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (qw, qz, sc)]
+    lin = L.PackedQuantLinear(L.QuantWeight.new_gptq(4, sym, dev[0], None if sym else dev[1], dev[2]))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    xd = bf16(x)
+    gemm.packed4_matmul(lin, xd, y)
+    codes = torch.from_numpy(nib.astype(np.int32)).cuda() - torch.from_numpy(np.repeat(zero, g, 0).astype(np.int32)).cuda()
+    w = codes.double() * dev[2].double().repeat_interleave(g, 0)
+    xd = xd.double()
+    assert ((y.double() - xd @ w).abs() <= 2.0**-19 * (xd.abs() @ w.abs())).all()
+
+
 # ------------------------------------------------------------------------------------------------------- MXFP4 experts, small batches
 def experts_layer(experts, hidden, inter, seed):
     from oxydllm_b200 import moe

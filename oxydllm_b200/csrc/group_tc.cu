@@ -30,8 +30,6 @@
 // 11.4 / 16.6 / 19.4 (14 / 19 / 22), 4096 x 28672 30.5 / 48 / 54 (55 / 59 / 61), 14336 x 4096 21 / 28 / 32 (28 / 34 / 38). A poll costs
 // about 120 clocks even where the phase is complete, so the polls of a stage are under way together (one after the other: 11.8 / 17.0 /
 // 19.7, 32.1 / 51 / 56, 21.8 / 30 / 34).
-#include <atomic>
-
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -649,8 +647,7 @@ int group_tc_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzer
         if (cost < best) { best = cost; ctas = cand; p.split = 1; }
         if (cand == sm_count()) break;
     }
-    static std::atomic<unsigned long long> calls{0}; // marks differ between calls, in no order that a stale value would have by chance
-    p.mark = ((calls.fetch_add(1, std::memory_order_relaxed) + 1) * 0x9E3779B97F4A7C15ull) >> 8;
+    p.mark = mx_call_mark();
     p.tickets = reinterpret_cast<unsigned long long *>(scratch);
     p.partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + ticket_bytes);
 

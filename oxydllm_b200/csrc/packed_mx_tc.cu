@@ -24,8 +24,6 @@
 //                 tile is shared with other CTAs, -> scratch, and the CTA that arrives last adds the parts in ascending k
 //                 (no CTA waits for another, the result does not depend on the order of arrival).
 // The pieces of up to 32 tokens are columns of one MMA (the fold adds them); above, two MMAs add into the same column.
-#include <atomic>
-
 #include "mx_common.cuh"
 
 namespace oxq {
@@ -61,7 +59,9 @@ static_assert(8 + 8 * PX_MAX_X <= PX_SF_COLS, "scales of A, then of every x slot
 struct PackedMxParams {
     const uint32_t *qzeros;
     const void *scales, *bias;
-    const unsigned char *sf;        // [unit][token block][1 or 2][512] block scales of x's pieces
+    const unsigned char *sf;        // [pair][unit][token block][1 or 2][512] block scales of x's pieces
+    const unsigned long long *second; // [unit][token block], a byte per group of 16 tokens, MX_...: whether they have a second pair of pieces there
+    const unsigned long long *any;  // this call's mark where some have
     void *y;
     int scales_f16, bias_dtype, y_dtype;
     int m, n, packed_out;
@@ -76,6 +76,7 @@ struct PackedMxParams {
     int gshift;                     // log2(group size)
     int fold_rows;                  // input rows per accumulator buffer: 128, or 64 where E4M3 weights have scale blocks of an odd number of 64s
     int units_per_tile, tiles;
+    size_t pair_sf;                 // bytes of a pair's block scales
     const float *scale_inv;         // E4M3: one scale per block_out x block_in weights, s_in blocks a row; null: 1
     int s_in, block_out, block_in;
     int sym;                        // GPTQ without stored zero points (zero 8)
@@ -128,44 +129,118 @@ __device__ __forceinline__ void px_unpack(uint32_t dst, const uint32_t (&t)[4], 
 __host__ __device__ __forceinline__ long long px_share(long long total, int ctas, long long i) { return total * i / ctas; }
 __host__ __device__ __forceinline__ int px_owner(long long total, int ctas, long long u) { return (int)(((u + 1) * ctas - 1) / total); }
 
-// ---- x -> two E4M3 pieces, block scales ---------------------------------------------------------------------------------------
-// Sixteen lanes hold the 128 k of a unit of one token. xq: [token block][piece][mpad tokens][k]; sf: a piece's rows of a tile in the
-// order tmem_cp_scales wants (merged: both pieces' rows in one 512-byte chunk).
-__global__ void __launch_bounds__(256)
-    packed_mx_split_kernel(const __nv_bfloat16 *x, unsigned char *xq, unsigned char *sf, int m, int k, int mpad, int token_blocks, int merged)
+// Whether any unit of x has a second pair of pieces: a word to load (behind pdl_wait()), and later, when it has come, to look at. The
+// vote makes the answer known to be the same in all lanes.
+__device__ __forceinline__ unsigned long long px_any_word(const PackedMxParams &p) { return *reinterpret_cast<const volatile unsigned long long *>(p.any); }
+__device__ __forceinline__ bool px_any_second(const PackedMxParams &p, unsigned long long word) { return __all_sync(0xFFFFFFFFu, word == p.mark); }
+constexpr int PX_GROUP = 16; // tokens that ask for second pairs together
+constexpr unsigned long long PX_BYTES = 0x0101010101010101ull;
+// The groups' bytes of a unit's second pairs, and those of them that are of a kind.
+__device__ __forceinline__ unsigned long long px_second(const PackedMxParams &p, int tb, int u)
+{
+    return ld_produced(p.second + (size_t)u * p.token_blocks + tb) & (~0ull >> (64 - p.mpad / PX_GROUP * 8));
+}
+// Units of [from, to) some of whose tokens have a second pair, in order, E4M3 before E5M2: body(unit, MX_...), until it returns false.
+template <typename Body> __device__ __forceinline__ bool px_second_units(const PackedMxParams &p, int tb, int from, int to, Body body)
+{
+    for (int u = from; u < to; u += 32) {
+        const int at = u + (int)(threadIdx.x & 31);
+        const unsigned long long k = at < to ? px_second(p, tb, at) : 0ull;
+        const unsigned e4m3 = __ballot_sync(0xFFFFFFFFu, (k & PX_BYTES * MX_SECOND_E4M3) != 0), e5m2 = __ballot_sync(0xFFFFFFFFu, (k & PX_BYTES * MX_SECOND_E5M2) != 0);
+        for (unsigned hit = e4m3 | e5m2; hit; hit &= hit - 1) {
+            const int i = __ffs(hit) - 1;
+            if ((e4m3 >> i & 1u) && !body(u + i, MX_SECOND_E4M3)) return false;
+            if ((e5m2 >> i & 1u) && !body(u + i, MX_SECOND_E5M2)) return false;
+        }
+    }
+    return true;
+}
+// What a CTA does, in order: its units of a tile, then those of them again some of whose tokens have a second pair of pieces (twice, if
+// of both kinds); the next tile.
+// All roles walk this list; one that is `first` of `step` that take turns does every step-th of it from the first-th on:
+// body(unit of the tile, pair, MX_..., token block, first feature), until it returns false. waited: behind pdl_wait() already. (The usual loop is a plain count, so that
+// what it computes stays in uniform registers: with one loop over both pairs a call took 10 to 20 % longer.)
+template <typename Body>
+__device__ __forceinline__ bool px_walk(const PackedMxParams &p, int tile, int from, int left, int first, int step, bool waited, Body body)
+{
+    int tb = tile % p.token_blocks, n0 = tile / p.token_blocks * PX_ROWS, skip = first;
+    bool ok = true, looked = false, any = false;
+    unsigned long long word = 0;
+    if (waited) word = px_any_word(p);
+    while (left > 0 && ok) {
+        const int to = min(p.units_per_tile, from + left);
+        int uk = from + skip;
+        for (; uk < to && ok; uk += step) ok = body(uk, 0, MX_ONE_PAIR, tb, n0);
+        skip = uk - to;
+        if (ok && !looked) {
+            if (!waited) {
+                pdl_wait();
+                word = px_any_word(p);
+            }
+            any = px_any_second(p, word);
+            looked = true;
+        }
+        if (ok && any)
+            ok = px_second_units(p, tb, from, to, [&](int u, int kind) {
+                if (skip > 0) {
+                    skip--;
+                    return true;
+                }
+                skip = step - 1;
+                return body(u, 1, kind, tb, n0);
+            });
+        left -= to - from;
+        from = 0;
+        if (++tb == p.token_blocks) { tb = 0; n0 += PX_ROWS; }
+    }
+    return ok;
+}
+
+// ---- x -> pieces, block scales ------------------------------------------------------------------------------------------------
+// A CTA takes a unit of a group of tokens, sixteen lanes the 128 k of a token. xq: [pair][token block][piece][mpad tokens][k]; sf: a piece's
+// rows of a tile in the order tmem_cp_scales wants (merged: both pieces' rows in one 512-byte chunk). The second pair is written for
+// all tokens of the group where one of them asks for it, and not at all elsewhere.
+__global__ void __launch_bounds__(16 * PX_GROUP)
+    packed_mx_split_kernel(const __nv_bfloat16 *x, unsigned char *xq, unsigned char *sf, unsigned char *second, unsigned long long *any,
+                           unsigned long long mark, int m, int k, int mpad, int token_blocks, int merged)
 {
     // Behind the wait everything ahead of this kernel is complete, so what starts early after the trigger may read the weights at once.
     pdl_wait();
     pdl_launch_dependents();
-    const int units = k / PX_UNIT, lane = threadIdx.x & 15;
-    const int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, real = item < m * units; // whole warps stay for the shuffles
-    const int tok = real ? item / units : 0, u = real ? item - tok * units : 0;
-    const uint4 raw = ld_produced(reinterpret_cast<const uint4 *>(x + (size_t)tok * k + (size_t)u * PX_UNIT) + lane);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    float v[8];
-    uint32_t amax = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        v[2 * i] = bf16_lo_f32(w[i]);
-        v[2 * i + 1] = bf16_hi_f32(w[i]);
-        amax = max(amax, max(w[i] << 16 & 0x7FFF0000u, w[i] & 0x7FFF0000u));
-    }
-#pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o)); // four lanes hold a block of 32
-    uint2 hi, lo;
-    const uint32_t s = mx_split8(v, amax, hi, lo);
-    if (!real) return;
-    const int tb = tok / mpad, row = tok - tb * mpad;
-    unsigned char *dst = xq + ((size_t)(tb * 2) * mpad + row) * k + (size_t)u * PX_UNIT + lane * 8;
-    *reinterpret_cast<uint2 *>(dst) = hi;
-    *reinterpret_cast<uint2 *>(dst + (size_t)mpad * k) = lo;
-    if ((lane & 3) == 0) {
+    const int u = blockIdx.x, units = gridDim.x, tb = blockIdx.y * PX_GROUP / mpad, lane = threadIdx.x & 15;
+    const int tok = blockIdx.y * PX_GROUP + (threadIdx.x >> 4), row = tok - tb * mpad;
+    const size_t sf_bytes = (merged ? 1 : 2) * PX_SF_BYTES;
+    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+    if (tok < m) raw = ld_produced(reinterpret_cast<const uint4 *>(x + (size_t)tok * k + (size_t)u * PX_UNIT) + lane);
+    auto store = [&](int pair, uint2 hi, uint2 lo) {
+        unsigned char *dst = xq + ((size_t)((pair * token_blocks + tb) * 2) * mpad + row) * k + (size_t)u * PX_UNIT + lane * 8;
+        *reinterpret_cast<uint2 *>(dst) = hi;
+        *reinterpret_cast<uint2 *>(dst + (size_t)mpad * k) = lo;
+    };
+    auto store_scale = [&](int pair, uint32_t s) {
         const int j = lane >> 2, lrow = merged ? row + mpad : row; // block of 32 within the unit; lo's row
-        unsigned char *c = sf + ((size_t)u * token_blocks + tb) * (merged ? PX_SF_BYTES : 2 * PX_SF_BYTES);
+        unsigned char *c = sf + ((size_t)(pair * units + u) * token_blocks + tb) * sf_bytes;
         c[(row & 31) * 16 + (row >> 5) * 4 + j] = (unsigned char)s;
         if (!merged) c += PX_SF_BYTES;
         c[(lrow & 31) * 16 + (lrow >> 5) * 4 + j] = (unsigned char)(s - 4u);
+    };
+    const MxBlock b = mx_block(raw);
+    float v[8];
+    uint2 hi, lo;
+    const uint32_t s = mx_first_pair(raw, b, v, hi, lo);
+    if (tok < m) store(0, hi, lo);
+    if (tok < m && (lane & 3) == 0) store_scale(0, s);
+    const int hit = __syncthreads_or(b.second != MX_ONE_PAIR), e5m2 = hit && __syncthreads_or(b.second == MX_SECOND_E5M2);
+    if (threadIdx.x == 0) {
+        second[((size_t)u * token_blocks + tb) * 8 + row / PX_GROUP] = (unsigned char)(!hit ? MX_ONE_PAIR : e5m2 ? MX_SECOND_E5M2 : MX_SECOND_E4M3);
+        if (hit) *any = mark;
     }
+    uint32_t s2 = 127; // where other groups of the tile have a second pair this one multiplies zeros, with a scale that is not NaN
+    if (hit) {
+        s2 = mx_second_pair(raw, v, s, e5m2, hi, lo);
+        if (tok < m) store(1, hi, lo);
+    }
+    if (tok < m && (lane & 3) == 0) store_scale(1, s2);
 }
 
 template <int V> struct PxInt { static constexpr int value = V; };
@@ -175,7 +250,8 @@ template <int V> struct PxInt { static constexpr int value = V; };
 template <int WT, int PARTS> constexpr int PX_THREADS = (PX_FOLD_WARP0<WT> + 4 * PARTS) * 32;
 template <int WT, int NCH, int PARTS>
 __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
-    packed_mx_tc_kernel(const PackedMxParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
+    packed_mx_tc_kernel(const PackedMxParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+                        const __grid_constant__ CUtensorMap gmap)
 {
     constexpr bool FP8 = WT == PX_FP8;
     constexpr int FOLD_WARP0 = PX_FOLD_WARP0<WT>, FOLD_WARPS = 4 * PARTS;
@@ -255,13 +331,10 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
         // ---- weights: everything ahead of the split kernel had finished when this kernel started -----------------------------
         const bool leader = elect_one();
         const int ring = FP8 ? S : R, zbytes = p.sym ? 0 : PX_Z_BYTES;
-        int n0 = first_tile / p.token_blocks * PX_ROWS, tb = first_tile % p.token_blocks;
-        int uk = first_unit, r = 0;
-        uint32_t ph = 0;
-        bool ok = true;
-        for (int it = 0; it < nunits && ok; it++) {
-            if (it >= ring) ok = mx_wait((FP8 ? empty : rawempty) + 8 * r, ph ^ 1u, p.flag, PX_CODE + 1);
-            PX_TRACE(0, it);
+        int r = 0, round = 0;
+        uint32_t ph = 1;
+        px_walk(p, first_tile, first_unit, nunits, 0, 1, false, [&](int uk, int, int, int, int n0) {
+            const bool ok = round == 0 || mx_wait((FP8 ? empty : rawempty) + 8 * r, ph, p.flag, PX_CODE + 1); // polls of fresh barriers cost 1 us a call
             if (ok && leader && !p.test_skip_loads) {
                 if (FP8) {
                     mbar_arrive_expect_tx(full + 8 * r, PX_A_BYTES);
@@ -276,44 +349,60 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                 }
             }
             __syncwarp();
-            if (++r == ring) { r = 0; ph ^= 1u; }
-            if (++uk == G) {
-                uk = 0;
-                if (++tb == p.token_blocks) { tb = 0; n0 += PX_ROWS; }
-            }
-        }
+            if (++r == ring) { r = 0; ph ^= 1u; round = 1; }
+            return ok;
+        });
     } else if (warp == 2) {
         // ---- x with its block scales, as soon as the MMAs that read the slot have completed ----------------------------------
         const bool leader = elect_one();
-        int tb = first_tile % p.token_blocks, uk = first_unit, x = 0;
+        int x = 0, done = 0;
         uint32_t xph = 1; // a fresh barrier passes parity 1
-        bool ok = true;
         pdl_wait(); // the pieces come from the kernel ahead
-        for (int it = 0; it < nunits && ok; it++) {
-            ok = mx_wait(xempty + 8 * x, xph, p.flag, PX_CODE + 5);
-            PX_TRACE(9, it);
-            if (ok && leader) {
+        bool ok = px_walk(p, first_tile, first_unit, nunits, 0, 1, true, [&](int uk, int pair, int kind, int tb, int) {
+            const bool ok = mx_wait(xempty + 8 * x, xph, p.flag, PX_CODE + 5);
+            if (pair && ok) { // group by group: zeros where there is no second pair of this kind
+                const unsigned long long k = px_second(p, tb, uk);
+                int groups = 0;
+                for (int g = 0; g < p.mpad / PX_GROUP; g++) {
+                    if ((int)(k >> (8 * g) & 0xFFu) == kind) groups++;
+                    else
+                        for (int i = lane; i < 2 * PX_GROUP * PX_UNIT / 16; i += 32) { // both pieces
+                            const uint32_t half = (uint32_t)(i / (PX_GROUP * PX_UNIT / 16) * p.x_bytes / 2), at = (uint32_t)(i % (PX_GROUP * PX_UNIT / 16) * 16);
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(x_base + (uint32_t)(x * p.x_bytes) + half + (uint32_t)(g * PX_GROUP * PX_UNIT) + at), "r"(0u) : "memory");
+                        }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
+                __syncwarp();
+                if (leader) {
+                    mbar_arrive_expect_tx(xfull + 8 * x, (uint32_t)(groups * 2 * PX_GROUP * PX_UNIT + p.sf_bytes));
+                    for (int g = 0; g < p.mpad / PX_GROUP; g++)
+                        if ((int)(k >> (8 * g) & 0xFFu) == kind)
+                            for (int piece = 0; piece < 2; piece++)
+                                tma_load_2d(x_base + (uint32_t)(x * p.x_bytes + piece * p.x_bytes / 2 + g * PX_GROUP * PX_UNIT), &gmap, xfull + 8 * x,
+                                            uk * PX_UNIT, ((p.token_blocks + tb) * 2 + piece) * p.mpad + g * PX_GROUP);
+                    bulk_copy_g2s(sf_base + (uint32_t)(x * p.sf_bytes), p.sf + p.pair_sf + ((size_t)uk * p.token_blocks + tb) * p.sf_bytes,
+                                  (uint32_t)p.sf_bytes, xfull + 8 * x);
+                }
+            } else if (ok && leader) {
                 mbar_arrive_expect_tx(xfull + 8 * x, (uint32_t)(p.x_bytes + p.sf_bytes));
                 tma_load_2d(x_base + (uint32_t)(x * p.x_bytes), &xmap, xfull + 8 * x, uk * PX_UNIT, tb * 2 * p.mpad);
-                bulk_copy_g2s(sf_base + (uint32_t)(x * p.sf_bytes), p.sf + ((size_t)uk * p.token_blocks + tb) * p.sf_bytes, (uint32_t)p.sf_bytes,
-                              xfull + 8 * x);
+                bulk_copy_g2s(sf_base + (uint32_t)(x * p.sf_bytes), p.sf + ((size_t)uk * p.token_blocks + tb) * p.sf_bytes,
+                              (uint32_t)p.sf_bytes, xfull + 8 * x);
             }
             __syncwarp();
             if (++x == X) { x = 0; xph ^= 1u; }
-            if (++uk == G) {
-                uk = 0;
-                if (++tb == p.token_blocks) tb = 0;
-            }
-        }
+            done++;
+            return ok;
+        });
         // The commits of the last units arrive here asynchronously: the CTA stays until they have.
-        for (int left = min(S, nunits), q = nunits - left; left > 0 && ok; left--, q++)
+        for (int left = min(S, done), q = done - left; left > 0 && ok; left--, q++)
             ok = mx_wait(empty + 8 * (q % S), (uint32_t)(q / S) & 1u, p.flag, PX_CODE + 11);
-        for (int left = min(X, nunits), q = nunits - left; left > 0 && ok; left--, q++)
+        for (int left = min(X, done), q = done - left; left > 0 && ok; left--, q++)
             ok = mx_wait(xempty + 8 * (q % X), (uint32_t)(q / X) & 1u, p.flag, PX_CODE + 11);
     } else if (warp < 4) {
         // ---- MMA issue: warps 1 and 3 take the units in turn (one alone took 900 clocks a unit, most of it polls and commits) -------
         const bool leader = elect_one();
-        const uint32_t idesc = mx_idesc(MX_E4M3, MERGED ? 2 * p.mpad : p.mpad);
+        const uint32_t idesc0 = mx_idesc(MX_E4M3, MERGED ? 2 * p.mpad : p.mpad);
         const uint64_t adesc0 = kmajor_sw128_desc(base), bdesc0 = kmajor_sw128_desc(x_base);
         const uint32_t x16 = (uint32_t)p.x_bytes >> 4, lo16 = x16 / 2; // 16-byte units
         auto issue = [&](auto unit_folds_) {
@@ -321,13 +410,14 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
             const int step = p.issuers, me = warp >> 1;
             int s = me, a = me * UF, x = me;
             uint32_t ph = 0, xph = 0, aph = 1; // aph: parity of the last release of the buffer (a fresh barrier passes parity 1)
-            bool ok = true;
-            for (int it = me; me < step && it < nunits && ok; it += step) {
-                if (me == 0) PX_TRACE(11, it);
+            if (me >= step) return;
+            pdl_wait();
+            px_walk(p, first_tile, first_unit, nunits, me, step, true, [&](int, int, int kind, int, int) {
+                const uint32_t idesc = kind == MX_SECOND_E5M2 ? idesc0 ^ MX_IDESC_B_E5M2 : idesc0;
+                bool ok;
                 const uint64_t da = adesc0 + (uint64_t)(s * (PX_A_BYTES >> 4)), db = bdesc0 + (uint64_t)(x * x16);
                 const uint32_t sfb = tmem_base + 8u + 8u * x;
                 ok = mx_wait3(xfull + 8 * x, xph, full + 8 * s, ph, accempty + 8 * a, aph, p.flag, PX_CODE + 2);
-                PX_TRACE(4, it);
 #pragma unroll
                 for (int f = 0; f < UF; f++) {
                     if (ok && f > 0) ok = mx_wait(accempty + 8 * a, aph, p.flag, PX_CODE + 9);
@@ -356,7 +446,6 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                     }
                     if (++a == p.accs) { a = 0; aph ^= 1u; }
                 }
-                PX_TRACE(5, it);
                 // on to this warp's next unit
                 s += step;
                 if (s >= S) { s -= S; ph ^= 1u; }
@@ -364,19 +453,19 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                 if (x >= X) { x -= X; xph ^= 1u; }
                 a += (step - 1) * UF;
                 if (a >= p.accs) { a -= p.accs; aph ^= 1u; }
-            }
+                return ok;
+            });
         };
         if (unit_folds == 1) issue(PxInt<1>{});
         else issue(PxInt<2>{});
     } else if (!FP8 && warp == 4) {
         // ---- scales, a unit at a time: weights, as warp 0's ---------------------------------------------------------------
         const bool leader = elect_one();
-        int n0 = first_tile / p.token_blocks * PX_ROWS, tb = first_tile % p.token_blocks, uk = first_unit, c = 0;
+        int c = 0;
         uint32_t cph = 1;
-        bool ok = true;
-        for (int it = 0; it < nunits && ok; it++) {
+        px_walk(p, first_tile, first_unit, nunits, 0, 1, false, [&](int uk, int, int, int, int n0) {
             const size_t group = (size_t)(((long long)uk * PX_UNIT) >> p.gshift);
-            ok = mx_wait(frempty + 8 * c, cph, p.flag, PX_CODE + 8);
+            const bool ok = mx_wait(frempty + 8 * c, cph, p.flag, PX_CODE + 8);
             if (ok && leader && !p.test_skip_loads) {
                 mbar_arrive_expect_tx(frfull + 8 * c, PX_SC_BYTES);
                 bulk_copy_g2s(fr_base + (uint32_t)(c * p.fr_bytes), reinterpret_cast<const uint16_t *>(p.scales) + group * p.n + n0, PX_SC_BYTES,
@@ -384,42 +473,64 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
             }
             __syncwarp();
             if (++c == PX_FR) { c = 0; cph ^= 1u; }
-            if (++uk == G) {
-                uk = 0;
-                if (++tb == p.token_blocks) { tb = 0; n0 += PX_ROWS; }
-            }
-        }
+            return ok;
+        });
     } else if (!FP8 && warp >= PX_UNPACK_WARP0 && warp < FOLD_WARP0) {
         // ---- unpack ----------------------------------------------------------------------------------------------
         const int team = (warp - PX_UNPACK_WARP0) / PX_TEAM_WARPS;
         const int ut = threadIdx.x - (PX_UNPACK_WARP0 + team * PX_TEAM_WARPS) * 32; // 0 .. 127
         const uint32_t src0 = 4u * ut, swz = (uint32_t)ut & 7u, dst0 = ((uint32_t)ut >> 3) * 1024u + swz * 128u; // out feature ut
         int s = team, r = team;
-        uint32_t ph = 0, rph = 0;
-        bool ok = true;
-        for (int it = team; it < nunits; it += PX_TEAMS) {
-            const bool t0 = mbar_test(rawfull + 8 * r, rph);
-            const bool t1 = it < S || mbar_test(empty + 8 * s, ph ^ 1u);
+        uint32_t ph = 1, rph = 0; // a fresh barrier passes parity 1
+        // px_walk's list, of which only the length matters here: one copy of the loop's body instead of two
+        int next = team, end = 0, tile = first_tile, from = first_unit, left = nunits; // this team's next, all so far; what is left of the list
+        bool ok = true, any = false, again = false;
+        unsigned long long word = 0;
+        while (true) {
+            while (ok && next >= end && left > 0) { // a tile's units, or those that come a second time, join the list
+                const int to = min(G, from + left);
+                if (!again) end += to - from;
+                else {
+                    if (tile == first_tile) {
+                        if (next <= team + PX_TEAMS) { // not loaded yet
+                            pdl_wait();
+                            word = px_any_word(p);
+                        }
+                        any = px_any_second(p, word);
+                    }
+                    if (any) px_second_units(p, tile % p.token_blocks, from, to, [&](int, int) { end++; return true; });
+                    left -= to - from;
+                    from = 0;
+                    tile++;
+                }
+                again = !again;
+            }
+            if (!ok || next >= end) break;
+            if (next == team + PX_TEAMS) { // with a unit done: not before the kernel ahead may have finished, nor when the answer is wanted
+                pdl_wait();
+                word = px_any_word(p);
+            }
+            next += PX_TEAMS;
+            const bool t0 = mbar_test(rawfull + 8 * r, rph), t1 = mbar_test(empty + 8 * s, ph);
             if (!t0) ok = mbar_wait(rawfull + 8 * r, rph, p.flag, PX_CODE + 3);
-            if (ok && !t1) ok = mbar_wait(empty + 8 * s, ph ^ 1u, p.flag, PX_CODE + 7);
+            if (ok && !t1) ok = mbar_wait(empty + 8 * s, ph, p.flag, PX_CODE + 7);
+            ok = __all_sync(0xFFFFFFFFu, ok);
             if (!ok) break;
-            if (ut == 0) PX_TRACE(1, it);
             const uint32_t src = raw_base + (uint32_t)(r * PX_RAW_BYTES) + src0, dst = base + (uint32_t)(s * PX_A_BYTES) + dst0;
-            uint32_t w[16];
+            uint32_t words[16];
 #pragma unroll
-            for (int i = 0; i < 16; i++) w[i] = px_lds32(src + i * 512u);
+            for (int i = 0; i < 16; i++) words[i] = px_lds32(src + i * 512u);
             uint32_t z = 8, table[4];
             if (!p.sym) z = ((px_lds32(raw_base + (uint32_t)(r * PX_RAW_BYTES) + PX_BOX_BYTES + 4u * (ut >> 3)) >> (4 * (ut & 7))) & 0xFu) + 1u; // stored zero + 1
             px_table(table, z);
 #pragma unroll
-            for (int i = 0; i < 8; i++) px_unpack(dst + (((uint32_t)i ^ swz) << 4), table, w[2 * i], w[2 * i + 1]);
+            for (int i = 0; i < 8; i++) px_unpack(dst + (((uint32_t)i ^ swz) << 4), table, words[2 * i], words[2 * i + 1]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
             __syncwarp();
             if (lane == 0) {
                 mx_arrive(full + 8 * s);
                 mx_arrive(rawempty + 8 * r);
             }
-            if (ut == 0) PX_TRACE(2, it);
             s += PX_TEAMS;
             if (s >= S) { s -= S; ph ^= 1u; }
             r += PX_TEAMS;
@@ -433,28 +544,39 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
         const int mh = 8 * ((part_id + 1) * chunks / PARTS - chunk0); // this warp's tokens
         const uint32_t tlane = tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)col0;
         const int et = threadIdx.x - FOLD_WARP0 * 32;
-        int a = 0, c = 0, tr = 0;
+        int a = 0, c = 0;
         uint32_t aph = 0, cph = 0;
         bool ok = true;
-        for (long long u = u0; u < u1;) {
-            const int tile = (int)(u / G);
-            const long long tile_u0 = (long long)tile * G, seg_end = min(u1, tile_u0 + G);
-            const int folds = (int)(seg_end - u) * unit_folds;
+        pdl_wait();
+        const bool any = px_any_second(p, px_any_word(p)); // what it waits for comes before x's first tile does
+        for (int tile = first_tile, from = first_unit, left = nunits; left > 0; tile++) {
+            const int to = min(G, from + left);
+            const long long tile_u0 = (long long)tile * G;
             const float *srow = FP8 && p.scale_inv ? p.scale_inv + (size_t)(tile / p.token_blocks * PX_ROWS / p.block_out) * p.s_in : nullptr;
-            const int k_first = (int)(u - tile_u0) * PX_UNIT;
-            float s_next = srow ? __ldg(srow + k_first / p.block_in) : 1.0f; // E4M3: the next fold's scale, asked for a fold ahead
+            float s_next = srow ? __ldg(srow + from * PX_UNIT / p.block_in) : 1.0f; // E4M3: the next fold's scale, asked for a fold ahead
             float tot[NCH * 8];
 #pragma unroll
             for (int i = 0; i < NCH * 8; i++) tot[i] = 0.0f;
+            int more = 0; // units of the tile that come a second time
+            if (any) px_second_units(p, tile % p.token_blocks, from, to, [&](int, int) { more++; return true; });
+            const int folds = (to - from) * unit_folds, row0 = from * PX_UNIT;
 #pragma unroll 1
-            for (int f = 0; f < folds && ok; f++) {
-                if (et == 0) PX_TRACE(6, tr);
+            for (int f = 0; f < folds + more * unit_folds && ok; f++) {
                 float sc = s_next;
-                if (FP8 && srow && f + 1 < folds) s_next = __ldg(srow + (k_first + (f + 1) * p.fold_rows) / p.block_in);
+                if (FP8 && srow) {
+                    if (f + 1 < folds) s_next = __ldg(srow + (row0 + (f + 1) * p.fold_rows) / p.block_in);
+                    else if (more) { // the unit of fold f + 1
+                        int nth = (f + 1 - folds) / unit_folds, row = 0;
+                        px_second_units(p, tile % p.token_blocks, from, to, [&](int u, int) {
+                            row = u * PX_UNIT + (f + 1) % unit_folds * p.fold_rows;
+                            return nth-- > 0;
+                        });
+                        s_next = __ldg(srow + row / p.block_in);
+                    }
+                }
                 if (FP8) ok = mx_wait(accfull + 8 * a, aph, p.flag, PX_CODE + 4);
                 else ok = mx_wait2(frfull + 8 * c, cph, accfull + 8 * a, aph, p.flag, PX_CODE + 4);
                 if (!ok) break;
-                if (et == 0) PX_TRACE(7, tr);
                 const uint32_t fr = fr_base + (uint32_t)(c * p.fr_bytes);
                 if constexpr (!FP8) {
                     uint16_t sraw;
@@ -491,14 +613,12 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                     mx_arrive(accempty + 8 * a);
                     if (!FP8) mx_arrive(frempty + 8 * c);
                 }
-                if (et == 0) PX_TRACE(8, tr);
-                tr++;
                 if (++a == p.accs) { a = 0; aph ^= 1u; }
                 if (++c == PX_FR) { c = 0; cph ^= 1u; }
             }
             const int tok0 = tile % p.token_blocks * p.mpad, n0 = tile / p.token_blocks * PX_ROWS;
             const int mt = min(p.mpad, p.m - tok0); // this tile's tokens
-            if (seg_end - u == G) {
+            if (to - from == G) {
                 if (ok) {
                     const float bv = p.bias ? load_as_f32(p.bias, p.bias_dtype, (size_t)p.col_base + n0 + feature) : 0.0f;
 #pragma unroll
@@ -574,7 +694,8 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(FOLD_WARPS * 32) : "memory"); // tail[1] is read by all before it is written again
             }
-            u = seg_end;
+            left -= to - from;
+            from = 0;
         }
         if (et == 0) PX_TRACE(10, 1);
     }
@@ -609,10 +730,10 @@ bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const vo
            aligned(x, 16) && aligned(weight, 16) && aligned(scale_inv, 4);
 }
 
-// The scratch area: x's pieces and their block scales, then tickets and parts of shared tiles.
+// The scratch area: x's two pairs of pieces, their block scales, which units have a second pair; then tickets and parts of shared tiles.
 struct PackedMxScratch {
     int token_blocks, mpad, merged, tiles;
-    size_t sf, tickets, partials, part_bytes; // offsets of the pieces' successors; bytes of a part
+    size_t sf, pair_sf, second, tickets, partials, part_bytes; // offsets of the pieces' successors; bytes of a part
 };
 static PackedMxScratch packed_mx_layout(int m, int k, int n)
 {
@@ -623,8 +744,10 @@ static PackedMxScratch packed_mx_layout(int m, int k, int n)
     s.tiles = n / PX_ROWS * s.token_blocks;
     const size_t rows = (size_t)s.token_blocks * s.mpad, units = (size_t)k / PX_UNIT;
     auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-    s.sf = up(2 * rows * k);
-    s.tickets = s.sf + up(units * s.token_blocks * (s.merged ? 1 : 2) * PX_SF_BYTES);
+    s.pair_sf = units * s.token_blocks * (s.merged ? 1 : 2) * PX_SF_BYTES;
+    s.sf = up(2 * 2 * rows * k);
+    s.second = s.sf + 2 * s.pair_sf;
+    s.tickets = s.second + up(8 + 8 * units * s.token_blocks); // the call's mark in front
     s.partials = s.tickets + up((size_t)s.tiles * sizeof(unsigned long long));
     s.part_bytes = (size_t)s.mpad * PX_ROWS * sizeof(float);
     return s;
@@ -638,7 +761,7 @@ size_t packed_mx_scratch_bytes(int m, int k, int n)
 }
 
 template <int WT, int NCH, int PARTS>
-static int packed_mx_launch(const PackedMxParams &p, const CUtensorMap &wmap, const CUtensorMap &xmap, int ctas, size_t smem, cudaStream_t st)
+static int packed_mx_launch(const PackedMxParams &p, const CUtensorMap (&maps)[3], int ctas, size_t smem, cudaStream_t st)
 {
     auto kern = packed_mx_tc_kernel<WT, NCH, PARTS>;
     static size_t configured[64] = {};
@@ -657,7 +780,7 @@ static int packed_mx_launch(const PackedMxParams &p, const CUtensorMap &wmap, co
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, kern, p, wmap, xmap));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, kern, p, maps[0], maps[1], maps[2]));
     return OXQ_OK;
 }
 
@@ -670,7 +793,8 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
     const int m = p.m, n = p.n;
     p.token_blocks = s.token_blocks; p.mpad = s.mpad; p.merged = s.merged; p.tiles = s.tiles;
     p.units_per_tile = k / PX_UNIT;
-    p.sf = sb + s.sf;
+    p.sf = sb + s.sf; p.pair_sf = s.pair_sf;
+    p.any = reinterpret_cast<const unsigned long long *>(sb + s.second); p.second = p.any + 1;
     p.x_bytes = 2 * p.mpad * PX_UNIT;
     p.sf_bytes = (p.merged ? 1 : 2) * PX_SF_BYTES;
     p.fr_bytes = wt == PX_FP8 ? 0 : PX_SC_BYTES;
@@ -718,34 +842,36 @@ static int packed_mx_run(PackedMxParams &p, int wt, const void *x, const void *w
         if (force ? c <= force : cost < best) { best = cost; ctas = cand; p.split = 1; }
         if (cand == sm_count()) break;
     }
-    static std::atomic<unsigned long long> calls{0}; // marks differ between calls, in no order that a stale value would have by chance
-    p.mark = ((calls.fetch_add(1, std::memory_order_relaxed) + 1) * 0x9E3779B97F4A7C15ull) >> 8;
+    p.mark = mx_call_mark();
     p.tickets = reinterpret_cast<unsigned long long *>(sb + s.tickets);
     p.partials = reinterpret_cast<float *>(sb + s.partials);
 
-    CUtensorMap wmap, xmap;
+    CUtensorMap maps[3]; // weights, x a token block at a time, x a group at a time
     CUresult r;
     if (wt == PX_FP8)
-        r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, weight, (uint64_t)k, (uint64_t)n, (uint64_t)k, PX_UNIT, PX_ROWS,
+        r = encode_tiled_2d(&maps[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, weight, (uint64_t)k, (uint64_t)n, (uint64_t)k, PX_UNIT, PX_ROWS,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     else
-        r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, weight, (uint64_t)n, (uint64_t)k / 8, (uint64_t)n * 4, PX_ROWS, PX_UNIT / 8,
+        r = encode_tiled_2d(&maps[0], CU_TENSOR_MAP_DATA_TYPE_UINT32, weight, (uint64_t)n, (uint64_t)k / 8, (uint64_t)n * 4, PX_ROWS, PX_UNIT / 8,
                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (weights) failed with CUresult %d", (int)r);
-    r = encode_tiled_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, sb, (uint64_t)k, (uint64_t)p.token_blocks * 2 * p.mpad, (uint64_t)k, PX_UNIT,
-                        (uint32_t)(2 * p.mpad), CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (x) failed with CUresult %d", (int)r);
+    for (int i = 1; i <= 2; i++) {
+        r = encode_tiled_2d(&maps[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, sb, (uint64_t)k, (uint64_t)2 * p.token_blocks * 2 * p.mpad, (uint64_t)k, PX_UNIT,
+                            (uint32_t)(i == 1 ? 2 * p.mpad : PX_GROUP), CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+        OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (x) failed with CUresult %d", (int)r);
+    }
 
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ceil_div(m * p.units_per_tile * 16, 256), 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.gridDim = dim3(p.units_per_tile, p.token_blocks * p.mpad / PX_GROUP, 1);
+    cfg.blockDim = dim3(16 * PX_GROUP, 1, 1);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, packed_mx_split_kernel, (const __nv_bfloat16 *)x, sb, sb + s.sf, m, k, p.mpad, p.token_blocks, p.merged));
-#define OXQ_PX_LAUNCH(WT, NCH, PARTS) return packed_mx_launch<WT, NCH, PARTS>(p, wmap, xmap, (int)ctas, smem, st)
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, packed_mx_split_kernel, (const __nv_bfloat16 *)x, sb, sb + s.sf, sb + s.second + 8,
+                                reinterpret_cast<unsigned long long *>(sb + s.second), p.mark, m, k, p.mpad, p.token_blocks, p.merged));
+#define OXQ_PX_LAUNCH(WT, NCH, PARTS) return packed_mx_launch<WT, NCH, PARTS>(p, maps, (int)ctas, smem, st)
     if (wt == PX_FP8) {
         if (p.mpad <= 16) OXQ_PX_LAUNCH(PX_FP8, 1, 2);
         if (p.mpad <= 32) OXQ_PX_LAUNCH(PX_FP8, 2, 2);

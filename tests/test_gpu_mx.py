@@ -1,7 +1,7 @@
 """The block-scaled tensor-core kernels (E4M3 weights, MXFP4 experts of small batches): sizes at their edges.
 
 Weights are operands as stored and a bf16 activation is the sum of two E4M3 pieces, exact but for 2^-21 of the largest of its block
-of 32; products are exact and sums are f32. Against 64-bit sums over the exact weights a value is off by a few dozen f32 roundings
+of 32, or of four, exact but for 2^-34, where half of the block is small beside its largest; products are exact and sums are f32. Against 64-bit sums over the exact weights a value is off by a few dozen f32 roundings
 of the sum of |x w| at most, so 2^-17 of that sum bounds it, plus one bf16 rounding of the result.
 """
 import numpy as np
@@ -96,8 +96,8 @@ def test_fp8_block_scaled_special_values_stay_special(cuda):
     assert np.isfinite(y[np.ix_(rows, cols)]).all()
 
 
-# folds of 64 and of 128 columns; merged pieces, two MMAs, several token blocks; scratch from the least that is taken (the pieces and
-# their block scales) to all that helps
+# folds of 64 and of 128 columns; merged pieces, two MMAs, several token blocks; scratch from the least that is taken (the pieces, their
+# block scales and which units have a second pair) to all that helps
 @pytest.mark.parametrize("m,n,k,s_out,s_in", [(512, 512, 1024, 4, 16), (512, 512, 1024, 4, 8), (20, 256, 512, 2, 8), (65, 128, 256, 1, 4)])
 def test_fp8_block_scaled_stays_inside_its_scratch(cuda, m, n, k, s_out, s_in):
     w8, scale, w = fp8_weights(n, k, s_out, s_in, seed=m)
@@ -106,7 +106,7 @@ def test_fp8_block_scaled_stays_inside_its_scratch(cuda, m, n, k, s_out, s_in):
     blocks = -(-m // 128)
     mpad = -(-(-(-m // blocks)) // 16) * 16
     up = lambda v: -(-v // 256) * 256  # noqa: E731
-    least = up(2 * blocks * mpad * k) + up(k // 128 * blocks * (512 if mpad <= 32 else 1024))
+    least = up(4 * blocks * mpad * k) + 2 * (k // 128 * blocks * (512 if mpad <= 32 else 1024)) + up(8 + 8 * (k // 128) * blocks)
     full = int(_lib.load().oxq_fp8_scratch_bytes(m, k, n, s_out, s_in))
     assert least < full
     for size in sorted({least, least + 256, least + (full - least) // 3, full, min(full, 1105920)}):
@@ -125,6 +125,68 @@ def test_fp8_block_scaled_stays_inside_its_scratch(cuda, m, n, k, s_out, s_in):
             _lib.call("oxq_fp8_gemm", *args, room.data_ptr(), 256 + size, None)
             gemm.check(room)
             assert (room[256 + size:] == 0xA5).all()
+
+
+def activations_with_outliers(m, k, seed):
+    """Values about 0.01 with 3e3 in each block of 32 (rows 0, 4, ...), with 1e4 in two columns (rows 1, 5, ...), with -1e6 in one (rows 2, 6,
+    ...), rows of ordinary values; and the columns of the outliers."""
+    x = 0.01 * synth.activations(m, k, seed=seed)
+    x[0::4, 5::32] = 3e3
+    x[1::4, [7, k // 2 + 9]] = 1e4
+    x[2::4, k - 20] = -1e6
+    x[3::4] *= 100.0
+    return synth.bf16_round(x), np.r_[5:k:32, 7, k // 2 + 9, k - 20]
+
+
+def outlier_bound(x, w):
+    """What f32 sums leave of 64-bit ones, and the activations' error."""
+    m, k = x.shape
+    block = np.repeat(np.abs(x).reshape(m, -1, 32).max(-1), 32, -1).astype(np.float64)
+    return 2.0**-17 * np.abs(x).astype(np.float64) @ np.abs(w).T + 2.0**-34 * block @ np.abs(w).T
+
+
+def special_activations(m, k, seed):
+    """Rows with one infinity, with two of both signs, with a NaN, others with an outlier, the rest ordinary."""
+    x, _ = activations_with_outliers(m, k, seed)
+    x[1, 40], x[2, [3, k - 1]], x[4, k // 2], x[5, [0, 1]] = np.inf, [np.inf, -np.inf], np.nan, -np.inf
+    return x, [r for r in range(m) if r not in (1, 2, 4, 5)]
+
+
+def same_special(y, x, w):
+    """Where 64-bit products and sums are infinite or NaN (an infinity times zero is), these are."""
+    with np.errstate(invalid="ignore"):
+        ref = x.astype(np.float64) @ w.T
+    for r in np.nonzero(~np.isfinite(x).all(1))[0]:
+        with np.errstate(invalid="ignore"):
+            p = x[r].astype(np.float64) * w
+        ref[r] = [np.nan if np.isnan(q).any() or (np.isposinf(q).any() and np.isneginf(q).any()) else
+                  np.inf if np.isposinf(q).any() else -np.inf if np.isneginf(q).any() else v for q, v in zip(p, ref[r])]
+    assert np.array_equal(np.isnan(y), np.isnan(ref))
+    assert np.array_equal(np.where(np.isinf(y), np.sign(y), 0), np.where(np.isinf(ref), np.sign(ref), 0))
+
+
+# folds of 128 and of 64 columns; merged pieces, two MMAs, several token blocks; whole tiles, shares inside tiles and across them
+@pytest.mark.parametrize("n,k,s_out,s_in", [(128, 128, 1, 1), (256, 1536, 2, 24), (19072, 256, 149, 2), (128, 4224, 1, 33)])
+@pytest.mark.parametrize("m", [9, 20, 65, 300])
+def test_fp8_zero_weights_beside_outliers(cuda, m, n, k, s_out, s_in):
+    w8, scale, w = fp8_weights(n, k, s_out, s_in, seed=m + k)
+    x, columns = activations_with_outliers(m, k, seed=m)
+    w8[1::2, columns], w[1::2, columns] = 0, 0.0
+    y = fp8_gemm(w8, scale, bf16(x), n, k)
+    assert (np.abs(y.double().cpu().numpy() - x.astype(np.float64) @ w.T) <= outlier_bound(x, w)).all()
+    assert torch.equal(y, fp8_gemm(w8, scale, bf16(x), n, k))
+
+
+@pytest.mark.parametrize("n,k,s_out,s_in", [(128, 256, 1, 4), (512, 1024, 4, 8)])
+@pytest.mark.parametrize("m", [9, 33, 140])
+def test_fp8_infinities(cuda, m, n, k, s_out, s_in):
+    w8, scale, w = fp8_weights(n, k, s_out, s_in, seed=m)
+    w8[::5, 40], w[::5, 40] = 0, 0.0
+    x, rest = special_activations(m, k, seed=m)
+    y = fp8_gemm(w8, scale, bf16(x), n, k).double().cpu().numpy()
+    same_special(y, x, w)
+    block = np.repeat(np.abs(x[rest]).reshape(len(rest), -1, 32).max(-1), 32, -1).astype(np.float64)
+    assert (np.abs(y[rest] - x[rest].astype(np.float64) @ w.T) <= outlier_bound(x[rest], w) + 2.0**-26 * block @ np.abs(w).T).all()
 
 
 @pytest.mark.parametrize("m", [9, 16])
@@ -200,6 +262,35 @@ def test_gptq_zero_weights_beside_large_activations(cuda, sym):
     w = codes.double() * dev[2].double().repeat_interleave(g, 0)
     xd = xd.double()
     assert ((y.double() - xd @ w).abs() <= 2.0**-19 * (xd.abs() @ w.abs())).all()
+
+
+@pytest.mark.parametrize("k,n,g,sym", [(1152, 36864, 128, True), (14336, 3072, 512, False)])
+@pytest.mark.parametrize("special", [False, True])
+def test_gptq_outliers_and_infinities(cuda, k, n, g, sym, special):
+    m = 16
+    rng = np.random.default_rng(k)
+    x, columns = activations_with_outliers(m, k, seed=k)
+    rest = list(range(m))
+    if special:
+        x, rest = special_activations(m, k, seed=k)
+    nib = rng.integers(0, 16, (k, n), dtype=np.uint32)
+    zero = np.full((k // g, n), 8, np.uint32) if sym else rng.integers(1, 16, (k // g, n), dtype=np.uint32)
+    nib[columns, 1::2] = zero[columns // g, 1::2]
+    nib[40, ::3] = zero[0, ::3]
+    qw = (nib.reshape(k // 8, 8, n) << (4 * np.arange(8, dtype=np.uint32))[None, :, None]).sum(1, dtype=np.uint32)
+    qz = ((zero - 1).reshape(k // g, n // 8, 8) << (4 * np.arange(8, dtype=np.uint32))).sum(2, dtype=np.uint32)
+    sc = (np.abs(rng.standard_normal((k // g, n)) * 0.02) / 7 + 1e-4).astype(np.float16)
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (qw, qz, sc)]
+    lin = L.PackedQuantLinear(L.QuantWeight.new_gptq(4, sym, dev[0], None if sym else dev[1], dev[2]))
+    y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+    gemm.packed4_matmul(lin, bf16(x), y)
+    w = ((nib.astype(np.int32) - np.repeat(zero, g, 0).astype(np.int32)) * np.repeat(sc.astype(np.float64), g, 0)).T
+    got = y.double().cpu().numpy()
+    if special:
+        same_special(got, x, w)
+    block = np.repeat(np.abs(x[rest]).reshape(len(rest), -1, 32).max(-1), 32, -1).astype(np.float64)
+    extra = 2.0**-26 * block @ np.abs(w).T if special else 0.0
+    assert (np.abs(got[rest] - x[rest].astype(np.float64) @ w.T) <= outlier_bound(x[rest], w) + extra).all()
 
 
 # ------------------------------------------------------------------------------------------------------- MXFP4 experts, small batches

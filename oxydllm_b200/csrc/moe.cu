@@ -4,7 +4,7 @@
 //   [dequantize -> grouped GEMM (down)]* -> weighted combine in ascending expert order.
 // Mirrors MoeFeedForward::forward + dispatch_sparse + MoeExpert::GptOss (moe.rs:466-499,
 // 563-607, 152-173); every reduction has a fixed order, so results are run-to-run identical.
-#include "oxq_common.cuh"
+#include "mx_common.cuh"
 
 namespace oxq {
 
@@ -23,11 +23,13 @@ int moe_fused_grouped(const void *a, int a_rows, const uint8_t *blocks, const ui
 int moe_mx_block_rows();
 size_t moe_mx_piece_bytes(int rows, int k);
 size_t moe_mx_scale_bytes(int rows, int k);
+size_t moe_mx_second_bytes(int rows, int k);
 bool moe_mx_supported(int n, int k, const void *blocks, const void *scales);
-int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, cudaStream_t st);
-int moe_mx_grouped(const void *pieces, const void *sfx, int rows_cap, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
-                   const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi, float limit,
-                   int *flag, cudaStream_t st);
+int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, void *second,
+                 unsigned long long mark, cudaStream_t st);
+int moe_mx_grouped(const void *pieces, const void *sfx, const void *second, unsigned long long mark, int rows_cap, const uint8_t *blocks,
+                   const uint8_t *scales, int experts, int n, int k, const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype,
+                   void *out, int ldo, int epi, float limit, int *flag, cudaStream_t st);
 bool mxfp4_gemv_batched_supported(int k, const void *blocks);
 int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const uint8_t *scales, const void *bias,
                        int bias_dtype, const int *pair_expert, int pairs, int e_lo, int e_hi, void *y, int y_dtype, int k,
@@ -440,7 +442,7 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct MoeLayout {
     size_t top_idx, top_w, counts, offsets, grp_beg, entries, perm, inv, xs, h, slab, total;
-    size_t h_scales, x_scales; // inside the slab
+    size_t h_scales, h_second, x_pieces, x_scales, x_second; // inside the slab
     int group_experts, n_groups, max_mt;
     bool decode; // few pairs: no dequantized slab, the slab region holds the f32 gate_up outputs
 };
@@ -477,12 +479,15 @@ static MoeLayout moe_layout(int tokens, int top_k, int n_exp, int hidden, int in
     L.xs = off; off = align_up(off + (pairs + 128) * hidden * 2, 256); // also the down-projection output
     L.h = off; off = align_up(off + (pairs + 128) * inter * 2, 256);
     L.decode = moe_decode_shape(pairs, hidden, inter);
-    // dequantized experts; or the f32 gate_up outputs; or, for the block-scaled kernel, the pieces of h, their scales and those of x's
-    // (x's pieces take as much as xs)
+    // dequantized experts; or the f32 gate_up outputs; or, for the block-scaled kernel, the pieces of h and of x with their scales and
+    // what says which of them have a second pair
     const int cap = (int)pairs + 128;
     L.h_scales = align_up(moe_mx_piece_bytes(cap, inter), 256);
-    L.x_scales = L.h_scales + align_up(moe_mx_scale_bytes(cap, inter), 256);
-    const size_t mx = L.x_scales + moe_mx_scale_bytes(cap, hidden), f32 = pairs * 2 * inter * sizeof(float);
+    L.h_second = L.h_scales + align_up(moe_mx_scale_bytes(cap, inter), 256);
+    L.x_pieces = L.h_second + align_up(moe_mx_second_bytes(cap, inter), 256);
+    L.x_scales = L.x_pieces + align_up(moe_mx_piece_bytes(cap, hidden), 256);
+    L.x_second = L.x_scales + align_up(moe_mx_scale_bytes(cap, hidden), 256);
+    const size_t mx = L.x_second + moe_mx_second_bytes(cap, hidden), f32 = pairs * 2 * inter * sizeof(float);
     const size_t dense = (size_t)ge * per_expert;
     L.slab = off; off = align_up(off + (L.decode ? (f32 > mx ? f32 : mx) : dense > mx ? dense : mx), 256);
     L.total = off;
@@ -594,15 +599,16 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     if (mx) {
         unsigned char *sb = reinterpret_cast<unsigned char *>(slab);
         OXQ_LAUNCH_CHECK("moe routing kernels");
-        int rc = moe_mx_split(x, perm, top_k, offsets + n_exp, hidden, a_rows, xs, sb + L.x_scales, st);
+        const unsigned long long mark = mx_call_mark();
+        int rc = moe_mx_split(x, perm, top_k, offsets + n_exp, hidden, a_rows, sb + L.x_pieces, sb + L.x_scales, sb + L.x_second, mark, st);
         if (rc) return rc;
-        rc = moe_mx_grouped(xs, sb + L.x_scales, a_rows, gu_blocks, gu_scales, num_experts, 2 * inter, hidden, entries, grp_beg, gu_bias,
-                            bias_dtype, h, inter, 1, limit, flag, st);
+        rc = moe_mx_grouped(sb + L.x_pieces, sb + L.x_scales, sb + L.x_second, mark, a_rows, gu_blocks, gu_scales, num_experts, 2 * inter, hidden,
+                            entries, grp_beg, gu_bias, bias_dtype, h, inter, 1, limit, flag, st);
         if (rc) return rc;
-        rc = moe_mx_split(h, nullptr, 1, offsets + n_exp, inter, a_rows, sb, sb + L.h_scales, st);
+        rc = moe_mx_split(h, nullptr, 1, offsets + n_exp, inter, a_rows, sb, sb + L.h_scales, sb + L.h_second, mark, st);
         if (rc) return rc;
-        rc = moe_mx_grouped(sb, sb + L.h_scales, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg, dn_bias,
-                            bias_dtype, xs, hidden, 0, limit, flag, st);
+        rc = moe_mx_grouped(sb, sb + L.h_scales, sb + L.h_second, mark, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg,
+                            dn_bias, bias_dtype, xs, hidden, 0, limit, flag, st);
         if (rc) return rc;
         OXQ_CUDA(launch_early(moe_combine_kernel, sm_count() * 8, 256, st, xs, top_idx, top_w, inv, tokens, top_k, hidden, expert_lo, expert_hi,
                               out, out_dtype));

@@ -3,7 +3,8 @@
 // writes bf16 weights into its operand tile and is the faster one from a few dozen rows per expert on.
 // Mirrors the expert half of MoeFeedForward::forward (moe.rs:466-499, dispatch_sparse 563-607).
 //
-// Activations are exact as two E4M3 pieces with block scales (mx_common.cuh), written by a kernel in front. A unit of work is (token
+// Activations are two E4M3 pieces with block scales (mx_common.cuh), written by a kernel in front; a stage in which a token block has
+// outliers, infinities or NaN comes a second time, at the unit's end, with a second pair of pieces. A unit of work is (token
 // block of one expert: up to 48 expert-sorted rows) x (128 out features); CTA b takes units b, b + grid, ... of the device-side
 // table, feature tiles fastest. The pieces are neighbouring columns of one MMA (hi | lo), and stages of 128 input columns go to two
 // accumulators in turn, so that two warps issue them; the epilogue adds the four. Roles:
@@ -43,7 +44,11 @@ struct MoeMxParams {
     const int4 *entries;   // token blocks: {first row in the expert-sorted matrix, rows, expert, -}
     const int *n_blocks;   // how many
     const uint8_t *scales; // [experts, n, k / 32]
-    const uint32_t *sfx;   // [stage][rows_cap] block scales of the rows' hi pieces
+    const uint32_t *sfx;   // [pair][stage][rows_cap] block scales of the rows' hi pieces
+    const unsigned char *second;   // [stage][rows_cap] MX_...: whether the row has a second pair of pieces there
+    const unsigned char *pieces;   // [pair][piece][rows_cap][k]
+    const unsigned long long *any; // `mark` where some have
+    unsigned long long mark;
     const void *bias;      // [experts, n] or null
     void *out;
     int *flag;
@@ -54,12 +59,13 @@ struct MoeMxParams {
     int test_skip_loads;   // self-test only: the weight producer issues nothing
 };
 
-// ---- rows -> two E4M3 pieces and block scales --------------------------------------------------------------------------------
-// Sixteen lanes hold 128 columns of a row. Row r is src[perm[r] / top_k] (perm null: src[r]); q: [piece][rows_cap][k];
-// sfx: [stage][rows_cap], a byte per 32 columns. k is a multiple of 32.
+// ---- rows -> pieces and block scales ---------------------------------------------------------------------------------------------
+// Sixteen lanes hold 128 columns of a row. Row r is src[perm[r] / top_k] (perm null: src[r]); q: [pair][piece][rows_cap][k]; sfx:
+// [pair][stage][rows_cap], a byte per 32 columns; second: [stage][rows_cap]. The second pair is written where a row has one, and not at
+// all elsewhere. k is a multiple of 32.
 __global__ void __launch_bounds__(256)
     moe_mx_split_kernel(const __nv_bfloat16 *src, const int *perm, int top_k, const int *total_rows, int k, int stages, int rows_cap,
-                        unsigned char *q, unsigned char *sfx)
+                        unsigned char *q, unsigned char *sfx, unsigned char *second, unsigned long long *any, unsigned long long mark)
 {
     pdl_wait();
     pdl_launch_dependents();
@@ -70,72 +76,82 @@ __global__ void __launch_bounds__(256)
         const int from = perm ? ld_produced(perm + row) / top_k : row;
         uint4 raw = make_uint4(0u, 0u, 0u, 0u);
         if (c < k) raw = ld_produced(reinterpret_cast<const uint4 *>(src + (size_t)from * k + c));
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-        float v[8];
-        uint32_t amax = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            v[2 * i] = bf16_lo_f32(w[i]);
-            v[2 * i + 1] = bf16_hi_f32(w[i]);
-            amax = max(amax, max(w[i] << 16 & 0x7FFF0000u, w[i] & 0x7FFF0000u));
-        }
-#pragma unroll
-        for (int o = 1; o <= 2; o <<= 1) amax = max(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o)); // four lanes hold a block of 32
-        uint2 hi, lo;
-        const uint32_t s = mx_split8(v, amax, hi, lo);
-        if (real && c < k) {
-            unsigned char *dst = q + (size_t)row * k + c;
+        const MxBlock b = mx_block(raw);
+        auto store = [&](int pair, uint2 hi, uint2 lo, uint32_t s) {
+            if (!real || c >= k) return;
+            unsigned char *dst = q + ((size_t)pair * 2 * rows_cap + row) * k + c;
             *reinterpret_cast<uint2 *>(dst) = hi;
             *reinterpret_cast<uint2 *>(dst + (size_t)rows_cap * k) = lo;
-            if ((lane & 3) == 0) sfx[((size_t)st * rows_cap + row) * 4 + (lane >> 2)] = (unsigned char)s;
+            if ((lane & 3) == 0) sfx[((size_t)(pair * stages + st) * rows_cap + row) * 4 + (lane >> 2)] = (unsigned char)s;
+        };
+        float v[8];
+        uint2 hi, lo;
+        const uint32_t s = mx_first_pair(raw, b, v, hi, lo);
+        store(0, hi, lo, s);
+        const unsigned half = 0xFFFFu << (threadIdx.x & 16); // the row's lanes of this warp
+        const unsigned ask = __ballot_sync(0xFFFFFFFFu, b.second != MX_ONE_PAIR), e5m2 = __ballot_sync(0xFFFFFFFFu, b.second == MX_SECOND_E5M2);
+        if (real && lane == 0) second[(size_t)st * rows_cap + row] = (unsigned char)(!(ask & half) ? MX_ONE_PAIR : (e5m2 & half) ? MX_SECOND_E5M2 : MX_SECOND_E4M3);
+        if (ask) { // some row of the warp
+            const uint32_t s2 = mx_second_pair(raw, v, s, (e5m2 & half) != 0, hi, lo);
+            if (ask & half) store(1, hi, lo, s2);
+            if (real && lane == 0) *any = mark;
         }
     }
 }
 
-__global__ void __launch_bounds__(MM_THREADS, 1)
-    moe_mx_kernel(const MoeMxParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
+// Stages in which rows of a token block have a second pair, in order, E4M3 before E5M2: body(stage, MX_...), until it returns false.
+template <typename Body> __device__ __forceinline__ bool mm_second_stages(const MoeMxParams &p, int4 en, Body body)
 {
-    extern __shared__ unsigned char smem_raw[];
-    pdl_launch_dependents();
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
-    unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    // A slots | rows' slots | ring of packed boxes | scales of A and of the rows per slot | barriers | tensor-memory address
+    for (int t = 0; t < p.stages; t += 32) {
+        const int at = t + (int)(threadIdx.x & 31);
+        unsigned kinds = 0; // of the rows, four at a time: all loads are under way together
+        if (at < p.stages) {
+            const size_t first = (size_t)at * p.rows_cap + en.x;
+            const unsigned *words = reinterpret_cast<const unsigned *>(p.second + (first & ~(size_t)3));
+            const int skip = (int)(first & 3), span = skip + en.y;
+#pragma unroll
+            for (int w = 0; w < MM_MAX_TOK / 4 + 1; w++)
+                if (4 * w < span) {
+                    unsigned v = ld_produced(words + w);
+                    if (w == 0) v &= ~0u << (8 * skip);
+                    if (4 * w + 4 > span) v &= ~0u >> (8 * (4 * w + 4 - span));
+                    kinds |= v;
+                }
+            kinds |= kinds >> 16;
+            kinds |= kinds >> 8;
+        }
+        const unsigned e4m3 = __ballot_sync(0xFFFFFFFFu, kinds & MX_SECOND_E4M3), e5m2 = __ballot_sync(0xFFFFFFFFu, kinds & MX_SECOND_E5M2);
+        for (unsigned hit = e4m3 | e5m2; hit; hit &= hit - 1) {
+            const int i = __ffs(hit) - 1;
+            if ((e4m3 >> i & 1u) && !body(t + i, MX_SECOND_E4M3)) return false;
+            if ((e5m2 >> i & 1u) && !body(t + i, MX_SECOND_E5M2)) return false;
+        }
+    }
+    return true;
+}
+// A unit's stages as all roles walk them: body(stage, pair, MX_...), until it returns false.
+template <bool SECOND, typename Body> __device__ __forceinline__ bool mm_stages(const MoeMxParams &p, int4 en, Body body)
+{
+    bool ok = true;
+    for (int it = 0; it < p.stages && ok; it++) ok = body(it, 0, MX_ONE_PAIR);
+    if (SECOND && ok) ok = mm_second_stages(p, en, [&](int it, int kind) { return body(it, 1, kind); });
+    return ok;
+}
+
+// Shared memory behind `base`: A slots | rows' slots | ring of packed boxes | scales of A and of the rows per slot | barriers | tensor-memory
+// address.
+constexpr int MM_BARS = MM_SLOTS * (MM_A_BYTES + MM_X_BYTES + 2 * MM_SF_BYTES) + MM_RAW * MM_RAW_BYTES;
+
+// What the warps do; SECOND: with stages that come a second time.
+template <bool SECOND>
+__device__ __forceinline__ void moe_mx_roles(const MoeMxParams &p, const CUtensorMap &wmap, const CUtensorMap &xmap, uint32_t base, uint32_t tmem_base, int n_units)
+{
     const uint32_t x_base = base + MM_SLOTS * MM_A_BYTES, raw_base = x_base + MM_SLOTS * MM_X_BYTES;
-    const uint32_t sf_base = raw_base + MM_RAW * MM_RAW_BYTES, bars = sf_base + MM_SLOTS * 2 * MM_SF_BYTES;
+    const uint32_t sf_base = raw_base + MM_RAW * MM_RAW_BYTES, bars = base + MM_BARS;
     const uint32_t rawfull = bars, rawempty = rawfull + 8 * MM_RAW, full = rawempty + 8 * MM_RAW, empty = full + 8 * MM_SLOTS,
                    tfull = empty + 8 * MM_SLOTS, tempty = tfull + 16;
-    volatile uint32_t *tail = reinterpret_cast<volatile uint32_t *>(base_ptr + (bars + 8 * MM_NUM_BARS - base));
-
-    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    if (warp == 0) {
-        if (lane < MM_RAW) {
-            mbar_init(rawfull + 8 * lane, 1);
-            mbar_init(rawempty + 8 * lane, MM_TEAM_WARPS);
-        }
-        if (lane < MM_SLOTS) {
-            mbar_init(full + 8 * lane, MM_TEAM_WARPS + 1); // the team's warps and the rows' producer
-            mbar_init(empty + 8 * lane, 1);
-        }
-        if (lane < 2) {
-            mbar_init(tfull + 8 * lane, 2); // both issuers
-            mbar_init(tempty + 8 * lane, MM_EPI_WARPS);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) { // the allocating warp also frees
-        tmem_alloc(bars + 8 * MM_NUM_BARS, 512u);
-        tmem_relinquish();
-    }
-    for (uint32_t i = threadIdx.x; i < MM_SLOTS * MM_A_BYTES / 16; i += MM_THREADS) // the unused half of every operand chunk
-        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + i * 16u), "r"(0u) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = tail[0], tmem_acc = tmem_base + MM_SF_COLS;
-    pdl_wait(); // table, rows and their scales come from kernels ahead; their time must not count as this kernel's waits
-    const int n_units = ld_produced(p.n_blocks) * p.tiles_n, T = p.stages;
-
+    const uint32_t tmem_acc = tmem_base + MM_SF_COLS;
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, T = p.stages;
     if (warp == 0) {
         // ---- packed nibbles --------------------------------------------------------------------------------------------
         const bool leader = elect_one();
@@ -144,16 +160,18 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
         bool ok = true;
         for (int u = blockIdx.x; ok && u < n_units && !p.test_skip_loads; u += gridDim.x) {
             const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
-            const int rowbase = ld_produced(p.entries + tb).z * p.n + f * MM_ROWS;
-            for (int it = 0; it < T && ok; it++) {
-                ok = mx_wait(rawempty + 8 * r, ph, p.flag, MM_CODE + 1);
+            const int4 en = ld_produced(p.entries + tb);
+            const int rowbase = en.z * p.n + f * MM_ROWS;
+            ok = mm_stages<SECOND>(p, en, [&](int it, int, int) {
+                const bool ok = mx_wait(rawempty + 8 * r, ph, p.flag, MM_CODE + 1);
                 if (ok && leader) {
                     mbar_arrive_expect_tx(rawfull + 8 * r, MM_RAW_BYTES);
                     tma_load_2d(raw_base + (uint32_t)(r * MM_RAW_BYTES), &wmap, rawfull + 8 * r, it * (MM_BK / 2), rowbase);
                 }
                 __syncwarp();
                 if (++r == MM_RAW) { r = 0; ph ^= 1u; }
-            }
+                return ok;
+            });
         }
     } else if (warp == 2) {
         // ---- both pieces of the block's rows ----------------------------------------------------------------------------------
@@ -162,11 +180,44 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
         uint32_t ph = 1;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x) {
-            const int4 en = ld_produced(p.entries + u / p.tiles_n);
+            const int tb = u / p.tiles_n;
+            const int4 en = ld_produced(p.entries + tb);
             const int boxes = (en.y + MM_XBOX_ROWS - 1) / MM_XBOX_ROWS;
-            for (int it = 0; it < T && ok; it++, done++) {
-                ok = mx_wait(empty + 8 * s, ph, p.flag, MM_CODE + 2);
-                if (ok && leader) {
+            ok = mm_stages<SECOND>(p, en, [&](int it, int pair, int kind) {
+                const bool ok = mx_wait(empty + 8 * s, ph, p.flag, MM_CODE + 2);
+                if (SECOND && pair && ok) { // 16 bytes at a time, zeros where the row has no second pair of this kind; lo's rows follow hi's
+                    constexpr int AHEAD = 4; // rows that a lane has on their way
+                    const int j = lane & 7, col = it * MM_BK + 16 * j, n16 = boxes * MM_XBOX_ROWS;
+                    for (int r0 = lane >> 3; r0 < n16; r0 += 4 * AHEAD) {
+                        uint4 v[2][AHEAD];
+                        bool has[AHEAD];
+#pragma unroll
+                        for (int i = 0; i < AHEAD; i++) {
+                            const int r = r0 + 4 * i;
+                            has[i] = r < en.y && col < p.k && ld_produced(p.second + (size_t)it * p.rows_cap + en.x + r) == kind;
+                        }
+#pragma unroll
+                        for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+                            for (int piece = 0; piece < 2; piece++) {
+                                v[piece][i] = make_uint4(0u, 0u, 0u, 0u);
+                                if (has[i])
+                                    v[piece][i] = ld_produced(reinterpret_cast<const uint4 *>(p.pieces + ((size_t)(2 + piece) * p.rows_cap + en.x + r0 + 4 * i) * p.k + col));
+                            }
+#pragma unroll
+                        for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+                            for (int piece = 0; piece < 2; piece++) {
+                                const int at = piece * n16 + r0 + 4 * i;
+                                if (r0 + 4 * i < n16)
+                                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(x_base + (uint32_t)(s * MM_X_BYTES + at * MM_BK + ((j ^ (at & 7)) << 4))),
+                                                 "r"(v[piece][i].x), "r"(v[piece][i].y), "r"(v[piece][i].z), "r"(v[piece][i].w) : "memory");
+                            }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the MMA
+                    __syncwarp();
+                    if (leader) mx_arrive(full + 8 * s);
+                } else if (ok && leader) {
                     mbar_arrive_expect_tx(full + 8 * s, (uint32_t)(2 * boxes * MM_XBOX_BYTES));
                     const uint32_t dst = x_base + (uint32_t)(s * MM_X_BYTES);
                     for (int b = 0; b < 2 * boxes; b++) { // lo's rows follow hi's
@@ -177,7 +228,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
                 }
                 __syncwarp();
                 if (++s == MM_SLOTS) { s = 0; ph ^= 1u; }
-            }
+                done++;
+                return ok;
+            });
         }
         // The commits of the last stages arrive here asynchronously: the CTA stays until they have.
         for (int left = min(MM_SLOTS, done), q = done - left; left > 0 && ok; left--, q++)
@@ -191,18 +244,21 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
         uint32_t ph = 0, parity = 0; // parity: of the stages counted so far
         bool ok = true;
         for (int u = blockIdx.x; ok && u < n_units; u += gridDim.x, ul++) {
-            const int n16 = (ld_produced(p.entries + u / p.tiles_n).y + 15) & ~15;
-            const uint32_t idesc = mx_idesc(MX_E2M1, 2 * n16);
+            const int4 en = ld_produced(p.entries + u / p.tiles_n);
+            const int n16 = (en.y + 15) & ~15;
+            const uint32_t idesc0 = mx_idesc(MX_E2M1, 2 * n16);
             const int buf = ul & 1;
             const uint32_t d = tmem_acc + (uint32_t)((2 * buf + me) * MM_ACC_COLS);
             ok = mx_wait(tempty + 8 * buf, (((uint32_t)ul >> 1) & 1u) ^ 1u, p.flag, MM_CODE + 3);
             bool first = true;
-            for (int it = 0; it < T && ok; it++) {
+            ok = ok && mm_stages<SECOND>(p, en, [&](int it, int, int kind) {
+                bool ok = true;
                 if (parity == (uint32_t)me) {
                     ok = mx_wait(full + 8 * s, ph, p.flag, MM_CODE + 4);
                     if (ok) {
                         tc_fence_after();
                         if (leader) {
+                            const uint32_t idesc = kind == MX_SECOND_E5M2 ? idesc0 ^ MX_IDESC_B_E5M2 : idesc0;
                             const uint32_t sfa = tmem_base + 8u * s, sfs = sf_base + (uint32_t)(s * 2 * MM_SF_BYTES);
                             tmem_cp_scales(sfa, sfs);
                             tmem_cp_scales(sfa + 4, sfs + MM_SF_BYTES);
@@ -220,7 +276,8 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
                 }
                 parity ^= 1u;
                 if (++s == MM_SLOTS) { s = 0; ph ^= 1u; }
-            }
+                return ok;
+            });
             if (ok && leader) umma_commit(tfull + 8 * buf);
             __syncwarp();
         }
@@ -246,7 +303,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
             const uint32_t *xrow = p.sfx + en.x + (has_row ? ut : 0);
             const int lo_row = n16 + ut;
             const uint32_t lo_at = (uint32_t)(lo_row & 31) * 16u + (uint32_t)(lo_row >> 5) * 4u;
-            for (int it = 0; it < T && ok; it++) {
+            ok = mm_stages<SECOND>(p, en, [&](int it, int pair, int kind) {
                 if (turn == team) {
                     // the scales come straight from L2 and are asked for ahead of the polls, which hide their latency; past the last
                     // out feature and past k: 1.0 (never used there, but no NaN)
@@ -263,11 +320,13 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
                             for (int j = 0; j < 4; j++) sa |= (it * 4 + j < p.nkb ? (uint32_t)__ldg(sp + j) : 127u) << (8 * j);
                         }
                     }
-                    const uint32_t sx = has_row ? ld_produced(xrow + (size_t)it * p.rows_cap) : 0x7F7F7F7Fu;
+                    uint32_t sx = 0x7F7F7F7Fu;
+                    if (has_row && (!SECOND || !pair || ld_produced(p.second + (size_t)it * p.rows_cap + en.x + ut) == kind))
+                        sx = ld_produced(xrow + (size_t)(pair * T + it) * p.rows_cap);
                     const bool t0 = mbar_test(rawfull + 8 * s, ph), t1 = !reused || mbar_test(empty + 8 * s, ph ^ 1u);
-                    if (!t0) ok = mbar_wait(rawfull + 8 * s, ph, p.flag, MM_CODE + 5);
+                    bool ok = t0 || mbar_wait(rawfull + 8 * s, ph, p.flag, MM_CODE + 5);
                     if (ok && !t1) ok = mbar_wait(empty + 8 * s, ph ^ 1u, p.flag, MM_CODE + 6);
-                    if (!ok) break;
+                    if (!__all_sync(0xFFFFFFFFu, ok)) return false;
                     const uint32_t src = raw_base + (uint32_t)(s * MM_RAW_BYTES) + src0, dst = base + (uint32_t)(s * MM_A_BYTES) + dst0;
                     uint4 w[4];
 #pragma unroll
@@ -293,16 +352,19 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
                 }
                 if (++turn == MM_TEAMS) turn = 0;
                 if (++s == MM_SLOTS) { s = 0; ph ^= 1u; reused = true; }
-            }
+                return true;
+            });
         }
     } else {
         // ---- epilogue: lane = out feature inside this warp's quarter of the accumulator rows ---------------------------------
         const int quad = warp & 3;
         __nv_bfloat16 *outp = reinterpret_cast<__nv_bfloat16 *>(p.out);
-        int ul = 0;
+        int ul = 0, before = 0; // stages so far
         for (int u = blockIdx.x; u < n_units; u += gridDim.x, ul++) {
             const int tb = u / p.tiles_n, f = u - tb * p.tiles_n;
             const int4 en = ld_produced(p.entries + tb);
+            int here = T;
+            if (SECOND) mm_second_stages(p, en, [&](int, int) { here++; return true; });
             const int n16 = (en.y + 15) & ~15, buf = ul & 1;
             const int feat = f * MM_ROWS + quad * 32 + lane;
             const bool fv = feat < p.n;
@@ -310,8 +372,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
             if (!mx_wait(tfull + 8 * buf, ((uint32_t)ul >> 1) & 1u, p.flag, MM_CODE + 4)) break;
             tc_fence_after();
             const uint32_t t0 = tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)(2 * buf * MM_ACC_COLS);
-            const bool two = T > 1; // a single stage leaves one of the accumulators alone
-            const uint32_t ta = two || !(ul & 1) ? t0 : t0 + MM_ACC_COLS, tb2 = two ? t0 + MM_ACC_COLS : ta;
+            const bool two = here > 1; // a single stage leaves one of the accumulators alone
+            const uint32_t ta = two || !(before & 1) ? t0 : t0 + MM_ACC_COLS, tb2 = two ? t0 + MM_ACC_COLS : ta;
+            before += here;
             for (int c0 = 0; c0 < n16; c0 += 8) {
                 uint32_t a[8], b[8], c[8], e[8];
                 tmem_ld_x8(ta + c0, a);
@@ -352,6 +415,56 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
             if (lane == 0) mx_arrive(tempty + 8 * buf);
         }
     }
+}
+// Two kernels, of which a call launches both and one returns at once: a launch costs less than the second pairs cost the usual path in
+// one kernel (340 tokens 192 us a layer with the code for both in a call, 248 in one loop).
+template <bool SECOND>
+__global__ void __launch_bounds__(MM_THREADS, 1)
+    moe_mx_kernel(const MoeMxParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
+{
+    extern __shared__ unsigned char smem_raw[];
+    pdl_launch_dependents();
+    if (SECOND) {
+        pdl_wait();
+        if (ld_produced(p.any) != p.mark) return;
+    }
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
+    unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t bars = base + MM_BARS;
+    const uint32_t rawfull = bars, rawempty = rawfull + 8 * MM_RAW, full = rawempty + 8 * MM_RAW, empty = full + 8 * MM_SLOTS,
+                   tfull = empty + 8 * MM_SLOTS, tempty = tfull + 16;
+    volatile uint32_t *tail = reinterpret_cast<volatile uint32_t *>(base_ptr + (bars + 8 * MM_NUM_BARS - base));
+
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    if (warp == 0) {
+        if (lane < MM_RAW) {
+            mbar_init(rawfull + 8 * lane, 1);
+            mbar_init(rawempty + 8 * lane, MM_TEAM_WARPS);
+        }
+        if (lane < MM_SLOTS) {
+            mbar_init(full + 8 * lane, MM_TEAM_WARPS + 1); // the team's warps and the rows' producer
+            mbar_init(empty + 8 * lane, 1);
+        }
+        if (lane < 2) {
+            mbar_init(tfull + 8 * lane, 2); // both issuers
+            mbar_init(tempty + 8 * lane, MM_EPI_WARPS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) { // the allocating warp also frees
+        tmem_alloc(bars + 8 * MM_NUM_BARS, 512u);
+        tmem_relinquish();
+    }
+    for (uint32_t i = threadIdx.x; i < MM_SLOTS * MM_A_BYTES / 16; i += MM_THREADS) // the unused half of every operand chunk
+        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + i * 16u), "r"(0u) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tail[0];
+    pdl_wait(); // table, rows and their scales come from kernels ahead; their time must not count as this kernel's waits
+    const int n_units = SECOND || ld_produced(p.any) != p.mark ? ld_produced(p.n_blocks) * p.tiles_n : 0;
+    moe_mx_roles<SECOND>(p, wmap, xmap, base, tmem_base, n_units);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -366,9 +479,10 @@ static thread_local int g_moe_mx_selftest_skip_loads = 0; // set only inside oxq
 int moe_mx_block_rows() { return MM_MAX_TOK; }
 
 static int moe_mx_stages(int k) { return (k + MM_BK - 1) / MM_BK; }
-// Bytes of the pieces and of the block scales of `rows` rows.
-size_t moe_mx_piece_bytes(int rows, int k) { return (size_t)2 * rows * k; }
-size_t moe_mx_scale_bytes(int rows, int k) { return (size_t)4 * rows * moe_mx_stages(k); }
+// Bytes of both pairs of pieces of `rows` rows, of their block scales, and of what says which have a second pair (the call's mark in front).
+size_t moe_mx_piece_bytes(int rows, int k) { return (size_t)4 * rows * k; }
+size_t moe_mx_scale_bytes(int rows, int k) { return (size_t)8 * rows * moe_mx_stages(k); }
+size_t moe_mx_second_bytes(int rows, int k) { return 16 + (size_t)rows * moe_mx_stages(k); } // (read in words of four)
 
 bool moe_mx_supported(int n, int k, const void *blocks, const void *scales)
 {
@@ -377,7 +491,8 @@ bool moe_mx_supported(int n, int k, const void *blocks, const void *scales)
 }
 
 // Row r of the pieces is src[perm[r] / top_k] (perm null: src[r]), for the rows that total_rows[0] counts.
-int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, cudaStream_t st)
+int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, void *second,
+                 unsigned long long mark, cudaStream_t st)
 {
     cudaLaunchConfig_t cfg = {};
     const long long blocks = (long long)rows_cap * moe_mx_stages(k) * 16 / 256 + 1;
@@ -389,17 +504,18 @@ int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_r
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
     OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_split_kernel, (const __nv_bfloat16 *)src, perm, top_k, total_rows, k, moe_mx_stages(k), rows_cap,
-                                (unsigned char *)pieces, (unsigned char *)sfx));
+                                (unsigned char *)pieces, (unsigned char *)sfx, (unsigned char *)second + 8, (unsigned long long *)second, mark));
     return OXQ_OK;
 }
 
 // out = epilogue(rows . W_e^T + bias_e) for every token block of the table. epi 0: bias; epi 1: clamped SwiGLU.
-int moe_mx_grouped(const void *pieces, const void *sfx, int rows_cap, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
+int moe_mx_grouped(const void *pieces, const void *sfx, const void *second, unsigned long long mark, int rows_cap, const uint8_t *blocks, const uint8_t *scales, int experts, int n, int k,
                    const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype, void *out, int ldo, int epi, float limit,
                    int *flag, cudaStream_t st)
 {
     MoeMxParams p = {};
     p.entries = entries; p.n_blocks = n_blocks; p.scales = scales; p.sfx = (const uint32_t *)sfx; p.bias = bias; p.out = out; p.flag = flag;
+    p.pieces = (const unsigned char *)pieces; p.any = (const unsigned long long *)second; p.second = (const unsigned char *)second + 8; p.mark = mark;
     p.n = n; p.k = k; p.nkb = k / 32; p.stages = moe_mx_stages(k); p.rows_cap = rows_cap;
     p.scale_bytes = p.nkb % 4 == 0 && aligned(scales, 4) ? 4 : p.nkb % 2 == 0 && aligned(scales, 2) ? 2 : 1;
     p.tiles_n = (n + MM_ROWS - 1) / MM_ROWS;
@@ -416,7 +532,8 @@ int moe_mx_grouped(const void *pieces, const void *sfx, int rows_cap, const uint
     int device = 0;
     OXQ_CUDA(cudaGetDevice(&device));
     if (device >= 64 || configured[device] < MM_SMEM) {
-        OXQ_CUDA(cudaFuncSetAttribute(moe_mx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
+        OXQ_CUDA(cudaFuncSetAttribute(moe_mx_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
+        OXQ_CUDA(cudaFuncSetAttribute(moe_mx_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
         if (device < 64) configured[device] = MM_SMEM;
     }
     cudaLaunchConfig_t cfg = {};
@@ -428,7 +545,8 @@ int moe_mx_grouped(const void *pieces, const void *sfx, int rows_cap, const uint
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_kernel, p, wmap, xmap));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_kernel<false>, p, wmap, xmap));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_kernel<true>, p, wmap, xmap));
     return OXQ_OK;
 }
 
@@ -445,7 +563,7 @@ OXQ_EXPORT int oxq_selftest_moe_mx_wait_expiry(void *workspace, size_t workspace
     unsigned char *b = reinterpret_cast<unsigned char *>(workspace);
     cudaStream_t st = (cudaStream_t)stream;
     const int n = 128, k = 128, rows = 16, cap = 64;
-    // table | pieces [2, 64, 128] | their scales | blocks [128, 64] | scales [128, 4] | out [16, 128] bf16, 64 KB apart
+    // table, no second pairs | pieces [2, 2, 64, 128] | their scales | blocks [128, 64] | scales [128, 4] | out [16, 128] bf16, 64 KB apart
     int4 *entries = reinterpret_cast<int4 *>(b + 4096);
     int *n_blocks = reinterpret_cast<int *>(b + 4096 + 64);
     const int4 en = make_int4(0, rows, 0, 0);
@@ -454,7 +572,7 @@ OXQ_EXPORT int oxq_selftest_moe_mx_wait_expiry(void *workspace, size_t workspace
     OXQ_CUDA(cudaMemcpyAsync(n_blocks, &one, sizeof(one), cudaMemcpyHostToDevice, st));
     OXQ_CUDA(cudaStreamSynchronize(st)); // the two host words above live on this stack frame
     oxq::g_moe_mx_selftest_skip_loads = 1;
-    const int rc = oxq::moe_mx_grouped(b + (1 << 16), b + (2 << 16), cap, b + (3 << 16), b + (4 << 16), 1, n, k, entries, n_blocks, nullptr, 0,
+    const int rc = oxq::moe_mx_grouped(b + (1 << 16), b + (2 << 16), b + 8192, oxq::mx_call_mark(), cap, b + (3 << 16), b + (4 << 16), 1, n, k, entries, n_blocks, nullptr, 0,
                                        b + (5 << 16), n, 0, 0.0f, reinterpret_cast<int *>(workspace), st);
     oxq::g_moe_mx_selftest_skip_loads = 0;
     return rc;

@@ -176,28 +176,6 @@ __device__ __forceinline__ uint32_t mx_second_pair(const uint4 &raw, float (&v)[
     return sf - (uint32_t)up;
 }
 
-// Eight neighbouring values of a block whose largest magnitude has the bits `amax`: hi and lo as E4M3 bytes, and the block's
-// scale byte (lo's is four less).
-__device__ __forceinline__ uint32_t mx_split8(const float (&v)[8], uint32_t amax, uint2 &hi, uint2 &lo)
-{
-    const uint32_t e = amax >> 23; // biased exponent
-    const uint32_t sf = e < 11u ? 4u : e - 7u;
-    const float mul = __uint_as_float((254u - sf) << 23);
-    uint16_t h[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        float a = v[2 * i] * mul, b = v[2 * i + 1] * mul;
-        if (e == 255u) { a += a - a; b += b - b; } // infinite -> NaN (the conversion would saturate)
-        h[i] = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-        const __half2_raw back = __nv_cvt_fp8x2_to_halfraw2(h[i], __NV_E4M3);
-        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&back));
-        l[i] = __nv_cvt_float2_to_fp8x2(make_float2((a - f.x) * 16.0f, (b - f.y) * 16.0f), __NV_SATFINITE, __NV_E4M3);
-    }
-    hi = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
-    lo = make_uint2((uint32_t)l[0] | ((uint32_t)l[1] << 16), (uint32_t)l[2] | ((uint32_t)l[3] << 16));
-    return sf;
-}
-
 // A number that no other call of this process has had, in no order that a stale value would have by chance, 56 bits.
 inline unsigned long long mx_call_mark()
 {

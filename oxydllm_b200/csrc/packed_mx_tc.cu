@@ -557,8 +557,16 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
             float tot[NCH * 8];
 #pragma unroll
             for (int i = 0; i < NCH * 8; i++) tot[i] = 0.0f;
-            int more = 0; // units of the tile that come a second time
-            if (any) px_second_units(p, tile % p.token_blocks, from, to, [&](int, int) { more++; return true; });
+            int more = 0, again = 0; // units of the tile that come a second time; lane i has the i-th, i + 32-nd, ... of them, 32 at a time
+            auto list = [&](int skip) {
+                more = 0;
+                px_second_units(p, tile % p.token_blocks, from, to, [&](int u, int) {
+                    if (more >= skip && more < skip + 32 && more - skip == lane) again = u;
+                    more++;
+                    return true;
+                });
+            };
+            if (any) list(0);
             const int folds = (to - from) * unit_folds, row0 = from * PX_UNIT;
 #pragma unroll 1
             for (int f = 0; f < folds + more * unit_folds && ok; f++) {
@@ -566,12 +574,9 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
                 if (FP8 && srow) {
                     if (f + 1 < folds) s_next = __ldg(srow + (row0 + (f + 1) * p.fold_rows) / p.block_in);
                     else if (more) { // the unit of fold f + 1
-                        int nth = (f + 1 - folds) / unit_folds, row = 0;
-                        px_second_units(p, tile % p.token_blocks, from, to, [&](int u, int) {
-                            row = u * PX_UNIT + (f + 1) % unit_folds * p.fold_rows;
-                            return nth-- > 0;
-                        });
-                        s_next = __ldg(srow + row / p.block_in);
+                        const int nth = (f + 1 - folds) / unit_folds, part = (f + 1 - folds) % unit_folds;
+                        if (nth && nth % 32 == 0 && part == 0 && nth < more) list(nth);
+                        s_next = __ldg(srow + (__shfl_sync(0xFFFFFFFFu, again, nth & 31) * PX_UNIT + part * p.fold_rows) / p.block_in);
                     }
                 }
                 if (FP8) ok = mx_wait(accfull + 8 * a, aph, p.flag, PX_CODE + 4);

@@ -294,9 +294,15 @@ def test_gptq_outliers_and_infinities(cuda, k, n, g, sym, special):
 
 
 # ------------------------------------------------------------------------------------------------------- MXFP4 experts, small batches
-def experts_layer(experts, hidden, inter, seed):
+def experts_layer(experts, hidden, inter, seed, zero_columns=()):
+    """A layer and its arrays; in `zero_columns` every other gate and up row of each expert is zero."""
     from oxydllm_b200 import moe
     d = synth.gptoss_moe(experts, hidden, inter, 1, seed=seed)
+    d["gu_blocks"] = np.array(d["gu_blocks"])
+    gu = d["gu_blocks"].reshape(experts, 2 * inter, hidden // 2)
+    for c in zero_columns:
+        gu[:, 2::4, c // 2] &= 0xF0 if c % 2 == 0 else 0x0F
+        gu[:, 3::4, c // 2] &= 0xF0 if c % 2 == 0 else 0x0F
     t = lambda a, dt=None: torch.from_numpy(np.ascontiguousarray(a)).to(dt or torch.uint8).cuda()  # noqa: E731
     layer = moe.GptOssMoe(t(d["gu_blocks"]), t(d["gu_scales"]), t(d["gu_bias"], torch.bfloat16), t(d["dn_blocks"]), t(d["dn_scales"]),
                           t(d["dn_bias"], torch.bfloat16), hidden=hidden, inter=inter, top_k=4)
@@ -325,6 +331,40 @@ def test_moe_small_batch_matches_64_bit_experts(cuda, hidden, inter, counts):
         ref = h @ dn.T + db[e]
         # h is rounded to bf16 (2^-9 of each), as is the result; sums and the activation are good to some 2^-17
         assert (np.abs(got[rows] - ref) <= 2.0**-8 * (np.abs(h) @ np.abs(dn).T + np.abs(ref)) + 1e-6).all(), (e, c)
+
+
+# outliers beside zero weights, infinities and NaN in some rows: stages that come a second time, one stage, several, a last one that is
+# short; token blocks with and without them in a CTA's units
+@pytest.mark.parametrize("hidden,inter", [(96, 32), (160, 224), (2880, 64), (512, 1600)])
+@pytest.mark.parametrize("special", [False, True])
+def test_moe_small_batch_outliers_and_infinities(cuda, hidden, inter, special):
+    counts = (50, 0, 33, 17)
+    x, columns = (special_activations if special else activations_with_outliers)(sum(counts), hidden, seed=hidden)
+    if special:
+        rest, columns = columns, activations_with_outliers(1, hidden, 0)[1]
+    layer, d = experts_layer(len(counts), hidden, inter, seed=hidden + inter, zero_columns=columns)
+    ids = np.random.default_rng(1).permutation(np.repeat(np.arange(len(counts)), counts))
+    y = layer.forward_experts(bf16(x), torch.from_numpy(ids).cuda())
+    layer.check()
+    got = y.double().cpu().numpy()
+    gb, db = (b.double().cpu().numpy() for b in (layer.gu_bias, layer.dn_bias))
+    for e, c in enumerate(counts):
+        rows = np.nonzero(ids == e)[0]
+        gu = oracle.mxfp4_dequant(d["gu_blocks"][e], d["gu_scales"][e], 2 * inter, hidden).astype(np.float64)
+        dn = oracle.mxfp4_dequant(d["dn_blocks"][e], d["dn_scales"][e], hidden, inter).astype(np.float64)
+        with np.errstate(invalid="ignore", over="ignore"):
+            a = np.stack([(x[r].astype(np.float64) * gu).sum(1) for r in rows]).reshape(len(rows), -1) + gb[e] if c else np.zeros((0, 2 * inter))
+            gate, up = np.fmin(a[:, 0::2], 7.0), np.fmin(np.fmax(a[:, 1::2], -7.0), 7.0)  # a NaN takes the limit
+            h = (up + 1) * gate / (1 + np.exp(-1.702 * gate))
+            ref = h @ dn.T + db[e]
+            # gate and up are good to 2^-17 of the sum of |x w|, their product moves by less than 16 times that
+            off = 16 * 2.0**-17 * np.minimum(np.abs(x[rows]).astype(np.float64) @ np.abs(gu).T, 1e30).reshape(len(rows), inter, 2).sum(-1)
+            bound = 2.0**-8 * (np.abs(h) @ np.abs(dn).T + np.abs(ref)) + off @ np.abs(dn).T + 1e-6
+        assert np.array_equal(np.isnan(got[rows]), np.isnan(ref)), e
+        ok = np.isfinite(ref) & np.isfinite(bound)
+        assert (np.abs(got[rows] - ref)[ok] <= bound[ok]).all(), (e, c)
+        if not special:
+            assert ok.all()
 
 
 # more than 44 rows an expert on average: weights unpacked into tensor memory by four teams in turn, accumulators round a ring of columns;

@@ -149,6 +149,49 @@ OXQ_EXPORT size_t oxq_gemm_workspace_bytes(int n, int k)
     return WS_HEADER + (size_t)slab_rows(n, k) * k * 2;
 }
 
+// What the code of a bounded wait stands for. Waits that are polled together report one code.
+static const char *wait_name(int code)
+{
+    switch (code) {
+    case 1: return "ring slot";
+    case 2: return "tile data";
+    case 3: return "accumulator ready, or packed weights";
+    case 4: return "accumulator free or ready";
+    case 5: return "meeting of the fold warps, or activation slot";
+    case 7: return "operand slot";
+    case 8: return "accumulator free";
+    // grouped 4-bit kernel
+    case 21: return "ring slot, or slot for scales";
+    case 22: return "operand tile, x, or accumulator free";
+    case 23: return "packed words";
+    case 24: return "scales, or accumulator ready";
+    case 25: return "x slot";
+    case 27: return "operand slot";
+    case 28: return "slot for scales";
+    case 29: return "accumulator free";
+    case 31: return "last MMAs";
+    // block-scaled kernel of FP8 and GPTQ layers
+    case 41: return "weight slot";
+    case 42: return "operands, x, or accumulator free";
+    case 43: return "packed words";
+    case 44: return "scales, or accumulator ready";
+    case 45: return "x slot";
+    case 47: return "operand slot";
+    case 48: return "slot for scales";
+    case 49: return "accumulator free";
+    case 51: return "last MMAs";
+    // block-scaled kernel of experts
+    case 61: return "weight slot";
+    case 62: return "row slot";
+    case 63: return "accumulator free";
+    case 64: return "operands, or accumulator ready";
+    case 65: return "packed words";
+    case 66: return "operand slot";
+    case 67: return "last MMAs";
+    default: return "not one of a kernel's";
+    }
+}
+
 OXQ_EXPORT int oxq_gemm_check(const void *workspace, void *stream)
 {
     clear_error();
@@ -160,14 +203,8 @@ OXQ_EXPORT int oxq_gemm_check(const void *workspace, void *stream)
         OXQ_CUDA(cudaMemsetAsync(const_cast<void *>(workspace), 0, WS_HEADER, (cudaStream_t)stream)); // flag and split-k tickets
         OXQ_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     }
-    OXQ_REQUIRE(flag == 0, OXQ_ERR_DEVICE_FLAG,
-                "tensor-core kernel: bounded wait %d ran out (1 = ring slot, 2 = tile data, 3 = accumulator ready, "
-                "4 = accumulator free, 5 = meeting of the fold warps; grouped 4-bit kernel: 21 = ring slot, 22 = operand tile, "
-                "23 = packed words, 24 = accumulator ready, 25 = x slot, 26 = x, 27 = operand slot, 28 = slot for scales, "
-                "29 = accumulator free, 30 = scales, 31 = last MMAs; block-scaled kernels: 41 = weight slot, 42 = operands or accumulator free, "
-                "43 = packed words, 44 = accumulator ready, 45 = x slot, 47 = operand slot, 49 = accumulator free, 51 = last MMAs, of the "
-                "experts: 61 = weight slot, 62 = row slot, 63 = accumulator free, 64 = operands or accumulator ready, 65 = packed words, "
-                "66 = operand slot, 67 = last MMAs) in a call since the last check", flag);
+    OXQ_REQUIRE(flag == 0, OXQ_ERR_DEVICE_FLAG, "tensor-core kernel: bounded wait %d ran out (%d = %s) in a call since the last check", flag, flag,
+                wait_name(flag));
     return OXQ_OK;
 }
 

@@ -297,8 +297,9 @@ int oxq_fp8_gemm(const void *x, int x_dtype, const uint8_t *weight, const float 
                  const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, void *workspace,
                  size_t workspace_bytes, void *stream);
 
-/* The kernel that oxq_fp8_gemm runs on medium batches, E4M3 weights as tensor-core operands and nothing rounded before the f32 sums, with
- * scratch of its own: oxq_fp8_scratch_bytes(m, k, n, s_out, s_in) bytes (0: not this shape) with any contents, 256-byte aligned, one
+/* The kernel that oxq_fp8_gemm runs on medium batches, E4M3 weights as tensor-core operands, with scratch of its own. Weights and scales
+ * are not rounded. Activations are exact down to 2^-13 of the largest in their block of 32 columns; smaller ones are off by at most
+ * 2^-21 of it where half of the block is above 2^-9 of it, and exact down to 2^-26 elsewhere. Scratch: oxq_fp8_scratch_bytes(m, k, n, s_out, s_in) bytes (0: not this shape) with any contents, 256-byte aligned, one
  * per call in flight. s_out, s_in: 0 without scales. flag_word as for oxq_packed4_matmul. OXQ_ERR_UNSUPPORTED for shapes that the
  * kernel does not take. */
 size_t oxq_fp8_scratch_bytes(int m, int k, int n, int s_out, int s_in);

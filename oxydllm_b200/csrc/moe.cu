@@ -42,13 +42,18 @@ constexpr int MOE_MAX_TOPK = 8;
 constexpr int MOE_DECODE_MAX_PAIRS = 64;
 // From more pairs than this one of the grouped kernels takes over, which read every expert that has rows once. By time alone it would be
 // 8: us a layer, GEMVs / block-scaled kernel, 32 experts of 2880 x 2880 at 1, 2, 3, 4, 8, 12 tokens (4 pairs each) 43 / 48, 66 / 67,
-// 87 / 76, 107 / 81, 190 / 107, 268 / 124. But the GEMVs keep gate and up in f32 up to the down projection, and a token's result there
-// is the same bits alone and in a batch.
+// 87 / 76, 107 / 81, 190 / 107, 268 / 124 (with two operand teams; three, and a second instance for outliers, have come since). But a token
+// has to get the same bits alone and in a batch of decoded sequences, and alone the GEMVs are the faster ones. Both kernels round the
+// activated product once, to bf16.
 constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
 // Rows per expert, on average, up to which the block-scaled kernel is the better one: above, most experts take two of its blocks of 48
 // rows, and the kernel that unpacks once for up to 192 or 256 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
 // 300, 384, 450 tokens: 124 / 183, 149 / 221, 169 / 228, 186 / 235, 237 / 240, 277 / 245; 16 of 2048 x 1024 at 30, 120, 200: 43 / 64,
-// 49 / 67, 70 / 70. Both have come down by about a tenth since (340 tokens 170 here, 400 tokens 204 there).
+// 49 / 67, 70 / 70. Both have come down by about a tenth since (340 tokens 173 here, 400 tokens 197 there). That is for pairs spread evenly.
+// The average is all that the host knows; other routings, this / that as it was with blocks of 256 rows: one expert in half of the tokens, 50,
+// 200, 340 tokens 135 / 215, 157 / 222, 177 / 235; two experts in all of them, 340 tokens 203 / 256; popularity falling as 1 / rank^1.2, 340
+// tokens 217 / 246; the same four experts for all, 50, 100, 200, 340 tokens 64 / 70, 78 / 78, 113 / 93, 155 / 121: only the last one loses,
+// from about 100 rows an expert with nothing beside them.
 constexpr int MOE_MX_ROWS = 44;
 constexpr int MOE_BLOCK_ROWS = 192; // of a token block of the kernel that unpacks, but for one per expert that may be larger
 

@@ -16,7 +16,8 @@
 //   warps 16..19  epilogue of the previous unit while the next one accumulates: bias, clamped SwiGLU (even row gate, odd row up).
 //
 // What bounds it: a stage's chain of polls, operand rows and arrival in a team. us a layer at 13 / 50 / 200 / 340 tokens, 32 experts of
-// 2880 x 2880, with two teams 122 / 148 / 167 / 194, with three 108 / 130 / 144 / 170; packed weights alone take 66 from HBM.
+// 2880 x 2880, with two teams 122 / 148 / 167 / 194, with three 108 / 130 / 144 / 170, with what outliers need 119 / 131 / 146 / 173; packed
+// weights alone take 66 from HBM. With an outlier in every block of 32 columns 50 tokens take 183.
 #include "mx_common.cuh"
 
 namespace oxq {

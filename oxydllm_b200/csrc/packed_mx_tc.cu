@@ -2,16 +2,17 @@
 //
 // Read as E4M3 a byte 0..16 is that integer times 2^-9 (subnormals and the first binade are evenly spaced), with a sign bit its negative,
 // so q - z of 4-bit weights is one byte, looked up in a table of 16 that each out feature has per group; the operand takes half the
-// shared memory of a bf16 one. E4M3 weights are not touched at all. Activations are two E4M3 pieces (mx_common.cuh); a small kernel in
-// front writes them with their block scales. A group's product leaves tensor memory once and meets the group's scale in f32:
+// shared memory of a bf16 one. E4M3 weights are not touched at all. Activations are two E4M3 pieces (mx_common.cuh says how exact); a
+// small kernel in front writes them with their block scales. Units in which tokens have outliers, infinities or NaN come a second time,
+// with a second pair of pieces (64 tokens on 4096 x 14336 20 us, 21 with an outlier in one column, 49 with one in every 32). A group's product leaves tensor memory once and meets the group's scale in f32:
 //   y[t, n] = sum over groups of s[g, n] * (sum over the group's k of (q[k, n] - z[g, n]) x[t, k]).
 // Nothing is rounded between the packed weight and the f32 total. (With codes 0..15 as operands and z times the sum of x taken off
 // afterwards a weight of zero beside a large x left the rounding of two large f32 numbers behind.)
 //
 // One CTA per SM walks an equal share of all (tile, unit) pairs (a tile is 128 out features x at most 128 tokens, a unit 128 input
 // rows), so every SM works for the whole launch whatever the number of tiles; the pipeline runs on across tile borders. Roles:
-//   warp 0        TMA: units of weights (8 KB of packed words with their zero points, or 16 KB of E4M3), as far ahead as the ring allows: this is what is in
-//                 flight from HBM;
+//   warp 0        TMA: units of weights (8 KB of packed words with their zero points, or 16 KB of E4M3), as far ahead as the ring
+//                 allows: this is what is in flight from HBM;
 //   warps 1, 3    tcgen05.mma kind::mxf8f6f4 on alternate units, weights [128 x 32] times both pieces of x, and the copies of x's
 //                 block scales to tensor memory;
 //   warp 2        TMA: the unit's pieces of x ([tokens, 128] bytes each, 128-byte swizzle) with their block scales;
@@ -715,7 +716,7 @@ __global__ void __launch_bounds__(PX_THREADS<WT, PARTS>, 1)
 
 // True when this kernel serves a GPTQ call and is the better one: its unpack is cheaper than that of csrc/group_tc.cu, but the kernel that
 // writes x's pieces costs a launch, so the layer has to be large, and the groups at least a unit. us here / there at 6 tokens: 4096 x
-// 14336 17.1 / 20.4, 14336 x 4096 19.7 / 22.0, 6144 x 8192 17.0 / 18.7; at 16 17.9 / 20.5, 20.7 / 22.2; with two unpack teams and codes
+// 14336 19.0 / 20.4, 14336 x 4096 21.2 / 22.0; at 16 19.6 / 20.5, 22.2 / 22.2 (17.2, 19.5, 17.9, 20.7 here without second pairs); with two unpack teams and codes
 // 0..15 as operands 4096 x 6144 at 16 tokens took 14.1 / 12.7, 2048 x 4096 10.8 / 10.3, 4096 x 14336 at 32 20.7 / 21.7, 14336 x 4096 24.2 / 23.2.
 bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
                          const void *scales)
@@ -726,8 +727,8 @@ bool packed_mx_supported(int m, int k, int n, int group_size, int scales_dtype, 
 }
 
 // Largest batch of E4M3 weights for this kernel, above it the dense copy of the weight and the GEMM on it are the better tool, us
-// here / there: 14336 x 4096 at 400 tokens 65 / 81, 600 79 / 104, 800 114 / 118, 1024 129 / 122; 4096 x 4096 at 256 22 / 35, 400
-// 25 / 30, 600 36 / 35.
+// here / there: 14336 x 4096 at 400 tokens 65 / 81, 600 79 / 104, 700 95 / 110, 800 114 / 118, 1024 129 / 122; 4096 x 4096 at 256 22 / 35,
+// 400 24 / 30, 600 36 / 35.
 static int fp8_mx_max_m(int n) { return n >= 8192 ? 768 : 512; }
 bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv)
 {

@@ -133,6 +133,15 @@ int oxq_gguf_dequant(int ggml_type, const void *blocks, void *w_out, int out_dty
 int oxq_gguf_gemv(int ggml_type, const void *x, int x_dtype, const void *blocks, const void *bias, int bias_dtype,
                   void *y, int y_dtype, int m, int k, int n, void *stream);
 
+/* The same matmul for Q4_0, Q8_0, Q4_K and Q6_K blocks and x from one token to several hundred, without a dense copy: blocks are streamed
+ * through mma.sync, integers times exact bf16 activations, scales in f32. oxq_gguf_scratch_bytes(type, m, k, n) is 0 where it does not
+ * serve a call (in_features a multiple of 256, 2048 for Q6_K; even out_features; m <= 512; x and blocks on 16 bytes) or other entries
+ * are the better ones; else the size of the scratch, any contents, 256-byte aligned, one per call in flight. flag_word as for
+ * oxq_packed4_matmul. Weights are taken in the order of the stream. No counterpart in the reference. */
+size_t oxq_gguf_scratch_bytes(int ggml_type, int m, int k, int n);
+int oxq_gguf_matmul(int ggml_type, const void *x, int x_dtype, const void *blocks, const void *bias, int bias_dtype, void *y,
+                    int y_dtype, int m, int k, int n, void *flag_word, void *scratch, size_t scratch_bytes, void *stream);
+
 /* ------------------------------------------------------------------- FP8
  * weight = E4M3fn bytes [n, k]; scale_inv f32 grid [s_out, s_in] tiling the
  * weight evenly (128x128 blocks: s_out = n/128, s_in = k/128; per-row: s_in = 1;

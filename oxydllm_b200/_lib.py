@@ -33,6 +33,8 @@ SIGNATURES = {
     "oxq_gptq_dequant": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp],
     "oxq_gguf_dequant": [_i, _vp, _vp, _i, _i, _i, _vp],
     "oxq_gguf_gemv": [_i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp],
+    "oxq_gguf_scratch_bytes": [_i, _i, _i, _i],
+    "oxq_gguf_matmul": [_i, _vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _i, _vp, _vp, _sz, _vp],
     "oxq_fp8_dequant": [_vp, _vp, _i, _i, _vp, _i, _i, _i, _vp],
     "oxq_fp8_gemv": [_vp, _i, _vp, _vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _vp],
     "oxq_mxfp4_dequant": [_vp, _vp, _vp, _i, _i, _i, _vp],
@@ -77,7 +79,7 @@ SIGNATURES = {
     "oxq_awq_gemm_noalloc_check": [_vp],
 }
 _RESTYPE = {"oxq_status_string": ctypes.c_char_p, "oxq_last_error": ctypes.c_char_p,
-            "oxq_gemm_workspace_bytes": ctypes.c_size_t, "oxq_packed4_scratch_bytes": ctypes.c_size_t, "oxq_packed4_full_scratch_bytes": ctypes.c_size_t, "oxq_fp8_scratch_bytes": ctypes.c_size_t, "oxq_decode_workspace_bytes": ctypes.c_size_t, "oxq_gptoss_moe_workspace_bytes": ctypes.c_size_t, "oxq_awq_gemm_noalloc_max_k": ctypes.c_size_t}
+            "oxq_gemm_workspace_bytes": ctypes.c_size_t, "oxq_packed4_scratch_bytes": ctypes.c_size_t, "oxq_packed4_full_scratch_bytes": ctypes.c_size_t, "oxq_fp8_scratch_bytes": ctypes.c_size_t, "oxq_gguf_scratch_bytes": ctypes.c_size_t, "oxq_decode_workspace_bytes": ctypes.c_size_t, "oxq_gptoss_moe_workspace_bytes": ctypes.c_size_t, "oxq_awq_gemm_noalloc_max_k": ctypes.c_size_t}
 
 _lib = None
 

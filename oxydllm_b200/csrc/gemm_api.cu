@@ -188,6 +188,10 @@ static const char *wait_name(int code)
     case 65: return "packed words";
     case 66: return "operand slot";
     case 67: return "last MMAs";
+    // GGUF stream kernel
+    case 81: return "ring slot";
+    case 82: return "blocks, x, or unpacked scales";
+    case 83: return "blocks";
     default: return "not one of a kernel's";
     }
 }

@@ -1,0 +1,261 @@
+// What the kernels that stream packed weights through mma.sync share: fragments, and how the CTAs that hold parts of an output
+// tile put it together.
+#pragma once
+
+#include "mx_common.cuh"
+
+namespace oxq {
+
+constexpr int ST_CODE = 80;           // wait codes 81 .. 83
+
+// D (+)= A B, m16n8k16, bf16 operands, f32 sums.
+__device__ __forceinline__ void st_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void st_mma_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) // D = A B
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+__device__ __forceinline__ void st_mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+__device__ __forceinline__ void st_mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void st_ldmatrix(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void st_ldmatrix_t(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// Loads from shared memory, plain ones: the compiler keeps them behind the wait ahead and is free to move them otherwise.
+template <typename T> __device__ __forceinline__ T st_lds(const unsigned char *p) { return *reinterpret_cast<const T *>(p); }
+__device__ __forceinline__ uint32_t st_and_or(uint32_t v, uint32_t mask, uint32_t magic) // (v & mask) | magic
+{
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(magic));
+    return r;
+}
+__device__ __forceinline__ uint32_t st_sub2(uint32_t a, uint32_t b) // bf16 pairs
+{
+    const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&a), *reinterpret_cast<const __nv_bfloat162 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&d);
+}
+
+__device__ __forceinline__ float2 st_f16x2(uint32_t two) { return __half22float2(*reinterpret_cast<const __half2 *>(&two)); }
+
+struct StreamOut {
+    const void *bias;
+    void *y;
+    int bias_dtype, y_dtype;
+    int m, n, ldy;               // n: out features of the weight
+    int tok_blocks, tok_step;    // tiles of the same out features, and their tokens: tile = feature tile * tok_blocks + token block
+    int gate;                    // columns 0 .. 127 of a tile are gates, 128 .. 255 their partners: y = act(gate) * up, 1 SiLU, 2 GeLU-tanh
+    int pairs;                   // two neighbouring outputs can be stored at once
+    int units_per_tile, total;   // units of k of a tile; of all tiles
+    int grain;                   // shares are whole multiples of this many units
+    float *partials;             // [CTA + tile][tok_step][out features of a tile] f32
+    unsigned long long *tickets; // per tile: this call's mark above, arrivals in the low byte
+    unsigned long long mark;
+};
+
+// Shares of the list of (tile, unit of k) pairs, unit fastest: the first unit of CTA i, and the CTA that holds unit u.
+__host__ __device__ __forceinline__ int st_share(const StreamOut &o, int ctas, int i) { return (int)((long long)(o.total / o.grain) * i / ctas) * o.grain; }
+__host__ __device__ __forceinline__ int st_owner(const StreamOut &o, int ctas, int u)
+{
+    return (int)((((long long)(u / o.grain) + 1) * ctas - 1) / (o.total / o.grain));
+}
+
+__device__ __forceinline__ float st_act(float g, float u, int act)
+{
+    if (act == 1) return g / (1.0f + __expf(-g)) * u;
+    const float t = tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g));
+    return 0.5f * g * (1.0f + t) * u;
+}
+
+__device__ __forceinline__ void st_store_pair(const StreamOut &o, size_t at, float a, float b)
+{
+    if (o.pairs) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+        *reinterpret_cast<__nv_bfloat162 *>(reinterpret_cast<__nv_bfloat16 *>(o.y) + at) = v;
+    } else {
+        store_as(o.y, o.y_dtype, at, a);
+        store_as(o.y, o.y_dtype, at + 1, b);
+    }
+}
+
+__device__ __forceinline__ int st_tokens(const StreamOut &o, int tile) { return min(o.tok_step, o.m - tile % o.tok_blocks * o.tok_step); }
+
+// Out features 2 i and 2 i + 1 of a tile of COLS (gate: those of the first half) for its token tok, from their sums. mend(sum, token, out
+// feature) may put something else in a sum's place.
+struct StKeep { __device__ __forceinline__ float operator()(float v, int, int) const { return v; } };
+template <int COLS, typename Mend>
+__device__ __forceinline__ void st_output(const StreamOut &o, Mend mend, int tile, int tok, int i, float2 v, float2 up)
+{
+    const int ft = tile / o.tok_blocks;
+    tok += tile % o.tok_blocks * o.tok_step;
+    if (o.gate) {
+        st_store_pair(o, (size_t)tok * o.ldy + ft * (COLS / 2) + 2 * i, st_act(v.x, up.x, o.gate), st_act(v.y, up.y, o.gate));
+        return;
+    }
+    const int col = ft * COLS + 2 * i;
+    if (col >= o.n) return;
+    v = make_float2(mend(v.x, tok, col), mend(v.y, tok, col + 1));
+    if (o.bias) {
+        v.x += load_as_f32(o.bias, o.bias_dtype, col);
+        v.y += load_as_f32(o.bias, o.bias_dtype, col + 1);
+    }
+    st_store_pair(o, (size_t)tok * o.ldy + col, v.x, v.y);
+}
+
+// What a CTA that is about to finish its last segment sees of the tile's ticket: read a while ahead, used in st_finish.
+__device__ __forceinline__ unsigned long long st_ticket(const StreamOut &o, int tile)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(__cvta_generic_to_global(o.tickets + tile)) : "memory");
+    return v;
+}
+
+// The sums of CTAs i_lo .. i_hi for token tok, columns 2 i and 2 i + 1 of a tile, in ascending k; that of CTA i_lo + me is `own`.
+template <int COLS>
+__device__ __forceinline__ float2 st_total(const StreamOut &o, int tile, int i_lo, int i_hi, int tok, int i, int me = -1, float2 own = make_float2(0.0f, 0.0f))
+{
+    const size_t pairs = (size_t)o.tok_step * (COLS / 2);
+    const float2 *src = reinterpret_cast<const float2 *>(o.partials) + (size_t)(i_lo + tile) * pairs + (size_t)tok * (COLS / 2) + i;
+    float2 s = make_float2(0.0f, 0.0f);
+    for (int q0 = 0; q0 <= i_hi - i_lo; q0 += 8) { // eight loads under way together
+        float2 v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            v[q] = make_float2(0.0f, 0.0f);
+            if (q0 + q <= i_hi - i_lo) v[q] = q0 + q == me ? own : __ldcg(src + (size_t)(q0 + q) * pairs);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++) { s.x += v[q].x; s.y += v[q].y; }
+    }
+    return s;
+}
+// One thread's arrival at a tile's ticket, for its CTA (whose sums a barrier has ordered before): whether it is the last of most + 1.
+__device__ __forceinline__ uint32_t st_arrive(const StreamOut &o, int tile, unsigned most)
+{
+    // The scratch area holds anything at first: a ticket without this call's mark counts as no arrival. The last one
+    // leaves the mark with a count of zero (a replayed graph comes back with the same mark).
+    unsigned long long *t = o.tickets + tile, old = *reinterpret_cast<volatile unsigned long long *>(t), seen;
+    unsigned count;
+    __threadfence(); // the sums before the ticket
+    for (;;) {
+        count = (old >> 8) == o.mark ? (unsigned)(old & 0xFFu) : 0u;
+        seen = atomicCAS(t, old, (o.mark << 8) | (count == most ? 0u : count + 1u));
+        if (seen == old) break; // fails only when another of the tile's CTAs came in between
+        old = seen;
+    }
+    __threadfence(); // the ticket before the others' sums
+    return count == most;
+}
+
+// End of this CTA's segment [u, seg_end) of a tile: `planes` partial tiles [token][PLANE] lie `stride` floats apart in `red`, all
+// THREADS threads that call this have written theirs. A whole tile goes to y; of a shared one every CTA leaves its sum in scratch, and the
+// CTA that arrives last adds the sums in ascending k: no CTA waits for another, and the result does not depend on the order of arrival.
+//
+// The four round trips to L2 that this takes (sums and ticket out, ticket and sums in) are about 3 us, a quarter of a whole call. A CTA whose
+// share goes on (final = false) leaves them to a helping warp (st_help). The first CTA of a tile, which comes to it last, mostly finds with
+// `ticket`, read before its last box, that all others have arrived: it takes their sums and its own from shared memory.
+// `last`: a shared word. `ok`: false after a wait gave up (nothing is stored, the flag word is set).
+template <int THREADS, int COLS, int PLANE, typename Mend>
+__device__ __forceinline__ void st_finish(const StreamOut &o, Mend mend, const float *red, int planes, int stride, int tile, int u, int seg_end, bool final,
+                                          unsigned long long ticket, bool ok, volatile uint32_t *last)
+{
+    const int et = threadIdx.x;
+    const int i_lo = st_owner(o, gridDim.x, tile * o.units_per_tile), i_hi = st_owner(o, gridDim.x, (tile + 1) * o.units_per_tile - 1);
+    const unsigned most = (unsigned)(i_hi - i_lo);
+    const bool whole = most == 0;
+    if (et == 0) *last = !whole && final && (ticket >> 8) == o.mark && (unsigned)(ticket & 0xFFu) == most;
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    auto own = [&](int tok, int i) {
+        float2 s = make_float2(0.0f, 0.0f);
+        for (int q = 0; q < planes; q++) {
+            const float2 v = *reinterpret_cast<const float2 *>(red + q * stride + tok * PLANE + 2 * i);
+            s.x += v.x;
+            s.y += v.y;
+        }
+        return s;
+    };
+    const int per = o.gate ? COLS / 4 : COLS / 2, tokens = st_tokens(o, tile); // results of a token, two at a time
+    if (whole) {
+        if (ok)
+            for (int x = et; x < tokens * per; x += THREADS) {
+                const int tok = x / per, i = x - tok * per;
+                st_output<COLS>(o, mend, tile, tok, i, own(tok, i), o.gate ? own(tok, i + COLS / 4) : make_float2(0.0f, 0.0f));
+            }
+        return;
+    }
+    const int me = (int)blockIdx.x - i_lo;
+    const bool early = *last; // all others' sums are there
+    auto total = [&](int tok, int i) { return early ? st_total<COLS>(o, tile, i_lo, i_hi, tok, i, me, own(tok, i)) : st_total<COLS>(o, tile, i_lo, i_hi, tok, i); };
+    auto outputs = [&](int first, int step) {
+        for (int x = first; x < tokens * per; x += step) {
+            const int tok = x / per, i = x - tok * per;
+            st_output<COLS>(o, mend, tile, tok, i, total(tok, i), o.gate ? total(tok, i + COLS / 4) : make_float2(0.0f, 0.0f));
+        }
+    };
+    if (early) {
+        if (et == 0) *reinterpret_cast<volatile unsigned long long *>(o.tickets + tile) = o.mark << 8; // as below
+        if (ok) outputs(et, THREADS);
+        return;
+    }
+    if (ok) {
+        float2 *part = reinterpret_cast<float2 *>(o.partials) + (size_t)(blockIdx.x + tile) * o.tok_step * (COLS / 2);
+        for (int x = et; x < tokens * (COLS / 2); x += THREADS) part[x] = own(x / (COLS / 2), x % (COLS / 2));
+    }
+    if (!final) { // st_help does the rest
+        asm volatile("bar.arrive 2, %0;" ::"n"(THREADS + 32) : "memory");
+        return;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    if (et == 0) *last = st_arrive(o, tile, most);
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    if (*last && ok) outputs(et, THREADS);
+}
+
+// The helping warp's part of a first segment that does not end the CTA's share: the ticket, while the others go on. Where it is the
+// tile's last, all THREADS threads put the tile together at the end (st_helped).
+template <int THREADS> __device__ __forceinline__ void st_help(const StreamOut &o, int tile, volatile uint32_t *helped)
+{
+    const int i_lo = st_owner(o, gridDim.x, tile * o.units_per_tile), i_hi = st_owner(o, gridDim.x, (tile + 1) * o.units_per_tile - 1);
+    asm volatile("bar.sync 2, %0;" ::"n"(THREADS + 32) : "memory");
+    if ((threadIdx.x & 31) == 0) *helped = st_arrive(o, tile, (unsigned)(i_hi - i_lo));
+    __syncwarp();
+    asm volatile("bar.arrive 3, %0;" ::"n"(THREADS + 32) : "memory");
+}
+template <int THREADS, int COLS, typename Mend>
+__device__ __forceinline__ void st_helped(const StreamOut &o, Mend mend, int tile, bool ok, volatile uint32_t *helped)
+{
+    asm volatile("bar.sync 3, %0;" ::"n"(THREADS + 32) : "memory");
+    if (!*helped || !ok) return;
+    const int i_lo = st_owner(o, gridDim.x, tile * o.units_per_tile), i_hi = st_owner(o, gridDim.x, (tile + 1) * o.units_per_tile - 1);
+    const int per = o.gate ? COLS / 4 : COLS / 2;
+    for (int x = threadIdx.x; x < st_tokens(o, tile) * per; x += THREADS) {
+        const int tok = x / per, i = x - tok * per;
+        st_output<COLS>(o, mend, tile, tok, i, st_total<COLS>(o, tile, i_lo, i_hi, tok, i),
+                        o.gate ? st_total<COLS>(o, tile, i_lo, i_hi, tok, i + COLS / 4) : make_float2(0.0f, 0.0f));
+    }
+}
+// Whether a CTA's first segment is one for the helping warp.
+__device__ __forceinline__ bool st_needs_help(const StreamOut &o, int u0, int u1) { return u0 % o.units_per_tile != 0 && (u0 / o.units_per_tile + 1) * o.units_per_tile < u1; }
+
+} // namespace oxq

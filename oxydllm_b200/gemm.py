@@ -181,6 +181,25 @@ def gguf_matmul(lin, x2, y):
               x2.shape[0], lin.in_features, lin.out_features, _p(ws), ws.numel(), _st())
 
 
+def gguf_stream_matmul(lin, x2, y) -> bool:
+    """``y = x2 . deq(W)^T (+ bias)`` by the stream kernel (``oxq_gguf_matmul``) with scratch of the call's own; False where another
+    kernel is the better one."""
+    m = x2.shape[0]
+    need = lin._scratch_bytes.get(m)
+    if need is None:
+        need = lin._scratch_bytes[m] = int(_lib.entry("oxq_gguf_scratch_bytes")(lin.ggml_type, m, lin.in_features, lin.out_features))
+    if not need:
+        return False
+    flag = _flags.get(x2.device.index)
+    if flag is None:
+        flag = _flag_words(x2.device)
+    scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
+    bp, bd = _bias(lin.bias)
+    _lib.call("oxq_gguf_matmul", lin.ggml_type, x2.data_ptr(), _dt(x2.dtype), lin.blocks.data_ptr(), bp, bd, y.data_ptr(), _dt(y.dtype),
+              m, lin.in_features, lin.out_features, flag.data_ptr(), scratch.data_ptr(), need, _st())
+    return True
+
+
 def mxfp4_matmul(lin, x2, y):
     ws = workspace(lin.out_features, lin.in_features, x2.device)
     bp, bd = _bias(lin.bias)

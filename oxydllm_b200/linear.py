@@ -498,6 +498,7 @@ class QLinear:
         self.out_features, self.in_features = out_features, in_features
         self.bias = None if bias is None else bias.contiguous()
         self.out_dtype = out_dtype
+        self._scratch_bytes: dict = {}  # of the stream kernel, by batch; 0 where it does not serve the call
 
     from_blocks = classmethod(lambda cls, *a, **k: cls(*a, **k))
 
@@ -512,7 +513,9 @@ class QLinear:
         x2, lead, m = _flatten_x(x, self.in_features, "QLinear")
         _require_cuda(x2, self.blocks, self.bias)
         y = x2.new_empty((m, self.out_features), dtype=self.out_dtype)
-        if m and m <= GEMV_MAX_M:
+        if m and x2.dtype == torch.bfloat16 and not (x2.data_ptr() | self.blocks.data_ptr()) & 15 and gemm.gguf_stream_matmul(self, x2, y):
+            pass
+        elif m and m <= GEMV_MAX_M:
             b = self.bias
             _lib.call("oxq_gguf_gemv", self.ggml_type, x2.data_ptr(), _dt(x2.dtype), self.blocks.data_ptr(), _p(b),
                       _dt(b.dtype) if b is not None else 0, y.data_ptr(), _dt(self.out_dtype), m, self.in_features,

@@ -4,7 +4,7 @@
 //   [dequantize -> grouped GEMM (down)]* -> weighted combine in ascending expert order.
 // Mirrors MoeFeedForward::forward + dispatch_sparse + MoeExpert::GptOss (moe.rs:466-499,
 // 563-607, 152-173); every reduction has a fixed order, so results are run-to-run identical.
-#include "mx_common.cuh"
+#include "moe_mx_split.cuh"
 
 namespace oxq {
 
@@ -25,27 +25,14 @@ size_t moe_mx_piece_bytes(int rows, int k);
 size_t moe_mx_scale_bytes(int rows, int k);
 size_t moe_mx_second_bytes(int rows, int k);
 bool moe_mx_supported(int n, int k, const void *blocks, const void *scales);
-int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, void *second,
+int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int most, int k, int rows_cap, void *pieces, void *sfx, void *second,
                  unsigned long long mark, cudaStream_t st);
 int moe_mx_grouped(const void *pieces, const void *sfx, const void *second, unsigned long long mark, int rows_cap, const uint8_t *blocks,
                    const uint8_t *scales, int experts, int n, int k, const int4 *entries, const int *n_blocks, const void *bias, int bias_dtype,
                    void *out, int ldo, int epi, float limit, int *flag, cudaStream_t st);
-bool mxfp4_gemv_batched_supported(int k, const void *blocks);
-int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const uint8_t *scales, const void *bias,
-                       int bias_dtype, const int *pair_expert, int pairs, int e_lo, int e_hi, void *y, int y_dtype, int k,
-                       int n, cudaStream_t st, const float *gu = nullptr, float limit = 0.0f);
 
 constexpr int MOE_MAX_EXPERTS = 256;
 constexpr int MOE_MAX_TOPK = 8;
-// Up to this many (token, slot) pairs the layer can run as batched single-token GEMVs on the packed
-// weights of the selected experts only (decode); above, it dequantizes expert groups for the grouped GEMM.
-constexpr int MOE_DECODE_MAX_PAIRS = 64;
-// From more pairs than this one of the grouped kernels takes over, which read every expert that has rows once. By time alone it would be
-// 8: us a layer, GEMVs / block-scaled kernel, 32 experts of 2880 x 2880 at 1, 2, 3, 4, 8, 12 tokens (4 pairs each) 43 / 48, 66 / 67,
-// 87 / 76, 107 / 81, 190 / 107, 268 / 124 (with two operand teams; three, and a second instance for outliers, have come since). But a token
-// has to get the same bits alone and in a batch of decoded sequences, and alone the GEMVs are the faster ones. Both kernels round the
-// activated product once, to bf16.
-constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
 // Rows per expert, on average, up to which the block-scaled kernel is the better one: above, most experts take two of its blocks of 48
 // rows, and the kernel that unpacks once for up to 192 or 256 is faster. us a layer, this / that, 32 experts of 2880 x 2880 at 13, 50, 200,
 // 300, 384, 450 tokens: 124 / 183, 149 / 221, 169 / 228, 186 / 235, 237 / 240, 277 / 245; 16 of 2048 x 1024 at 30, 120, 200: 43 / 64,
@@ -57,22 +44,19 @@ constexpr int MOE_DECODE_FUSED_FROM_PAIRS = 48;
 constexpr int MOE_MX_ROWS = 44;
 constexpr int MOE_BLOCK_ROWS = 192; // of a token block of the kernel that unpacks, but for one per expert that may be larger
 
-// One warp per token: f32 softmax over all experts, k rounds of arg-max (ties: lower index),
-// optional renormalisation by the sum of the selected probabilities (moe.rs:472-487).
-__global__ void __launch_bounds__(256)
-moe_route_kernel(const void *logits, int dtype, int tokens, int experts, int top_k, int norm_topk, int *top_idx, float *top_w)
+// One warp: f32 softmax over all experts of a token, k rounds of arg-max (ties: lower index) (moe.rs:472-487); PER: experts a
+// lane; denom: the sum of the selected probabilities.
+template <int PER>
+__device__ __forceinline__ void moe_route_token(const void *logits, int dtype, int token, int experts, int top_k, int (&picked_e)[MOE_MAX_TOPK],
+                                                float (&picked_w)[MOE_MAX_TOPK], float &denom)
 {
-    pdl_wait(); // the logits are the kernel ahead's, and what is written may still be read
-    pdl_launch_dependents();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= tokens) return;
-    constexpr int PER = MOE_MAX_EXPERTS / 32;
+    const int lane = threadIdx.x & 31;
     float v[PER];
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < PER; i++) {
         const int e = lane + 32 * i;
-        v[i] = e < experts ? load_as_f32(logits, dtype, (size_t)warp * experts + e) : -INFINITY;
+        v[i] = e < experts ? load_as_f32(logits, dtype, (size_t)token * experts + e) : -INFINITY;
         mx = fmaxf(mx, v[i]);
     }
 #pragma unroll
@@ -89,9 +73,18 @@ moe_route_kernel(const void *logits, int dtype, int tokens, int experts, int top
 #pragma unroll
     for (int i = 0; i < PER; i++) v[i] = (lane + 32 * i) < experts ? v[i] / sum : -1.0f;
 
-    float denom = 0.0f, picked_w[MOE_MAX_TOPK];
-    int picked_e[MOE_MAX_TOPK];
+    denom = 0.0f;
     for (int s = 0; s < top_k; s++) {
+        if (PER == 1) { // probabilities order as their bits do; 0 stands for taken ones, and NaN
+            const uint32_t key = v[0] >= 0.0f ? __float_as_uint(v[0]) + 1u : 0u, most = __reduce_max_sync(0xFFFFFFFFu, key);
+            if (most) {
+                picked_e[s] = __ffs(__ballot_sync(0xFFFFFFFFu, key == most)) - 1;
+                picked_w[s] = __uint_as_float(most - 1u);
+                denom += picked_w[s];
+                if (picked_e[s] == lane) v[0] = -1.0f;
+                continue;
+            }
+        }
         float best = -2.0f;
         int best_e = 0x7FFFFFFF;
 #pragma unroll
@@ -114,6 +107,20 @@ moe_route_kernel(const void *logits, int dtype, int tokens, int experts, int top
                 if (lane + 32 * i == best_e) v[i] = -1.0f; // taken
         }
     }
+}
+
+// One warp per token; optional renormalisation by the sum of the selected probabilities.
+template <int PER>
+__global__ void __launch_bounds__(256)
+moe_route_kernel(const void *logits, int dtype, int tokens, int experts, int top_k, int norm_topk, int *top_idx, float *top_w)
+{
+    pdl_wait(); // the logits are the kernel ahead's, and what is written may still be read
+    pdl_launch_dependents();
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (warp >= tokens) return;
+    int picked_e[MOE_MAX_TOPK];
+    float picked_w[MOE_MAX_TOPK], denom;
+    moe_route_token<PER>(logits, dtype, warp, experts, top_k, picked_e, picked_w, denom);
     if (lane == 0)
         for (int s = 0; s < top_k; s++) {
             top_idx[(size_t)warp * top_k + s] = picked_e[s];
@@ -266,6 +273,70 @@ moe_dispatch_small_kernel(const int *top_idx, int pairs, int e_lo, int n_exp, in
             perm[pos] = pair;
             inv[pair] = pos;
         }
+}
+
+// All that comes in front of the block-scaled expert kernel for a batch of up to MOE_FRONT_PAIRS pairs in one launch: routing, positions
+// by expert, the table of token blocks and the pieces of x. Every CTA routes all tokens for itself and writes its share of the pieces, the last one the
+// tables. Bounded by that chain of latencies, about 5 us. us a layer in a graph, 32 experts of 2880 x 2880 at 1 / 2 / 8 tokens: 41.3 / 56.4 / 94 (in three
+// launches 44 / 59 / 96; with the loops of the router over 256 experts 44.9 / 59.8 / 96.9). Batches of up to 48 pairs were single-token GEMVs before, one a pair:
+// 42.2 / 64 / 188, 12 tokens 267 against 110; 16 of 2048 x 1024, one token, 26.9 against 27.9. A token has the same bits alone and in a batch.
+constexpr int MOE_FRONT_PAIRS = 64;
+constexpr int MOE_SMALL_MAX_K = 81912; // wider layers keep the dense fallback for blocks off 16 bytes
+struct MoeFrontParams {
+    const void *logits;
+    const int *given; // not null: rows that already carry their expert, weight one
+    const __nv_bfloat16 *x;
+    int logits_dtype, tokens, experts, top_k, norm_topk, e_lo, n_exp, max_rows;
+    int *top_idx, *offsets, *n_blocks, *inv;
+    float *top_w;
+    int4 *entries;
+    MoeMxPieces pieces;
+};
+__global__ void __launch_bounds__(MOE_MAX_EXPERTS)
+moe_front_kernel(const MoeFrontParams p)
+{
+    __shared__ int ids[MOE_FRONT_PAIRS], perm[MOE_FRONT_PAIRS], scratch[64];
+    pdl_wait();
+    pdl_launch_dependents(); // the expert kernel behind reads weights ahead of its own wait: whatever wrote them has finished
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pairs = p.tokens * p.top_k;
+    const bool tables = blockIdx.x + 1 == gridDim.x; // the last CTA writes these, the others the pieces
+    if (p.given) {
+        if (tid < pairs) {
+            ids[tid] = ld_produced(p.given + tid);
+            if (tables) p.top_idx[tid] = ids[tid], p.top_w[tid] = 1.0f;
+        }
+    } else {
+        for (int t = warp; t < p.tokens; t += MOE_MAX_EXPERTS / 32) {
+            int picked_e[MOE_MAX_TOPK];
+            float picked_w[MOE_MAX_TOPK], denom;
+            if (p.experts <= 32) moe_route_token<1>(p.logits, p.logits_dtype, t, p.experts, p.top_k, picked_e, picked_w, denom);
+            else moe_route_token<MOE_MAX_EXPERTS / 32>(p.logits, p.logits_dtype, t, p.experts, p.top_k, picked_e, picked_w, denom);
+            if (lane == 0)
+                for (int s = 0; s < p.top_k; s++) {
+                    ids[t * p.top_k + s] = picked_e[s];
+                    if (tables) {
+                        p.top_idx[t * p.top_k + s] = picked_e[s];
+                        p.top_w[t * p.top_k + s] = p.norm_topk ? picked_w[s] / denom : picked_w[s];
+                    }
+                }
+        }
+    }
+    __syncthreads();
+    auto local = [&](int e) { return e >= p.e_lo && e < p.e_lo + p.n_exp; };
+    int pos = 0;
+    const bool mine = tid < pairs && local(ids[tid]);
+    if (mine) { // ascending experts, pairs of an expert in their order
+        for (int j = 0; j < pairs; j++) pos += local(ids[j]) && (ids[j] < ids[tid] || (ids[j] == ids[tid] && j < tid));
+        perm[pos] = tid;
+        if (tables) p.inv[tid] = pos;
+    }
+    const int rows = __syncthreads_count(mine);
+    if (tables) {
+        int c = 0;
+        if (tid < p.n_exp)
+            for (int j = 0; j < pairs; j++) c += ids[j] == p.e_lo + tid;
+        moe_plan_expert(c, p.n_exp, p.e_lo, p.max_rows, p.offsets, p.entries, p.n_blocks, scratch);
+    } else moe_mx_split_rows(p.x, rows, p.pieces, gridDim.x - 1, [&](int row) { return perm[row] / p.top_k; });
 }
 
 // Stable partition: position of pair i among the pairs of its expert, in pair (= token) order.
@@ -449,14 +520,8 @@ struct MoeLayout {
     size_t top_idx, top_w, counts, offsets, grp_beg, entries, perm, inv, xs, h, slab, total;
     size_t h_scales, h_second, x_pieces, x_scales, x_second; // inside the slab
     int group_experts, n_groups, max_mt;
-    bool decode; // few pairs: no dequantized slab, the slab region holds the f32 gate_up outputs
+    bool small; // few pairs: no dequantized slab, the block-scaled kernel serves every layer
 };
-
-static bool moe_decode_shape(size_t pairs, int hidden, int inter)
-{
-    return pairs <= (size_t)MOE_DECODE_MAX_PAIRS && hidden % 32 == 0 && inter % 32 == 0 &&
-           mxfp4_gemv_batched_supported(hidden, nullptr) && mxfp4_gemv_batched_supported(inter, nullptr);
-}
 
 static MoeLayout moe_layout(int tokens, int top_k, int n_exp, int hidden, int inter)
 {
@@ -483,8 +548,8 @@ static MoeLayout moe_layout(int tokens, int top_k, int n_exp, int hidden, int in
     L.inv = off; off = align_up(off + pairs * 4, 256);
     L.xs = off; off = align_up(off + (pairs + 128) * hidden * 2, 256); // also the down-projection output
     L.h = off; off = align_up(off + (pairs + 128) * inter * 2, 256);
-    L.decode = moe_decode_shape(pairs, hidden, inter);
-    // dequantized experts; or the f32 gate_up outputs; or, for the block-scaled kernel, the pieces of h and of x with their scales and
+    L.small = pairs <= (size_t)MOE_FRONT_PAIRS && hidden <= MOE_SMALL_MAX_K && inter <= MOE_SMALL_MAX_K;
+    // dequantized experts; or, for the block-scaled kernel, the pieces of h and of x with their scales and
     // what says which of them have a second pair
     const int cap = (int)pairs + 128;
     L.h_scales = align_up(moe_mx_piece_bytes(cap, inter), 256);
@@ -492,9 +557,9 @@ static MoeLayout moe_layout(int tokens, int top_k, int n_exp, int hidden, int in
     L.x_pieces = L.h_second + align_up(moe_mx_second_bytes(cap, inter), 256);
     L.x_scales = L.x_pieces + align_up(moe_mx_piece_bytes(cap, hidden), 256);
     L.x_second = L.x_scales + align_up(moe_mx_scale_bytes(cap, hidden), 256);
-    const size_t mx = L.x_second + moe_mx_second_bytes(cap, hidden), f32 = pairs * 2 * inter * sizeof(float);
+    const size_t mx = L.x_second + moe_mx_second_bytes(cap, hidden);
     const size_t dense = (size_t)ge * per_expert;
-    L.slab = off; off = align_up(off + (L.decode ? (f32 > mx ? f32 : mx) : dense > mx ? dense : mx), 256);
+    L.slab = off; off = align_up(off + (L.small || dense < mx ? mx : dense), 256);
     L.total = off;
     return L;
 }
@@ -557,9 +622,6 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     __nv_bfloat16 *slab = reinterpret_cast<__nv_bfloat16 *>(ws + L.slab);
     const int pairs = tokens * top_k;
 
-    if (given_ids) moe_assign_kernel<<<ceil_div(tokens, 256), 256, 0, st>>>(given_ids, tokens, top_idx, top_w);
-    else OXQ_CUDA(launch_early(moe_route_kernel, ceil_div(tokens * 32, 256), 256, st, router_logits, logits_dtype, tokens, num_experts, top_k,
-                               norm_topk, top_idx, top_w));
     const int a_rows = pairs + 128;
     // Both projections through the kernel that unpacks the MXFP4 blocks inside the tensor-core loop, where it takes the shapes:
     // no dequantized slab, one launch per projection over all experts.
@@ -569,29 +631,23 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
     // their experts are all local.
     const int spread = given_ids ? n_exp : num_experts;
     // Up to a few dozen rows per expert: the codes as tensor-core operands, nothing unpacked.
-    const bool mx = pairs <= MOE_MX_ROWS * spread && moe_mx_supported(2 * inter, hidden, gu_blocks, gu_scales) &&
+    const bool mx = (pairs <= MOE_MX_ROWS * spread || pairs <= MOE_FRONT_PAIRS) && moe_mx_supported(2 * inter, hidden, gu_blocks, gu_scales) &&
                     moe_mx_supported(hidden, inter, dn_blocks, dn_scales);
-    if (L.decode && !((fused || mx) && pairs > MOE_DECODE_FUSED_FROM_PAIRS)) {
-        OXQ_REQUIRE(aligned(gu_blocks, 16) && aligned(dn_blocks, 16), OXQ_ERR_BAD_ALIGN,
-                    "oxq_gptoss_moe_forward: expert blocks must be 16-byte aligned");
-        // Decode: only the selected experts' packed weights are read. gate_up (f32 out, bias folded) ->
-        // down on its SwiGLU (into the xs buffer, bf16) -> combine, row = pair.
-        OXQ_LAUNCH_CHECK("moe_route_kernel");
-        float *gu = reinterpret_cast<float *>(slab);
-        int rc = mxfp4_gemv_batched(x, top_k, gu_blocks, gu_scales, gu_bias, bias_dtype, top_idx, pairs, expert_lo, expert_hi,
-                                    gu, OXQ_F32, hidden, 2 * inter, st);
-        if (rc) return rc;
-        rc = mxfp4_gemv_batched(x, 1, dn_blocks, dn_scales, dn_bias, bias_dtype, top_idx, pairs, expert_lo, expert_hi, xs,
-                                OXQ_BF16, inter, hidden, st, gu, limit);
-        if (rc) return rc;
-        OXQ_CUDA(launch_early(moe_combine_kernel, ceil_div(tokens * ceil_div(hidden / 8, 32) * 32, 256), 256, st, xs, top_idx, top_w, nullptr,
-                              tokens, top_k, hidden, expert_lo, expert_hi, out, out_dtype));
-        return OXQ_OK;
-    }
+    const bool front = mx && pairs <= MOE_FRONT_PAIRS; // routing is part of a larger kernel
+    OXQ_REQUIRE(!L.small || (aligned(gu_blocks, 16) && aligned(dn_blocks, 16)), OXQ_ERR_BAD_ALIGN,
+                "oxq_gptoss_moe_forward: expert blocks must be 16-byte aligned");
+    if (given_ids && !front) moe_assign_kernel<<<ceil_div(tokens, 256), 256, 0, st>>>(given_ids, tokens, top_idx, top_w);
+    else if (!front && num_experts <= 32)
+        OXQ_CUDA(launch_early(moe_route_kernel<1>, ceil_div(tokens * 32, 256), 256, st, router_logits, logits_dtype, tokens, num_experts, top_k,
+                              norm_topk, top_idx, top_w));
+    else if (!front)
+        OXQ_CUDA(launch_early(moe_route_kernel<MOE_MAX_EXPERTS / 32>, ceil_div(tokens * 32, 256), 256, st, router_logits, logits_dtype, tokens,
+                              num_experts, top_k, norm_topk, top_idx, top_w));
     // the grouped kernel's table of token blocks goes where the m-tile table of the dense path would (same capacity bound);
     // grp_beg[0] then holds the number of blocks
     const int block_rows = mx ? moe_mx_block_rows() : moe_fused_block_rows(pairs / spread);
-    if ((fused || mx) && pairs <= MOE_SMALL_PAIRS) {
+    if (front) {
+    } else if ((fused || mx) && pairs <= MOE_SMALL_PAIRS) {
         OXQ_CUDA(launch_early(moe_dispatch_small_kernel, 1, 1024, st, top_idx, pairs, expert_lo, n_exp, block_rows, counts, offsets, entries,
                               grp_beg, perm, inv));
     } else {
@@ -605,18 +661,27 @@ static int moe_forward_impl(const void *x, int x_dtype, const void *router_logit
         unsigned char *sb = reinterpret_cast<unsigned char *>(slab);
         OXQ_LAUNCH_CHECK("moe routing kernels");
         const unsigned long long mark = mx_call_mark();
-        int rc = moe_mx_split(x, perm, top_k, offsets + n_exp, hidden, a_rows, sb + L.x_pieces, sb + L.x_scales, sb + L.x_second, mark, st);
+        int rc = OXQ_OK;
+        if (front) {
+            MoeFrontParams f = {};
+            f.logits = router_logits; f.given = given_ids; f.x = (const __nv_bfloat16 *)x; f.logits_dtype = logits_dtype; f.tokens = tokens;
+            f.experts = num_experts; f.top_k = top_k; f.norm_topk = norm_topk; f.e_lo = expert_lo; f.n_exp = n_exp; f.max_rows = block_rows;
+            f.top_idx = top_idx; f.offsets = offsets; f.n_blocks = grp_beg; f.inv = inv; f.top_w = top_w; f.entries = entries;
+            f.pieces = moe_mx_pieces(hidden, a_rows, sb + L.x_pieces, sb + L.x_scales, sb + L.x_second, mark);
+            OXQ_CUDA(launch_early(moe_front_kernel, ceil_div(pairs * f.pieces.stages * 16, MOE_MAX_EXPERTS) + 1, MOE_MAX_EXPERTS, st, f));
+        } else rc = moe_mx_split(x, perm, top_k, offsets + n_exp, pairs, hidden, a_rows, sb + L.x_pieces, sb + L.x_scales, sb + L.x_second, mark, st);
         if (rc) return rc;
         rc = moe_mx_grouped(sb + L.x_pieces, sb + L.x_scales, sb + L.x_second, mark, a_rows, gu_blocks, gu_scales, num_experts, 2 * inter, hidden,
                             entries, grp_beg, gu_bias, bias_dtype, h, inter, 1, limit, flag, st);
         if (rc) return rc;
-        rc = moe_mx_split(h, nullptr, 1, offsets + n_exp, inter, a_rows, sb, sb + L.h_scales, sb + L.h_second, mark, st);
+        rc = moe_mx_split(h, nullptr, 1, offsets + n_exp, pairs, inter, a_rows, sb, sb + L.h_scales, sb + L.h_second, mark, st);
         if (rc) return rc;
         rc = moe_mx_grouped(sb, sb + L.h_scales, sb + L.h_second, mark, a_rows, dn_blocks, dn_scales, num_experts, hidden, inter, entries, grp_beg,
                             dn_bias, bias_dtype, xs, hidden, 0, limit, flag, st);
         if (rc) return rc;
-        OXQ_CUDA(launch_early(moe_combine_kernel, sm_count() * 8, 256, st, xs, top_idx, top_w, inv, tokens, top_k, hidden, expert_lo, expert_hi,
-                              out, out_dtype));
+        const int warps = tokens * ceil_div(hidden / 8, 32), most = sm_count() * 64; // a warp takes 32 pieces of 16 bytes of a token
+        OXQ_CUDA(launch_early(moe_combine_kernel, ceil_div(warps < most ? warps : most, 8), 256, st, xs, top_idx, top_w, inv, tokens, top_k, hidden,
+                              expert_lo, expert_hi, out, out_dtype));
         return OXQ_OK;
     }
     moe_gather_kernel<<<sm_count() * 8, 256, 0, st>>>((const __nv_bfloat16 *)x, perm, offsets + n_exp, top_k, hidden, xs);
@@ -732,7 +797,8 @@ OXQ_EXPORT int oxq_moe_route(const float *router_logits, int tokens, int num_exp
                     top_k <= num_experts,
                 OXQ_ERR_BAD_SHAPE, "oxq_moe_route: tokens %d, experts %d (max %d), top_k %d (max %d)", tokens, num_experts,
                 MOE_MAX_EXPERTS, top_k, MOE_MAX_TOPK);
-    moe_route_kernel<<<ceil_div(tokens * 32, 256), 256, 0, (cudaStream_t)stream>>>(router_logits, OXQ_F32, tokens, num_experts,
+    auto kern = num_experts <= 32 ? moe_route_kernel<1> : moe_route_kernel<MOE_MAX_EXPERTS / 32>;
+    kern<<<ceil_div(tokens * 32, 256), 256, 0, (cudaStream_t)stream>>>(router_logits, OXQ_F32, tokens, num_experts,
                                                                                     top_k, norm_topk, top_idx, top_w);
     OXQ_LAUNCH_CHECK("moe_route_kernel");
     return OXQ_OK;

@@ -18,12 +18,11 @@
 // What bounds it: a stage's chain of polls, operand rows and arrival in a team. us a layer at 13 / 50 / 200 / 340 tokens, 32 experts of
 // 2880 x 2880, with two teams 122 / 148 / 167 / 194, with three 108 / 130 / 144 / 170, with what outliers need 119 / 131 / 146 / 173; packed
 // weights alone take 66 from HBM. With an outlier in every block of 32 columns 50 tokens take 183.
-#include "mx_common.cuh"
+#include "moe_mx_split.cuh"
 
 namespace oxq {
 
 constexpr int MM_ROWS = 128;                 // out features per unit
-constexpr int MM_BK = 128;                   // input columns per stage
 constexpr int MM_MAX_TOK = 48;               // rows of a token block
 constexpr int MM_TEAMS = 3, MM_ISSUERS = 2, MM_TEAM_WARPS = 4, MM_UNPACK_WARPS = MM_TEAMS * MM_TEAM_WARPS, MM_EPI_WARPS = 4;
 constexpr int MM_EPI_WARP0 = 4 + MM_UNPACK_WARPS;
@@ -61,43 +60,13 @@ struct MoeMxParams {
 };
 
 // ---- rows -> pieces and block scales ---------------------------------------------------------------------------------------------
-// Sixteen lanes hold 128 columns of a row. Row r is src[perm[r] / top_k] (perm null: src[r]); q: [pair][piece][rows_cap][k]; sfx:
-// [pair][stage][rows_cap], a byte per 32 columns; second: [stage][rows_cap]. The second pair is written where a row has one, and not at
-// all elsewhere. k is a multiple of 32.
+// Row r is src[perm[r] / top_k] (perm null: src[r]).
 __global__ void __launch_bounds__(256)
-    moe_mx_split_kernel(const __nv_bfloat16 *src, const int *perm, int top_k, const int *total_rows, int k, int stages, int rows_cap,
-                        unsigned char *q, unsigned char *sfx, unsigned char *second, unsigned long long *any, unsigned long long mark)
+    moe_mx_split_kernel(const __nv_bfloat16 *src, const int *perm, int top_k, const int *total_rows, const MoeMxPieces q)
 {
     pdl_wait();
     pdl_launch_dependents();
-    const int rows = ld_produced(total_rows), lane = threadIdx.x & 15;
-    for (int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; (item & ~1) < rows * stages; item += (gridDim.x * blockDim.x) >> 4) {
-        const bool real = item < rows * stages; // the other half of a warp may be past the end: it stays for the shuffles
-        const int row = real ? item / stages : 0, st = real ? item - row * stages : 0, c = st * MM_BK + lane * 8;
-        const int from = perm ? ld_produced(perm + row) / top_k : row;
-        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-        if (c < k) raw = ld_produced(reinterpret_cast<const uint4 *>(src + (size_t)from * k + c));
-        const MxBlock b = mx_block(raw);
-        auto store = [&](int pair, uint2 hi, uint2 lo, uint32_t s) {
-            if (!real || c >= k) return;
-            unsigned char *dst = q + ((size_t)pair * 2 * rows_cap + row) * k + c;
-            *reinterpret_cast<uint2 *>(dst) = hi;
-            *reinterpret_cast<uint2 *>(dst + (size_t)rows_cap * k) = lo;
-            if ((lane & 3) == 0) sfx[((size_t)(pair * stages + st) * rows_cap + row) * 4 + (lane >> 2)] = (unsigned char)s;
-        };
-        float v[8];
-        uint2 hi, lo;
-        const uint32_t s = mx_first_pair(raw, b, v, hi, lo);
-        store(0, hi, lo, s);
-        const unsigned half = 0xFFFFu << (threadIdx.x & 16); // the row's lanes of this warp
-        const unsigned ask = __ballot_sync(0xFFFFFFFFu, b.second != MX_ONE_PAIR), e5m2 = __ballot_sync(0xFFFFFFFFu, b.second == MX_SECOND_E5M2);
-        if (real && lane == 0) second[(size_t)st * rows_cap + row] = (unsigned char)(!(ask & half) ? MX_ONE_PAIR : (e5m2 & half) ? MX_SECOND_E5M2 : MX_SECOND_E4M3);
-        if (ask) { // some row of the warp
-            const uint32_t s2 = mx_second_pair(raw, v, s, (e5m2 & half) != 0, hi, lo);
-            if (ask & half) store(1, hi, lo, s2);
-            if (real && lane == 0) *any = mark;
-        }
-    }
+    moe_mx_split_rows(src, ld_produced(total_rows), q, gridDim.x, [&](int row) { return perm ? ld_produced(perm + row) / top_k : row; });
 }
 
 // Stages in which rows of a token block have a second pair, in order, E4M3 before E5M2: body(stage, MX_...), until it returns false.
@@ -417,18 +386,13 @@ __device__ __forceinline__ void moe_mx_roles(const MoeMxParams &p, const CUtenso
         }
     }
 }
-// Two kernels, of which a call launches both and one returns at once: a launch costs less than the second pairs cost the usual path in
-// one kernel (340 tokens 192 us a layer with the code for both in a call, 248 in one loop).
-template <bool SECOND>
+// Without and with the code for second pairs, whole: in one loop 340 tokens took 248 us a layer, with what they need in a call 192, as
+// two kernels of which one returns at once 181 (50 tokens 139), chosen by a vote, which keeps what the loops compute in uniform registers, 180 (137).
 __global__ void __launch_bounds__(MM_THREADS, 1)
     moe_mx_kernel(const MoeMxParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
 {
     extern __shared__ unsigned char smem_raw[];
     pdl_launch_dependents();
-    if (SECOND) {
-        pdl_wait();
-        if (ld_produced(p.any) != p.mark) return;
-    }
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand slots want 1 KB alignment
     unsigned char *base_ptr = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t bars = base + MM_BARS;
@@ -464,8 +428,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem_base = tail[0];
     pdl_wait(); // table, rows and their scales come from kernels ahead; their time must not count as this kernel's waits
-    const int n_units = SECOND || ld_produced(p.any) != p.mark ? ld_produced(p.n_blocks) * p.tiles_n : 0;
-    moe_mx_roles<SECOND>(p, wmap, xmap, base, tmem_base, n_units);
+    const int n_units = ld_produced(p.n_blocks) * p.tiles_n;
+    if (__any_sync(0xFFFFFFFFu, ld_produced(p.any) == p.mark)) moe_mx_roles<true>(p, wmap, xmap, base, tmem_base, n_units);
+    else moe_mx_roles<false>(p, wmap, xmap, base, tmem_base, n_units);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -479,7 +444,6 @@ static thread_local int g_moe_mx_selftest_skip_loads = 0; // set only inside oxq
 // Rows of a token block.
 int moe_mx_block_rows() { return MM_MAX_TOK; }
 
-static int moe_mx_stages(int k) { return (k + MM_BK - 1) / MM_BK; }
 // Bytes of both pairs of pieces of `rows` rows, of their block scales, and of what says which have a second pair (the call's mark in front).
 size_t moe_mx_piece_bytes(int rows, int k) { return (size_t)4 * rows * k; }
 size_t moe_mx_scale_bytes(int rows, int k) { return (size_t)8 * rows * moe_mx_stages(k); }
@@ -491,12 +455,12 @@ bool moe_mx_supported(int n, int k, const void *blocks, const void *scales)
     return n > 0 && n % 2 == 0 && k >= 32 && k % 32 == 0 && scales != nullptr && aligned(blocks, 16);
 }
 
-// Row r of the pieces is src[perm[r] / top_k] (perm null: src[r]), for the rows that total_rows[0] counts.
-int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int k, int rows_cap, void *pieces, void *sfx, void *second,
+// Row r of the pieces is src[perm[r] / top_k] (perm null: src[r]), for the rows that total_rows[0] counts, at most `most`.
+int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_rows, int most, int k, int rows_cap, void *pieces, void *sfx, void *second,
                  unsigned long long mark, cudaStream_t st)
 {
     cudaLaunchConfig_t cfg = {};
-    const long long blocks = (long long)rows_cap * moe_mx_stages(k) * 16 / 256 + 1;
+    const long long blocks = (long long)most * moe_mx_stages(k) * 16 / 256 + 1;
     cfg.gridDim = dim3((unsigned)(blocks < 8 * sm_count() ? blocks : 8 * sm_count()), 1, 1);
     cfg.blockDim = dim3(256, 1, 1);
     cfg.stream = st;
@@ -504,8 +468,8 @@ int moe_mx_split(const void *src, const int *perm, int top_k, const int *total_r
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_split_kernel, (const __nv_bfloat16 *)src, perm, top_k, total_rows, k, moe_mx_stages(k), rows_cap,
-                                (unsigned char *)pieces, (unsigned char *)sfx, (unsigned char *)second + 8, (unsigned long long *)second, mark));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_split_kernel, (const __nv_bfloat16 *)src, perm, top_k, total_rows,
+                                moe_mx_pieces(k, rows_cap, pieces, sfx, second, mark)));
     return OXQ_OK;
 }
 
@@ -533,8 +497,7 @@ int moe_mx_grouped(const void *pieces, const void *sfx, const void *second, unsi
     int device = 0;
     OXQ_CUDA(cudaGetDevice(&device));
     if (device >= 64 || configured[device] < MM_SMEM) {
-        OXQ_CUDA(cudaFuncSetAttribute(moe_mx_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
-        OXQ_CUDA(cudaFuncSetAttribute(moe_mx_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
+        OXQ_CUDA(cudaFuncSetAttribute(moe_mx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM));
         if (device < 64) configured[device] = MM_SMEM;
     }
     cudaLaunchConfig_t cfg = {};
@@ -546,8 +509,7 @@ int moe_mx_grouped(const void *pieces, const void *sfx, const void *second, unsi
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_kernel<false>, p, wmap, xmap));
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_kernel<true>, p, wmap, xmap));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, moe_mx_kernel, p, wmap, xmap));
     return OXQ_OK;
 }
 

@@ -32,13 +32,6 @@ struct Mx4GemvParams {
     int m, k, n;
     int row_tiles, k_warps; // warps of a CTA = row_tiles x k_warps
     int token_split;        // neighbouring CTAs that share their rows and take 8*MT tokens each (>= 1)
-    // Batched single-token mode (MoE decode): grid z = (token, slot) pair; the pair's expert id selects
-    // the weight, bias and scale slices, its token (pair / x_div) the x row, and y row = pair.
-    const int *pair_expert; // null: plain mode
-    int x_div, e_lo, e_hi;
-    const float *gu; // not null: the x row of a pair is the clamped SwiGLU of gu[pair][2 k] (gate and up columns in turn), as bf16
-    float limit;
-    int tiles;       // row groups (16 * row_tiles rows): a CTA takes every gridDim.x-th of them with the x it has staged
 };
 
 __device__ __forceinline__ void mx4_mma_f16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2])
@@ -65,7 +58,6 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
 {
     extern __shared__ __align__(16) unsigned char smem[];
     pdl_launch_dependents();
-    if (p.pair_expert) pdl_wait(); // the routing table comes from the kernel before this one
     cg::cluster_group cluster = cg::this_cluster();
     const int nrt = p.row_tiles, ks = (int)gridDim.y, rank = (int)blockIdx.y; // cluster = the y extent of the grid
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
@@ -73,18 +65,6 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     const int zt = blockIdx.x % p.token_split, bx = blockIdx.x / p.token_split;
     const int m0 = zt * 8 * MT, m_loc = min(8 * MT, p.m - m0); // this CTA's tokens [m0, m0 + m_loc)
     const int nb = p.k >> 5;                       // blocks per row
-    const uint8_t *blocks = p.blocks, *scales = p.scales;
-    const __nv_bfloat16 *xin = p.x;
-    size_t bias_off = 0, y_off = 0;
-    if (p.pair_expert) {
-        const int pair = blockIdx.z, e = p.pair_expert[pair];
-        if (e < p.e_lo || e >= p.e_hi) return; // the same for every CTA of the cluster: nobody waits for this one
-        blocks += (size_t)e * p.n * nb * 16;
-        scales += (size_t)e * p.n * nb;
-        xin += (size_t)(pair / p.x_div) * p.k;
-        bias_off = (size_t)e * p.n;
-        y_off = (size_t)pair * p.n;
-    }
     const int bl = nb / ks, b_cta = rank * bl;     // this CTA's blocks
     const int wb = bl / p.k_warps, b_off = kw * wb; // this warp's part of them
     const int kl = bl << 5, k_cta = b_cta << 5;
@@ -93,47 +73,26 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     float *red = reinterpret_cast<float *>(smem + (size_t)m_loc * xrow * 2); // [warp][MT*4][lane]
     float *zeros = red + blockDim.x * MT * 4; // 16 bytes of zeros: what lanes without a token read as x
 
-    const uint32_t *q0, *q1;
-    const uint8_t *s0p, *s1p;
+    // the first blocks of this warp's rows
+    const int n0 = (bx * nrt + rt) * 16;
+    const int r0 = min(n0 + g, p.n - 1), r1 = min(n0 + g + 8, p.n - 1); // past-the-end rows re-read the last row
+    const uint32_t *q0 = reinterpret_cast<const uint32_t *>(p.blocks + ((size_t)r0 * nb + b_cta + b_off) * 16) + c;
+    const uint32_t *q1 = reinterpret_cast<const uint32_t *>(p.blocks + ((size_t)r1 * nb + b_cta + b_off) * 16) + c;
+    const uint8_t *s0p = p.scales + (size_t)r0 * nb + b_cta + b_off, *s1p = p.scales + (size_t)r1 * nb + b_cta + b_off;
     uint32_t buf0[D], buf1[D], sb0[D], sb1[D];
-    auto start = [&](int group) { // the first blocks of a row group
-        const int n0 = (group * nrt + rt) * 16;
-        const int r0 = min(n0 + g, p.n - 1), r1 = min(n0 + g + 8, p.n - 1); // past-the-end rows re-read the last row
-        q0 = reinterpret_cast<const uint32_t *>(blocks + ((size_t)r0 * nb + b_cta + b_off) * 16) + c;
-        q1 = reinterpret_cast<const uint32_t *>(blocks + ((size_t)r1 * nb + b_cta + b_off) * 16) + c;
-        s0p = scales + (size_t)r0 * nb + b_cta + b_off;
-        s1p = scales + (size_t)r1 * nb + b_cta + b_off;
 #pragma unroll
-        for (int d = 0; d < D; d++)
-            if (d < wb) {
-                buf0[d] = __ldg(q0 + 4 * d);
-                buf1[d] = __ldg(q1 + 4 * d);
-                sb0[d] = __ldg(s0p + d);
-                sb1[d] = __ldg(s1p + d);
-            }
-    };
-    const int stride = (int)gridDim.x / p.token_split;
-    int group = bx;
-    start(group);
+    for (int d = 0; d < D; d++)
+        if (d < wb) {
+            buf0[d] = __ldg(q0 + 4 * d);
+            buf1[d] = __ldg(q1 + 4 * d);
+            sb0[d] = __ldg(s0p + d);
+            sb1[d] = __ldg(s1p + d);
+        }
 
     if (tid < 4) zeros[tid] = 0.0f;
-    if (!p.pair_expert) pdl_wait(); // x may come from the kernel before this one; the first weights are already on their way
-    if (p.gu) { // one row: SwiGLU of the pair's gate and up values, rounded to bf16 as the layer's activations are
-        const float4 *src = reinterpret_cast<const float4 *>(p.gu + (size_t)blockIdx.z * 2 * p.k + 2 * k_cta);
-        uint32_t *dst = reinterpret_cast<uint32_t *>(xs);
-        for (int i = tid; i < (kl >> 1); i += blockDim.x) {
-            const float4 v = ld_produced(src + i);
-            float h[2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float gate = fminf(e ? v.z : v.x, p.limit), up = fminf(fmaxf(e ? v.w : v.y, -p.limit), p.limit);
-                const float sig = __fdividef(1.0f, __expf(-1.702f * gate) + 1.0f);
-                h[e] = __bfloat162float(__float2bfloat16_rn((up + 1.0f) * (gate * sig)));
-            }
-            dst[i] = f32x2_to_f16x2_sat(h[0], h[1]);
-        }
-    } else for (int row = 0; row < m_loc; row++) {
-        const uint2 *src = reinterpret_cast<const uint2 *>(xin + (size_t)(m0 + row) * p.k + k_cta);
+    pdl_wait(); // x may come from the kernel before this one; the first weights are already on their way
+    for (int row = 0; row < m_loc; row++) {
+        const uint2 *src = reinterpret_cast<const uint2 *>(p.x + (size_t)(m0 + row) * p.k + k_cta);
         uint2 *dst = reinterpret_cast<uint2 *>(xs + (size_t)row * xrow);
         for (int q4 = tid; q4 < (kl >> 2); q4 += blockDim.x) {
             const uint2 raw = ld_produced(src + q4);
@@ -143,7 +102,6 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     }
     __syncthreads();
 
-    for (;;) {
     // This lane's x for fragment column g of token tile mt: 8 halves per block, or the zeros (stride 0).
     const uint4 *xp[MT];
     int xstep[MT];
@@ -198,53 +156,31 @@ __global__ void __launch_bounds__(256, MT == 1 ? 4 : MT == 2 ? 3 : 2) mxfp4_gemv
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
         for (int e = 0; e < 4; e++) red[(warp * MT * 4 + mt * 4 + e) * 32 + lane] = tot[mt][e];
-    const int done = group;
-    group += stride;
-    if (group < p.tiles) start(group); // the next rows are on their way while this group is put together
     if (ks > 1) cluster.sync(); else __syncthreads();
 
     // Every (row tile, accumulator slot, lane) is summed by one thread of the cluster, in ascending k.
     const int slots = nrt * MT * 4 * 32;
     for (int o = rank * blockDim.x + tid; o < slots; o += ks * blockDim.x) {
         const int ln = o & 31, e = (o >> 5) & 3, mt = (o >> 7) % MT, wt = (o >> 7) / MT;
-        const int nn = (done * nrt + wt) * 16 + (ln >> 2) + 8 * (e >> 1), row = 8 * mt + 2 * (ln & 3) + (e & 1);
+        const int nn = (bx * nrt + wt) * 16 + (ln >> 2) + 8 * (e >> 1), row = 8 * mt + 2 * (ln & 3) + (e & 1);
         if (nn < p.n && row < m_loc) {
             float sum = 0.0f;
             for (int q = 0; q < ks; q++) {
                 const float *src = ks > 1 ? cluster.map_shared_rank(red, q) : red;
                 for (int w = 0; w < p.k_warps; w++) sum += src[((w * nrt + wt) * MT * 4 + mt * 4 + e) * 32 + ln];
             }
-            if (p.bias) sum += load_as_f32(p.bias, p.bias_dtype, bias_off + nn);
-            store_as(p.y, p.y_dtype, y_off + (size_t)(m0 + row) * p.n + nn, sum);
+            if (p.bias) sum += load_as_f32(p.bias, p.bias_dtype, nn);
+            store_as(p.y, p.y_dtype, (size_t)(m0 + row) * p.n + nn, sum);
         }
     }
-    if (ks > 1) cluster.sync(); // nobody leaves, or writes the next sums, while a peer may still read its shared memory
-    if (group >= p.tiles) break;
-    if (ks == 1) __syncthreads();
-    }
+    if (ks > 1) cluster.sync(); // nobody leaves while a peer may still read its shared memory
 }
 
-template <int MT, int D> static int launch_mx4(Mx4GemvParams p, int ks, cudaStream_t st, int batch = 1)
+template <int MT, int D> static int launch_mx4(const Mx4GemvParams &p, int ks, cudaStream_t st)
 {
-    p.tiles = ceil_div(p.n, 16 * p.row_tiles);
     const int nw = p.row_tiles * p.k_warps;
     const int m_cta = p.m < 8 * MT ? p.m : 8 * MT;
     const size_t smem = (size_t)m_cta * (p.k / ks + 8) * 2 + (size_t)nw * MT * 4 * 32 * 4 + 16;
-    // Batched: a CTA takes `groups` row groups of a pair with the x it has staged once. A launch is as many rounds of resident CTAs
-    // (at 64 registers a thread 1024 threads fit an SM) as it needs, each of `groups` steps plus the staging: a quarter of a step,
-    // three quarters where the activation is computed with it. The cheapest of 1 .. 8 is taken: with shares that just miss one round
-    // (32 pairs, 5760 x 2880: 768 CTAs where 740 fit) the expert layer took 235 us for 8 tokens.
-    int ctas = p.tiles;
-    if (batch > 1 && ks == 1) {
-        const int by_smem = (int)(228 * 1024 / (smem + 1024)), by_threads = 1024 / (nw * 32);
-        const int resident = sm_count() * (by_smem < by_threads ? by_smem : by_threads);
-        long long least = -1;
-        for (int groups = 1; groups <= 8; groups++) {
-            const int cand = ceil_div(p.tiles, groups);
-            const long long cost = (long long)ceil_div(cand * batch, resident) * (8 * groups + (p.gu ? 6 : 2));
-            if (least < 0 || cost < least) { least = cost; ctas = cand; }
-        }
-    }
     auto kern = mxfp4_gemv_kernel<MT, D>;
     static size_t configured[64] = {};
     int device = 0;
@@ -254,7 +190,7 @@ template <int MT, int D> static int launch_mx4(Mx4GemvParams p, int ks, cudaStre
         if (device < 64) configured[device] = smem;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas * p.token_split, ks, batch);
+    cfg.gridDim = dim3(ceil_div(p.n, 16 * p.row_tiles) * p.token_split, ks, 1);
     cfg.blockDim = dim3(nw * 32, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -313,35 +249,7 @@ int mxfp4_gemv_fast(const void *x, const uint8_t *blocks, const uint8_t *scales,
     }
     p.row_tiles = nrt; p.k_warps = kw;
     p.token_split = ceil_div(m, 8); // 8 tokens per CTA; more on neighbouring CTAs
-    p.pair_expert = nullptr; p.x_div = 1; p.e_lo = p.e_hi = 0; p.gu = nullptr; p.limit = 0.0f;
     return launch_mx4<1, 4>(p, ks, st);
-}
-
-// One single-token GEMV per (token, slot) pair against the pair's expert, all pairs in one launch:
-// y[pair, :] = x[pair / x_div, :] . W[expert(pair)]^T + bias[expert(pair)]; pairs whose expert lies
-// outside [e_lo, e_hi) are skipped (their y rows stay untouched). gu not null: the x row of a pair is the clamped SwiGLU of
-// gu[pair, 2 k] instead. blocks / scales / bias are the
-// stacked tensors of all experts ([E, n, k/32, 16], [E, n, k/32], [E, n]).
-bool mxfp4_gemv_batched_supported(int k, const void *blocks)
-{
-    int a, b, c;
-    return k % 32 == 0 && (reinterpret_cast<uintptr_t>(blocks) & 15) == 0 && mx4_pick(1, k, a, b, c) &&
-           (size_t)(k + 8) * 2 <= 160 * 1024;
-}
-
-int mxfp4_gemv_batched(const void *x, int x_div, const uint8_t *blocks, const uint8_t *scales, const void *bias,
-                       int bias_dtype, const int *pair_expert, int pairs, int e_lo, int e_hi, void *y, int y_dtype, int k,
-                       int n, cudaStream_t st, const float *gu, float limit)
-{
-    Mx4GemvParams p;
-    p.gu = gu; p.limit = limit;
-    p.x = (const __nv_bfloat16 *)x; p.blocks = blocks; p.scales = scales; p.bias = bias; p.y = y;
-    p.bias_dtype = bias_dtype; p.y_dtype = y_dtype; p.m = 1; p.k = k; p.n = n;
-    int nrt = 2, kw = 4, ks = 1;
-    mx4_pick(1, k, nrt, kw, ks);
-    p.row_tiles = nrt; p.k_warps = kw; p.token_split = 1;
-    p.pair_expert = pair_expert; p.x_div = x_div; p.e_lo = e_lo; p.e_hi = e_hi;
-    return launch_mx4<1, 4>(p, ks, st, pairs);
 }
 
 } // namespace oxq

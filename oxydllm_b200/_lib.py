@@ -6,7 +6,9 @@ missing it is built in-tree with nvcc; if that fails, importing raises.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import warnings
 
 from . import build as _build
 
@@ -134,3 +136,24 @@ def call(name: str, *args) -> None:
     rc = entry(name)(*args)
     if rc != 0:
         fail(name, rc)
+
+
+_host = None
+
+
+def host():
+    """The native host side of decode calls (``csrc/host_ops.cpp``), or None where it cannot be built: the callers' Python code does the same."""
+    global _host
+    if _host is None:
+        try:
+            path = _build.build_host()
+            spec = importlib.util.spec_from_file_location("oxydllm_b200._host", path)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            lib = load()
+            mod.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in SIGNATURES})
+            _host = mod
+        except (RuntimeError, OSError, ImportError, KeyError) as e:
+            warnings.warn(f"oxydllm_b200: calls take a few microseconds longer without the host extension ({e})")
+            _host = False
+    return _host or None

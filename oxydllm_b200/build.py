@@ -9,6 +9,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(_HERE, "csrc")
@@ -57,5 +58,37 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def host_path() -> str:
+    return os.path.join(_HERE, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_host(force: bool = False) -> str:
+    """Compile ``csrc/host_ops.cpp`` against the installed torch into the extension module ``_host``; returns its path."""
+    import torch
+    src, out = os.path.join(CSRC, "host_ops.cpp"), host_path()
+    header = os.path.join(_HERE, "..", "include", "oxq.h")
+    fresh = lambda: os.path.exists(out) and os.path.getmtime(out) >= max(os.path.getmtime(src), os.path.getmtime(header))  # noqa: E731
+    if not force and fresh():
+        return out
+    root = os.path.dirname(torch.__file__)
+    with open(out + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if not force and fresh():
+            return out
+        tmp = f"{out}.{os.getpid()}.tmp"
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I" + os.path.join(root, "include"),
+               "-I" + sysconfig.get_paths()["include"], "-I/usr/local/cuda/include", "-o", tmp, src, "-L" + os.path.join(root, "lib"),
+               "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode:
+            if os.path.exists(tmp):
+                os.remove(tmp)
+            raise RuntimeError("g++ failed building the host extension:\n" + res.stderr[-4000:])
+        os.replace(tmp, out)
+    return out
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_host(force="--force" in sys.argv))

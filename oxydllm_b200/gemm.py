@@ -22,6 +22,19 @@ def _dt(t: torch.dtype) -> int:
         raise ValueError(f"unsupported dtype {t}") from None
 
 _workspaces: dict = {}
+_native = None
+
+
+def native():
+    """The host extension with this module's buffers in its hands, or None without it."""
+    global _native
+    if _native is None:
+        _native = _lib.host() or False
+        if _native:
+            for kind, bufs in enumerate((_flags, _workspaces)):
+                for buf in bufs.values():
+                    _native.keep(kind, buf)
+    return _native or None
 
 
 def workspace_bytes(n: int, k: int) -> int:
@@ -36,6 +49,8 @@ def workspace(n: int, k: int, device) -> torch.Tensor:
     if buf is None or buf.numel() < need:
         buf = torch.zeros(need, dtype=torch.uint8, device=device)
         _workspaces[key] = buf
+        if _native:
+            _native.keep(1, buf)
     return buf
 
 
@@ -77,6 +92,8 @@ def _flag_words(device) -> torch.Tensor:
     buf = _flags.get(key)
     if buf is None:
         buf = _flags[key] = torch.zeros(256, dtype=torch.uint8, device=torch.device("cuda", key))
+        if _native:
+            _native.keep(0, buf)
     return buf
 
 
@@ -185,14 +202,10 @@ def gguf_stream_matmul(lin, x2, y) -> bool:
     """``y = x2 . deq(W)^T (+ bias)`` by the stream kernel (``oxq_gguf_matmul``) with scratch of the call's own; False where another
     kernel is the better one."""
     m = x2.shape[0]
-    need = lin._scratch_bytes.get(m)
-    if need is None:
-        need = lin._scratch_bytes[m] = int(_lib.entry("oxq_gguf_scratch_bytes")(lin.ggml_type, m, lin.in_features, lin.out_features))
+    need = int(_lib.entry("oxq_gguf_scratch_bytes")(lin.ggml_type, m, lin.in_features, lin.out_features))
     if not need:
         return False
-    flag = _flags.get(x2.device.index)
-    if flag is None:
-        flag = _flag_words(x2.device)
+    flag = _flag_words(x2.device)
     scratch = torch.empty(need, dtype=torch.uint8, device=x2.device)
     bp, bd = _bias(lin.bias)
     _lib.call("oxq_gguf_matmul", lin.ggml_type, x2.data_ptr(), _dt(x2.dtype), lin.blocks.data_ptr(), bp, bd, y.data_ptr(), _dt(y.dtype),

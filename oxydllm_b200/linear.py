@@ -315,6 +315,12 @@ class PackedQuantLinear:
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""
+        host = gemm.native() if out is None else None
+        if host is not None:  # plain CUDA tensors; everything else is checked and done below
+            y = host.packed4(x, self.qweight, self.qzeros, self.scales, self.bias, self.in_features, self.out_features, self.group_size, self.bits,
+                             self.pack_dim == "in", self.sym, self._batches)
+            if y is not None:
+                return y
         x2, lead, m = _flatten_x(x, self.in_features, "PackedQuantLinear")
         if not x2.is_cuda:
             _require_cuda(x2)
@@ -383,6 +389,11 @@ class GatedFfnProjection:
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lin = self.gate_up
+        host = gemm.native()
+        if host is not None:
+            y = host.ffn(x, lin.qweight, lin.qzeros, lin.scales, lin.in_features, self.intermediate, lin.group_size, ACTIVATIONS[self.activation])
+            if y is not None:
+                return y
         x2, lead, m = _flatten_x(x, lin.in_features, "GatedFfnProjection")
         if not x2.is_cuda:
             _require_cuda(x2)
@@ -458,6 +469,11 @@ class Fp8Linear:
         return AWQ_FUSED_MIN_M - 1 if fused else GEMV_MAX_M
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        host = gemm.native()
+        if host is not None:
+            y = host.fp8(x, self.weight, self.scale_inv, self.bias, self.in_features, self.out_features, FP8_UNALIGNED_GEMV_MAX_M)
+            if y is not None:
+                return y
         s, s_out, s_in = self._grid()
         x2, lead, m = _flatten_x(x, self.in_features, "Fp8Linear")
         _require_cuda(x2, self.weight, self.bias)
@@ -498,7 +514,6 @@ class QLinear:
         self.out_features, self.in_features = out_features, in_features
         self.bias = None if bias is None else bias.contiguous()
         self.out_dtype = out_dtype
-        self._scratch_bytes: dict = {}  # of the stream kernel, by batch; 0 where it does not serve the call
 
     from_blocks = classmethod(lambda cls, *a, **k: cls(*a, **k))
 
@@ -510,6 +525,11 @@ class QLinear:
         return out
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        host = gemm.native()
+        if host is not None:
+            y = host.gguf(x, self.blocks, self.bias, self.ggml_type, self.in_features, self.out_features, gemm._DT.get(self.out_dtype, -1), GEMV_MAX_M)
+            if y is not None:
+                return y
         x2, lead, m = _flatten_x(x, self.in_features, "QLinear")
         _require_cuda(x2, self.blocks, self.bias)
         y = x2.new_empty((m, self.out_features), dtype=self.out_dtype)

@@ -315,7 +315,7 @@ class PackedQuantLinear:
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""
-        host = gemm.native() if out is None else None
+        host = gemm.native() if out is None and x.is_cuda else None
         if host is not None:  # plain CUDA tensors; everything else is checked and done below
             y = host.packed4(x, self.qweight, self.qzeros, self.scales, self.bias, self.in_features, self.out_features, self.group_size, self.bits,
                              self.pack_dim == "in", self.sym, self._batches)
@@ -389,7 +389,7 @@ class GatedFfnProjection:
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lin = self.gate_up
-        host = gemm.native()
+        host = gemm.native() if x.is_cuda else None
         if host is not None:
             y = host.ffn(x, lin.qweight, lin.qzeros, lin.scales, lin.in_features, self.intermediate, lin.group_size, ACTIVATIONS[self.activation])
             if y is not None:
@@ -469,7 +469,7 @@ class Fp8Linear:
         return AWQ_FUSED_MIN_M - 1 if fused else GEMV_MAX_M
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        host = gemm.native()
+        host = gemm.native() if x.is_cuda else None
         if host is not None:
             y = host.fp8(x, self.weight, self.scale_inv, self.bias, self.in_features, self.out_features, FP8_UNALIGNED_GEMV_MAX_M)
             if y is not None:
@@ -525,7 +525,7 @@ class QLinear:
         return out
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        host = gemm.native()
+        host = gemm.native() if x.is_cuda else None
         if host is not None:
             y = host.gguf(x, self.blocks, self.bias, self.ggml_type, self.in_features, self.out_features, gemm._DT.get(self.out_dtype, -1), GEMV_MAX_M)
             if y is not None:

@@ -21,18 +21,6 @@ __device__ __forceinline__ void st_mma_first(float (&d)[4], uint32_t a0, uint32_
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
-__device__ __forceinline__ void st_mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
-}
-__device__ __forceinline__ void st_mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void st_ldmatrix(uint32_t (&r)[4], uint32_t addr)
 {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -70,7 +58,7 @@ struct StreamOut {
     int units_per_tile, total;   // units of k of a tile; of all tiles
     int grain;                   // shares are whole multiples of this many units
     float *partials;             // [CTA + tile][tok_step][out features of a tile] f32
-    unsigned long long *tickets; // per tile: this call's mark above, arrivals in the low byte
+    unsigned long long *flags;   // [CTA + tile]: this call's mark once the CTA's sum of the tile is in scratch
     unsigned long long mark;
 };
 
@@ -79,6 +67,26 @@ __host__ __device__ __forceinline__ int st_share(const StreamOut &o, int ctas, i
 __host__ __device__ __forceinline__ int st_owner(const StreamOut &o, int ctas, int u)
 {
     return (int)((((long long)(u / o.grain) + 1) * ctas - 1) / (o.total / o.grain));
+}
+
+// How many CTAs share the list, and whether they share tiles (o.grain). In hundredths of a microsecond: a unit takes `unit`; a tile in c equal
+// parts costs part0 + part1 c to put together, shares that cross tile borders `cross`. Each share says by a mark of its own that its sum is there: counting the
+// shares of a tile down with atomics on one word took 0.6 us a share (Q4_0, 2048 x 1024, one token: 7.6 us, with marks 6.4).
+inline int st_ctas(StreamOut &o, int unit, int part0, int part1, int cross)
+{
+    const int sms = sm_count(), tiles = o.total / o.units_per_tile;
+    int best = ceil_div(tiles, sms) * o.units_per_tile * unit, ctas = tiles < sms ? tiles : sms;
+    o.grain = o.units_per_tile;
+    for (int c = 2; tiles * c <= sms && c <= o.units_per_tile; c++) {
+        const int cost = ceil_div(o.units_per_tile, c) * unit + part0 + part1 * c;
+        if (cost < best) { best = cost; ctas = tiles * c; o.grain = 1; }
+    }
+    if (o.total >= 2 * sms && tiles % sms != 0) {
+        const int cost = ceil_div(o.total, sms) * unit + cross;
+        if (cost < best) { best = cost; ctas = sms; o.grain = 1; }
+    }
+    if (const char *e = tuning_env("ST_CTAS")) { ctas = atoi(e) < o.total ? atoi(e) : o.total; o.grain = 1; }
+    return ctas;
 }
 
 __device__ __forceinline__ float st_act(float g, float u, int act)
@@ -123,14 +131,6 @@ __device__ __forceinline__ void st_output(const StreamOut &o, Mend mend, int til
     st_store_pair(o, (size_t)tok * o.ldy + col, v.x, v.y);
 }
 
-// What a CTA that is about to finish its last segment sees of the tile's ticket: read a while ahead, used in st_finish.
-__device__ __forceinline__ unsigned long long st_ticket(const StreamOut &o, int tile)
-{
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(__cvta_generic_to_global(o.tickets + tile)) : "memory");
-    return v;
-}
-
 // The sums of CTAs i_lo .. i_hi for token tok, columns 2 i and 2 i + 1 of a tile, in ascending k; that of CTA i_lo + me is `own`.
 template <int COLS>
 __device__ __forceinline__ float2 st_total(const StreamOut &o, int tile, int i_lo, int i_hi, int tok, int i, int me = -1, float2 own = make_float2(0.0f, 0.0f))
@@ -150,41 +150,52 @@ __device__ __forceinline__ float2 st_total(const StreamOut &o, int tile, int i_l
     }
     return s;
 }
-// One thread's arrival at a tile's ticket, for its CTA (whose sums a barrier has ordered before): whether it is the last of most + 1.
-__device__ __forceinline__ uint32_t st_arrive(const StreamOut &o, int tile, unsigned most)
+// One warp: whether the sums of CTAs i_lo .. i_hi of a tile, but for this CTA's, are all in scratch. They may be read if so.
+__device__ __forceinline__ bool st_others(const StreamOut &o, int tile, int i_lo, int i_hi)
 {
-    // The scratch area holds anything at first: a ticket without this call's mark counts as no arrival. The last one
-    // leaves the mark with a count of zero (a replayed graph comes back with the same mark).
-    unsigned long long *t = o.tickets + tile, old = *reinterpret_cast<volatile unsigned long long *>(t), seen;
-    unsigned count;
-    __threadfence(); // the sums before the ticket
-    for (;;) {
-        count = (old >> 8) == o.mark ? (unsigned)(old & 0xFFu) : 0u;
-        seen = atomicCAS(t, old, (o.mark << 8) | (count == most ? 0u : count + 1u));
-        if (seen == old) break; // fails only when another of the tile's CTAs came in between
-        old = seen;
+    bool all = true;
+    for (int i = i_lo + (int)(threadIdx.x & 31); i <= i_hi; i += 32)
+        all = all && (i == (int)blockIdx.x || *reinterpret_cast<volatile unsigned long long *>(o.flags + i + tile) == o.mark);
+    all = __all_sync(0xFFFFFFFFu, all);
+    if (all) __threadfence(); // the flags before the sums
+    return all;
+}
+// One warp sets its CTA's flag, whose sum a barrier has ordered before; true where all flags of the tile are set. Of all that set one the last
+// sees them all, and so may another just before it: both then put the same tile together. The flags are cleared for a replayed
+// graph, which comes back with the same mark; what the scratch area holds at first is not the mark. (A counter per tile, which has to be swapped in with the
+// mark, took 0.6 us for every CTA of the tile: 4096 x 4096 in 8 parts 11.6 us.)
+__device__ __forceinline__ bool st_arrive(const StreamOut &o, int tile, int i_lo, int i_hi)
+{
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence(); // the sum before the flag
+        *reinterpret_cast<volatile unsigned long long *>(o.flags + blockIdx.x + tile) = o.mark;
+        __threadfence(); // this flag before the others' are read
     }
-    __threadfence(); // the ticket before the others' sums
-    return count == most;
+    __syncwarp();
+    return st_others(o, tile, i_lo, i_hi);
+}
+__device__ __forceinline__ void st_clear(const StreamOut &o, int tile, int i_lo, int i_hi)
+{
+    for (int i = i_lo + (int)(threadIdx.x & 31); i <= i_hi; i += 32) *reinterpret_cast<volatile unsigned long long *>(o.flags + i + tile) = 0ull;
 }
 
 // End of this CTA's segment [u, seg_end) of a tile: `planes` partial tiles [token][PLANE] lie `stride` floats apart in `red`, all
 // THREADS threads that call this have written theirs. A whole tile goes to y; of a shared one every CTA leaves its sum in scratch, and the
 // CTA that arrives last adds the sums in ascending k: no CTA waits for another, and the result does not depend on the order of arrival.
 //
-// The four round trips to L2 that this takes (sums and ticket out, ticket and sums in) are about 3 us, a quarter of a whole call. A CTA whose
-// share goes on (final = false) leaves them to a helping warp (st_help). The first CTA of a tile, which comes to it last, mostly finds with
-// `ticket`, read before its last box, that all others have arrived: it takes their sums and its own from shared memory.
+// The round trips to L2 that this takes (sums and flag out, flags and sums in) are about 2 us. A CTA whose share goes on (final = false) leaves them
+// to a helping warp (st_help). The first CTA of a tile, which comes to it last, mostly knows from before its last box (`others`, the first warp's st_others)
+// that all others have arrived: it takes their sums and its own from shared memory.
 // `last`: a shared word. `ok`: false after a wait gave up (nothing is stored, the flag word is set).
 template <int THREADS, int COLS, int PLANE, typename Mend>
 __device__ __forceinline__ void st_finish(const StreamOut &o, Mend mend, const float *red, int planes, int stride, int tile, int u, int seg_end, bool final,
-                                          unsigned long long ticket, bool ok, volatile uint32_t *last)
+                                          bool others, bool ok, volatile uint32_t *last)
 {
     const int et = threadIdx.x;
     const int i_lo = st_owner(o, gridDim.x, tile * o.units_per_tile), i_hi = st_owner(o, gridDim.x, (tile + 1) * o.units_per_tile - 1);
     const unsigned most = (unsigned)(i_hi - i_lo);
     const bool whole = most == 0;
-    if (et == 0) *last = !whole && final && (ticket >> 8) == o.mark && (unsigned)(ticket & 0xFFu) == most;
+    if (et == 0) *last = !whole && final && others;
     asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
     auto own = [&](int tok, int i) {
         float2 s = make_float2(0.0f, 0.0f);
@@ -214,7 +225,7 @@ __device__ __forceinline__ void st_finish(const StreamOut &o, Mend mend, const f
         }
     };
     if (early) {
-        if (et == 0) *reinterpret_cast<volatile unsigned long long *>(o.tickets + tile) = o.mark << 8; // as below
+        if (et < 32) st_clear(o, tile, i_lo, i_hi);
         if (ok) outputs(et, THREADS);
         return;
     }
@@ -227,18 +238,24 @@ __device__ __forceinline__ void st_finish(const StreamOut &o, Mend mend, const f
         return;
     }
     asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
-    if (et == 0) *last = st_arrive(o, tile, most);
+    if (et < 32) {
+        const bool all = st_arrive(o, tile, i_lo, i_hi);
+        if (all) st_clear(o, tile, i_lo, i_hi);
+        if (et == 0) *last = all;
+    }
     asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
     if (*last && ok) outputs(et, THREADS);
 }
 
-// The helping warp's part of a first segment that does not end the CTA's share: the ticket, while the others go on. Where it is the
+// The helping warp's part of a first segment that does not end the CTA's share: the flag, while the others go on. Where it is the
 // tile's last, all THREADS threads put the tile together at the end (st_helped).
 template <int THREADS> __device__ __forceinline__ void st_help(const StreamOut &o, int tile, volatile uint32_t *helped)
 {
     const int i_lo = st_owner(o, gridDim.x, tile * o.units_per_tile), i_hi = st_owner(o, gridDim.x, (tile + 1) * o.units_per_tile - 1);
     asm volatile("bar.sync 2, %0;" ::"n"(THREADS + 32) : "memory");
-    if ((threadIdx.x & 31) == 0) *helped = st_arrive(o, tile, (unsigned)(i_hi - i_lo));
+    const bool all = st_arrive(o, tile, i_lo, i_hi);
+    if (all) st_clear(o, tile, i_lo, i_hi);
+    if ((threadIdx.x & 31) == 0) *helped = all;
     __syncwarp();
     asm volatile("bar.arrive 3, %0;" ::"n"(THREADS + 32) : "memory");
 }

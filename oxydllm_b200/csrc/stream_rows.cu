@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(KQ * 128 + 128, 1)
     const SrMend<TYPE> mend{p.x, p.blocks, p.k};
     float tot[2][MT][4];
     bool ok = true;
-    unsigned long long ticket = 0;
+    bool others = false;
     for (int u = u0; u < u1;) {
         const int tile = u / G, seg_end = min(u1, (tile + 1) * G), first_unit = u;
 #pragma unroll
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(KQ * 128 + 128, 1)
                 for (int i = 0; i < 4; i++) tot[t][mt][i] = 0.0f;
 #pragma unroll 1
         for (; u < seg_end; u++) {
-            if (u + 1 == seg_end && seg_end == u1 && threadIdx.x == 0) ticket = st_ticket(p.out, tile);
+            if (u + 1 == seg_end && seg_end == u1 && warp == 0) others = st_others(p.out, tile, st_owner(p.out, gridDim.x, tile * G), st_owner(p.out, gridDim.x, (tile + 1) * G - 1));
             if (Fm::TABLE) ok = ok && mx_wait2(full + 8 * s, ph, ready + 8 * s, ph, p.flag, ST_CODE + 2);
             else ok = ok && mx_wait(full + 8 * s, ph, p.flag, ST_CODE + 2);
             if (!ok) continue;
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(KQ * 128 + 128, 1)
                 at[8] = tot[t][mt][2];
                 at[SR_PLANE + 8] = tot[t][mt][3];
             }
-        st_finish<SR_CONSUMERS, SR_ROWS, SR_PLANE>(p.out, mend, red, KQ, 8 * MT * SR_PLANE, tile, first_unit, seg_end, seg_end == u1, ticket, ok, &last);
+        st_finish<SR_CONSUMERS, SR_ROWS, SR_PLANE>(p.out, mend, red, KQ, 8 * MT * SR_PLANE, tile, first_unit, seg_end, seg_end == u1, others, ok, &last);
     }
     if (help) st_helped<SR_CONSUMERS, SR_ROWS>(p.out, mend, u0 / G, ok, &helped);
 }
@@ -393,7 +393,7 @@ static int sr_block_tokens(int m) // tokens of a tile
     const int blocks = ceil_div(m, SR_MAX_BLOCK);
     return ceil_div(ceil_div(m, blocks), 8) * 8;
 }
-static size_t sr_ticket_bytes(int tiles) { return ((size_t)tiles * sizeof(unsigned long long) + 255) / 256 * 256; }
+static size_t sr_flag_bytes(int tiles) { return ((size_t)(sm_count() + tiles) * sizeof(unsigned long long) + 255) / 256 * 256; }
 
 bool gguf_stream_supported(int type, int m, int k, int n, const void *x, const void *blocks)
 {
@@ -409,7 +409,7 @@ bool gguf_stream_supported(int type, int m, int k, int n, const void *x, const v
 size_t gguf_stream_scratch_bytes(int m, int n)
 {
     const int step = sr_block_tokens(m), tiles = ceil_div(n, SR_ROWS) * ceil_div(m, step);
-    return sr_ticket_bytes(tiles) + (size_t)(sm_count() + tiles) * step * SR_ROWS * sizeof(float);
+    return sr_flag_bytes(tiles) + (size_t)(sm_count() + tiles) * step * SR_ROWS * sizeof(float);
 }
 
 template <int TYPE, int MT, int KQ>
@@ -443,30 +443,6 @@ static int sr_launch(StreamRowsParams &p, const CUtensorMap &wmap, const CUtenso
     return OXQ_OK;
 }
 
-// How many CTAs share the list, and whether they share tiles. In hundredths of a microsecond, fitted to Q4_0 on 4096 x 4096 and 4096 x
-// 14336 at 1 to 64 tokens: a unit takes 55 up to eight tokens, 65 / 85 / 175 at 16 / 32 / 64; a tile in c equal parts costs 130 + 50 c
-// (250 + 90 c at 32 tokens) to put together; shares that cross tile borders 450 (840 at 32). 4096 x 4096 in 1 / 2 / 4 parts, one token,
-// 13.0 / 10.6 / 9.8 us, 148 equal shares 10.7; 4096 x 14336 in whole tiles 14.1, equal shares 15.4 (64 tokens 36.5 against 43.4).
-static int sr_ctas(StreamOut &o)
-{
-    const int sms = sm_count(), tiles = o.total / o.units_per_tile, mb = o.tok_step > 8 ? o.tok_step - 8 : 0;
-    const int unit = o.tok_step > 32 ? 85 + (o.tok_step - 32) * 45 / 16 : 55 + mb * 5 / 4;
-    int best = ceil_div(tiles, sms) * o.units_per_tile * unit, ctas = tiles < sms ? tiles : sms;
-    o.grain = o.units_per_tile;
-    for (int c = 2; tiles * c <= sms && c <= o.units_per_tile; c++) {
-        const int cost = ceil_div(o.units_per_tile, c) * unit + 130 + 5 * mb + c * (50 + mb * 5 / 3);
-        if (cost < best) { best = cost; ctas = tiles * c; o.grain = 1; }
-    }
-    if (o.total >= 2 * sms && tiles % sms != 0) {
-        const int cost = ceil_div(o.total, sms) * unit + 450 + 16 * mb;
-        if (cost < best) { best = cost; ctas = sms; o.grain = 1; }
-    }
-#ifdef OXQ_TUNING
-    if (const char *e = tuning_env("SR_CTAS")) { ctas = atoi(e) < o.total ? atoi(e) : o.total; o.grain = 1; }
-#endif
-    return ctas;
-}
-
 template <int TYPE>
 static int sr_run(StreamRowsParams &p, const void *x, const void *blocks, int k, cudaStream_t st)
 {
@@ -481,7 +457,9 @@ static int sr_run(StreamRowsParams &p, const void *x, const void *blocks, int k,
     r = encode_tiled_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, x, (uint64_t)k / 2, (uint64_t)o.m, (uint64_t)k * 2, SR_X_PITCH / 4, 8 * mt,
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (x) failed with CUresult %d", (int)r);
-    const int ctas = sr_ctas(p.out);
+    // a unit, in hundredths of a us: 55 up to eight tokens, 65 / 85 / 175 at 16 / 32 / 64
+    const int more = o.tok_step > 8 ? o.tok_step - 8 : 0;
+    const int ctas = st_ctas(p.out, o.tok_step > 32 ? 85 + (o.tok_step - 32) * 45 / 16 : 55 + more * 5 / 4, 150 + 6 * more, 10 + more * 5 / 4, 450 + 16 * more);
     const char *e4 = tuning_env("SR_KQ");
     const int kq = e4 ? atoi(e4) : 2;
     switch (mt) {
@@ -507,8 +485,8 @@ int gguf_stream_matmul(int type, const void *x, const void *blocks, const void *
     const int tiles = ceil_div(n, SR_ROWS) * o.tok_blocks;
     o.total = tiles * o.units_per_tile;
     o.mark = mx_call_mark();
-    o.tickets = reinterpret_cast<unsigned long long *>(scratch);
-    o.partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + sr_ticket_bytes(tiles));
+    o.flags = reinterpret_cast<unsigned long long *>(scratch);
+    o.partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + sr_flag_bytes(tiles));
     switch (type) {
     case OXQ_GGML_Q4_0: return sr_run<OXQ_GGML_Q4_0>(p, x, blocks, k, st);
     case OXQ_GGML_Q8_0: return sr_run<OXQ_GGML_Q8_0>(p, x, blocks, k, st);
@@ -521,28 +499,34 @@ int gguf_stream_matmul(int type, const void *x, const void *blocks, const void *
 
 using namespace oxq;
 
-// Where the other kernels are the faster ones. Up to 32 tokens those are the GEMVs: on small layers, with few tokens, us there / here:
-// Q4_0 2048 x 1024 at 1 / 4 / 8 / 16 tokens 4.0 / 5.9 / 8.6 / 13.5 against 7.6 / 7.7 / 7.8 / 9.0, 2048 x 6144 at one token 7.4 against 8.3, 4096
-// x 4096 13.6 against 10.1, 4096 x 14336 at 8 tokens 81 against 14; Q8_0 2048 x 1024 at 4 / 8 tokens 7.6 / 9.9 against 9.2; Q4_K 4096 x 4096 at
-// 1 / 8 / 16 tokens 5.6 / 9.8 / 15.7 against 11.1 / 11.7 / 14.5, 14336 x 4096 at 1 / 4 / 8 14.6 / 31.8 / 183 against 19; 4096 x 14336 at one 18.9
-// against 17.3; Q6_K has a kernel of its own for wide layers, 4096 x 14336 at 1 / 8 tokens 14.7 / 17.3 against 19.4. Above 32 tokens they are the dense
-// copy and its GEMM, about 0.9 us a million weights and 4 us a thousand of k (4096 x 4096 31 us, 14336 x 4096 111 at 64 and 128 tokens), against 20 us
-// and 0.0133 (Q4_0) to 0.0225 (Q4_K) a unit of 64 tokens here (4096 x 14336 at 64 tokens 36.5 to 57.8 us, 68 to 70 there).
+// Where the other kernels are the faster ones. Up to 32 tokens those are the GEMVs: on small layers, with few tokens, us there / here, in graphs of calls on
+// different weights. Q4_0: 2048 x 1024 at 4 / 8 tokens 6.0 / 8.6 against 6.5 / 7.3, 2048 x 2560 at 2 / 4 6.8 / 8.2 against 7.3, 4096 x 1024 at 1 / 2 6.6 / 7.9 against
+// 7.3, 2048 x 6144 at 2 / 4 8.4 / 10.5 against 9.1, 2048 x 11264 at one 13.4 against 9.7. Q8_0: 2048 x 1024 at 2 / 4 6.4 / 7.6 against 6.6, 4096 x 1024 at one 11.5 against
+// 8.1. Q4_K: 2048 x 1024 at 8 / 12 / 16 / 32 6.6 / 10.5 / 12.7 / 12.8 against 7.7 / 9.7 / 10.3 / 14.5, 4096 x 4096 at 1 / 8 / 12 5.6 / 9.8 / 13.4 against 10.1 / 11.0 / 13.0, 2048 x 6144
+// at 2 / 4 7.9 / 10.1 against 9.4, 2048 x 11264 at 1 / 2 10.1 / 11.6 against 10.6, 14336 x 4096 at 1 / 2 / 4 14.6 / 16.7 / 31.6 against 18.1, 14336 x 1024 at 1 / 2 9.9 / 12.5
+// against 10.5, 4096 x 14336 at one 19.0 against 17.2. Q6_K, which has a kernel of its own for wide layers (4096 x 14336 at 1 / 8 14.7 / 17.3 against 19.4): 4096 x 1024 at
+// 4 / 8 7.6 / 11.2 against 8.7 / 9.4, 4096 x 4096 at one 12.6 against 11.2, 4096 x 6144 at 1 / 2 12.9 / 14.2 against 13.4.
+// Above 32 tokens they are the dense copy and its GEMM, about 0.9 us a million weights and 4 us a thousand of k (4096 x 4096 31 us, 14336 x 4096 111 at 64 and
+// 128 tokens), against 20 us and 0.0133 (Q4_0) to 0.0225 (Q4_K) a unit of 64 tokens here (4096 x 14336 at 64 tokens 36.5 to 57.8 us, 68 to 70 there).
 static bool gguf_stream_faster(int type, int m, int k, int n)
 {
+    if (const char *e = tuning_env("SR_ROUTE")) return atoi(e) != 0;
     const long long w = (long long)k * n, mw = m * w;
     if (m <= 32) {
         switch (type) {
-        case OXQ_GGML_Q4_0: return mw >= 14000000;
-        case OXQ_GGML_Q8_0: return mw >= 12000000;
+        case OXQ_GGML_Q4_0:
+            if (k >= 4096) return mw >= 8000000;
+            return m >= 8 ? mw >= 14000000 : w >= (m >= 4 ? 5000000 : 20000000);
+        case OXQ_GGML_Q8_0: return mw >= (k >= 4096 ? 4000000 : k >= 2048 ? 5000000 : 12000000);
         case OXQ_GGML_Q4_K:
-            if (m >= 16) return w >= 8000000;
-            if (m >= 8) return k > 4096 || n >= 6144;
-            if (m >= 4) return n >= 6144 || w >= 40000000;
+            if (m >= 12) return w >= (m <= 16 ? 2000000 : 4000000);
+            if (m >= 4) return k > 4096 || n >= 6144;
+            if (m >= 2) return n >= 10240 || (k >= 12288 && n <= 2048);
             return n >= 12288 && w >= 50000000;
         default:
             if (m <= 8 && n >= 9472) return false;
-            return mw >= 80000000 || (k >= 4096 && w >= 14000000);
+            if (m >= 8) return mw >= 30000000;
+            return k >= 4096 && w >= 14000000 && (m >= 2 || n <= k);
         }
     }
     const int slope = type == OXQ_GGML_Q4_0 ? 133 : type == OXQ_GGML_Q8_0 ? 155 : type == OXQ_GGML_Q4_K ? 225 : 180;

@@ -54,6 +54,7 @@ SIGNATURES = {
     "oxq_gemm_workspace_init": [_vp, _vp],
     "oxq_awq_gemm": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp],
     "oxq_packed4_max_m": [_i, _i, _i],
+    "oxq_packed4_streams": [_i, _i, _i, _i, _i],
     "oxq_packed4_scratch_bytes": [_i, _i],
     "oxq_packed4_full_scratch_bytes": [_i, _i, _i, _i, _i],
     "oxq_packed4_matmul": [_vp, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _sz, _vp],

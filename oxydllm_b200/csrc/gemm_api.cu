@@ -40,21 +40,42 @@ int packed_mx_matmul(const void *x, const uint32_t *qweight, const uint32_t *qze
 bool fp8_mx_supported(int m, int k, int n, int block_out, int block_in, const void *x, const void *weight, const void *scale_inv);
 int fp8_mx_matmul(const void *x, const uint8_t *weight, const float *scale_inv, int s_in, int block_out, int block_in, const void *bias,
                   int bias_dtype, void *y, int y_dtype, int m, int k, int n, int *flag, cudaStream_t st, void *scratch, size_t scratch_bytes);
+bool stream4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros,
+                       const void *scales, int gate);
+bool stream4_faster(int m, int k, int n, int group_size, int gptq);
+size_t stream4_scratch_bytes(int m, int n);
+int stream4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, const void *bias, int bias_dtype, void *y,
+                   int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag, cudaStream_t st, int gptq, int sym, int gate,
+                   void *scratch, size_t scratch_bytes);
 int awq_fused_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy,
                      int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
 
-// The 4-bit matmuls without a dense copy of the weight: csrc/group_tc.cu up to group_tc_max_m tokens, then csrc/fused_tc.cu up to 256.
-static bool packed4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
-                              const void *qzeros, const void *scales)
+// The 4-bit matmuls without a dense copy of the weight: csrc/stream4.cu for the few tokens that stream4_faster says, csrc/group_tc.cu up to
+// group_tc_max_m tokens, then csrc/fused_tc.cu up to 256.
+static bool packed4_streams(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros, const void *scales,
+                            int gptq, int gate = 0)
 {
-    return group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
+    return stream4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gate) && stream4_faster(m, k, n, group_size, gptq);
+}
+static bool packed4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
+                              const void *qzeros, const void *scales, int gptq)
+{
+    return packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) || group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
            (aligned(qzeros, 16) && awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales));
 }
 static int packed4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype,
                           const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base,
                           int ldy, int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes)
 {
+    if (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq)) {
+        const int rc = stream4_matmul(x, qweight, qzeros, scales, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base, ldy, flag, st, gptq,
+                                      sym, 0, scratch, scratch_bytes);
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc; // scratch too small for the parts of tiles
+    }
+    if (!group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) &&
+        !(aligned(qzeros, 16) && awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales)))
+        return OXQ_ERR_UNSUPPORTED;
     if (gptq && packed_mx_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales)) {
         const int rc = packed_mx_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base,
                                         ldy, flag, st, sym, scratch, scratch_bytes);
@@ -188,10 +209,10 @@ static const char *wait_name(int code)
     case 65: return "packed words";
     case 66: return "operand slot";
     case 67: return "last MMAs";
-    // GGUF stream kernel
+    // stream kernels (GGUF; 4-bit of few tokens)
     case 81: return "ring slot";
-    case 82: return "blocks, x, or unpacked scales";
-    case 83: return "blocks";
+    case 82: return "weights, x, or unpacked scales";
+    case 83: return "weights";
     default: return "not one of a kernel's";
     }
 }
@@ -235,7 +256,7 @@ OXQ_EXPORT int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight,
     int rc = prepare("oxq_awq_gemm", c, x, x_dtype, bias, bias_dtype, y, y_dtype, m, k, n, workspace, workspace_bytes, stream);
     if (rc) return rc;
     // Up to 256 tokens: unpack inside the tensor-core kernel, no dense copy of the weight.
-    if (packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales))
+    if (packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, 0))
     {
         rc = packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n, c.flag,
                               c.st, 0, 0, c.slab, c.slab_bytes);
@@ -254,10 +275,17 @@ OXQ_EXPORT int oxq_packed4_max_m(int k, int n, int group_size)
                ? group_tc_max_m(n, group_size) : 0;
 }
 
+OXQ_EXPORT int oxq_packed4_streams(int m, int k, int n, int group_size, int gptq)
+{
+    return stream4_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, 0) && stream4_faster(m, k, n, group_size, gptq);
+}
+
 OXQ_EXPORT size_t oxq_packed4_full_scratch_bytes(int m, int k, int n, int group_size, int gptq)
 {
     if (m <= 0 || k <= 0 || n <= 0 || n % 128 != 0 || k % 128 != 0 || group_size <= 0) return 0;
-    const size_t own = group_tc_scratch_bytes(m, n);
+    size_t own = group_tc_scratch_bytes(m, n);
+    if (stream4_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, 0) && stream4_faster(m, k, n, group_size, gptq))
+        own = own > stream4_scratch_bytes(m, n) ? own : stream4_scratch_bytes(m, n);
     const bool mxs = gptq && packed_mx_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr);
     const size_t mx = mxs ? packed_mx_scratch_bytes(m, k, n) : 0;
     return mx > own ? mx : own;
@@ -282,8 +310,9 @@ OXQ_EXPORT int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qw
                 "oxq_packed4_matmul: shape [%d, %d] incompatible with pack factor 8 / group size %d", n, k, group_size);
     OXQ_REQUIRE(aligned(scratch, 256) && aligned(flag_word, 4), OXQ_ERR_BAD_ALIGN, "oxq_packed4_matmul: scratch must be 256-byte aligned");
     if (use_sym) qzeros = nullptr;
-    OXQ_REQUIRE(group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales), OXQ_ERR_UNSUPPORTED,
-                "oxq_packed4_matmul: out_features %d, in_features %d, group size %d or the alignment are not served", n, k, group_size);
+    OXQ_REQUIRE(group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
+                    (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) && scratch_bytes >= stream4_scratch_bytes(m, n)),
+                OXQ_ERR_UNSUPPORTED, "oxq_packed4_matmul: out_features %d, in_features %d, group size %d or the alignment are not served", n, k, group_size);
     return packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n,
                           reinterpret_cast<int *>(flag_word), (cudaStream_t)stream, gptq, use_sym, scratch, scratch_bytes);
 }
@@ -328,7 +357,7 @@ OXQ_EXPORT int oxq_awq_gemm_tp(const void *x, int x_dtype, const uint32_t *qweig
     if (rc) return rc;
     c.col_base = col_base; c.ldy = n_full;
     rc = OXQ_ERR_UNSUPPORTED;
-    if (packed4_supported(m, k, n_local, group_size, scales_dtype, x, qweight, qzeros, scales)) // decode-sized batches: no slab
+    if (packed4_supported(m, k, n_local, group_size, scales_dtype, x, qweight, qzeros, scales, 0)) // decode-sized batches: no slab
         rc = packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n_local, group_size,
                               col_base, n_full, c.flag, c.st, 0, 0, c.slab, c.slab_bytes);
     if (rc == OXQ_ERR_UNSUPPORTED)
@@ -371,7 +400,7 @@ OXQ_EXPORT int oxq_gptq_gemm(const void *x, int x_dtype, const uint32_t *qweight
     int rc = prepare("oxq_gptq_gemm", c, x, x_dtype, bias, bias_dtype, y, y_dtype, m, k, n, workspace, workspace_bytes, stream);
     if (rc) return rc;
     // 4-bit, up to 256 tokens: unpack inside the tensor-core kernel (the same kernel as AWQ with the K-major operand).
-    if (bits == 4 && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, use_sym ? nullptr : qzeros, scales))
+    if (bits == 4 && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, use_sym ? nullptr : qzeros, scales, 1))
     {
         rc = packed4_matmul(x, qweight, use_sym ? nullptr : qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n,
                               group_size, 0, n, c.flag, c.st, 1, use_sym, c.slab, c.slab_bytes);
@@ -591,7 +620,12 @@ OXQ_EXPORT int oxq_awq_ffn_gate_up(const void *x, int x_dtype, const uint32_t *q
         OXQ_CUDA(cudaLaunchKernelEx(&cfg, gated_act_rows_kernel, (const __nv_bfloat16 *)c.slab, (__nv_bfloat16 *)y, m, inter, activation));
         return OXQ_OK;
     };
-    if (m > oxq_awq_gemv_max_m(k, n, group_size) && gu_bytes <= c.slab_bytes && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales)) {
+    if (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, 0, activation)) { // gate and up meet in one tile: no row block, one launch
+        rc = stream4_matmul(x, qweight, qzeros, scales, nullptr, 0, y, OXQ_BF16, m, k, n, group_size, 0, inter, c.flag, c.st, 0, 0, activation, c.slab,
+                            c.slab_bytes);
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc;
+    }
+    if (m > oxq_awq_gemv_max_m(k, n, group_size) && gu_bytes <= c.slab_bytes && packed4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, 0)) {
         // The kernel that unpacks inside the tensor-core loop writes the row block (no dense copy of the weight); what the slab
         // holds behind the block is its scratch. 2 x 14336 out features, k = 4096, at 8 / 16 tokens: the GEMV 33 / 48 us, this
         // kernel 30 us.

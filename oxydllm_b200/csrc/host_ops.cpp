@@ -23,7 +23,7 @@ at::Tensor *g_flags[MAX_DEVICES], *g_workspaces[MAX_DEVICES];
 
 #define ENTRIES(X)                                                                                                                        \
     X(oxq_gguf_scratch_bytes) X(oxq_gguf_matmul) X(oxq_gguf_gemv) X(oxq_awq_gemv) X(oxq_w8a16_gemv) X(oxq_gptq_gemv)                      \
-    X(oxq_packed4_full_scratch_bytes) X(oxq_packed4_matmul) X(oxq_awq_ffn_gate_up) X(oxq_gemm_workspace_bytes) X(oxq_fp8_gemv)            \
+    X(oxq_packed4_full_scratch_bytes) X(oxq_packed4_streams) X(oxq_packed4_matmul) X(oxq_awq_ffn_gate_up) X(oxq_gemm_workspace_bytes) X(oxq_fp8_gemv)            \
     X(oxq_fp8_scratch_bytes) X(oxq_fp8_matmul)
 struct Entries {
 #define X(name) decltype(&::name) name;
@@ -186,7 +186,9 @@ PyObject *packed4(PyObject *const *a)
     const int m = (int)c.m;
     const void *x = c.x->data_ptr();
     const bool aligned = ((bits(x) | bits(p.qw) | bits(p.qz) | bits(p.sc)) & 15) == 0;
-    if (m <= (aligned ? gemv : unaligned)) {
+    // PackedQuantLinear._streams
+    const bool streams = aligned && nbits == 4 && p.sc_dt == OXQ_F16 && !(in && grouped && m <= gemv) && g.oxq_packed4_streams(m, k, n, group, in);
+    if (!streams && m <= (aligned ? gemv : unaligned)) {
         at::Tensor y = result(c, n, at::kBFloat16);
         void *yp = y.data_ptr();
         return finish(y, [&] {
@@ -194,7 +196,7 @@ PyObject *packed4(PyObject *const *a)
             return (nbits == 4 ? g.oxq_awq_gemv : g.oxq_w8a16_gemv)(x, OXQ_BF16, p.qw, p.qz, p.sc, p.sc_dt, b, b_dt, yp, OXQ_BF16, m, k, n, group, c.stream);
         });
     }
-    if (!aligned || m > grouped || !g_flags[c.device]) Py_RETURN_NONE;
+    if (!aligned || (!streams && m > grouped) || !g_flags[c.device]) Py_RETURN_NONE;
     const size_t need = g.oxq_packed4_full_scratch_bytes(m, k, n, group, in);
     at::Tensor y = result(c, n, at::kBFloat16), scratch = empty(c, {(int64_t)need}, at::kByte);
     void *yp = y.data_ptr(), *flag = g_flags[c.device]->data_ptr(), *sp = scratch.data_ptr();

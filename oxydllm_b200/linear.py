@@ -313,6 +313,14 @@ class PackedQuantLinear:
             return most, 0, few
         return most, few if k <= max(reach - 1024, 1024) else 1, few
 
+    def _streams(self, m: int) -> bool:
+        """Whether the kernel that streams the packed words through mma.sync is the best one for a batch (``oxq_packed4_streams``; the one
+        or two tokens of short GPTQ layers that ``_batches`` leaves to the GEMV stay there)."""
+        grouped, few, _ = self._batches
+        gptq = self.pack_dim == "in"
+        return (self.bits == 4 and self.scales.dtype == torch.float16 and not (gptq and grouped and m <= few)
+                and bool(_lib.entry("oxq_packed4_streams")(m, self.in_features, self.out_features, self.group_size, int(gptq))))
+
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``out``: optional preallocated contiguous ``[m, out_features]`` result tensor of x's dtype and device."""
         host = gemm.native() if out is None and x.is_cuda else None
@@ -336,7 +344,9 @@ class PackedQuantLinear:
         if m:
             grouped_max_m, gemv_max_m, unaligned_max_m = self._batches
             aligned = (x2.data_ptr() | tensors[0] | tensors[1] | tensors[2]) & 15 == 0
-            if m <= (gemv_max_m if aligned else unaligned_max_m):
+            if aligned and self._streams(m):
+                gemm.packed4_matmul(self, x2, y, tensors)
+            elif m <= (gemv_max_m if aligned else unaligned_max_m):
                 self._gemv(x2, y, m, tensors)
             elif aligned and m <= grouped_max_m:
                 gemm.packed4_matmul(self, x2, y, tensors)

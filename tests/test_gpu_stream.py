@@ -1,4 +1,5 @@
-"""The kernel that streams GGUF blocks through mma.sync (``oxq_gguf_matmul``), at the sizes where it can go wrong, against the oracle."""
+"""The kernels that stream GGUF blocks (``oxq_gguf_matmul``) and 4-bit words (``oxq_packed4_matmul`` where ``oxq_packed4_streams``) through mma.sync, at the
+sizes where they can go wrong, against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -96,3 +97,81 @@ def test_scratch_that_is_too_small_is_refused(cuda):
     with pytest.raises(_lib.OxqError):
         _lib.call("oxq_gguf_matmul", lin.ggml_type, x.data_ptr(), _lib.OXQ_BF16, lin.blocks.data_ptr(), 0, 0, y.data_ptr(), _lib.OXQ_BF16, 4, k, n,
                   gemm._flag_words(x.device).data_ptr(), scratch.data_ptr(), need - 256, gemm._st())
+
+
+def packed_layer(fmt, k, n, g, seed, bias=None):
+    """An AWQ ("awq") or GPTQ ("gptq", symmetric "sym") layer of random words and its weights [n, k] in 64 bits."""
+    rng = np.random.default_rng(seed)
+    words = lambda *shape: rng.integers(0, 2**32, shape, dtype=np.uint64).astype(np.uint32)
+    qw, qz = words(*((k, n // 8) if fmt == "awq" else (k // 8, n))), words(k // g, n // 8)
+    sc = rng.uniform(-0.02, 0.02, (k // g, n)).astype(np.float16)
+    dev = [torch.from_numpy(a.view(np.int32)).cuda() for a in (qw, qz)] + [torch.from_numpy(sc).cuda()]
+    raw = L.QuantWeight.new_awq(4, *dev) if fmt == "awq" else L.QuantWeight.new_gptq(4, fmt == "sym", *dev)
+    w = oracle.awq_dequant(qw, qz, sc) if fmt == "awq" else oracle.gptq_dequant(qw, qz, sc, 4, fmt == "sym")
+    return L.PackedQuantLinear(raw, bias), w.astype(np.float64)
+
+
+def packed(lin, x, out_dtype=torch.float32):
+    y = torch.full((x.shape[0], lin.out_features), 9.0, dtype=out_dtype, device="cuda")
+    gemm.packed4_matmul(lin, x, y)
+    gemm.check(gemm._flag_words(x.device))
+    return y
+
+
+# one unit and one tile; half a tile (n = 128, 384, 896); groups of 32, 64, 128, 256 and more; token blocks of 8 and 16, and two to four of them; few tiles in many
+# parts, shares across tile borders (n = 20480: 80 tiles on 148 SMs; 37888: 148 tiles)
+PACKED_SIZES = [("gptq", 1, 2048, 128, 32), ("gptq", 4, 128, 128, 128), ("gptq", 3, 1024, 384, 64), ("sym", 8, 4096, 896, 128), ("gptq", 9, 4096, 1152, 32), ("sym", 33, 4096, 128, 32),
+                ("gptq", 64, 4096, 1280, 32), ("gptq", 16, 2048, 37888, 64), ("gptq", 5, 4096, 512, 1024), ("sym", 2, 14336, 1024, 256), ("gptq", 16, 4096, 20480, 128),
+                ("awq", 1, 5632, 128, 128), ("awq", 8, 5632, 384, 128), ("awq", 3, 5632, 256, 512), ("awq", 8, 14336, 896, 64), ("awq", 9, 2048, 512, 32), ("awq", 17, 4096, 384, 32),
+                ("awq", 64, 4096, 1280, 32), ("awq", 1, 7168, 128, 32), ("awq", 16, 4096, 20480, 128), ("awq", 12, 8192, 3584, 64), ("awq", 7, 2048, 37888, 128)]
+
+
+@pytest.mark.parametrize("fmt,m,k,n,g", PACKED_SIZES)
+def test_packed_stream_matches_oracle(cuda, fmt, m, k, n, g):
+    assert _lib.entry("oxq_packed4_streams")(m, k, n, g, int(fmt != "awq")) == 1
+    x, bias = synth.activations(m, k, seed=k + m), synth.bf16_round(np.random.default_rng(1).standard_normal(n).astype(np.float32))
+    lin, w = packed_layer(fmt, k, n, g, m + n, torch.from_numpy(bias).to(torch.bfloat16).cuda())
+    xc = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
+    got = packed(lin, xc)
+    # products of small integers and bf16 values are exact; the f32 sums of k of them are off by less than 2^-17 of the sum of magnitudes
+    ref, mass = x.astype(np.float64) @ w.T + bias, np.abs(x).astype(np.float64) @ np.abs(w).T + np.abs(bias)
+    assert (np.abs(got.double().cpu().numpy() - ref) <= 2.0**-17 * mass + 1e-6).all()
+    assert torch.equal(packed(lin, xc), got)  # the same bits again
+    y = lin.forward(xc)
+    assert lin._streams(m) and torch.equal(y, got.to(torch.bfloat16))  # what the layer takes
+
+
+def test_packed_stream_infinite_and_missing_activations(cuda):
+    for fmt, k, n, g in (("awq", 5632, 384, 128), ("gptq", 4096, 384, 64), ("sym", 4096, 384, 32)):
+        lin, w = packed_layer(fmt, k, n, g, 3)
+        x = synth.activations(3, k, seed=4)
+        x[0, 5], x[1, 700] = np.inf, np.nan
+        got = packed(lin, torch.from_numpy(x).to(torch.bfloat16).cuda()).cpu().numpy()
+        sign = np.sign(w[:, 5])
+        assert np.array_equal(got[0][sign != 0], np.where(sign > 0, np.inf, -np.inf)[sign != 0]) and np.isnan(got[0][sign == 0]).all()
+        assert np.isnan(got[1]).all()
+        ref, mass = x[2].astype(np.float64) @ w.T, np.abs(x[2]).astype(np.float64) @ np.abs(w).T
+        assert (np.abs(got[2] - ref) <= 2.0**-17 * mass + 1e-6).all()
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("m,k,inter,g", [(1, 5632, 128, 128), (8, 5632, 1152, 64), (16, 4096, 10240, 128), (33, 4096, 640, 32), (7, 2048, 18944, 128)])
+def test_gate_and_up_meet_in_one_tile(cuda, m, k, inter, g, act):
+    assert _lib.entry("oxq_packed4_streams")(m, k, 2 * inter, g, 0) == 1
+    lin, w = packed_layer("awq", k, 2 * inter, g, m + inter)
+    x = synth.activations(m, k, seed=m)
+    xc = torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()
+    y = L.GatedFfnProjection(lin, act).forward(xc)
+    gate, up = (torch.from_numpy(x.astype(np.float64) @ w[i * inter:(i + 1) * inter].T) for i in (0, 1))
+    f = torch.nn.functional.silu(gate) if act == "silu" else torch.nn.functional.gelu(gate, approximate="tanh")
+    # one bf16 rounding, and sums that are off by 2^-17 of their magnitudes in a function whose slope is at most 1.13
+    mass = [torch.from_numpy(np.abs(x).astype(np.float64) @ np.abs(w[i * inter:(i + 1) * inter]).T) * 2.0**-17 for i in (0, 1)]
+    bound = 2.0**-8 * (f * up).abs() + 1.13 * mass[0] * up.abs() + mass[1] * (f.abs() + mass[0]) + 2.0**-18 * (f * up).abs() + 1e-6
+    assert ((y.double().cpu() - f * up).abs() <= bound).all()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        again = L.GatedFfnProjection(lin, act).forward(xc)
+    for _ in range(3):  # marks of an earlier replay are not taken for this one's
+        again.fill_(9.0)
+        graph.replay()
+        assert torch.equal(again, y)

@@ -263,8 +263,9 @@ int oxq_awq_gemm(const void *x, int x_dtype, const uint32_t *qweight, const uint
  * OXQ_ERR_UNSUPPORTED for shapes the kernel does not take. gptq = 0: AWQ layout (qzeros required); 1: GPTQ layout (sym != 0 or
  * qzeros null: zero point 8). */
 int oxq_packed4_max_m(int k, int n, int group_size);
-/* 1 where oxq_packed4_matmul streams the packed words of this call through mma.sync (few tokens; groups of 32 up to 64; f16 scales, scratch of
- * oxq_packed4_full_scratch_bytes) and that is faster than the GEMVs and the other kernels; also beyond oxq_packed4_max_m. */
+/* 1 where oxq_packed4_matmul streams the packed words of this call (through mma.sync or tensor memory; f16 scales, scratch of
+ * oxq_packed4_full_scratch_bytes) and that is faster than the GEMVs and the other kernels; up to 256 tokens, also beyond oxq_packed4_max_m and for
+ * groups of 32. */
 int oxq_packed4_streams(int m, int k, int n, int group_size, int gptq);
 size_t oxq_packed4_scratch_bytes(int m, int n);
 size_t oxq_packed4_full_scratch_bytes(int m, int k, int n, int group_size, int gptq);

@@ -47,12 +47,24 @@ size_t stream4_scratch_bytes(int m, int n);
 int stream4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, const void *bias, int bias_dtype, void *y,
                    int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag, cudaStream_t st, int gptq, int sym, int gate,
                    void *scratch, size_t scratch_bytes);
+bool wide4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros, const void *scales,
+                     int gate);
+bool wide4_faster(int m, int k, int n, int group_size, int gptq);
+size_t wide4_scratch_bytes(int m, int k, int n, int group_size, int gate);
+int wide4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias, int bias_dtype,
+                 void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy, int *flag, cudaStream_t st, int gptq, int sym, int gate,
+                 void *scratch, size_t scratch_bytes);
 int awq_fused_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype, const void *bias,
                      int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base, int ldy,
                      int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes);
 
-// The 4-bit matmuls without a dense copy of the weight: csrc/stream4.cu for the few tokens that stream4_faster says, csrc/group_tc.cu up to
-// group_tc_max_m tokens, then csrc/fused_tc.cu up to 256.
+// The 4-bit matmuls without a dense copy of the weight: csrc/wide4.cu where wide4_faster says, csrc/stream4.cu for the few tokens that stream4_faster says,
+// csrc/group_tc.cu up to group_tc_max_m tokens, then csrc/fused_tc.cu up to 256.
+static bool packed4_wide(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros, const void *scales,
+                         int gptq, int gate = 0)
+{
+    return wide4_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gate) && wide4_faster(m, k, n, group_size, gptq);
+}
 static bool packed4_streams(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight, const void *qzeros, const void *scales,
                             int gptq, int gate = 0)
 {
@@ -61,17 +73,23 @@ static bool packed4_streams(int m, int k, int n, int group_size, int scales_dtyp
 static bool packed4_supported(int m, int k, int n, int group_size, int scales_dtype, const void *x, const void *qweight,
                               const void *qzeros, const void *scales, int gptq)
 {
-    return packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) || group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
+    return packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) ||
+           packed4_wide(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) || group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
            (aligned(qzeros, 16) && awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales));
 }
 static int packed4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int scales_dtype,
                           const void *bias, int bias_dtype, void *y, int y_dtype, int m, int k, int n, int group_size, int col_base,
                           int ldy, int *flag, cudaStream_t st, int gptq, int sym, void *scratch, size_t scratch_bytes)
 {
+    if (packed4_wide(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq)) {
+        const int rc = wide4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base, ldy, flag, st,
+                                    gptq, sym, 0, scratch, scratch_bytes);
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc; // scratch too small for the parts of tiles
+    }
     if (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq)) {
         const int rc = stream4_matmul(x, qweight, qzeros, scales, bias, bias_dtype, y, y_dtype, m, k, n, group_size, col_base, ldy, flag, st, gptq,
                                       sym, 0, scratch, scratch_bytes);
-        if (rc != OXQ_ERR_UNSUPPORTED) return rc; // scratch too small for the parts of tiles
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc;
     }
     if (!group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) &&
         !(aligned(qzeros, 16) && awq_fused_supported(m, k, n, group_size, scales_dtype, x, qweight, scales)))
@@ -209,10 +227,12 @@ static const char *wait_name(int code)
     case 65: return "packed words";
     case 66: return "operand slot";
     case 67: return "last MMAs";
-    // stream kernels (GGUF; 4-bit of few tokens)
+    // stream kernels (GGUF; 4-bit on mma.sync; 4-bit through tensor memory)
     case 81: return "ring slot";
     case 82: return "weights, x, or unpacked scales";
     case 83: return "weights";
+    case 84: return "operand or accumulator slot";
+    case 85: return "products";
     default: return "not one of a kernel's";
     }
 }
@@ -277,15 +297,18 @@ OXQ_EXPORT int oxq_packed4_max_m(int k, int n, int group_size)
 
 OXQ_EXPORT int oxq_packed4_streams(int m, int k, int n, int group_size, int gptq)
 {
-    return stream4_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, 0) && stream4_faster(m, k, n, group_size, gptq);
+    return packed4_streams(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, gptq) ||
+           packed4_wide(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, gptq);
 }
 
 OXQ_EXPORT size_t oxq_packed4_full_scratch_bytes(int m, int k, int n, int group_size, int gptq)
 {
     if (m <= 0 || k <= 0 || n <= 0 || n % 128 != 0 || k % 128 != 0 || group_size <= 0) return 0;
     size_t own = group_tc_scratch_bytes(m, n);
-    if (stream4_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, 0) && stream4_faster(m, k, n, group_size, gptq))
+    if (packed4_streams(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, gptq))
         own = own > stream4_scratch_bytes(m, n) ? own : stream4_scratch_bytes(m, n);
+    if (packed4_wide(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr, gptq))
+        own = own > wide4_scratch_bytes(m, k, n, group_size, 0) ? own : wide4_scratch_bytes(m, k, n, group_size, 0);
     const bool mxs = gptq && packed_mx_supported(m, k, n, group_size, OXQ_F16, nullptr, nullptr, nullptr, nullptr);
     const size_t mx = mxs ? packed_mx_scratch_bytes(m, k, n) : 0;
     return mx > own ? mx : own;
@@ -311,7 +334,8 @@ OXQ_EXPORT int oxq_packed4_matmul(const void *x, int x_dtype, const uint32_t *qw
     OXQ_REQUIRE(aligned(scratch, 256) && aligned(flag_word, 4), OXQ_ERR_BAD_ALIGN, "oxq_packed4_matmul: scratch must be 256-byte aligned");
     if (use_sym) qzeros = nullptr;
     OXQ_REQUIRE(group_tc_supported(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales) ||
-                    (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) && scratch_bytes >= stream4_scratch_bytes(m, n)),
+                    (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) && scratch_bytes >= stream4_scratch_bytes(m, n)) ||
+                    (packed4_wide(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, gptq) && scratch_bytes >= wide4_scratch_bytes(m, k, n, group_size, 0)),
                 OXQ_ERR_UNSUPPORTED, "oxq_packed4_matmul: out_features %d, in_features %d, group size %d or the alignment are not served", n, k, group_size);
     return packed4_matmul(x, qweight, qzeros, scales, scales_dtype, bias, bias_dtype, y, y_dtype, m, k, n, group_size, 0, n,
                           reinterpret_cast<int *>(flag_word), (cudaStream_t)stream, gptq, use_sym, scratch, scratch_bytes);
@@ -620,7 +644,12 @@ OXQ_EXPORT int oxq_awq_ffn_gate_up(const void *x, int x_dtype, const uint32_t *q
         OXQ_CUDA(cudaLaunchKernelEx(&cfg, gated_act_rows_kernel, (const __nv_bfloat16 *)c.slab, (__nv_bfloat16 *)y, m, inter, activation));
         return OXQ_OK;
     };
-    if (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, 0, activation)) { // gate and up meet in one tile: no row block, one launch
+    if (packed4_wide(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, 0, activation)) { // gate and up meet in one tile: no row block, one launch
+        rc = wide4_matmul(x, qweight, qzeros, scales, scales_dtype, nullptr, 0, y, OXQ_BF16, m, k, n, group_size, 0, inter, c.flag, c.st, 0, 0, activation,
+                          c.slab, c.slab_bytes);
+        if (rc != OXQ_ERR_UNSUPPORTED) return rc;
+    }
+    if (packed4_streams(m, k, n, group_size, scales_dtype, x, qweight, qzeros, scales, 0, activation)) {
         rc = stream4_matmul(x, qweight, qzeros, scales, nullptr, 0, y, OXQ_BF16, m, k, n, group_size, 0, inter, c.flag, c.st, 0, 0, activation, c.slab,
                             c.slab_bytes);
         if (rc != OXQ_ERR_UNSUPPORTED) return rc;

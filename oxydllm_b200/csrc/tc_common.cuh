@@ -184,16 +184,16 @@ inline EncodeTiledFn encode_tiled_fn()
 }
 
 
-// Tiled tensor maps of two and three dimensions through a small per-thread cache. A tensor map is a pure function of these arguments,
+// Tiled tensor maps of two to four dimensions through a small per-thread cache. A tensor map is a pure function of these arguments,
 // and the driver call that encodes one costs several microseconds, which a decode call cannot afford on every launch.
-inline CUresult encode_tiled_3d(CUtensorMap *out, CUtensorMapDataType dtype, const void *ptr, uint64_t dim0, uint64_t dim1, uint64_t dim2,
-                                uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2,
-                                CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promo)
+inline CUresult encode_tiled_4d(CUtensorMap *out, CUtensorMapDataType dtype, const void *ptr, uint64_t dim0, uint64_t dim1, uint64_t dim2, uint64_t dim3,
+                                uint64_t stride1_bytes, uint64_t stride2_bytes, uint64_t stride3_bytes, uint32_t box0, uint32_t box1, uint32_t box2,
+                                uint32_t box3, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promo)
 {
     struct Entry {
         const void *ptr;
-        uint64_t dim0, dim1, dim2, stride1, stride2;
-        uint32_t box0, box1, box2;
+        uint64_t dim0, dim1, dim2, dim3, stride1, stride2, stride3;
+        uint32_t box0, box1, box2, box3;
         int dtype, swizzle, promo, valid;
         CUtensorMap map;
     };
@@ -201,26 +201,32 @@ inline CUresult encode_tiled_3d(CUtensorMap *out, CUtensorMapDataType dtype, con
     static thread_local Entry cache[SLOTS];
     const uintptr_t a = reinterpret_cast<uintptr_t>(ptr);
     Entry &e = cache[((a >> 8) ^ (a >> 20) ^ box1 ^ (dim1 << 3)) & (SLOTS - 1)];
-    if (e.valid && e.ptr == ptr && e.dim0 == dim0 && e.dim1 == dim1 && e.dim2 == dim2 && e.stride1 == stride1_bytes &&
-        e.stride2 == stride2_bytes && e.box0 == box0 && e.box1 == box1 && e.box2 == box2 && e.dtype == (int)dtype &&
+    if (e.valid && e.ptr == ptr && e.dim0 == dim0 && e.dim1 == dim1 && e.dim2 == dim2 && e.dim3 == dim3 && e.stride1 == stride1_bytes &&
+        e.stride2 == stride2_bytes && e.stride3 == stride3_bytes && e.box0 == box0 && e.box1 == box1 && e.box2 == box2 && e.box3 == box3 && e.dtype == (int)dtype &&
         e.swizzle == (int)swizzle && e.promo == (int)promo) {
         *out = e.map;
         return CUDA_SUCCESS;
     }
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return CUDA_ERROR_NOT_SUPPORTED;
-    const cuuint64_t dims[3] = {dim0, dim1, dim2};
-    const cuuint64_t strides[2] = {stride1_bytes, stride2_bytes};
-    const cuuint32_t box[3] = {box0, box1, box2};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = fn(out, dtype, dim2 ? 3 : 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint64_t dims[4] = {dim0, dim1, dim2, dim3};
+    const cuuint64_t strides[3] = {stride1_bytes, stride2_bytes, stride3_bytes};
+    const cuuint32_t box[4] = {box0, box1, box2, box3};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = fn(out, dtype, dim3 ? 4 : dim2 ? 3 : 2, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           swizzle, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS) {
-        e.ptr = ptr; e.dim0 = dim0; e.dim1 = dim1; e.dim2 = dim2; e.stride1 = stride1_bytes; e.stride2 = stride2_bytes;
-        e.box0 = box0; e.box1 = box1; e.box2 = box2; e.dtype = (int)dtype; e.swizzle = (int)swizzle; e.promo = (int)promo;
+        e.ptr = ptr; e.dim0 = dim0; e.dim1 = dim1; e.dim2 = dim2; e.dim3 = dim3; e.stride1 = stride1_bytes; e.stride2 = stride2_bytes;
+        e.stride3 = stride3_bytes; e.box0 = box0; e.box1 = box1; e.box2 = box2; e.box3 = box3; e.dtype = (int)dtype; e.swizzle = (int)swizzle; e.promo = (int)promo;
         e.map = *out; e.valid = 1;
     }
     return r;
+}
+inline CUresult encode_tiled_3d(CUtensorMap *out, CUtensorMapDataType dtype, const void *ptr, uint64_t dim0, uint64_t dim1, uint64_t dim2,
+                                uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2,
+                                CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promo)
+{
+    return encode_tiled_4d(out, dtype, ptr, dim0, dim1, dim2, 0, stride1_bytes, stride2_bytes, 0, box0, box1, box2, 0, swizzle, promo);
 }
 inline CUresult encode_tiled_2d(CUtensorMap *out, CUtensorMapDataType dtype, const void *ptr, uint64_t dim0, uint64_t dim1,
                                 uint64_t stride1_bytes, uint32_t box0, uint32_t box1, CUtensorMapSwizzle swizzle,

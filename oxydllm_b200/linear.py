@@ -314,8 +314,8 @@ class PackedQuantLinear:
         return most, few if k <= max(reach - 1024, 1024) else 1, few
 
     def _streams(self, m: int) -> bool:
-        """Whether the kernel that streams the packed words through mma.sync is the best one for a batch (``oxq_packed4_streams``; the one
-        or two tokens of short GPTQ layers that ``_batches`` leaves to the GEMV stay there)."""
+        """Whether the kernels that stream the packed words (``csrc/stream4.cu``, ``csrc/wide4.cu``) are the best ones for a batch
+        (``oxq_packed4_streams``; the one or two tokens of short GPTQ layers that ``_batches`` leaves to the GEMV stay there)."""
         grouped, few, _ = self._batches
         gptq = self.pack_dim == "in"
         return (self.bits == 4 and self.scales.dtype == torch.float16 and not (gptq and grouped and m <= few)

@@ -1,5 +1,5 @@
-"""The kernels that stream GGUF blocks (``oxq_gguf_matmul``) and 4-bit words (``oxq_packed4_matmul`` where ``oxq_packed4_streams``) through mma.sync, at the
-sizes where they can go wrong, against the oracle."""
+"""The kernels that stream GGUF blocks (``oxq_gguf_matmul``) and 4-bit words (``oxq_packed4_matmul`` where ``oxq_packed4_streams``) through mma.sync or
+tensor memory, at the sizes where they can go wrong, against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -121,12 +121,20 @@ def packed(lin, x, out_dtype=torch.float32):
 # one unit and one tile; half a tile (n = 128, 384, 896); groups of 32, 64, 128, 256 and more; token blocks of 8 and 16, and two to four of them; few tiles in many
 # parts, shares across tile borders (n = 20480: 80 tiles on 148 SMs; 37888: 148 tiles)
 PACKED_SIZES = [("gptq", 1, 2048, 128, 32), ("gptq", 4, 128, 128, 128), ("gptq", 3, 1024, 384, 64), ("sym", 8, 4096, 896, 128), ("gptq", 9, 4096, 1152, 32), ("sym", 33, 4096, 128, 32),
-                ("gptq", 64, 4096, 1280, 32), ("gptq", 16, 2048, 37888, 64), ("gptq", 5, 4096, 512, 1024), ("sym", 2, 14336, 1024, 256), ("gptq", 16, 4096, 20480, 128),
+                ("gptq", 16, 2048, 37888, 64), ("gptq", 5, 4096, 512, 1024), ("sym", 2, 14336, 1024, 256), ("gptq", 16, 4096, 20480, 128),
                 ("awq", 1, 5632, 128, 128), ("awq", 8, 5632, 384, 128), ("awq", 3, 5632, 256, 512), ("awq", 8, 14336, 896, 64), ("awq", 9, 2048, 512, 32), ("awq", 17, 4096, 384, 32),
-                ("awq", 64, 4096, 1280, 32), ("awq", 1, 7168, 128, 32), ("awq", 16, 4096, 20480, 128), ("awq", 12, 8192, 3584, 64), ("awq", 7, 2048, 37888, 128)]
+                ("awq", 1, 7168, 128, 32), ("awq", 16, 4096, 20480, 128), ("awq", 12, 8192, 3584, 64), ("awq", 7, 2048, 37888, 128)]
+
+# through tensor memory: half a tile; every width of a tile of tokens and its edges; two and three blocks of tokens; groups of 32 to 1024; whole tiles, one
+# a CTA (n = 37888); clusters of two (n = 16384), five (6144) and eight; shares across tile borders (n = 38144: 149 tiles)
+WIDE_SIZES = [("awq", 9, 1024, 128, 128), ("awq", 16, 1024, 256, 64), ("awq", 17, 1024, 384, 128), ("awq", 32, 2048, 640, 64), ("awq", 33, 1024, 128, 32), ("awq", 48, 4096, 6144, 256),
+              ("awq", 64, 3072, 16384, 64), ("awq", 65, 2048, 384, 1024), ("awq", 80, 2048, 37888, 128), ("awq", 96, 4096, 1024, 32), ("awq", 97, 2048, 1280, 64), ("awq", 192, 1024, 896, 128),
+              ("awq", 193, 2048, 384, 128), ("awq", 256, 1024, 640, 64), ("awq", 17, 2048, 38144, 128), ("awq", 96, 1024, 38144, 64), ("awq", 3, 2048, 11264, 128),
+              ("gptq", 3, 2048, 128, 128), ("gptq", 9, 1024, 384, 128), ("sym", 31, 2048, 1152, 64), ("gptq", 49, 1024, 2048, 32), ("gptq", 77, 2048, 6144, 128), ("sym", 95, 14336, 128, 512),
+              ("gptq", 112, 2048, 1024, 64), ("gptq", 40, 3072, 38144, 128), ("gptq", 20, 8192, 2048, 256)]
 
 
-@pytest.mark.parametrize("fmt,m,k,n,g", PACKED_SIZES)
+@pytest.mark.parametrize("fmt,m,k,n,g", PACKED_SIZES + WIDE_SIZES)
 def test_packed_stream_matches_oracle(cuda, fmt, m, k, n, g):
     assert _lib.entry("oxq_packed4_streams")(m, k, n, g, int(fmt != "awq")) == 1
     x, bias = synth.activations(m, k, seed=k + m), synth.bf16_round(np.random.default_rng(1).standard_normal(n).astype(np.float32))
@@ -142,20 +150,21 @@ def test_packed_stream_matches_oracle(cuda, fmt, m, k, n, g):
 
 
 def test_packed_stream_infinite_and_missing_activations(cuda):
-    for fmt, k, n, g in (("awq", 5632, 384, 128), ("gptq", 4096, 384, 64), ("sym", 4096, 384, 32)):
+    for fmt, k, n, g, m in (("awq", 5632, 384, 128, 3), ("gptq", 16384, 384, 64, 3), ("sym", 4096, 384, 32, 3), ("awq", 2048, 384, 64, 40), ("gptq", 2048, 384, 32, 70)):
         lin, w = packed_layer(fmt, k, n, g, 3)
-        x = synth.activations(3, k, seed=4)
+        x = synth.activations(m, k, seed=4)
         x[0, 5], x[1, 700] = np.inf, np.nan
         got = packed(lin, torch.from_numpy(x).to(torch.bfloat16).cuda()).cpu().numpy()
         sign = np.sign(w[:, 5])
         assert np.array_equal(got[0][sign != 0], np.where(sign > 0, np.inf, -np.inf)[sign != 0]) and np.isnan(got[0][sign == 0]).all()
         assert np.isnan(got[1]).all()
-        ref, mass = x[2].astype(np.float64) @ w.T, np.abs(x[2]).astype(np.float64) @ np.abs(w).T
-        assert (np.abs(got[2] - ref) <= 2.0**-17 * mass + 1e-6).all()
+        ref, mass = x[2:].astype(np.float64) @ w.T, np.abs(x[2:]).astype(np.float64) @ np.abs(w).T
+        assert (np.abs(got[2:] - ref) <= 2.0**-17 * mass + 1e-6).all()
 
 
 @pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
-@pytest.mark.parametrize("m,k,inter,g", [(1, 5632, 128, 128), (8, 5632, 1152, 64), (16, 4096, 10240, 128), (33, 4096, 640, 32), (7, 2048, 18944, 128)])
+@pytest.mark.parametrize("m,k,inter,g", [(1, 5632, 128, 128), (8, 5632, 1152, 64), (16, 4096, 10240, 128), (33, 4096, 640, 32), (7, 2048, 18944, 128), (9, 2048, 640, 64), (20, 2048, 18944, 128),
+                                       (96, 1024, 19072, 128), (33, 1024, 19072, 64), (150, 2048, 384, 128)])
 def test_gate_and_up_meet_in_one_tile(cuda, m, k, inter, g, act):
     assert _lib.entry("oxq_packed4_streams")(m, k, 2 * inter, g, 0) == 1
     lin, w = packed_layer("awq", k, 2 * inter, g, m + inter)
@@ -175,3 +184,15 @@ def test_gate_and_up_meet_in_one_tile(cuda, m, k, inter, g, act):
         again.fill_(9.0)
         graph.replay()
         assert torch.equal(again, y)
+
+
+def test_wide_kernel_takes_bf16_scales(cuda):
+    k, n, g, m = 2048, 640, 64, 20
+    rng = np.random.default_rng(5)
+    qw, qz = (rng.integers(0, 2**32, shape, dtype=np.uint64).astype(np.uint32) for shape in ((k, n // 8), (k // g, n // 8)))
+    sc = synth.bf16_round(rng.uniform(0.001, 0.02, (k // g, n)).astype(np.float32))
+    lin = L.PackedQuantLinear(L.QuantWeight.new_awq(4, *(torch.from_numpy(a.view(np.int32)).cuda() for a in (qw, qz)), torch.from_numpy(sc).to(torch.bfloat16).cuda()))
+    x = synth.activations(m, k, seed=1)
+    w = oracle.awq_dequant(qw, qz, np.ones_like(sc, dtype=np.float16)).astype(np.float64) * np.repeat(sc.astype(np.float64), g, axis=0).T
+    got = packed(lin, torch.from_numpy(np.ascontiguousarray(x)).to(torch.bfloat16).cuda()).double().cpu().numpy()
+    assert (np.abs(got - x.astype(np.float64) @ w.T) <= 2.0**-17 * (np.abs(x).astype(np.float64) @ np.abs(w).T) + 1e-6).all()

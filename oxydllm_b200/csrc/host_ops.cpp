@@ -23,7 +23,7 @@ at::Tensor *g_flags[MAX_DEVICES], *g_workspaces[MAX_DEVICES];
 
 #define ENTRIES(X)                                                                                                                        \
     X(oxq_gguf_scratch_bytes) X(oxq_gguf_matmul) X(oxq_gguf_gemv) X(oxq_awq_gemv) X(oxq_w8a16_gemv) X(oxq_gptq_gemv)                      \
-    X(oxq_packed4_full_scratch_bytes) X(oxq_packed4_streams) X(oxq_packed4_matmul) X(oxq_awq_ffn_gate_up) X(oxq_gemm_workspace_bytes) X(oxq_fp8_gemv)            \
+    X(oxq_packed4_full_scratch_bytes) X(oxq_packed4_streams) X(oxq_packed4_matmul) X(oxq_awq_gemm) X(oxq_gptq_gemm) X(oxq_awq_ffn_gate_up) X(oxq_gemm_workspace_bytes) X(oxq_fp8_gemv)            \
     X(oxq_fp8_scratch_bytes) X(oxq_fp8_matmul)
 struct Entries {
 #define X(name) decltype(&::name) name;
@@ -196,7 +196,19 @@ PyObject *packed4(PyObject *const *a)
             return (nbits == 4 ? g.oxq_awq_gemv : g.oxq_w8a16_gemv)(x, OXQ_BF16, p.qw, p.qz, p.sc, p.sc_dt, b, b_dt, yp, OXQ_BF16, m, k, n, group, c.stream);
         });
     }
-    if (!aligned || (!streams && m > grouped) || !g_flags[c.device]) Py_RETURN_NONE;
+    if (!aligned || !g_flags[c.device]) Py_RETURN_NONE;
+    if (!streams && m > grouped) { // the dense copy and its GEMM: 15.8 us a call of 327 x 3072 x 1024 by way of Python were the call itself
+        if (nbits != 4 || (!in && !p.qz) || !g_workspaces[c.device]) Py_RETURN_NONE;
+        const at::Tensor ws = *g_workspaces[c.device]; // ours until the launch is done, should another thread let it grow
+        const size_t bytes = (size_t)ws.numel();
+        if (bytes < g.oxq_gemm_workspace_bytes(n, k)) Py_RETURN_NONE; // Python lets it grow
+        at::Tensor y = result(c, n, at::kBFloat16);
+        void *yp = y.data_ptr(), *wp = ws.data_ptr();
+        return finish(y, [&] {
+            if (in) return g.oxq_gptq_gemm(x, OXQ_BF16, p.qw, p.qz, p.sc, p.sc_dt, b, b_dt, yp, OXQ_BF16, m, k, n, group, nbits, sym || !p.qz, wp, bytes, c.stream);
+            return g.oxq_awq_gemm(x, OXQ_BF16, p.qw, p.qz, p.sc, p.sc_dt, b, b_dt, yp, OXQ_BF16, m, k, n, group, wp, bytes, c.stream);
+        });
+    }
     const size_t need = g.oxq_packed4_full_scratch_bytes(m, k, n, group, in);
     at::Tensor y = result(c, n, at::kBFloat16), scratch = empty(c, {(int64_t)need}, at::kByte);
     void *yp = y.data_ptr(), *flag = g_flags[c.device]->data_ptr(), *sp = scratch.data_ptr();

@@ -318,7 +318,7 @@ class PackedQuantLinear:
         (``oxq_packed4_streams``; the one or two tokens of short GPTQ layers that ``_batches`` leaves to the GEMV stay there)."""
         grouped, few, _ = self._batches
         gptq = self.pack_dim == "in"
-        return (self.bits == 4 and self.scales.dtype == torch.float16 and not (gptq and grouped and m <= few)
+        return (self.bits == 4 and m <= 256 and self.scales.dtype == torch.float16 and not (gptq and grouped and m <= few)
                 and bool(_lib.entry("oxq_packed4_streams")(m, self.in_features, self.out_features, self.group_size, int(gptq))))
 
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

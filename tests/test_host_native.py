@@ -36,7 +36,7 @@ def _layers():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("m", [1, 3, 8, 9, 16, 33, 70])
+@pytest.mark.parametrize("m", [1, 3, 8, 9, 16, 33, 70, 300])
 def test_same_results_as_the_python_code(cuda, m, monkeypatch):
     """Batches on both sides of the choices, x of two and three dimensions, on 16 and 8 bytes, and strided."""
     flat = torch.from_numpy(synth.activations(2 * m, 512, seed=m)).to(torch.bfloat16).cuda()

@@ -1,4 +1,4 @@
-// AWQ / GPTQ W4A16 matmul of up to 256 tokens (above the batches that group_tc.cu takes) with the dequantization
+// AWQ / GPTQ W4A16 matmul of up to 256 tokens (above the batches that group_tc.cu and wide4.cu take) with the dequantization
 // fused into the tensor-core kernel: the packed words are read from HBM once and no dense copy of the weight is ever written.
 //
 // One CTA owns 128 out features and walks k in stages of 64 input rows:

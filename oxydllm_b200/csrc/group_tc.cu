@@ -1,4 +1,5 @@
-// AWQ and GPTQ 4-bit matmul with the unpack inside the tensor-core kernel and the quantization scale behind it.
+// AWQ and GPTQ 4-bit matmul with the unpack inside the tensor-core kernel and the quantization scale behind it: what csrc/stream4.cu and csrc/wide4.cu leave, mostly
+// wide layers from 97 tokens on and up to 16 tokens of bf16 scales.
 //
 // The operand that meets the activations is the integer q - z (exact in bf16); a quantization group's product
 // leaves tensor memory once, is multiplied by the group's scale in f32 and added to f32 totals in registers:

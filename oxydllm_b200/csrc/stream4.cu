@@ -28,9 +28,7 @@ constexpr int S4_MAX_STAGES = 4;
 constexpr int S4_MAX_BLOCK = 16;                       // tokens of a tile
 
 struct Stream4Params {
-    const uint32_t *qzeros;
-    const uint16_t *scales;
-    int sym, n, packed_out;
+    int sym, n;
     int gshift;       // log2(group size)
     int stages;
     int half1;        // out feature at which the second half of tile 0 begins
@@ -39,13 +37,15 @@ struct Stream4Params {
     StreamOut out;
 };
 
+struct Stream4Maps { CUtensorMap words, x, scales, zeros; };
+
 // NG: quantization groups of a unit, 1, 2 or 4. MT: eights of tokens.
 template <bool GPTQ, int NG, int MT>
 __global__ void __launch_bounds__(S4_THREADS, 1)
-    packed4_stream_kernel(const Stream4Params p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap)
+    packed4_stream_kernel(const Stream4Params p, const __grid_constant__ Stream4Maps maps)
 {
     constexpr int KG = S4_KG, SLOT = S4_W_BYTES + 2 * MT * S4_X_BYTES; // x: [64 rows][eight tokens]
-    constexpr int Z_AT = 2 * NG * 256, META = (2 * NG * (256 + 64) + 127) / 128 * 128; // scales [half][group][128], zero points [half][group][16 words]
+    constexpr int Z_AT = 2 * NG * 256, META = (2 * NG * (256 + 64) + 127) / 128 * 128; // scales [group][half][128], zero points [group][half][16 words]
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[KG * S4_MAX_STAGES * 2];
     __shared__ uint32_t last, helped;
@@ -62,8 +62,10 @@ __global__ void __launch_bounds__(S4_THREADS, 1)
             mbar_init(empty + 8 * s, 4);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.words) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.scales) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.zeros) : "memory");
     }
     __syncthreads();
     pdl_wait();
@@ -78,35 +80,23 @@ __global__ void __launch_bounds__(S4_THREADS, 1)
         return;
     }
     if (warp >= 4 * KG) {
-        // ---- producer of one k group -----------------------------------------------------------------------------
-        const uint32_t meta = (uint32_t)NG * (256u + (p.sym ? 0u : 64u));
+        // ---- producer of one k group: four copies a unit (about 130 clocks each to issue; eight, for each half and group: 19.0 us, with four 18.6, 4096 x 28672) -----------------------------
+        const uint32_t bytes = S4_W_BYTES + 2 * MT * S4_X_BYTES + (uint32_t)NG * (p.sym ? 512u : 640u);
         for (int u = u0; u < u1;) {
             const int tile = u / G, seg_end = min(u1, (tile + 1) * G), cnt = seg_end - u;
-            const int f0 = tile / p.out.tok_blocks * p.tile_step, f1 = f0 + p.half1; // first out features of the halves
-            const int halves = f1 < p.n ? 2 : 1, tok0 = tile % p.out.tok_blocks * p.out.tok_step;
-            int k0 = (u + cnt * kg / KG - tile * G) * S4_UNIT;
-            for (const int end = (u + cnt * (kg + 1) / KG - tile * G) * S4_UNIT; k0 < end; k0 += S4_UNIT) {
+            const int ft = tile / p.out.tok_blocks, block = p.out.gate ? ft : 2 * ft, tok0 = tile % p.out.tok_blocks * p.out.tok_step; // block: of 128 out features
+            int kb = u + cnt * kg / KG - tile * G;
+            for (const int end = u + cnt * (kg + 1) / KG - tile * G; kb < end; kb++) {
                 if (!mx_wait(empty + 8 * s, ph ^ 1u, p.flag, ST_CODE + 1)) return;
                 const uint32_t slot = smem_u32(slots) + (uint32_t)((kg * S + s) * SLOT), sc = smem_u32(metas) + (uint32_t)((kg * S + s) * META), bar = full + 8 * s;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(bar, (uint32_t)halves * (S4_HALF_BYTES + meta) + 2 * MT * S4_X_BYTES);
-                    for (int h = 0; h < halves; h++) {
-                        const int f = h ? f1 : f0;
-                        if constexpr (GPTQ)
-                            asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                                         ::"r"(slot + h * S4_HALF_BYTES), "l"(&wmap), "r"(bar), "r"(0), "r"(k0 >> 3), "r"(f >> 5) : "memory");
-                        else tma_load_2d(slot + h * S4_HALF_BYTES, &wmap, bar, f >> 3, k0);
-                        const size_t row = (size_t)(k0 >> p.gshift);
-                        const uint16_t *scales = p.scales + row * p.n + f;
-                        const uint32_t *zeros = p.qzeros + row * p.packed_out + (f >> 3);
-#pragma unroll
-                        for (int g = 0; g < NG; g++) {
-                            bulk_copy_g2s(sc + (uint32_t)(h * NG + g) * 256u, scales + (size_t)g * p.n, 256, bar);
-                            if (!p.sym) bulk_copy_g2s(sc + Z_AT + (uint32_t)(h * NG + g) * 64u, zeros + (size_t)g * p.packed_out, 64, bar);
-                        }
-                    }
-                    tma_load_2d(slot + S4_W_BYTES, &xmap, bar, k0, tok0);
-                    tma_load_2d(slot + S4_W_BYTES + MT * S4_X_BYTES, &xmap, bar, k0 + 64, tok0);
+                    mbar_arrive_expect_tx(bar, bytes);
+                    const int group = (kb * S4_UNIT) >> p.gshift;
+                    if constexpr (GPTQ) st_load_3d(slot, &maps.words, bar, kb * (S4_UNIT / 8), block * 4);
+                    else st_load_4d(slot, &maps.words, bar, kb * S4_UNIT, block, 0);
+                    st_load_3d(slot + S4_W_BYTES, &maps.x, bar, tok0, 2 * kb);
+                    st_load_4d(sc, &maps.scales, bar, block, 0, group);
+                    if (!p.sym) st_load_4d(sc + Z_AT, &maps.zeros, bar, block, 0, group);
                 }
                 __syncwarp();
                 if (++s == S) { s = 0; ph ^= 1u; }
@@ -126,8 +116,8 @@ __global__ void __launch_bounds__(S4_THREADS, 1)
     // GPTQ: four neighbouring out features of a packed row (eight input rows); [block of 32 features][16 packed rows][128 bytes], swizzled
     const int q_off = half * S4_HALF_BYTES + (cg & 1) * 4096;
     const uint32_t odd = (g & 1) ? 0x7632u : 0x5410u;
-    const int sc_off = half * NG * 256 + (cg & 1) * 128 + (GPTQ ? g * 8 : (g >> 1) * 16);
-    const int z_off = Z_AT + half * NG * 64 + (cg & 1) * 32 + (g >> 1) * 4;
+    const int sc_off = half * 256 + (cg & 1) * 128 + (GPTQ ? g * 8 : (g >> 1) * 16);
+    const int z_off = Z_AT + half * 64 + (cg & 1) * 32 + (g >> 1) * 4;
     float tot[4][MT][4];
     bool ok = true;
     bool others = false;
@@ -152,7 +142,7 @@ __global__ void __launch_bounds__(S4_THREADS, 1)
                 // zero points: bf16 pairs 128 + z. AWQ: out features of 16-bit halves g and g + 8; GPTQ: 4 g .. 4 g + 3 of the two blocks of 32
                 uint32_t zz[8];
                 {
-                    const unsigned char *at = sc + z_off + grp * 64;
+                    const unsigned char *at = sc + z_off + grp * 128;
                     const bool none = GPTQ && p.sym;
                     const uint32_t w[2] = {none ? 0x77777777u : st_lds<uint32_t>(at), none ? 0x77777777u : st_lds<uint32_t>(at + 16)};
 #pragma unroll
@@ -223,7 +213,7 @@ __global__ void __launch_bounds__(S4_THREADS, 1)
                     }
                 }
                 // scales of the accumulator rows g and g + 8 of the four products
-                const unsigned char *at = sc + sc_off + grp * 256;
+                const unsigned char *at = sc + sc_off + grp * 512;
                 float2 s01[2], s23[2];
                 if constexpr (!GPTQ) {
                     const uint4 lo = st_lds<uint4>(at), hi = st_lds<uint4>(at + 64);
@@ -324,7 +314,7 @@ size_t stream4_scratch_bytes(int m, int n)
 }
 
 template <bool GPTQ, int NG, int MT>
-static int s4_launch(Stream4Params &p, const CUtensorMap &wmap, const CUtensorMap &xmap, int ctas, cudaStream_t st)
+static int s4_launch(Stream4Params &p, const Stream4Maps &maps, int ctas, cudaStream_t st)
 {
     auto kern = packed4_stream_kernel<GPTQ, NG, MT>;
     const size_t slot = S4_W_BYTES + 2 * MT * S4_X_BYTES + (2 * NG * (256 + 64) + 127) / 128 * 128;
@@ -348,7 +338,7 @@ static int s4_launch(Stream4Params &p, const CUtensorMap &wmap, const CUtensorMa
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     allow_early_start(attr, cfg.numAttrs);
-    OXQ_CUDA(cudaLaunchKernelEx(&cfg, kern, p, wmap, xmap));
+    OXQ_CUDA(cudaLaunchKernelEx(&cfg, kern, p, maps));
     return OXQ_OK;
 }
 
@@ -359,9 +349,8 @@ int stream4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzero
 {
     if (!scratch || scratch_bytes < stream4_scratch_bytes(m, n)) return OXQ_ERR_UNSUPPORTED;
     Stream4Params p = {};
-    p.qzeros = qzeros; p.scales = reinterpret_cast<const uint16_t *>(scales);
     p.sym = (gptq && (sym || qzeros == nullptr)) ? 1 : 0;
-    p.n = n; p.packed_out = n / 8; p.flag = flag;
+    p.n = n; p.flag = flag;
     while ((1 << p.gshift) < group_size) p.gshift += 1;
     p.tile_step = gate ? S4_COLS / 2 : S4_COLS;
     p.half1 = gate ? n / 2 : S4_COLS / 2;
@@ -380,23 +369,17 @@ int stream4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzero
     o.partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + s4_flag_bytes(tiles));
     const int ctas = st_ctas(o, o.tok_step <= 8 ? 40 : 55, 235 + 13 * o.tok_step, 12 + 17 * o.tok_step / 10, 600 + 45 * o.tok_step);
 
-    CUtensorMap wmap, xmap;
-    CUresult r;
-    if (gptq)
-        r = encode_tiled_3d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, 32, (uint64_t)k / 8, (uint64_t)n / 32, (uint64_t)n * 4, 128, 32,
-                            S4_UNIT / 8, 4, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    else
-        r = encode_tiled_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, (uint64_t)p.packed_out, (uint64_t)k, (uint64_t)p.packed_out * 4, 16,
-                            S4_UNIT, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (weights) failed with CUresult %d", (int)r);
     const int mt = o.tok_step <= 8 ? 1 : 2;
-    r = encode_tiled_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, (uint64_t)k, (uint64_t)m, (uint64_t)k * 2, 64, 8 * mt,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    Stream4Maps maps;
+    const int rc = st_packed4_maps(maps.words, maps.scales, maps.zeros, qweight, p.sym ? nullptr : qzeros, scales, k, n, group_size, gptq, gate);
+    if (rc) return rc;
+    const CUresult r = encode_tiled_3d(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, 64, (uint64_t)m, (uint64_t)k / 64, (uint64_t)k * 2, 128, 64, 8 * mt, 2,
+                                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (x) failed with CUresult %d", (int)r);
     const int ng = group_size >= 128 ? 1 : group_size == 64 ? 2 : 4;
 #define S4_RUN(GPTQ_, MT_)                                                                                                      \
-    return ng == 1 ? s4_launch<GPTQ_, 1, MT_>(p, wmap, xmap, ctas, st) : ng == 2 ? s4_launch<GPTQ_, 2, MT_>(p, wmap, xmap, ctas, st) \
-                                                                       : s4_launch<GPTQ_, 4, MT_>(p, wmap, xmap, ctas, st)
+    return ng == 1 ? s4_launch<GPTQ_, 1, MT_>(p, maps, ctas, st) : ng == 2 ? s4_launch<GPTQ_, 2, MT_>(p, maps, ctas, st) \
+                                                                       : s4_launch<GPTQ_, 4, MT_>(p, maps, ctas, st)
     if (gptq && mt == 1) S4_RUN(true, 1);
     if (gptq) S4_RUN(true, 2);
     if (mt == 1) S4_RUN(false, 1);

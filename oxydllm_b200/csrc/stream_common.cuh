@@ -47,6 +47,45 @@ __device__ __forceinline__ uint32_t st_sub2(uint32_t a, uint32_t b) // bf16 pair
 
 __device__ __forceinline__ float2 st_f16x2(uint32_t two) { return __half22float2(*reinterpret_cast<const __half2 *>(&two)); }
 
+__device__ __forceinline__ void st_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c1, int c2, int c3)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+__device__ __forceinline__ void st_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c1, int c2)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2) : "memory");
+}
+
+// Tensor maps of a 4-bit weight for units of 128 input rows x two blocks of 128 out features, of 16-bit scales and of zero points (null: none) for the
+// groups of a unit. For a gated projection dimension 2 of a pair is the gate's block and 3 its partner's, else the two are neighbours in one dimension; a block
+// beyond n reads as zeros.
+inline int st_packed4_maps(CUtensorMap &words, CUtensorMap &smap, CUtensorMap &zmap, const uint32_t *qweight, const uint32_t *qzeros, const void *scales, int k,
+                           int n, int group_size, int gptq, int gate)
+{
+    const uint64_t blocks = gate ? (uint64_t)n / 256 : (uint64_t)n / 128, pair = gate ? 2 : 1, row4 = (uint64_t)n / 2, row2 = (uint64_t)n * 2;
+    const uint32_t box_blocks = gate ? 1 : 2, box_pair = gate ? 2 : 1, groups = group_size >= 128 ? 1 : 128 / group_size;
+    CUresult r;
+    if (gptq)
+        r = encode_tiled_3d(&words, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, 32, (uint64_t)k / 8, (uint64_t)n / 32, (uint64_t)n * 4, 128, 32, 16, 8,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    else
+        r = encode_tiled_4d(&words, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, 16, (uint64_t)k, blocks, pair, row4, 64, gate ? row4 / 2 : row4, 16, 128, box_blocks,
+                            box_pair, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (weights) failed with CUresult %d", (int)r);
+    r = encode_tiled_4d(&smap, CU_TENSOR_MAP_DATA_TYPE_UINT16, scales, 128, blocks, pair, (uint64_t)k / group_size, 256, gate ? row2 / 2 : 256, row2, 128, box_blocks,
+                        box_pair, groups, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (scales) failed with CUresult %d", (int)r);
+    zmap = smap;
+    if (qzeros) {
+        r = encode_tiled_4d(&zmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, qzeros, 16, blocks, pair, (uint64_t)k / group_size, 64, gate ? row4 / 2 : 64, row4, 16, box_blocks,
+                            box_pair, groups, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+        OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (zero points) failed with CUresult %d", (int)r);
+    }
+    return OXQ_OK;
+}
+
 struct StreamOut {
     const void *bias;
     void *y;

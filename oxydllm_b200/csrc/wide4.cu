@@ -49,16 +49,6 @@ struct Wide4Params {
 template <int V> struct W4Int { static constexpr int value = V; };
 struct Wide4Maps { CUtensorMap words, x, scales, zeros; };
 
-__device__ __forceinline__ void w4_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c1, int c2, int c3)
-{
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ void w4_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c1, int c2)
-{
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2) : "memory");
-}
 __device__ __forceinline__ void w4_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void w4_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ float w4_peer(uint32_t addr, int rank) // shared memory of a CTA of the cluster
@@ -156,12 +146,12 @@ __global__ void __launch_bounds__(W4_THREADS, 1)
                         mbar_arrive_expect_tx(bar, bytes);
                         const int group = (kb * W4_UNIT) >> p.gshift;
                         if (warp == 0) {
-                            if constexpr (GPTQ) w4_load_3d(slot, &maps.words, bar, kb * (W4_UNIT / 8), block * 4);
-                            else w4_load_4d(slot, &maps.words, bar, kb * W4_UNIT, block, 0);
-                            if (!p.sym) w4_load_4d(slot + z_at, &maps.zeros, bar, block, 0, group);
+                            if constexpr (GPTQ) st_load_3d(slot, &maps.words, bar, kb * (W4_UNIT / 8), block * 4);
+                            else st_load_4d(slot, &maps.words, bar, kb * W4_UNIT, block, 0);
+                            if (!p.sym) st_load_4d(slot + z_at, &maps.zeros, bar, block, 0, group);
                         } else {
-                            w4_load_3d(slot + W4_W_BYTES, &maps.x, bar, tok0, 2 * kb);
-                            w4_load_4d(slot + s_at, &maps.scales, bar, block, 0, group);
+                            st_load_3d(slot + W4_W_BYTES, &maps.x, bar, tok0, 2 * kb);
+                            st_load_4d(slot + s_at, &maps.scales, bar, block, 0, group);
                         }
                     }
                     __syncwarp();
@@ -690,31 +680,12 @@ int wide4_matmul(const void *x, const uint32_t *qweight, const uint32_t *qzeros,
     o.flags = reinterpret_cast<unsigned long long *>(scratch);
     o.partials = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + w4_flag_bytes(tiles));
     const int ctas = w4_plan(o, p.npad, p.groups, p.cluster);
-    // Blocks of 128 out features: for a gated projection dimension 2 of a pair is the gate's block and 3 its partner's, else two neighbours of one dimension;
-    // a block beyond n reads as zeros.
     Wide4Maps maps;
-    const uint64_t blocks = gate ? (uint64_t)n / 256 : (uint64_t)n / 128, pair = gate ? 2 : 1, row4 = (uint64_t)n / 2, row2 = (uint64_t)n * 2;
-    const uint32_t box_blocks = gate ? 1 : 2, box_pair = gate ? 2 : 1;
-    CUresult r;
-    if (gptq)
-        r = encode_tiled_3d(&maps.words, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, 32, (uint64_t)k / 8, (uint64_t)n / 32, (uint64_t)n * 4, 128, 32,
-                            W4_UNIT / 8, 8, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    else
-        r = encode_tiled_4d(&maps.words, CU_TENSOR_MAP_DATA_TYPE_UINT32, qweight, 16, (uint64_t)k, blocks, pair, row4, 64, gate ? row4 / 2 : row4, 16, W4_UNIT, box_blocks,
-                            box_pair, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (weights) failed with CUresult %d", (int)r);
-    r = encode_tiled_3d(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, 64, (uint64_t)m, (uint64_t)k / 64, (uint64_t)k * 2, 128, 64, (uint32_t)p.npad, 2,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    const int rc = st_packed4_maps(maps.words, maps.scales, maps.zeros, qweight, p.sym ? nullptr : qzeros, scales, k, n, group_size, gptq, gate);
+    if (rc) return rc;
+    const CUresult r = encode_tiled_3d(&maps.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, 64, (uint64_t)m, (uint64_t)k / 64, (uint64_t)k * 2, 128, 64, (uint32_t)p.npad, 2,
+                                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (x) failed with CUresult %d", (int)r);
-    r = encode_tiled_4d(&maps.scales, CU_TENSOR_MAP_DATA_TYPE_UINT16, scales, 128, blocks, pair, (uint64_t)k / group_size, 256, gate ? row2 / 2 : 256, row2, 128,
-                        box_blocks, box_pair, (uint32_t)p.groups, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-    OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (scales) failed with CUresult %d", (int)r);
-    maps.zeros = maps.scales;
-    if (!p.sym) {
-        r = encode_tiled_4d(&maps.zeros, CU_TENSOR_MAP_DATA_TYPE_UINT32, qzeros, 16, blocks, pair, (uint64_t)k / group_size, 64, gate ? row4 / 2 : 64, row4, 16,
-                            box_blocks, box_pair, (uint32_t)p.groups, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-        OXQ_REQUIRE(r == CUDA_SUCCESS, OXQ_ERR_CUDA, "cuTensorMapEncodeTiled (zero points) failed with CUresult %d", (int)r);
-    }
 #define W4_RUN(GPTQ_)                                                                   \
     switch (p.npad / 16) {                                                              \
     case 1: return w4_launch<GPTQ_, 1>(p, maps, ctas, st);                        \
